@@ -469,7 +469,8 @@ int rte_transpose_f32(const float* src, void* dst, int32_t rows, int32_t cols, i
  * row norms of w_down.  Candidates = union of the top up_m / gate_m / product_m neurons under |up_hat|*wn,
  * |silu(gate_hat)|*wn, |up_hat*silu(gate_hat)|*wn; selected = top top_k candidates under |up*silu(gate)|*wn
  * (ties: lowest index).  z_masked bf16 [rows, F] = selected ? up*silu(gate) : 0; selected uint8 [rows, F] and
- * cand_count int32 [rows] optional.  max(up_m, gate_m, product_m) >= top_k is required.
+ * cand_count int32 [rows] optional.  max(up_m, gate_m, product_m) >= top_k is required; wd_norm is not negative; hats
+ * and wd_norm start on 16 bytes, ug and z_masked on 8, selected on 4 (RTE_ERR_ALIGNMENT otherwise).
  * rte_svd_ffn_swiglu_bwd: dug bf16 [rows, 2F] = SwiGLU backward of dz bf16 [rows, F] on selected neurons, else 0.
  * rte_row_norm_f32: out[r] = ||w[r, :]||_2.                                                                    */
 int rte_svd_ffn_select(const float* hats, const void* ug, const float* wd_norm, void* z_masked, uint8_t* selected,

@@ -45,6 +45,40 @@ def test_radix_select_is_the_stable_topk_with_constructed_ties(rows, F_, k):
     assert (cnt.cpu() == k).all() and (z.cpu() == 0).all()
 
 
+@pytest.mark.parametrize("rows,F_,k", [(5000, 104, 13), (3, 4, 1), (64, 2048, 2047), (40, 9984, 700), (2500, 256, 256)])
+def test_threshold_search_selects_the_k_largest_in_every_row(rows, F_, k):
+    """The threshold search over many tokens per warp: rows of continuous scores (it ends on a probe or by ranking the
+    last few keys), rows of two values (more equal keys than it ranks) and rows of very different scale in turn."""
+    ops = CudaOps(DEV)
+    g = torch.Generator().manual_seed(rows + F_)
+    uh = torch.randn(rows, F_, generator=g) * torch.logspace(-6, 6, rows).roll(rows // 2).unsqueeze(1)
+    uh[::3] = (uh[::3] > 0).float()
+    hats = torch.cat([uh, torch.zeros(rows, F_)], dim=1)
+    ug = torch.cat([uh, torch.ones(rows, F_)], dim=1).bfloat16()
+    z = torch.empty(rows, F_, dtype=torch.bfloat16, device=DEV)
+    sel = torch.empty(rows, F_, dtype=torch.uint8, device=DEV)
+    cnt = torch.empty(rows, dtype=torch.int32, device=DEV)
+    ops.svd_ffn_select(hats.to(DEV), ug.to(DEV), torch.ones(F_, device=DEV), z, sel, cnt, up_m=k, gate_m=0, product_m=0, top_k=k)
+    torch.cuda.synchronize()
+    want = O.topk_membership(uh.abs(), k)
+    assert torch.equal(sel.cpu().bool(), want) and (cnt.cpu() == k).all()
+    assert torch.equal(z.cpu() != 0, want & (ug[:, :F_] != 0))
+
+
+@pytest.mark.parametrize("rows,F_", [(37, 2048), (5, 100)])            # eight neurons per thread | one
+def test_swiglu_backward_of_the_selected_neurons(rows, F_):
+    ops = CudaOps(DEV)
+    g = torch.Generator().manual_seed(F_)
+    ug, dz = (torch.randn(rows, n, generator=g).bfloat16() for n in (2 * F_, F_))
+    sel = torch.rand(rows, F_, generator=g) < 0.15
+    dug = torch.empty(rows, 2 * F_, dtype=torch.bfloat16, device=DEV)
+    ops.svd_ffn_swiglu_bwd(ug.to(DEV), dz.to(DEV), sel.to(torch.uint8).to(DEV), dug)
+    leaf = ug.float().requires_grad_()
+    (leaf[:, :F_] * torch.nn.functional.silu(leaf[:, F_:]) * sel * dz.float()).sum().backward()
+    _close(dug, leaf.grad)
+    assert (dug.cpu().view(rows, 2, F_)[~sel.unsqueeze(1).expand(rows, 2, F_)] == 0).all()
+
+
 def _module(t, c, max_tokens):
     dev = lambda k: t[k].to(DEV)  # noqa: E731
     return SVDFactorSparseFFN(dev("w_up"), dev("w_gate"), dev("w_down"), t["up_a"], t["up_b"], t["gate_a"], t["gate_b"],
