@@ -60,6 +60,7 @@ template <int HD, int SMAX>
 __global__ void __launch_bounds__(ATT_THREADS)
 attn_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, int ld, int sec, __nv_bfloat16* __restrict__ y, int ldy,
                 float* __restrict__ lse, const float* __restrict__ rope, int S, int H) {
+  rte::after_previous_grid();
   constexpr int LDS = AttCfg<HD>::LDS, DPL = AttCfg<HD>::DPL, NT = SMAX / 32;
   extern __shared__ __align__(16) uint8_t smraw[];
   __nv_bfloat16* sq = reinterpret_cast<__nv_bfloat16*>(smraw);
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(ATT_THREADS)
 attn_bwd_kernel(const __nv_bfloat16* __restrict__ qkv, int ld, int sec, const __nv_bfloat16* __restrict__ y,
                 const __nv_bfloat16* __restrict__ dy, int ldy, const float* __restrict__ lse,
                 __nv_bfloat16* __restrict__ dqkv, const float* __restrict__ rope, int S, int H) {
+  rte::after_previous_grid();
   constexpr int LDS = AttCfg<HD>::LDS, DPL = AttCfg<HD>::DPL, NT = SMAX / 32;
   extern __shared__ __align__(16) uint8_t smraw[];
   __nv_bfloat16* sq = reinterpret_cast<__nv_bfloat16*>(smraw);
@@ -271,7 +273,7 @@ int launch_fwd(const void* qkv, int ld, int sec, void* y, int ldy, float* lse, c
       return RTE_ERR_LAUNCH;
     set = true;
   }
-  attn_fwd_kernel<HD, SMAX><<<B * H, ATT_THREADS, smem, st>>>(reinterpret_cast<const __nv_bfloat16*>(qkv), ld, sec,
+  rte::launch(attn_fwd_kernel<HD, SMAX>, B * H, ATT_THREADS, smem, st, reinterpret_cast<const __nv_bfloat16*>(qkv), ld, sec,
       reinterpret_cast<__nv_bfloat16*>(y), ldy, lse, rope, S, H);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -286,7 +288,7 @@ int launch_bwd(const void* qkv, int ld, int sec, const void* y, const void* dy, 
       return RTE_ERR_LAUNCH;
     set = true;
   }
-  attn_bwd_kernel<HD, SMAX><<<B * H, ATT_THREADS, smem, st>>>(reinterpret_cast<const __nv_bfloat16*>(qkv), ld, sec,
+  rte::launch(attn_bwd_kernel<HD, SMAX>, B * H, ATT_THREADS, smem, st, reinterpret_cast<const __nv_bfloat16*>(qkv), ld, sec,
       reinterpret_cast<const __nv_bfloat16*>(y), reinterpret_cast<const __nv_bfloat16*>(dy), ldy, lse,
       reinterpret_cast<__nv_bfloat16*>(dqkv), rope, S, H);
   RTE_LAUNCH_CHECK();
@@ -294,6 +296,7 @@ int launch_bwd(const void* qkv, int ld, int sec, const void* y, const void* dy, 
 }
 
 __global__ void rope_table_kernel(float* __restrict__ out, int S, int hd) {
+  rte::after_previous_grid();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= S * (hd / 2)) return;
   float sn, cs;
@@ -308,6 +311,7 @@ __global__ void rope_table_kernel(float* __restrict__ out, int S, int hd) {
 template <typename T>
 __global__ void rope_apply_kernel(const T* __restrict__ x, const float* __restrict__ cs, const float* __restrict__ sn,
                                   T* __restrict__ out, long long pairs, int S, int hd, int adjoint) {
+  rte::after_previous_grid();
   const int hp = hd / 2;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < pairs; i += (long long)gridDim.x * blockDim.x) {
     const int pr = (int)(i % hp);
@@ -369,7 +373,7 @@ __global__ void rope_apply_kernel(const T* __restrict__ x, const float* __restri
 extern "C" int rte_rope_table(float* out, int32_t S, int32_t head_dim, rte_stream_t stream) {
   RTE_CHECK_ARG(out && S > 0 && head_dim > 0 && head_dim % 2 == 0);
   const int n = S * (head_dim / 2);
-  rope_table_kernel<<<rte::ceil_div(n, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(out, S, head_dim);
+  rte::launch(rope_table_kernel, rte::ceil_div(n, 256), 256, 0, reinterpret_cast<cudaStream_t>(stream), out, S, head_dim);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -382,10 +386,10 @@ extern "C" int rte_rope_apply(const void* x, const float* cos_tab, const float* 
   if (g > 148 * 16) g = 148 * 16;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (is_bf16)
-    rope_apply_kernel<__nv_bfloat16><<<(int)g, 256, 0, st>>>(reinterpret_cast<const __nv_bfloat16*>(x), cos_tab, sin_tab,
+    rte::launch(rope_apply_kernel<__nv_bfloat16>, (int)g, 256, 0, st, reinterpret_cast<const __nv_bfloat16*>(x), cos_tab, sin_tab,
                                                             reinterpret_cast<__nv_bfloat16*>(out), pairs, S, head_dim, adjoint);
   else
-    rope_apply_kernel<float><<<(int)g, 256, 0, st>>>(reinterpret_cast<const float*>(x), cos_tab, sin_tab,
+    rte::launch(rope_apply_kernel<float>, (int)g, 256, 0, st, reinterpret_cast<const float*>(x), cos_tab, sin_tab,
                                                     reinterpret_cast<float*>(out), pairs, S, head_dim, adjoint);
   RTE_LAUNCH_CHECK();
   return RTE_OK;

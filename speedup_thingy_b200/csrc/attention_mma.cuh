@@ -198,6 +198,7 @@ __global__ void __launch_bounds__(NTHR, (SMAX <= 64 && HD <= 64) ? 6 : 1)
 fwd_kernel(const __nv_bfloat16* __restrict__ qkv, int ld, int sec, __nv_bfloat16* __restrict__ y, int ldy,
            float* __restrict__ lse, const float* __restrict__ rope, int S, int H,
            __nv_bfloat16* __restrict__ ym, const int32_t* __restrict__ mask_row, const float* __restrict__ mask_tab) {
+  rte::after_previous_grid();
   constexpr int LDS = HD + 8, KT = SMAX / 8;
   extern __shared__ __align__(16) uint8_t smraw[];
   __nv_bfloat16* sq = reinterpret_cast<__nv_bfloat16*>(smraw);       // [QB][LDS]
@@ -341,6 +342,7 @@ bwd_kernel(const __nv_bfloat16* __restrict__ qkv, int ld, int sec, const __nv_bf
            const __nv_bfloat16* __restrict__ dy, int ldy, const float* __restrict__ lse,
            __nv_bfloat16* __restrict__ dqkv, const float* __restrict__ rope, int S, int H,
            const int32_t* __restrict__ mask_row, const float* __restrict__ mask_tab) {
+  rte::after_previous_grid();
   constexpr int LDS = HD + 8;
   extern __shared__ __align__(16) uint8_t smraw[];
   __nv_bfloat16* sq = reinterpret_cast<__nv_bfloat16*>(smraw);
@@ -486,8 +488,7 @@ int launch_fwd(const void* qkv, int ld, int sec, void* y, int ldy, float* lse, c
     if (cudaFuncSetAttribute(fwd_kernel<HD, SMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return RTE_ERR_LAUNCH;
     set = true;
   }
-  fwd_kernel<HD, SMAX><<<dim3(B * H, rte::ceil_div(S, QB)), NTHR, smem, st>>>(
-      reinterpret_cast<const __nv_bfloat16*>(qkv), ld, sec, reinterpret_cast<__nv_bfloat16*>(y), ldy, lse, rope, S, H,
+  rte::launch(fwd_kernel<HD, SMAX>, dim3(B * H, rte::ceil_div(S, QB)), NTHR, smem, st, reinterpret_cast<const __nv_bfloat16*>(qkv), ld, sec, reinterpret_cast<__nv_bfloat16*>(y), ldy, lse, rope, S, H,
       reinterpret_cast<__nv_bfloat16*>(ym), mask_row, mask_tab);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -512,9 +513,9 @@ int launch_bwd(const void* qkv, int ld, int sec, const void* y, const void* dy, 
   const auto* dy16 = reinterpret_cast<const __nv_bfloat16*>(dy);
   auto* dq16 = reinterpret_cast<__nv_bfloat16*>(dqkv);
   if (mask_row != nullptr)
-    bwd_kernel<HD, SMAX, true><<<grid, NTHR, smem, st>>>(q16, ld, sec, y16, dy16, ldy, lse, dq16, rope, S, H, mask_row, mask_tab);
+    rte::launch(bwd_kernel<HD, SMAX, true>, grid, NTHR, smem, st, q16, ld, sec, y16, dy16, ldy, lse, dq16, rope, S, H, mask_row, mask_tab);
   else
-    bwd_kernel<HD, SMAX, false><<<grid, NTHR, smem, st>>>(q16, ld, sec, y16, dy16, ldy, lse, dq16, rope, S, H, nullptr, nullptr);
+    rte::launch(bwd_kernel<HD, SMAX, false>, grid, NTHR, smem, st, q16, ld, sec, y16, dy16, ldy, lse, dq16, rope, S, H, nullptr, nullptr);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }

@@ -23,6 +23,7 @@ inline int grid_for(long long n, int block, int cap = 148 * 8) {
 
 __global__ void gather_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ idx, uint4* __restrict__ dst,
                                    int n, long long row16) {
+  rte::after_previous_grid();
   const long long total = (long long)n * row16;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int r = int(i / row16);
@@ -32,6 +33,7 @@ __global__ void gather_rows_kernel(const uint4* __restrict__ src, const int32_t*
 
 __global__ void scatter_add_rows_kernel(float* __restrict__ dst, const int32_t* __restrict__ idx, const float* __restrict__ src,
                                         int n, long long row) {
+  rte::after_previous_grid();
   const long long total = (long long)n * row;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int r = int(i / row);
@@ -43,6 +45,7 @@ __global__ void scatter_add_rows_kernel(float* __restrict__ dst, const int32_t* 
 __global__ void audit_route_kernel(const int32_t* __restrict__ by_pass, const int32_t* __restrict__ depth,
                                    const int32_t* __restrict__ idx, int32_t* __restrict__ rid, int32_t* __restrict__ active,
                                    int n, int T) {
+  rte::after_previous_grid();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n * T) return;
   const int t = i / n, s = i % n, b = idx[s];
@@ -52,6 +55,7 @@ __global__ void audit_route_kernel(const int32_t* __restrict__ by_pass, const in
 
 __global__ void colmask_mul_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ rid,
                                    const float* __restrict__ table, int S, __nv_bfloat16* __restrict__ out, int rows, int cols) {
+  rte::after_previous_grid();
   const long long total = (long long)rows * cols;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int r = int(i / cols), c = int(i % cols);
@@ -61,6 +65,7 @@ __global__ void colmask_mul_kernel(const __nv_bfloat16* __restrict__ x, const in
 
 __global__ void swiglu_masked_fwd_kernel(const __nv_bfloat16* __restrict__ ug, const int32_t* __restrict__ rid,
                                          const float* __restrict__ table, int S, __nv_bfloat16* __restrict__ z, int rows, int F) {
+  rte::after_previous_grid();
   const long long total = (long long)rows * F;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int r = int(i / F), j = int(i % F);
@@ -72,6 +77,7 @@ __global__ void swiglu_masked_fwd_kernel(const __nv_bfloat16* __restrict__ ug, c
 __global__ void swiglu_masked_bwd_kernel(const __nv_bfloat16* __restrict__ ug, const __nv_bfloat16* __restrict__ dz,
                                          const int32_t* __restrict__ rid, const float* __restrict__ table, int S,
                                          __nv_bfloat16* __restrict__ dug, int rows, int F) {
+  rte::after_previous_grid();
   const long long total = (long long)rows * F;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int r = int(i / F), j = int(i % F);
@@ -86,6 +92,7 @@ __global__ void swiglu_masked_bwd_kernel(const __nv_bfloat16* __restrict__ ug, c
 __global__ void scaled_residual_fwd_kernel(const float* __restrict__ base, const float* __restrict__ branch,
                                            const float* __restrict__ scale, const int32_t* __restrict__ active,
                                            const float* __restrict__ pass, float* __restrict__ out, int n, long long se) {
+  rte::after_previous_grid();
   const float s = *scale;
   const long long total = (long long)n * se;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -100,6 +107,7 @@ scaled_residual_bwd_kernel(const float* __restrict__ dout, const float* __restri
                            float* __restrict__ db32, float* __restrict__ dpass, float* __restrict__ dscale_part,
                            const int32_t* __restrict__ frozen_active, const float* __restrict__ frozen_src, int n,
                            long long se) {
+  rte::after_previous_grid();
   __shared__ float red[32];
   const float s = *scale;
   const long long total = (long long)n * se;
@@ -134,6 +142,7 @@ __global__ void __cluster_dims__(DISTILL_CTAS, 1, 1) __launch_bounds__(NTHR)
 macro_distill_kernel(const float* __restrict__ hot, const float* __restrict__ exact, const float* __restrict__ h0,
                      float l_dir, float l_rms, float l_normed, float l_raw, float* __restrict__ terms,
                      float* __restrict__ dhot, int n, int S, int d) {
+  rte::after_previous_grid();
   constexpr int NW = NTHR / 32;
   __shared__ float wpart[NW][3];
   __shared__ float cta_part[3];        // read by the other CTAs of the cluster
@@ -232,6 +241,7 @@ __global__ void __launch_bounds__(NTHR)
 kl_distill_kernel(const __nv_bfloat16* __restrict__ hot, const __nv_bfloat16* __restrict__ exact, float inv_temp, float coef,
                   const int32_t* __restrict__ idx, int S, __nv_bfloat16* __restrict__ dlog, int ld, float* __restrict__ dsep,
                   float* __restrict__ kl_rows, float* __restrict__ kl1_rows, int V) {
+  rte::after_previous_grid();
   __shared__ float red[32];
   const int row = blockIdx.x;
   const __nv_bfloat16* hr = hot + (size_t)row * V;
@@ -286,6 +296,7 @@ kl_distill_kernel(const __nv_bfloat16* __restrict__ hot, const __nv_bfloat16* __
 // dst[(idx[row / S] * S + row % S) * ld + c] += src[row * V + c]   (bf16 destination, f32 addend, one rounding)
 __global__ void add_rows_f32_to_bf16_kernel(__nv_bfloat16* __restrict__ dst, int ld, const int32_t* __restrict__ idx, int S,
                                             const float* __restrict__ src, int rows, int V) {
+  rte::after_previous_grid();
   const long long total = (long long)rows * V;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int row = int(i / V), c = int(i % V);
@@ -302,6 +313,7 @@ __global__ void add_rows_f32_to_bf16_kernel(__nv_bfloat16* __restrict__ dst, int
 __global__ void audit_clip_kernel(const float* __restrict__ hot_loss, const float* __restrict__ exact_loss,
                                   const int32_t* __restrict__ idx, int n, float inv_p, const float* __restrict__ inv_p_slot,
                                   float clip, float* __restrict__ f_hot, float* __restrict__ f_exact) {
+  rte::after_previous_grid();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   if (inv_p_slot) inv_p = inv_p_slot[j];            // per-sample inclusion probabilities (Bernoulli sampler)
@@ -314,6 +326,7 @@ __global__ void audit_clip_kernel(const float* __restrict__ hot_loss, const floa
 // x[(row_of(r)) * ld + c] *= scale[r / S]  with row_of(r) = idx ? idx[r / S] * S + r % S : r   (bf16, one rounding)
 __global__ void scale_rows_bf16_kernel(__nv_bfloat16* __restrict__ x, int ld, const int32_t* __restrict__ idx, int S,
                                        const float* __restrict__ scale, int rows, int V) {
+  rte::after_previous_grid();
   const long long total = (long long)rows * V;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int row = int(i / V), c = int(i % V);
@@ -347,6 +360,7 @@ audit_sample_kernel(const float* __restrict__ entropy, const int32_t* __restrict
                     float* __restrict__ valid, float* __restrict__ inv_p,
                     float* __restrict__ dist_scale, float* __restrict__ row_weight, float* __restrict__ row_weight_a,
                     float* __restrict__ stats, int32_t* __restrict__ none_audited, int* __restrict__ status) {
+  rte::after_previous_grid();
   __shared__ int scan[1024];
   __shared__ int sel[1024];
   __shared__ int chosen[1024];
@@ -426,6 +440,7 @@ audit_sample_kernel(const float* __restrict__ entropy, const int32_t* __restrict
 
 // x[j, :] *= factor[j]  (fp32 rows of row_len elements)
 __global__ void scale_rows_f32_kernel(float* __restrict__ x, const float* __restrict__ factor, int n, long long row_len) {
+  rte::after_previous_grid();
   const long long total = (long long)n * row_len;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
     x[i] *= factor[i / row_len];
@@ -435,6 +450,7 @@ __global__ void scale_rows_f32_kernel(float* __restrict__ x, const float* __rest
 // then recent = max(1 - sum_j valid_j cos_j / sum_j valid_j, 0) when any slot is valid (audit.py:213-218), else unchanged.
 __global__ void __launch_bounds__(NTHR)
 rows_cosine_kernel(const float* __restrict__ a, const float* __restrict__ b, long long row_len, float* __restrict__ cos_out) {
+  rte::after_previous_grid();
   __shared__ float red[32];
   const float* x = a + (size_t)blockIdx.x * row_len;
   const float* y = b + (size_t)blockIdx.x * row_len;
@@ -444,6 +460,7 @@ rows_cosine_kernel(const float* __restrict__ a, const float* __restrict__ b, lon
   if (threadIdx.x == 0) cos_out[blockIdx.x] = sxy / (fmaxf(sqrtf(sxx), 1e-8f) * fmaxf(sqrtf(syy), 1e-8f));
 }
 __global__ void audit_recent_kernel(const float* __restrict__ cos_in, const float* __restrict__ valid, int n, float* __restrict__ recent) {
+  rte::after_previous_grid();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   float s = 0.f, c = 0.f;
   for (int j = 0; j < n; ++j) { s += valid[j] * cos_in[j]; c += valid[j]; }
@@ -455,6 +472,7 @@ __global__ void audit_recent_kernel(const float* __restrict__ cos_in, const floa
 __global__ void __launch_bounds__(1024)
 alignment_sums_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ z, long long row_len,
                       float* __restrict__ out) {
+  rte::after_previous_grid();
   __shared__ float red[32];
   const float* x = a + (size_t)blockIdx.x * row_len;
   const float* y = b + (size_t)blockIdx.x * row_len;
@@ -492,7 +510,7 @@ alignment_sums_kernel(const float* __restrict__ a, const float* __restrict__ b, 
 extern "C" int rte_audit_clip(const float* hot_loss, const float* exact_loss, const int32_t* idx, int32_t n, float inv_p,
                               const float* inv_p_slot, float clip, float* f_hot, float* f_exact, rte_stream_t stream) {
   RTE_CHECK_ARG(hot_loss && exact_loss && idx && f_hot && f_exact && n > 0 && clip >= 0.f);
-  audit_clip_kernel<<<rte::ceil_div(n, 128), 128, 0, ST(stream)>>>(hot_loss, exact_loss, idx, n, inv_p, inv_p_slot, clip, f_hot,
+  rte::launch(audit_clip_kernel, rte::ceil_div(n, 128), 128, 0, ST(stream), hot_loss, exact_loss, idx, n, inv_p, inv_p_slot, clip, f_hot,
                                                                    f_exact);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -501,8 +519,7 @@ extern "C" int rte_audit_clip(const float* hot_loss, const float* exact_loss, co
 extern "C" int rte_scale_rows_bf16(void* x_bf16, int32_t ld, const int32_t* idx, int32_t S, const float* scale, int32_t rows,
                                    int32_t V, rte_stream_t stream) {
   RTE_CHECK_ARG(x_bf16 && scale && S > 0 && rows > 0 && V > 0 && ld >= V);
-  scale_rows_bf16_kernel<<<grid_for((long long)rows * V, NTHR), NTHR, 0, ST(stream)>>>(
-      reinterpret_cast<__nv_bfloat16*>(x_bf16), ld, idx, S, scale, rows, V);
+  rte::launch(scale_rows_bf16_kernel, grid_for((long long)rows * V, NTHR), NTHR, 0, ST(stream), reinterpret_cast<__nv_bfloat16*>(x_bf16), ld, idx, S, scale, rows, V);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -511,8 +528,7 @@ extern "C" int rte_gather_rows(const void* src, const int32_t* idx, void* dst, i
   RTE_CHECK_ARG(src && idx && dst && n > 0 && row_bytes > 0);
   if ((row_bytes % 16) || (reinterpret_cast<uintptr_t>(src) & 15) || (reinterpret_cast<uintptr_t>(dst) & 15)) return RTE_ERR_ALIGNMENT;
   const long long row16 = row_bytes / 16;
-  gather_rows_kernel<<<grid_for((long long)n * row16, NTHR), NTHR, 0, ST(stream)>>>(
-      reinterpret_cast<const uint4*>(src), idx, reinterpret_cast<uint4*>(dst), n, row16);
+  rte::launch(gather_rows_kernel, grid_for((long long)n * row16, NTHR), NTHR, 0, ST(stream), reinterpret_cast<const uint4*>(src), idx, reinterpret_cast<uint4*>(dst), n, row16);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -520,7 +536,7 @@ extern "C" int rte_gather_rows(const void* src, const int32_t* idx, void* dst, i
 extern "C" int rte_scatter_add_rows_f32(float* dst, const int32_t* idx, const float* src, int32_t n, int64_t row_elems,
                                         rte_stream_t stream) {
   RTE_CHECK_ARG(dst && idx && src && n > 0 && row_elems > 0);
-  scatter_add_rows_kernel<<<grid_for((long long)n * row_elems, NTHR), NTHR, 0, ST(stream)>>>(dst, idx, src, n, row_elems);
+  rte::launch(scatter_add_rows_kernel, grid_for((long long)n * row_elems, NTHR), NTHR, 0, ST(stream), dst, idx, src, n, row_elems);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -528,7 +544,7 @@ extern "C" int rte_scatter_add_rows_f32(float* dst, const int32_t* idx, const fl
 extern "C" int rte_audit_route(const int32_t* recipe_id_by_pass, const int32_t* depth, const int32_t* idx, int32_t* rid_out,
                                int32_t* active_out, int32_t n, int32_t T, rte_stream_t stream) {
   RTE_CHECK_ARG(recipe_id_by_pass && depth && idx && rid_out && active_out && n > 0 && T > 0);
-  audit_route_kernel<<<rte::ceil_div(n * T, 128), 128, 0, ST(stream)>>>(recipe_id_by_pass, depth, idx, rid_out, active_out, n, T);
+  rte::launch(audit_route_kernel, rte::ceil_div(n * T, 128), 128, 0, ST(stream), recipe_id_by_pass, depth, idx, rid_out, active_out, n, T);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -536,8 +552,7 @@ extern "C" int rte_audit_route(const int32_t* recipe_id_by_pass, const int32_t* 
 extern "C" int rte_colmask_mul_bf16(const void* x, const int32_t* rid, const float* table, int32_t S, void* out, int32_t rows,
                                     int32_t cols, rte_stream_t stream) {
   RTE_CHECK_ARG(x && rid && table && out && S > 0 && rows > 0 && cols > 0);
-  colmask_mul_kernel<<<grid_for((long long)rows * cols, NTHR), NTHR, 0, ST(stream)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), rid, table, S, reinterpret_cast<__nv_bfloat16*>(out), rows, cols);
+  rte::launch(colmask_mul_kernel, grid_for((long long)rows * cols, NTHR), NTHR, 0, ST(stream), reinterpret_cast<const __nv_bfloat16*>(x), rid, table, S, reinterpret_cast<__nv_bfloat16*>(out), rows, cols);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -545,8 +560,7 @@ extern "C" int rte_colmask_mul_bf16(const void* x, const int32_t* rid, const flo
 extern "C" int rte_swiglu_masked_fwd(const void* ug, const int32_t* rid, const float* table, int32_t S, void* z, int32_t rows,
                                      int32_t F, rte_stream_t stream) {
   RTE_CHECK_ARG(ug && rid && table && z && S > 0 && rows > 0 && F > 0);
-  swiglu_masked_fwd_kernel<<<grid_for((long long)rows * F, NTHR), NTHR, 0, ST(stream)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(ug), rid, table, S, reinterpret_cast<__nv_bfloat16*>(z), rows, F);
+  rte::launch(swiglu_masked_fwd_kernel, grid_for((long long)rows * F, NTHR), NTHR, 0, ST(stream), reinterpret_cast<const __nv_bfloat16*>(ug), rid, table, S, reinterpret_cast<__nv_bfloat16*>(z), rows, F);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -554,8 +568,7 @@ extern "C" int rte_swiglu_masked_fwd(const void* ug, const int32_t* rid, const f
 extern "C" int rte_swiglu_masked_bwd(const void* ug, const void* dz, const int32_t* rid, const float* table, int32_t S,
                                      void* dug, int32_t rows, int32_t F, rte_stream_t stream) {
   RTE_CHECK_ARG(ug && dz && rid && table && dug && S > 0 && rows > 0 && F > 0);
-  swiglu_masked_bwd_kernel<<<grid_for((long long)rows * F, NTHR), NTHR, 0, ST(stream)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(ug), reinterpret_cast<const __nv_bfloat16*>(dz), rid, table, S,
+  rte::launch(swiglu_masked_bwd_kernel, grid_for((long long)rows * F, NTHR), NTHR, 0, ST(stream), reinterpret_cast<const __nv_bfloat16*>(ug), reinterpret_cast<const __nv_bfloat16*>(dz), rid, table, S,
       reinterpret_cast<__nv_bfloat16*>(dug), rows, F);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -565,7 +578,7 @@ extern "C" int rte_scaled_residual_fwd(const float* base, const float* branch, c
                                        const float* passthrough, float* out, int32_t n, int64_t sample_elems,
                                        rte_stream_t stream) {
   RTE_CHECK_ARG(base && branch && scale && out && n > 0 && sample_elems > 0 && (active == nullptr || passthrough != nullptr));
-  scaled_residual_fwd_kernel<<<grid_for((long long)n * sample_elems, NTHR), NTHR, 0, ST(stream)>>>(base, branch, scale, active,
+  rte::launch(scaled_residual_fwd_kernel, grid_for((long long)n * sample_elems, NTHR), NTHR, 0, ST(stream), base, branch, scale, active,
                                                                                                  passthrough, out, n, sample_elems);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -584,7 +597,7 @@ extern "C" int rte_scaled_residual_bwd(const float* dout, const float* branch, c
     if (grid > max_partials) grid = max_partials;
   }
   if (n_partials) *n_partials = grid;
-  scaled_residual_bwd_kernel<<<grid, NTHR, 0, ST(stream)>>>(dout, branch, scale, active, dbase,
+  rte::launch(scaled_residual_bwd_kernel, grid, NTHR, 0, ST(stream), dout, branch, scale, active, dbase,
       reinterpret_cast<__nv_bfloat16*>(dbranch_bf16), dbranch_f32_accum, dpassthrough, dscale_partial, frozen_active,
       frozen_src, n, sample_elems);
   RTE_LAUNCH_CHECK();
@@ -595,7 +608,7 @@ extern "C" int rte_macro_distill(const float* hot, const float* exact, const flo
                                  float l_normed, float l_raw, float* terms, float* dhot, int32_t n, int32_t S, int32_t d,
                                  rte_stream_t stream) {
   RTE_CHECK_ARG(hot && exact && h0 && terms && dhot && n > 0 && S > 0 && d > 0);
-  macro_distill_kernel<<<n * DISTILL_CTAS, NTHR, 0, ST(stream)>>>(hot, exact, h0, l_dir, l_rms, l_normed, l_raw, terms, dhot, n, S, d);
+  rte::launch(macro_distill_kernel, n * DISTILL_CTAS, NTHR, 0, ST(stream), hot, exact, h0, l_dir, l_rms, l_normed, l_raw, terms, dhot, n, S, d);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -605,7 +618,7 @@ extern "C" int rte_kl_distill(const void* hot_logits, const void* exact_logits, 
                               rte_stream_t stream) {
   RTE_CHECK_ARG(hot_logits && exact_logits && idx && dlogits_hot && kl_rows && temp > 0.f && S > 0 && rows > 0 && V > 0 &&
                 ld_dlogits >= V);
-  kl_distill_kernel<false><<<rows, NTHR, 0, ST(stream)>>>(reinterpret_cast<const __nv_bfloat16*>(hot_logits),
+  rte::launch(kl_distill_kernel<false>, rows, NTHR, 0, ST(stream), reinterpret_cast<const __nv_bfloat16*>(hot_logits),
       reinterpret_cast<const __nv_bfloat16*>(exact_logits), 1.f / temp, coef, idx, S,
       reinterpret_cast<__nv_bfloat16*>(dlogits_hot), ld_dlogits, nullptr, kl_rows, nullptr, V);
   RTE_LAUNCH_CHECK();
@@ -615,7 +628,7 @@ extern "C" int rte_kl_distill(const void* hot_logits, const void* exact_logits, 
 extern "C" int rte_kl_distill_grad(const void* hot_logits, const void* exact_logits, float temp, float coef, float* dgrad,
                                    float* kl_rows, float* kl1_rows, int32_t rows, int32_t V, rte_stream_t stream) {
   RTE_CHECK_ARG(hot_logits && exact_logits && kl_rows && temp > 0.f && rows > 0 && V > 0);
-  kl_distill_kernel<true><<<rows, NTHR, 0, ST(stream)>>>(reinterpret_cast<const __nv_bfloat16*>(hot_logits),
+  rte::launch(kl_distill_kernel<true>, rows, NTHR, 0, ST(stream), reinterpret_cast<const __nv_bfloat16*>(hot_logits),
       reinterpret_cast<const __nv_bfloat16*>(exact_logits), 1.f / temp, coef, nullptr, 1, nullptr, 0, dgrad, kl_rows, kl1_rows, V);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -624,8 +637,7 @@ extern "C" int rte_kl_distill_grad(const void* hot_logits, const void* exact_log
 extern "C" int rte_add_rows_f32_to_bf16(void* dst_bf16, int32_t ld, const int32_t* idx, int32_t S, const float* src,
                                         int32_t rows, int32_t V, rte_stream_t stream) {
   RTE_CHECK_ARG(dst_bf16 && idx && src && S > 0 && rows > 0 && V > 0 && ld >= V);
-  add_rows_f32_to_bf16_kernel<<<grid_for((long long)rows * V, NTHR), NTHR, 0, ST(stream)>>>(
-      reinterpret_cast<__nv_bfloat16*>(dst_bf16), ld, idx, S, src, rows, V);
+  rte::launch(add_rows_f32_to_bf16_kernel, grid_for((long long)rows * V, NTHR), NTHR, 0, ST(stream), reinterpret_cast<__nv_bfloat16*>(dst_bf16), ld, idx, S, src, rows, V);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -641,7 +653,7 @@ extern "C" int rte_audit_sample_bernoulli(const float* entropy, const int32_t* r
   P.p_min = prm->p_min; P.p_max = prm->p_max; P.alpha = prm->alpha; P.beta = prm->beta; P.gamma = prm->gamma;
   P.cov_min = prm->coverage_min; P.cov_beta = prm->coverage_beta; P.inv_rk = prm->inv_r_plus_k; P.w0 = prm->w0;
   P.B = prm->B; P.R = prm->R; P.cap = prm->cap; P.n_cap = prm->n_cap; P.weight_mode = prm->weight_mode;
-  audit_sample_kernel<<<1, 1024, 0, ST(stream)>>>(entropy, recipe_id, u, perm_table, ema, recent, P, idx, idx_scatter, valid, inv_p,
+  rte::launch(audit_sample_kernel, 1, 1024, 0, ST(stream), entropy, recipe_id, u, perm_table, ema, recent, P, idx, idx_scatter, valid, inv_p,
                                                   dist_scale, row_weight, row_weight_a, stats, none_audited, status);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -649,7 +661,7 @@ extern "C" int rte_audit_sample_bernoulli(const float* entropy, const int32_t* r
 
 extern "C" int rte_scale_rows_f32(float* x, const float* factor, int32_t n, int64_t row_len, rte_stream_t stream) {
   RTE_CHECK_ARG(x && factor && n > 0 && row_len > 0);
-  scale_rows_f32_kernel<<<grid_for((long long)n * row_len, NTHR), NTHR, 0, ST(stream)>>>(x, factor, n, row_len);
+  rte::launch(scale_rows_f32_kernel, grid_for((long long)n * row_len, NTHR), NTHR, 0, ST(stream), x, factor, n, row_len);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -657,9 +669,9 @@ extern "C" int rte_scale_rows_f32(float* x, const float* factor, int32_t n, int6
 extern "C" int rte_audit_recent_residual(const float* hot_end, const float* exact_end, const float* valid, int32_t n,
                                          int64_t row_len, float* cos_scratch, float* recent, rte_stream_t stream) {
   RTE_CHECK_ARG(hot_end && exact_end && valid && cos_scratch && recent && n > 0 && row_len > 0);
-  rows_cosine_kernel<<<n, NTHR, 0, ST(stream)>>>(hot_end, exact_end, row_len, cos_scratch);
+  rte::launch(rows_cosine_kernel, n, NTHR, 0, ST(stream), hot_end, exact_end, row_len, cos_scratch);
   RTE_LAUNCH_CHECK();
-  audit_recent_kernel<<<1, 32, 0, ST(stream)>>>(cos_scratch, valid, n, recent);
+  rte::launch(audit_recent_kernel, 1, 32, 0, ST(stream), cos_scratch, valid, n, recent);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -667,7 +679,7 @@ extern "C" int rte_audit_recent_residual(const float* hot_end, const float* exac
 extern "C" int rte_audit_alignment_sums(const float* hot_end, const float* exact_end, const float* h0, int32_t n, int64_t row_len,
                                         float* out, rte_stream_t stream) {
   RTE_CHECK_ARG(hot_end && exact_end && h0 && out && n > 0 && row_len > 0);
-  alignment_sums_kernel<<<n, 1024, 0, ST(stream)>>>(hot_end, exact_end, h0, row_len, out);
+  rte::launch(alignment_sums_kernel, n, 1024, 0, ST(stream), hot_end, exact_end, h0, row_len, out);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }

@@ -25,6 +25,7 @@ constexpr int MAX_CLUSTERS = 64;
 __global__ void __launch_bounds__(256)
 cluster_route_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ centers, int32_t* __restrict__ assign,
                      float* __restrict__ scores_out, int n, int W, int C) {
+  rte::after_previous_grid();
   extern __shared__ float sc[];              // centres [C][W] when they fit
   const bool in_smem = (size_t)C * W * sizeof(float) <= 96 * 1024;
   if (in_smem) {
@@ -53,6 +54,7 @@ __global__ void __launch_bounds__(PACK_THREADS)
 cluster_pack_kernel(const int32_t* __restrict__ assign, int n, int C, int cap, int32_t* __restrict__ perm,
                     int32_t* __restrict__ pos, int32_t* __restrict__ counts, int32_t* __restrict__ offsets,
                     int32_t* __restrict__ tile_group, int32_t* __restrict__ kblocks, int* status) {
+  rte::after_previous_grid();
   __shared__ int cnt[MAX_CLUSTERS];
   __shared__ int base[MAX_CLUSTERS + 1];
   __shared__ int wc[PACK_THREADS / 32][MAX_CLUSTERS];
@@ -122,6 +124,7 @@ cluster_pack_kernel(const int32_t* __restrict__ assign, int n, int C, int cap, i
 template <typename TS, typename TD>
 __global__ void __launch_bounds__(256)
 gather_convert_kernel(const TS* __restrict__ src, const int32_t* __restrict__ idx, TD* __restrict__ dst, long long n_out, int d) {
+  rte::after_previous_grid();
   const int d4 = d >> 2;
   const long long total = n_out * d4;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -144,6 +147,7 @@ gather_convert_kernel(const TS* __restrict__ src, const int32_t* __restrict__ id
 __global__ void __launch_bounds__(256)
 csr_row_reduce_kernel(const float* __restrict__ src, const int32_t* __restrict__ row_ptr, const int32_t* __restrict__ rows,
                       float* __restrict__ dense, long long n_dense, int d, int accumulate) {
+  rte::after_previous_grid();
   const int d4 = d >> 2;
   const long long total = n_dense * d4;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -161,6 +165,7 @@ csr_row_reduce_kernel(const float* __restrict__ src, const int32_t* __restrict__
 template <typename TD>
 __global__ void __launch_bounds__(256)
 transpose_kernel(const float* __restrict__ src, TD* __restrict__ dst, int R, int C, int accumulate) {
+  rte::after_previous_grid();
   __shared__ float tile[32][33];
   const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;          // 32 x 8
@@ -201,7 +206,7 @@ extern "C" int rte_cluster_route(const float* q, int32_t ldq, const float* cente
       set = true;
     }
   }
-  cluster_route_kernel<<<rte::ceil_div(n_tokens, 8), 256, use, ST(stream)>>>(q, ldq, centers, assignments, scores_out, n_tokens,
+  rte::launch(cluster_route_kernel, rte::ceil_div(n_tokens, 8), 256, use, ST(stream), q, ldq, centers, assignments, scores_out, n_tokens,
                                                                             width, n_clusters);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -213,7 +218,7 @@ extern "C" int rte_cluster_pack(const int32_t* assignments, int32_t n_tokens, in
   RTE_CHECK_ARG(assignments && perm && pos && counts && offsets && tile_group && kblocks && n_tokens > 0 && n_clusters > 0);
   RTE_CHECK_ARG(capacity_rows > 0 && capacity_rows % 128 == 0);
   if (n_clusters > MAX_CLUSTERS) return RTE_ERR_UNSUPPORTED;
-  cluster_pack_kernel<<<1, PACK_THREADS, 0, ST(stream)>>>(assignments, n_tokens, n_clusters, capacity_rows, perm, pos, counts,
+  rte::launch(cluster_pack_kernel, 1, PACK_THREADS, 0, ST(stream), assignments, n_tokens, n_clusters, capacity_rows, perm, pos, counts,
                                                           offsets, tile_group, kblocks, status);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -224,10 +229,10 @@ extern "C" int rte_gather_rows_convert(const void* src, int32_t src_bf16, const 
   RTE_CHECK_ARG(src && idx && dst && n_out > 0 && d > 0 && d % 4 == 0);
   const int g = grid_for(n_out * (d / 4), 256);
   using bf = __nv_bfloat16;
-  if (src_bf16 && dst_bf16) gather_convert_kernel<bf, bf><<<g, 256, 0, ST(stream)>>>((const bf*)src, idx, (bf*)dst, n_out, d);
-  else if (src_bf16) gather_convert_kernel<bf, float><<<g, 256, 0, ST(stream)>>>((const bf*)src, idx, (float*)dst, n_out, d);
-  else if (dst_bf16) gather_convert_kernel<float, bf><<<g, 256, 0, ST(stream)>>>((const float*)src, idx, (bf*)dst, n_out, d);
-  else gather_convert_kernel<float, float><<<g, 256, 0, ST(stream)>>>((const float*)src, idx, (float*)dst, n_out, d);
+  if (src_bf16 && dst_bf16) rte::launch(gather_convert_kernel<bf, bf>, g, 256, 0, ST(stream), (const bf*)src, idx, (bf*)dst, n_out, d);
+  else if (src_bf16) rte::launch(gather_convert_kernel<bf, float>, g, 256, 0, ST(stream), (const bf*)src, idx, (float*)dst, n_out, d);
+  else if (dst_bf16) rte::launch(gather_convert_kernel<float, bf>, g, 256, 0, ST(stream), (const float*)src, idx, (bf*)dst, n_out, d);
+  else rte::launch(gather_convert_kernel<float, float>, g, 256, 0, ST(stream), (const float*)src, idx, (float*)dst, n_out, d);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -236,7 +241,7 @@ extern "C" int rte_csr_row_reduce_f32(const float* src, const int32_t* row_ptr, 
                                       int64_t n_dense_rows, int32_t d, int32_t accumulate, rte_stream_t stream) {
   RTE_CHECK_ARG(src && row_ptr && rows && dense && n_dense_rows > 0 && d > 0 && d % 4 == 0);
   if ((reinterpret_cast<uintptr_t>(src) & 15) || (reinterpret_cast<uintptr_t>(dense) & 15)) return RTE_ERR_ALIGNMENT;
-  csr_row_reduce_kernel<<<grid_for(n_dense_rows * (d / 4), 256), 256, 0, ST(stream)>>>(src, row_ptr, rows, dense, n_dense_rows, d,
+  rte::launch(csr_row_reduce_kernel, grid_for(n_dense_rows * (d / 4), 256), 256, 0, ST(stream), src, row_ptr, rows, dense, n_dense_rows, d,
                                                                                      accumulate);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -246,8 +251,8 @@ extern "C" int rte_transpose_f32(const float* src, void* dst, int32_t rows, int3
                                  rte_stream_t stream) {
   RTE_CHECK_ARG(src && dst && rows > 0 && cols > 0);
   dim3 grid(rte::ceil_div(cols, 32), rte::ceil_div(rows, 32));
-  if (dst_bf16) transpose_kernel<__nv_bfloat16><<<grid, 256, 0, ST(stream)>>>(src, (__nv_bfloat16*)dst, rows, cols, accumulate);
-  else transpose_kernel<float><<<grid, 256, 0, ST(stream)>>>(src, (float*)dst, rows, cols, accumulate);
+  if (dst_bf16) rte::launch(transpose_kernel<__nv_bfloat16>, grid, 256, 0, ST(stream), src, (__nv_bfloat16*)dst, rows, cols, accumulate);
+  else rte::launch(transpose_kernel<float>, grid, 256, 0, ST(stream), src, (float*)dst, rows, cols, accumulate);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }

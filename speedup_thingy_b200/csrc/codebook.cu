@@ -11,6 +11,7 @@ namespace {
 // out[r, :] = x[r, :] / max(||x[r, :]||_2, 1e-12); one warp per row.
 __global__ void __launch_bounds__(256)
 normalize_rows_kernel(const float* __restrict__ x, float* __restrict__ out, int n, int W) {
+  rte::after_previous_grid();
   const int lane = threadIdx.x & 31, row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= n) return;
   const float* xr = x + (size_t)row * W;
@@ -27,6 +28,7 @@ normalize_rows_kernel(const float* __restrict__ x, float* __restrict__ out, int 
 __global__ void __launch_bounds__(256)
 cluster_reduce_kernel(const float* __restrict__ x, const int32_t* __restrict__ assign, const float* __restrict__ old,
                       float* __restrict__ out, int32_t* __restrict__ counts, int n, int W, int mode) {
+  rte::after_previous_grid();
   __shared__ float red[32];
   __shared__ int32_t sa[1024];
   const int c = blockIdx.x, col = blockIdx.y * 256 + threadIdx.x;
@@ -65,6 +67,7 @@ cluster_reduce_kernel(const float* __restrict__ x, const int32_t* __restrict__ a
 __global__ void __launch_bounds__(256)
 pool_scores_kernel(const float* __restrict__ up_hat, const float* __restrict__ gate_hat, const float* __restrict__ wd_norm,
                    float* __restrict__ out, long long total, int F, int mode) {
+  rte::after_previous_grid();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const float u = up_hat[i], g = gate_hat[i], w = wd_norm[i % F];
     const float ga = g / (1.f + expf(-g));
@@ -77,7 +80,7 @@ pool_scores_kernel(const float* __restrict__ up_hat, const float* __restrict__ g
 
 extern "C" int rte_normalize_rows_f32(const float* x, float* out, int32_t n, int32_t W, rte_stream_t stream) {
   RTE_CHECK_ARG(x && out && n > 0 && W > 0);
-  normalize_rows_kernel<<<rte::ceil_div(n, 8), 256, 0, ST(stream)>>>(x, out, n, W);
+  rte::launch(normalize_rows_kernel, rte::ceil_div(n, 8), 256, 0, ST(stream), x, out, n, W);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -86,7 +89,7 @@ extern "C" int rte_kmeans_update(const float* x_normed, const int32_t* assignmen
                                  int32_t* counts, int32_t n, int32_t W, int32_t C, rte_stream_t stream) {
   RTE_CHECK_ARG(x_normed && assignments && centers_old && centers_new && n > 0 && W > 0 && C > 0);
   if (W > 256) return RTE_ERR_UNSUPPORTED;          // the centre's norm is taken inside one CTA
-  cluster_reduce_kernel<<<dim3(C, 1), 256, 0, ST(stream)>>>(x_normed, assignments, centers_old, centers_new, counts, n, W, 0);
+  rte::launch(cluster_reduce_kernel, dim3(C, 1), 256, 0, ST(stream), x_normed, assignments, centers_old, centers_new, counts, n, W, 0);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -94,7 +97,7 @@ extern "C" int rte_kmeans_update(const float* x_normed, const int32_t* assignmen
 extern "C" int rte_cluster_aggregate(const float* scores, const int32_t* assignments, float* out, int32_t n, int32_t F, int32_t C,
                                      int32_t use_max, rte_stream_t stream) {
   RTE_CHECK_ARG(scores && assignments && out && n > 0 && F > 0 && C > 0);
-  cluster_reduce_kernel<<<dim3(C, rte::ceil_div(F, 256)), 256, 0, ST(stream)>>>(scores, assignments, nullptr, out, nullptr, n, F,
+  rte::launch(cluster_reduce_kernel, dim3(C, rte::ceil_div(F, 256)), 256, 0, ST(stream), scores, assignments, nullptr, out, nullptr, n, F,
                                                                                use_max ? 2 : 1);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -106,7 +109,7 @@ extern "C" int rte_cluster_pool_scores(const float* up_hat, const float* gate_ha
   const long long total = (long long)n * F;
   long long g = (total + 255) / 256;
   if (g > 148 * 16) g = 148 * 16;
-  pool_scores_kernel<<<(int)g, 256, 0, ST(stream)>>>(up_hat, gate_hat, wd_norm, out, total, F, mode);
+  rte::launch(pool_scores_kernel, (int)g, 256, 0, ST(stream), up_hat, gate_hat, wd_norm, out, total, F, mode);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }

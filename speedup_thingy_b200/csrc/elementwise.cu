@@ -15,6 +15,7 @@ using rte::warp_sum;
 // ------------------------------------------------------------------ embedding
 __global__ void embed_fwd_kernel(const int64_t* __restrict__ tokens, const float* __restrict__ table,
                                  float* __restrict__ out, int n_tokens, int d, int vocab, int* status) {
+  rte::after_previous_grid();
   const int d4 = d >> 2;
   const long long total = (long long)n_tokens * d4;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -36,6 +37,7 @@ constexpr float EMBED_FX_SCALE = 1099511627776.f;          // 2^40
 __global__ void embed_bwd_accum_kernel(const int64_t* __restrict__ tokens, const float* __restrict__ dx,
                                        unsigned long long* __restrict__ accum, float* __restrict__ dtable,
                                        int n_tokens, int d, int vocab, int* status) {
+  rte::after_previous_grid();
   const long long total = (long long)n_tokens * d;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int t = int(i / d), c = int(i % d);
@@ -51,6 +53,7 @@ __global__ void embed_bwd_accum_kernel(const int64_t* __restrict__ tokens, const
 }
 
 __global__ void embed_bwd_apply_kernel(const unsigned long long* __restrict__ accum, float* __restrict__ dtable, long long n) {
+  rte::after_previous_grid();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const long long q = (long long)accum[i];
     if (q != 0) dtable[i] += __ll2float_rn(q) * (1.f / EMBED_FX_SCALE);
@@ -66,6 +69,7 @@ __global__ void __launch_bounds__(256)
 rmsnorm_fwd_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ fg,
                    const float* __restrict__ fb, __nv_bfloat16* __restrict__ y16, float* __restrict__ y32,
                    float* __restrict__ rstd, int rows, int d, float eps) {
+  rte::after_previous_grid();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -119,6 +123,7 @@ residual_rmsnorm_fwd_kernel(const float* __restrict__ base, const float* __restr
                             float* __restrict__ x_out, const float* __restrict__ w, const float* __restrict__ fg,
                             const float* __restrict__ fb, __nv_bfloat16* __restrict__ y16, float* __restrict__ rstd, int rows, int d,
                             float eps, int branch_splits, long long branch_stride, float* __restrict__ branch_out) {
+  rte::after_previous_grid();
   // branch_splits > 1: `branch` holds that many split-K partials of the branch, branch_stride floats apart; they are
   // summed here in split order (what rte_reduce_splits would have produced) and the sum is kept in branch_out.
   const int lane = threadIdx.x & 31;
@@ -198,6 +203,7 @@ rmsnorm_bwd_kernel(const float* __restrict__ x, const float* __restrict__ w, con
                    const float* __restrict__ dy32, const float* __restrict__ dres, float* __restrict__ dx32,
                    __nv_bfloat16* __restrict__ dx16, float* __restrict__ dw_part, float* __restrict__ dg_part,
                    float* __restrict__ db_part, int rows, int d, int dy_splits, long long dy_stride) {
+  rte::after_previous_grid();
   // dy_splits > 1: dy32 holds that many split-K partials of dy, dy_stride floats apart, summed here in split order
   extern __shared__ float sm[];   // [3][warps][d] when parameter gradients are requested
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
@@ -383,6 +389,7 @@ rmsnorm_bwd_kernel(const float* __restrict__ x, const float* __restrict__ w, con
 // fixed order (deterministic).
 __global__ void __launch_bounds__(1024)
 colsum_kernel(const float* __restrict__ part, int n_rows, int d, float* __restrict__ out, int accumulate) {
+  rte::after_previous_grid();
   __shared__ float sm[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
@@ -407,6 +414,7 @@ struct ColsumJobs { ColsumJob j[3]; };
 
 __global__ void __launch_bounds__(1024)
 colsum3_kernel(ColsumJobs jobs, int n_rows, int d) {
+  rte::after_previous_grid();
   __shared__ float sm[32][33];
   const ColsumJob job = jobs.j[blockIdx.y];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -432,6 +440,7 @@ __global__ void __launch_bounds__(256)
 ce_kernel(const __nv_bfloat16* __restrict__ logits, int ldl, const int64_t* __restrict__ targets,
           const float* __restrict__ row_weight, int S, float* __restrict__ loss_tok,
           __nv_bfloat16* __restrict__ dlogits, int rows, int V, int* status) {
+  rte::after_previous_grid();
   __shared__ float red[32];
   const int row = blockIdx.x;
   if (row >= rows) return;
@@ -487,6 +496,7 @@ ce_kernel(const __nv_bfloat16* __restrict__ logits, int ldl, const int64_t* __re
 }
 
 __global__ void segment_sum_kernel(const float* __restrict__ in, float* __restrict__ out, int n_seg, int seg_len) {
+  rte::after_previous_grid();
   __shared__ float red[32];
   const int seg = blockIdx.x;
   if (seg >= n_seg) return;
@@ -499,6 +509,7 @@ __global__ void segment_sum_kernel(const float* __restrict__ in, float* __restri
 // ------------------------------------------------------------------ small vector kernels
 __global__ void reduce_splits_kernel(const float* __restrict__ ws, int splits, long long stride, long long n4,
                                      float* __restrict__ out, int accumulate) {
+  rte::after_previous_grid();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
     float4 acc = accumulate ? reinterpret_cast<float4*>(out)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     for (int s = 0; s < splits; ++s) {
@@ -510,6 +521,7 @@ __global__ void reduce_splits_kernel(const float* __restrict__ ws, int splits, l
 }
 __global__ void reduce_splits_tail_kernel(const float* __restrict__ ws, int splits, long long stride, long long start,
                                           long long n, float* __restrict__ out, int accumulate) {
+  rte::after_previous_grid();
   const long long i = start + blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   float acc = accumulate ? out[i] : 0.f;
@@ -518,6 +530,7 @@ __global__ void reduce_splits_tail_kernel(const float* __restrict__ ws, int spli
 }
 
 __global__ void cast_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long n) {
+  rte::after_previous_grid();
   const long long n4 = n >> 2;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
     const float4 t = reinterpret_cast<const float4*>(src)[i];
@@ -527,16 +540,20 @@ __global__ void cast_kernel(const float* __restrict__ src, __nv_bfloat16* __rest
     dst[i] = __float2bfloat16_rn(src[i]);
 }
 __global__ void fill_kernel(float* __restrict__ dst, float value, long long n) {
+  rte::after_previous_grid();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) dst[i] = value;
 }
 __global__ void add_kernel(float* __restrict__ dst, const float* __restrict__ src, long long n) {
+  rte::after_previous_grid();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) dst[i] += src[i];
 }
 __global__ void add_guarded_kernel(float* __restrict__ dst, const float* __restrict__ src, long long n, const int32_t* __restrict__ skip) {
+  rte::after_previous_grid();
   if (*skip != 0) return;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) dst[i] += src[i];
 }
 __global__ void axpy_rows_kernel(float* __restrict__ dst, const float* __restrict__ vec, float alpha, int rows, int seg, int d) {
+  rte::after_previous_grid();
   const long long total = (long long)rows * d;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int r = int(i / d), c = int(i % d);
@@ -555,6 +572,7 @@ adamw_kernel(const rte_adamw_tensor* __restrict__ table, const int32_t* __restri
              const int32_t* __restrict__ step_count, float beta1, float beta2, float eps, float wd,
              const float* __restrict__ grad_scale, const int32_t* __restrict__ skip, float* __restrict__ metric_partial,
              const int32_t* __restrict__ absent_flag, const uint8_t* __restrict__ absent_mask) {
+  rte::after_previous_grid();
   __shared__ float red[32];
   const int ti = chunk_tensor[blockIdx.x];
   // dropped step, or a tensor that received no gradient in this step (torch.optim.AdamW skips `grad is None`: no decay,
@@ -595,6 +613,7 @@ adamw_kernel(const rte_adamw_tensor* __restrict__ table, const int32_t* __restri
 __global__ void adamw_step_kernel(const rte_adamw_tensor* __restrict__ table, int n_tensors, int32_t* step_count,
                                   const int32_t* __restrict__ skip, const int32_t* __restrict__ absent_flag,
                                   const uint8_t* __restrict__ absent_mask) {
+  rte::after_previous_grid();
   if (skip != nullptr && *skip != 0) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n_tensors && !(absent_flag != nullptr && *absent_flag != 0 && absent_mask[i] != 0)) step_count[table[i].step_slot] += 1;
@@ -604,6 +623,7 @@ __global__ void adamw_step_kernel(const rte_adamw_tensor* __restrict__ table, in
 __global__ void __launch_bounds__(256)
 adamw_metric_kernel(const int32_t* __restrict__ chunk_tensor, const int32_t* __restrict__ metric_group, long long total_chunks,
                     const float* __restrict__ partial, float* __restrict__ out) {
+  rte::after_previous_grid();
   __shared__ float red[32];
   float a = 0.f, b = 0.f;
   for (long long c = threadIdx.x; c < total_chunks; c += blockDim.x)
@@ -616,6 +636,7 @@ adamw_metric_kernel(const int32_t* __restrict__ chunk_tensor, const int32_t* __r
 __global__ void __launch_bounds__(256)
 nonfinite_guard_kernel(const float* __restrict__ a, int na, const float* __restrict__ b, int nb, const float* __restrict__ c, int nc,
                        int32_t* skip, float* flag_out) {
+  rte::after_previous_grid();
   __shared__ int bad;
   if (threadIdx.x == 0) bad = 0;
   __syncthreads();
@@ -631,6 +652,7 @@ nonfinite_guard_kernel(const float* __restrict__ a, int na, const float* __restr
 __global__ void __launch_bounds__(256)
 gradnorm_partial_kernel(const rte_adamw_tensor* __restrict__ table, const int32_t* __restrict__ chunk_tensor,
                         const int32_t* __restrict__ chunk_index, float* __restrict__ partial) {
+  rte::after_previous_grid();
   __shared__ float red[32];
   const rte_adamw_tensor t = table[chunk_tensor[blockIdx.x]];
   const long long base = (long long)chunk_index[blockIdx.x] * RTE_ADAMW_CHUNK;
@@ -643,6 +665,7 @@ gradnorm_partial_kernel(const rte_adamw_tensor* __restrict__ table, const int32_
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 __global__ void gradnorm_final_kernel(const float* __restrict__ partial, long long n, float* sumsq, float max_norm, float* clip_coef) {
+  rte::after_previous_grid();
   __shared__ float red[32];
   float s = 0.f;
   for (long long i = threadIdx.x; i < n; i += blockDim.x) s += partial[i];
@@ -685,6 +708,7 @@ int gradnorm_scratch_for_current_device(float** out) {
 // candidates in that order, so no scratch copy of the row is needed.
 __global__ void __launch_bounds__(256)
 topk_kernel(const float* __restrict__ scores, int ld, int rows, int n, int k, int32_t* __restrict__ idx, float* __restrict__ vals) {
+  rte::after_previous_grid();
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -729,6 +753,7 @@ __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
 }
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ ug, __nv_bfloat16* __restrict__ z, long long rows, int F) {
+  rte::after_previous_grid();
   const int f8 = F >> 3;
   const long long total = rows * f8;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -745,6 +770,7 @@ swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ ug, __nv_bfloat16* __restric
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ ug, const __nv_bfloat16* __restrict__ dz, __nv_bfloat16* __restrict__ dug,
                   long long rows, int F) {
+  rte::after_previous_grid();
   const int f8 = F >> 3;
   const long long total = rows * f8;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -794,7 +820,7 @@ extern "C" const char* rte_status_string(int code) {
 extern "C" int rte_embed_fwd(const int64_t* tokens, const float* table, float* out, int32_t n_tokens, int32_t d,
                              int32_t vocab, int32_t* status, rte_stream_t stream) {
   RTE_CHECK_ARG(tokens && table && out && n_tokens > 0 && d > 0 && d % 4 == 0);
-  embed_fwd_kernel<<<grid_for((long long)n_tokens * (d / 4), 256), 256, 0, ST(stream)>>>(tokens, table, out, n_tokens, d, vocab, status);
+  rte::launch(embed_fwd_kernel, grid_for((long long)n_tokens * (d / 4), 256), 256, 0, ST(stream), tokens, table, out, n_tokens, d, vocab, status);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -803,9 +829,8 @@ extern "C" int rte_embed_bwd(const int64_t* tokens, const float* dx, float* dtab
   RTE_CHECK_ARG(tokens && dx && dtable && accum && n_tokens > 0 && d > 0 && vocab > 0);
   const long long n = (long long)vocab * d;
   if (cudaMemsetAsync(accum, 0, (size_t)n * sizeof(int64_t), ST(stream)) != cudaSuccess) return RTE_ERR_LAUNCH;
-  embed_bwd_accum_kernel<<<grid_for((long long)n_tokens * d, 256), 256, 0, ST(stream)>>>(
-      tokens, dx, reinterpret_cast<unsigned long long*>(accum), dtable, n_tokens, d, vocab, status);
-  embed_bwd_apply_kernel<<<grid_for(n, 256), 256, 0, ST(stream)>>>(reinterpret_cast<const unsigned long long*>(accum), dtable, n);
+  rte::launch(embed_bwd_accum_kernel, grid_for((long long)n_tokens * d, 256), 256, 0, ST(stream), tokens, dx, reinterpret_cast<unsigned long long*>(accum), dtable, n_tokens, d, vocab, status);
+  rte::launch(embed_bwd_apply_kernel, grid_for(n, 256), 256, 0, ST(stream), reinterpret_cast<const unsigned long long*>(accum), dtable, n);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -817,7 +842,7 @@ extern "C" int rte_rmsnorm_fwd(const float* x, const float* w, const float* film
   RTE_CHECK_ARG((film_gamma == nullptr) == (film_beta == nullptr));
   if (d > 128 * RN_MAX_V4) return RTE_ERR_UNSUPPORTED;
 #define RTE_RN_FWD(NV)                                                                            \
-  rmsnorm_fwd_kernel<NV><<<rte::ceil_div(rows, 8), 256, 0, ST(stream)>>>(x, w, film_gamma, film_beta, \
+  rte::launch(rmsnorm_fwd_kernel<NV>, rte::ceil_div(rows, 8), 256, 0, ST(stream), x, w, film_gamma, film_beta, \
       reinterpret_cast<__nv_bfloat16*>(y_bf16), y_f32, rstd, rows, d, eps)
   if (d <= 128) RTE_RN_FWD(1);
   else if (d <= 256) RTE_RN_FWD(2);
@@ -850,7 +875,7 @@ extern "C" int rte_residual_rmsnorm_fwd_splits(const float* base, const float* b
   RTE_CHECK_ARG((film_gamma == nullptr) == (film_beta == nullptr));
   if (d > 128 * RN_MAX_V4) return RTE_ERR_UNSUPPORTED;
 #define RTE_RRN_FWD(NV)                                                                                              \
-  residual_rmsnorm_fwd_kernel<NV><<<rte::ceil_div(rows, 8), 256, 0, ST(stream)>>>(base, branch, scale, active, passthrough, \
+  rte::launch(residual_rmsnorm_fwd_kernel<NV>, rte::ceil_div(rows, 8), 256, 0, ST(stream), base, branch, scale, active, passthrough, \
       S, add2, scale2, x1_out, x_out, w, film_gamma, film_beta, reinterpret_cast<__nv_bfloat16*>(y_bf16), rstd, rows, d, eps, \
       branch_splits, (long long)branch_split_stride, branch_out)
   if (d <= 128) RTE_RRN_FWD(1);
@@ -908,7 +933,7 @@ extern "C" int rte_rmsnorm_bwd_splits(const float* x, const float* w, const floa
         set = true;                                                                                              \
       }                                                                                                          \
     }                                                                                                            \
-    rmsnorm_bwd_kernel<NV, FILM><<<grid, 256, smem, ST(stream)>>>(x, w, film_gamma, rstd,                              \
+    rte::launch(rmsnorm_bwd_kernel<NV, FILM>, grid, 256, smem, ST(stream), x, w, film_gamma, rstd,                              \
         reinterpret_cast<const __nv_bfloat16*>(dy_bf16), dy_f32, dres, dx_f32,                                   \
         reinterpret_cast<__nv_bfloat16*>(dx_bf16), dw_partial, dgamma_partial, dbeta_partial, rows, d,           \
         dy_splits, (long long)dy_split_stride);                                                                  \
@@ -927,7 +952,7 @@ extern "C" int rte_rmsnorm_bwd_splits(const float* x, const float* w, const floa
 extern "C" int rte_colsum_partials(const float* partial, int32_t n_rows, int32_t d, float* out, int32_t accumulate,
                                    rte_stream_t stream) {
   RTE_CHECK_ARG(partial && out && n_rows > 0 && d > 0);
-  colsum_kernel<<<rte::ceil_div(d, 32), 1024, 0, ST(stream)>>>(partial, n_rows, d, out, accumulate);
+  rte::launch(colsum_kernel, rte::ceil_div(d, 32), 1024, 0, ST(stream), partial, n_rows, d, out, accumulate);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -941,7 +966,7 @@ extern "C" int rte_colsum_partials3(const float* const* partials, float* const* 
     RTE_CHECK_ARG(partials[k] && outs[k]);
     jobs.j[i] = ColsumJob{partials[k], outs[k], accumulate[k]};
   }
-  colsum3_kernel<<<dim3(rte::ceil_div(d, 32), count), 1024, 0, ST(stream)>>>(jobs, n_rows, d);
+  rte::launch(colsum3_kernel, dim3(rte::ceil_div(d, 32), count), 1024, 0, ST(stream), jobs, n_rows, d);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -951,7 +976,7 @@ extern "C" int rte_ce_fwd_bwd(const void* logits, int32_t ldl, const int64_t* ta
                               rte_stream_t stream) {
   RTE_CHECK_ARG(logits && targets && loss_tok && rows > 0 && V > 0 && ldl >= V && S > 0);
   RTE_CHECK_ARG(dlogits == nullptr || row_weight != nullptr);
-  ce_kernel<<<rows, 256, 0, ST(stream)>>>(reinterpret_cast<const __nv_bfloat16*>(logits), ldl, targets, row_weight, S,
+  rte::launch(ce_kernel, rows, 256, 0, ST(stream), reinterpret_cast<const __nv_bfloat16*>(logits), ldl, targets, row_weight, S,
                                           loss_tok, reinterpret_cast<__nv_bfloat16*>(dlogits), rows, V, status);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -959,7 +984,7 @@ extern "C" int rte_ce_fwd_bwd(const void* logits, int32_t ldl, const int64_t* ta
 
 extern "C" int rte_segment_sum(const float* in, float* out, int32_t n_seg, int32_t seg_len, rte_stream_t stream) {
   RTE_CHECK_ARG(in && out && n_seg > 0 && seg_len > 0);
-  segment_sum_kernel<<<n_seg, 128, 0, ST(stream)>>>(in, out, n_seg, seg_len);
+  rte::launch(segment_sum_kernel, n_seg, 128, 0, ST(stream), in, out, n_seg, seg_len);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -971,12 +996,12 @@ extern "C" int rte_reduce_splits(const float* ws, int32_t splits, int64_t split_
                    ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
   const long long n4 = vec ? (n >> 2) : 0;
   if (n4 > 0) {
-    reduce_splits_kernel<<<grid_for(n4, 256), 256, 0, ST(stream)>>>(ws, splits, split_stride, n4, out, accumulate);
+    rte::launch(reduce_splits_kernel, grid_for(n4, 256), 256, 0, ST(stream), ws, splits, split_stride, n4, out, accumulate);
     RTE_LAUNCH_CHECK();
   }
   const long long rest = n - n4 * 4;
   if (rest > 0) {
-    reduce_splits_tail_kernel<<<(int)rte::ceil_div64(rest, 256), 256, 0, ST(stream)>>>(ws, splits, split_stride, n4 * 4, n, out, accumulate);
+    rte::launch(reduce_splits_tail_kernel, (int)rte::ceil_div64(rest, 256), 256, 0, ST(stream), ws, splits, split_stride, n4 * 4, n, out, accumulate);
     RTE_LAUNCH_CHECK();
   }
   return RTE_OK;
@@ -985,7 +1010,7 @@ extern "C" int rte_reduce_splits(const float* ws, int32_t splits, int64_t split_
 extern "C" int rte_swiglu_fwd(const void* ug, void* z, int64_t rows, int32_t F, rte_stream_t stream) {
   RTE_CHECK_ARG(ug && z && rows > 0 && F > 0 && F % 8 == 0);
   if ((reinterpret_cast<uintptr_t>(ug) & 15) || (reinterpret_cast<uintptr_t>(z) & 15)) return RTE_ERR_ALIGNMENT;
-  swiglu_fwd_kernel<<<grid_for(rows * (F / 8), 256), 256, 0, ST(stream)>>>(reinterpret_cast<const __nv_bfloat16*>(ug),
+  rte::launch(swiglu_fwd_kernel, grid_for(rows * (F / 8), 256), 256, 0, ST(stream), reinterpret_cast<const __nv_bfloat16*>(ug),
                                                                           reinterpret_cast<__nv_bfloat16*>(z), rows, F);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -994,8 +1019,7 @@ extern "C" int rte_swiglu_bwd(const void* ug, const void* dz, void* dug, int64_t
   RTE_CHECK_ARG(ug && dz && dug && rows > 0 && F > 0 && F % 8 == 0);
   if ((reinterpret_cast<uintptr_t>(ug) & 15) || (reinterpret_cast<uintptr_t>(dz) & 15) || (reinterpret_cast<uintptr_t>(dug) & 15))
     return RTE_ERR_ALIGNMENT;
-  swiglu_bwd_kernel<<<grid_for(rows * (F / 8), 256), 256, 0, ST(stream)>>>(
-      reinterpret_cast<const __nv_bfloat16*>(ug), reinterpret_cast<const __nv_bfloat16*>(dz), reinterpret_cast<__nv_bfloat16*>(dug), rows, F);
+  rte::launch(swiglu_bwd_kernel, grid_for(rows * (F / 8), 256), 256, 0, ST(stream), reinterpret_cast<const __nv_bfloat16*>(ug), reinterpret_cast<const __nv_bfloat16*>(dz), reinterpret_cast<__nv_bfloat16*>(dug), rows, F);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -1003,26 +1027,26 @@ extern "C" int rte_swiglu_bwd(const void* ug, const void* dz, void* dug, int64_t
 extern "C" int rte_cast_f32_bf16(const float* src, void* dst, int64_t n, rte_stream_t stream) {
   RTE_CHECK_ARG(src && dst && n > 0);
   if ((reinterpret_cast<uintptr_t>(src) & 15) || (reinterpret_cast<uintptr_t>(dst) & 7)) return RTE_ERR_ALIGNMENT;
-  cast_kernel<<<grid_for(n / 4 + 1, 256), 256, 0, ST(stream)>>>(src, reinterpret_cast<__nv_bfloat16*>(dst), n);
+  rte::launch(cast_kernel, grid_for(n / 4 + 1, 256), 256, 0, ST(stream), src, reinterpret_cast<__nv_bfloat16*>(dst), n);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
 extern "C" int rte_fill_f32(float* dst, float value, int64_t n, rte_stream_t stream) {
   RTE_CHECK_ARG(dst && n > 0);
-  fill_kernel<<<grid_for(n, 256), 256, 0, ST(stream)>>>(dst, value, n);
+  rte::launch(fill_kernel, grid_for(n, 256), 256, 0, ST(stream), dst, value, n);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
 extern "C" int rte_add_f32(float* dst, const float* src, int64_t n, rte_stream_t stream) {
   RTE_CHECK_ARG(src && dst && n > 0);
-  add_kernel<<<grid_for(n, 256), 256, 0, ST(stream)>>>(dst, src, n);
+  rte::launch(add_kernel, grid_for(n, 256), 256, 0, ST(stream), dst, src, n);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
 extern "C" int rte_axpy_rows_f32(float* dst, const float* vec, float alpha, int32_t rows, int32_t seg, int32_t d,
                                  rte_stream_t stream) {
   RTE_CHECK_ARG(dst && vec && rows > 0 && seg > 0 && d > 0);
-  axpy_rows_kernel<<<grid_for((long long)rows * d, 256), 256, 0, ST(stream)>>>(dst, vec, alpha, rows, seg, d);
+  rte::launch(axpy_rows_kernel, grid_for((long long)rows * d, 256), 256, 0, ST(stream), dst, vec, alpha, rows, seg, d);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -1041,15 +1065,15 @@ extern "C" int rte_adamw_multi_tensor_ex(const rte_adamw_tensor* table, int32_t 
     RTE_CHECK_ARG(ex->metric_partial && ex->metric_group && ex->n_metric_groups > 0);
     mpart = ex->metric_partial;
   }
-  adamw_kernel<<<(unsigned)total_chunks, 256, 0, ST(stream)>>>(table, chunk_tensor, chunk_index, lr_table, step_count,
+  rte::launch(adamw_kernel, (unsigned)total_chunks, 256, 0, ST(stream), table, chunk_tensor, chunk_index, lr_table, step_count,
                                                                beta1, beta2, eps, weight_decay, grad_scale, skip, mpart,
                                                                absent_flag, absent_mask);
   RTE_LAUNCH_CHECK();
-  adamw_step_kernel<<<rte::ceil_div(n_tensors, 128), 128, 0, ST(stream)>>>(table, n_tensors, step_count, skip, absent_flag,
+  rte::launch(adamw_step_kernel, rte::ceil_div(n_tensors, 128), 128, 0, ST(stream), table, n_tensors, step_count, skip, absent_flag,
                                                                            absent_mask);
   RTE_LAUNCH_CHECK();
   if (mpart) {
-    adamw_metric_kernel<<<ex->n_metric_groups, 256, 0, ST(stream)>>>(chunk_tensor, ex->metric_group, total_chunks, mpart,
+    rte::launch(adamw_metric_kernel, ex->n_metric_groups, 256, 0, ST(stream), chunk_tensor, ex->metric_group, total_chunks, mpart,
                                                                      ex->metric_out);
     RTE_LAUNCH_CHECK();
   }
@@ -1066,7 +1090,7 @@ extern "C" int rte_adamw_multi_tensor(const rte_adamw_tensor* table, int32_t n_t
 
 extern "C" int rte_add_f32_guarded(float* dst, const float* src, int64_t n, const int32_t* skip, rte_stream_t stream) {
   RTE_CHECK_ARG(dst && src && skip && n > 0);
-  add_guarded_kernel<<<grid_for(n, 256), 256, 0, ST(stream)>>>(dst, src, n, skip);
+  rte::launch(add_guarded_kernel, grid_for(n, 256), 256, 0, ST(stream), dst, src, n, skip);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -1074,7 +1098,7 @@ extern "C" int rte_add_f32_guarded(float* dst, const float* src, int64_t n, cons
 extern "C" int rte_nonfinite_guard(const float* a, int32_t na, const float* b, int32_t nb, const float* c, int32_t nc,
                                    int32_t* skip, float* flag_out, rte_stream_t stream) {
   RTE_CHECK_ARG(skip && na >= 0 && nb >= 0 && nc >= 0 && (a || na == 0) && (b || nb == 0) && (c || nc == 0));
-  nonfinite_guard_kernel<<<1, 256, 0, ST(stream)>>>(a, na, b, nb, c, nc, skip, flag_out);
+  rte::launch(nonfinite_guard_kernel, 1, 256, 0, ST(stream), a, na, b, nb, c, nc, skip, flag_out);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -1083,9 +1107,9 @@ extern "C" int rte_grad_norm_multi_tensor(const rte_adamw_tensor* table, int64_t
                                           const int32_t* chunk_index, float* partial, float* sumsq, float max_norm,
                                           float* clip_coef, rte_stream_t stream) {
   RTE_CHECK_ARG(table && chunk_tensor && chunk_index && partial && sumsq && total_chunks > 0);
-  gradnorm_partial_kernel<<<(unsigned)total_chunks, 256, 0, ST(stream)>>>(table, chunk_tensor, chunk_index, partial);
+  rte::launch(gradnorm_partial_kernel, (unsigned)total_chunks, 256, 0, ST(stream), table, chunk_tensor, chunk_index, partial);
   RTE_LAUNCH_CHECK();
-  gradnorm_final_kernel<<<1, 1024, 0, ST(stream)>>>(partial, total_chunks, sumsq, max_norm, clip_coef);
+  rte::launch(gradnorm_final_kernel, 1, 1024, 0, ST(stream), partial, total_chunks, sumsq, max_norm, clip_coef);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -1103,9 +1127,9 @@ extern "C" int rte_grad_norm_multi_tensor_static(const rte_adamw_tensor* table, 
   float* partial = nullptr;
   const int rc = gradnorm_scratch_for_current_device(&partial);
   if (rc != RTE_OK) return rc;
-  gradnorm_partial_kernel<<<(unsigned)total_chunks, 256, 0, ST(stream)>>>(table, chunk_tensor, chunk_index, partial);
+  rte::launch(gradnorm_partial_kernel, (unsigned)total_chunks, 256, 0, ST(stream), table, chunk_tensor, chunk_index, partial);
   RTE_LAUNCH_CHECK();
-  gradnorm_final_kernel<<<1, 1024, 0, ST(stream)>>>(partial, total_chunks, sumsq, max_norm, clip_coef);
+  rte::launch(gradnorm_final_kernel, 1, 1024, 0, ST(stream), partial, total_chunks, sumsq, max_norm, clip_coef);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -1113,7 +1137,7 @@ extern "C" int rte_grad_norm_multi_tensor_static(const rte_adamw_tensor* table, 
 extern "C" int rte_topk_lowest_index(const float* scores, int32_t ld, int32_t rows, int32_t n, int32_t k,
                                      int32_t* idx, float* vals, rte_stream_t stream) {
   RTE_CHECK_ARG(scores && rows > 0 && n > 0 && k > 0 && k <= n && ld >= n && (idx || vals));
-  topk_kernel<<<rte::ceil_div(rows, 8), 256, 0, ST(stream)>>>(scores, ld, rows, n, k, idx, vals);
+  rte::launch(topk_kernel, rte::ceil_div(rows, 8), 256, 0, ST(stream), scores, ld, rows, n, k, idx, vals);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }

@@ -30,6 +30,7 @@ __global__ void __launch_bounds__(NTHR)
 phi_prep_kernel(const float* __restrict__ h0, const float* __restrict__ v, const int32_t* __restrict__ rid,
                 const int32_t* __restrict__ sid, float* __restrict__ rstd, float* __restrict__ pooled,
                 float* __restrict__ pa, PhiDims D, float eps) {
+  rte::after_previous_grid();
   extern __shared__ float sm[];            // rstd_s[S] then pooled_s[d]
   float* rs = sm;
   float* ps = sm + D.S;
@@ -64,6 +65,7 @@ __global__ void __launch_bounds__(NTHR)
 phi_act_kernel(const float* __restrict__ h0, const float* __restrict__ hx, const float* __restrict__ rstd,
                const float* __restrict__ pa, const float* __restrict__ v, const int32_t* __restrict__ rid,
                const int32_t* __restrict__ sid, float* __restrict__ act, PhiDims D) {
+  rte::after_previous_grid();
   __shared__ float sx[TT][CH + 1];
   __shared__ float sv1[CH][MMAX];
   __shared__ float sv3[CH][MMAX];
@@ -144,6 +146,7 @@ phi_out_kernel(const float* __restrict__ h0, const float* __restrict__ act, cons
                const float* __restrict__ u, const float* __restrict__ bias, const float* __restrict__ scale,
                const int32_t* __restrict__ rid, const int32_t* __restrict__ sid, float s_cfg,
                const float* __restrict__ dout, float* __restrict__ out, float* __restrict__ dupd, PhiDims D) {
+  rte::after_previous_grid();
   __shared__ float ssa[TT][MMAX];
   const int tiles = rte::ceil_div(D.S, TT);
   const int b = blockIdx.x / tiles, tok0 = (blockIdx.x % tiles) * TT;
@@ -184,6 +187,7 @@ phi_out_kernel(const float* __restrict__ h0, const float* __restrict__ act, cons
 __global__ void __launch_bounds__(NTHR)
 phi_da_kernel(const float* __restrict__ dupd, const float* __restrict__ act, const float* __restrict__ u,
               const int32_t* __restrict__ rid, const int32_t* __restrict__ sid, float* __restrict__ da, PhiDims D) {
+  rte::after_previous_grid();
   __shared__ float sd[TT][CH + 1];
   __shared__ float su[MMAX][CH + 1];
   const int tiles = rte::ceil_div(D.S, TT);
@@ -283,6 +287,7 @@ __device__ __forceinline__ float pick(const float4& v, int s) { return s == 0 ? 
 __global__ void __launch_bounds__(NTHR)
 phi_da_mma_kernel(const float* __restrict__ dupd, const float* __restrict__ act, const float* __restrict__ u,
                   const int32_t* __restrict__ rid, const int32_t* __restrict__ sid, float* __restrict__ da, PhiDims D) {
+  rte::after_previous_grid();
   const int tiles = rte::ceil_div(D.S, TT);
   const int b = blockIdx.x / tiles, tok0 = (blockIdx.x % tiles) * TT;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
@@ -347,6 +352,7 @@ __global__ void __launch_bounds__(NTHR)
 phi_act_mma_kernel(const float* __restrict__ h0, const float* __restrict__ hx, const float* __restrict__ rstd,
                    const float* __restrict__ pa, const float* __restrict__ vt, long long vt_ld,
                    const int32_t* __restrict__ rid, const int32_t* __restrict__ sid, float* __restrict__ act, PhiDims D) {
+  rte::after_previous_grid();
   const int tiles = rte::ceil_div(D.S, TT);
   const int b = blockIdx.x / tiles, tok0 = (blockIdx.x % tiles) * TT;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
@@ -434,6 +440,7 @@ phi_out_mma_kernel(const float* __restrict__ h0, const float* __restrict__ act, 
                    const float* __restrict__ ut, long long ut_ld, const float* __restrict__ bias,
                    const float* __restrict__ scale, const int32_t* __restrict__ rid, const int32_t* __restrict__ sid,
                    float s_cfg, const float* __restrict__ dout, float* __restrict__ out, float* __restrict__ dupd, PhiDims D) {
+  rte::after_previous_grid();
   const int tiles = rte::ceil_div(D.S, TT);
   const int b = blockIdx.x / tiles, tok0 = (blockIdx.x % tiles) * TT;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
@@ -521,6 +528,7 @@ phi_out_mma_kernel(const float* __restrict__ h0, const float* __restrict__ act, 
 __global__ void __launch_bounds__(NTHR)
 phi_pu_kernel(const float* __restrict__ h0, const float* __restrict__ act, const float* __restrict__ dupd,
               float* __restrict__ pu, float* __restrict__ pg, float* __restrict__ pb, PhiDims D) {
+  rte::after_previous_grid();
   extern __shared__ float ssa[];     // [S][m]
   const int cblocks = rte::ceil_div(D.d, NTHR);
   const int b = blockIdx.x / cblocks, c = (blockIdx.x % cblocks) * NTHR + threadIdx.x;
@@ -573,6 +581,7 @@ constexpr int PV_ROWS = 32;       // rows of v per CTA (one 128-byte line of h0 
 __global__ void __launch_bounds__(NTHR)
 phi_pv_kernel(const float* __restrict__ h0, const float* __restrict__ hx, const float* __restrict__ rstd,
               const float* __restrict__ pooled, const float* __restrict__ da, float* __restrict__ pv, PhiDims D) {
+  rte::after_previous_grid();
   extern __shared__ float sm[];      // sda[S][m], rs[S], sx[S][PV_ROWS], sx3[S][PV_ROWS]
   float* sda = sm;
   float* rs = sm + D.S * D.m;
@@ -610,6 +619,7 @@ phi_pv_kernel(const float* __restrict__ h0, const float* __restrict__ hx, const 
 __global__ void __launch_bounds__(NTHR)
 phi_dpool_kernel(const float* __restrict__ da, const float* __restrict__ v, const int32_t* __restrict__ rid,
                  const int32_t* __restrict__ sid, float* __restrict__ dpool, PhiDims D) {
+  rte::after_previous_grid();
   __shared__ float ssum[MMAX];
   const int b = blockIdx.x;
   for (int j = threadIdx.x; j < D.m; j += NTHR) {
@@ -631,6 +641,7 @@ __global__ void __launch_bounds__(NTHR)
 phi_dz_kernel(const float* __restrict__ h0, const float* __restrict__ rstd, const float* __restrict__ da,
               const float* __restrict__ dpool, const float* __restrict__ v, const int32_t* __restrict__ rid,
               const int32_t* __restrict__ sid, float* dh0, float* dhx, PhiDims D) {
+  rte::after_previous_grid();
   __shared__ float sv1[CH][MMAX + 1];
   __shared__ float sv3[CH][MMAX + 1];
   __shared__ float sda[TT][MMAX];
@@ -736,6 +747,7 @@ __global__ void __launch_bounds__(NTHR, KC == 1 ? 2 : 1)
 phi_dz_mma_kernel(const float* __restrict__ h0, const float* __restrict__ rstd, const float* __restrict__ da,
                   const float* __restrict__ dpool, const float* __restrict__ v, const int32_t* __restrict__ rid,
                   const int32_t* __restrict__ sid, float* dh0, float* dhx, PhiDims D) {
+  rte::after_previous_grid();
   __shared__ float sdot[TT][4];
   const int tiles = rte::ceil_div(D.S, TT);
   const int b = blockIdx.x / tiles, tok0 = (blockIdx.x % tiles) * TT;
@@ -873,6 +885,7 @@ phi_dz_mma_kernel(const float* __restrict__ h0, const float* __restrict__ rstd, 
 __global__ void __launch_bounds__(NTHR)
 phi_reduce_keys_kernel(const float* __restrict__ partial, const int32_t* __restrict__ rid, const int32_t* __restrict__ sid,
                        float* __restrict__ out, int B, int K, long long elems) {
+  rte::after_previous_grid();
   __shared__ int members[1024];
   __shared__ int n_members;
   const int key = blockIdx.y;
@@ -898,6 +911,7 @@ constexpr int SQD_BLOCKS = 592;
 __global__ void __launch_bounds__(256)
 sqdiff_grad_kernel(const float* __restrict__ a, const float* __restrict__ b, long long n, float coef,
                    float* __restrict__ g, float* __restrict__ partial) {
+  rte::after_previous_grid();
   __shared__ float red[32];
   float s = 0.f;
   for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
@@ -909,6 +923,7 @@ sqdiff_grad_kernel(const float* __restrict__ a, const float* __restrict__ b, lon
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 __global__ void sqdiff_final_kernel(const float* __restrict__ partial, int n, float* __restrict__ out, int accumulate) {
+  rte::after_previous_grid();
   __shared__ float red[32];
   float s = 0.f;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += partial[i];
@@ -955,30 +970,30 @@ int phi_fwd_impl(const float* h0, const float* hx, const rte_phi_params* p, cons
   // `act` doubles as the home of pa (B*m floats) is NOT safe; pa lives at the tail of `pooled`'s
   // companion: callers give pooled >= B*d + B*m floats.
   float* pa = pooled + (size_t)B * d;
-  phi_prep_kernel<<<B, NTHR, (size_t)(S + d) * sizeof(float), ST(stream)>>>(h0, p->v, recipe_id, stride_id, rstd, pooled, pa, D, eps);
+  rte::launch(phi_prep_kernel, B, NTHR, (size_t)(S + d) * sizeof(float), ST(stream), h0, p->v, recipe_id, stride_id, rstd, pooled, pa, D, eps);
   RTE_LAUNCH_CHECK();
   if (phi_tensor_path(p, h0, out, act, d, m) && (reinterpret_cast<uintptr_t>(hx) & 15) == 0) {
     const long long vt_ld = (long long)p->n_keys * 3 * d, ut_ld = (long long)p->n_keys * m;
     const float* ut = p->wt + (size_t)m * vt_ld;
-    if (hx != h0) phi_act_mma_kernel<true><<<B * tiles, NTHR, 0, ST(stream)>>>(h0, hx, rstd, pa, p->wt, vt_ld, recipe_id, stride_id, act, D);
-    else phi_act_mma_kernel<false><<<B * tiles, NTHR, 0, ST(stream)>>>(h0, hx, rstd, pa, p->wt, vt_ld, recipe_id, stride_id, act, D);
+    if (hx != h0) rte::launch(phi_act_mma_kernel<true>, B * tiles, NTHR, 0, ST(stream), h0, hx, rstd, pa, p->wt, vt_ld, recipe_id, stride_id, act, D);
+    else rte::launch(phi_act_mma_kernel<false>, B * tiles, NTHR, 0, ST(stream), h0, hx, rstd, pa, p->wt, vt_ld, recipe_id, stride_id, act, D);
     RTE_LAUNCH_CHECK();
     if (m <= 32)
-      phi_out_mma_kernel<0, 1><<<B * tiles, NTHR, 0, ST(stream)>>>(h0, act, p->gain, ut, ut_ld, p->bias, p->scale, recipe_id,
+      rte::launch(phi_out_mma_kernel<0, 1>, B * tiles, NTHR, 0, ST(stream), h0, act, p->gain, ut, ut_ld, p->bias, p->scale, recipe_id,
                                                                    stride_id, s_cfg, nullptr, out, nullptr, D);
     else
-      phi_out_mma_kernel<0, 2><<<B * tiles, NTHR, 0, ST(stream)>>>(h0, act, p->gain, ut, ut_ld, p->bias, p->scale, recipe_id,
+      rte::launch(phi_out_mma_kernel<0, 2>, B * tiles, NTHR, 0, ST(stream), h0, act, p->gain, ut, ut_ld, p->bias, p->scale, recipe_id,
                                                                    stride_id, s_cfg, nullptr, out, nullptr, D);
     RTE_LAUNCH_CHECK();
     return RTE_OK;
   }
-  phi_act_kernel<<<B * tiles, NTHR, 0, ST(stream)>>>(h0, hx, rstd, pa, p->v, recipe_id, stride_id, act, D);
+  rte::launch(phi_act_kernel, B * tiles, NTHR, 0, ST(stream), h0, hx, rstd, pa, p->v, recipe_id, stride_id, act, D);
   RTE_LAUNCH_CHECK();
   if (m <= 32)
-    phi_out_kernel<0, 32><<<B * tiles, NTHR, 0, ST(stream)>>>(h0, act, p->gain, p->u, p->bias, p->scale, recipe_id, stride_id,
+    rte::launch(phi_out_kernel<0, 32>, B * tiles, NTHR, 0, ST(stream), h0, act, p->gain, p->u, p->bias, p->scale, recipe_id, stride_id,
                                                               s_cfg, nullptr, out, nullptr, D);
   else
-    phi_out_kernel<0, 64><<<B * tiles, NTHR, 0, ST(stream)>>>(h0, act, p->gain, p->u, p->bias, p->scale, recipe_id, stride_id,
+    rte::launch(phi_out_kernel<0, 64>, B * tiles, NTHR, 0, ST(stream), h0, act, p->gain, p->u, p->bias, p->scale, recipe_id, stride_id,
                                                               s_cfg, nullptr, out, nullptr, D);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -1033,30 +1048,30 @@ int phi_bwd_data_impl(const float* h0, const float* dout, const rte_phi_params* 
     const long long vt_ld = (long long)p->n_keys * 3 * d, ut_ld = (long long)p->n_keys * m;
     const float* ut = p->wt + (size_t)m * vt_ld;
     if (m <= 32)
-      phi_out_mma_kernel<1, 1><<<B * tiles, NTHR, 0, ST(stream)>>>(h0, act, p->gain, ut, ut_ld, p->bias, p->scale, recipe_id,
+      rte::launch(phi_out_mma_kernel<1, 1>, B * tiles, NTHR, 0, ST(stream), h0, act, p->gain, ut, ut_ld, p->bias, p->scale, recipe_id,
                                                                    stride_id, s_cfg, dout, dh0, x.dupd, D);
     else
-      phi_out_mma_kernel<1, 2><<<B * tiles, NTHR, 0, ST(stream)>>>(h0, act, p->gain, ut, ut_ld, p->bias, p->scale, recipe_id,
+      rte::launch(phi_out_mma_kernel<1, 2>, B * tiles, NTHR, 0, ST(stream), h0, act, p->gain, ut, ut_ld, p->bias, p->scale, recipe_id,
                                                                    stride_id, s_cfg, dout, dh0, x.dupd, D);
   } else if (m <= 32)
-    phi_out_kernel<1, 32><<<B * tiles, NTHR, 0, ST(stream)>>>(h0, act, p->gain, p->u, p->bias, p->scale, recipe_id, stride_id,
+    rte::launch(phi_out_kernel<1, 32>, B * tiles, NTHR, 0, ST(stream), h0, act, p->gain, p->u, p->bias, p->scale, recipe_id, stride_id,
                                                               s_cfg, dout, dh0, x.dupd, D);
   else
-    phi_out_kernel<1, 64><<<B * tiles, NTHR, 0, ST(stream)>>>(h0, act, p->gain, p->u, p->bias, p->scale, recipe_id, stride_id,
+    rte::launch(phi_out_kernel<1, 64>, B * tiles, NTHR, 0, ST(stream), h0, act, p->gain, p->u, p->bias, p->scale, recipe_id, stride_id,
                                                               s_cfg, dout, dh0, x.dupd, D);
   RTE_LAUNCH_CHECK();
   // tensor-core (3xTF32) products with 16-byte operand loads; other shapes keep the scalar kernels
   const bool mma = d % 32 == 0 && m % 4 == 0 && ((reinterpret_cast<uintptr_t>(scratch) | reinterpret_cast<uintptr_t>(h0) |
                    reinterpret_cast<uintptr_t>(dh0) | reinterpret_cast<uintptr_t>(dhx) | reinterpret_cast<uintptr_t>(p->u) |
                    reinterpret_cast<uintptr_t>(p->v)) & 15) == 0;
-  if (mma) phi_da_mma_kernel<<<B * tiles, NTHR, 0, ST(stream)>>>(x.dupd, act, p->u, recipe_id, stride_id, x.da, D);
-  else phi_da_kernel<<<B * tiles, NTHR, 0, ST(stream)>>>(x.dupd, act, p->u, recipe_id, stride_id, x.da, D);
+  if (mma) rte::launch(phi_da_mma_kernel, B * tiles, NTHR, 0, ST(stream), x.dupd, act, p->u, recipe_id, stride_id, x.da, D);
+  else rte::launch(phi_da_kernel, B * tiles, NTHR, 0, ST(stream), x.dupd, act, p->u, recipe_id, stride_id, x.da, D);
   RTE_LAUNCH_CHECK();
-  phi_dpool_kernel<<<B, NTHR, 0, ST(stream)>>>(x.da, p->v, recipe_id, stride_id, x.dpool, D);
+  rte::launch(phi_dpool_kernel, B, NTHR, 0, ST(stream), x.da, p->v, recipe_id, stride_id, x.dpool, D);
   RTE_LAUNCH_CHECK();
-  if (mma && m <= 32) phi_dz_mma_kernel<1><<<B * tiles, NTHR, 0, ST(stream)>>>(h0, rstd, x.da, x.dpool, p->v, recipe_id, stride_id, dh0, dhx, D);
-  else if (mma) phi_dz_mma_kernel<2><<<B * tiles, NTHR, 0, ST(stream)>>>(h0, rstd, x.da, x.dpool, p->v, recipe_id, stride_id, dh0, dhx, D);
-  else phi_dz_kernel<<<B * tiles, NTHR, 0, ST(stream)>>>(h0, rstd, x.da, x.dpool, p->v, recipe_id, stride_id, dh0, dhx, D);
+  if (mma && m <= 32) rte::launch(phi_dz_mma_kernel<1>, B * tiles, NTHR, 0, ST(stream), h0, rstd, x.da, x.dpool, p->v, recipe_id, stride_id, dh0, dhx, D);
+  else if (mma) rte::launch(phi_dz_mma_kernel<2>, B * tiles, NTHR, 0, ST(stream), h0, rstd, x.da, x.dpool, p->v, recipe_id, stride_id, dh0, dhx, D);
+  else rte::launch(phi_dz_kernel, B * tiles, NTHR, 0, ST(stream), h0, rstd, x.da, x.dpool, p->v, recipe_id, stride_id, dh0, dhx, D);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -1094,19 +1109,19 @@ int phi_bwd_params_impl(const float* h0, const float* hx, const int32_t* recipe_
       set = true;
     }
   }
-  phi_pu_kernel<<<B * rte::ceil_div(d, NTHR), NTHR, smem_pu, ST(stream)>>>(h0, act, x.dupd, x.pu, x.pg, x.pb, D);
+  rte::launch(phi_pu_kernel, B * rte::ceil_div(d, NTHR), NTHR, smem_pu, ST(stream), h0, act, x.dupd, x.pu, x.pg, x.pb, D);
   RTE_LAUNCH_CHECK();
-  phi_pv_kernel<<<B * rte::ceil_div(d, PV_ROWS), NTHR, smem_pv, ST(stream)>>>(h0, hx, rstd, pooled, x.da, x.pv, D);
+  rte::launch(phi_pv_kernel, B * rte::ceil_div(d, PV_ROWS), NTHR, smem_pv, ST(stream), h0, hx, rstd, pooled, x.da, x.pv, D);
   RTE_LAUNCH_CHECK();
   const int n_keys = R * K_strides;
   const long long eu = (long long)m * d, ev = (long long)3 * d * m, ed = d;
-  phi_reduce_keys_kernel<<<dim3((unsigned)rte::ceil_div64(eu, NTHR), n_keys), NTHR, 0, ST(stream)>>>(x.pu, recipe_id, stride_id, g->u, B, K_strides, eu);
+  rte::launch(phi_reduce_keys_kernel, dim3((unsigned)rte::ceil_div64(eu, NTHR), n_keys), NTHR, 0, ST(stream), x.pu, recipe_id, stride_id, g->u, B, K_strides, eu);
   RTE_LAUNCH_CHECK();
-  phi_reduce_keys_kernel<<<dim3((unsigned)rte::ceil_div64(ev, NTHR), n_keys), NTHR, 0, ST(stream)>>>(x.pv, recipe_id, stride_id, g->v, B, K_strides, ev);
+  rte::launch(phi_reduce_keys_kernel, dim3((unsigned)rte::ceil_div64(ev, NTHR), n_keys), NTHR, 0, ST(stream), x.pv, recipe_id, stride_id, g->v, B, K_strides, ev);
   RTE_LAUNCH_CHECK();
-  phi_reduce_keys_kernel<<<dim3((unsigned)rte::ceil_div64(ed, NTHR), n_keys), NTHR, 0, ST(stream)>>>(x.pg, recipe_id, stride_id, g->gain, B, K_strides, ed);
+  rte::launch(phi_reduce_keys_kernel, dim3((unsigned)rte::ceil_div64(ed, NTHR), n_keys), NTHR, 0, ST(stream), x.pg, recipe_id, stride_id, g->gain, B, K_strides, ed);
   RTE_LAUNCH_CHECK();
-  phi_reduce_keys_kernel<<<dim3((unsigned)rte::ceil_div64(ed, NTHR), n_keys), NTHR, 0, ST(stream)>>>(x.pb, recipe_id, stride_id, g->bias, B, K_strides, ed);
+  rte::launch(phi_reduce_keys_kernel, dim3((unsigned)rte::ceil_div64(ed, NTHR), n_keys), NTHR, 0, ST(stream), x.pb, recipe_id, stride_id, g->bias, B, K_strides, ed);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -1149,9 +1164,9 @@ extern "C" int rte_macro_phi_bwd(const float* h0, const float* dout, const rte_p
 extern "C" int rte_sqdiff_grad(const float* a, const float* b, int64_t n, float coef, float* g, float* partial, float* sum_out,
                                int32_t accumulate, rte_stream_t stream) {
   RTE_CHECK_ARG(a && b && g && partial && sum_out && n > 0);
-  sqdiff_grad_kernel<<<SQD_BLOCKS, 256, 0, ST(stream)>>>(a, b, n, coef, g, partial);
+  rte::launch(sqdiff_grad_kernel, SQD_BLOCKS, 256, 0, ST(stream), a, b, n, coef, g, partial);
   RTE_LAUNCH_CHECK();
-  sqdiff_final_kernel<<<1, 1024, 0, ST(stream)>>>(partial, SQD_BLOCKS, sum_out, accumulate);
+  rte::launch(sqdiff_final_kernel, 1, 1024, 0, ST(stream), partial, SQD_BLOCKS, sum_out, accumulate);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }

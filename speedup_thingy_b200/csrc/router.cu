@@ -12,6 +12,7 @@ constexpr int NTHR = 256;
 
 __global__ void __launch_bounds__(NTHR)
 pool_kernel(const float* __restrict__ h0, float* __restrict__ pooled, int S, int d) {
+  rte::after_previous_grid();
   const int b = blockIdx.y, c = blockIdx.x * NTHR + threadIdx.x;
   if (c >= d) return;
   float acc = 0.f;
@@ -40,6 +41,7 @@ __global__ void __launch_bounds__(NTHR)
 router_hidden_kernel(const float* __restrict__ pooled, const float* __restrict__ w0a, const float* __restrict__ b0a,
                      float* __restrict__ prea, const float* __restrict__ w0b, const float* __restrict__ b0b,
                      float* __restrict__ preb, int B, int d, int hid) {
+  rte::after_previous_grid();
   extern __shared__ float xs[];                 // [RH_SAMPLES][d]
   const float* w0 = blockIdx.z == 0 ? w0a : w0b;
   const float* b0 = blockIdx.z == 0 ? b0a : b0b;
@@ -91,6 +93,7 @@ __device__ void head_logits(const float* __restrict__ pre, const float* __restri
 __global__ void __launch_bounds__(NTHR)
 router_fwd_kernel(rte_router_weights w, const int32_t* __restrict__ depth_values, rte_router_out o, int d, int hid,
                   int R, int K, int T, int fixed_recipe, int fixed_depth_id) {
+  rte::after_previous_grid();
   extern __shared__ float sm[];   // hs[hid]
   __shared__ float rl[RTE_ROUTER_MAX_R], dl[RTE_ROUTER_MAX_K];
   float* hs = sm;
@@ -135,6 +138,7 @@ __global__ void __launch_bounds__(NTHR)
 aux_kernel(const float* __restrict__ recipe_probs, const float* __restrict__ expected_depth, float lambda_load,
            float lambda_depth, float* __restrict__ aux, float* __restrict__ mean_prob, const float* __restrict__ mean_given,
            int B, int R) {
+  rte::after_previous_grid();
   __shared__ float red[32];
   __shared__ float mp[RTE_ROUTER_MAX_R];
   for (int r = threadIdx.x; r < R; r += NTHR) {
@@ -180,6 +184,7 @@ router_bwd_sample_kernel(rte_router_weights w, rte_router_out o, const int32_t* 
                          const float* __restrict__ mean_prob, float lambda_load, float lambda_depth,
                          float* __restrict__ dpre_r, float* __restrict__ dpre_d, float* __restrict__ dlog_r,
                          float* __restrict__ dlog_d, float* __restrict__ dh0, int B, int S, int d, int hid, int R, int K) {
+  rte::after_previous_grid();
   extern __shared__ float sm[];   // dhr[hid], dhd[hid]
   __shared__ float dlr[RTE_ROUTER_MAX_R], dld[RTE_ROUTER_MAX_K];
   float* dhr = sm;
@@ -211,6 +216,7 @@ router_bwd_sample_kernel(rte_router_weights w, rte_router_out o, const int32_t* 
 // dst[r,:] += sum_p vec[p][r / seg,:]   (nparts partial vectors, part_stride floats apart, added in fixed order)
 __global__ void bcast_add_kernel(float* __restrict__ dst, const float* __restrict__ vec, int rows, int seg, int d, int nparts,
                                  long long part_stride) {
+  rte::after_previous_grid();
   const long long total = (long long)rows * (d >> 2);
   const int d4 = d >> 2;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -230,6 +236,7 @@ __global__ void bcast_add_kernel(float* __restrict__ dst, const float* __restric
 __global__ void __launch_bounds__(NTHR)
 router_dpooled_kernel(const float* __restrict__ w0r, const float* __restrict__ w0d, const float* __restrict__ dpre_r,
                       const float* __restrict__ dpre_d, float* __restrict__ dpooled, int B, int S, int d, int hid) {
+  rte::after_previous_grid();
   extern __shared__ float sm[];            // sr[4][hid], sd[4][hid], comb[4][128]
   float* sr = sm;
   float* sd = sm + 4 * hid;
@@ -275,6 +282,7 @@ router_dpooled_kernel(const float* __restrict__ w0r, const float* __restrict__ w
 __global__ void __launch_bounds__(NTHR)
 router_dw0_kernel(const float* __restrict__ dpre, const float* __restrict__ pooled, float* __restrict__ dw0,
                   float* __restrict__ db0, int B, int d, int hid) {
+  rte::after_previous_grid();
   const long long i = blockIdx.x * (long long)NTHR + threadIdx.x;
   if (i >= (long long)hid * d) return;
   const int j = int(i / d), c = int(i % d);
@@ -292,6 +300,7 @@ router_dw0_kernel(const float* __restrict__ dpre, const float* __restrict__ pool
 __global__ void __launch_bounds__(NTHR)
 router_dw2_kernel(const float* __restrict__ dlog, const float* __restrict__ pre, float* __restrict__ dw2,
                   float* __restrict__ db2, int B, int hid, int nout) {
+  rte::after_previous_grid();
   __shared__ float sa[8][33], sb[8][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + tx;
@@ -340,12 +349,11 @@ extern "C" int rte_router_fwd(const float* h0, const rte_router_weights* w, cons
       set = true;
     }
   }
-  pool_kernel<<<dim3(rte::ceil_div(d, NTHR), B), NTHR, 0, ST(stream)>>>(h0, out->pooled, S, d);
+  rte::launch(pool_kernel, dim3(rte::ceil_div(d, NTHR), B), NTHR, 0, ST(stream), h0, out->pooled, S, d);
   RTE_LAUNCH_CHECK();
-  router_hidden_kernel<<<dim3(rte::ceil_div(hid, RH_ROWS), rte::ceil_div(B, RH_SAMPLES), 2), NTHR, smem_h, ST(stream)>>>(
-      out->pooled, w->r_w0, w->r_b0, out->r_hidden_pre, w->d_w0, w->d_b0, out->d_hidden_pre, B, d, hid);
+  rte::launch(router_hidden_kernel, dim3(rte::ceil_div(hid, RH_ROWS), rte::ceil_div(B, RH_SAMPLES), 2), NTHR, smem_h, ST(stream), out->pooled, w->r_w0, w->r_b0, out->r_hidden_pre, w->d_w0, w->d_b0, out->d_hidden_pre, B, d, hid);
   RTE_LAUNCH_CHECK();
-  router_fwd_kernel<<<B, NTHR, smem, ST(stream)>>>(*w, depth_values, *out, d, hid, R, K, T, fixed_recipe, fixed_depth_id);
+  rte::launch(router_fwd_kernel, B, NTHR, smem, ST(stream), *w, depth_values, *out, d, hid, R, K, T, fixed_recipe, fixed_depth_id);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -354,6 +362,7 @@ extern "C" int rte_router_fwd(const float* h0, const rte_router_weights* w, cons
 // the batch mean over the global batch, which rte_router_aux_bwd_data then takes as `mean_prob_in`.
 __global__ void __launch_bounds__(NTHR)
 mean_prob_kernel(const float* __restrict__ recipe_probs, float* __restrict__ out, float scale, int B, int R) {
+  rte::after_previous_grid();
   for (int r = threadIdx.x; r < R; r += NTHR) {
     float acc = 0.f;
     for (int b = 0; b < B; ++b) acc += recipe_probs[(size_t)b * R + r];
@@ -363,7 +372,7 @@ mean_prob_kernel(const float* __restrict__ recipe_probs, float* __restrict__ out
 
 extern "C" int rte_router_mean_prob(const float* recipe_probs, float* out, float scale, int32_t B, int32_t R, rte_stream_t stream) {
   RTE_CHECK_ARG(recipe_probs && out && B > 0 && R > 0 && R <= RTE_ROUTER_MAX_R);
-  mean_prob_kernel<<<1, NTHR, 0, ST(stream)>>>(recipe_probs, out, scale, B, R);
+  rte::launch(mean_prob_kernel, 1, NTHR, 0, ST(stream), recipe_probs, out, scale, B, R);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -385,25 +394,24 @@ extern "C" int rte_router_aux_bwd_data(const rte_router_weights* w, const rte_ro
   float* dlog_d = dlog_r + (size_t)B * R;           // [B, K]
   float* dpooled = scratch + (((size_t)RTE_ROUTER_MAX_R + (size_t)B * (2 * hid + R + K) + 3) & ~(size_t)3);   // [B, d], 16-byte aligned
   if (reinterpret_cast<uintptr_t>(scratch) & 15) return RTE_ERR_ALIGNMENT;
-  aux_kernel<<<1, NTHR, 0, ST(stream)>>>(fwd->recipe_probs, fwd->expected_depth, lambda_load, lambda_depth, aux, mean_prob,
+  rte::launch(aux_kernel, 1, NTHR, 0, ST(stream), fwd->recipe_probs, fwd->expected_depth, lambda_load, lambda_depth, aux, mean_prob,
                                          mean_prob_in, B, R);
   RTE_LAUNCH_CHECK();
   const size_t smem = (size_t)2 * hid * sizeof(float);
   if (smem > 48 * 1024) return RTE_ERR_UNSUPPORTED;
-  router_bwd_sample_kernel<<<B, NTHR, smem, ST(stream)>>>(*w, *fwd, depth_values, mean_prob, lambda_load, lambda_depth,
+  rte::launch(router_bwd_sample_kernel, B, NTHR, smem, ST(stream), *w, *fwd, depth_values, mean_prob, lambda_load, lambda_depth,
                                                           dpre_r, dpre_d, dlog_r, dlog_d, dh0, B, S, d, hid, R, K);
   RTE_LAUNCH_CHECK();
   const size_t smem_dp = (size_t)(8 * hid + 4 * 128) * sizeof(float);
   if (smem_dp > 48 * 1024) return RTE_ERR_UNSUPPORTED;
-  router_dpooled_kernel<<<dim3(rte::ceil_div(B, 4) * rte::ceil_div(d, 128), RTE_ROUTER_DPOOLED_PARTS), NTHR, smem_dp, ST(stream)>>>(
-      w->r_w0, w->d_w0, dpre_r, dpre_d, dpooled, B, S, d, hid);
+  rte::launch(router_dpooled_kernel, dim3(rte::ceil_div(B, 4) * rte::ceil_div(d, 128), RTE_ROUTER_DPOOLED_PARTS), NTHR, smem_dp, ST(stream), w->r_w0, w->d_w0, dpre_r, dpre_d, dpooled, B, S, d, hid);
   RTE_LAUNCH_CHECK();
   if (d % 4 != 0) return RTE_ERR_UNSUPPORTED;
   if (dh0) {
     long long n4 = (long long)B * S * (d / 4);
     int grid = (int)((n4 + NTHR - 1) / NTHR);
     if (grid > 148 * 8) grid = 148 * 8;
-    bcast_add_kernel<<<grid, NTHR, 0, ST(stream)>>>(dh0, dpooled, B * S, S, d, RTE_ROUTER_DPOOLED_PARTS, (long long)B * d);
+    rte::launch(bcast_add_kernel, grid, NTHR, 0, ST(stream), dh0, dpooled, B * S, S, d, RTE_ROUTER_DPOOLED_PARTS, (long long)B * d);
     RTE_LAUNCH_CHECK();
   }
   return RTE_OK;
@@ -419,7 +427,7 @@ extern "C" int rte_router_aux_add_dh0(float* dh0, const float* scratch, int32_t 
   long long n4 = (long long)B * S * (d / 4);
   int grid = (int)((n4 + NTHR - 1) / NTHR);
   if (grid > 148 * 8) grid = 148 * 8;
-  bcast_add_kernel<<<grid, NTHR, 0, ST(stream)>>>(dh0, dpooled, B * S, S, d, RTE_ROUTER_DPOOLED_PARTS, (long long)B * d);
+  rte::launch(bcast_add_kernel, grid, NTHR, 0, ST(stream), dh0, dpooled, B * S, S, d, RTE_ROUTER_DPOOLED_PARTS, (long long)B * d);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -434,13 +442,13 @@ extern "C" int rte_router_aux_bwd_params(const rte_router_out* fwd, const rte_ro
   float* dlog_r = dpre_d + (size_t)B * hid;
   float* dlog_d = dlog_r + (size_t)B * R;
   const int g0 = (int)rte::ceil_div64((long long)hid * d, NTHR);
-  router_dw0_kernel<<<g0, NTHR, 0, ST(stream)>>>(dpre_r, fwd->pooled, grads->r_w0, grads->r_b0, B, d, hid);
+  rte::launch(router_dw0_kernel, g0, NTHR, 0, ST(stream), dpre_r, fwd->pooled, grads->r_w0, grads->r_b0, B, d, hid);
   RTE_LAUNCH_CHECK();
-  router_dw0_kernel<<<g0, NTHR, 0, ST(stream)>>>(dpre_d, fwd->pooled, grads->d_w0, grads->d_b0, B, d, hid);
+  rte::launch(router_dw0_kernel, g0, NTHR, 0, ST(stream), dpre_d, fwd->pooled, grads->d_w0, grads->d_b0, B, d, hid);
   RTE_LAUNCH_CHECK();
-  router_dw2_kernel<<<rte::ceil_div(R * hid, 32), NTHR, 0, ST(stream)>>>(dlog_r, fwd->r_hidden_pre, grads->r_w2, grads->r_b2, B, hid, R);
+  rte::launch(router_dw2_kernel, rte::ceil_div(R * hid, 32), NTHR, 0, ST(stream), dlog_r, fwd->r_hidden_pre, grads->r_w2, grads->r_b2, B, hid, R);
   RTE_LAUNCH_CHECK();
-  router_dw2_kernel<<<rte::ceil_div(K * hid, 32), NTHR, 0, ST(stream)>>>(dlog_d, fwd->d_hidden_pre, grads->d_w2, grads->d_b2, B, hid, K);
+  rte::launch(router_dw2_kernel, rte::ceil_div(K * hid, 32), NTHR, 0, ST(stream), dlog_d, fwd->d_hidden_pre, grads->d_w2, grads->d_b2, B, hid, K);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }

@@ -33,6 +33,31 @@ namespace rte {
 __host__ __device__ inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 __host__ __device__ inline long long ceil_div64(long long a, long long b) { return (a + b - 1) / b; }
 
+// Programmatic dependent launch: a kernel launched with the attribute may start while the kernel before it in the stream
+// still runs.  grid_dependency_wait returns once that kernel has completed and its writes are visible (at once without the
+// attribute); nothing the kernel before may touch is read or written ahead of it.  grid_dependents_launch lets the next
+// such kernel begin its own set-up.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+__device__ __forceinline__ void after_previous_grid() { grid_dependency_wait(); grid_dependents_launch(); }
+
+// Launches a kernel that begins with after_previous_grid() so that its start overlaps the end of the kernel before it.
+template <typename... P, typename... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);      // (an error stays pending for RTE_LAUNCH_CHECK)
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(SB_WARPS * 32)
 shortlist_build_kernel(const int64_t* __restrict__ targets, const int32_t* __restrict__ top_clusters,
                        const int32_t* __restrict__ random_negs, int32_t* __restrict__ shortlist,
                        int32_t* __restrict__ dup_count, int rows, ShortlistDims D, int* status) {
+  rte::after_previous_grid();
   extern __shared__ uint32_t seen_all[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row = blockIdx.x * SB_WARPS + warp;
@@ -89,6 +90,7 @@ shortlist_ce_kernel(const __nv_bfloat16* __restrict__ hidden, const __nv_bfloat1
                     const int32_t* __restrict__ shortlist, const float* __restrict__ row_weight, int S,
                     float* __restrict__ loss_tok, __nv_bfloat16* __restrict__ logits_out,
                     __nv_bfloat16* __restrict__ dense, int d, int V, int K) {
+  rte::after_previous_grid();
   extern __shared__ float sm[];          // hs[d], lg[K]
   __shared__ float red[32];
   float* hs = sm;
@@ -138,6 +140,7 @@ shortlist_ce_kernel(const __nv_bfloat16* __restrict__ hidden, const __nv_bfloat1
 __global__ void __launch_bounds__(128)
 shortlist_ce_logits_kernel(__nv_bfloat16* __restrict__ logits, const int32_t* __restrict__ shortlist,
                            const float* __restrict__ row_weight, int S, float* __restrict__ loss_tok, int V, int K) {
+  rte::after_previous_grid();
   extern __shared__ float lg[];          // [K]
   __shared__ float red[32];
   const int row = blockIdx.x;
@@ -166,6 +169,7 @@ shortlist_ce_logits_kernel(__nv_bfloat16* __restrict__ logits, const int32_t* __
 __global__ void __launch_bounds__(128)
 scatter_cols_kernel(const __nv_bfloat16* __restrict__ vals, const int32_t* __restrict__ ids, __nv_bfloat16* __restrict__ dense,
                     int V, int K) {
+  rte::after_previous_grid();
   const int row = blockIdx.x;
   uint4* dr = reinterpret_cast<uint4*>(dense + (size_t)row * V);
   for (int i = threadIdx.x; i < V / 8; i += blockDim.x) dr[i] = make_uint4(0u, 0u, 0u, 0u);
@@ -178,6 +182,7 @@ scatter_cols_kernel(const __nv_bfloat16* __restrict__ vals, const int32_t* __res
 
 // out[i] = hash(seed, i) mod vocab  (counter-based, reproducible; used when no host-drawn negatives are supplied)
 __global__ void random_tokens_kernel(int32_t* __restrict__ out, long long n, int vocab, const int64_t* __restrict__ seed) {
+  rte::after_previous_grid();
   const unsigned long long s = (unsigned long long)(*seed);
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     unsigned long long z = s * 0x9E3779B97F4A7C15ull + (unsigned long long)i + 0x632BE59BD9B4E019ull;
@@ -208,8 +213,7 @@ extern "C" int rte_shortlist_build(const int64_t* targets, const int32_t* top_cl
       set = true;
     }
   }
-  shortlist_build_kernel<<<rte::ceil_div(rows, SB_WARPS), SB_WARPS * 32, smem, ST(stream)>>>(
-      targets, top_clusters, random_negs ? random_negs : top_clusters, shortlist, dup_count, rows, D, status);
+  rte::launch(shortlist_build_kernel, rte::ceil_div(rows, SB_WARPS), SB_WARPS * 32, smem, ST(stream), targets, top_clusters, random_negs ? random_negs : top_clusters, shortlist, dup_count, rows, D, status);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -222,7 +226,7 @@ extern "C" int rte_shortlist_ce(const void* hidden, const void* W, const int32_t
   if ((reinterpret_cast<uintptr_t>(W) & 15) || (dlogits_dense && (reinterpret_cast<uintptr_t>(dlogits_dense) & 15))) return RTE_ERR_ALIGNMENT;
   const size_t smem = (size_t)(d + K) * sizeof(float);
   if (smem > 48 * 1024) return RTE_ERR_UNSUPPORTED;
-  shortlist_ce_kernel<<<rows, 128, smem, ST(stream)>>>(reinterpret_cast<const __nv_bfloat16*>(hidden),
+  rte::launch(shortlist_ce_kernel, rows, 128, smem, ST(stream), reinterpret_cast<const __nv_bfloat16*>(hidden),
       reinterpret_cast<const __nv_bfloat16*>(W), shortlist, row_weight, S, loss_tok,
       reinterpret_cast<__nv_bfloat16*>(logits_out), reinterpret_cast<__nv_bfloat16*>(dlogits_dense), d, V, K);
   RTE_LAUNCH_CHECK();
@@ -235,7 +239,7 @@ extern "C" int rte_shortlist_ce_from_logits(void* logits_inout, const int32_t* s
   if (reinterpret_cast<uintptr_t>(logits_inout) & 15) return RTE_ERR_ALIGNMENT;
   const size_t smem = (size_t)K * sizeof(float);
   if (smem > 48 * 1024) return RTE_ERR_UNSUPPORTED;
-  shortlist_ce_logits_kernel<<<rows, 128, smem, ST(stream)>>>(reinterpret_cast<__nv_bfloat16*>(logits_inout), shortlist, row_weight,
+  rte::launch(shortlist_ce_logits_kernel, rows, 128, smem, ST(stream), reinterpret_cast<__nv_bfloat16*>(logits_inout), shortlist, row_weight,
                                                              S, loss_tok, V, K);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -245,7 +249,7 @@ extern "C" int rte_scatter_cols_bf16(const void* vals, const int32_t* ids, void*
                                      rte_stream_t stream) {
   RTE_CHECK_ARG(vals && ids && dense && rows > 0 && V > 0 && V % 8 == 0 && K > 0);
   if (reinterpret_cast<uintptr_t>(dense) & 15) return RTE_ERR_ALIGNMENT;
-  scatter_cols_kernel<<<rows, 128, 0, ST(stream)>>>(reinterpret_cast<const __nv_bfloat16*>(vals), ids,
+  rte::launch(scatter_cols_kernel, rows, 128, 0, ST(stream), reinterpret_cast<const __nv_bfloat16*>(vals), ids,
                                                     reinterpret_cast<__nv_bfloat16*>(dense), V, K);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -255,7 +259,7 @@ extern "C" int rte_random_tokens(int32_t* out, int64_t n, int32_t vocab, const i
   RTE_CHECK_ARG(out && seed && n > 0 && vocab > 0);
   long long g = (n + 255) / 256;
   if (g > 148 * 8) g = 148 * 8;
-  random_tokens_kernel<<<(int)g, 256, 0, ST(stream)>>>(out, n, vocab, seed);
+  rte::launch(random_tokens_kernel, (int)g, 256, 0, ST(stream), out, n, vocab, seed);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }

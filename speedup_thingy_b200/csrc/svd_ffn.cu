@@ -181,6 +181,7 @@ __global__ void __launch_bounds__(SEL_MAX_WARPS * 32, 4)
 svd_select_kernel(const float* __restrict__ hats, const __nv_bfloat16* __restrict__ ug, const float* __restrict__ wn,
                   __nv_bfloat16* __restrict__ z_masked, uint8_t* __restrict__ selected, int32_t* __restrict__ cand_count,
                   int rows, int F, int up_m, int gate_m, int product_m, int top_k) {
+  rte::after_previous_grid();
   extern __shared__ __align__(16) uint8_t sm_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, n4 = F / 4;
   uint8_t* base = sm_raw + warp * sel_warp_bytes(F);
@@ -262,6 +263,7 @@ __device__ __forceinline__ void swiglu_grad(bool on, float u, float g, float d, 
 __global__ void __launch_bounds__(256)
 svd_swiglu_bwd8_kernel(const __nv_bfloat16* __restrict__ ug, const __nv_bfloat16* __restrict__ dz, const uint8_t* __restrict__ selected,
                        __nv_bfloat16* __restrict__ dug, long long groups, int f8) {
+  rte::after_previous_grid();
   const uint4* ug8 = reinterpret_cast<const uint4*>(ug);
   const uint4* dz8 = reinterpret_cast<const uint4*>(dz);
   const uint2* sel8 = reinterpret_cast<const uint2*>(selected);
@@ -296,6 +298,7 @@ svd_swiglu_bwd8_kernel(const __nv_bfloat16* __restrict__ ug, const __nv_bfloat16
 __global__ void __launch_bounds__(256)
 svd_swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ ug, const __nv_bfloat16* __restrict__ dz, const uint8_t* __restrict__ selected,
                       __nv_bfloat16* __restrict__ dug, long long rows, int F) {
+  rte::after_previous_grid();
   const long long total = rows * F;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const long long r = i / F;
@@ -308,6 +311,7 @@ svd_swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ ug, const __nv_bfloat16*
 }
 
 __global__ void row_norm_kernel(const float* __restrict__ w, float* __restrict__ out, int rows, int d) {
+  rte::after_previous_grid();
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   float s = 0.f;
@@ -345,8 +349,7 @@ extern "C" int rte_svd_ffn_select(const float* hats, const void* ug, const float
   const int sms = rte_device_sm_count();
   int grid = rte::ceil_div(rows, warps);
   if (grid > sms * resident) grid = sms * resident;
-  svd_select_kernel<<<grid, warps * 32, warps * warp_bytes, ST(stream)>>>(
-      hats, reinterpret_cast<const __nv_bfloat16*>(ug), wd_norm, reinterpret_cast<__nv_bfloat16*>(z_masked), selected, cand_count,
+  rte::launch(svd_select_kernel, grid, warps * 32, warps * warp_bytes, ST(stream), hats, reinterpret_cast<const __nv_bfloat16*>(ug), wd_norm, reinterpret_cast<__nv_bfloat16*>(z_masked), selected, cand_count,
       rows, F, up_m, gate_m, product_m, top_k);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
@@ -362,16 +365,16 @@ extern "C" int rte_svd_ffn_swiglu_bwd(const void* ug, const void* dz, const uint
   long long g = ((wide ? rows * F / 8 : rows * F) + 255) / 256;
   if (g > 148 * 16) g = 148 * 16;
   if (wide)
-    svd_swiglu_bwd8_kernel<<<(int)g, 256, 0, ST(stream)>>>(u, z, selected, out, rows * (F / 8), F / 8);
+    rte::launch(svd_swiglu_bwd8_kernel, (int)g, 256, 0, ST(stream), u, z, selected, out, rows * (F / 8), F / 8);
   else
-    svd_swiglu_bwd_kernel<<<(int)g, 256, 0, ST(stream)>>>(u, z, selected, out, rows, F);
+    rte::launch(svd_swiglu_bwd_kernel, (int)g, 256, 0, ST(stream), u, z, selected, out, rows, F);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
 
 extern "C" int rte_row_norm_f32(const float* w, float* out, int32_t rows, int32_t d, rte_stream_t stream) {
   RTE_CHECK_ARG(w && out && rows > 0 && d > 0);
-  row_norm_kernel<<<rte::ceil_div(rows, 8), 256, 0, ST(stream)>>>(w, out, rows, d);
+  rte::launch(row_norm_kernel, rte::ceil_div(rows, 8), 256, 0, ST(stream), w, out, rows, d);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
