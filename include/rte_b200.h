@@ -93,9 +93,10 @@ typedef struct rte_gemm_args {
    * [split_kblocks[s], split_kblocks[s+1]) (device int32 [splits+1]) into C + s*split_stride; an empty range gives
    * zeros.  RTE_EPI_F32 only.  NULL = equal splits.                                                             */
   const int32_t* split_kblocks;
-  /* Tile shape (0 = chosen by the library).  tile_n: 128 or 256 columns per tile.  cta_pair: 1 = every tile is
-   * 128 rows on one CTA; otherwise a product with more than 128 rows (and neither grouping nor ragged splits) runs
-   * 256-row tiles on pairs of CTAs (tcgen05 cta_group::2), each CTA loading half of the tile's B operand.       */
+  /* Both 0: the library picks the kernel (this one, rte_gemm_bf16_tile or rte_gemm_bf16_small) and its tile by size.
+   * Otherwise the persistent kernel runs with tile_n = 128 or 256 columns per tile (0: either) and cta_pair = 1: tiles
+   * of 128 rows on one CTA; 2: 256-row tiles on pairs of CTAs (tcgen05 cta_group::2, each CTA loading half of the
+   * tile's B operand) where the product has more than 128 rows and neither grouping nor ragged splits; 0: either.  */
   int32_t tile_n;
   int32_t cta_pair;
   /* rte_gemm_bf16_small with splits > 1 only: reduce the partial results inside the launch.  The CTA that finishes
@@ -108,9 +109,16 @@ typedef struct rte_gemm_args {
 } rte_gemm_args;
 
 int rte_gemm_bf16(const rte_gemm_args* args, rte_stream_t stream);
-/* The tile shape rte_gemm_bf16 would use for `args` (M, N, epilogue, grouping, tile hints and max_ctas are read) and
+/* How many splits (1 .. max_splits) a product with fp32 output and a long reduction should be cut into when its partials
+ * are added by rte_reduce_splits; 1: one rte_gemm_bf16 launch is faster.                                             */
+int rte_gemm_wgrad_splits(const rte_gemm_args* args, int32_t max_splits);
+/* The tile shape the persistent kernel would use for `args` (M, N, epilogue, grouping, tile hints and max_ctas are read) and
  * how many tiles run at the same time: what a caller needs to choose a split count.  Any output may be NULL.  */
 int rte_gemm_tile_plan(const rte_gemm_args* args, int32_t* tile_m, int32_t* tile_n, int32_t* concurrent_tiles);
+/* The same product for FEW TILES: one 128 x tile_n tile per CTA (tile_n 64 or 128), the reduction split over the `ksplit`
+ * (1..8, at most one per 64-wide k-block) CTAs of a cluster, which add their partial tiles in rank order.  RTE_EPI_BF16 or
+ * RTE_EPI_F32 (+R); no grouping, no splits; either major for either operand.                                       */
+int rte_gemm_bf16_tile(const rte_gemm_args* args, int32_t tile_n, int32_t ksplit, rte_stream_t stream);
 /* The same product for FEW ROWS (the audited samples' replay, models.py:605-679: M = one or two samples): one
  * 128-thread CTA per 64x64 output tile, cp.async + mma.sync, no tensor maps or TMEM set-up, so a dependent chain of
  * such launches is not dominated by set-up time.  Subset of rte_gemm_args: A K-major, B either major, RTE_EPI_BF16

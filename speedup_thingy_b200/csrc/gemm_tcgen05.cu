@@ -27,10 +27,9 @@
 // slow axis), which is what the weight- and data-gradient GEMMs of the training
 // step need; no transposed copies are ever made.
 
-#include <cuda.h>
 #include <stdlib.h>
 
-#include "rte_common.cuh"
+#include "tcgen05_ptx.cuh"
 
 namespace {
 
@@ -41,7 +40,6 @@ constexpr int NUM_THREADS = 320;   // warp 0 producer, warp 1 MMA issuer, warps 
 constexpr int EPI_WARPS = 8;
 constexpr int SLOT_BYTES = 4096;       // one epilogue staging slot: 32 rows x 128 bytes
 constexpr int MAX_DYN_SMEM = 232448;   // 227 KB of dynamic shared memory per CTA
-constexpr uint32_t WAIT_LIMIT = 24u * 1000u * 1000u;   // polls (with back-off) before a wait gives up
 
 #ifdef RTE_GEMM_DIAG
 constexpr bool DIAG = true;    // timing diagnostics: RTE_GEMM_DIAG_FLAGS bit 0 = no stores, 1 = no MMAs, 2 = no loads
@@ -67,172 +65,6 @@ struct KParams {
   const int* split_kb;      // ragged split-K: k-block range [split_kb[s], split_kb[s+1]) of split s, else null
   int* status;
 };
-
-// ------------------------------------------------------------------ PTX wrappers
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
-
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-// Address of this CTA's shared-memory location `addr` as seen in CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t mapa_cluster(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-// Arrive on a barrier of another CTA of the cluster (`bar` is a shared::cluster address from mapa_cluster).
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-template <int CTAS>
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  if (CTAS == 1) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-  } else {      // arrivals may come from the peer CTA: cluster-scope acquire
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-  }
-  return ok != 0;
-}
-// Bounded wait: returns false when the limit ran out.
-template <int CTAS>
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-  for (uint32_t i = 0; i < WAIT_LIMIT; ++i) {
-    if (mbar_test<CTAS>(bar, parity)) return true;
-    if (i > 128) __nanosleep(i > 4096 ? 128 : 32);
-  }
-  return false;
-}
-__device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-// `bar`: CTAS = 1 the CTA's own barrier; CTAS = 2 the LEADER CTA's barrier (shared::cluster address), which counts the
-// bytes of both CTAs' loads.
-template <int CTAS>
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
-  if (CTAS == 1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-        : "memory");
-  } else {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
-        : "memory");
-  }
-}
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t src, int x, int y, int z) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(x), "r"(y), "r"(z)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-__device__ __forceinline__ void prefetch_tmap(const CUtensorMap* map) {
-  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
-}
-
-template <int CTAS>
-__device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
-  if (CTAS == 1) asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols) : "memory");
-  else asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols) : "memory");
-}
-template <int CTAS>
-__device__ __forceinline__ void tmem_relinquish() {
-  if (CTAS == 1) asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  else asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-template <int CTAS>
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-  if (CTAS == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-  else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// Arrives on `bar` once the MMAs issued so far have completed; CTAS = 2: on the barrier at the same offset in BOTH CTAs.
-template <int CTAS>
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  if (CTAS == 1) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-  } else {
-    const uint16_t both = 3;
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                 ::"r"(bar), "h"(both) : "memory");
-  }
-}
-template <int CTAS>
-__device__ __forceinline__ void tc_mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  if (CTAS == 1) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-  }
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// Shared-memory matrix descriptor (128-byte swizzle, descriptor version 1 for sm_100).
-//  K-major tile : rows of 128 B, 8-row groups 1024 B apart (stride byte offset), leading offset unused.
-//  MN-major tile: 64-element (128 B) runs along MN, 8 k-rows per 1024 B atom (stride byte offset),
-//                 next 64 MN elements 8192 B further (leading byte offset).
-__device__ __forceinline__ uint64_t make_smem_desc(uint32_t saddr, bool mn_major) {
-  uint64_t desc = static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
-  desc |= static_cast<uint64_t>(mn_major ? (8192u >> 4) : 1u) << 16;
-  desc |= static_cast<uint64_t>(1024u >> 4) << 32;
-  desc |= 1ull << 46;
-  desc |= 2ull << 61;
-  return desc;
-}
 
 // ------------------------------------------------------------------ epilogue helpers
 // SiLU / sigmoid for the fused epilogues: ex2.approx + the fast divide (2 ulp), with no slow path for huge or
@@ -374,17 +206,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     tmem_alloc<CTAS>(tmem_slot, TMEM_COLS);     // CTAS = 2: one warp of EACH CTA of the pair takes part
     tmem_relinquish<CTAS>();
   }
+  rte::grid_dependency_wait();
   tc_fence_before();
   if (CTAS == 2) cluster_sync_all(); else __syncthreads();     // barriers of both CTAs are initialised beyond here
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot_ptr;
+  rte::grid_dependents_launch();
 
   const int tiles = p.num_m_blocks * p.num_n_blocks;
   const int total_work = tiles * p.splits;
 
   if (warp == 0) {
     // ---------------- TMA producer (in both CTAs of a pair: each fills its own shared memory) ----------------
-    if (lane == 0) {
+    // (the whole warp runs the loop; one elected lane issues -- see elect_one)
+    {
       int stage = 0; uint32_t phase = 0; bool ok = true;
       for (int w = unit; w < total_work && ok; w += n_units) {
         const int split = w / tiles, t = w % tiles;
@@ -400,16 +235,17 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const int kb1 = p.split_kb ? p.split_kb[split + 1] : min(kb0 + p.kblocks_per_split, p.kblocks_total);
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait<CTAS>(empty_bar(stage), phase ^ 1u)) {
-            if (p.status) atomicExch(p.status, RTE_DEV_WAIT_TIMEOUT_PRODUCER);
+            if (p.status && lane == 0) atomicExch(p.status, RTE_DEV_WAIT_TIMEOUT_PRODUCER);
             *err_flag = 1;
             ok = false; break;
           }
           const uint32_t sa = smem_base + stage * L::STAGE_BYTES, sb = sa + L::A_BYTES;
           if (DIAG && (p.diag & 4)) {
-            if (leader) mbar_arrive(full_bar(stage));
+            if (leader && lane == 0) mbar_arrive(full_bar(stage));
             if (++stage == STAGES) { stage = 0; phase ^= 1u; }
             continue;
           }
+          if (elect_one()) {
           // the leader's barrier counts the bytes of both CTAs' loads of this stage
           if (leader) mbar_arrive_expect_tx(full_bar(stage), L::STAGE_BYTES * CTAS);
           const uint32_t fb = (CTAS == 2) ? mapa_cluster(full_bar(stage), 0) : full_bar(stage);
@@ -438,17 +274,19 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             for (int j = 0; j < L::B_ROWS / 64; ++j)
               tma_load_2d<CTAS>(sb + j * 8192, &tmap_b, fb, n0 + c_lo + 64 * j, boff + k0);
           }
+          }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
       }
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (one thread; with CTAS = 2 the leader CTA's, for both CTAs) ----------------
-    if (lane == 0 && leader) {
+    if (leader) {
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(p.a_mn) << 15) | (uint32_t(p.b_mn) << 16) |
                              (uint32_t(BN >> 3) << 17) | (uint32_t((BM * CTAS) >> 4) << 24);
       const uint32_t a_step = p.a_mn ? (UMMA_K * 128u) >> 4 : (UMMA_K * 2u) >> 4;
       const uint32_t b_step = p.b_mn ? (UMMA_K * 128u) >> 4 : (UMMA_K * 2u) >> 4;
+      const uint64_t adesc0 = make_smem_desc(smem_base, p.a_mn != 0), bdesc0 = make_smem_desc(smem_base + L::A_BYTES, p.b_mn != 0);
       int stage = 0; uint32_t phase = 0; int acc = 0; uint32_t acc_phase = 0; bool ok = true;
       for (int w = unit; w < total_work && ok; w += n_units) {
         const int split = w / tiles;
@@ -456,7 +294,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const int kb0 = p.split_kb ? p.split_kb[split] : split * p.kblocks_per_split;
         const int kb1 = p.split_kb ? p.split_kb[split + 1] : min(kb0 + p.kblocks_per_split, p.kblocks_total);
         if (!mbar_wait<CTAS>(tempty_bar(acc), acc_phase ^ 1u)) {
-          if (p.status) atomicExch(p.status, RTE_DEV_WAIT_TIMEOUT_MMA);
+          if (p.status && lane == 0) atomicExch(p.status, RTE_DEV_WAIT_TIMEOUT_MMA);
           *err_flag = 1;
           ok = false; break;
         }
@@ -464,23 +302,24 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait<CTAS>(full_bar(stage), phase)) {
-            if (p.status) atomicExch(p.status, RTE_DEV_WAIT_TIMEOUT_MMA);
+            if (p.status && lane == 0) atomicExch(p.status, RTE_DEV_WAIT_TIMEOUT_MMA);
             *err_flag = 1;
             ok = false; break;
           }
           tc_fence_after();
-          const uint32_t sa = smem_base + stage * L::STAGE_BYTES, sb = sa + L::A_BYTES;
-          const uint64_t adesc = make_smem_desc(sa, p.a_mn != 0), bdesc = make_smem_desc(sb, p.b_mn != 0);
-          if (!(DIAG && (p.diag & 2)))
+          const uint64_t off = uint64_t(uint32_t(stage) * uint32_t(L::STAGE_BYTES >> 4));     // (addresses stay below the field's end)
+          if (elect_one()) {
+            if (!(DIAG && (p.diag & 2)))
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k)
-            tc_mma_bf16<CTAS>(d_tmem, adesc + uint64_t(k * a_step), bdesc + uint64_t(k * b_step), idesc,
-                              (kb > kb0 || k > 0) ? 1u : 0u);
-          tc_commit<CTAS>(empty_bar(stage));       // frees the stage (in both CTAs) once these MMAs have read it
+            for (int k = 0; k < BK / UMMA_K; ++k)
+              tc_mma_bf16<CTAS>(d_tmem, adesc0 + off + uint64_t(k * a_step), bdesc0 + off + uint64_t(k * b_step), idesc,
+                                (kb > kb0 || k > 0) ? 1u : 0u);
+            tc_commit<CTAS>(empty_bar(stage));       // frees the stage (in both CTAs) once these MMAs have read it
+          }
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
-        tc_commit<CTAS>(tfull_bar(acc));           // accumulator complete -> epilogue (of both CTAs)
+        if (elect_one()) tc_commit<CTAS>(tfull_bar(acc));           // accumulator complete -> epilogue (of both CTAs)
         if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
       }
     }
@@ -783,7 +622,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       }
       if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
     }
-    if (lane == 0) bulk_wait_all();            // this warp's stores have left shared memory and reached global memory
+    if (lane == 0) bulk_wait_read<0>();        // this warp's stores have left shared memory (the grid's end makes them visible)
   }
 
   // ---------------- teardown ----------------
@@ -802,38 +641,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 }
 
 // ------------------------------------------------------------------ host side
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn get_encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (fn == nullptr) {
-    void* sym = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres) != cudaSuccess ||
-        qres != cudaDriverEntryPointSuccess)
-      return nullptr;
-    fn = reinterpret_cast<EncodeTiledFn>(sym);
-  }
-  return fn;
-}
-
-// 2-D bf16 tensor map over a row-major [rows, cols] matrix with row stride ld: box = box_cols x box_rows,
-// 128-byte swizzle, out-of-range elements read as zero.
-int make_tmap(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld, int box_cols, int box_rows) {
-  EncodeTiledFn fn = get_encode_fn();
-  if (!fn) return RTE_ERR_TENSOR_MAP;
-  cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2ull};
-  cuuint32_t box[2] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows)};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? RTE_OK : RTE_ERR_TENSOR_MAP;
-}
-
 // 3-D tensor map for the epilogue's bulk stores: [planes, rows, cols] with a box of 32 rows x 128 bytes
 // (64 bf16 or 32 fp32 columns) and the 128-byte swizzle of the staging slots.
 int make_store_tmap(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld, long long planes,
@@ -851,17 +658,83 @@ int make_store_tmap(CUtensorMap* map, const void* base, long long rows, long lon
   return r == CUDA_SUCCESS ? RTE_OK : RTE_ERR_TENSOR_MAP;
 }
 
-// Tile shape of a product: BN columns per tile, one CTA (128 rows) or a CTA pair (256 rows) per tile.
+// ------------------------------------------------------------------ which kernel, which tile
+// Times in microseconds fitted to measurements (launches in a graph, operands in L2, M 64..16384, N 128..5000, K 64..8192):
+// a launch costs a set-up and epilogue that depend on the tile and on what is written, plus a main loop whose k-blocks
+// take longer once every SM pulls its operands from L2.  Picked by the sum: many tiles -> 256-row pairs (least operand
+// traffic), one wave of tiles or less -> the smallest tile that still fits one wave, few tiles with a long reduction -> the
+// reduction split over a cluster (gemm_tile.cu), a short reduction with few rows -> mma.sync tiles (gemm_small.cu).
+// Against one fixed rule (256-column pairs above 128 rows), e.g. 512 x 384 x 128: 6.6 -> 2.6 us, 512 x 384 x 1152 with
+// residual 17.3 -> 6.3 us, 1050 x 512 x 4096: 26.4 -> 12 us, 5000 x 384 x 384 with residual 13.9 -> 5.9 us.
 struct TileConfig { int bn, ctas; };
+struct Choice { int kernel; TileConfig tile; int ksplit; float us; };      // kernel: 0 persistent, 1 cluster tile, 2 mma.sync
 
-TileConfig pick_tile(const rte_gemm_args* a) {
+float persistent_us(const rte_gemm_args* a, TileConfig t, int splits, int sms) {
+  const int i = (t.bn == 256 ? 0 : 2) + (t.ctas == 2 ? 0 : 1);              // 256 pair | 256 | 128 pair | 128
+  static const float base_bf16[4] = {5.2f, 4.0f, 4.5f, 3.2f}, base_f32[4] = {6.3f, 5.4f, 5.3f, 3.9f}, base_res[4] = {10.1f, 8.9f, 7.5f, 5.7f};
+  static const float slope_idle[4] = {0.277f, 0.27f, 0.19f, 0.20f}, slope_busy[4] = {0.36f, 0.38f, 0.24f, 0.25f};
+  static const float store_bf16[4] = {2.6f, 1.7f, 1.85f, 1.1f};             // a further tile's stores, when longer than its main loop
+  const bool f32 = a->epilogue == RTE_EPI_F32, res = f32 && a->R != nullptr;
+  const int cols = a->epilogue == RTE_EPI_SWIGLU_FWD ? 2 * a->b_pair_offset : a->N;
+  const int units = rte::ceil_div(a->M, BM * t.ctas) * rte::ceil_div(cols, t.bn) * splits;
+  const int conc = (a->max_ctas > 0 ? a->max_ctas : sms) / t.ctas, waves = rte::ceil_div(units, conc > 0 ? conc : 1);
+  const float kb = float(rte::ceil_div(rte::ceil_div(a->K, BK), splits));
+  const float slope = waves > 1 ? slope_busy[i] : slope_idle[i] + (slope_busy[i] - slope_idle[i]) * float(units) / float(conc);
+  const float store = store_bf16[i] * (res ? 3.8f : f32 ? 2.f : 1.f);
+  const float loop = kb * slope;
+  return (res ? base_res[i] : f32 ? base_f32[i] : base_bf16[i]) + loop + float(waves - 1) * (loop > store ? loop : store);
+}
+
+float tile_us(const rte_gemm_args* a, int bn, int ksplit, int sms) {
+  const int grid = rte::ceil_div(a->M, BM) * rte::ceil_div(a->N, bn) * ksplit, kb = rte::ceil_div(a->K, BK);
+  const float full = float(a->max_ctas > 0 ? a->max_ctas : sms) / float(sms);
+  // clusters of 2 / 4 / 8 that are resident together (a cluster sits inside one GPC)
+  const int limit = int(full * (ksplit == 1 ? 148.f : ksplit == 2 ? 146.f : ksplit == 4 ? 132.f : 112.f));
+  if (ksplit > kb || grid > 2 * limit || (ksplit > 1 && grid > limit)) return 1e9f;
+  static const float base64[4] = {3.0f, 4.3f, 3.9f, 4.2f}, base128[4] = {4.1f, 6.2f, 5.4f, 5.4f};
+  const float base = (bn == 64 ? base64 : base128)[ksplit == 1 ? 0 : ksplit == 2 ? 1 : ksplit == 4 ? 2 : 3];
+  const float per = float(rte::ceil_div(kb, ksplit)) * 0.21f, f32 = a->epilogue == RTE_EPI_F32 ? (bn == 64 ? 0.2f : 0.5f) : 0.f;
+  return base + f32 + (grid <= limit ? per : 1.f + 2.2f * per);
+}
+
+float small_us(const rte_gemm_args* a) {
+  if (a->K % 8 != 0 || a->a_mn_major || (a->b_mn_major && a->N % 8 != 0)) return 1e9f;
+  const int rows = rte::ceil_div(a->M, 64), wide = rte::ceil_div(a->N, 64) * rows, ctas = wide < 74 ? rte::ceil_div(a->N, 32) * rows : wide;
+  if (ctas > 148) return 1e9f;
+  const float kb = float(rte::ceil_div(a->K, BK));
+  return 2.0f + (a->R != nullptr ? 0.2f : 0.f) + kb * (wide < 74 ? 0.28f : 0.53f);
+}
+
+TileConfig pick_tile(const rte_gemm_args* a, int splits, int sms, float* us = nullptr) {
   const bool grouped = a->tile_group != nullptr || a->split_kblocks != nullptr;   // per-128-row-block bookkeeping
-  TileConfig c;
-  c.ctas = (!grouped && a->M > BM) ? 2 : 1;
-  if (a->cta_pair == 1) c.ctas = 1;
-  c.bn = (a->N >= 192) ? 256 : 128;
-  if (a->tile_n == 128 || a->tile_n == 256) c.bn = a->tile_n;
-  if (a->epilogue == RTE_EPI_SWIGLU_FWD) c.bn = 256;       // the paired epilogue takes 64 (up, gate) pairs per warp
+  TileConfig best = {256, 1};
+  float best_us = 1e30f;
+  for (int bn = 128; bn <= 256; bn += 128)
+    for (int ctas = 1; ctas <= 2; ++ctas) {
+      if (ctas == 2 && (grouped || a->cta_pair == 1 || a->M <= BM)) continue;
+      if (ctas == 1 && a->cta_pair == 2 && !grouped && a->M > BM) continue;
+      if ((a->tile_n == 128 || a->tile_n == 256) && bn != a->tile_n) continue;
+      if (a->epilogue == RTE_EPI_SWIGLU_FWD && bn != 256) continue;            // the paired epilogue takes 64 (up, gate) pairs per warp
+      const float t = persistent_us(a, {bn, ctas}, splits, sms);
+      if (t < best_us) { best_us = t; best = {bn, ctas}; }
+    }
+  if (us) *us = best_us;
+  return best;
+}
+
+Choice choose(const rte_gemm_args* a, int splits, int sms) {
+  Choice c = {0, {0, 0}, 1, 0.f};
+  c.tile = pick_tile(a, splits, sms, &c.us);
+  if (a->tile_n != 0 || a->cta_pair != 0 || splits > 1 || a->tile_group != nullptr || a->split_kblocks != nullptr ||
+      (a->epilogue != RTE_EPI_BF16 && a->epilogue != RTE_EPI_F32))
+    return c;
+  for (int bn = 64; bn <= 128; bn += 64)
+    for (int ks = 1; ks <= 8; ks *= 2) {
+      const float t = tile_us(a, bn, ks, sms);
+      if (t < c.us) c = {1, {bn, 1}, ks, t};
+    }
+  const float t = small_us(a);
+  if (t < c.us) c = {2, {0, 0}, 1, t};
   return c;
 }
 
@@ -911,10 +784,12 @@ int launch(const rte_gemm_args* a, const CUtensorMap& ta, const CUtensorMap& tb,
   cfg.blockDim = dim3(NUM_THREADS);
   cfg.dynamicSmemBytes = L::TOTAL;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CTAS; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr; cfg.numAttrs = (CTAS == 2) ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = CTAS; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = (CTAS == 2) ? 2 : 1;
   if (cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, CTAS>, ta, tb, tc, tc2, kp) != cudaSuccess) {
     (void)cudaGetLastError();
     return RTE_ERR_LAUNCH;
@@ -937,7 +812,7 @@ extern "C" int rte_device_sm_count(void) {
 
 extern "C" int rte_gemm_tile_plan(const rte_gemm_args* a, int32_t* tile_m, int32_t* tile_n, int32_t* concurrent) {
   RTE_CHECK_ARG(a != nullptr && a->M > 0 && a->N > 0);
-  const TileConfig c = pick_tile(a);
+  const TileConfig c = pick_tile(a, a->splits < 1 ? 1 : a->splits, rte_device_sm_count());
   if (tile_m) *tile_m = BM * c.ctas;
   if (tile_n) *tile_n = c.bn;
   if (concurrent) {
@@ -949,6 +824,22 @@ extern "C" int rte_gemm_tile_plan(const rte_gemm_args* a, int32_t* tile_m, int32
     *concurrent = u;
   }
   return RTE_OK;
+}
+
+extern "C" int rte_gemm_wgrad_splits(const rte_gemm_args* a, int32_t max_splits) {
+  if (a == nullptr || a->M <= 0 || a->N <= 0 || a->K <= 0) return 1;
+  const int sms = rte_device_sm_count(), kb = rte::ceil_div(a->K, BK);
+  if (sms <= 0) return 1;
+  float best = choose(a, 1, sms).us;
+  int splits = 1;
+  for (int s = 2; s <= max_splits && s * 4 <= kb; ++s) {
+    if (rte::ceil_div(kb, rte::ceil_div(kb, s)) != s) continue;               // every split gets k-blocks
+    float us;
+    pick_tile(a, s, sms, &us);
+    us += 1.8f + float(s + 1) * float(a->M) * float(a->N) * 4e-6f / 5.f;        // ... and one launch adds the partials
+    if (us < best) { best = us; splits = s; }
+  }
+  return splits;
 }
 
 extern "C" int rte_gemm_bf16(const rte_gemm_args* a, rte_stream_t stream) {
@@ -966,8 +857,12 @@ extern "C" int rte_gemm_bf16(const rte_gemm_args* a, rte_stream_t stream) {
   }
   if (swiglu_b) RTE_CHECK_ARG(a->R != nullptr && a->b_pair_offset == a->N);
 
-  const TileConfig tile = pick_tile(a);
-  const int bn = tile.bn, ctas = tile.ctas;
+  const int sms = rte_device_sm_count();
+  if (sms <= 0) return RTE_ERR_NO_DEVICE;
+  const Choice c = choose(a, splits, sms);
+  if (c.kernel == 1) return rte_gemm_bf16_tile(a, c.tile.bn, c.ksplit, stream);
+  if (c.kernel == 2) return rte_gemm_bf16_small(a, stream);
+  const int bn = c.tile.bn, ctas = c.tile.ctas;
 
   KParams kp;
   kp.diag = 0;
@@ -1046,8 +941,6 @@ extern "C" int rte_gemm_bf16(const rte_gemm_args* a, rte_stream_t stream) {
   kp.tma_store = tma_ok ? 1 : 0;
   if (DIAG && (kp.diag & 16)) kp.tma_store = 0;
 
-  const int sms = rte_device_sm_count();
-  if (sms <= 0) return RTE_ERR_NO_DEVICE;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (ctas == 2)
     return bn == 256 ? launch<256, 2>(a, ta, tb, tc, tc2, kp, sms, st) : launch<128, 2>(a, ta, tb, tc, tc2, kp, sms, st);

@@ -44,7 +44,8 @@ class CudaOps:
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.launches = 0          # kernels-entry calls issued (for bench accounting)
         self._split_ws: torch.Tensor | None = None
-        self.small_gemm_rows = 256  # products with at most this many rows go to the few-row kernel (0: never)
+        self._splits: dict[tuple[int, int, int, int], int] = {}      # pick_splits by size
+        self.small_gemm_rows = 256  # split products with at most this many rows go to the few-row kernel (0: every product to the persistent kernel)
         # ... and so can weight gradients over that few rows (RTE_SMALL_WGRAD=1).  Off by default: inside the training
         # step its hundreds of small CTAs on the replay's high-priority stream displace the hot pass (measured 2.04 ms
         # per step against 1.72 ms with these products on the tcgen05 kernel's 32 tiles).
@@ -57,8 +58,8 @@ class CudaOps:
         self._split_counters = torch.zeros(1024, dtype=torch.int32, device=self.device)      # per-tile arrival counters
         self.few_rows_max_splits = int(os.environ.get("RTE_FEWROW_SPLITS", "4"))
         self.gemm_max_ctas = 0     # 0 = one persistent CTA per SM; smaller values leave SMs to kernels of other streams
-        # tile hints passed to every tcgen05 GEMM (0 = the library's choice): RTE_GEMM_PAIR=0 keeps every tile on one
-        # CTA (no cta_group::2 pairs), RTE_GEMM_TILE_N forces 128 or 256 columns per tile
+        # tile hints passed to every GEMM (0 = the library's choice of kernel and tile): RTE_GEMM_PAIR=0 keeps every tile on
+        # one CTA of the persistent kernel, RTE_GEMM_TILE_N forces it with 128 or 256 columns per tile
         self.gemm_cta_pair = 1 if os.environ.get("RTE_GEMM_PAIR", "1") == "0" else 0
         self.gemm_tile_n = int(os.environ.get("RTE_GEMM_TILE_N", "0"))
         # When set, launches that only produce PARAMETER gradients (weight-gradient GEMMs with their split reduction,
@@ -124,33 +125,27 @@ class CudaOps:
         args.n_groups, args.b_group_stride = n_groups, b_group_stride
         args.split_kblocks = split_kblocks.data_ptr() if split_kblocks is not None else None
         args.tile_n = self.gemm_tile_n if tile_n is None else tile_n
-        args.cta_pair = self.gemm_cta_pair if cta_pair is None else cta_pair
+        args.cta_pair = cta_pair if cta_pair is not None else 2 if (self.small_gemm_rows == 0 and not self.gemm_cta_pair) else self.gemm_cta_pair
         if split_reduce is not None:          # (counters, final output, accumulate): the few-row kernel reduces its splits itself
             args.split_counters, args.split_out = split_reduce[0].data_ptr(), split_reduce[1].data_ptr()
             args.split_accumulate = int(split_reduce[2])
-        # few output rows, or (weight gradient of a few rows: A and B stored [K, *]) a reduction over few rows
+        # few output rows with split-K partials for a consumer that sums them, or (weight gradient of a few rows: A and B
+        # stored [K, *]) a reduction over few rows; every other product goes to the kernel the library picks by size
         few_rows = (epilogue in (A.EPI_BF16, A.EPI_F32) and tile_group is None and split_kblocks is None and K % 8 == 0
                     and (not b_mn or N % 8 == 0)
-                    and ((not a_mn and M <= self.small_gemm_rows)
+                    and ((not a_mn and M <= self.small_gemm_rows and splits > 1)
                          or (a_mn and b_mn and self.small_wgrad and K <= self.small_gemm_rows and epilogue == A.EPI_F32 and M % 8 == 0 and splits == 1)))
         self._call("rte_gemm_bf16_small" if few_rows else "rte_gemm_bf16", C.byref(args), self.stream)
 
     def pick_splits(self, M: int, N: int, K: int) -> int:
         """Split count for a reduction-heavy GEMM whose output has few tiles (weight gradients)."""
-        args = A.GemmArgs()
-        args.M, args.N, args.K, args.epilogue = M, N, K, A.EPI_F32
-        args.max_ctas, args.tile_n, args.cta_pair = self.gemm_max_ctas, self.gemm_tile_n, self.gemm_cta_pair
-        tm, tn, conc = C.c_int32(0), C.c_int32(0), C.c_int32(0)
-        A.check(self.lib.rte_gemm_tile_plan(C.byref(args), C.byref(tm), C.byref(tn), C.byref(conc)), "rte_gemm_tile_plan")
-        tiles = -(-M // tm.value) * -(-N // tn.value)
-        kblocks = -(-K // 64)
-        want = max(1, min(conc.value // max(tiles, 1), kblocks // 8 if kblocks >= 16 else 1, 16))
-        while want > 1:
-            per = -(-kblocks // want)
-            if -(-kblocks // per) == want:
-                break
-            want -= 1
-        return max(want, 1)
+        key = (M, N, K, self.gemm_max_ctas)
+        if key not in self._splits:
+            args = A.GemmArgs()
+            args.M, args.N, args.K, args.epilogue, args.a_mn_major, args.b_mn_major = M, N, K, A.EPI_F32, 1, 1
+            args.max_ctas, args.tile_n, args.cta_pair = self.gemm_max_ctas, self.gemm_tile_n, self.gemm_cta_pair
+            self._splits[key] = int(self.lib.rte_gemm_wgrad_splits(C.byref(args), 16))
+        return self._splits[key]
 
     def gemm_wgrad(self, a_t, b_t, out, *, M: int, N: int, K: int, accumulate: bool = False,
                    lda: int | None = None, ldb: int | None = None, ws=None) -> None:

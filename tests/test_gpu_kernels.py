@@ -56,6 +56,36 @@ def test_gemm_bf16_all_majors(ops, M, N, K, a_mn, b_mn):
     _close(out, ref, 1e-2, f"gemm {M}x{N}x{K} a_mn={a_mn} b_mn={b_mn}")
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (70, 104, 136), (300, 200, 136), (200, 136, 520), (1050, 384, 1152), (512, 64, 2048)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+def test_gemm_cluster_tiles(ops, M, N, K, a_mn, b_mn):
+    """rte_gemm_bf16_tile: both tile widths, every split of the reduction over a cluster, ragged rows / columns / k-blocks,
+    each epilogue (a residual in place among them)."""
+    if (a_mn and M % 8) or (b_mn and N % 8):
+        pytest.skip("MN-major operands need an MN extent that is a multiple of 8")
+    import ctypes as C
+
+    from speedup_thingy_b200 import _abi as A
+    g = torch.Generator().manual_seed(M + N + K)
+    a, b, r = _bf(torch.randn(M, K, generator=g)), _bf(torch.randn(N, K, generator=g)), torch.randn(M, N, generator=g)
+    ref = a.float() @ b.float().t()
+    a_dev, b_dev = (a.t().contiguous() if a_mn else a).to(DEV), (b.t().contiguous() if b_mn else b).to(DEV)
+    args = A.GemmArgs()
+    args.M, args.N, args.K, args.splits, args.status = M, N, K, 1, ops.status.data_ptr()
+    args.A, args.lda, args.a_mn_major = a_dev.data_ptr(), a_dev.stride(0), int(a_mn)
+    args.B, args.ldb, args.b_mn_major = b_dev.data_ptr(), b_dev.stride(0), int(b_mn)
+    for bn in (64, 128):
+        for ks in (k for k in (1, 2, 3, 8) if k <= -(-K // 64)):
+            for mode in ("bf16", "f32", "f32_residual"):
+                out = r.to(DEV) if mode == "f32_residual" else torch.full((M, N), 7.0, device=DEV, dtype=torch.bfloat16 if mode == "bf16" else torch.float32)
+                args.C, args.ldc, args.epilogue = out.data_ptr(), N, A.EPI_BF16 if mode == "bf16" else A.EPI_F32
+                args.R, args.ldr = (out.data_ptr(), N) if mode == "f32_residual" else (None, 0)
+                A.check(ops.lib.rte_gemm_bf16_tile(C.byref(args), bn, ks, ops.stream), "rte_gemm_bf16_tile")
+                torch.cuda.synchronize()
+                ops.check_status()
+                _close(out, ref + r if mode == "f32_residual" else ref, 1e-2 if mode == "bf16" else 2e-3, f"{M}x{N}x{K} tile {bn} ksplit {ks} {mode}")
+
+
 @pytest.mark.parametrize("M,N,K", [(64, 1536, 512), (64, 512, 4096), (70, 104, 136), (256, 2048, 512), (1, 8, 8), (130, 96, 72)])
 @pytest.mark.parametrize("b_mn", [False, True])
 @pytest.mark.parametrize("mode", ["bf16", "f32_residual", "f32_split"])
