@@ -496,7 +496,7 @@ def main() -> None:
                                           "all": [m / K for m in ms_regions]},
             "e2e": {"value": tokens * K / (ms_e2e / 1e3), "unit": "tokens/s",
                     "h2d_bytes_per_step": 2 * B * S * 8 + (4 * eng.audit_k + B * 4 if eng.audit is not None else 0),
-                    "d2h_bytes_per_step": eng._results.numel() * 4 + 4,
+                    "d2h_bytes_per_step": eng._results.numel() * 4,
                     "api": "TrainEngine.train_steps(batches): two steps in flight, each step's loss read on the host",
                     "regions_ms_per_step": [m / K for m in e2e_regions],
                     "synchronous_train_step": tokens * K / (ms_e2e_sync / 1e3)},

@@ -427,6 +427,8 @@ int rte_grad_norm_multi_tensor(const rte_adamw_tensor* table, int64_t total_chun
  *   against slot 0 -> loss_tok; logits_out bf16 [rows, K] optional; dlogits_dense bf16 [rows, V] (optional) receives
  *   row_weight[row/S] * (softmax - onehot(0)) at the shortlisted ids and zero elsewhere.
  * rte_random_tokens: counter-based pseudo-random ids in [0, vocab) from a device-resident seed.                 */
+/* Host: out[i] = what torch.randint(0, range, ..., generator=torch.Generator().manual_seed(seed)) draws, 0 < range < 2^28. */
+int rte_host_randint(uint64_t seed, int64_t n, int32_t range, int32_t* out);
 int rte_shortlist_build(const int64_t* targets, const int32_t* top_clusters, const int32_t* random_negs,
                         int32_t* shortlist, int32_t* dup_count, int32_t rows, int32_t V, int32_t C, int32_t TC,
                         int32_t HN, int32_t RN, int32_t K, int32_t* status, rte_stream_t stream);

@@ -99,7 +99,7 @@ class AuditReplay:
         (the `recursive_exact` mode, where no hot pass shares them) instead of a private mirror."""
         from .engine import _Block, _Temps
 
-        self.eng, self.k = eng, k
+        self.eng, self.k, self.direct = eng, k, direct_grads
         self._stage = None
         self._prepared = None
         self._prelude_copied = None
@@ -196,8 +196,9 @@ class AuditReplay:
         PR = 128
         self.partials = [[(e(PR, d), e(PR, d), e(PR, d)) for _ in range(2)] for _ in range(T)]
         self.coda_tmps = [_Temps(Ma, cfg, dev) for _ in range(cfg.n_coda)]
-        self.dx16_alt = e(Ma, d, dtype=bf)
-        self.P = 64
+        # bf16 gradient between the coda blocks: one buffer each, the deferred weight gradients still read them
+        self.coda_dx16 = [self.tmp.dx16] + [e(Ma, d, dtype=bf) for _ in range(cfg.n_coda)]
+        self.P = 296               # partial sums per pass of the scalar parameters' gradients (one per CTA of their launch)
         self.part_alpha, self.part_attn, self.part_mlp = e(T * self.P), e(T * self.P), e(T * self.P)
         # The replay runs on its own stream beside the hot pass, so the gradients it contributes to parameters the
         # hot pass also touches (final norm, coda, tied embedding) are written to a private mirror of those slices of
@@ -243,31 +244,24 @@ class AuditReplay:
 
     # ------------------------------------------------------------------ host side, once per step
     def prepare(self, step_seed: int) -> None:
-        """Host half of `choose` for a coming step: the seeded permutation and the control-variate weights, written to
-        a pinned staging pair.  Three pairs rotate: with up to two steps queued on the device, the pair written here for
-        step i+2 is the one step i-1 used, whose copy has completed by the time that step was collected."""
+        """Host half of `choose` for a coming step: the seeded permutation and the control-variate weights.  (The padded
+        samplers write theirs to a pinned staging set.  Three sets rotate: with up to two steps queued on the device, the
+        set written here for step i+2 is the one step i-1 used, whose copy has completed by the time that step was
+        collected.)"""
         eng = self.eng
         if self.bernoulli:
             return self._prepare_bernoulli(step_seed)
         if self.scheduled:
             return self._prepare_scheduled(step_seed)
-        if self._stage is None:
-            pin = eng.device.type == "cuda"
-            self._stage = [(torch.empty(self.k, dtype=torch.int32, pin_memory=pin),
-                            torch.empty(eng.B, dtype=torch.float32, pin_memory=pin)) for _ in range(3)]
-            self._stage_next = 0
         gen = torch.Generator().manual_seed(step_seed)
         chosen = torch.sort(torch.randperm(eng.B, generator=gen)[: self.k]).values
-        h_idx, h_rw = self._stage[self._stage_next]
         w0 = 1.0 / (eng.B * eng.S * eng.loss_div)
-        h_idx.copy_(chosen)
-        h_rw.fill_(w0)
+        rw = torch.full((eng.B,), w0, dtype=torch.float32)
         if self.grad and self.clip is None:
-            h_rw[chosen] = w0 * (1.0 - 1.0 / self.p_inc)                 # d corrected / d hot on audited samples
+            rw[chosen] = w0 * (1.0 - 1.0 / self.p_inc)                   # d corrected / d hot on audited samples
         # (with a residual clip the factor depends on the losses: `clip_hot` applies it on the device;
         #  without gradient correction the audited samples keep their plain weight)
-        self._prepared = (step_seed, chosen, h_idx, h_rw)
-        self._stage_next = (self._stage_next + 1) % 3
+        self._prepared = (step_seed, chosen, rw)
 
     def _prepare_bernoulli(self, step_seed: int) -> None:
         """Host half of the Bernoulli sampler: the uniforms `torch.bernoulli(p, generator)` compares p with (the same
@@ -356,9 +350,10 @@ class AuditReplay:
         if eng._core_absent is not None:
             eng._core_absent.mul_(eng._none_audited)      # stays 1 only while nobody has been audited in this cycle
 
-    def choose(self, step_seed: int) -> None:
+    def choose(self, step_seed: int, image: dict) -> None:
         """Fixed-count sampler: first k entries of a seeded CPU permutation (audit.py:99-116); writes the subset
-        indices and the control-variate weights of the hot rows."""
+        indices and the control-variate weights of the hot rows into the host `image` of the step's inputs (the padded
+        samplers queue copies of their own staging sets)."""
         eng = self.eng
         if self._prepared is None or self._prepared[0] != step_seed:
             self.prepare(step_seed)
@@ -380,10 +375,10 @@ class AuditReplay:
                 eng._none_audited.copy_(h_none, non_blocking=True)
             self.last_chosen = chosen
             return
-        _, chosen, h_idx, h_rw = self._prepared
+        _, chosen, rw = self._prepared
         self._prepared = None
-        self.idx.copy_(h_idx, non_blocking=True)
-        eng.row_weight.copy_(h_rw, non_blocking=True)
+        image["idx"].copy_(chosen)
+        image["row_weight"].copy_(rw)
         self.last_chosen = chosen
 
     # ------------------------------------------------------------------ forward
@@ -605,11 +600,10 @@ class AuditReplay:
         o.rmsnorm_bwd(self.x_last, p["final_norm.weight"], self.rstd_f, t.dn16, None, t.dxa, t.dx16,
                       gs["final_norm.weight"], t.partial)
         dcur, dalt = t.dxa, t.dxb
-        in16, out16 = t.dx16, self.dx16_alt          # distinct: the deferred wd gradient still reads the block's input
         for i, blk in enumerate(reversed(self.coda)):
-            eng._block_bwd(blk, dcur, in16, dalt, out16, t.dxc, tmp=self.coda_tmps[i], mark_ready=False, grads=gs, ws=self.ws)
+            eng._block_bwd(blk, dcur, self.coda_dx16[i], dalt, self.coda_dx16[i + 1], t.dxc, tmp=self.coda_tmps[i], mark_ready=False, grads=gs,
+                           ws=self.ws)
             dcur, dalt = dalt, dcur
-            in16, out16 = out16, in16
         self._defer_param_grads(False)
         # the head's weight gradients are queued: `merge_head` may add them to the hot pass's from here on
         self.head_w_done = None
@@ -699,7 +693,7 @@ class AuditReplay:
         self._defer_param_grads(False)
         if not self.own_prelude:                      # (own_prelude: `finish_core` does this off the chain)
             self._scalar_grads()
-            if eng._param_stream is not None:         # the replay's stream ends only when its weight gradients have
+            if eng._param_stream is not None and not self.direct:      # the replay's stream ends only when its weight gradients have
                 torch.cuda.current_stream(eng.device).wait_stream(eng._param_stream)
 
     # ------------------------------------------------------------------ the grouped block (recursive_deferred_grouped_exact)
@@ -800,8 +794,6 @@ class AuditReplay:
             o.gemm_wgrad(st["n1"], st["dqkv16"], g["core.attn.wqkv"][0], M=d, N=3 * d, K=K, ws=self.ws)
         self._defer_param_grads(False)
         self._scalar_grads()
-        if eng._param_stream is not None:
-            torch.cuda.current_stream(eng.device).wait_stream(eng._param_stream)
 
     def _scalar_grads(self) -> None:
         """Scalar parameters of the core: per-CTA partial sums -> gradients, in fixed order (slots of part_* beyond the
@@ -917,38 +909,40 @@ class AuditReplay:
     def loss_terms(self, hot_per_sample: torch.Tensor, host: dict, chosen: torch.Tensor | None = None) -> dict[str, float]:
         """Host-side assembly of the audited quantities for the reported loss (training.py:1381-1385) from the
         step's fetched results (`terms`, `exact_loss`, `kl_sum` already on the host)."""
-        tr, n, Ma, d = self.eng.tr, self.n, self.Ma, self.eng.cfg.d_model
+        eng = self.eng
+        tr, n, Ma, d = eng.tr, self.n, self.Ma, eng.cfg.d_model
         temp = max(float(tr.distill_temperature), 1e-6)
         if self.padded:
             return self._loss_terms_padded(hot_per_sample, host, temp)
-        terms = host["terms"]
-        exact = host["exact_loss"].clone()
-        hot = hot_per_sample[self.last_chosen if chosen is None else chosen]
-        aux = dict(delta_dir=tr.lambda_delta_dir * float(terms[:, 0].mean()),
-                   delta_rms=tr.lambda_delta_rms * float(terms[:, 1].mean()),
-                   endpoint_normed=tr.lambda_endpoint_normed * float(terms[:, 2].sum()) / (Ma * d),
-                   endpoint_raw=tr.lambda_endpoint_raw * float(terms[:, 3].sum()) / (Ma * d),
-                   kl=tr.lambda_kl * float(host["kl_sum"]) / n * temp * temp)
-        residual = exact - hot
+        # (plain numbers: a handful of samples, and a tensor operation costs a microsecond each)
+        vals, r0 = host["vals"], 8 + 2 * eng.B
+        terms, exact = vals[r0:r0 + 4 * n], vals[r0 + 4 * n:r0 + 5 * n]
+        hot = [vals[8 + i] for i in (self.last_chosen if chosen is None else chosen).tolist()]
+        aux = dict(delta_dir=tr.lambda_delta_dir * sum(terms[0::4]) / n, delta_rms=tr.lambda_delta_rms * sum(terms[1::4]) / n,
+                   endpoint_normed=tr.lambda_endpoint_normed * sum(terms[2::4]) / (Ma * d),
+                   endpoint_raw=tr.lambda_endpoint_raw * sum(terms[3::4]) / (Ma * d),
+                   kl=tr.lambda_kl * vals[r0 + 5 * n] / n * temp * temp)
+        residual = [x - h for x, h in zip(exact, hot)]
         res = self.residual_metrics(residual)
         if self.clip_reported is not None:
-            residual = residual.clamp(-float(self.clip_reported), float(self.clip_reported))
-        res["clipped_loss_residual"] = float(residual.mean())
+            c = float(self.clip_reported)
+            residual = [min(max(r, -c), c) for r in residual]
+        res["clipped_loss_residual"] = sum(residual) / n
         # the control variate is part of the loss only under gradient correction; its value is reported either way
-        corr = float((residual / self.p_inc).sum())
-        align = self.alignment_metrics(host["align"], float(hot.mean()) / self.S, float(exact.mean()) / self.S,
-                                       kl1=self._kl1_total(host, temp))
+        corr = sum(residual) / self.p_inc
+        sums = [vals[r0 + 5 * n + 1 + 8 * i:r0 + 5 * n + 9 + 8 * i] for i in range(n)]
+        align = self.alignment_metrics(sums, sum(hot) / n / self.S, sum(exact) / n / self.S, kl1=self._kl1_total(host, temp))
         return dict(correction=corr if self.grad else 0.0, correction_metric=corr, exact=exact, aux=aux, alignment=align,
                     residual=res)
 
     @staticmethod
-    def residual_metrics(residual: torch.Tensor) -> dict[str, float]:
+    def residual_metrics(residual: list[float]) -> dict[str, float]:
         """audit.py:306-310,363: mean / std / variance (population) of exact - hot over the audited samples, before
         any clip."""
-        r = residual.double()
-        var = float(r.var(unbiased=False)) if r.numel() else 0.0
-        return dict(audit_residual_mean=float(r.mean()), audit_residual_std=var ** 0.5, audit_residual_var=var,
-                    loss_residual=float(r.mean()))
+        n = len(residual)
+        mean = sum(residual) / n if n else math.nan
+        var = sum((r - mean) ** 2 for r in residual) / n if n else 0.0
+        return dict(audit_residual_mean=mean, audit_residual_std=var ** 0.5, audit_residual_var=var, loss_residual=mean)
 
     def _kl1_total(self, host: dict, temp: float) -> float | None:
         """Sum over the audited rows of KL(exact || hot) at temperature 1 (None with the shortlist head, which keeps no
@@ -958,27 +952,29 @@ class AuditReplay:
             return None
         return float(host["kl_sum"]) if temp == 1.0 else float(host["align"][0, 7])
 
-    def alignment_metrics(self, sums: torch.Tensor, hot_nll: float | None = None, exact_nll: float | None = None,
+    def alignment_metrics(self, sums: list[list[float]], hot_nll: float | None = None, exact_nll: float | None = None,
                           kl1: float | None = None) -> dict:
         """macro_alignment_metrics and compute_residual_metrics (macro.py:499-546, audit.py:207-243) from the
         per-sample sums of `rte_audit_alignment_sums` (`sums`: the audited samples' rows only) and the summed
         temperature-1 KL of the audited rows' logits (`kl1`)."""
-        L = float(self.S * self.eng.cfg.d_model)
-        s = sums.double()
-        ab, aa, bb, dd, pp, ee, pe = (s[:, k] for k in range(7))
-        eps = 1e-8
-        cos = (ab / (aa.sqrt().clamp_min(eps) * bb.sqrt().clamp_min(eps))).mean()
-        dcos = (pe / (pp.sqrt().clamp_min(eps) * ee.sqrt().clamp_min(eps))).mean()
-        macro_norm, exact_norm = (aa / L).sqrt().mean(), (bb / L).sqrt().mean()
-        pred_rms, exact_rms = (pp / L).sqrt().mean(), (ee / L).sqrt().mean()
-        out = dict(hidden_cosine_exact_macro=float(cos), hidden_mse_exact_macro=float(dd.sum() / (L * s.shape[0])),
-                   macro_norm=float(macro_norm), exact_norm=float(exact_norm),
-                   macro_exact_norm_ratio=float(macro_norm / exact_norm.clamp_min(1e-8)),
-                   delta_cosine_exact_macro=float(dcos), delta_rms_exact=float(exact_rms), delta_rms_pred=float(pred_rms),
-                   delta_rms_ratio=float(pred_rms / exact_rms.clamp_min(1e-8)))
+        L, n, eps = float(self.S * self.eng.cfg.d_model), len(sums), 1e-8
+        root = math.sqrt
+
+        def mean(values) -> float:
+            return sum(values) / n
+
+        # columns: a.b, a.a, b.b, |a - b|^2, p.p, e.e, p.e  (a, b: endpoints; p, e: their deltas to h0)
+        cos = mean(s[0] / (max(root(s[1]), eps) * max(root(s[2]), eps)) for s in sums)
+        dcos = mean(s[6] / (max(root(s[4]), eps) * max(root(s[5]), eps)) for s in sums)
+        macro_norm, exact_norm = mean(root(s[1] / L) for s in sums), mean(root(s[2] / L) for s in sums)
+        pred_rms, exact_rms = mean(root(s[4] / L) for s in sums), mean(root(s[5] / L) for s in sums)
+        out = dict(hidden_cosine_exact_macro=cos, hidden_mse_exact_macro=sum(s[3] for s in sums) / (L * n),
+                   macro_norm=macro_norm, exact_norm=exact_norm, macro_exact_norm_ratio=macro_norm / max(exact_norm, 1e-8),
+                   delta_cosine_exact_macro=dcos, delta_rms_exact=exact_rms, delta_rms_pred=pred_rms,
+                   delta_rms_ratio=pred_rms / max(exact_rms, 1e-8))
         out.update(hidden_cosine=out["hidden_cosine_exact_macro"], hidden_residual_l2=out["hidden_mse_exact_macro"] ** 0.5)
         if kl1 is not None:
-            out["logit_kl_exact_macro"] = out["logit_kl"] = kl1 / (s.shape[0] * self.S)
+            out["logit_kl_exact_macro"] = out["logit_kl"] = kl1 / (n * self.S)
         if hot_nll is not None and exact_nll is not None:
             out["hot_exact_nll_gap"] = hot_nll - exact_nll
         return out
@@ -994,7 +990,7 @@ class AuditReplay:
                    p_inclusion=float(stats[3]))
         zero = dict(delta_dir=0.0, delta_rms=0.0, endpoint_normed=0.0, endpoint_raw=0.0, kl=0.0)
         if a == 0:
-            return dict(correction=0.0, correction_metric=0.0, exact=host["exact_loss"][:0].clone(), aux=zero, **out)
+            return dict(correction=0.0, correction_metric=0.0, exact=[], aux=zero, **out)
         terms, exact, inv_p = host["terms"][:a], host["exact_loss"][:a].clone(), host["audit_inv_p"][:a]
         aux = dict(delta_dir=tr.lambda_delta_dir * float(terms[:, 0].mean()),
                    delta_rms=tr.lambda_delta_rms * float(terms[:, 1].mean()),
@@ -1002,12 +998,12 @@ class AuditReplay:
                    endpoint_raw=tr.lambda_endpoint_raw * float(terms[:, 3].sum()) / (a * S * d),
                    kl=tr.lambda_kl * float(host["kl_sum"]) / a * temp * temp)
         residual = exact - hot_per_sample[chosen]
-        res = self.residual_metrics(residual)
+        res = self.residual_metrics(residual.tolist())
         if self.clip_reported is not None:
             residual = residual.clamp(-float(self.clip_reported), float(self.clip_reported))
         res["clipped_loss_residual"] = float(residual.mean())
         corr = float((residual * inv_p).sum())
-        align = self.alignment_metrics(host["align"][:a], float(hot_per_sample[chosen].mean()) / S, float(exact.mean()) / S,
+        align = self.alignment_metrics(host["align"][:a].tolist(), float(hot_per_sample[chosen].mean()) / S, float(exact.mean()) / S,
                                        kl1=self._kl1_total(host, temp))
-        return dict(correction=corr if self.grad else 0.0, correction_metric=corr, exact=exact, aux=aux, alignment=align,
+        return dict(correction=corr if self.grad else 0.0, correction_metric=corr, exact=exact.tolist(), aux=aux, alignment=align,
                     residual=res, **out)

@@ -252,6 +252,45 @@ class _Block:
         self.x_in: torch.Tensor | None = None
 
 
+class _StepInputs:
+    """What the host hands the device per step -- [audited ids | loss weights | tokens | targets] -- in one device
+    allocation with three pinned host images in rotation (as many as steps can be in flight plus one), so that a step's
+    inputs are one host-to-device copy whatever the batch tensors are."""
+
+    def __init__(self, B: int, S: int, k: int, device: torch.device, neg: int = 0):
+        def up(n: int) -> int:
+            return -(-n // 256) * 256
+
+        self.shapes = [("idx", torch.int32, (k,)), ("row_weight", torch.float32, (B,)), ("tokens", torch.int64, (B, S)),
+                       ("targets", torch.int64, (B, S)), ("negatives", torch.int32, (B * S, neg))]
+        self.offsets, total = {}, 0
+        for name, dt, shape in self.shapes:
+            self.offsets[name] = total
+            total += up(math.prod(shape) * torch.empty(0, dtype=dt).element_size())
+        self.total = total
+        self.flat = torch.zeros(total, dtype=torch.uint8, device=device)
+        self.dev = self.views(self.flat)
+        self.images = [torch.zeros(total, dtype=torch.uint8, pin_memory=device.type == "cuda") for _ in range(3)]
+        self.host = [self.views(t) for t in self.images]
+        self.next = 0
+
+    def views(self, flat: torch.Tensor) -> dict[str, torch.Tensor]:
+        out = {}
+        for name, dt, shape in self.shapes:
+            lo = self.offsets[name]
+            out[name] = flat[lo:lo + math.prod(shape) * torch.empty(0, dtype=dt).element_size()].view(dt).view(shape)
+        return out
+
+    def image(self) -> int:
+        i, self.next = self.next, (self.next + 1) % 3
+        return i
+
+    def send(self, i: int, first: str, last: str | None = None) -> None:
+        """Image i from field `first` up to (not including) field `last`, stream-ordered."""
+        lo, hi = self.offsets[first], self.total if last is None else self.offsets[last]
+        self.flat[lo:hi].copy_(self.images[i][lo:hi], non_blocking=True)
+
+
 class _Temps:
     """Scratch tensors of one block-backward pass over M tokens (reused by every block)."""
 
@@ -276,6 +315,7 @@ class TrainEngine:
         self.config = config
         self.cfg, self.tr = config.model, config.training
         self.device = torch.device(device)
+        own_ops = ops is None
         if ops is None:
             from .ops import CudaOps  # raises when CUDA or the library is missing: no fallback
             ops = CudaOps(self.device)
@@ -469,8 +509,11 @@ class TrainEngine:
         # ---- activations
         M, d, V, B, S = self.M, cfg.d_model, cfg.vocab_size, self.B, self.S
         e = lambda *shape, dtype=f32: torch.empty(*shape, dtype=dtype, device=dev)  # noqa: E731
-        self.tokens = torch.zeros(B, S, dtype=torch.int64, device=dev)
-        self.targets = torch.zeros(B, S, dtype=torch.int64, device=dev)
+        # (a padded audit draws or stages its subset and loss weights in its own buffers)
+        self._own_subset = bool(self.audit_k) and not self.audit_padded
+        self.inputs = _StepInputs(B, S, self.audit_k if self._own_subset else 0, dev,
+                                  self.oc.random_negatives if self.shortlist else 0)
+        self.tokens, self.targets = self.inputs.dev["tokens"], self.inputs.dev["targets"]
         self.embed_accum = torch.zeros(cfg.vocab_size * cfg.d_model, dtype=torch.int64, device=dev)   # embed_bwd scratch
         self.x0 = e(M, d)
         if self.dense:
@@ -484,19 +527,24 @@ class TrainEngine:
         self.logits = e(M, V, dtype=bf)
         # Everything the host reads back after a step lives in ONE buffer, so that it is one device-to-host copy:
         #   scalars[8] | loss_per_sample[B] | recipe_id[B] (int32) | audit terms[k,4] | audit exact_loss[k] | kl_sum[1]
-        #   | per metric group (sum grad^2, sum param^2)
+        #   | per metric group (sum grad^2, sum param^2) | status word (int32)
         k_a = self.audit_k or 0
         n_mg = len(METRIC_GROUPS)
         # (Bernoulli sampler, scheduled count: + audited sample ids[k] (int32) | 1 / inclusion probability[k] | sampler
         #  statistics[4];  every audit: + alignment sums[k,8] (macro.py:499-546)
         self._audit_extra = 8 * k_a + ((2 * k_a + 4) if self.audit_padded else 0)
-        self._results = torch.zeros(8 + 2 * B + 5 * k_a + 1 + self._audit_extra + 2 * n_mg, dtype=f32, device=dev)
+        self._results = torch.zeros(8 + 2 * B + 5 * k_a + 1 + self._audit_extra + 2 * n_mg + 1, dtype=f32, device=dev)
+        # (the status word of the engine's own launch table is the last word of it)
+        self._status_inside = own_ops and hasattr(ops, "status")
+        if self._status_inside:
+            ops.status = self._results[-1:].view(torch.int32)
         self.loss_tok = e(M)
         # [0]=sum loss, [1]=aux load, [2]=aux depth, [3]=sumsq, [4]=clip, [5]=1.0 when the step was dropped (non-finite)
         self.scalars = self._results[0:8]
         self.loss_per_sample = self._results[8:8 + B]
-        self._metric_sums = self._results[8 + 2 * B + 5 * k_a + 1 + self._audit_extra:].view(n_mg, 2)
-        self.row_weight = torch.full((B,), 1.0 / (B * S * self.loss_div), dtype=f32, device=dev)
+        self._metrics_at = 8 + 2 * B + 5 * k_a + 1 + self._audit_extra
+        self._metric_sums = self._results[self._metrics_at:self._metrics_at + 2 * n_mg].view(n_mg, 2)
+        self.row_weight = self.inputs.dev["row_weight"].fill_(1.0 / (B * S * self.loss_div))
         # backward temporaries
         self.tmp = _Temps(M, cfg, dev)
         # Weight-gradient launches of the hot pass run on their own stream beside the data-gradient chain (they fill the
@@ -554,7 +602,9 @@ class TrainEngine:
             ops.cast_bf16(self.params["shortlist_head.cluster_router.weight"], self.cluster_w16)
             self.cluster_logits = e(M, oc.num_clusters)
             self.top_clusters = e(M, self.sl_tc, dtype=i32)
-            self.random_negs = torch.zeros(M, max(oc.random_negatives, 1), dtype=i32, device=dev)
+            self.random_negs = self.inputs.dev["negatives"] if oc.random_negatives else torch.zeros(M, 1, dtype=i32, device=dev)
+            self._negatives = torch.zeros(M, oc.random_negatives, dtype=i32)      # drawn ahead for the step `_negatives_seed`
+            self._negatives_seed: int | None = None
             self.shortlist_ids = e(M, oc.shortlist_max_tokens, dtype=i32)
             self.shortlist_dups = e(M, dtype=i32)
         self.audit = None
@@ -564,7 +614,7 @@ class TrainEngine:
         self._side_stream = torch.cuda.Stream(device=dev, priority=-1) if (self.audit_k and dev.type == "cuda") else None
         if self._side_stream is not None and hasattr(ops, "gemm_max_ctas"):
             ops.gemm_max_ctas = max(ops.sm_count - int(os.environ.get("RTE_SIDE_SMS", "8")), 1)
-        self._param_stream = torch.cuda.Stream(device=dev) if (self.audit_k and dev.type == "cuda") else None
+        self._param_stream = torch.cuda.Stream(device=dev) if ((self.audit_k or self.exact) and dev.type == "cuda") else None
         self._merge_stream = torch.cuda.Stream(device=dev) if (self.audit_k and dev.type == "cuda") else None
         self.exact_core = None
         if self.exact:
@@ -604,6 +654,8 @@ class TrainEngine:
             self.audit.exact_loss = self._results[r0 + 4 * k_a:r0 + 5 * k_a]
             self.audit.kl_sum = self._results[r0 + 5 * k_a:r0 + 5 * k_a + 1]
             self.audit.align = self._results[r0 + 5 * k_a + 1:r0 + 13 * k_a + 1].view(k_a, 8)
+            if self._own_subset:
+                self.audit.idx = self.audit.idx_scatter = self.inputs.dev["idx"]
             if self.audit_padded:
                 x0 = r0 + 13 * k_a + 1
                 self.audit.sampler_block = self._results[x0:x0 + 2 * k_a + 4]       # the three views below, contiguous
@@ -622,6 +674,7 @@ class TrainEngine:
         self._slot_next = 0
         self._pending: list[dict[str, Any]] = []
         self._launches_per_step: int | None = None
+        self._lr_groups_present: set[str] | None = None
 
     # ------------------------------------------------------------------ data-parallel gradient exchange
     def _grad_completion_order(self) -> list[str]:
@@ -945,7 +998,7 @@ class TrainEngine:
     # ------------------------------------------------------------------ forward + backward
     def _forward_backward_exact(self, forward_only: bool = False) -> None:
         """`recursive_exact`: embed -> prelude -> router -> t_max banked passes for every sample -> coda -> logits ->
-        cross entropy (models.py:202-228, 416-512), then the same chain backwards; one stream."""
+        cross entropy (models.py:202-228, 416-512), then the same chain backwards, weight gradients on their own stream."""
         o, cfg, p, g, tr, a = self.ops, self.cfg, self.params, self.grads, self.tr, self.exact_core
         M, d, B, S = self.M, cfg.d_model, self.B, self.S
         tokens = self.tokens.view(-1)
@@ -984,9 +1037,16 @@ class TrainEngine:
                              mean_prob=self._global_mean_prob())
         g16 = self.grad16
         o.cast_bf16(dcur, g16[0])
+        # (weight gradients stay on the parameter-gradient stream throughout: `a` has put the coda's and core's there)
+        ps = self._param_stream if hasattr(o, "param_stream") else None
+        if ps is not None:
+            o.param_stream = ps
         for j, blk in enumerate(reversed(self.prelude)):
             self._block_bwd(blk, dcur, g16[j], dalt, g16[j + 1], self.dxc, tmp=self.block_tmps[j], mark_ready=False)
             dcur, dalt = dalt, dcur
+        if ps is not None:
+            o.param_stream = None
+            torch.cuda.current_stream(self.device).wait_stream(ps)       # (the embedding gradient starts from the logits product's share)
         o.embed_bwd(tokens, dcur, g["embed.weight"], self.embed_accum)
         self._grad_ready(*self.trainable)
         self._finish_backward()
@@ -1027,7 +1087,8 @@ class TrainEngine:
                          hid=cfg.router_hidden_dim, R=cfg.recipe_count, K=len(cfg.depth_choices), T=cfg.t_max,
                          fixed_recipe=tr.fixed_recipe, fixed_depth_id=fixed_depth_id)
             self._router_early = None
-            if not tr.disable_router_aux and self._misc_param_stream is not None and self._hot_param_stream is not None:
+            if (not tr.disable_router_aux and not forward_only and self._misc_param_stream is not None
+                    and self._hot_param_stream is not None):
                 # The auxiliary losses' backward needs no upstream gradient: all of it except the add into d h0 runs
                 # here, on the parameter-gradient stream, beside the rest of the forward pass.
                 ms = self._misc_param_stream
@@ -1330,19 +1391,51 @@ class TrainEngine:
             o.fill_(self.accum_flat, 0.0)
 
     # ------------------------------------------------------------------ public API
-    def _load_batch(self, batch) -> None:
+    def _check_batch(self, batch):
         tokens, targets = batch
         if tuple(tokens.shape) != (self.B, self.S) or tuple(targets.shape) != (self.B, self.S):
             raise ValueError(f"batch must be [{self.B}, {self.S}] int64 token ids")
-        self.tokens.copy_(tokens, non_blocking=True)
-        self.targets.copy_(targets, non_blocking=True)
+        return tokens, targets
+
+    def _load_batch(self, batch, negatives_seed: int | None = None) -> None:
+        """Queues the copy of a step's inputs: the batch, the audited subset with its loss weights, the random negatives.
+        Host tensors are copied into the pinned image first, so the batch may be reused as soon as this returns."""
+        tokens, targets = self._check_batch(batch)
+        inp = self.inputs
+        i = inp.image()
+        host, on_host = inp.host[i], not (tokens.is_cuda or targets.is_cuda)
+        if on_host:
+            host["tokens"].copy_(tokens)
+            host["targets"].copy_(targets)
         if self.audit is not None:
-            self.audit.choose(self.tr.seed + 10_000 + self.global_step)
-        if self.shortlist and self.oc.random_negatives > 0:
+            self.audit.choose(self.tr.seed + 10_000 + self.global_step, host)
+        negatives = self.shortlist and self.oc.random_negatives > 0
+        if negatives:
             # the reference draws them with a generator seeded by seed + step (output.py:86-94, training.py:1364)
-            gen = torch.Generator().manual_seed(self.tr.seed + self.global_step)
-            rn = torch.randint(0, self.cfg.vocab_size, (self.B, self.S, self.oc.random_negatives), generator=gen)
-            self.random_negs.copy_(rn.view(self.M, -1).to(torch.int32), non_blocking=True)
+            seed = self.tr.seed + self.global_step if negatives_seed is None else negatives_seed
+            if self._negatives_seed != seed:
+                self._draw_negatives(seed)
+            host["negatives"].copy_(self._negatives)
+        first = "idx" if (self._own_subset and self.audit is not None) else "tokens"
+        if on_host:
+            inp.send(i, first)
+        else:
+            if first == "idx":
+                inp.send(i, "idx", "tokens")
+            if negatives:
+                inp.send(i, "negatives")
+            self.tokens.copy_(tokens, non_blocking=True)
+            self.targets.copy_(targets, non_blocking=True)
+
+    def _draw_negatives(self, seed: int) -> None:
+        n = self._negatives.numel()
+        lib = getattr(self.ops, "lib", None)
+        if lib is not None and self.cfg.vocab_size < 2 ** 28:
+            A.check(lib.rte_host_randint(seed, n, self.cfg.vocab_size, self._negatives.data_ptr()), "rte_host_randint")
+        else:
+            gen = torch.Generator().manual_seed(seed)
+            self._negatives.view(-1).copy_(torch.randint(0, self.cfg.vocab_size, (n,), generator=gen))
+        self._negatives_seed = seed
 
     def _run_step_kernels(self, optimizer: bool, accumulate: bool = False) -> None:
         """`optimizer`: forward + backward + optimiser (the last micro-batch of an accumulation cycle, or every call
@@ -1412,27 +1505,41 @@ class TrainEngine:
         if self._pending:
             raise RuntimeError("steps are in flight: collect() them before evaluating")
         audit, self.audit = self.audit, None              # evaluation never replays audited samples
-        total, n = 0.0, 0
+        sums, n = [], 0
+        cuda = self.device.type == "cuda"
+        sent = [None] * 3                                  # per pinned image: the copies that last read it
         try:
             for batch in batches:
-                tokens, targets = batch
-                if tuple(tokens.shape) != (self.B, self.S):
-                    raise ValueError(f"batch must be [{self.B}, {self.S}] int64 token ids")
-                self.tokens.copy_(tokens, non_blocking=True)
-                self.targets.copy_(targets, non_blocking=True)
-                if self.shortlist and self.oc.random_negatives > 0:
-                    gen = torch.Generator().manual_seed(self.tr.seed)       # `forward_macro(..., seed=0)` + config seed
-                    rn = torch.randint(0, self.cfg.vocab_size, (self.B, self.S, self.oc.random_negatives), generator=gen)
-                    self.random_negs.copy_(rn.view(self.M, -1).to(torch.int32), non_blocking=True)
-                self._forward_backward(forward_only=True)
-                total += float(self.loss_per_sample.sum())
+                i = self.inputs.next
+                if sent[i] is not None:
+                    sent[i].synchronize()
+                # (`forward_macro(..., seed=0)` + config seed: the same negatives for every batch)
+                self._load_batch(batch, negatives_seed=self.tr.seed)
+                if cuda:
+                    sent[i] = torch.cuda.Event()
+                    sent[i].record(torch.cuda.current_stream(self.device))
+                self._run_forward()
+                sums.append(self.loss_per_sample.sum())    # read once, after the last batch
                 n += self.B
         finally:
             self.audit = audit
         if hasattr(self.ops, "check_status"):
             self.ops.check_status()
-        mean = total / max(n, 1)
+        mean = sum(torch.stack(sums).tolist()) / n if sums else 0.0
         return {"mode": self.tr.mode, "eval_loss_per_sample": mean, "eval_nll_per_token": mean / self.S, "samples": n}
+
+    def _run_forward(self) -> None:
+        """The forward pass of the batch loaded last, as a captured graph (the launches of one forward take the host
+        longer than the device)."""
+        if not self.use_cuda_graph:
+            return self._forward_backward(forward_only=True)
+        if self._graphs.get("forward") is None:
+            torch.cuda.synchronize(self.device)
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                self._forward_backward(forward_only=True)
+            self._graphs["forward"] = graph
+        self._graphs["forward"].replay()
 
     def _host_slot(self, i: int) -> dict[str, Any]:
         """Pinned host buffers for the results of one in-flight step (two slots alternate)."""
@@ -1444,12 +1551,12 @@ class TrainEngine:
             h = torch.empty(self._results.shape, dtype=torch.float32, pin_memory=cuda)
             r0 = 8 + 2 * B
             self._host_slots[i] = {
-                "flat": h, "status": torch.zeros(1, dtype=torch.int32, pin_memory=cuda),
+                "flat": h, "status": h[-1:].view(torch.int32) if self._status_inside else torch.zeros(1, dtype=torch.int32, pin_memory=cuda),
                 "event": torch.cuda.Event() if cuda else None,
                 "scalars": h[0:8], "loss_per_sample": h[8:8 + B], "recipe_id": h[8 + B:8 + 2 * B].view(torch.int32),
                 "terms": h[r0:r0 + 4 * k_a].view(k_a, 4), "exact_loss": h[r0 + 4 * k_a:r0 + 5 * k_a],
                 "kl_sum": h[r0 + 5 * k_a:r0 + 5 * k_a + 1],
-                "metric_sums": h[r0 + 5 * k_a + 1 + self._audit_extra:].view(len(METRIC_GROUPS), 2)}
+                "metric_sums": h[self._metrics_at:self._metrics_at + 2 * len(METRIC_GROUPS)].view(len(METRIC_GROUPS), 2)}
             if k_a:
                 self._host_slots[i]["align"] = h[r0 + 5 * k_a + 1:r0 + 13 * k_a + 1].view(k_a, 8)
             if self.audit_padded:
@@ -1464,7 +1571,7 @@ class TrainEngine:
         slot = self._host_slot(self._slot_next)
         self._slot_next ^= 1
         slot["flat"].copy_(self._results, non_blocking=True)
-        if hasattr(self.ops, "status"):
+        if hasattr(self.ops, "status") and not self._status_inside:
             slot["status"].copy_(self.ops.status, non_blocking=True)
         if slot["event"] is not None:
             slot["event"].record(torch.cuda.current_stream(self.device))
@@ -1476,25 +1583,26 @@ class TrainEngine:
             slot["event"].synchronize()
         if int(slot["status"][0]) != 0:
             self.ops.check_status()                          # raises with the decoded device status
+        slot["vals"] = slot["flat"].tolist()                 # (numbers the host reads one by one: a tensor index costs 1 us)
         self._host = slot
         return slot
 
     def _assemble_loss(self, host: dict[str, Any] | None = None) -> float:
         if host is None:
             host = self._wait_fetch(self._queue_fetch())
-        vals = host["scalars"]
-        loss = float(vals[0]) / (self.B * self.S)          # this rank's shard
+        vals = host["vals"]
+        loss = vals[0] / (self.B * self.S)          # this rank's shard
         if self.audit is not None:
             terms = self.audit.loss_terms(host["loss_per_sample"], host, host["chosen"])
             loss += terms["correction"] / (self.B * self.S) + sum(terms["aux"].values())
             self.last_audit = terms
         if getattr(self, "cons_pairs", None):
-            cons = self.tr.lambda_cons * float(vals[6]) / (len(self.cons_pairs) * self.M * self.cfg.d_model)
+            cons = self.tr.lambda_cons * vals[6] / (len(self.cons_pairs) * self.M * self.cfg.d_model)
             loss += cons
             self.last_consistency = cons
         if not self.dense and not self.tr.disable_router_aux:
-            cover = float(torch.relu(self.tr.coverage_min - self.usage_ema).square().sum()) * self.tr.lambda_cover
-            loss += (float(vals[1]) + float(vals[2])) * self.loss_div + cover
+            cover = sum(max(self.tr.coverage_min - u, 0.0) ** 2 for u in self.usage_ema.tolist()) * self.tr.lambda_cover
+            loss += (vals[1] + vals[2]) * self.loss_div + cover
         return loss
 
     MAX_IN_FLIGHT = 2
@@ -1529,16 +1637,20 @@ class TrainEngine:
             # host work for the NEXT step (the seeded permutation of its audited subset) while the device runs this one
             # (under the count schedule the next step's count is only known once this step has been collected)
             self.audit.prepare(self.tr.seed + 10_000 + self.global_step)
+        if self.shortlist and self.oc.random_negatives > 0 and self._negatives_seed != self.tr.seed + self.global_step:
+            self._draw_negatives(self.tr.seed + self.global_step)          # likewise
 
     def _grad_metrics(self, host: dict[str, Any]) -> dict[str, float]:
         """training.py:386-443 from the per-group sums the AdamW launch left in the results buffer: gradient norm (after
         clipping) and lr * |g| / |p| per optimizer group, plus the core's per-pass FiLM / scale sub-groups."""
-        sums = host["metric_sums"]
-        gsq = [float(sums[i, 0]) for i in range(len(METRIC_GROUPS))]
-        psq = [float(sums[i, 1]) + self._static_param_sq[i] for i in range(len(METRIC_GROUPS))]
+        at = self._metrics_at
+        gsq = host["vals"][at:at + 2 * len(METRIC_GROUPS):2]
+        psq = [v + q for v, q in zip(host["vals"][at + 1:at + 2 * len(METRIC_GROUPS):2], self._static_param_sq)]
         core, film, scale = (METRIC_GROUPS.index(x) for x in ("core", "pass_film", "pass_scale"))
         out: dict[str, float] = {}
-        present = {lr_group_of(n, self.cfg.topology) for n in self.params if not n.startswith("shortlist_head.")}
+        if self._lr_groups_present is None:
+            self._lr_groups_present = {lr_group_of(n, self.cfg.topology) for n in self.params if not n.startswith("shortlist_head.")}
+        present = self._lr_groups_present
         for i, name in enumerate(LR_GROUPS):
             if name not in present:
                 continue
@@ -1560,7 +1672,8 @@ class TrainEngine:
         host = self._wait_fetch(self._pending.pop(0))
         loss = self._assemble_loss(host)
         metrics: dict[str, Any] = {"mode": self.tr.mode, "loss": loss, "lr": host["lr"][LR_GROUPS[0] if not self.dense else "dense"]}
-        skipped = float(host["scalars"][5]) != 0.0
+        vals = host["vals"]
+        skipped = vals[5] != 0.0
         stepped = bool(host["stepping"]) and not skipped
         metrics["did_optimizer_step"] = stepped
         if skipped:
@@ -1583,9 +1696,9 @@ class TrainEngine:
                            audit_requested_probability=la.get("p_requested", self.audit.p_inc),
                            audit_candidate_count=float(la.get("candidates", audited)),
                            macro_distill_loss=sum(la["aux"].values()),
-                           hot_lm_loss=float(host["scalars"][0]) / (B * S),
-                           corrected_lm_loss=(float(host["scalars"][0]) + la["correction"]) / (B * S),
-                           corrected_metric_loss=(float(host["scalars"][0]) + la["correction_metric"]) / (B * S))
+                           hot_lm_loss=vals[0] / (B * S),
+                           corrected_lm_loss=(vals[0] + la["correction"]) / (B * S),
+                           corrected_metric_loss=(vals[0] + la["correction_metric"]) / (B * S))
             metrics.update({f"macro_{k}_loss": v for k, v in la["aux"].items()})
             metrics.update(la.get("alignment", {}))
             metrics.update(la.get("residual", {}))
@@ -1595,16 +1708,19 @@ class TrainEngine:
                     self.audit.update_schedule(metrics)                  # audit.py:365: decides the next step's count
                 metrics["audit_schedule_next_count"] = float(self.audit.count)
             if audited:
-                metrics["exact_eval_nll"] = float(la["exact"].mean()) / S
+                metrics["exact_eval_nll"] = sum(la["exact"]) / len(la["exact"]) / S
         if getattr(self, "cons_pairs", None):
             metrics["macro_consistency_loss"] = self.last_consistency
         if not self.dense:
-            ids = host["recipe_id"].long()
+            ids = host["recipe_id"].tolist()
             if getattr(self, "exact_schedule", None) is not None:        # the schedule is what ran (models.py:480-497)
-                ids = torch.tensor(self.exact_schedule, dtype=torch.long).repeat(self.B)
-            counts = torch.bincount(ids, minlength=self.cfg.recipe_count).float()
-            self.usage_ema.mul_(self.tr.coverage_beta).add_(counts / counts.sum().clamp_min(1.0), alpha=1.0 - self.tr.coverage_beta)
-            metrics["unique_recipes_per_batch"] = int(ids.unique().numel())
+                ids = list(self.exact_schedule) * self.B
+            counts = [0] * self.cfg.recipe_count
+            for r in ids:
+                counts[r] += 1
+            share = torch.tensor(counts, dtype=torch.float32).div_(max(len(ids), 1))
+            self.usage_ema.mul_(self.tr.coverage_beta).add_(share, alpha=1.0 - self.tr.coverage_beta)
+            metrics["unique_recipes_per_batch"] = sum(1 for c in counts if c)
             metrics.update(self._budget)
         self.tokens_seen += self.B * self.S
         metrics["tokens_seen"] = self.tokens_seen
