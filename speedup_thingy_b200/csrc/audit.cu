@@ -21,24 +21,44 @@ inline int grid_for(long long n, int block, int cap = 148 * 8) {
   return (int)g;
 }
 
+// The replay's and the exact modes' row passes.  They move a few MB at most, so what bounds them is latency: every thread
+// takes one 16- or 32-byte group, its row comes from blockIdx.y or one 32-bit division per group (a 64-bit division per
+// element, as before, is most of such a kernel: scaled_residual_bwd over 1050 x 384 took 19.7 us).
+inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 __global__ void gather_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ idx, uint4* __restrict__ dst,
-                                   int n, long long row16) {
+                                   int n, long long row16) {                    // long rows: blockIdx.y = row
   rte::after_previous_grid();
-  const long long total = (long long)n * row16;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int r = int(i / row16);
-    dst[i] = src[(long long)idx[r] * row16 + (i % row16)];
+  const uint4* from = src + (long long)idx[blockIdx.y] * row16;
+  uint4* to = dst + (long long)blockIdx.y * row16;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < row16; i += (long long)gridDim.x * blockDim.x) to[i] = from[i];
+}
+__global__ void gather_short_rows_kernel(const uint4* __restrict__ src, const int32_t* __restrict__ idx, uint4* __restrict__ dst,
+                                         unsigned total, unsigned row16) {
+  rte::after_previous_grid();
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const unsigned r = i / row16;
+    dst[i] = src[(size_t)idx[r] * row16 + (i - r * row16)];
   }
 }
 
 __global__ void scatter_add_rows_kernel(float* __restrict__ dst, const int32_t* __restrict__ idx, const float* __restrict__ src,
-                                        int n, long long row) {
+                                        int n, long long row, int wide) {
   rte::after_previous_grid();
-  const long long total = (long long)n * row;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int r = int(i / row);
-    if (idx[r] < 0) continue;                       // unused slot of a capacity-padded subset
-    dst[(long long)idx[r] * row + (i % row)] += src[i];
+  const int r = idx[blockIdx.y];
+  if (r < 0) return;                                // unused slot of a capacity-padded subset
+  float* to = dst + (long long)r * row;
+  const float* from = src + (long long)blockIdx.y * row;
+  const long long at = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  if (wide) {
+    for (long long i = at; i < row / 4; i += step) {
+      float4 a = reinterpret_cast<float4*>(to)[i];
+      const float4 b = reinterpret_cast<const float4*>(from)[i];
+      a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+      reinterpret_cast<float4*>(to)[i] = a;
+    }
+  } else {
+    for (long long i = at; i < row; i += step) to[i] += from[i];
   }
 }
 
@@ -53,6 +73,73 @@ __global__ void audit_route_kernel(const int32_t* __restrict__ by_pass, const in
   active[i] = depth[b] > t ? 1 : 0;
 }
 
+// Eight columns of one row per thread: f(row, first column, offset of the group in a [rows, cols] matrix).
+template <typename Fn>
+__device__ __forceinline__ void for_groups8(int rows, int cols, Fn f) {
+  const unsigned c8 = (unsigned)cols / 8, total = (unsigned)rows * c8;
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const unsigned r = i / c8, c = (i - r * c8) * 8;
+    f((int)r, (int)c, (size_t)i * 8);
+  }
+}
+struct Row8 { float v[8]; };
+__device__ __forceinline__ Row8 load8(const __nv_bfloat16* p) {
+  const uint4 w = *reinterpret_cast<const uint4*>(p);
+  const float2 a = rte::unpack_bf16x2(w.x), b = rte::unpack_bf16x2(w.y), c = rte::unpack_bf16x2(w.z), d = rte::unpack_bf16x2(w.w);
+  return {{a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y}};
+}
+__device__ __forceinline__ Row8 load8(const float* p) {
+  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+  return {{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}};
+}
+__device__ __forceinline__ void store8(__nv_bfloat16* p, const Row8& x) {
+  *reinterpret_cast<uint4*>(p) = make_uint4(rte::pack_bf16x2(x.v[0], x.v[1]), rte::pack_bf16x2(x.v[2], x.v[3]),
+                                            rte::pack_bf16x2(x.v[4], x.v[5]), rte::pack_bf16x2(x.v[6], x.v[7]));
+}
+
+__global__ void colmask_mul8_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ rid,
+                                    const float* __restrict__ table, int S, __nv_bfloat16* __restrict__ out, int rows, int cols) {
+  rte::after_previous_grid();
+  for_groups8(rows, cols, [&](int r, int c, size_t at) {
+    Row8 v = load8(x + at);
+    const Row8 m = load8(table + (size_t)rid[r / S] * cols + c);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v.v[j] *= m.v[j];
+    store8(out + at, v);
+  });
+}
+__global__ void swiglu_masked_fwd8_kernel(const __nv_bfloat16* __restrict__ ug, const int32_t* __restrict__ rid,
+                                          const float* __restrict__ table, int S, __nv_bfloat16* __restrict__ z, int rows, int F) {
+  rte::after_previous_grid();
+  for_groups8(rows, F, [&](int r, int j0, size_t at) {
+    const Row8 up = load8(ug + (size_t)r * 2 * F + j0), g = load8(ug + (size_t)r * 2 * F + F + j0);
+    const Row8 m = load8(table + (size_t)rid[r / S] * F + j0);
+    Row8 o;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) o.v[j] = up.v[j] * rte::silu_f(g.v[j]) * m.v[j];
+    store8(z + at, o);
+  });
+}
+__global__ void swiglu_masked_bwd8_kernel(const __nv_bfloat16* __restrict__ ug, const __nv_bfloat16* __restrict__ dz,
+                                          const int32_t* __restrict__ rid, const float* __restrict__ table, int S,
+                                          __nv_bfloat16* __restrict__ dug, int rows, int F) {
+  rte::after_previous_grid();
+  for_groups8(rows, F, [&](int r, int j0, size_t at) {
+    const size_t o = (size_t)r * 2 * F + j0;
+    const Row8 up = load8(ug + o), g = load8(ug + o + F), m = load8(table + (size_t)rid[r / S] * F + j0), dzv = load8(dz + at);
+    Row8 du, dg;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float d = dzv.v[j] * m.v[j], sg = rte::sigmoid_f(g.v[j]);
+      du.v[j] = d * g.v[j] * sg;
+      dg.v[j] = d * up.v[j] * sg * (1.f + g.v[j] * (1.f - sg));
+    }
+    store8(dug + o, du);
+    store8(dug + o + F, dg);
+  });
+}
+
+// one element per thread: columns that are no multiple of eight, or rows off the 16-byte grid
 __global__ void colmask_mul_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ rid,
                                    const float* __restrict__ table, int S, __nv_bfloat16* __restrict__ out, int rows, int cols) {
   rte::after_previous_grid();
@@ -89,40 +176,85 @@ __global__ void swiglu_masked_bwd_kernel(const __nv_bfloat16* __restrict__ ug, c
   }
 }
 
-__global__ void scaled_residual_fwd_kernel(const float* __restrict__ base, const float* __restrict__ branch,
-                                           const float* __restrict__ scale, const int32_t* __restrict__ active,
-                                           const float* __restrict__ pass, float* __restrict__ out, int n, long long se) {
+// V = 4: sample_elems is a multiple of four and every pointer starts on 16 bytes; else V = 1.
+template <int V> struct Group;
+template <> struct Group<1> { float v[1]; };
+template <> struct __align__(16) Group<4> { float v[4]; };
+template <int V>
+__device__ __forceinline__ Group<V> get(const float* p, unsigned i) { return reinterpret_cast<const Group<V>*>(p)[i]; }
+template <int V>
+__device__ __forceinline__ void put(float* p, unsigned i, const Group<V>& g) { reinterpret_cast<Group<V>*>(p)[i] = g; }
+
+template <int V>
+__global__ void __launch_bounds__(NTHR)
+scaled_residual_fwd_kernel(const float* __restrict__ base, const float* __restrict__ branch,
+                           const float* __restrict__ scale, const int32_t* __restrict__ active,
+                           const float* __restrict__ pass, float* __restrict__ out, unsigned groups, unsigned per_sample) {
   rte::after_previous_grid();
   const float s = *scale;
-  const long long total = (long long)n * se;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const bool on = active == nullptr || active[i / se] != 0;
-    out[i] = on ? base[i] + s * branch[i] : pass[i];
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < groups; i += gridDim.x * blockDim.x) {
+    const bool on = active == nullptr || active[i / per_sample] != 0;
+    Group<V> o;
+    if (on) {
+      const Group<V> a = get<V>(base, i), b = get<V>(branch, i);
+#pragma unroll
+      for (int j = 0; j < V; ++j) o.v[j] = a.v[j] + s * b.v[j];
+    } else {
+      o = get<V>(pass, i);
+    }
+    put<V>(out, i, o);
   }
 }
 
+template <int V>
 __global__ void __launch_bounds__(NTHR)
 scaled_residual_bwd_kernel(const float* __restrict__ dout, const float* __restrict__ branch, const float* __restrict__ scale,
                            const int32_t* __restrict__ active, float* __restrict__ dbase, __nv_bfloat16* __restrict__ db16,
                            float* __restrict__ db32, float* __restrict__ dpass, float* __restrict__ dscale_part,
-                           const int32_t* __restrict__ frozen_active, const float* __restrict__ frozen_src, int n,
-                           long long se) {
+                           const int32_t* __restrict__ frozen_active, const float* __restrict__ frozen_src, unsigned groups,
+                           unsigned per_sample) {
   rte::after_previous_grid();
   __shared__ float red[32];
   const float s = *scale;
-  const long long total = (long long)n * se;
   float acc = 0.f;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const bool on = active == nullptr || active[i / se] != 0;
-    const float g = dout[i];
-    if (on) acc += g * branch[i];
-    if (dpass && !on) dpass[i] += g;
-    if (db16) db16[i] = __float2bfloat16_rn(on ? s * g : 0.f);
-    if (db32 && on) db32[i] += s * g;
+#pragma unroll 2
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < groups; i += gridDim.x * blockDim.x) {
+    const unsigned sample = i / per_sample;
+    const bool on = active == nullptr || active[sample] != 0;
+    const Group<V> g = get<V>(dout, i), br = get<V>(branch, i);
+#pragma unroll
+    for (int j = 0; j < V; ++j)
+      if (on) acc += g.v[j] * br.v[j];
+    if (dpass && !on) {
+      Group<V> p = get<V>(dpass, i);
+#pragma unroll
+      for (int j = 0; j < V; ++j) p.v[j] += g.v[j];
+      put<V>(dpass, i, p);
+    }
+    if (db16) {
+      if constexpr (V == 4) {
+        reinterpret_cast<uint2*>(db16)[i] = on ? make_uint2(rte::pack_bf16x2(s * g.v[0], s * g.v[1]), rte::pack_bf16x2(s * g.v[2], s * g.v[3]))
+                                               : make_uint2(0u, 0u);
+      } else {
+        db16[i] = __float2bfloat16_rn(on ? s * g.v[0] : 0.f);
+      }
+    }
+    if (db32 && on) {
+      Group<V> p = get<V>(db32, i);
+#pragma unroll
+      for (int j = 0; j < V; ++j) p.v[j] += s * g.v[j];
+      put<V>(db32, i, p);
+    }
     if (dbase) {
-      float o = on ? g : 0.f;
-      if (frozen_src && frozen_active[i / se] == 0) o += frozen_src[i];     // samples frozen in this pass: hand-through
-      dbase[i] = o;
+      Group<V> o;
+#pragma unroll
+      for (int j = 0; j < V; ++j) o.v[j] = on ? g.v[j] : 0.f;
+      if (frozen_src && frozen_active[sample] == 0) {      // samples frozen in this pass: hand-through
+        const Group<V> f = get<V>(frozen_src, i);
+#pragma unroll
+        for (int j = 0; j < V; ++j) o.v[j] += f.v[j];
+      }
+      put<V>(dbase, i, o);
     }
   }
   acc = rte::block_sum(acc, red);
@@ -528,7 +660,13 @@ extern "C" int rte_gather_rows(const void* src, const int32_t* idx, void* dst, i
   RTE_CHECK_ARG(src && idx && dst && n > 0 && row_bytes > 0);
   if ((row_bytes % 16) || (reinterpret_cast<uintptr_t>(src) & 15) || (reinterpret_cast<uintptr_t>(dst) & 15)) return RTE_ERR_ALIGNMENT;
   const long long row16 = row_bytes / 16;
-  rte::launch(gather_rows_kernel, grid_for((long long)n * row16, NTHR), NTHR, 0, ST(stream), reinterpret_cast<const uint4*>(src), idx, reinterpret_cast<uint4*>(dst), n, row16);
+  const auto* from = reinterpret_cast<const uint4*>(src);
+  auto* to = reinterpret_cast<uint4*>(dst);
+  if (row16 < NTHR && (long long)n * row16 < (1ll << 32))
+    rte::launch(gather_short_rows_kernel, grid_for((long long)n * row16, NTHR, 148 * 16), NTHR, 0, ST(stream), from, idx, to, (unsigned)(n * row16), (unsigned)row16);
+  else
+    for (int at = 0; at < n; at += 65535)                 // (gridDim.y)
+      rte::launch(gather_rows_kernel, dim3(grid_for(row16, NTHR, 1184), n - at < 65535 ? n - at : 65535), NTHR, 0, ST(stream), from, idx + at, to + at * row16, n, row16);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -536,7 +674,10 @@ extern "C" int rte_gather_rows(const void* src, const int32_t* idx, void* dst, i
 extern "C" int rte_scatter_add_rows_f32(float* dst, const int32_t* idx, const float* src, int32_t n, int64_t row_elems,
                                         rte_stream_t stream) {
   RTE_CHECK_ARG(dst && idx && src && n > 0 && row_elems > 0);
-  rte::launch(scatter_add_rows_kernel, grid_for((long long)n * row_elems, NTHR), NTHR, 0, ST(stream), dst, idx, src, n, row_elems);
+  const int wide = row_elems % 4 == 0 && aligned16(dst) && aligned16(src);
+  for (int at = 0; at < n; at += 65535)
+    rte::launch(scatter_add_rows_kernel, dim3(grid_for(wide ? row_elems / 4 : row_elems, NTHR, 1184), n - at < 65535 ? n - at : 65535), NTHR, 0, ST(stream),
+                dst, idx + at, src + at * row_elems, n, row_elems, wide);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -552,7 +693,9 @@ extern "C" int rte_audit_route(const int32_t* recipe_id_by_pass, const int32_t* 
 extern "C" int rte_colmask_mul_bf16(const void* x, const int32_t* rid, const float* table, int32_t S, void* out, int32_t rows,
                                     int32_t cols, rte_stream_t stream) {
   RTE_CHECK_ARG(x && rid && table && out && S > 0 && rows > 0 && cols > 0);
-  rte::launch(colmask_mul_kernel, grid_for((long long)rows * cols, NTHR), NTHR, 0, ST(stream), reinterpret_cast<const __nv_bfloat16*>(x), rid, table, S, reinterpret_cast<__nv_bfloat16*>(out), rows, cols);
+  const bool wide = cols % 8 == 0 && (long long)rows * cols < (1ll << 33) && aligned16(x) && aligned16(out) && aligned16(table);
+  rte::launch(wide ? colmask_mul8_kernel : colmask_mul_kernel, grid_for((long long)rows * cols / (wide ? 8 : 1), 128), 128, 0, ST(stream),
+              reinterpret_cast<const __nv_bfloat16*>(x), rid, table, S, reinterpret_cast<__nv_bfloat16*>(out), rows, cols);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -560,7 +703,9 @@ extern "C" int rte_colmask_mul_bf16(const void* x, const int32_t* rid, const flo
 extern "C" int rte_swiglu_masked_fwd(const void* ug, const int32_t* rid, const float* table, int32_t S, void* z, int32_t rows,
                                      int32_t F, rte_stream_t stream) {
   RTE_CHECK_ARG(ug && rid && table && z && S > 0 && rows > 0 && F > 0);
-  rte::launch(swiglu_masked_fwd_kernel, grid_for((long long)rows * F, NTHR), NTHR, 0, ST(stream), reinterpret_cast<const __nv_bfloat16*>(ug), rid, table, S, reinterpret_cast<__nv_bfloat16*>(z), rows, F);
+  const bool wide = F % 8 == 0 && (long long)rows * F < (1ll << 33) && aligned16(ug) && aligned16(z) && aligned16(table);
+  rte::launch(wide ? swiglu_masked_fwd8_kernel : swiglu_masked_fwd_kernel, grid_for((long long)rows * F / (wide ? 8 : 1), 128), 128, 0, ST(stream),
+              reinterpret_cast<const __nv_bfloat16*>(ug), rid, table, S, reinterpret_cast<__nv_bfloat16*>(z), rows, F);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -568,8 +713,10 @@ extern "C" int rte_swiglu_masked_fwd(const void* ug, const int32_t* rid, const f
 extern "C" int rte_swiglu_masked_bwd(const void* ug, const void* dz, const int32_t* rid, const float* table, int32_t S,
                                      void* dug, int32_t rows, int32_t F, rte_stream_t stream) {
   RTE_CHECK_ARG(ug && dz && rid && table && dug && S > 0 && rows > 0 && F > 0);
-  rte::launch(swiglu_masked_bwd_kernel, grid_for((long long)rows * F, NTHR), NTHR, 0, ST(stream), reinterpret_cast<const __nv_bfloat16*>(ug), reinterpret_cast<const __nv_bfloat16*>(dz), rid, table, S,
-      reinterpret_cast<__nv_bfloat16*>(dug), rows, F);
+  const bool wide = F % 8 == 0 && (long long)rows * F < (1ll << 33) && aligned16(ug) && aligned16(dz) && aligned16(dug) && aligned16(table);
+  rte::launch(wide ? swiglu_masked_bwd8_kernel : swiglu_masked_bwd_kernel, grid_for((long long)rows * F / (wide ? 8 : 1), 128), 128, 0, ST(stream),
+              reinterpret_cast<const __nv_bfloat16*>(ug), reinterpret_cast<const __nv_bfloat16*>(dz), rid, table, S,
+              reinterpret_cast<__nv_bfloat16*>(dug), rows, F);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -578,8 +725,11 @@ extern "C" int rte_scaled_residual_fwd(const float* base, const float* branch, c
                                        const float* passthrough, float* out, int32_t n, int64_t sample_elems,
                                        rte_stream_t stream) {
   RTE_CHECK_ARG(base && branch && scale && out && n > 0 && sample_elems > 0 && (active == nullptr || passthrough != nullptr));
-  rte::launch(scaled_residual_fwd_kernel, grid_for((long long)n * sample_elems, NTHR), NTHR, 0, ST(stream), base, branch, scale, active,
-                                                                                                 passthrough, out, n, sample_elems);
+  RTE_CHECK_ARG((long long)n * sample_elems < (1ll << 32));
+  const bool wide = sample_elems % 4 == 0 && aligned16(base) && aligned16(branch) && aligned16(out) && aligned16(passthrough);
+  const int v = wide ? 4 : 1;
+  rte::launch(wide ? scaled_residual_fwd_kernel<4> : scaled_residual_fwd_kernel<1>, grid_for((long long)n * sample_elems / v, NTHR), NTHR, 0, ST(stream),
+              base, branch, scale, active, passthrough, out, (unsigned)(n * sample_elems / v), (unsigned)(sample_elems / v));
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -591,15 +741,19 @@ extern "C" int rte_scaled_residual_bwd(const float* dout, const float* branch, c
                                        int64_t sample_elems, rte_stream_t stream) {
   RTE_CHECK_ARG(dout && branch && scale && n > 0 && sample_elems > 0);
   RTE_CHECK_ARG((frozen_active == nullptr) == (frozen_src == nullptr) && (frozen_src == nullptr || dbase != nullptr));
-  int grid = grid_for((long long)n * sample_elems, NTHR, 64);
+  RTE_CHECK_ARG((long long)n * sample_elems < (1ll << 32));
+  const bool wide = sample_elems % 4 == 0 && aligned16(dout) && aligned16(branch) && aligned16(dbase) && aligned16(dbranch_bf16) &&
+                    aligned16(dbranch_f32_accum) && aligned16(dpassthrough) && aligned16(frozen_src);
+  const int v = wide ? 4 : 1;
+  int grid = grid_for((long long)n * sample_elems / v, NTHR, 592);
   if (dscale_partial) {
     RTE_CHECK_ARG(max_partials >= 1);
     if (grid > max_partials) grid = max_partials;
   }
   if (n_partials) *n_partials = grid;
-  rte::launch(scaled_residual_bwd_kernel, grid, NTHR, 0, ST(stream), dout, branch, scale, active, dbase,
-      reinterpret_cast<__nv_bfloat16*>(dbranch_bf16), dbranch_f32_accum, dpassthrough, dscale_partial, frozen_active,
-      frozen_src, n, sample_elems);
+  rte::launch(wide ? scaled_residual_bwd_kernel<4> : scaled_residual_bwd_kernel<1>, grid, NTHR, 0, ST(stream), dout, branch, scale, active, dbase,
+              reinterpret_cast<__nv_bfloat16*>(dbranch_bf16), dbranch_f32_accum, dpassthrough, dscale_partial, frozen_active,
+              frozen_src, (unsigned)(n * sample_elems / v), (unsigned)(sample_elems / v));
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }

@@ -1031,3 +1031,35 @@ def test_alignment_sums_match_their_definition(ops, L):
     torch.cuda.synchronize()
     assert torch.allclose(got.cpu(), want, rtol=1e-4, atol=1e-2)
     assert torch.equal(got[:, 7].cpu(), torch.full((n,), 9.0))
+
+
+@pytest.mark.parametrize("n,S,cols", [(3, 5, 64), (2, 3, 20), (300, 7, 8)])       # groups of eight columns | one column at a time | many samples
+def test_row_passes_of_the_replay(ops, n, S, cols):
+    """Recipe-masked SwiGLU, column mask, scaled residual, row gather and scatter, wide and narrow, against the emulation."""
+    from tests.emul_ops import EmulOps
+    emu, g, rows = EmulOps(), torch.Generator().manual_seed(cols), n * S
+    table, rid = torch.rand(4, cols, generator=g), torch.randint(0, 4, (n,), generator=g).to(torch.int32)
+    ug, dz = _bf(torch.randn(rows, 2 * cols, generator=g)), _bf(torch.randn(rows, cols, generator=g))
+    base, branch, dout, frozen = (torch.randn(rows, cols, generator=g) for _ in range(4))
+    scale, active = torch.tensor([0.7]), (torch.arange(n) % 3 != 1).to(torch.int32)
+    src16, idx = torch.randint(0, 1000, (n, 8), generator=g), torch.randint(0, n, (n,), generator=g).to(torch.int32)
+    perm = torch.randperm(n, generator=g).to(torch.int32)
+    perm[0] = -1
+
+    def run(o, dev):
+        t = [x.to(dev) for x in (table, rid, ug, dz, base, branch, dout, frozen, scale, active, src16, idx, perm)]
+        table_, rid_, ug_, dz_, base_, branch_, dout_, frozen_, scale_, active_, src_, idx_, perm_ = t
+        z, dug, masked, d16 = (torch.zeros(rows, c, dtype=torch.bfloat16, device=dev) for c in (cols, 2 * cols, cols, cols))
+        out, dbase, acc, scat = (torch.zeros(rows, cols, device=dev) for _ in range(4))
+        part, got = torch.zeros(296, device=dev), torch.zeros_like(src_)
+        o.swiglu_masked_fwd(ug_, rid_, table_, S, z, rows, cols)
+        o.swiglu_masked_bwd(ug_, dz_, rid_, table_, S, dug, rows, cols)
+        o.colmask_mul(dz_, rid_, table_, S, masked, rows, cols)
+        o.scaled_residual_fwd(base_, branch_, scale_, active_, frozen_, out, n, S * cols)
+        o.scaled_residual_bwd(dout_, branch_, scale_, active_, dbase, d16, acc, None, part, n, S * cols, frozen_active=active_, frozen_src=frozen_)
+        o.gather_rows(src_, idx_, got, n, 64)
+        o.scatter_add_rows(scat, perm_, base_, n, S * cols)
+        return [x.detach().float().cpu() for x in (z, dug, masked, out, dbase, d16, acc, part.sum(), got, scat)]
+
+    for a, b in zip(run(ops, DEV), run(emu, "cpu")):
+        assert (a - b).abs().max() <= 1e-2 * max(b.abs().max().item(), 1e-3)
