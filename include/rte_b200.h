@@ -230,6 +230,9 @@ int rte_attn_bwd_masked(const void* qkv, int32_t ld_qkv, int32_t sec, const void
 int rte_ce_fwd_bwd(const void* logits, int32_t ldl, const int64_t* targets, const float* row_weight,
                    int32_t S, float* loss_tok, void* dlogits, int32_t rows, int32_t V, int32_t* status,
                    rte_stream_t stream);
+/* The same over f32 logits and gradients.                                                                              */
+int rte_ce_fwd_bwd_f32(const float* logits, int32_t ldl, const int64_t* targets, const float* row_weight, int32_t S,
+                       float* loss_tok, float* dlogits, int32_t rows, int32_t V, int32_t* status, rte_stream_t stream);
 /* out[b] = sum_s in[b*S + s]  (per-sample loss sums, models.py:75) */
 int rte_segment_sum(const float* in, float* out, int32_t n_seg, int32_t seg_len, rte_stream_t stream);
 
