@@ -129,6 +129,23 @@ int rte_gemm_bf16_small(const rte_gemm_args* args, rte_stream_t stream);
 int rte_reduce_splits(const float* ws, int32_t splits, int64_t split_stride, int64_t n, float* out,
                       int32_t accumulate, rte_stream_t stream);
 
+/* ---------------------------------------------------- operator table passes (kernels/reference.py:9-28,40-41)
+ * rte_cast_many_f32_bf16: up to four tensors in one launch (host arrays of device pointers / element counts).
+ * rte_rmsnorm_op_fwd: y f32 = x (+ res) (y may be NULL), out = y * rsqrt(mean(y^2) + eps) * w, sum = y in sum's type when
+ *   res is given; x, res, w, out, sum are bf16 or f32 each ([rows, d], w [d]); rstd f32 [rows]; w_f32 f32 [d] optional copy.
+ * rte_rope_views: q and k [B, H, S, hd] views (strides in elements for B, H, S; unit along hd) rotated by cos / sin [S, hd].
+ * rte_pack_qkv: q, k, v views -> bf16 rows [B * S, 3 * H * hd] as the attention kernels read them.                     */
+int rte_cast_many_f32_bf16(const float* const* src, void* const* dst, const int64_t* n, int32_t count, rte_stream_t stream);
+int rte_rmsnorm_op_fwd(const void* x, int32_t x_bf16, const void* res, int32_t res_bf16, const void* w, int32_t w_bf16, float* y,
+                       void* out, int32_t out_bf16, void* sum, int32_t sum_bf16, float* rstd, float* w_f32, int32_t rows, int32_t d,
+                       float eps, rte_stream_t stream);
+int rte_rope_views(const void* q, const int64_t* q_strides, const void* k, const int64_t* k_strides, void* q_out,
+                   const int64_t* qo_strides, void* k_out, const int64_t* ko_strides, const float* cos_tab, const float* sin_tab,
+                   int32_t B, int32_t H, int32_t S, int32_t hd, int32_t is_bf16, int32_t adjoint, rte_stream_t stream);
+int rte_pack_qkv(const void* q, const int64_t* q_strides, const void* k, const int64_t* k_strides, const void* v,
+                 const int64_t* v_strides, void* qkv, int32_t B, int32_t H, int32_t S, int32_t hd, int32_t is_bf16,
+                 rte_stream_t stream);
+
 /* ---------------------------------------------------- embedding (models.py:136,693) */
 int rte_embed_fwd(const int64_t* tokens, const float* table, float* out, int32_t n_tokens, int32_t d,
                   int32_t vocab, int32_t* status, rte_stream_t stream);

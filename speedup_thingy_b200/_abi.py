@@ -101,6 +101,10 @@ PROTOTYPES = {
     "rte_gemm_bf16": (C.c_int, [P(GemmArgs), c_vp]),
     "rte_gemm_bf16_small": (C.c_int, [P(GemmArgs), c_vp]),
     "rte_gemm_bf16_tile": (C.c_int, [P(GemmArgs), C.c_int32, C.c_int32, c_vp]),
+    "rte_cast_many_f32_bf16": (C.c_int, [c_vp, c_vp, c_vp, c_i32, c_vp]),
+    "rte_rmsnorm_op_fwd": (C.c_int, [c_vp, c_i32, c_vp, c_i32, c_vp, c_i32, c_vp, c_vp, c_i32, c_vp, c_i32, c_vp, c_vp, c_i32, c_i32, C.c_float, c_vp]),
+    "rte_rope_views": (C.c_int, [c_vp] * 10 + [c_i32] * 6 + [c_vp]),
+    "rte_pack_qkv": (C.c_int, [c_vp] * 7 + [c_i32] * 5 + [c_vp]),
     "rte_ce_fwd_bwd_f32": (C.c_int, [c_vp, c_i32, c_vp, c_vp, c_i32, c_vp, c_vp, c_i32, c_i32, c_vp, c_vp]),
     "rte_host_randint": (C.c_int, [C.c_uint64, c_i64, C.c_int32, c_vp]),
     "rte_gemm_wgrad_splits": (C.c_int, [P(GemmArgs), C.c_int32]),
@@ -228,6 +232,28 @@ def load() -> C.CDLL:
         fn.argtypes = argtypes
     _lib = lib
     return lib
+
+
+_host = None
+
+
+def load_host():
+    """The native autograd operators over the C ABI (csrc/host_ops.cpp); raises if they have not been built."""
+    global _host
+    if _host is None:
+        import importlib.util
+
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+
+        load()
+        path = LIB_PATH.parent / "_rte_host.so"
+        if not path.exists():
+            raise RteError(f"{path} is missing: build it with `python -m speedup_thingy_b200.build`")
+        spec = importlib.util.spec_from_file_location("_rte_host", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _host = module
+    return _host
 
 
 def check(code: int, what: str) -> None:

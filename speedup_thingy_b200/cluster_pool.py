@@ -96,7 +96,11 @@ class StaticClusterPoolSwiGLU:
         self.dxp = e(self.cap, d, dtype=f32)
         self.dwug_pool, self.dwd_pool = e(C * 2 * Mc, d, dtype=f32), e(C * Mc, d, dtype=f32)
         self.dwdT = e(F, d, dtype=f32)
-        self._tokens = 0
+        names = ("selector16 centers idx_ug idx_d wug16 wdT16 wug_pool wd_pool q assign pos perm tile_group counts offsets kblocks x16 "
+                 "xp ugp zp yp dyp dzp dugp dxp dwug_pool dwd_pool dwdT").split()
+        self._native = A.load_host().PoolModule(
+            {**{k: getattr(self, k) for k in names}, "status": self.ops.status, "ug_ptr": self.csr_ug[0], "ug_rows": self.csr_ug[1],
+             "d_ptr": self.csr_d[0], "d_rows": self.csr_d[1]}, dict(rank=r, C=C, Mc=Mc, cap=self.cap, d=d, F=F))
 
     # ------------------------------------------------------------------ routing / packing
     def route(self, x: torch.Tensor, scores: torch.Tensor | None = None) -> torch.Tensor:
@@ -126,47 +130,15 @@ class StaticClusterPoolSwiGLU:
         router, as cluster_pool_ffn_forward_from_assignments does."""
         if not x.is_cuda:
             raise RuntimeError("strict_cuda: StaticClusterPoolSwiGLU needs CUDA tensors (no CPU or Triton path)")
-        o, d, Mc, C = self.ops, self.d, self.Mc, self.C
-        flat = x.reshape(-1, d).contiguous()
-        N = flat.shape[0]
+        N = x.numel() // self.d
         if N > self.max_tokens:
             raise ValueError(f"{N} tokens exceed max_tokens={self.max_tokens}")
-        self._tokens = N
-        a = self.route(flat) if assignments is None else assignments.to(torch.int32).contiguous()
-        self.pack(a)
-        self.prepare_pools()
-        o.gather_rows_convert(flat, self.perm, self.xp)                                   # pack + cast, zero padding rows
-        grp = dict(tile_group=self.tile_group, n_groups=C)
-        o.gemm(self.xp, self.wug_pool, self.ugp, M=self.cap, N=2 * Mc, K=d, b_group_stride=2 * Mc, **grp)
-        # pooled (up | gate) per cluster: columns [0, Mc) = up, [Mc, 2Mc) = gate of the cluster's candidates
-        o.swiglu_fwd(self.ugp, self.zp, self.cap, Mc)
-        o.gemm(self.zp, self.wd_pool, self.yp, M=self.cap, N=d, K=Mc, b_mn=True, epilogue=A.EPI_F32,
-               b_group_stride=Mc, **grp)
-        out = torch.empty(N, d, dtype=torch.float32, device=x.device)
-        o.gather_rows_convert(self.yp, self.pos[:N], out)
-        return out.view(*x.shape[:-1], d)
+        return self._native.forward(x.detach(), self.wug, self.wd, assignments)
 
     def backward(self, dout: torch.Tensor, dwug: torch.Tensor, dwd: torch.Tensor, accumulate: bool = False) -> torch.Tensor:
         """Gradients of the last forward: returns dx fp32 and writes (or adds) the dense weight gradients
         dwug [2F, d], dwd [d, F] (rows of neurons outside every used pool receive exact zeros)."""
-        o, d, Mc, C, N = self.ops, self.d, self.Mc, self.C, self._tokens
-        grp = dict(tile_group=self.tile_group, n_groups=C)
-        o.gather_rows_convert(dout.reshape(-1, d).contiguous(), self.perm, self.dyp)
-        o.gemm(self.dyp, self.wd_pool, self.dzp, M=self.cap, N=Mc, K=d, b_group_stride=Mc, **grp)
-        o.swiglu_bwd(self.ugp, self.dzp, self.dugp, self.cap, Mc)
-        o.gemm(self.dugp, self.wug_pool, self.dxp, M=self.cap, N=d, K=2 * Mc, b_mn=True, epilogue=A.EPI_F32,
-               b_group_stride=2 * Mc, **grp)
-        # per-cluster weight gradients: the reduction runs over the cluster's packed rows (ragged split-K)
-        o.gemm(self.zp, self.dyp, self.dwd_pool, M=Mc, N=d, K=self.cap, a_mn=True, b_mn=True, epilogue=A.EPI_F32,
-               splits=C, split_stride=Mc * d, split_kblocks=self.kblocks, ldc=d)
-        o.gemm(self.dugp, self.xp, self.dwug_pool, M=2 * Mc, N=d, K=self.cap, a_mn=True, b_mn=True, epilogue=A.EPI_F32,
-               splits=C, split_stride=2 * Mc * d, split_kblocks=self.kblocks, ldc=d)
-        o.csr_row_reduce(self.dwug_pool, *self.csr_ug, dwug, accumulate)
-        o.csr_row_reduce(self.dwd_pool, *self.csr_d, self.dwdT, False)
-        o.transpose(self.dwdT, dwd, accumulate)
-        dx = torch.empty(N, d, dtype=torch.float32, device=dout.device)
-        o.gather_rows_convert(self.dxp, self.pos[:N], dx)
-        return dx.view(dout.shape)
+        return self._native.backward(dout.detach(), dwug, dwd, accumulate)
 
     def dense_forward(self, x: torch.Tensor) -> torch.Tensor:
         """The un-pooled FFN (layers.py:184-186) through the same GEMM kernel, for comparisons."""

@@ -6,8 +6,9 @@ six operators the reference model actually calls -- ``k_fused_rmsnorm`` (layers.
 (layers.py:50), ``k_flash_causal_dense`` (layers.py:73), ``k_flash_causal_grouped`` (layers.py:725),
 ``k_out_proj_grouped`` (layers.py:727), ``k_logits_shortlist`` (output.py:125) -- and the benchmarked
 ``k_logits_full`` / ``k_qkv_dense`` / ``k_cross_entropy_unreduced`` through the sm_100a kernels of the C ABI.
-Every operator is a ``torch.autograd.Function`` whose forward and backward are C-ABI launches; tensors go in
-and come out as the reference's do (fresh outputs, inputs untouched, non-contiguous inputs made contiguous).
+Every operator is an autograd function whose forward and backward are C-ABI launches, native where it is called per layer
+(csrc/host_ops.cpp: the host spends 4 us per launch there against 15-20 us from Python); tensors go in and come out as the
+reference's do (fresh outputs, inputs untouched, non-contiguous inputs accepted).
 
 There is no fallback: CPU tensors raise ``RuntimeError`` mentioning ``strict_cuda`` whatever the flag says
 (optimized.py:51-55), and a missing library or device raises when the first operator is called.
@@ -57,8 +58,16 @@ def _require_cuda_tensor(*tensors) -> None:
 def _ops_for(t: torch.Tensor) -> CudaOps:
     idx = t.device.index if t.device.index is not None else torch.cuda.current_device()
     if idx not in _OPS:
-        _OPS[idx] = CudaOps(torch.device("cuda", idx))
+        ops = CudaOps(torch.device("cuda", idx))
+        A.load_host().bind_status(ops.status)
+        _OPS[idx] = ops
     return _OPS[idx]
+
+
+def _native(t: torch.Tensor):
+    """The native operators, with the launch table of `t`'s device in place."""
+    _ops_for(t)
+    return A.load_host()
 
 
 def _bf16(t: torch.Tensor) -> torch.Tensor:
@@ -75,120 +84,24 @@ def _check_gemm_dims(*dims: int) -> None:
 
 
 # --------------------------------------------------------------------------- RMSNorm (reference.py:9-17)
-class _RmsNorm(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, weight, residual, eps):
-        ops = _ops_for(x)
-        y = _f32(x)
-        if residual is not None:
-            y = y.clone() if y.data_ptr() == x.data_ptr() else y
-            ops.add_(y, _f32(residual))
-        d = y.shape[-1]
-        w = _f32(weight)
-        out = torch.empty_like(y)
-        rstd = torch.empty(y.numel() // d, dtype=torch.float32, device=y.device)
-        ops.rmsnorm_fwd(y, w, None, rstd, y_f32=out, eps=eps)
-        ctx.save_for_backward(y, w, rstd)
-        ctx.has_residual = residual is not None
-        ctx.in_dtypes = (x.dtype, weight.dtype, None if residual is None else residual.dtype)
-        out_dtype = torch.result_type(x, weight)
-        if residual is None:
-            return out.to(out_dtype), None
-        return out.to(out_dtype), y.to(torch.result_type(x, residual))
-
-    @staticmethod
-    def backward(ctx, d_out, d_sum):
-        y, w, rstd = ctx.saved_tensors
-        ops = _ops_for(y)
-        d = y.shape[-1]
-        rows = y.numel() // d
-        dx = torch.empty_like(y)
-        dw = torch.empty_like(w)
-        partial = torch.empty(8 * ops.sm_count, d, dtype=torch.float32, device=y.device)
-        dres = _f32(d_sum) if (ctx.has_residual and d_sum is not None) else None
-        d_out = _f32(d_out) if d_out is not None else torch.zeros_like(y)
-        ops.rmsnorm_bwd(y, w, rstd, d_out, dres, dx, None, dw, partial, rows=rows)
-        xd, wd, rd = ctx.in_dtypes
-        return dx.to(xd), dw.to(wd), (dx.to(rd) if ctx.has_residual else None), None
-
-
 def k_fused_rmsnorm(x, weight, residual=None, eps: float = 1e-5):
     """(rmsnorm(x [+ residual]) * weight, x + residual | None), statistics in fp32 (reference.py:9-17)."""
     _require_cuda_tensor(x, weight, residual)
     if x.shape[-1] != weight.shape[-1]:
         raise ValueError("k_fused_rmsnorm: weight must match the last dimension of x")
-    return _RmsNorm.apply(x, weight, residual, float(eps))
+    return _native(x).rmsnorm(x, weight, residual, float(eps))
 
 
 # --------------------------------------------------------------------------- rotary embedding (reference.py:20-28)
-class _Rope(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, cos, sin):
-        ops = _ops_for(q)
-        S, hd = q.shape[-2], q.shape[-1]
-        c, s = _f32(cos).reshape(S, hd), _f32(sin).reshape(S, hd)
-        outs = []
-        for t in (q, k):
-            src = t.detach().contiguous()
-            if src.dtype not in (torch.float32, torch.bfloat16):
-                src = src.float()
-            out = torch.empty_like(src)
-            ops.rope_apply(src, c, s, out, rows=src.numel() // (S * hd), S=S, head_dim=hd)
-            outs.append(out.to(t.dtype))
-        ctx.save_for_backward(c, s)
-        return tuple(outs)
-
-    @staticmethod
-    def backward(ctx, dq, dk):
-        c, s = ctx.saved_tensors
-        ops = _ops_for(c)
-        S, hd = c.shape
-        grads = []
-        for g in (dq, dk):
-            src = g.contiguous() if g.dtype in (torch.float32, torch.bfloat16) else g.float().contiguous()
-            out = torch.empty_like(src)
-            ops.rope_apply(src, c, s, out, rows=src.numel() // (S * hd), S=S, head_dim=hd, adjoint=True)
-            grads.append(out.to(g.dtype))
-        return grads[0], grads[1], None, None
-
-
 def k_rope_apply(q, k, cos, sin):
     """q*cos + rotate_half(q)*sin on adjacent pairs, same for k; cos/sin [S, head_dim] (reference.py:20-28)."""
     _require_cuda_tensor(q, k, cos, sin)
     if q.shape[-2:] != k.shape[-2:] or cos.shape[-2:] != q.shape[-2:] or cos.numel() != q.shape[-2] * q.shape[-1]:
         raise ValueError("k_rope_apply: q/k [..., S, head_dim] with cos/sin [S, head_dim]")
-    return _Rope.apply(q, k, cos, sin)
+    return _native(q).rope(q, k, cos, sin)
 
 
 # --------------------------------------------------------------------------- causal attention (reference.py:40-41,54-55)
-class _FlashCausal(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v):
-        ops = _ops_for(q)
-        B, H, S, hd = q.shape
-        # the kernels read one packed [B*S, 3*H*hd] buffer, columns (q | k | v), head-major inside each
-        qkv = torch.stack([q.detach(), k.detach(), v.detach()], dim=0).to(torch.bfloat16)      # [3,B,H,S,hd]
-        qkv = qkv.permute(1, 3, 0, 2, 4).contiguous().view(B * S, 3 * H * hd)
-        y = torch.empty(B * S, H * hd, dtype=torch.bfloat16, device=q.device)
-        lse = torch.empty(B * H * S, dtype=torch.float32, device=q.device)
-        ops.attn_fwd(qkv, y, lse, B=B, S=S, n_heads=H, head_dim=hd, rope=ops.identity_rope_table(S, hd))
-        ctx.save_for_backward(qkv, y, lse)
-        ctx.dims = (B, H, S, hd)
-        ctx.in_dtype = q.dtype
-        return y.view(B, S, H, hd).permute(0, 2, 1, 3).to(q.dtype)
-
-    @staticmethod
-    def backward(ctx, d_out):
-        qkv, y, lse = ctx.saved_tensors
-        ops = _ops_for(qkv)
-        B, H, S, hd = ctx.dims
-        dy = d_out.permute(0, 2, 1, 3).to(torch.bfloat16).contiguous().view(B * S, H * hd)
-        dqkv = torch.empty_like(qkv)
-        ops.attn_bwd(qkv, y, dy, lse, dqkv, B=B, S=S, n_heads=H, head_dim=hd, rope=ops.identity_rope_table(S, hd))
-        g = dqkv.view(B, S, 3, H, hd).permute(2, 0, 3, 1, 4).to(ctx.in_dtype)
-        return g[0], g[1], g[2]
-
-
 def k_flash_causal_dense(q, k, v):
     """softmax(q k^T / sqrt(head_dim), causal) v over [B, H, S, head_dim] (reference.py:40-41)."""
     _require_cuda_tensor(q, k, v)
@@ -196,85 +109,17 @@ def k_flash_causal_dense(q, k, v):
         raise ValueError("k_flash_causal_*: q, k, v must share the shape [B, H, S, head_dim]")
     if q.shape[2] > 256 or q.shape[3] not in (8, 16, 32, 64, 128):
         raise ValueError("k_flash_causal_*: S <= 256 and head_dim in {8,16,32,64,128}")
-    return _FlashCausal.apply(q, k, v)
+    return _native(q).attention(q, k, v, _ops_for(q).identity_rope_table(q.shape[2], q.shape[3]))
 
 
 k_flash_causal_grouped = k_flash_causal_dense          # same arithmetic over the active heads (reference.py:54-55)
 
 
 # --------------------------------------------------------------------------- GEMM-bearing operators
-def _mm_io(ops: CudaOps, x16, w16, out_dtype):
-    """x16 [M, in] @ w16 [in, out] (weight stored input-major, the banked layout of layers.py:690-696)."""
-    M, K = x16.shape
-    N = w16.shape[1]
-    out = torch.empty(M, N, dtype=torch.bfloat16, device=x16.device)
-    ops.gemm(x16, w16, out, M=M, N=N, K=K, b_mn=True)
-    return out if out_dtype == torch.bfloat16 else out.to(out_dtype)
-
-
-class _MatmulIO(torch.autograd.Function):
-    """y = x @ w, w [in, out]."""
-
-    @staticmethod
-    def forward(ctx, x, w):
-        ops = _ops_for(x)
-        x16, w16 = _bf16(x).view(-1, x.shape[-1]), _bf16(w)
-        _check_gemm_dims(x16.shape[1], w16.shape[1])
-        ctx.save_for_backward(x16, w16)
-        ctx.meta = (x.shape, x.dtype, w.dtype)
-        return _mm_io(ops, x16, w16, x.dtype).view(*x.shape[:-1], w.shape[1])
-
-    @staticmethod
-    def backward(ctx, dy):
-        x16, w16 = ctx.saved_tensors
-        ops = _ops_for(x16)
-        xshape, xd, wd = ctx.meta
-        M, K = x16.shape
-        N = w16.shape[1]
-        dy16 = _bf16(dy).view(M, N)
-        dx = torch.empty(M, K, dtype=torch.float32, device=x16.device)
-        ops.gemm(dy16, w16, dx, M=M, N=K, K=N, epilogue=A.EPI_F32)                 # dy [M,out] . w[in,out]^T
-        dw = torch.empty(K, N, dtype=torch.float32, device=x16.device)
-        ops.gemm_wgrad(x16, dy16, dw, M=K, N=N, K=M)                                # x^T dy, reduction over tokens
-        return dx.view(xshape).to(xd), dw.to(wd)
-
-
-class _MatmulOI(torch.autograd.Function):
-    """y = x @ w^T, w [out, in] (nn.Linear / tied-embedding layout)."""
-
-    @staticmethod
-    def forward(ctx, x, w):
-        ops = _ops_for(x)
-        x16, w16 = _bf16(x).view(-1, x.shape[-1]), _bf16(w)
-        _check_gemm_dims(x16.shape[1])
-        M, K = x16.shape
-        N = w16.shape[0]
-        out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
-        ops.gemm(x16, w16, out, M=M, N=N, K=K)
-        ctx.save_for_backward(x16, w16)
-        ctx.meta = (x.shape, x.dtype, w.dtype)
-        return out.to(x.dtype).view(*x.shape[:-1], N)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x16, w16 = ctx.saved_tensors
-        ops = _ops_for(x16)
-        xshape, xd, wd = ctx.meta
-        M, K = x16.shape
-        N = w16.shape[0]
-        _check_gemm_dims(N)
-        dy16 = _bf16(dy).view(M, N)
-        dx = torch.empty(M, K, dtype=torch.float32, device=x16.device)
-        ops.gemm(dy16, w16, dx, M=M, N=K, K=N, b_mn=True, epilogue=A.EPI_F32)      # dy [M,out] . w[out,in]
-        dw = torch.empty(N, K, dtype=torch.float32, device=x16.device)
-        ops.gemm_wgrad(dy16, x16, dw, M=N, N=K, K=M)                                # dy^T x
-        return dx.view(xshape).to(xd), dw.to(wd)
-
-
 def k_qkv_dense(x, wq, wk, wv):
     """(x @ wq, x @ wk, x @ wv), weights [in, out] (reference.py:31-37)."""
     _require_cuda_tensor(x, wq, wk, wv)
-    return _MatmulIO.apply(x, wq), _MatmulIO.apply(x, wk), _MatmulIO.apply(x, wv)
+    return _native(x).qkv_dense(x, wq, wk, wv)
 
 
 def k_logits_full(hidden, vocab_weight):
@@ -282,48 +127,15 @@ def k_logits_full(hidden, vocab_weight):
     _require_cuda_tensor(hidden, vocab_weight)
     if hidden.shape[-1] != vocab_weight.shape[-1]:
         raise ValueError("k_logits_full: hidden [..., d] against vocab_weight [V, d]")
-    return _MatmulOI.apply(hidden, vocab_weight)
-
-
-class _OutProjGrouped(torch.autograd.Function):
-    """x @ wo[row_indices, :] with the selected rows gathered by the C-ABI row gather (reference.py:58-59)."""
-
-    @staticmethod
-    def forward(ctx, x, wo, row_indices):
-        ops = _ops_for(x)
-        idx = row_indices.detach().to(torch.int32).contiguous()
-        n, dout = idx.numel(), wo.shape[1]
-        _check_gemm_dims(n, dout)
-        wo16 = _bf16(wo)
-        sel = torch.empty(n, dout, dtype=torch.bfloat16, device=x.device)
-        ops.gather_rows(wo16, idx, sel, n, dout * 2)
-        x16 = _bf16(x).view(-1, n)
-        ctx.save_for_backward(x16, sel, idx)
-        ctx.meta = (x.shape, x.dtype, wo.dtype, wo.shape)
-        return _mm_io(ops, x16, sel, x.dtype).view(*x.shape[:-1], dout)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x16, sel, idx = ctx.saved_tensors
-        ops = _ops_for(x16)
-        xshape, xd, wd, wshape = ctx.meta
-        M, n = x16.shape
-        dout = sel.shape[1]
-        dy16 = _bf16(dy).view(M, dout)
-        dx = torch.empty(M, n, dtype=torch.float32, device=x16.device)
-        ops.gemm(dy16, sel, dx, M=M, N=n, K=dout, epilogue=A.EPI_F32)
-        dsel = torch.empty(n, dout, dtype=torch.float32, device=x16.device)
-        ops.gemm_wgrad(x16, dy16, dsel, M=n, N=dout, K=M)
-        dwo = torch.zeros(wshape, dtype=torch.float32, device=x16.device)
-        ops.scatter_add_rows(dwo, idx, dsel, n, dout)
-        return dx.view(xshape).to(xd), dwo.to(wd), None
+    return _native(hidden).matmul_oi(hidden, vocab_weight)
 
 
 def k_out_proj_grouped(x, wo, row_indices):
+    """x @ wo[row_indices, :] with the selected rows gathered by the C-ABI row gather (reference.py:58-59)."""
     _require_cuda_tensor(x, wo, row_indices)
     if x.shape[-1] != row_indices.numel():
         raise ValueError("k_out_proj_grouped: x [..., len(row_indices)]")
-    return _OutProjGrouped.apply(x, wo, row_indices)
+    return _native(x).out_proj(x, wo, row_indices)
 
 
 # --------------------------------------------------------------------------- shortlist logits (reference.py:141-143)
@@ -370,35 +182,11 @@ def k_logits_shortlist(hidden, vocab_weight, shortlist):
 
 
 # --------------------------------------------------------------------------- cross entropy (reference.py:146-147)
-class _CrossEntropy(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, logits, targets):
-        ops = _ops_for(logits)
-        V = logits.shape[-1]
-        lg = _bf16(logits).view(-1, V)
-        tg = targets.detach().to(torch.int64).contiguous().view(-1)
-        loss = torch.empty(lg.shape[0], dtype=torch.float32, device=logits.device)
-        ops.ce_fwd_bwd(lg, tg, None, 1, loss, None)
-        ctx.save_for_backward(lg, tg)
-        ctx.meta = (logits.shape, logits.dtype)
-        return loss.view_as(targets)
-
-    @staticmethod
-    def backward(ctx, dloss):
-        lg, tg = ctx.saved_tensors
-        ops = _ops_for(lg)
-        shape, dt = ctx.meta
-        dlogits = torch.empty_like(lg)
-        scratch = torch.empty(lg.shape[0], dtype=torch.float32, device=lg.device)
-        ops.ce_fwd_bwd(lg, tg, _f32(dloss).view(-1), 1, scratch, dlogits)          # (softmax - onehot) * dloss[row]
-        return dlogits.view(shape).to(dt), None
-
-
 def k_cross_entropy_unreduced(logits, targets):
     _require_cuda_tensor(logits, targets)
     if logits.shape[:-1] != targets.shape:
         raise ValueError("k_cross_entropy_unreduced: logits [..., V] with targets [...]")
-    return _CrossEntropy.apply(logits, targets)
+    return _native(logits).cross_entropy(logits, targets)
 
 
 # --------------------------------------------------------------------------- host-side helpers of the table
@@ -523,58 +311,16 @@ def k_macro_phi(h, h0, d_gain, v, u, bias, eps: float = 1e-5):
     normed, _ = k_fused_rmsnorm(h, torch.ones(h.shape[-1], device=h.device, dtype=h.dtype), None, eps)
     pooled = normed.mean(dim=1, keepdim=True).expand_as(normed)
     z = torch.cat([normed, pooled, h0], dim=-1)
-    low = _MatmulIO.apply(torch.nn.functional.silu(_MatmulIO.apply(z, v)), u)
+    native = _native(z)
+    low = native.matmul_io(torch.nn.functional.silu(native.matmul_io(z, v)), u)
     return h + d_gain * h + low + bias
 
 
 # --------------------------------------------------------------------------- packed SwiGLU FFN
-class _PackedSwiGLUFFN(torch.autograd.Function):
-    """(x @ wug^T -> (up | gate)) -> up * silu(gate) -> @ wdown_rows, saving (x, wug, wdown_rows, ug, z) in bf16
-    exactly as the reference's _TritonPackedSwiGLUFFN does (kernels/active_swiglu_triton.py:62-108)."""
-
-    @staticmethod
-    def forward(ctx, x, wug, wdown_rows):
-        ops = _ops_for(x)
-        N, d = x.shape
-        m = wug.shape[0] // 2
-        x16, wug16, wd16 = _bf16(x), _bf16(wug), _bf16(wdown_rows)
-        ug = torch.empty(N, 2 * m, dtype=torch.bfloat16, device=x.device)
-        z = torch.empty(N, m, dtype=torch.bfloat16, device=x.device)
-        y = torch.empty(N, d, dtype=torch.float32, device=x.device)
-        if m % 64 == 0 and N <= 1024:        # small batches: SwiGLU fused into the GEMM epilogue
-            ops.gemm(x16, wug16, z, M=N, N=2 * m, K=d, epilogue=A.EPI_SWIGLU_FWD, out2=ug, pair=m)
-        else:                                # large batches: plain-store GEMM + one vectorised pass is faster
-            ops.gemm(x16, wug16, ug, M=N, N=2 * m, K=d)
-            ops.swiglu_fwd(ug, z, N, m)
-        ops.gemm(z, wd16, y, M=N, N=d, K=m, b_mn=True, epilogue=A.EPI_F32)
-        ctx.save_for_backward(x16, wug16, wd16, ug, z)
-        ctx.dtypes = (x.dtype, wug.dtype, wdown_rows.dtype)
-        return y.to(x.dtype)
-
-    @staticmethod
-    def backward(ctx, dy):
-        x16, wug16, wd16, ug, z = ctx.saved_tensors
-        ops = _ops_for(x16)
-        N, d = x16.shape
-        m = wd16.shape[0]
-        dy16 = _bf16(dy)
-        dz = torch.empty(N, m, dtype=torch.bfloat16, device=x16.device)
-        dug = torch.empty(N, 2 * m, dtype=torch.bfloat16, device=x16.device)
-        ops.gemm(dy16, wd16, dz, M=N, N=m, K=d)
-        ops.swiglu_bwd(ug, dz, dug, N, m)
-        dx = torch.empty(N, d, dtype=torch.float32, device=x16.device)
-        ops.gemm(dug, wug16, dx, M=N, N=d, K=2 * m, b_mn=True, epilogue=A.EPI_F32)
-        dwug = torch.empty(2 * m, d, dtype=torch.float32, device=x16.device)
-        ops.gemm_wgrad(dug, x16, dwug, M=2 * m, N=d, K=N)
-        dwd = torch.empty(m, d, dtype=torch.float32, device=x16.device)
-        ops.gemm_wgrad(z, dy16, dwd, M=m, N=d, K=N)
-        xd, ud, dd = ctx.dtypes
-        return dx.to(xd), dwug.to(ud), dwd.to(dd)
-
-
 def packed_swiglu_ffn(x, wug, wdown_rows):
     """Drop-in for ``triton_packed_swiglu_ffn`` (kernels/active_swiglu_triton.py:111-125; layers.py:90-116,284-339):
-    x [tokens, d], wug [2*active_m, d] = (up rows | gate rows), wdown_rows [active_m, d].  Same shape errors."""
+    x [tokens, d], wug [2*active_m, d] = (up rows | gate rows), wdown_rows [active_m, d].  Same shape errors;
+    saves (x, wug, wdown_rows, ug, z) in bf16 as the reference's _TritonPackedSwiGLUFFN does (:62-108)."""
     _require_cuda_tensor(x, wug, wdown_rows)
     if x.ndim != 2 or wug.ndim != 2 or wdown_rows.ndim != 2:
         raise ValueError("expected x [N,D], wug [2M,D], wdown_rows [M,D]")
@@ -583,7 +329,7 @@ def packed_swiglu_ffn(x, wug, wdown_rows):
     if wdown_rows.shape[0] != wug.shape[0] // 2:
         raise ValueError("wdown_rows first dimension must match M")
     _check_gemm_dims(x.shape[1], wdown_rows.shape[0])
-    return _PackedSwiGLUFFN.apply(x, wug, wdown_rows)
+    return _native(x).packed_ffn(x, wug, wdown_rows)
 
 
 triton_packed_swiglu_ffn = packed_swiglu_ffn          # the symbol layers.py:12-22 imports

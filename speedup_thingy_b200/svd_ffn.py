@@ -68,48 +68,27 @@ class SVDFactorSparseFFN:
         self.cand_count = e(N, dtype=torch.int32)
         self.dout16, self.dz, self.dug = e(N, d), e(N, F), e(N, 2 * F)
         self.dwug = e(2 * F, d, dtype=f32)
-        self._tokens = 0
+        names = "selector16 up_b16 gate_b16 wug16 wd16 wn x16 q16 hats ug z selected cand_count dout16 dz dug dwug".split()
+        self._native = A.load_host().SvdModule(
+            {**{k: getattr(self, k) for k in names}, "status": self.ops.status},
+            dict(rank=r, F=F, d=d, up_m=self.up_m, gate_m=self.gate_m, product_m=self.product_m, top_k=self.top_k))
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         if not x.is_cuda:
             raise RuntimeError("strict_cuda: SVDFactorSparseFFN needs CUDA tensors (no CPU or Triton path)")
-        o, d, F, r = self.ops, self.d, self.F, self.rank
-        flat = x.reshape(-1, d).contiguous()
-        N = self._tokens = flat.shape[0]
+        N = x.numel() // self.d
         if N > self.max_tokens:
             raise ValueError(f"{N} tokens exceed max_tokens={self.max_tokens}")
-        x16, q16, hats, ug, z = self.x16[:N], self.q16[:N], self.hats[:N], self.ug[:N], self.z[:N]
-        o.cast_bf16(flat, x16) if flat.dtype == torch.float32 else x16.copy_(flat)
-        o.cast_bf16(self.w_up, self.wug16[:F])
-        o.cast_bf16(self.w_gate, self.wug16[F:])
-        o.cast_bf16(self.w_down, self.wd16)
-        o.row_norm(self.w_down, self.wn)
-        o.gemm(x16, self.selector16, q16, M=N, N=2 * r, K=d)
-        o.gemm(q16, self.up_b16, hats, M=N, N=F, K=r, b_mn=True, epilogue=A.EPI_F32, lda=2 * r, ldc=2 * F)
-        o.gemm(q16[:, r:], self.gate_b16, hats[:, F:], M=N, N=F, K=r, b_mn=True, epilogue=A.EPI_F32, lda=2 * r, ldc=2 * F)
-        o.gemm(x16, self.wug16, ug, M=N, N=2 * F, K=d)
-        o.svd_ffn_select(hats, ug, self.wn, z, self.selected[:N], self.cand_count[:N], up_m=self.up_m, gate_m=self.gate_m,
-                         product_m=self.product_m, top_k=self.top_k)
-        out = torch.empty(N, d, dtype=torch.float32, device=x.device)
-        o.gemm(z, self.wd16, out, M=N, N=d, K=F, b_mn=True, epilogue=A.EPI_F32)
-        return out.view(*x.shape[:-1], d)
+        return self._native.forward(x.detach(), self.w_up, self.w_gate, self.w_down)
 
     def backward(self, dout: torch.Tensor, dw_up, dw_gate, dw_down) -> torch.Tensor:
         """Gradients of the last forward: returns dx (fp32) and fills dw_up, dw_gate, dw_down [F, d] (fp32);
         neurons no token selected receive exact zeros."""
-        o, d, F, N = self.ops, self.d, self.F, self._tokens
-        x16, ug, z, dz, dug, dout16 = self.x16[:N], self.ug[:N], self.z[:N], self.dz[:N], self.dug[:N], self.dout16[:N]
-        flat = dout.reshape(-1, d).contiguous()
-        o.cast_bf16(flat, dout16) if flat.dtype == torch.float32 else dout16.copy_(flat)
-        o.gemm(dout16, self.wd16, dz, M=N, N=F, K=d)
-        o.svd_ffn_swiglu_bwd(ug, dz, self.selected[:N], dug)
-        dx = torch.empty(N, d, dtype=torch.float32, device=dout.device)
-        o.gemm(dug, self.wug16, dx, M=N, N=d, K=2 * F, b_mn=True, epilogue=A.EPI_F32)
-        o.gemm_wgrad(dug, x16, self.dwug, M=2 * F, N=d, K=N)
-        dw_up.copy_(self.dwug[:F])
-        dw_gate.copy_(self.dwug[F:])
-        o.gemm_wgrad(z, dout16, dw_down, M=F, N=d, K=N)
-        return dx.view(dout.shape)
+        return self._native.backward(dout.detach(), dw_up, dw_gate, dw_down)
+
+    @property
+    def _tokens(self) -> int:
+        return self._native.tokens
 
     @property
     def avg_candidate_size(self) -> float:
@@ -131,7 +110,8 @@ class _SvdFfnFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         m = ctx.module
-        g = [torch.empty_like(m.w_up), torch.empty_like(m.w_gate), torch.empty_like(m.w_down)]
+        both = torch.empty(2 * m.F, m.d, dtype=torch.float32, device=dout.device)      # one product writes both gradients
+        g = [both[: m.F], both[m.F:], torch.empty_like(m.w_down)]
         dx = m.backward(dout.contiguous(), *g)
         return dx, g[0], g[1], g[2], None
 

@@ -303,3 +303,101 @@ def test_pack_by_recipe_round_trip_and_grads():
     assert torch.equal(hg.grad.cpu(), want)
     mask = K.k_sample_audit_mask(torch.full((64,), 0.25, device=DEV), 5)
     assert mask.dtype == torch.bool and mask.shape == (64,)
+
+
+@pytest.mark.parametrize("rows,V,dtype", [(5, 8, torch.bfloat16), (33, 1000, torch.bfloat16), (64, 2056, torch.bfloat16), (7, 2047, torch.bfloat16),
+                                          (9, 32768, torch.bfloat16), (3, 65544, torch.bfloat16), (17, 4, torch.float32), (33, 2047, torch.float32),
+                                          (20, 4100, torch.float32), (4, 32772, torch.float32)])
+def test_cross_entropy_row_widths(rows, V, dtype):
+    """Widths around the register limits of the row kernel, and the rows that only the general kernel takes."""
+    gen = torch.Generator().manual_seed(V)
+    logits = (3 * torch.randn(rows, V, generator=gen)).to(dtype)
+    targets = torch.randint(0, V, (rows,), generator=gen)
+    targets[0], targets[-1] = V - 1, 0
+    weight = torch.randn(rows, generator=gen)
+    ref = logits.float().clone().requires_grad_(True)
+    ref_loss = torch.nn.functional.cross_entropy(ref, targets, reduction="none")
+    (ref_loss * weight).sum().backward()
+    x = logits.cuda().requires_grad_(True)
+    loss = K.k_cross_entropy_unreduced(x, targets.cuda())
+    (loss * weight.cuda()).sum().backward()
+    assert torch.allclose(loss.cpu(), ref_loss, atol=1e-4, rtol=1e-5)
+    assert torch.allclose(x.grad.cpu().float(), ref.grad, atol=1e-5, rtol=1e-2 if dtype == torch.bfloat16 else 1e-4)
+
+
+@pytest.mark.parametrize("d", [4, 132, 512, 2048])
+@pytest.mark.parametrize("xt,wt,rt", [(torch.bfloat16, torch.bfloat16, None), (torch.bfloat16, torch.float32, torch.float32), (torch.float32, torch.bfloat16, torch.bfloat16),
+                                      (torch.float16, torch.float32, None)])
+def test_rmsnorm_row_widths_and_types(d, xt, wt, rt):
+    gen = torch.Generator().manual_seed(d)
+    x, w, g = torch.randn(11, d, generator=gen).to(xt), torch.randn(d, generator=gen).to(wt), torch.randn(11, d, generator=gen)
+    r = torch.randn(11, d, generator=gen).to(rt) if rt is not None else None
+    leaves = [t.float().requires_grad_(True) for t in (x, w) + ((r,) if r is not None else ())]
+    y = leaves[0] + leaves[2] if r is not None else leaves[0]
+    ref = y * torch.rsqrt(y.pow(2).mean(-1, keepdim=True) + 1e-5) * leaves[1]
+    (ref * g).sum().backward()
+    dev = [t.detach().cuda().requires_grad_(True) for t in (x, w) + ((r,) if r is not None else ())]
+    out, total = K.k_fused_rmsnorm(dev[0], dev[1], dev[2] if r is not None else None)
+    assert out.dtype == torch.result_type(x, w) and (total is None) == (r is None)
+    (out.float() * g.cuda()).sum().backward()
+    tol = 2e-2 if torch.bfloat16 in (out.dtype, xt, wt, rt) else 2e-3 if xt == torch.float16 else 1e-5
+    assert torch.allclose(out.cpu().float(), ref.detach(), atol=tol, rtol=tol)
+    if r is not None:
+        assert total.dtype == torch.result_type(x, r) and torch.allclose(total.cpu().float(), y.detach(), atol=tol, rtol=tol)
+    for a, b in zip(dev, leaves):
+        assert a.grad.dtype == a.dtype and torch.allclose(a.grad.cpu().float(), b.grad, atol=tol * max(1.0, b.grad.abs().max().item()), rtol=tol)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("layout", ["heads_first", "tokens_first", "odd_offset"])
+def test_rope_and_attention_take_strided_views(layout, dtype):
+    """q, k, v as a projection leaves them ([B, S, H, hd] transposed), contiguous, and on no 16-byte boundary."""
+    B, H, S, hd = 2, 3, 37, 16
+    gen = torch.Generator().manual_seed(0)
+    base = [torch.randn(B, H, S, hd, generator=gen).to(dtype) for _ in range(3)]
+
+    def place(t):
+        t = t.cuda()
+        if layout == "tokens_first":
+            return t.transpose(1, 2).contiguous().transpose(1, 2)
+        if layout == "odd_offset":
+            return torch.cat([t.new_zeros(B, H, S, 1), t], dim=-1)[..., 1:]
+        return t
+
+    ang = torch.randn(S, hd, generator=gen)
+    cos, sin = ang.cos(), ang.sin()
+    rot = lambda t: torch.stack([-t[..., 1::2], t[..., 0::2]], -1).flatten(-2)  # noqa: E731
+    q, k, v = (place(t) for t in base)
+    rq, rk = K.k_rope_apply(q, k, cos.cuda(), sin.cuda())
+    tol = 2e-2 if dtype == torch.bfloat16 else 1e-5
+    for got, t in ((rq, base[0]), (rk, base[1])):
+        assert got.is_contiguous() and torch.allclose(got.cpu().float(), t.float() * cos + rot(t.float()) * sin, atol=tol, rtol=tol)
+    out = K.k_flash_causal_dense(q, k, v)
+    ref = torch.nn.functional.scaled_dot_product_attention(*(t.bfloat16().float() for t in base), is_causal=True)
+    assert out.dtype == dtype and torch.allclose(out.cpu().float(), ref, atol=3e-2, rtol=3e-2)
+
+
+@pytest.mark.parametrize("N,d,m", [(7001, 64, 2048), (6900, 64, 2048)])
+def test_packed_swiglu_on_both_sides_of_the_fusion_rule(N, d, m):
+    gen = torch.Generator().manual_seed(N)
+    x, wug, wd = (0.2 * torch.randn(*s, generator=gen) for s in ((N, d), (2 * m, d), (m, d)))
+    g = torch.randn(N, d, generator=gen)
+    res = []
+    for dev in ("cpu", "cuda"):
+        t = [a.to(dev).detach().clone().requires_grad_(True) for a in (x, wug, wd)]
+        if dev == "cuda":
+            y = K.packed_swiglu_ffn(*t)
+        else:
+            ug = t[0] @ t[1].t()
+            y = (ug[:, :m] * torch.nn.functional.silu(ug[:, m:])) @ t[2]
+        (y * g.to(dev)).sum().backward()
+        res.append([y.detach().cpu()] + [a.grad.cpu() for a in t])
+    for a, b in zip(*res):
+        assert (a - b).norm() <= 1e-2 * a.norm()
+
+
+def test_products_of_an_odd_width_write_fp32_rows():
+    x, w = torch.randn(70, 64, device="cuda"), torch.randn(2047, 64, device="cuda")
+    ref = x.bfloat16().float() @ w.bfloat16().float().t()
+    got = K.k_logits_full(x, w)
+    assert got.dtype == torch.float32 and torch.allclose(got, ref, atol=1e-3, rtol=1e-3)
