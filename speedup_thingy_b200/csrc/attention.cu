@@ -351,10 +351,13 @@ __global__ void rope_apply_kernel(const T* __restrict__ x, const float* __restri
   } while (0)
 
 // Tensor-core path for the head sizes the mma.sync tiles cover; everything else falls through to the
-// SIMT kernels above (tiny heads of the test configurations).  Needs 16-byte aligned rows for ldmatrix.
-#define RTE_ATT_MMA_DISPATCH(FN, ...)                                          \
+// SIMT kernels above (tiny heads of the test configurations).  Needs rows on 16-byte boundaries.
+static bool rows_on_16(const void* a, const void* b, const void* c = nullptr, const void* d = nullptr) {
+  return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(d)) & 15) == 0;
+}
+#define RTE_ATT_MMA_DISPATCH(ALIGNED, FN, ...)                                 \
   do {                                                                         \
-    if (ld_qkv % 8 == 0 && sec % 8 == 0 && ld_y % 8 == 0) {                    \
+    if (ld_qkv % 8 == 0 && sec % 8 == 0 && ld_y % 8 == 0 && (ALIGNED)) {       \
       const int smax = S <= 64 ? 64 : S <= 128 ? 128 : 256;                    \
       switch (head_dim * 1000 + smax) {                                        \
         case 32064: return FN<32, 64>(__VA_ARGS__);                            \
@@ -400,7 +403,7 @@ extern "C" int rte_attn_fwd(const void* qkv, int32_t ld_qkv, int32_t sec, void* 
                             rte_stream_t stream) {
   RTE_CHECK_ARG(qkv && y && lse && B > 0 && S > 0 && S <= 256 && n_heads > 0 && ld_qkv % 2 == 0 && sec % 2 == 0);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  RTE_ATT_MMA_DISPATCH(attn_mma::launch_fwd, qkv, ld_qkv, sec, y, ld_y, lse, rope_table, B, S, n_heads, st);
+  RTE_ATT_MMA_DISPATCH(rows_on_16(qkv, y, rope_table), attn_mma::launch_fwd, qkv, ld_qkv, sec, y, ld_y, lse, rope_table, B, S, n_heads, st);
   RTE_ATT_DISPATCH(launch_fwd, qkv, ld_qkv, sec, y, ld_y, lse, rope_table, B, S, n_heads, st);
 }
 
@@ -413,8 +416,8 @@ extern "C" int rte_attn_fwd_masked(const void* qkv, int32_t ld_qkv, int32_t sec,
   RTE_CHECK_ARG(qkv && y && y_masked && lse && mask_row && mask_table && B > 0 && S > 0 && S <= 256 && n_heads > 0 &&
                 ld_qkv % 2 == 0 && sec % 2 == 0);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (ld_y == n_heads * head_dim && (reinterpret_cast<uintptr_t>(mask_table) & 7) == 0) {
-    RTE_ATT_MMA_DISPATCH(attn_mma::launch_fwd, qkv, ld_qkv, sec, y, ld_y, lse, rope_table, B, S, n_heads, st, y_masked, mask_row,
+  if (ld_y == n_heads * head_dim && rows_on_16(mask_table, y_masked)) {
+    RTE_ATT_MMA_DISPATCH(rows_on_16(qkv, y, rope_table), attn_mma::launch_fwd, qkv, ld_qkv, sec, y, ld_y, lse, rope_table, B, S, n_heads, st, y_masked, mask_row,
                          mask_table);
   }
   const int rc = rte_attn_fwd(qkv, ld_qkv, sec, y, ld_y, lse, rope_table, B, S, n_heads, head_dim, stream);
@@ -435,7 +438,8 @@ extern "C" int rte_attn_bwd_masked(const void* qkv, int32_t ld_qkv, int32_t sec,
                 ld_qkv % 2 == 0 && sec % 2 == 0 && ld_y % 2 == 0);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (ld_y == n_heads * head_dim) {
-    RTE_ATT_MMA_DISPATCH(attn_mma::launch_bwd, qkv, ld_qkv, sec, y, dy, ld_y, lse, dqkv, rope_table, B, S, n_heads, st, mask_row,
+    RTE_ATT_MMA_DISPATCH(rows_on_16(qkv, y, dy, dqkv) && rows_on_16(rope_table, mask_table), attn_mma::launch_bwd, qkv, ld_qkv, sec, y, dy, ld_y, lse,
+                         dqkv, rope_table, B, S, n_heads, st, mask_row,
                          mask_table);
   } else {
     return RTE_ERR_UNSUPPORTED;
@@ -451,6 +455,7 @@ extern "C" int rte_attn_bwd(const void* qkv, int32_t ld_qkv, int32_t sec, const 
   RTE_CHECK_ARG(qkv && y && dy && lse && dqkv && B > 0 && S > 0 && S <= 256 && n_heads > 0 && ld_qkv % 2 == 0 &&
                 sec % 2 == 0 && ld_y % 2 == 0);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  RTE_ATT_MMA_DISPATCH(attn_mma::launch_bwd, qkv, ld_qkv, sec, y, dy, ld_y, lse, dqkv, rope_table, B, S, n_heads, st);
+  RTE_ATT_MMA_DISPATCH(rows_on_16(qkv, y, dy, dqkv) && rows_on_16(rope_table, nullptr), attn_mma::launch_bwd, qkv, ld_qkv, sec, y, dy, ld_y, lse, dqkv,
+                       rope_table, B, S, n_heads, st);
   RTE_ATT_DISPATCH(launch_bwd, qkv, ld_qkv, sec, y, dy, ld_y, lse, dqkv, rope_table, B, S, n_heads, st);
 }
