@@ -435,8 +435,12 @@ colsum3_kernel(ColsumJobs jobs, int n_rows, int d) {
 }
 
 // ------------------------------------------------------------------ cross entropy
+// Rows are handled in 16-byte groups of W logits.  `off` is the number of elements between the 16-byte boundary at or
+// before the row and the row itself: group g holds logits g * W - off ..., its slots outside [0, V) read as -inf and are
+// never touched in memory, so rows of any width and alignment take the same kernels.  EVEN: every row starts on a
+// boundary and has whole groups only (without the checks 8192 x 2048 takes 20.5 us instead of 26.6).
 template <typename T>
-struct CeVec;                                    // one 16-byte group of logits
+struct CeVec;
 template <>
 struct CeVec<__nv_bfloat16> {
   static constexpr int W = 8;
@@ -461,127 +465,209 @@ struct CeVec<float> {
 __device__ __forceinline__ float to_f(float x) { return x; }
 __device__ __forceinline__ float to_f(__nv_bfloat16 x) { return __bfloat162float(x); }
 
-// One CTA of THREADS per row, the row in registers (at most NV 16-byte groups per thread): logits are read once, maximum
-// and sum of exponentials meet in one block reduction, the gradient is written from the registers.  Bound by HBM; the CTA
-// is as small as the row allows so that many rows are in flight per SM.  8192 x 2048 bf16 with gradient: 33.4 us with a
-// row read three times by 256 threads -> 24.6 us (67 MB).
-template <typename T, int THREADS, int NV>
+template <bool EVEN, typename T>
+__device__ __forceinline__ uint4 ce_load(const T* row, int at, int V) {          // at = g * W - off
+  constexpr int W = CeVec<T>::W;
+  if (EVEN || (at >= 0 && at + W <= V)) return *reinterpret_cast<const uint4*>(row + at);
+  float v[W];
+#pragma unroll
+  for (int j = 0; j < W; ++j) v[j] = at + j >= 0 && at + j < V ? to_f(row[at + j]) : -INFINITY;
+  return CeVec<T>::pack(v);
+}
+template <bool EVEN, typename T>
+__device__ __forceinline__ void ce_store(T* row, int at, int V, bool whole, const float (&v)[CeVec<T>::W]) {    // whole: a group of `row` is 16-byte aligned
+  constexpr int W = CeVec<T>::W;
+  if (EVEN || (whole && at >= 0 && at + W <= V)) { *reinterpret_cast<uint4*>(row + at) = CeVec<T>::pack(v); return; }
+#pragma unroll
+  for (int j = 0; j < W; ++j)
+    if (at + j >= 0 && at + j < V) row[at + j] = (T)v[j];
+}
+template <typename T>
+__device__ __forceinline__ int ce_offset(const T* row) { return int(reinterpret_cast<uintptr_t>(row) & 15) / (int)sizeof(T); }
+
+__device__ __forceinline__ int ce_target(const int64_t* targets, int row, int V, int* status) {
+  const long long t = targets[row];
+  if (t >= 0 && t < V) return (int)t;
+  if (status && threadIdx.x == 0) atomicExch(status, RTE_DEV_INDEX_OUT_OF_RANGE);
+  return 0;
+}
+// (maximum, sum of exponentials) of the row from every warp's
+template <int WARPS>
+__device__ __forceinline__ float ce_lse(const float (&red_m)[WARPS], const float (&red_s)[WARPS]) {
+  float mx = red_m[0], se = 0.f;
+#pragma unroll
+  for (int w = 1; w < WARPS; ++w) mx = fmaxf(mx, red_m[w]);
+#pragma unroll
+  for (int w = 0; w < WARPS; ++w) se += red_m[w] == -INFINITY ? 0.f : red_s[w] * __expf(red_m[w] - mx);      // (a warp without columns)
+  return mx + __logf(se);
+}
+
+// One CTA of THREADS per row, the row in registers (at most NV groups per thread): logits are read once, maximum and sum
+// of exponentials meet in one block reduction, the gradient is written from the exponentials.  Bound by HBM and, close
+// behind, by the instructions per element, so the CTA is as small as the row allows (many rows in flight per SM) and only
+// the group that holds the target looks for it.  With gradient, against a kernel that read a row three times with 256
+// threads: bf16 8192 x 2048 38.9 -> 20.5 us (67 MB), 8192 x 8192 84.9 -> 61.4 us.
+template <typename T, int THREADS, int NV, bool EVEN>
 __global__ void __launch_bounds__(THREADS)
 ce_row_kernel(const T* __restrict__ logits, int ldl, const int64_t* __restrict__ targets, const float* __restrict__ row_weight, int S,
               float* __restrict__ loss_tok, T* __restrict__ dlogits, int V, int* status) {
   rte::after_previous_grid();
   constexpr int W = CeVec<T>::W, WARPS = THREADS / 32;
   __shared__ float red_m[WARPS], red_s[WARPS], target_logit;
-  const int row = blockIdx.x, groups = V / W, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint4* lr = reinterpret_cast<const uint4*>(logits + (size_t)row * ldl);
-  uint4 raw[NV];
+  const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const T* lr = logits + (size_t)row * ldl;
+  const int off = EVEN ? 0 : ce_offset(lr), groups = (V + off + W - 1) / W;
+  float e[NV][W];
+  {
+    uint4 raw[NV];
 #pragma unroll
-  for (int i = 0; i < NV; ++i)
-    if (int(threadIdx.x) + i * THREADS < groups) raw[i] = lr[threadIdx.x + i * THREADS];
-  long long tgt = targets[row];
-  if (tgt < 0 || tgt >= V) {
-    if (status && threadIdx.x == 0) atomicExch(status, RTE_DEV_INDEX_OUT_OF_RANGE);
-    tgt = 0;
+    for (int i = 0; i < NV; ++i) {
+      const int g = int(threadIdx.x) + i * THREADS;
+      if (g < groups) raw[i] = ce_load<EVEN>(lr, g * W - off, V);
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+      if (int(threadIdx.x) + i * THREADS < groups) CeVec<T>::unpack(raw[i], e[i]);
   }
+  const int tgt = ce_target(targets, row, V, status), tg = (tgt + off) / W, tj = (tgt + off) % W;
   float m = -INFINITY;
 #pragma unroll
   for (int i = 0; i < NV; ++i)
     if (int(threadIdx.x) + i * THREADS < groups) {
-      float v[W];
-      CeVec<T>::unpack(raw[i], v);
 #pragma unroll
-      for (int j = 0; j < W; ++j) m = fmaxf(m, v[j]);
+      for (int j = 0; j < W; ++j) m = fmaxf(m, e[i][j]);
     }
   m = rte::warp_max(m);
   float s = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i)
     if (int(threadIdx.x) + i * THREADS < groups) {
-      float v[W];
-      CeVec<T>::unpack(raw[i], v);
-#pragma unroll
-      for (int j = 0; j < W; ++j) s += __expf(v[j] - m);
-      if (int(threadIdx.x) + i * THREADS == int(tgt) / W) {
+      if (int(threadIdx.x) + i * THREADS == tg) {
 #pragma unroll
         for (int j = 0; j < W; ++j)
-          if (j == int(tgt) % W) target_logit = v[j];
+          if (j == tj) target_logit = e[i][j];
       }
+#pragma unroll
+      for (int j = 0; j < W; ++j) s += e[i][j] = __expf(e[i][j] - m);
     }
   s = warp_sum(s);
   if (lane == 0) { red_m[warp] = m; red_s[warp] = s; }
   __syncthreads();
-  float mx = red_m[0];
-#pragma unroll
-  for (int w = 1; w < WARPS; ++w) mx = fmaxf(mx, red_m[w]);
-  float se = 0.f;
-#pragma unroll
-  for (int w = 0; w < WARPS; ++w) se += red_m[w] == -INFINITY ? 0.f : red_s[w] * __expf(red_m[w] - mx);      // (a warp without columns)
-  const float lse = mx + __logf(se);
+  const float lse = ce_lse(red_m, red_s);
   if (threadIdx.x == 0) loss_tok[row] = lse - target_logit;
   if (dlogits == nullptr) return;
-  const float wgt = row_weight[row / S];
-  uint4* dr = reinterpret_cast<uint4*>(dlogits + (size_t)row * ldl);
+  const float wgt = row_weight[row / S], scale = wgt * __expf(m - lse);
+  T* dr = dlogits + (size_t)row * ldl;
+  const bool whole = EVEN || ce_offset(dr) == off;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int g = int(threadIdx.x) + i * THREADS;
     if (g < groups) {
-      float v[W];
-      CeVec<T>::unpack(raw[i], v);
 #pragma unroll
-      for (int j = 0; j < W; ++j) v[j] = wgt * (__expf(v[j] - lse) - ((g * W + j) == tgt ? 1.f : 0.f));
-      dr[g] = CeVec<T>::pack(v);
+      for (int j = 0; j < W; ++j) e[i][j] *= scale;
+      if (g == tg) {
+#pragma unroll
+        for (int j = 0; j < W; ++j)
+          if (j == tj) e[i][j] -= wgt;
+      }
+      ce_store<EVEN>(dr, g * W - off, V, whole, e[i]);
     }
   }
 }
 
-// Rows that do not start on 16 bytes, a column count that is no multiple of a group, or rows longer than the registers
-// of 1024 threads: one CTA per row, the row read three times.
-template <typename T>
-__global__ void __launch_bounds__(256)
-ce_kernel(const T* __restrict__ logits, int ldl, const int64_t* __restrict__ targets, const float* __restrict__ row_weight, int S,
-          float* __restrict__ loss_tok, T* __restrict__ dlogits, int V, int* status) {
+// Rows of more than 16 KB: a CTA that holds such a row leaves its SM waiting between its phases (8192 x 32768 bf16 took
+// 369 us in registers of 1024 threads).  Five CTAs per SM stream their rows instead: one pass from HBM with a running
+// maximum and sum, and, for the gradient, a second one that finds the row in L2 (148 x 5 rows of 64 KB are 48 MB).
+// 8192 x 32768 with gradient: 299 -> 231 us (1.07 GB), loss alone 150 -> 133 us.
+template <typename T, bool EVEN>
+__global__ void __launch_bounds__(256, 5)
+ce_stream_kernel(const T* __restrict__ logits, int ldl, const int64_t* __restrict__ targets, const float* __restrict__ row_weight, int S,
+                 float* __restrict__ loss_tok, T* dlogits, int V, int* status) {
   rte::after_previous_grid();
-  __shared__ float red[32];
-  const int row = blockIdx.x;
+  constexpr int W = CeVec<T>::W, U = 4;
+  __shared__ float red_m[8], red_s[8];
+  const int row = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const T* lr = logits + (size_t)row * ldl;
-  long long tgt = targets[row];
-  if (tgt < 0 || tgt >= V) {
-    if (status && threadIdx.x == 0) atomicExch(status, RTE_DEV_INDEX_OUT_OF_RANGE);
-    tgt = 0;
+  const int off = EVEN ? 0 : ce_offset(lr), groups = (V + off + W - 1) / W;
+  const int tgt = ce_target(targets, row, V, status), tg = (tgt + off) / W, tj = (tgt + off) % W;
+  const float tl = threadIdx.x == 0 ? to_f(lr[tgt]) : 0.f;           // (before the gradient may overwrite the row)
+  float m = -INFINITY, s = 0.f;
+  for (int g0 = threadIdx.x; g0 < groups; g0 += 256 * U) {
+    uint4 raw[U];
+#pragma unroll
+    for (int i = 0; i < U; ++i)
+      if (g0 + 256 * i < groups) raw[i] = ce_load<EVEN>(lr, (g0 + 256 * i) * W - off, V);
+#pragma unroll
+    for (int i = 0; i < U; ++i)
+      if (g0 + 256 * i < groups) {
+        float v[W];
+        CeVec<T>::unpack(raw[i], v);
+        float gm = v[0];
+#pragma unroll
+        for (int j = 1; j < W; ++j) gm = fmaxf(gm, v[j]);
+        if (gm > m) { s *= __expf(m - gm); m = gm; }
+        if (m > -INFINITY) {
+#pragma unroll
+          for (int j = 0; j < W; ++j) s += __expf(v[j] - m);
+        }
+      }
   }
-  float mx = -INFINITY;
-  for (int c = threadIdx.x; c < V; c += blockDim.x) mx = fmaxf(mx, to_f(lr[c]));
-  mx = block_max(mx, red);
-  float se = 0.f;
-  for (int c = threadIdx.x; c < V; c += blockDim.x) se += __expf(to_f(lr[c]) - mx);
-  se = block_sum(se, red);
-  const float lse = mx + __logf(se), tl = to_f(lr[tgt]);
+  const float wm = rte::warp_max(m);
+  s = warp_sum(m == -INFINITY ? 0.f : s * __expf(m - wm));
+  if (lane == 0) { red_m[warp] = wm; red_s[warp] = s; }
+  __syncthreads();
+  const float lse = ce_lse(red_m, red_s);
   if (threadIdx.x == 0) loss_tok[row] = lse - tl;
   if (dlogits == nullptr) return;
-  __syncthreads();   // every thread has read lr[tgt] before an aliasing dlogits row is overwritten
   const float wgt = row_weight[row / S];
   T* dr = dlogits + (size_t)row * ldl;
-  for (int c = threadIdx.x; c < V; c += blockDim.x) dr[c] = (T)(wgt * (__expf(to_f(lr[c]) - lse) - (c == tgt ? 1.f : 0.f)));
+  const bool whole = EVEN || ce_offset(dr) == off;
+  for (int g0 = threadIdx.x; g0 < groups; g0 += 256 * U) {
+    uint4 raw[U];
+#pragma unroll
+    for (int i = 0; i < U; ++i)
+      if (g0 + 256 * i < groups) raw[i] = ce_load<EVEN>(lr, (g0 + 256 * i) * W - off, V);
+#pragma unroll
+    for (int i = 0; i < U; ++i) {
+      const int g = g0 + 256 * i;
+      if (g < groups) {
+        float v[W];
+        CeVec<T>::unpack(raw[i], v);
+#pragma unroll
+        for (int j = 0; j < W; ++j) v[j] = wgt * __expf(v[j] - lse);
+        if (g == tg) {
+#pragma unroll
+          for (int j = 0; j < W; ++j)
+            if (j == tj) v[j] -= wgt;
+        }
+        ce_store<EVEN>(dr, g * W - off, V, whole, v);
+      }
+    }
+  }
 }
 
+template <bool EVEN, typename T>
+int launch_ce_rows(const T* logits, int ldl, const int64_t* targets, const float* row_weight, int S, float* loss_tok, T* dlogits, int rows, int V,
+                   int* status, cudaStream_t st) {
+  constexpr int W = CeVec<T>::W;
+  const int groups = EVEN ? V / W : (V + 2 * (W - 1)) / W;
+#define RTE_CE(THREADS, NV) \
+  rte::launch(ce_row_kernel<T, THREADS, NV, EVEN>, rows, THREADS, 0, st, logits, ldl, targets, row_weight, S, loss_tok, dlogits, V, status)
+  if (groups <= 128) RTE_CE(64, 2);
+  else if (groups <= 256) RTE_CE(64, 4);
+  else if (groups <= 512) RTE_CE(128, 4);
+  else if (groups <= 1024) RTE_CE(256, 4);
+  else rte::launch(ce_stream_kernel<T, EVEN>, rows, 256, 0, st, logits, ldl, targets, row_weight, S, loss_tok, dlogits, V, status);
+#undef RTE_CE
+  RTE_LAUNCH_CHECK();
+  return RTE_OK;
+}
 template <typename T>
 int launch_ce(const T* logits, int ldl, const int64_t* targets, const float* row_weight, int S, float* loss_tok, T* dlogits, int rows, int V,
               int* status, cudaStream_t st) {
   constexpr int W = CeVec<T>::W;
-  const bool wide = V % W == 0 && ldl % W == 0 && ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(dlogits)) & 15) == 0;
-  const int groups = V / W;
-#define RTE_CE(THREADS, NV) rte::launch(ce_row_kernel<T, THREADS, NV>, rows, THREADS, 0, st, logits, ldl, targets, row_weight, S, loss_tok, dlogits, V, status)
-  if (!wide || groups > 8192) rte::launch(ce_kernel<T>, rows, 256, 0, st, logits, ldl, targets, row_weight, S, loss_tok, dlogits, V, status);
-  else if (groups <= 128) RTE_CE(64, 2);
-  else if (groups <= 256) RTE_CE(64, 4);
-  else if (groups <= 512) RTE_CE(128, 4);
-  else if (groups <= 1024) RTE_CE(256, 4);
-  else if (groups <= 2048) RTE_CE(512, 4);
-  else if (groups <= 4096) RTE_CE(1024, 4);
-  else RTE_CE(1024, 8);
-#undef RTE_CE
-  RTE_LAUNCH_CHECK();
-  return RTE_OK;
+  const bool even = V % W == 0 && ldl % W == 0 && ((reinterpret_cast<uintptr_t>(logits) | reinterpret_cast<uintptr_t>(dlogits)) & 15) == 0;
+  return (even ? launch_ce_rows<true, T> : launch_ce_rows<false, T>)(logits, ldl, targets, row_weight, S, loss_tok, dlogits, rows, V, status, st);
 }
 
 __global__ void segment_sum_kernel(const float* __restrict__ in, float* __restrict__ out, int n_seg, int seg_len) {

@@ -306,7 +306,8 @@ def test_pack_by_recipe_round_trip_and_grads():
 
 
 @pytest.mark.parametrize("rows,V,dtype", [(5, 8, torch.bfloat16), (33, 1000, torch.bfloat16), (64, 2056, torch.bfloat16), (7, 2047, torch.bfloat16),
-                                          (9, 32768, torch.bfloat16), (3, 65544, torch.bfloat16), (17, 4, torch.float32), (33, 2047, torch.float32),
+                                          (9, 32768, torch.bfloat16), (3, 65541, torch.bfloat16), (3, 8192, torch.bfloat16), (5, 8191, torch.bfloat16),
+                                          (11, 3, torch.bfloat16), (17, 4, torch.float32), (33, 2047, torch.float32),
                                           (20, 4100, torch.float32), (4, 32772, torch.float32)])
 def test_cross_entropy_row_widths(rows, V, dtype):
     """Widths around the register limits of the row kernel, and the rows that only the general kernel takes."""
