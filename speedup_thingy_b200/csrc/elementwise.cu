@@ -188,200 +188,150 @@ residual_rmsnorm_fwd_kernel(const float* __restrict__ base, const float* __restr
   }
 }
 
-// Backward.  y = xhat * w * (1 + fg) + fb with xhat = x * rstd.
-//   g  = dy * (1 + fg) * w          (gradient wrt xhat)
-//   dx = rstd * (g - xhat * mean(g * xhat)) + dres
-//   dw += dy * (1 + fg) * xhat,  dfg += dy * xhat * w,  dfb += dy
-// Each CTA walks rows blockIdx.x, blockIdx.x + gridDim.x, ...; column-wise partial sums for the
-// parameter gradients are kept in registers per warp, combined through shared memory at the end
-// and written to row blockIdx.x of the partial buffers (deterministic, no atomics).
-// FILM = false drops the FiLM accumulators (and a third of the registers) for the plain-norm launches.
-template <int NV, bool FILM>
-__global__ void __launch_bounds__(256, NV <= 4 ? 2 : 1)
+// RMSNorm(+FiLM) backward: dx = r * (g - xh * mean(g * xh)) + dres with xh = x * r, g = dy * (1 + gamma) * w, plus per-CTA
+// column sums for the weight and FiLM gradients, written to row blockIdx.x of the partial buffers (deterministic, no
+// atomics).  dy_splits > 1: dy32 holds that many split-K partials of dy, dy_stride floats apart, summed in split order.
+//
+// A thread owns four columns: blockDim.x threads span a row, blockDim.y rows run side by side, ROWS rows of each are in
+// flight.  The column sums are then 4 (FiLM: 12) registers per thread whatever the width, so the loads of all ROWS rows
+// (x, dy, residual gradient) fit ahead of the first use; a warp per row held d / 32 columns per lane and, beyond d = 512,
+// one row at a time (with the column sums, us: 8192 x 1024 80 -> 34, 16384 x 512 42 -> 34, 8192 x 512 15.8 -> 13.9, 64 x
+// 512 5.3 -> 3.4).  One barrier per ROWS rows joins the row sums of the warps.  FILM = false drops the FiLM accumulators.
+constexpr int RN_ROWS = 4;
+template <int N>
+__device__ __forceinline__ void warp_sums(float (&v)[N]) {
+#pragma unroll
+  for (int u = 0; u < N; ++u) v[u] = warp_sum(v[u]);
+}
+// four sums at once: the first two exchanges halve the values a lane carries (6 shuffles + 4 to spread, not 20)
+template <>
+__device__ __forceinline__ void warp_sums<4>(float (&v)[4]) {
+  const int lane = threadIdx.x & 31;
+  const float a0 = lane & 16 ? v[2] : v[0], a1 = lane & 16 ? v[3] : v[1], b0 = lane & 16 ? v[0] : v[2], b1 = lane & 16 ? v[1] : v[3];
+  const float c0 = a0 + __shfl_xor_sync(0xffffffffu, b0, 16), c1 = a1 + __shfl_xor_sync(0xffffffffu, b1, 16);
+  float t = (lane & 8 ? c1 : c0) + __shfl_xor_sync(0xffffffffu, lane & 8 ? c0 : c1, 8);
+  t += __shfl_xor_sync(0xffffffffu, t, 4);
+  t += __shfl_xor_sync(0xffffffffu, t, 2);
+  t += __shfl_xor_sync(0xffffffffu, t, 1);
+#pragma unroll
+  for (int u = 0; u < 4; ++u) v[u] = __shfl_sync(0xffffffffu, t, 8 * u);
+}
+
+template <int ROWS, bool FILM, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, ROWS == 1 ? 2 : 768 / BLOCK)
 rmsnorm_bwd_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ fg,
                    const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dy16,
                    const float* __restrict__ dy32, const float* __restrict__ dres, float* __restrict__ dx32,
                    __nv_bfloat16* __restrict__ dx16, float* __restrict__ dw_part, float* __restrict__ dg_part,
                    float* __restrict__ db_part, int rows, int d, int dy_splits, long long dy_stride) {
   rte::after_previous_grid();
-  // dy_splits > 1: dy32 holds that many split-K partials of dy, dy_stride floats apart, summed here in split order
-  extern __shared__ float sm[];   // [3][warps][d] when parameter gradients are requested
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  const int d4 = d >> 2;
-  constexpr int NF = FILM ? NV : 1;
-  float4 aw[NV], ag[NF], ab[NF];
-#pragma unroll
-  for (int i = 0; i < NV; ++i) aw[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-  for (int i = 0; i < NF; ++i) ag[i] = ab[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  const bool want_w = dw_part != nullptr, want_f = FILM && dg_part != nullptr;
-
-  int row = blockIdx.x * nwarp + warp;
-  const int stride = gridDim.x * nwarp;
-  if constexpr (!FILM && NV <= 4) {
-    // Two rows per trip with all loads of both rows issued before the first use: a warp that walks its rows one at a
-    // time keeps too few bytes in flight to cover the memory latency (the plain-norm launches of the hot pass).
-    for (; dy_splits <= 1 && row + stride < rows; row += 2 * stride) {
-      const int rw[2] = {row, row + stride};
-      float rr[2];
-      float4 xh[2][NV], g[2][NV], dyv[2][NV];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        rr[u] = rstd[rw[u]];
-        const float4* xr = reinterpret_cast<const float4*>(x + (size_t)rw[u] * d);
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-          const int c = lane + 32 * i;
-          if (c < d4) {
-            xh[u][i] = xr[c];
-            if (dy16) {
-              const uint2 pk = reinterpret_cast<const uint2*>(dy16 + (size_t)rw[u] * d)[c];
-              const float2 a = rte::unpack_bf16x2(pk.x), b = rte::unpack_bf16x2(pk.y);
-              dyv[u][i] = make_float4(a.x, a.y, b.x, b.y);
-            } else {
-              dyv[u][i] = reinterpret_cast<const float4*>(dy32 + (size_t)rw[u] * d)[c];
-            }
-          }
-        }
-      }
-      float dot[2] = {0.f, 0.f};
-#pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const int c = lane + 32 * i;
-        if (c < d4) {
-          const float4 ww = w ? reinterpret_cast<const float4*>(w)[c] : make_float4(1.f, 1.f, 1.f, 1.f);
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const float r = rr[u];
-            const float4 xv = xh[u][i], dv = dyv[u][i];
-            const float4 h = make_float4(xv.x * r, xv.y * r, xv.z * r, xv.w * r);
-            xh[u][i] = h;
-            if (want_w) { aw[i].x += dv.x * h.x; aw[i].y += dv.y * h.y; aw[i].z += dv.z * h.z; aw[i].w += dv.w * h.w; }
-            g[u][i] = make_float4(dv.x * ww.x, dv.y * ww.y, dv.z * ww.z, dv.w * ww.w);
-            dot[u] += g[u][i].x * h.x + g[u][i].y * h.y + g[u][i].z * h.z + g[u][i].w * h.w;
-          }
-        }
-      }
-      dot[0] = warp_sum(dot[0]) / (float)d;
-      dot[1] = warp_sum(dot[1]) / (float)d;
-      if (dres) {                                    // the residual gradient of both rows, loads first
-#pragma unroll
-        for (int u = 0; u < 2; ++u)
-#pragma unroll
-          for (int i = 0; i < NV; ++i) {
-            const int c = lane + 32 * i;
-            if (c < d4) dyv[u][i] = reinterpret_cast<const float4*>(dres + (size_t)rw[u] * d)[c];
-          }
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-          const int c = lane + 32 * i;
-          if (c < d4) {
-            const float r = rr[u], dt = dot[u];
-            float4 o = make_float4(r * (g[u][i].x - xh[u][i].x * dt), r * (g[u][i].y - xh[u][i].y * dt),
-                                   r * (g[u][i].z - xh[u][i].z * dt), r * (g[u][i].w - xh[u][i].w * dt));
-            if (dres) { const float4 t = dyv[u][i]; o.x += t.x; o.y += t.y; o.z += t.z; o.w += t.w; }
-            if (dx32) reinterpret_cast<float4*>(dx32 + (size_t)rw[u] * d)[c] = o;
-            if (dx16) {
-              uint2 pk = make_uint2(rte::pack_bf16x2(o.x, o.y), rte::pack_bf16x2(o.z, o.w));
-              reinterpret_cast<uint2*>(dx16 + (size_t)rw[u] * d)[c] = pk;
-            }
-          }
-        }
-    }
+  __shared__ float red[2][ROWS][BLOCK / 32];
+  __shared__ float4 comb[BLOCK];
+  const int c = threadIdx.x, d4 = d >> 2, nw = blockDim.x >> 5, gy = blockDim.y, warp0 = threadIdx.y * nw;
+  const bool on = c < d4;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 ww = !on ? zero : w ? reinterpret_cast<const float4*>(w)[c] : make_float4(1.f, 1.f, 1.f, 1.f);
+  float4 f1 = make_float4(1.f, 1.f, 1.f, 1.f);
+  if (FILM && fg && on) {
+    const float4 t = reinterpret_cast<const float4*>(fg)[c];
+    f1 = make_float4(1.f + t.x, 1.f + t.y, 1.f + t.z, 1.f + t.w);
   }
-  for (; row < rows; row += stride) {
-    const float r = rstd[row];
-    const float4* xr = reinterpret_cast<const float4*>(x + (size_t)row * d);
-    float4 xh[NV], g[NV];
-    float dot = 0.f;
+  const float4 wf = make_float4(ww.x * f1.x, ww.y * f1.y, ww.z * f1.z, ww.w * f1.w);
+  float4 aw = zero, ag = zero, ab = zero;
+  const int step = gridDim.x * gy;
+  int buf = 0;
+  for (int row0 = blockIdx.x * gy; row0 < rows; row0 += step * ROWS, buf ^= 1) {      // (the same trips for all rows of a CTA)
+    float4 xh[ROWS], g[ROWS], res[ROWS];
+    float r[ROWS], dot[ROWS];
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int c = lane + 32 * i;
-      if (c < d4) {
-        float4 xv = xr[c];
-        xh[i] = make_float4(xv.x * r, xv.y * r, xv.z * r, xv.w * r);
-        float4 dyv;
+    for (int u = 0; u < ROWS; ++u) {
+      const int row = row0 + threadIdx.y + u * step;
+      xh[u] = g[u] = res[u] = zero;
+      r[u] = 0.f;
+      if (row < rows && on) {
+        const size_t at = (size_t)row * d4 + c;
+        r[u] = rstd[row];
+        xh[u] = reinterpret_cast<const float4*>(x)[at];
         if (dy16) {
-          const uint2 pk = reinterpret_cast<const uint2*>(dy16 + (size_t)row * d)[c];
+          const uint2 pk = reinterpret_cast<const uint2*>(dy16)[at];
           const float2 a = rte::unpack_bf16x2(pk.x), b = rte::unpack_bf16x2(pk.y);
-          dyv = make_float4(a.x, a.y, b.x, b.y);
+          g[u] = make_float4(a.x, a.y, b.x, b.y);
         } else {
-          dyv = reinterpret_cast<const float4*>(dy32 + (size_t)row * d)[c];
+          g[u] = reinterpret_cast<const float4*>(dy32)[at];
+        }
+        if (dres) res[u] = reinterpret_cast<const float4*>(dres)[at];
+      }
+    }
+    if (dy_splits > 1) {
+#pragma unroll
+      for (int u = 0; u < ROWS; ++u) {
+        const int row = row0 + threadIdx.y + u * step;
+        if (row < rows && on)
           for (int s = 1; s < dy_splits; ++s) {
-            const float4 t = reinterpret_cast<const float4*>(dy32 + (size_t)s * dy_stride + (size_t)row * d)[c];
-            dyv.x += t.x; dyv.y += t.y; dyv.z += t.z; dyv.w += t.w;
+            const float4 t = reinterpret_cast<const float4*>(dy32 + (size_t)s * dy_stride)[(size_t)row * d4 + c];
+            g[u].x += t.x; g[u].y += t.y; g[u].z += t.z; g[u].w += t.w;
           }
-        }
-        float4 ww = w ? reinterpret_cast<const float4*>(w)[c] : make_float4(1.f, 1.f, 1.f, 1.f);
-        float4 f1 = make_float4(1.f, 1.f, 1.f, 1.f);
-        if (FILM && fg) {
-          const float4 t = reinterpret_cast<const float4*>(fg)[c];
-          f1 = make_float4(1.f + t.x, 1.f + t.y, 1.f + t.z, 1.f + t.w);
-        }
-        if (want_w) {
-          aw[i].x += dyv.x * f1.x * xh[i].x; aw[i].y += dyv.y * f1.y * xh[i].y;
-          aw[i].z += dyv.z * f1.z * xh[i].z; aw[i].w += dyv.w * f1.w * xh[i].w;
-        }
-        if constexpr (FILM) {
-          if (want_f) {
-            ag[i].x += dyv.x * xh[i].x * ww.x; ag[i].y += dyv.y * xh[i].y * ww.y;
-            ag[i].z += dyv.z * xh[i].z * ww.z; ag[i].w += dyv.w * xh[i].w * ww.w;
-            ab[i].x += dyv.x; ab[i].y += dyv.y; ab[i].z += dyv.z; ab[i].w += dyv.w;
-          }
-        }
-        g[i] = make_float4(dyv.x * f1.x * ww.x, dyv.y * f1.y * ww.y, dyv.z * f1.z * ww.z, dyv.w * f1.w * ww.w);
-        dot += g[i].x * xh[i].x + g[i].y * xh[i].y + g[i].z * xh[i].z + g[i].w * xh[i].w;
       }
     }
-    dot = warp_sum(dot) / (float)d;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int c = lane + 32 * i;
-      if (c < d4) {
-        float4 o = make_float4(r * (g[i].x - xh[i].x * dot), r * (g[i].y - xh[i].y * dot),
-                               r * (g[i].z - xh[i].z * dot), r * (g[i].w - xh[i].w * dot));
-        if (dres) {
-          const float4 t = reinterpret_cast<const float4*>(dres + (size_t)row * d)[c];
-          o.x += t.x; o.y += t.y; o.z += t.z; o.w += t.w;
-        }
-        if (dx32) reinterpret_cast<float4*>(dx32 + (size_t)row * d)[c] = o;
-        if (dx16) {
-          uint2 pk = make_uint2(rte::pack_bf16x2(o.x, o.y), rte::pack_bf16x2(o.z, o.w));
-          reinterpret_cast<uint2*>(dx16 + (size_t)row * d)[c] = pk;
-        }
-      }
-    }
-  }
-  if (!want_w && !want_f) return;
-  // combine the warps' column sums
-  float* sw = sm;
-  float* sg = sm + (size_t)nwarp * d;
-  float* sb = sm + (size_t)2 * nwarp * d;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int c = lane + 32 * i;
-    if (c < d4) {
-      if (want_w) reinterpret_cast<float4*>(sw + (size_t)warp * d)[c] = aw[i];
+    for (int u = 0; u < ROWS; ++u) {
+      float4& h = xh[u];
+      const float4 dv = g[u];
+      h.x *= r[u]; h.y *= r[u]; h.z *= r[u]; h.w *= r[u];
+      const float4 p = make_float4(dv.x * h.x, dv.y * h.y, dv.z * h.z, dv.w * h.w);
+      aw.x += p.x * f1.x; aw.y += p.y * f1.y; aw.z += p.z * f1.z; aw.w += p.w * f1.w;
       if constexpr (FILM) {
-        if (want_f) {
-          reinterpret_cast<float4*>(sg + (size_t)warp * d)[c] = ag[i];
-          reinterpret_cast<float4*>(sb + (size_t)warp * d)[c] = ab[i];
-        }
+        ag.x += p.x * ww.x; ag.y += p.y * ww.y; ag.z += p.z * ww.z; ag.w += p.w * ww.w;
+        ab.x += dv.x; ab.y += dv.y; ab.z += dv.z; ab.w += dv.w;
+      }
+      dot[u] = p.x * wf.x + p.y * wf.y + p.z * wf.z + p.w * wf.w;
+      g[u] = make_float4(dv.x * wf.x, dv.y * wf.y, dv.z * wf.z, dv.w * wf.w);
+    }
+    warp_sums(dot);
+    if (nw > 1) {
+      if ((c & 31) == 0) {
+#pragma unroll
+        for (int u = 0; u < ROWS; ++u) red[buf][u][warp0 + (c >> 5)] = dot[u];
+      }
+      __syncthreads();                                                 // (two buffers: the next trip's writes need no second barrier)
+#pragma unroll
+      for (int u = 0; u < ROWS; ++u) {
+        dot[u] = 0.f;
+        for (int k = 0; k < nw; ++k) dot[u] += red[buf][u][warp0 + k];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < ROWS; ++u) {
+      const int row = row0 + threadIdx.y + u * step;
+      if (row < rows && on) {
+        const size_t at = (size_t)row * d4 + c;
+        const float mean = dot[u] / (float)d, q = r[u];
+        const float4 o = make_float4(q * (g[u].x - xh[u].x * mean) + res[u].x, q * (g[u].y - xh[u].y * mean) + res[u].y,
+                                     q * (g[u].z - xh[u].z * mean) + res[u].z, q * (g[u].w - xh[u].w * mean) + res[u].w);
+        if (dx32) reinterpret_cast<float4*>(dx32)[at] = o;
+        if (dx16) reinterpret_cast<uint2*>(dx16)[at] = make_uint2(rte::pack_bf16x2(o.x, o.y), rte::pack_bf16x2(o.z, o.w));
       }
     }
   }
-  __syncthreads();
-  for (int c = threadIdx.x; c < d; c += blockDim.x) {
-    float tw = 0.f, tg = 0.f, tb = 0.f;
-    for (int k = 0; k < nwarp; ++k) {
-      if (want_w) tw += sw[(size_t)k * d + c];
-      if (want_f) { tg += sg[(size_t)k * d + c]; tb += sb[(size_t)k * d + c]; }
+  // column sums of the CTA's rows
+  auto write = [&](float* part, const float4& sum) {
+    float4 t = sum;
+    if (gy > 1) {
+      __syncthreads();
+      comb[threadIdx.y * blockDim.x + c] = sum;
+      __syncthreads();
+      if (threadIdx.y == 0)
+        for (int k = 1; k < gy; ++k) {
+          const float4 v = comb[k * blockDim.x + c];
+          t.x += v.x; t.y += v.y; t.z += v.z; t.w += v.w;
+        }
     }
-    if (want_w) dw_part[(size_t)blockIdx.x * d + c] = tw;
-    if (want_f) { dg_part[(size_t)blockIdx.x * d + c] = tg; db_part[(size_t)blockIdx.x * d + c] = tb; }
+    if (threadIdx.y == 0 && on) reinterpret_cast<float4*>(part + (size_t)blockIdx.x * d)[c] = t;
+  };
+  if (dw_part) write(dw_part, aw);
+  if (FILM && dg_part) {
+    write(dg_part, ag);
+    write(db_part, ab);
   }
 }
 
@@ -1082,44 +1032,28 @@ extern "C" int rte_rmsnorm_bwd_splits(const float* x, const float* w, const floa
                                                       dy_split_stride >= (int64_t)rows * d)));
   RTE_CHECK_ARG((dgamma_partial == nullptr) == (dbeta_partial == nullptr));
   if (d > 128 * RN_MAX_V4) return RTE_ERR_UNSUPPORTED;
-  const bool grads = dw_partial || dgamma_partial;
-  int grid = rte::ceil_div(rows, 8);
-  // one wave of CTAs (each writes one partial row): three fit an SM without FiLM accumulators at d <= 512
-  const int cap = 148 * ((film_gamma || dgamma_partial || d > 512) ? 2 : 3);
-  if (grid > cap) grid = cap;
+  const bool film = film_gamma || dgamma_partial, grads = dw_partial || dgamma_partial;
+  const int across = rte::ceil_div(d, 128) * 32, block = d <= 1024 ? 256 : 512, down = block / across;
+  // ROWS rows in flight per thread once every SM has its CTAs; fewer rows spread over as many CTAs as there are
+  const int most = 148 * (768 / block);
+  const bool few = rows <= most * down;
+  int grid = rte::ceil_div(rows, down * (few ? 1 : film ? 2 : RN_ROWS));
+  if (grid > most) grid = most;
   if (grads) {
     RTE_CHECK_ARG(max_partials >= 1);
     if (grid > max_partials) grid = max_partials;
   }
   if (n_partials) *n_partials = grid;
-  const size_t smem = grads ? (size_t)(dgamma_partial ? 3 : 1) * 8 * d * sizeof(float) : 0;
-#define RTE_RN_BWD(NV)                                                                                           \
-  do {                                                                                                           \
-    if (film_gamma || dgamma_partial) RTE_RN_BWD_F(NV, true); else RTE_RN_BWD_F(NV, false);                      \
-  } while (0)
-#define RTE_RN_BWD_F(NV, FILM)                                                                                   \
-  do {                                                                                                           \
-    if (smem > 48 * 1024) {                                                                                      \
-      static bool set = false;                                                                                   \
-      if (!set) {                                                                                                \
-        if (cudaFuncSetAttribute(rmsnorm_bwd_kernel<NV, FILM>, cudaFuncAttributeMaxDynamicSharedMemorySize,            \
-                                 200 * 1024) != cudaSuccess)                                                     \
-          return RTE_ERR_LAUNCH;                                                                                 \
-        set = true;                                                                                              \
-      }                                                                                                          \
-    }                                                                                                            \
-    rte::launch(rmsnorm_bwd_kernel<NV, FILM>, grid, 256, smem, ST(stream), x, w, film_gamma, rstd,                              \
-        reinterpret_cast<const __nv_bfloat16*>(dy_bf16), dy_f32, dres, dx_f32,                                   \
-        reinterpret_cast<__nv_bfloat16*>(dx_bf16), dw_partial, dgamma_partial, dbeta_partial, rows, d,           \
-        dy_splits, (long long)dy_split_stride);                                                                  \
-  } while (0)
-  if (d <= 128) RTE_RN_BWD(1);
-  else if (d <= 256) RTE_RN_BWD(2);
-  else if (d <= 512) RTE_RN_BWD(4);
-  else if (d <= 1024) RTE_RN_BWD(8);
-  else RTE_RN_BWD(16);
+#define RTE_RN_BWD(ROWS, FILM, BLOCK)                                                                            \
+  rte::launch(rmsnorm_bwd_kernel<ROWS, FILM, BLOCK>, grid, dim3(across, down), 0, ST(stream), x, w, film_gamma, rstd, \
+              reinterpret_cast<const __nv_bfloat16*>(dy_bf16), dy_f32, dres, dx_f32,                             \
+              reinterpret_cast<__nv_bfloat16*>(dx_bf16), dw_partial, dgamma_partial, dbeta_partial, rows, d,     \
+              dy_splits, (long long)dy_split_stride)
+#define RTE_RN_BWD_B(ROWS, FILM) do { if (block == 256) RTE_RN_BWD(ROWS, FILM, 256); else RTE_RN_BWD(ROWS, FILM, 512); } while (0)
+  if (few) { if (film) RTE_RN_BWD_B(1, true); else RTE_RN_BWD_B(1, false); }
+  else { if (film) RTE_RN_BWD_B(2, true); else RTE_RN_BWD_B(RN_ROWS, false); }
+#undef RTE_RN_BWD_B
 #undef RTE_RN_BWD
-#undef RTE_RN_BWD_F
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }

@@ -243,6 +243,33 @@ def test_rmsnorm_fwd_bwd(ops, rows, d):
             _close(dbt, fbr.grad, 1e-4, "film dbeta")
 
 
+@pytest.mark.parametrize("rows,d", [(1, 4), (1777, 132), (3557, 128), (889, 512), (1791, 1024), (297, 1028), (301, 2048)])
+@pytest.mark.parametrize("film", [False, True])
+def test_rmsnorm_bwd_row_and_column_edges(ops, rows, d, film):
+    """One row in flight and several, widths that do not fill a warp, more rows than the launch has CTAs (also with a cap)."""
+    g = torch.Generator().manual_seed(rows)
+    x, dy, dres = (torch.randn(rows, d, generator=g).to(DEV) for _ in range(3))
+    w, fg = torch.randn(d, generator=g).to(DEV), (0.1 * torch.randn(d, generator=g)).to(DEV)
+    xr, wr, fr = x.clone().requires_grad_(True), w.clone().requires_grad_(True), fg.clone().requires_grad_(True)
+    y = xr * torch.rsqrt(xr.pow(2).mean(-1, keepdim=True) + 1e-5) * wr
+    if film:
+        y = y * (1 + fr)
+    y.backward(dy.bfloat16().float())
+    rstd = torch.rsqrt(x.pow(2).mean(-1) + 1e-5)
+    for cap in (1184, 3):
+        dx, dx16 = torch.empty_like(x), torch.empty(rows, d, dtype=torch.bfloat16, device=DEV)
+        dw, dgm, dbt = (torch.empty(d, device=DEV) for _ in range(3))
+        part, pg, pb = (torch.empty(cap, d, device=DEV) for _ in range(3))
+        kw = dict(film_gamma=fg, dgamma_out=dgm, dbeta_out=dbt, partial_g=pg, partial_b=pb) if film else {}
+        ops.rmsnorm_bwd(x, w, rstd, dy.bfloat16(), dres, dx, dx16, dw, part, **kw)
+        _close(dx, xr.grad + dres, 1e-4, "dx")
+        _close(dx16, xr.grad + dres, 1e-2, "dx bf16")
+        _close(dw, wr.grad, 1e-4, "dw")
+        if film:
+            _close(dgm, fr.grad, 1e-4, "dgamma")
+            _close(dbt, dy.bfloat16().float().sum(0), 1e-4, "dbeta")
+
+
 @pytest.mark.parametrize("B,S,V", [(4, 16, 96), (8, 64, 2048), (3, 5, 1000)])
 def test_cross_entropy_fwd_bwd(ops, B, S, V):
     g = torch.Generator().manual_seed(V)
