@@ -459,9 +459,9 @@ struct CrossEntropy : Function<CrossEntropy> {
 Tensor cross_entropy(const Tensor& logits, const Tensor& targets) { return CrossEntropy::apply(logits, targets)[0]; }
 
 // --------------------------------------------------------------------------- packed SwiGLU FFN
-// The SwiGLU pass rides in the product's epilogue where that is faster: from about 14 M hidden activations on
-// (8192 x 2048: 53.6 -> 44.8 us forward, 8192 x 4096: 138 -> 110; 5000 x 1536: 24.8 -> 26.1, so not below).
-constexpr int64_t SWIGLU_FUSE_MIN = 14000000;
+// The SwiGLU pass rides in the product's epilogue where that is faster: from about 12 M hidden activations on
+// (us: 8192 x 2048 54.6 -> 45.6 forward, 6144 x 2048 42.3 -> 38.8; 4096 x 2048 even, 8192 x 1024 23.2 -> 25.7).
+constexpr int64_t SWIGLU_FUSE_MIN = 12000000;
 
 struct PackedFfn : Function<PackedFfn> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& wug, const Tensor& wdown) {

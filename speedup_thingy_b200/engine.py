@@ -935,8 +935,9 @@ class TrainEngine:
         return [f"router.{m}.{i}.{k}" for m in ("recipe_mlp", "depth_mlp") for i in (0, 2) for k in ("weight", "bias")]
 
     def _fuse_swiglu(self, rows: int) -> bool:
-        """SwiGLU inside the tcgen05 GEMM's epilogue only between the few-row kernel's range and the large-M range."""
-        return getattr(self.ops, "small_gemm_rows", 0) < rows <= self.swiglu_fuse_max_rows
+        """SwiGLU inside the tcgen05 GEMM's epilogue for large activations (swiglu_fuse_max_rows = 0: never).  Below the line
+        the separate pass finds its input in L2 and the product can take the kernels for few tiles."""
+        return self.swiglu_fuse_max_rows > 0 and rows * self.cfg.d_ff >= getattr(self.ops, "swiglu_fuse_min", 0)
 
     def _block_fwd(self, blk: _Block, x_in: torch.Tensor) -> torch.Tensor:
         o, cfg, p, sh, M = self.ops, self.cfg, self.params, self.shadow, blk.M

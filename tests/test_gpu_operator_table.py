@@ -378,7 +378,7 @@ def test_rope_and_attention_take_strided_views(layout, dtype):
     assert out.dtype == dtype and torch.allclose(out.cpu().float(), ref, atol=3e-2, rtol=3e-2)
 
 
-@pytest.mark.parametrize("N,d,m", [(7001, 64, 2048), (6900, 64, 2048)])
+@pytest.mark.parametrize("N,d,m", [(5901, 64, 2048), (5800, 64, 2048)])
 def test_packed_swiglu_on_both_sides_of_the_fusion_rule(N, d, m):
     gen = torch.Generator().manual_seed(N)
     x, wug, wd = (0.2 * torch.randn(*s, generator=gen) for s in ((N, d), (2 * m, d), (m, d)))
