@@ -25,9 +25,104 @@ __device__ __forceinline__ size_t key_of(const int32_t* rid, const int32_t* sid,
   return (size_t)rid[b] * K + sid[b];
 }
 
-// rstd per token, pooled = mean_S(rmsnorm(h0)) per sample, pa = pooled @ v[d:2d, :]
-__global__ void __launch_bounds__(NTHR)
+// rstd per token, pooled = mean_S(rmsnorm(h0)) per sample, pa = pooled @ v[d:2d, :].
+// A cluster of PREP_CTAS CTAs per sample: warps take tokens, a token stays in registers between its norm and the column
+// sums (one pass over h0), the CTAs add their column sums and products through distributed shared memory in rank order.
+// One CTA per sample left most SMs without work and read h0 twice: 32 x 256 x 1024 136 -> 29 us in the step (34 MB).
+constexpr int PREP_CTAS = 8;
+
+__device__ __forceinline__ float dsmem_read(const float* p, int rank) {
+  uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(p)), r;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(r) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+
+// NV float4 per lane hold a token (d <= 128 * NV, d % 4 == 0)
+template <int NV>
+__global__ void __cluster_dims__(PREP_CTAS, 1, 1) __launch_bounds__(NTHR)
 phi_prep_kernel(const float* __restrict__ h0, const float* __restrict__ v, const int32_t* __restrict__ rid,
+                const int32_t* __restrict__ sid, float* __restrict__ rstd, float* __restrict__ pooled,
+                float* __restrict__ pa, PhiDims D, float eps) {
+  rte::after_previous_grid();
+  extern __shared__ float sm[];            // warp sums [NTHR / 32][d] -> (row 0) this CTA's column sums; then pooled [d], products [m]
+  constexpr int WARPS = NTHR / 32;
+  float* ps = sm + (size_t)WARPS * D.d;
+  float* pj = ps + D.d;
+  const int b = blockIdx.x / PREP_CTAS, rank = blockIdx.x % PREP_CTAS, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d4 = D.d >> 2;
+  const float4* hb = reinterpret_cast<const float4*>(h0 + (size_t)b * D.S * D.d);
+  float4 acc[NV];
+#pragma unroll
+  for (int i = 0; i < NV; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s = rank * WARPS + warp; s < D.S; s += PREP_CTAS * WARPS) {
+    float4 x[NV];
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const int c = lane + 32 * i;
+      x[i] = c < d4 ? hb[(size_t)s * d4 + c] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) ss += x[i].x * x[i].x + x[i].y * x[i].y + x[i].z * x[i].z + x[i].w * x[i].w;
+    const float r = rsqrtf(rte::warp_sum(ss) / (float)D.d + eps);
+    if (lane == 0) rstd[(size_t)b * D.S + s] = r;
+#pragma unroll
+    for (int i = 0; i < NV; ++i) { acc[i].x += x[i].x * r; acc[i].y += x[i].y * r; acc[i].z += x[i].z * r; acc[i].w += x[i].w * r; }
+  }
+#pragma unroll
+  for (int i = 0; i < NV; ++i)
+    if (lane + 32 * i < d4) reinterpret_cast<float4*>(sm + (size_t)warp * D.d)[lane + 32 * i] = acc[i];
+  __syncthreads();
+  for (int c = threadIdx.x; c < D.d; c += NTHR) {
+    float t = sm[c];
+#pragma unroll
+    for (int w = 1; w < WARPS; ++w) t += sm[(size_t)w * D.d + c];
+    sm[c] = t;
+  }
+  cluster_sync();
+  // this CTA's slice of the columns: sum over the cluster, then its part of the product
+  const int per = rte::ceil_div(D.d, PREP_CTAS), c0 = rank * per, n = min(D.d, c0 + per) - c0;
+  for (int c = threadIdx.x; c < n; c += NTHR) {
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < PREP_CTAS; ++k) t += dsmem_read(sm + c0 + c, k);
+    t /= (float)D.S;
+    ps[c] = t;
+    pooled[(size_t)b * D.d + c0 + c] = t;
+  }
+  __syncthreads();
+  // threads = column groups x ranks: neighbouring threads read neighbouring elements of v
+  float* part = ps + rte::ceil_div(D.d, 4) * 4 + MMAX;                 // [NTHR]
+  const int mw = D.m <= 32 ? 32 : 64, j = threadIdx.x % mw, cg = threadIdx.x / mw, groups = NTHR / mw;
+  const float* v2 = v + (key_of(rid, sid, b, D.K) * 3 * D.d + D.d + c0) * D.m;
+  float t = 0.f;
+  if (j < D.m)
+    for (int c = cg; c < n; c += groups) t += ps[c] * v2[(size_t)c * D.m + j];
+  part[threadIdx.x] = t;
+  __syncthreads();
+  if (threadIdx.x < D.m) {
+    t = 0.f;
+    for (int k = 0; k < groups; ++k) t += part[k * mw + threadIdx.x];
+    pj[threadIdx.x] = t;
+  }
+  cluster_sync();
+  if (rank == 0 && threadIdx.x < D.m) {
+    t = 0.f;
+#pragma unroll
+    for (int k = 0; k < PREP_CTAS; ++k) t += dsmem_read(pj + threadIdx.x, k);
+    pa[(size_t)b * D.m + threadIdx.x] = t;
+  }
+  cluster_sync();                          // (no CTA leaves while another reads its shared memory)
+}
+inline size_t prep_smem(int d) { return ((size_t)(NTHR / 32 + 1) * d + 4 + MMAX + NTHR) * sizeof(float); }
+
+// The same for widths the registers do not hold (d > 2048 or d % 4 != 0) or rows off 16 bytes: one CTA per sample.
+__global__ void __launch_bounds__(NTHR)
+phi_prep_any_kernel(const float* __restrict__ h0, const float* __restrict__ v, const int32_t* __restrict__ rid,
                 const int32_t* __restrict__ sid, float* __restrict__ rstd, float* __restrict__ pooled,
                 float* __restrict__ pa, PhiDims D, float eps) {
   rte::after_previous_grid();
@@ -269,11 +364,12 @@ __device__ __forceinline__ void mma_3xtf32(float (&c)[4], const uint32_t (&ah)[4
   mma_tf32(c, ah, bh);
 }
 
-// Both kernels read their operands with 16-byte loads.  Inside a chunk of 32 reduction indices the mma's logical
-// k-slot (step s, slot t or t+4) is mapped to the physical index 8t+s or 8t+4+s: lane t then needs the eight
-// consecutive values [8t, 8t+8) of its rows -- two float4 -- and A and B use the same permutation, so the sum is
-// unchanged.
-struct Frag8 { float4 lo, hi; };     // physical indices 8t..8t+3 and 8t+4..8t+7 of one row
+// The kernels read their operands with 16-byte loads.  Inside a chunk of 32 reduction indices the mma's logical k-slot
+// (step s, slot t or t+4) is mapped to a physical index, the same for A and B, so the sum is unchanged.  Where the
+// reduction runs over columns (da, act) it is 4t+s or 16+4t+s: a quad reads 64 contiguous bytes per load, whole sectors
+// (with 8t+s the two loads each touched every sector of the line).  Where it runs over the rank (out, dz) it is 8t+s or
+// 8t+4+s.
+struct Frag8 { float4 lo, hi; };     // the values of slots t and t+4, four steps each
 __device__ __forceinline__ Frag8 load8(const float* p, bool ok) {
   Frag8 f;
   if (ok) { f.lo = *reinterpret_cast<const float4*>(p); f.hi = *reinterpret_cast<const float4*>(p + 4); }
@@ -282,52 +378,93 @@ __device__ __forceinline__ Frag8 load8(const float* p, bool ok) {
 }
 __device__ __forceinline__ float pick(const float4& v, int s) { return s == 0 ? v.x : s == 1 ? v.y : s == 2 ? v.z : v.w; }
 
-// da[tok, j] = silu'(act[tok,j]) * sum_c dupd[tok,c] * u[j,c]:  M = tokens, N = rank, K = d  (d % 32 == 0).
-// Eight warps = 2 token tiles x 4 column groups; group ng owns rank columns [8ng, 8ng+8) and [8ng+32, 8ng+40).
-__global__ void __launch_bounds__(NTHR)
+__device__ __forceinline__ Frag8 load_k32(const float* row, int t, bool ok) {
+  Frag8 f;
+  if (ok) { f.lo = *reinterpret_cast<const float4*>(row + 4 * t); f.hi = *reinterpret_cast<const float4*>(row + 16 + 4 * t); }
+  else { f.lo = make_float4(0.f, 0.f, 0.f, 0.f); f.hi = f.lo; }
+  return f;
+}
+struct SplitA { uint32_t h[4][4], l[4][4]; };         // [step][fragment register]
+__device__ __forceinline__ SplitA split_a(const Frag8& x0, const Frag8& x1) {
+  SplitA a;
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    split_tf32(pick(x0.lo, s), a.h[s][0], a.l[s][0]);
+    split_tf32(pick(x1.lo, s), a.h[s][1], a.l[s][1]);
+    split_tf32(pick(x0.hi, s), a.h[s][2], a.l[s][2]);
+    split_tf32(pick(x1.hi, s), a.h[s][3], a.l[s][3]);
+  }
+  return a;
+}
+__device__ __forceinline__ void mma_chunk(float (&c)[4], const SplitA& a, const Frag8& w) {
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    uint32_t f[2], fl[2];
+    split_tf32(pick(w.lo, s), f[0], fl[0]);
+    split_tf32(pick(w.hi, s), f[1], fl[1]);
+    mma_3xtf32(c, a.h[s], a.l[s], f, fl);
+  }
+}
+
+// The two products of 32 tokens with a key's weights over all d columns (d % 32 == 0): warps = 2 token tiles x 4 slices of
+// the reduction (chunks of 32 columns, every fourth one), each with all ranks (NT tiles of 8), so a token's values are
+// loaded and split once; the slices meet in shared memory in slice order.  (With the ranks divided over the warps instead,
+// every warp read and split every token: bound by L1.)
+constexpr int KSLICES = 4;
+template <int NT>
+__device__ __forceinline__ bool sum_slices(float (&acc)[NT][4], float (&red)[KSLICES - 1][2][NT * 4][32], int mt, int slice, int lane) {
+  if (slice > 0) {
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) red[slice - 1][mt][4 * i + e][lane] = acc[i][e];
+  }
+  __syncthreads();
+  if (slice > 0) return false;
+#pragma unroll
+  for (int k = 0; k < KSLICES - 1; ++k)
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][e] += red[k][mt][4 * i + e][lane];
+  return true;
+}
+
+// da[tok, j] = silu'(act[tok,j]) * sum_c dupd[tok,c] * u[j,c]:  M = tokens, N = rank, K = d.  32 x 256 x 1024, rank 32:
+// 41 -> 27 us in the step.
+template <int NT>
+__global__ void __launch_bounds__(NTHR, 2)
 phi_da_mma_kernel(const float* __restrict__ dupd, const float* __restrict__ act, const float* __restrict__ u,
                   const int32_t* __restrict__ rid, const int32_t* __restrict__ sid, float* __restrict__ da, PhiDims D) {
   rte::after_previous_grid();
+  __shared__ float red[KSLICES - 1][2][NT * 4][32];
   const int tiles = rte::ceil_div(D.S, TT);
   const int b = blockIdx.x / tiles, tok0 = (blockIdx.x % tiles) * TT;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  const int mt = warp & 1, ng = warp >> 1;
-  const int n_tiles = rte::ceil_div(D.m, 8);
-  if (ng >= n_tiles) return;                         // warp-uniform; the kernel has no barrier
-  const bool two = ng + 4 < n_tiles;
+  const int mt = warp & 1, slice = warp >> 1;
   const float* ub = u + key_of(rid, sid, b, D.K) * D.m * D.d;
   const int r0 = tok0 + mt * 16 + g, r1 = r0 + 8;
   const bool ok0 = r0 < D.S, ok1 = r1 < D.S;
-  const float* a0p = dupd + ((size_t)b * D.S + (ok0 ? r0 : 0)) * D.d + 8 * t;
-  const float* a1p = dupd + ((size_t)b * D.S + (ok1 ? r1 : 0)) * D.d + 8 * t;
-  const int j0 = ng * 8 + g, j1 = j0 + 32;
-  const bool okb0 = j0 < D.m, okb1 = two && j1 < D.m;
-  const float* b0p = ub + (size_t)(okb0 ? j0 : 0) * D.d + 8 * t;
-  const float* b1p = ub + (size_t)(okb1 ? j1 : 0) * D.d + 8 * t;
-  float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 2
-  for (int k0 = 0; k0 < D.d; k0 += 32) {
-    const Frag8 x0 = load8(a0p + k0, ok0), x1 = load8(a1p + k0, ok1);
-    const Frag8 w0 = load8(b0p + k0, okb0);
-    Frag8 w1;
-    if (two) w1 = load8(b1p + k0, okb1);
+  const float* a0p = dupd + ((size_t)b * D.S + (ok0 ? r0 : 0)) * D.d;
+  const float* a1p = dupd + ((size_t)b * D.S + (ok1 ? r1 : 0)) * D.d;
+  float acc[NT][4];
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      uint32_t a[4], al[4], f[2], fl[2];
-      split_tf32(pick(x0.lo, s), a[0], al[0]);
-      split_tf32(pick(x1.lo, s), a[1], al[1]);
-      split_tf32(pick(x0.hi, s), a[2], al[2]);
-      split_tf32(pick(x1.hi, s), a[3], al[3]);
-      split_tf32(pick(w0.lo, s), f[0], fl[0]);
-      split_tf32(pick(w0.hi, s), f[1], fl[1]);
-      mma_3xtf32(c0, a, al, f, fl);
-      if (two) {
-        split_tf32(pick(w1.lo, s), f[0], fl[0]);
-        split_tf32(pick(w1.hi, s), f[1], fl[1]);
-        mma_3xtf32(c1, a, al, f, fl);
-      }
+  for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+  for (int k0 = 32 * slice; k0 < D.d; k0 += 32 * KSLICES) {
+    const Frag8 x0 = load_k32(a0p + k0, t, ok0), x1 = load_k32(a1p + k0, t, ok1);
+    Frag8 w[NT <= 4 ? NT : 1];
+    if constexpr (NT <= 4) {                          // all weights requested ahead of the first product
+#pragma unroll
+      for (int i = 0; i < NT; ++i) w[i] = load_k32(ub + (size_t)min(8 * i + g, D.m - 1) * D.d + k0, t, 8 * i + g < D.m);
+    }
+    const SplitA a = split_a(x0, x1);
+#pragma unroll
+    for (int i = 0; i < NT; ++i) {
+      if constexpr (NT <= 4) mma_chunk(acc[i], a, w[i]);
+      else mma_chunk(acc[i], a, load_k32(ub + (size_t)min(8 * i + g, D.m - 1) * D.d + k0, t, 8 * i + g < D.m));
     }
   }
+  if (!sum_slices<NT>(acc, red, mt, slice, lane)) return;
   auto put = [&](int row, int col, float x) {
     if (row < D.S && col < D.m) {
       const size_t idx = ((size_t)b * D.S + row) * D.m + col;
@@ -335,98 +472,67 @@ phi_da_mma_kernel(const float* __restrict__ dupd, const float* __restrict__ act,
       da[idx] = x * sg * (1.f + av * (1.f - sg));
     }
   };
-  const int col0 = ng * 8 + 2 * t;
-  put(r0, col0, c0[0]); put(r0, col0 + 1, c0[1]); put(r1, col0, c0[2]); put(r1, col0 + 1, c0[3]);
-  if (two) { put(r0, col0 + 32, c1[0]); put(r0, col0 + 33, c1[1]); put(r1, col0 + 32, c1[2]); put(r1, col0 + 33, c1[3]); }
+#pragma unroll
+  for (int i = 0; i < NT; ++i) {
+    const int col = 8 * i + 2 * t;
+    put(r0, col, acc[i][0]); put(r0, col + 1, acc[i][1]); put(r1, col, acc[i][2]); put(r1, col + 1, acc[i][3]);
+  }
 }
 
 // ---- Forward products on tensor cores.  They need the reduction index contiguous per output column, i.e. the
 // TRANSPOSED parameters: wt = vt [m][keys*3d] (vt[j][key*3d + c] = v[key][c][j]) followed by
 // ut [d][keys*m] (ut[c][key*m + j] = u[key][j][c]), refreshed once per step by rte_macro_phi_prepare.
 
-// act[tok, j] = pa[b, j] + rstd[tok] * (h0 @ v1)[tok, j] + (hx @ v3)[tok, j]:  M = tokens, N = rank, K = d (d % 32 == 0).
-// Same warp layout as phi_da_mma_kernel; two accumulators per rank tile (with hx == h0, the hot path, the v1 and v3
-// slices share the A fragments; otherwise the v3 slice gets fragments of its own).
-template <bool OWN3>
-__global__ void __launch_bounds__(NTHR)
+// act[tok, j] = pa[b, j] + rstd[tok] * (h0 @ v1)[tok, j] + (hx @ v3)[tok, j]:  M = tokens, N = rank, K = d.  With hx == h0,
+// the hot path, both products share the token fragments.  32 x 256 x 1024, rank 32: 85 -> 47 us in the step.
+template <int NT, bool OWN3>
+__global__ void __launch_bounds__(NTHR, NT <= 4 ? 2 : 1)
 phi_act_mma_kernel(const float* __restrict__ h0, const float* __restrict__ hx, const float* __restrict__ rstd,
                    const float* __restrict__ pa, const float* __restrict__ vt, long long vt_ld,
                    const int32_t* __restrict__ rid, const int32_t* __restrict__ sid, float* __restrict__ act, PhiDims D) {
   rte::after_previous_grid();
+  __shared__ float red[KSLICES - 1][2][NT * 4][32];
   const int tiles = rte::ceil_div(D.S, TT);
   const int b = blockIdx.x / tiles, tok0 = (blockIdx.x % tiles) * TT;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  const int mt = warp & 1, ng = warp >> 1;
-  const int n_tiles = rte::ceil_div(D.m, 8);
-  if (ng >= n_tiles) return;                         // warp-uniform; the kernel has no barrier
-  const bool two = ng + 4 < n_tiles;
-  const size_t koff = key_of(rid, sid, b, D.K) * 3 * D.d;
+  const int mt = warp & 1, slice = warp >> 1;
+  const float* vk = vt + key_of(rid, sid, b, D.K) * 3 * D.d;
   const int r0 = tok0 + mt * 16 + g, r1 = r0 + 8;
   const bool ok0 = r0 < D.S, ok1 = r1 < D.S;
-  const float* a0p = h0 + ((size_t)b * D.S + (ok0 ? r0 : 0)) * D.d + 8 * t;
-  const float* a1p = h0 + ((size_t)b * D.S + (ok1 ? r1 : 0)) * D.d + 8 * t;
-  // OWN3: hx is a different tensor than h0 (a compile-time switch: the hot path keeps its register footprint)
-  const float* x0p = hx + ((size_t)b * D.S + (ok0 ? r0 : 0)) * D.d + 8 * t;
-  const float* x1p = hx + ((size_t)b * D.S + (ok1 ? r1 : 0)) * D.d + 8 * t;
-  const int j0 = ng * 8 + g, j1 = j0 + 32;
-  const bool okb0 = j0 < D.m, okb1 = two && j1 < D.m;
-  const float* b0p = vt + (size_t)(okb0 ? j0 : 0) * vt_ld + koff + 8 * t;
-  const float* b1p = vt + (size_t)(okb1 ? j1 : 0) * vt_ld + koff + 8 * t;
-  float p1[2][4], p3[2][4];
+  const size_t row0 = ((size_t)b * D.S + (ok0 ? r0 : 0)) * D.d, row1 = ((size_t)b * D.S + (ok1 ? r1 : 0)) * D.d;
+  float p1[NT][4], p3[NT][4];
 #pragma unroll
-  for (int q = 0; q < 2; ++q)
+  for (int i = 0; i < NT; ++i)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) p1[q][e] = p3[q][e] = 0.f;
-#pragma unroll 2
-  for (int k0 = 0; k0 < D.d; k0 += 32) {
-    const Frag8 x0 = load8(a0p + k0, ok0), x1 = load8(a1p + k0, ok1);
-    Frag8 z0 = x0, z1 = x1;                          // A operand of the v3 slice
-    if constexpr (OWN3) { z0 = load8(x0p + k0, ok0); z1 = load8(x1p + k0, ok1); }
-    const Frag8 w1 = load8(b0p + k0, okb0), w3 = load8(b0p + 2 * D.d + k0, okb0);
-    Frag8 y1, y3;
-    if (two) { y1 = load8(b1p + k0, okb1); y3 = load8(b1p + 2 * D.d + k0, okb1); }
+    for (int e = 0; e < 4; ++e) p1[i][e] = p3[i][e] = 0.f;
+#pragma unroll 1
+  for (int k0 = 32 * slice; k0 < D.d; k0 += 32 * KSLICES) {
+    const SplitA a = split_a(load_k32(h0 + row0 + k0, t, ok0), load_k32(h0 + row1 + k0, t, ok1));
 #pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      uint32_t a[4], al[4], c[4], cl[4], f[2], fl[2];
-      split_tf32(pick(x0.lo, s), a[0], al[0]);
-      split_tf32(pick(x1.lo, s), a[1], al[1]);
-      split_tf32(pick(x0.hi, s), a[2], al[2]);
-      split_tf32(pick(x1.hi, s), a[3], al[3]);
-      if constexpr (OWN3) {
-        split_tf32(pick(z0.lo, s), c[0], cl[0]);
-        split_tf32(pick(z1.lo, s), c[1], cl[1]);
-        split_tf32(pick(z0.hi, s), c[2], cl[2]);
-        split_tf32(pick(z1.hi, s), c[3], cl[3]);
-      } else {
+    for (int i = 0; i < NT; ++i) mma_chunk(p1[i], a, load_k32(vk + (size_t)min(8 * i + g, D.m - 1) * vt_ld + k0, t, 8 * i + g < D.m));
+    if constexpr (OWN3) {
+      const SplitA c = split_a(load_k32(hx + row0 + k0, t, ok0), load_k32(hx + row1 + k0, t, ok1));
 #pragma unroll
-        for (int e = 0; e < 4; ++e) { c[e] = a[e]; cl[e] = al[e]; }
-      }
-      split_tf32(pick(w1.lo, s), f[0], fl[0]);
-      split_tf32(pick(w1.hi, s), f[1], fl[1]);
-      mma_3xtf32(p1[0], a, al, f, fl);
-      split_tf32(pick(w3.lo, s), f[0], fl[0]);
-      split_tf32(pick(w3.hi, s), f[1], fl[1]);
-      mma_3xtf32(p3[0], c, cl, f, fl);
-      if (two) {
-        split_tf32(pick(y1.lo, s), f[0], fl[0]);
-        split_tf32(pick(y1.hi, s), f[1], fl[1]);
-        mma_3xtf32(p1[1], a, al, f, fl);
-        split_tf32(pick(y3.lo, s), f[0], fl[0]);
-        split_tf32(pick(y3.hi, s), f[1], fl[1]);
-        mma_3xtf32(p3[1], c, cl, f, fl);
-      }
+      for (int i = 0; i < NT; ++i) mma_chunk(p3[i], c, load_k32(vk + (size_t)min(8 * i + g, D.m - 1) * vt_ld + 2 * D.d + k0, t, 8 * i + g < D.m));
+    } else {
+#pragma unroll
+      for (int i = 0; i < NT; ++i) mma_chunk(p3[i], a, load_k32(vk + (size_t)min(8 * i + g, D.m - 1) * vt_ld + 2 * D.d + k0, t, 8 * i + g < D.m));
     }
   }
   const float rs0 = ok0 ? rstd[(size_t)b * D.S + r0] : 0.f, rs1 = ok1 ? rstd[(size_t)b * D.S + r1] : 0.f;
-  auto put = [&](int row, int col, float rs, float a1v, float a3v) {
-    if (row < D.S && col < D.m) act[((size_t)b * D.S + row) * D.m + col] = pa[(size_t)b * D.m + col] + rs * a1v + a3v;
+#pragma unroll
+  for (int i = 0; i < NT; ++i) {
+    p1[i][0] = rs0 * p1[i][0] + p3[i][0]; p1[i][1] = rs0 * p1[i][1] + p3[i][1];
+    p1[i][2] = rs1 * p1[i][2] + p3[i][2]; p1[i][3] = rs1 * p1[i][3] + p3[i][3];
+  }
+  if (!sum_slices<NT>(p1, red, mt, slice, lane)) return;
+  auto put = [&](int row, int col, float x) {
+    if (row < D.S && col < D.m) act[((size_t)b * D.S + row) * D.m + col] = pa[(size_t)b * D.m + col] + x;
   };
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    if (q == 1 && !two) break;
-    const int col0 = ng * 8 + 2 * t + 32 * q;
-    put(r0, col0, rs0, p1[q][0], p3[q][0]); put(r0, col0 + 1, rs0, p1[q][1], p3[q][1]);
-    put(r1, col0, rs1, p1[q][2], p3[q][2]); put(r1, col0 + 1, rs1, p1[q][3], p3[q][3]);
+  for (int i = 0; i < NT; ++i) {
+    const int col = 8 * i + 2 * t;
+    put(r0, col, p1[i][0]); put(r0, col + 1, p1[i][1]); put(r1, col, p1[i][2]); put(r1, col + 1, p1[i][3]);
   }
 }
 
@@ -524,116 +630,161 @@ phi_out_mma_kernel(const float* __restrict__ h0, const float* __restrict__ act, 
   }
 }
 
-// Per-sample parameter gradients of u, gain, bias:  pu[b][j,c], pg[b][c], pb[b][c].
-__global__ void __launch_bounds__(NTHR)
-phi_pu_kernel(const float* __restrict__ h0, const float* __restrict__ act, const float* __restrict__ dupd,
-              float* __restrict__ pu, float* __restrict__ pg, float* __restrict__ pb, PhiDims D) {
+// Per-sample parameter gradients, all of them in one launch over the tokens of a sample (M = columns c, K = tokens s):
+//   pu[b][j, c]  = sum_s silu(act[s,j]) * dupd[s,c],   pg[b][c] = sum_s dupd[s,c] * h0[s,c],   pb[b][c] = sum_s dupd[s,c]
+//   pv[b][c', j]: c' <  d  sum_s h0[s,c]*rstd[s] * da[s,j]
+//                 c' < 2d  pooled[b,c] * sum_s da[s,j]
+//                 else     sum_s hx[s,c] * da[s,j]                  (hx == h0 on the hot path: the operand is split once)
+// 3xTF32 products: a warp owns 16 columns and all ranks (NT tiles of 8); its A operand is the transpose of [token, column]
+// rows read straight from global memory (eight neighbouring columns per token: whole sectors), da and silu(act) of
+// PG_TOK tokens at a time are staged in shared memory for the CTA's eight warps.  The scalar kernels this replaces were
+// bound by four shared-memory reads per product term: 32 x 256 x 1024, rank 32: 307 -> 92 us in the step.
+constexpr int PG_TOK = 64;
+
+template <int NT, bool OWN3>
+__global__ void __launch_bounds__(NTHR, NT <= 4 ? 2 : 1)
+phi_param_grads_kernel(const float* __restrict__ h0, const float* __restrict__ hx, const float* __restrict__ rstd, const float* __restrict__ pooled,
+                       const float* __restrict__ act, const float* __restrict__ dupd, const float* __restrict__ da, float* __restrict__ pu,
+                       float* __restrict__ pg, float* __restrict__ pb, float* __restrict__ pv, PhiDims D) {
   rte::after_previous_grid();
-  extern __shared__ float ssa[];     // [S][m]
-  const int cblocks = rte::ceil_div(D.d, NTHR);
-  const int b = blockIdx.x / cblocks, c = (blockIdx.x % cblocks) * NTHR + threadIdx.x;
-  for (int i = threadIdx.x; i < D.S * D.m; i += NTHR) ssa[i] = rte::silu_f(act[(size_t)b * D.S * D.m + i]);
-  __syncthreads();
-  if (c >= D.d) return;
-  float au[MMAX];
+  constexpr int LD = 8 * NT + 8;                                       // (+8: the four tokens of a fragment fall into different banks)
+  __shared__ float sda[PG_TOK * LD], ssa[PG_TOK * LD], srs[PG_TOK];
+  __shared__ float part[NTHR], stot[8 * NT];                           // column sums of da: per thread, then whole
+  const int cblocks = rte::ceil_div(D.d, 128);
+  const int b = blockIdx.x / cblocks, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+  const int c0 = (blockIdx.x % cblocks) * 128 + warp * 16 + g, c1 = c0 + 8;      // this lane's rows of the products
+  const bool ok0 = c0 < D.d, ok1 = c1 < D.d;
+  const size_t base = (size_t)b * D.S * D.d;
+  float uu[NT][4], v1[NT][4], v3[NT][4];
 #pragma unroll
-  for (int j = 0; j < MMAX; ++j) au[j] = 0.f;
-  float ag = 0.f, ab = 0.f;
-  if (D.m % 4 == 0) {                 // four ranks per shared-memory read
-    const int m4 = D.m >> 2;
+  for (int i = 0; i < NT; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) uu[i][e] = v1[i][e] = v3[i][e] = 0.f;
+  float ag0 = 0.f, ag1 = 0.f, ab0 = 0.f, ab1 = 0.f, colsum = 0.f;
+  for (int s0 = 0; s0 < D.S; s0 += PG_TOK) {
+    const int n = min(PG_TOK, D.S - s0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < PG_TOK * 8 * NT; i += NTHR) {
+      const int s = i / (8 * NT), j = i % (8 * NT);
+      const bool in = s < n && j < D.m;
+      const size_t at = ((size_t)b * D.S + s0 + s) * D.m + j;
+      sda[s * LD + j] = in ? da[at] : 0.f;
+      ssa[s * LD + j] = in ? rte::silu_f(act[at]) : 0.f;
+    }
+    for (int i = threadIdx.x; i < PG_TOK; i += NTHR) srs[i] = i < n ? rstd[(size_t)b * D.S + s0 + i] : 0.f;
+    __syncthreads();
+    for (int s = threadIdx.x / (8 * NT); s < n; s += NTHR / (8 * NT)) colsum += sda[s * LD + threadIdx.x % (8 * NT)];
 #pragma unroll 2
-    for (int s = 0; s < D.S; ++s) {
-      const size_t idx = ((size_t)b * D.S + s) * D.d + c;
-      const float du = dupd[idx];
-      ag += du * h0[idx];
-      ab += du;
-      const float4* row = reinterpret_cast<const float4*>(ssa + s * D.m);
+    for (int k = 0; k < n; k += 8) {
+      const int sa = s0 + k + t, sb = sa + 4;
+      const bool ta = sa < D.S, tb = sb < D.S;
+      float h[4], du[4], x3[4];
+      const size_t ra = base + (size_t)sa * D.d, rb = base + (size_t)sb * D.d;
+      h[0] = ta && ok0 ? h0[ra + c0] : 0.f;  h[1] = ta && ok1 ? h0[ra + c1] : 0.f;
+      h[2] = tb && ok0 ? h0[rb + c0] : 0.f;  h[3] = tb && ok1 ? h0[rb + c1] : 0.f;
+      du[0] = ta && ok0 ? dupd[ra + c0] : 0.f;  du[1] = ta && ok1 ? dupd[ra + c1] : 0.f;
+      du[2] = tb && ok0 ? dupd[rb + c0] : 0.f;  du[3] = tb && ok1 ? dupd[rb + c1] : 0.f;
+      if constexpr (OWN3) {
+        x3[0] = ta && ok0 ? hx[ra + c0] : 0.f;  x3[1] = ta && ok1 ? hx[ra + c1] : 0.f;
+        x3[2] = tb && ok0 ? hx[rb + c0] : 0.f;  x3[3] = tb && ok1 ? hx[rb + c1] : 0.f;
+      }
+      ag0 += du[0] * h[0] + du[2] * h[2];
+      ag1 += du[1] * h[1] + du[3] * h[3];
+      ab0 += du[0] + du[2];
+      ab1 += du[1] + du[3];
+      const float rsa = srs[k + t], rsb = srs[k + t + 4];
+      uint32_t dh[4], dl[4], h1[4], l1[4], h3[4], l3[4];
 #pragma unroll
-      for (int j4 = 0; j4 < MMAX / 4; ++j4) {
-        if (j4 < m4) {
-          const float4 sv = row[j4];
-          au[4 * j4] += sv.x * du; au[4 * j4 + 1] += sv.y * du; au[4 * j4 + 2] += sv.z * du; au[4 * j4 + 3] += sv.w * du;
-        }
+      for (int e = 0; e < 4; ++e) {
+        split_tf32(du[e], dh[e], dl[e]);
+        split_tf32(h[e] * (e < 2 ? rsa : rsb), h1[e], l1[e]);
+        if constexpr (OWN3) split_tf32(x3[e], h3[e], l3[e]);
+        else split_tf32(h[e], h3[e], l3[e]);
+      }
+#pragma unroll
+      for (int i = 0; i < NT; ++i) {
+        uint32_t fh[2], fl[2];
+        split_tf32(ssa[(k + t) * LD + 8 * i + g], fh[0], fl[0]);
+        split_tf32(ssa[(k + t + 4) * LD + 8 * i + g], fh[1], fl[1]);
+        mma_3xtf32(uu[i], dh, dl, fh, fl);
+        split_tf32(sda[(k + t) * LD + 8 * i + g], fh[0], fl[0]);
+        split_tf32(sda[(k + t + 4) * LD + 8 * i + g], fh[1], fl[1]);
+        mma_3xtf32(v1[i], h1, l1, fh, fl);
+        mma_3xtf32(v3[i], h3, l3, fh, fl);
       }
     }
-  } else {
-    for (int s = 0; s < D.S; ++s) {
-      const size_t idx = ((size_t)b * D.S + s) * D.d + c;
-      const float du = dupd[idx];
-      ag += du * h0[idx];
-      ab += du;
-#pragma unroll
-      for (int j = 0; j < MMAX; ++j) if (j < D.m) au[j] += ssa[s * D.m + j] * du;
-    }
   }
-  pg[(size_t)b * D.d + c] = ag;
-  pb[(size_t)b * D.d + c] = ab;
+  part[threadIdx.x] = colsum;
+  __syncthreads();
+  if (threadIdx.x < 8 * NT) {
+    float a = 0.f;
 #pragma unroll
-  for (int j = 0; j < MMAX; ++j) if (j < D.m) pu[((size_t)b * D.m + j) * D.d + c] = au[j];
-}
-
-// Per-sample gradient of v:  pv[b][c', j] for c' in [0, 3d):
-//   c' <  d  : sum_s h0[s,c]*rstd[s] * da[s,j]
-//   c' < 2d  : pooled[b,c] * sum_s da[s,j]
-//   else     : sum_s hx[s,c] * da[s,j]          (hx == h0 on the hot path)
-constexpr int PV_ROWS = 32;       // rows of v per CTA (one 128-byte line of h0 per token)
-
-__global__ void __launch_bounds__(NTHR)
-phi_pv_kernel(const float* __restrict__ h0, const float* __restrict__ hx, const float* __restrict__ rstd,
-              const float* __restrict__ pooled, const float* __restrict__ da, float* __restrict__ pv, PhiDims D) {
-  rte::after_previous_grid();
-  extern __shared__ float sm[];      // sda[S][m], rs[S], sx[S][PV_ROWS], sx3[S][PV_ROWS]
-  float* sda = sm;
-  float* rs = sm + D.S * D.m;
-  float* sx = rs + D.S;
-  float* sx3 = sx + D.S * PV_ROWS;
-  constexpr int ROWS = PV_ROWS;
-  const int rblocks = rte::ceil_div(D.d, ROWS);
-  const int b = blockIdx.x / rblocks, c0 = (blockIdx.x % rblocks) * ROWS;
-  for (int i = threadIdx.x; i < D.S * D.m; i += NTHR) sda[i] = da[(size_t)b * D.S * D.m + i];
-  for (int i = threadIdx.x; i < D.S; i += NTHR) rs[i] = rstd[(size_t)b * D.S + i];
-  for (int i = threadIdx.x; i < D.S * ROWS; i += NTHR) {
-    const int s = i / ROWS, r = i % ROWS;
-    sx[i] = (c0 + r < D.d) ? h0[((size_t)b * D.S + s) * D.d + c0 + r] : 0.f;
-    sx3[i] = (c0 + r < D.d) ? hx[((size_t)b * D.S + s) * D.d + c0 + r] : 0.f;
+    for (int k = 0; k < NTHR / (8 * NT); ++k) a += part[k * 8 * NT + threadIdx.x];
+    stot[threadIdx.x] = a;
   }
   __syncthreads();
+  ag0 += __shfl_xor_sync(0xffffffffu, ag0, 1); ag0 += __shfl_xor_sync(0xffffffffu, ag0, 2);
+  ag1 += __shfl_xor_sync(0xffffffffu, ag1, 1); ag1 += __shfl_xor_sync(0xffffffffu, ag1, 2);
+  ab0 += __shfl_xor_sync(0xffffffffu, ab0, 1); ab0 += __shfl_xor_sync(0xffffffffu, ab0, 2);
+  ab1 += __shfl_xor_sync(0xffffffffu, ab1, 1); ab1 += __shfl_xor_sync(0xffffffffu, ab1, 2);
+  if (t == 0 && ok0) { pg[(size_t)b * D.d + c0] = ag0; pb[(size_t)b * D.d + c0] = ab0; }
+  if (t == 0 && ok1) { pg[(size_t)b * D.d + c1] = ag1; pb[(size_t)b * D.d + c1] = ab1; }
   float* pvb = pv + (size_t)b * 3 * D.d * D.m;
-  for (int o = threadIdx.x; o < ROWS * D.m; o += NTHR) {
-    const int r = o / D.m, j = o % D.m, c = c0 + r;
-    if (c >= D.d) continue;
-    float a1 = 0.f, a2 = 0.f, a3 = 0.f;
-    for (int s = 0; s < D.S; ++s) {
-      const float dv = sda[s * D.m + j], x = sx[s * ROWS + r];
-      a1 += x * rs[s] * dv;
-      a2 += dv;
-      a3 += sx3[s * ROWS + r] * dv;
-    }
-    pvb[(size_t)c * D.m + j] = a1;
-    pvb[(size_t)(D.d + c) * D.m + j] = pooled[(size_t)b * D.d + c] * a2;
-    pvb[(size_t)(2 * D.d + c) * D.m + j] = a3;
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const int c = half ? c1 : c0;
+    if (!(half ? ok1 : ok0)) continue;
+    const float pool = pooled[(size_t)b * D.d + c];
+#pragma unroll
+    for (int i = 0; i < NT; ++i)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int j = 8 * i + 2 * t + q;
+        if (j < D.m) {
+          pu[((size_t)b * D.m + j) * D.d + c] = uu[i][2 * half + q];
+          pvb[(size_t)c * D.m + j] = v1[i][2 * half + q];
+          pvb[(size_t)(D.d + c) * D.m + j] = pool * stot[j];
+          pvb[(size_t)(2 * D.d + c) * D.m + j] = v3[i][2 * half + q];
+        }
+      }
   }
 }
 
-// sda[b, j] = sum_s da[b,s,j]  ->  dpool[b, c] = (1/S) * sum_j sda[b,j] * v2[c,j]
+// sda[b, j] = sum_s da[b,s,j]  ->  dpool[b, c] = (1/S) * sum_j sda[b,j] * v2[c,j]      (a CTA per sample and 256 columns)
 __global__ void __launch_bounds__(NTHR)
 phi_dpool_kernel(const float* __restrict__ da, const float* __restrict__ v, const int32_t* __restrict__ rid,
                  const int32_t* __restrict__ sid, float* __restrict__ dpool, PhiDims D) {
   rte::after_previous_grid();
-  __shared__ float ssum[MMAX];
-  const int b = blockIdx.x;
-  for (int j = threadIdx.x; j < D.m; j += NTHR) {
-    float a = 0.f;
-    for (int s = 0; s < D.S; ++s) a += da[((size_t)b * D.S + s) * D.m + j];
-    ssum[j] = a;
+  __shared__ float part[NTHR], ssum[MMAX];
+  const int cblocks = rte::ceil_div(D.d, NTHR);
+  const int b = blockIdx.x / cblocks, c = (blockIdx.x % cblocks) * NTHR + threadIdx.x;
+  const int mw = D.m <= 32 ? 32 : 64, j = threadIdx.x % mw, groups = NTHR / mw;
+  float a = 0.f;
+  if (j < D.m) {
+#pragma unroll 8
+    for (int s = threadIdx.x / mw; s < D.S; s += groups) a += da[((size_t)b * D.S + s) * D.m + j];
+  }
+  part[threadIdx.x] = a;
+  __syncthreads();
+  if (threadIdx.x < D.m) {
+    a = 0.f;
+    for (int k = 0; k < groups; ++k) a += part[k * mw + threadIdx.x];
+    ssum[threadIdx.x] = a;
   }
   __syncthreads();
-  const float* v2 = v + (key_of(rid, sid, b, D.K) * 3 * D.d + D.d) * D.m;
-  for (int c = threadIdx.x; c < D.d; c += NTHR) {
-    float a = 0.f;
-    for (int j = 0; j < D.m; ++j) a += ssum[j] * v2[(size_t)c * D.m + j];
-    dpool[(size_t)b * D.d + c] = a / (float)D.S;
+  if (c >= D.d) return;
+  const float* v2 = v + (key_of(rid, sid, b, D.K) * 3 * D.d + D.d + c) * D.m;
+  a = 0.f;
+  if (D.m % 4 == 0 && (reinterpret_cast<uintptr_t>(v) & 15) == 0) {
+#pragma unroll 8
+    for (int q = 0; q < D.m; q += 4) {
+      const float4 w = *reinterpret_cast<const float4*>(v2 + q);
+      a += ssum[q] * w.x + ssum[q + 1] * w.y + ssum[q + 2] * w.z + ssum[q + 3] * w.w;
+    }
+  } else {
+    for (int q = 0; q < D.m; ++q) a += ssum[q] * v2[q];
   }
+  dpool[(size_t)b * D.d + c] = a / (float)D.S;
 }
 
 // dhx[tok,:] += da @ v3^T;  dh0[tok,:] += rmsnorm_backward(da @ v1^T + dpool[b,:])     (one warp per token; dhx may be dh0)
@@ -881,28 +1032,55 @@ phi_dz_mma_kernel(const float* __restrict__ h0, const float* __restrict__ rstd, 
   }
 }
 
-// out[key][e] = sum over samples b with key(b) == key, in sample order, of partial[b][e]   (blockIdx.y = key)
+// out[key][e] = sum over samples b with key(b) == key, in sample order, of partial[b][e]   (blockIdx.y = key), for the
+// four parameters in one launch.  The member list is compacted by ballots: one thread walking the samples' ids waited
+// for memory B times before the first addition (32 samples x 1024, rank 32: four launches of 75 us together -> one of 17).
+struct KeyJobs { const float* partial[4]; float* out[4]; long long elems[4]; int first_block[5]; };
+
 __global__ void __launch_bounds__(NTHR)
-phi_reduce_keys_kernel(const float* __restrict__ partial, const int32_t* __restrict__ rid, const int32_t* __restrict__ sid,
-                       float* __restrict__ out, int B, int K, long long elems) {
+phi_reduce_keys_kernel(const KeyJobs jobs, const int32_t* __restrict__ rid, const int32_t* __restrict__ sid, int B, int K) {
   rte::after_previous_grid();
   __shared__ int members[1024];
-  __shared__ int n_members;
-  const int key = blockIdx.y;
-  if (threadIdx.x == 0) {
-    int n = 0;
-    for (int b = 0; b < B && n < 1024; ++b)
-      if (rid[b] * K + sid[b] == key) members[n++] = b;
-    n_members = n;
+  __shared__ int warp_count[NTHR / 32];
+  const int key = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int n = 0;
+  for (int b0 = 0; b0 < B; b0 += NTHR) {
+    const int b = b0 + threadIdx.x;
+    const bool mine = b < B && rid[b] * K + sid[b] == key;
+    const unsigned votes = __ballot_sync(0xffffffffu, mine);
+    if (lane == 0) warp_count[warp] = __popc(votes);
+    __syncthreads();
+    int at = n + __popc(votes & ((1u << lane) - 1));
+#pragma unroll
+    for (int w = 0; w < NTHR / 32; ++w) {
+      if (w < warp) at += warp_count[w];
+      n += warp_count[w];
+    }
+    if (mine) members[at] = b;
+    __syncthreads();
   }
-  __syncthreads();
-  const long long e = blockIdx.x * (long long)NTHR + threadIdx.x;
+  int q = 0;
+  while (q < 3 && (int)blockIdx.x >= jobs.first_block[q + 1]) ++q;
+  const long long elems = jobs.elems[q], e = ((long long)blockIdx.x - jobs.first_block[q]) * (4 * NTHR) + 4 * threadIdx.x;
+  const float* partial = jobs.partial[q];
+  float* out = jobs.out[q] + (size_t)key * elems;
   if (e >= elems) return;
-  float acc = 0.f;
-  const int n = n_members;
+  if (elems % 4 == 0 && ((reinterpret_cast<uintptr_t>(partial) | reinterpret_cast<uintptr_t>(jobs.out[q])) & 15) == 0) {
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int i = 0; i < n; ++i) {
+      const float4 x = *reinterpret_cast<const float4*>(partial + (size_t)members[i] * elems + e);
+      acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
+    }
+    *reinterpret_cast<float4*>(out + e) = acc;
+  } else {
+    for (long long f = e; f < min(elems, e + 4); ++f) {
+      float acc = 0.f;
 #pragma unroll 4
-  for (int i = 0; i < n; ++i) acc += partial[(size_t)members[i] * elems + e];
-  out[(size_t)key * elems + e] = acc;
+      for (int i = 0; i < n; ++i) acc += partial[(size_t)members[i] * elems + f];
+      out[f] = acc;
+    }
+  }
 }
 
 // Mean-squared-error pieces of the consistency term (macro.py:359): g[i] = coef * (a[i] - b[i]) and one partial sum of
@@ -970,13 +1148,31 @@ int phi_fwd_impl(const float* h0, const float* hx, const rte_phi_params* p, cons
   // `act` doubles as the home of pa (B*m floats) is NOT safe; pa lives at the tail of `pooled`'s
   // companion: callers give pooled >= B*d + B*m floats.
   float* pa = pooled + (size_t)B * d;
-  rte::launch(phi_prep_kernel, B, NTHR, (size_t)(S + d) * sizeof(float), ST(stream), h0, p->v, recipe_id, stride_id, rstd, pooled, pa, D, eps);
+  if (d % 4 == 0 && d <= 2048 && (reinterpret_cast<uintptr_t>(h0) & 15) == 0) {
+#define RTE_PREP(NV)                                                                                                         \
+  do {                                                                                                                       \
+    if (prep_smem(128 * NV) > 48 * 1024 &&                                                                                   \
+        cudaFuncSetAttribute(phi_prep_kernel<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_smem(128 * NV)) != cudaSuccess) \
+      return RTE_ERR_LAUNCH;                                                                                                 \
+    rte::launch(phi_prep_kernel<NV>, B * PREP_CTAS, NTHR, prep_smem(d), ST(stream), h0, p->v, recipe_id, stride_id, rstd, pooled, pa, D, eps); \
+  } while (0)
+    if (d <= 128) RTE_PREP(1);
+    else if (d <= 256) RTE_PREP(2);
+    else if (d <= 512) RTE_PREP(4);
+    else if (d <= 1024) RTE_PREP(8);
+    else RTE_PREP(16);
+#undef RTE_PREP
+  } else {
+    rte::launch(phi_prep_any_kernel, B, NTHR, (size_t)(S + d) * sizeof(float), ST(stream), h0, p->v, recipe_id, stride_id, rstd, pooled, pa, D, eps);
+  }
   RTE_LAUNCH_CHECK();
   if (phi_tensor_path(p, h0, out, act, d, m) && (reinterpret_cast<uintptr_t>(hx) & 15) == 0) {
     const long long vt_ld = (long long)p->n_keys * 3 * d, ut_ld = (long long)p->n_keys * m;
     const float* ut = p->wt + (size_t)m * vt_ld;
-    if (hx != h0) rte::launch(phi_act_mma_kernel<true>, B * tiles, NTHR, 0, ST(stream), h0, hx, rstd, pa, p->wt, vt_ld, recipe_id, stride_id, act, D);
-    else rte::launch(phi_act_mma_kernel<false>, B * tiles, NTHR, 0, ST(stream), h0, hx, rstd, pa, p->wt, vt_ld, recipe_id, stride_id, act, D);
+#define RTE_ACT(NT, OWN3) rte::launch(phi_act_mma_kernel<NT, OWN3>, B * tiles, NTHR, 0, ST(stream), h0, hx, rstd, pa, p->wt, vt_ld, recipe_id, stride_id, act, D)
+    if (m <= 32) { if (hx != h0) RTE_ACT(4, true); else RTE_ACT(4, false); }
+    else { if (hx != h0) RTE_ACT(8, true); else RTE_ACT(8, false); }
+#undef RTE_ACT
     RTE_LAUNCH_CHECK();
     if (m <= 32)
       rte::launch(phi_out_mma_kernel<0, 1>, B * tiles, NTHR, 0, ST(stream), h0, act, p->gain, ut, ut_ld, p->bias, p->scale, recipe_id,
@@ -1064,10 +1260,11 @@ int phi_bwd_data_impl(const float* h0, const float* dout, const rte_phi_params* 
   const bool mma = d % 32 == 0 && m % 4 == 0 && ((reinterpret_cast<uintptr_t>(scratch) | reinterpret_cast<uintptr_t>(h0) |
                    reinterpret_cast<uintptr_t>(dh0) | reinterpret_cast<uintptr_t>(dhx) | reinterpret_cast<uintptr_t>(p->u) |
                    reinterpret_cast<uintptr_t>(p->v)) & 15) == 0;
-  if (mma) rte::launch(phi_da_mma_kernel, B * tiles, NTHR, 0, ST(stream), x.dupd, act, p->u, recipe_id, stride_id, x.da, D);
+  if (mma && m <= 32) rte::launch(phi_da_mma_kernel<4>, B * tiles, NTHR, 0, ST(stream), x.dupd, act, p->u, recipe_id, stride_id, x.da, D);
+  else if (mma) rte::launch(phi_da_mma_kernel<8>, B * tiles, NTHR, 0, ST(stream), x.dupd, act, p->u, recipe_id, stride_id, x.da, D);
   else rte::launch(phi_da_kernel, B * tiles, NTHR, 0, ST(stream), x.dupd, act, p->u, recipe_id, stride_id, x.da, D);
   RTE_LAUNCH_CHECK();
-  rte::launch(phi_dpool_kernel, B, NTHR, 0, ST(stream), x.da, p->v, recipe_id, stride_id, x.dpool, D);
+  rte::launch(phi_dpool_kernel, B * rte::ceil_div(d, NTHR), NTHR, 0, ST(stream), x.da, p->v, recipe_id, stride_id, x.dpool, D);
   RTE_LAUNCH_CHECK();
   if (mma && m <= 32) rte::launch(phi_dz_mma_kernel<1>, B * tiles, NTHR, 0, ST(stream), h0, rstd, x.da, x.dpool, p->v, recipe_id, stride_id, dh0, dhx, D);
   else if (mma) rte::launch(phi_dz_mma_kernel<2>, B * tiles, NTHR, 0, ST(stream), h0, rstd, x.da, x.dpool, p->v, recipe_id, stride_id, dh0, dhx, D);
@@ -1098,30 +1295,15 @@ int phi_bwd_params_impl(const float* h0, const float* hx, const int32_t* recipe_
   if (m > MMAX || B > 1024) return RTE_ERR_UNSUPPORTED;
   PhiDims D{B, S, d, m, K_strides};
   const PhiBwdScratch x = phi_scratch(scratch, B, S, d, m);
-  const size_t smem_pu = (size_t)S * m * sizeof(float);
-  const size_t smem_pv = ((size_t)S * m + S + 2 * (size_t)S * PV_ROWS) * sizeof(float);
-  if (smem_pu > 48 * 1024 || smem_pv > 48 * 1024) {
-    static bool set = false;
-    if (!set) {
-      if (cudaFuncSetAttribute(phi_pu_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess ||
-          cudaFuncSetAttribute(phi_pv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
-        return RTE_ERR_LAUNCH;
-      set = true;
-    }
-  }
-  rte::launch(phi_pu_kernel, B * rte::ceil_div(d, NTHR), NTHR, smem_pu, ST(stream), h0, act, x.dupd, x.pu, x.pg, x.pb, D);
+  const int grid = B * rte::ceil_div(d, 128);
+#define RTE_PG(NT, OWN3) rte::launch(phi_param_grads_kernel<NT, OWN3>, grid, NTHR, 0, ST(stream), h0, hx, rstd, pooled, act, x.dupd, x.da, x.pu, x.pg, x.pb, x.pv, D)
+  if (m <= 32) { if (hx != h0) RTE_PG(4, true); else RTE_PG(4, false); }
+  else { if (hx != h0) RTE_PG(8, true); else RTE_PG(8, false); }
+#undef RTE_PG
   RTE_LAUNCH_CHECK();
-  rte::launch(phi_pv_kernel, B * rte::ceil_div(d, PV_ROWS), NTHR, smem_pv, ST(stream), h0, hx, rstd, pooled, x.da, x.pv, D);
-  RTE_LAUNCH_CHECK();
-  const int n_keys = R * K_strides;
-  const long long eu = (long long)m * d, ev = (long long)3 * d * m, ed = d;
-  rte::launch(phi_reduce_keys_kernel, dim3((unsigned)rte::ceil_div64(eu, NTHR), n_keys), NTHR, 0, ST(stream), x.pu, recipe_id, stride_id, g->u, B, K_strides, eu);
-  RTE_LAUNCH_CHECK();
-  rte::launch(phi_reduce_keys_kernel, dim3((unsigned)rte::ceil_div64(ev, NTHR), n_keys), NTHR, 0, ST(stream), x.pv, recipe_id, stride_id, g->v, B, K_strides, ev);
-  RTE_LAUNCH_CHECK();
-  rte::launch(phi_reduce_keys_kernel, dim3((unsigned)rte::ceil_div64(ed, NTHR), n_keys), NTHR, 0, ST(stream), x.pg, recipe_id, stride_id, g->gain, B, K_strides, ed);
-  RTE_LAUNCH_CHECK();
-  rte::launch(phi_reduce_keys_kernel, dim3((unsigned)rte::ceil_div64(ed, NTHR), n_keys), NTHR, 0, ST(stream), x.pb, recipe_id, stride_id, g->bias, B, K_strides, ed);
+  KeyJobs jobs = {{x.pv, x.pu, x.pg, x.pb}, {g->v, g->u, g->gain, g->bias}, {(long long)3 * d * m, (long long)m * d, d, d}, {0}};
+  for (int q = 0; q < 4; ++q) jobs.first_block[q + 1] = jobs.first_block[q] + (int)rte::ceil_div64(jobs.elems[q], 4 * NTHR);
+  rte::launch(phi_reduce_keys_kernel, dim3((unsigned)jobs.first_block[4], R * K_strides), NTHR, 0, ST(stream), jobs, recipe_id, stride_id, B, K_strides);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
