@@ -10,14 +10,37 @@ namespace {
 
 constexpr int NTHR = 256;
 
+__device__ __forceinline__ float4 load4(const float* p, bool wide) {
+  return wide ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+
+// pooled[b,c] = mean over s.  CTA = one sample x 128 columns; its eight warps take every eighth token, eight loads in flight
+// each (a thread per column walking all S tokens: 32 x 256 x 1024 50 -> 19 us for 34 MB).
 __global__ void __launch_bounds__(NTHR)
 pool_kernel(const float* __restrict__ h0, float* __restrict__ pooled, int S, int d) {
   rte::after_previous_grid();
-  const int b = blockIdx.y, c = blockIdx.x * NTHR + threadIdx.x;
-  if (c >= d) return;
-  float acc = 0.f;
-  for (int s = 0; s < S; ++s) acc += h0[((size_t)b * S + s) * d + c];
-  pooled[(size_t)b * d + c] = acc / (float)S;
+  __shared__ float4 part[NTHR];
+  const int b = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 128 + 4 * lane;
+  const bool wide = (reinterpret_cast<uintptr_t>(h0) & 15) == 0;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (c < d) {
+    const float* p = h0 + (size_t)b * S * d + c;
+#pragma unroll 8
+    for (int s = warp; s < S; s += NTHR / 32) {
+      const float4 x = load4(p + (size_t)s * d, wide);
+      acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
+    }
+  }
+  part[threadIdx.x] = acc;
+  __syncthreads();
+  if (threadIdx.x < 128) {
+    const int col = blockIdx.x * 128 + threadIdx.x;
+    const float* q = reinterpret_cast<const float*>(part) + threadIdx.x;
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < NTHR / 32; ++w) t += q[128 * w];
+    if (col < d) pooled[(size_t)b * d + col] = t / (float)S;
+  }
 }
 
 __device__ __forceinline__ int argmax_lowest(const float* v, int n) {
@@ -34,9 +57,10 @@ __device__ __forceinline__ void softmax_small(const float* logits, float* probs,
   for (int i = 0; i < n; ++i) probs[i] *= inv;
 }
 
-// Hidden layer of one router MLP for 16 samples x 32 hidden rows per CTA: every weight row is read once per
-// 16 samples (kept in registers as float4 chunks) and dotted with the samples' pooled vectors held in smem.
-constexpr int RH_SAMPLES = 16, RH_ROWS = 32;
+// Hidden layer of one router MLP for 16 samples x 32 hidden rows per CTA: the samples' pooled vectors sit in shared memory
+// and a warp dots its four weight rows with them together, so one shared read feeds four products (a row at a time the
+// kernel was bound by those reads: 32 samples x 1024 -> 1024 46 -> 20 us).
+constexpr int RH_SAMPLES = 16, RH_ROWS = 32, RH_PER_WARP = RH_ROWS / (NTHR / 32);
 __global__ void __launch_bounds__(NTHR)
 router_hidden_kernel(const float* __restrict__ pooled, const float* __restrict__ w0a, const float* __restrict__ b0a,
                      float* __restrict__ prea, const float* __restrict__ w0b, const float* __restrict__ b0b,
@@ -47,31 +71,40 @@ router_hidden_kernel(const float* __restrict__ pooled, const float* __restrict__
   const float* b0 = blockIdx.z == 0 ? b0a : b0b;
   float* pre = blockIdx.z == 0 ? prea : preb;
   const int s0 = blockIdx.y * RH_SAMPLES, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < RH_SAMPLES * d; i += NTHR) {
-    const int s = s0 + i / d;
-    xs[i] = s < B ? pooled[(size_t)s * d + i % d] : 0.f;
-  }
+  const int d4 = d >> 2, n = min(RH_SAMPLES, B - s0) * d4;          // (the samples' vectors are contiguous)
+  const bool wide = (reinterpret_cast<uintptr_t>(pooled) & 15) == 0;
+  for (int i = threadIdx.x; i < RH_SAMPLES * d4; i += NTHR)
+    reinterpret_cast<float4*>(xs)[i] = i < n ? load4(pooled + (size_t)s0 * d + 4 * (size_t)i, wide) : make_float4(0.f, 0.f, 0.f, 0.f);
   __syncthreads();
-  const int d4 = d >> 2;
-  for (int r = 0; r < RH_ROWS / (NTHR / 32); ++r) {
-    const int j = blockIdx.x * RH_ROWS + warp * (RH_ROWS / (NTHR / 32)) + r;
-    if (j >= hid) break;
-    float acc[RH_SAMPLES];
+  const int j0 = blockIdx.x * RH_ROWS + warp * RH_PER_WARP;
+  if (j0 >= hid) return;
+  float acc[RH_PER_WARP][RH_SAMPLES];
 #pragma unroll
-    for (int q = 0; q < RH_SAMPLES; ++q) acc[q] = 0.f;
-    for (int c = lane; c < d4; c += 32) {
-      const float4 w = reinterpret_cast<const float4*>(w0 + (size_t)j * d)[c];
+  for (int r = 0; r < RH_PER_WARP; ++r)
 #pragma unroll
-      for (int q = 0; q < RH_SAMPLES; ++q) {
-        const float4 x = reinterpret_cast<const float4*>(xs + (size_t)q * d)[c];
-        acc[q] += w.x * x.x + w.y * x.y + w.z * x.z + w.w * x.w;
-      }
-    }
+    for (int q = 0; q < RH_SAMPLES; ++q) acc[r][q] = 0.f;
+  const bool wide_w = (reinterpret_cast<uintptr_t>(w0) & 15) == 0;
+  for (int c = lane; c < d4; c += 32) {
+    float4 w[RH_PER_WARP];
+#pragma unroll
+    for (int r = 0; r < RH_PER_WARP; ++r) w[r] = load4(w0 + (size_t)min(j0 + r, hid - 1) * d + 4 * c, wide_w);
 #pragma unroll
     for (int q = 0; q < RH_SAMPLES; ++q) {
-      const float v = rte::warp_sum(acc[q]);
-      if (lane == 0 && s0 + q < B) pre[(size_t)(s0 + q) * hid + j] = v + b0[j];
+      const float4 x = reinterpret_cast<const float4*>(xs)[q * d4 + c];
+#pragma unroll
+      for (int r = 0; r < RH_PER_WARP; ++r) acc[r][q] += w[r].x * x.x + w[r].y * x.y + w[r].z * x.z + w[r].w * x.w;
     }
+  }
+#pragma unroll
+  for (int r = 0; r < RH_PER_WARP; ++r) {
+    const int j = j0 + r;
+    float mine = 0.f;
+#pragma unroll
+    for (int q = 0; q < RH_SAMPLES; ++q) {
+      const float v = rte::warp_sum(acc[r][q]);
+      if (lane == q) mine = v;
+    }
+    if (lane < RH_SAMPLES && s0 + lane < B && j < hid) pre[(size_t)(s0 + lane) * hid + j] = mine + b0[j];
   }
 }
 
@@ -101,7 +134,7 @@ router_fwd_kernel(rte_router_weights w, const int32_t* __restrict__ depth_values
   head_logits(o.r_hidden_pre + (size_t)b * hid, w.r_w2, w.r_b2, hs, rl, hid, R);
   head_logits(o.d_hidden_pre + (size_t)b * hid, w.d_w2, w.d_b2, hs, dl, hid, K);
   if (threadIdx.x == 0) {
-    float rp[RTE_ROUTER_MAX_R], dp[RTE_ROUTER_MAX_K], tmp[RTE_ROUTER_MAX_R], tp[RTE_ROUTER_MAX_R];
+    float rp[RTE_ROUTER_MAX_R], dp[RTE_ROUTER_MAX_K];
     softmax_small(rl, rp, R);
     softmax_small(dl, dp, K);
     float rent = 0.f, dent = 0.f, ed = 0.f;
@@ -118,7 +151,12 @@ router_fwd_kernel(rte_router_weights w, const int32_t* __restrict__ depth_values
     o.expected_depth[b] = ed;
     o.router_entropy[b] = rent + dent;
     o.recipe_id[b] = fixed_recipe >= 0 ? fixed_recipe : argmax_lowest(rp, R);
-    for (int t = 0; t < T; ++t) {
+    const int did = fixed_depth_id >= 0 ? fixed_depth_id : argmax_lowest(dp, K);
+    o.depth_id[b] = did;
+    o.depth[b] = depth_values[did];
+  } else if (threadIdx.x >= 32) {              // a thread per pass, next to the sample's own softmaxes
+    float tmp[RTE_ROUTER_MAX_R], tp[RTE_ROUTER_MAX_R];
+    for (int t = threadIdx.x - 32; t < T; t += NTHR - 32) {
       int id = fixed_recipe;
       if (fixed_recipe < 0) {
         for (int r = 0; r < R; ++r) tmp[r] = rl[r] + w.pass_recipe_bias[t * R + r];
@@ -127,9 +165,6 @@ router_fwd_kernel(rte_router_weights w, const int32_t* __restrict__ depth_values
       }
       o.recipe_id_by_pass[(size_t)b * T + t] = id;
     }
-    const int did = fixed_depth_id >= 0 ? fixed_depth_id : argmax_lowest(dp, K);
-    o.depth_id[b] = did;
-    o.depth[b] = depth_values[did];
   }
 }
 
@@ -213,88 +248,144 @@ router_bwd_sample_kernel(rte_router_weights w, rte_router_out o, const int32_t* 
   mlp_backward_sample(w.d_w0, w.d_w2, dld, o.d_hidden_pre + (size_t)b * hid, dpre_d + (size_t)b * hid, dhd, d, hid, K);
 }
 
-// dst[r,:] += sum_p vec[p][r / seg,:]   (nparts partial vectors, part_stride floats apart, added in fixed order)
-__global__ void bcast_add_kernel(float* __restrict__ dst, const float* __restrict__ vec, int rows, int seg, int d, int nparts,
-                                 long long part_stride) {
+// dst[r,:] += sum_p vec[p][r / seg,:]   (nparts partial vectors, part_stride floats apart, added in fixed order).  CTA = 256
+// float4 columns of one segment and 32 of its rows: the vector is added up once per thread, eight rows are in flight.
+constexpr int BC_ROWS = 32;
+__global__ void __launch_bounds__(NTHR)
+bcast_add_kernel(float* __restrict__ dst, const float* __restrict__ vec, int rows, int seg, int d, int nparts, long long part_stride) {
   rte::after_previous_grid();
-  const long long total = (long long)rows * (d >> 2);
-  const int d4 = d >> 2;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const int r = int(i / d4), c = int(i % d4);
-    float4 a = reinterpret_cast<float4*>(dst)[i];
-    for (int p = 0; p < nparts; ++p) {
-      const float4 v = reinterpret_cast<const float4*>(vec + p * part_stride)[(size_t)(r / seg) * d4 + c];
-      a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
-    }
-    reinterpret_cast<float4*>(dst)[i] = a;
+  const int d4 = d >> 2, b = blockIdx.z, c = blockIdx.x * NTHR + threadIdx.x;
+  if (c >= d4) return;
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int p = 0; p < nparts; ++p) {
+    const float4 t = reinterpret_cast<const float4*>(vec + p * part_stride)[(size_t)b * d4 + c];
+    v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
+  }
+  const int r0 = blockIdx.y * BC_ROWS, r1 = min(min(seg, r0 + BC_ROWS), rows - b * seg);
+  float4* q = reinterpret_cast<float4*>(dst) + (size_t)b * seg * d4 + c;
+#pragma unroll 8
+  for (int r = r0; r < r1; ++r) {
+    float4 a = q[(size_t)r * d4];
+    a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+    q[(size_t)r * d4] = a;
   }
 }
 
 // dpooled[part][b,:] = (dpre_r[b, J] @ W0r[J,:] + dpre_d[b, J] @ W0d[J,:]) / S over the part's slice J of the hidden
-// dimension (blockIdx.y = part).  CTA = 4 samples x 128 columns; the two halves of the block split J again and are
-// combined through shared memory.  The broadcast kernel adds the parts in fixed order.
+// dimension (blockIdx.y = part).  CTA = DP_SAMPLES samples x 128 columns (a float4 per lane); its eight warps take every
+// eighth j and meet in shared memory in warp order.  The broadcast kernel adds the parts in fixed order.  32 samples x
+// 1024 58 -> 20 us.
+constexpr int DP_SAMPLES = 8, DP_WARPS = NTHR / 32;
 __global__ void __launch_bounds__(NTHR)
 router_dpooled_kernel(const float* __restrict__ w0r, const float* __restrict__ w0d, const float* __restrict__ dpre_r,
                       const float* __restrict__ dpre_d, float* __restrict__ dpooled, int B, int S, int d, int hid) {
   rte::after_previous_grid();
-  extern __shared__ float sm[];            // sr[4][hid], sd[4][hid], comb[4][128]
-  float* sr = sm;
-  float* sd = sm + 4 * hid;
-  float* comb = sm + 8 * hid;
-  const int cblocks = rte::ceil_div(d, 128);
-  const int b0 = (blockIdx.x / cblocks) * 4, c = (blockIdx.x % cblocks) * 128 + (threadIdx.x & 127);
-  const int half = threadIdx.x >> 7;
+  extern __shared__ float sm[];            // sr[part_len][DP_SAMPLES], sd[part_len][DP_SAMPLES]
+  __shared__ float4 comb[DP_WARPS / 2][DP_SAMPLES][32];
+  const int cblocks = rte::ceil_div(d, 128), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int b0 = (blockIdx.x / cblocks) * DP_SAMPLES, c = (blockIdx.x % cblocks) * 128 + 4 * lane;
   const int part_len = (hid + (int)gridDim.y - 1) / (int)gridDim.y;
-  const int p_lo = blockIdx.y * part_len, p_hi = min(hid, p_lo + part_len);
+  const int p_lo = min(hid, (int)blockIdx.y * part_len), len = min(hid, p_lo + part_len) - p_lo;
+  float* sr = sm;
+  float* sd = sm + part_len * DP_SAMPLES;
   dpooled += (size_t)blockIdx.y * B * d;
-  for (int i = threadIdx.x; i < 4 * hid; i += NTHR) {
-    const int bb = b0 + i / hid;
-    sr[i] = bb < B ? dpre_r[(size_t)bb * hid + i % hid] : 0.f;
-    sd[i] = bb < B ? dpre_d[(size_t)bb * hid + i % hid] : 0.f;
-  }
-  __syncthreads();
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  if (c < d) {
-    const int jh = (p_hi - p_lo + 1) / 2, j_lo = p_lo + half * jh, j_hi = min(p_hi, j_lo + jh);
-#pragma unroll 8
-    for (int j = j_lo; j < j_hi; ++j) {
-      const float wr = w0r[(size_t)j * d + c], wd = w0d[(size_t)j * d + c];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) acc[q] += wr * sr[q * hid + j] + wd * sd[q * hid + j];
+  for (int q = warp; q < DP_SAMPLES; q += DP_WARPS) {
+    const int bb = b0 + q;
+    for (int j = lane; j < len; j += 32) {
+      sr[j * DP_SAMPLES + q] = bb < B ? dpre_r[(size_t)bb * hid + p_lo + j] : 0.f;
+      sd[j * DP_SAMPLES + q] = bb < B ? dpre_d[(size_t)bb * hid + p_lo + j] : 0.f;
     }
   }
-  if (half == 1) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) comb[q * 128 + (threadIdx.x & 127)] = acc[q];
-  }
   __syncthreads();
-  if (half == 0 && c < d) {
+  float4 acc[DP_SAMPLES];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int bb = b0 + q;
-      if (bb >= B) break;
-      dpooled[(size_t)bb * d + c] = (acc[q] + comb[q * 128 + threadIdx.x]) / (float)S;
+  for (int q = 0; q < DP_SAMPLES; ++q) acc[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (c < d) {
+    const bool wide = ((reinterpret_cast<uintptr_t>(w0r) | reinterpret_cast<uintptr_t>(w0d)) & 15) == 0;
+#pragma unroll 4
+    for (int j = warp; j < len; j += DP_WARPS) {
+      const float4 wr = load4(w0r + (size_t)(p_lo + j) * d + c, wide), wd = load4(w0d + (size_t)(p_lo + j) * d + c, wide);
+#pragma unroll
+      for (int q = 0; q < DP_SAMPLES; ++q) {
+        const float r = sr[j * DP_SAMPLES + q], e = sd[j * DP_SAMPLES + q];
+        acc[q].x += wr.x * r + wd.x * e;
+        acc[q].y += wr.y * r + wd.y * e;
+        acc[q].z += wr.z * r + wd.z * e;
+        acc[q].w += wr.w * r + wd.w * e;
+      }
+    }
+  }
+  // warps 4-7 onto 0-3, then the rest of the tree
+#pragma unroll
+  for (int w = DP_WARPS / 2; w > 0; w >>= 1) {
+    if (warp >= w && warp < 2 * w) {
+#pragma unroll
+      for (int q = 0; q < DP_SAMPLES; ++q) comb[warp - w][q][lane] = acc[q];
+    }
+    __syncthreads();
+    if (warp < w) {
+#pragma unroll
+      for (int q = 0; q < DP_SAMPLES; ++q) {
+        const float4 v = comb[warp][q][lane];
+        acc[q].x += v.x; acc[q].y += v.y; acc[q].z += v.z; acc[q].w += v.w;
+      }
+    }
+    __syncthreads();
+  }
+  if (warp == 0 && c < d) {
+    const float inv = 1.f / (float)S;
+#pragma unroll
+    for (int q = 0; q < DP_SAMPLES; ++q) {
+      if (b0 + q >= B) break;
+      float* o = dpooled + (size_t)(b0 + q) * d + c;
+      o[0] = acc[q].x * inv; o[1] = acc[q].y * inv; o[2] = acc[q].z * inv; o[3] = acc[q].w * inv;
     }
   }
 }
 
-// dW0[j,c] = sum_b dpre[b,j] * pooled[b,c];  db0[j] = sum_b dpre[b,j]
+// dW0[j,c] = sum_b dpre[b,j] * pooled[b,c];  db0[j] = sum_b dpre[b,j], for both MLPs (blockIdx.z).  CTA = 64 x 64 outputs, 16
+// per thread, 16 samples at a time in shared memory (an output per thread read both operands from L1 for every product:
+// 32 samples x 1024 x 1024, both MLPs 167 -> 13 us).
+constexpr int W0_TILE = 64, W0_SAMPLES = 16;
+struct Dw0Job { const float* dpre; float* dw0; float* db0; };
+struct Dw0Jobs { Dw0Job job[2]; };
 __global__ void __launch_bounds__(NTHR)
-router_dw0_kernel(const float* __restrict__ dpre, const float* __restrict__ pooled, float* __restrict__ dw0,
-                  float* __restrict__ db0, int B, int d, int hid) {
+router_dw0_kernel(const Dw0Jobs jobs, const float* __restrict__ pooled, int B, int d, int hid) {
   rte::after_previous_grid();
-  const long long i = blockIdx.x * (long long)NTHR + threadIdx.x;
-  if (i >= (long long)hid * d) return;
-  const int j = int(i / d), c = int(i % d);
-  float acc = 0.f, accb = 0.f;
-#pragma unroll 8
-  for (int b = 0; b < B; ++b) {
-    const float v = dpre[(size_t)b * hid + j];
-    acc += v * pooled[(size_t)b * d + c];
-    accb += v;
+  __shared__ float sj[W0_SAMPLES][W0_TILE], sc[W0_SAMPLES][W0_TILE];
+  const Dw0Job& job = jobs.job[blockIdx.z];
+  const int j0 = blockIdx.y * W0_TILE, c0 = blockIdx.x * W0_TILE, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  float acc[4][4], accb = 0.f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[i][k] = 0.f;
+  for (int b0 = 0; b0 < B; b0 += W0_SAMPLES) {
+    __syncthreads();
+#pragma unroll
+    for (int i = threadIdx.x; i < W0_SAMPLES * W0_TILE; i += NTHR) {
+      const int b = b0 + i / W0_TILE, q = i % W0_TILE;
+      sj[i / W0_TILE][q] = b < B && j0 + q < hid ? job.dpre[(size_t)b * hid + j0 + q] : 0.f;
+      sc[i / W0_TILE][q] = b < B && c0 + q < d ? pooled[(size_t)b * d + c0 + q] : 0.f;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int b = 0; b < W0_SAMPLES; ++b) {
+      const float4 x = *reinterpret_cast<const float4*>(&sc[b][4 * tx]), v = *reinterpret_cast<const float4*>(&sj[b][4 * ty]);
+      const float vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        acc[i][0] += vv[i] * x.x; acc[i][1] += vv[i] * x.y; acc[i][2] += vv[i] * x.z; acc[i][3] += vv[i] * x.w;
+      }
+      if (blockIdx.x == 0 && threadIdx.x < W0_TILE) accb += sj[b][threadIdx.x];
+    }
   }
-  dw0[i] = acc;
-  if (c == 0) db0[j] = accb;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (j0 + 4 * ty + i < hid && c0 + 4 * tx + k < d) job.dw0[(size_t)(j0 + 4 * ty + i) * d + c0 + 4 * tx + k] = acc[i][k];
+  if (blockIdx.x == 0 && threadIdx.x < W0_TILE && j0 + threadIdx.x < hid) job.db0[j0 + threadIdx.x] = accb;
 }
 // dW2[r,j] = sum_b dlog[b,r] * silu(pre[b,j]);  db2[r] = sum_b dlog[b,r].  32 outputs x 8 sample groups per CTA.
 __global__ void __launch_bounds__(NTHR)
@@ -349,7 +440,7 @@ extern "C" int rte_router_fwd(const float* h0, const rte_router_weights* w, cons
       set = true;
     }
   }
-  rte::launch(pool_kernel, dim3(rte::ceil_div(d, NTHR), B), NTHR, 0, ST(stream), h0, out->pooled, S, d);
+  rte::launch(pool_kernel, dim3(rte::ceil_div(d, 128), B), NTHR, 0, ST(stream), h0, out->pooled, S, d);
   RTE_LAUNCH_CHECK();
   rte::launch(router_hidden_kernel, dim3(rte::ceil_div(hid, RH_ROWS), rte::ceil_div(B, RH_SAMPLES), 2), NTHR, smem_h, ST(stream), out->pooled, w->r_w0, w->r_b0, out->r_hidden_pre, w->d_w0, w->d_b0, out->d_hidden_pre, B, d, hid);
   RTE_LAUNCH_CHECK();
@@ -402,16 +493,15 @@ extern "C" int rte_router_aux_bwd_data(const rte_router_weights* w, const rte_ro
   rte::launch(router_bwd_sample_kernel, B, NTHR, smem, ST(stream), *w, *fwd, depth_values, mean_prob, lambda_load, lambda_depth,
                                                           dpre_r, dpre_d, dlog_r, dlog_d, dh0, B, S, d, hid, R, K);
   RTE_LAUNCH_CHECK();
-  const size_t smem_dp = (size_t)(8 * hid + 4 * 128) * sizeof(float);
-  if (smem_dp > 48 * 1024) return RTE_ERR_UNSUPPORTED;
-  rte::launch(router_dpooled_kernel, dim3(rte::ceil_div(B, 4) * rte::ceil_div(d, 128), RTE_ROUTER_DPOOLED_PARTS), NTHR, smem_dp, ST(stream), w->r_w0, w->d_w0, dpre_r, dpre_d, dpooled, B, S, d, hid);
+  const size_t smem_dp = (size_t)2 * rte::ceil_div(hid, RTE_ROUTER_DPOOLED_PARTS) * DP_SAMPLES * sizeof(float);
+  if (smem_dp > 32 * 1024 &&
+      cudaFuncSetAttribute(router_dpooled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dp) != cudaSuccess)
+    return RTE_ERR_LAUNCH;
+  rte::launch(router_dpooled_kernel, dim3(rte::ceil_div(B, DP_SAMPLES) * rte::ceil_div(d, 128), RTE_ROUTER_DPOOLED_PARTS), NTHR, smem_dp, ST(stream), w->r_w0, w->d_w0, dpre_r, dpre_d, dpooled, B, S, d, hid);
   RTE_LAUNCH_CHECK();
   if (d % 4 != 0) return RTE_ERR_UNSUPPORTED;
   if (dh0) {
-    long long n4 = (long long)B * S * (d / 4);
-    int grid = (int)((n4 + NTHR - 1) / NTHR);
-    if (grid > 148 * 8) grid = 148 * 8;
-    rte::launch(bcast_add_kernel, grid, NTHR, 0, ST(stream), dh0, dpooled, B * S, S, d, RTE_ROUTER_DPOOLED_PARTS, (long long)B * d);
+    rte::launch(bcast_add_kernel, dim3(rte::ceil_div(d / 4, NTHR), rte::ceil_div(S, BC_ROWS), B), NTHR, 0, ST(stream), dh0, dpooled, B * S, S, d, RTE_ROUTER_DPOOLED_PARTS, (long long)B * d);
     RTE_LAUNCH_CHECK();
   }
   return RTE_OK;
@@ -424,10 +514,7 @@ extern "C" int rte_router_aux_add_dh0(float* dh0, const float* scratch, int32_t 
   if (d % 4 != 0) return RTE_ERR_UNSUPPORTED;
   if (reinterpret_cast<uintptr_t>(scratch) & 15) return RTE_ERR_ALIGNMENT;
   const float* dpooled = scratch + (((size_t)RTE_ROUTER_MAX_R + (size_t)B * (2 * hid + R + K) + 3) & ~(size_t)3);
-  long long n4 = (long long)B * S * (d / 4);
-  int grid = (int)((n4 + NTHR - 1) / NTHR);
-  if (grid > 148 * 8) grid = 148 * 8;
-  rte::launch(bcast_add_kernel, grid, NTHR, 0, ST(stream), dh0, dpooled, B * S, S, d, RTE_ROUTER_DPOOLED_PARTS, (long long)B * d);
+  rte::launch(bcast_add_kernel, dim3(rte::ceil_div(d / 4, NTHR), rte::ceil_div(S, BC_ROWS), B), NTHR, 0, ST(stream), dh0, dpooled, B * S, S, d, RTE_ROUTER_DPOOLED_PARTS, (long long)B * d);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -441,10 +528,8 @@ extern "C" int rte_router_aux_bwd_params(const rte_router_out* fwd, const rte_ro
   float* dpre_d = dpre_r + (size_t)B * hid;
   float* dlog_r = dpre_d + (size_t)B * hid;
   float* dlog_d = dlog_r + (size_t)B * R;
-  const int g0 = (int)rte::ceil_div64((long long)hid * d, NTHR);
-  rte::launch(router_dw0_kernel, g0, NTHR, 0, ST(stream), dpre_r, fwd->pooled, grads->r_w0, grads->r_b0, B, d, hid);
-  RTE_LAUNCH_CHECK();
-  rte::launch(router_dw0_kernel, g0, NTHR, 0, ST(stream), dpre_d, fwd->pooled, grads->d_w0, grads->d_b0, B, d, hid);
+  const Dw0Jobs jobs = {{{dpre_r, grads->r_w0, grads->r_b0}, {dpre_d, grads->d_w0, grads->d_b0}}};
+  rte::launch(router_dw0_kernel, dim3(rte::ceil_div(d, W0_TILE), rte::ceil_div(hid, W0_TILE), 2), NTHR, 0, ST(stream), jobs, fwd->pooled, B, d, hid);
   RTE_LAUNCH_CHECK();
   rte::launch(router_dw2_kernel, rte::ceil_div(R * hid, 32), NTHR, 0, ST(stream), dlog_r, fwd->r_hidden_pre, grads->r_w2, grads->r_b2, B, hid, R);
   RTE_LAUNCH_CHECK();
