@@ -1061,26 +1061,14 @@ phi_reduce_keys_kernel(const KeyJobs jobs, const int32_t* __restrict__ rid, cons
   }
   int q = 0;
   while (q < 3 && (int)blockIdx.x >= jobs.first_block[q + 1]) ++q;
-  const long long elems = jobs.elems[q], e = ((long long)blockIdx.x - jobs.first_block[q]) * (4 * NTHR) + 4 * threadIdx.x;
+  const long long elems = jobs.elems[q], e = ((long long)blockIdx.x - jobs.first_block[q]) * NTHR + threadIdx.x;
   const float* partial = jobs.partial[q];
   float* out = jobs.out[q] + (size_t)key * elems;
-  if (e >= elems) return;
-  if (elems % 4 == 0 && ((reinterpret_cast<uintptr_t>(partial) | reinterpret_cast<uintptr_t>(jobs.out[q])) & 15) == 0) {
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-    for (int i = 0; i < n; ++i) {
-      const float4 x = *reinterpret_cast<const float4*>(partial + (size_t)members[i] * elems + e);
-      acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
-    }
-    *reinterpret_cast<float4*>(out + e) = acc;
-  } else {
-    for (long long f = e; f < min(elems, e + 4); ++f) {
-      float acc = 0.f;
-#pragma unroll 4
-      for (int i = 0; i < n; ++i) acc += partial[(size_t)members[i] * elems + f];
-      out[f] = acc;
-    }
-  }
+  if (e >= elems) return;          // (an element per thread: often one key has most samples, and only its CTAs work)
+  float acc = 0.f;
+#pragma unroll 16
+  for (int i = 0; i < n; ++i) acc += partial[(size_t)members[i] * elems + e];
+  out[e] = acc;
 }
 
 // Mean-squared-error pieces of the consistency term (macro.py:359): g[i] = coef * (a[i] - b[i]) and one partial sum of
@@ -1302,7 +1290,7 @@ int phi_bwd_params_impl(const float* h0, const float* hx, const int32_t* recipe_
 #undef RTE_PG
   RTE_LAUNCH_CHECK();
   KeyJobs jobs = {{x.pv, x.pu, x.pg, x.pb}, {g->v, g->u, g->gain, g->bias}, {(long long)3 * d * m, (long long)m * d, d, d}, {0}};
-  for (int q = 0; q < 4; ++q) jobs.first_block[q + 1] = jobs.first_block[q] + (int)rte::ceil_div64(jobs.elems[q], 4 * NTHR);
+  for (int q = 0; q < 4; ++q) jobs.first_block[q + 1] = jobs.first_block[q] + (int)rte::ceil_div64(jobs.elems[q], NTHR);
   rte::launch(phi_reduce_keys_kernel, dim3((unsigned)jobs.first_block[4], R * K_strides), NTHR, 0, ST(stream), jobs, recipe_id, stride_id, B, K_strides);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
