@@ -661,14 +661,20 @@ __global__ void segment_sum_kernel(const float* __restrict__ in, float* __restri
 }
 
 // ------------------------------------------------------------------ small vector kernels
-__global__ void reduce_splits_kernel(const float* __restrict__ ws, int splits, long long stride, long long n4,
-                                     float* __restrict__ out, int accumulate) {
+// (up to eight partials of an element are requested together)
+__global__ void __launch_bounds__(256)
+reduce_splits_kernel(const float* __restrict__ ws, int splits, long long stride, long long n4, float* __restrict__ out, int accumulate) {
   rte::after_previous_grid();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4; i += (long long)gridDim.x * blockDim.x) {
     float4 acc = accumulate ? reinterpret_cast<float4*>(out)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = 0; s < splits; ++s) {
-      const float4 t = reinterpret_cast<const float4*>(ws + (size_t)s * stride)[i];
-      acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w;
+    for (int s0 = 0; s0 < splits; s0 += 8) {
+      float4 t[8];
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+        if (s0 + s < splits) t[s] = reinterpret_cast<const float4*>(ws + (size_t)(s0 + s) * stride)[i];
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+        if (s0 + s < splits) { acc.x += t[s].x; acc.y += t[s].y; acc.z += t[s].z; acc.w += t[s].w; }
     }
     reinterpret_cast<float4*>(out)[i] = acc;
   }
