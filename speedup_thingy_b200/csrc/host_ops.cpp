@@ -514,14 +514,14 @@ void cast_into(const Dev& dev, const Tensor& src, const Tensor& dst) {
 }
 
 struct PoolModule {
-  Tensor status, selector16, centers, idx_ug, idx_d, ug_ptr, ug_rows, d_ptr, d_rows, wug16, wdT16, wug_pool, wd_pool, q, assign, pos, perm, tile_group, counts,
+  Tensor status, selector16, centers, idx_ug, idx_d, ug_ptr, ug_rows, d_ptr, d_rows, wdT16, wug_pool, wd_pool, q, assign, pos, perm, tile_group, counts,
       offsets, kblocks, x16, xp, ugp, zp, yp, dyp, dzp, dugp, dxp, dwug_pool, dwd_pool, dwdT;
   int64_t rank = 0, C = 0, Mc = 0, cap = 0, d = 0, F = 0, tokens = 0;
 
   explicit PoolModule(const std::map<std::string, Tensor>& t, const std::map<std::string, int64_t>& n) {
     const std::pair<const char*, Tensor*> fields[] = {
         {"status", &status}, {"selector16", &selector16}, {"centers", &centers}, {"idx_ug", &idx_ug}, {"idx_d", &idx_d}, {"ug_ptr", &ug_ptr},
-        {"ug_rows", &ug_rows}, {"d_ptr", &d_ptr}, {"d_rows", &d_rows}, {"wug16", &wug16}, {"wdT16", &wdT16}, {"wug_pool", &wug_pool}, {"wd_pool", &wd_pool},
+        {"ug_rows", &ug_rows}, {"d_ptr", &d_ptr}, {"d_rows", &d_rows}, {"wdT16", &wdT16}, {"wug_pool", &wug_pool}, {"wd_pool", &wd_pool},
         {"q", &q}, {"assign", &assign}, {"pos", &pos}, {"perm", &perm}, {"tile_group", &tile_group}, {"counts", &counts}, {"offsets", &offsets},
         {"kblocks", &kblocks}, {"x16", &x16}, {"xp", &xp}, {"ugp", &ugp}, {"zp", &zp}, {"yp", &yp}, {"dyp", &dyp}, {"dzp", &dzp}, {"dugp", &dugp}, {"dxp", &dxp},
         {"dwug_pool", &dwug_pool}, {"dwd_pool", &dwd_pool}, {"dwdT", &dwdT}};
@@ -540,9 +540,8 @@ struct PoolModule {
           "rte_cluster_pack");
   }
   void prepare_pools(const Dev& dev, const Tensor& wug, const Tensor& wd) {
-    cast_into(dev, wug, wug16);
+    gather(dev, wug, idx_ug, wug_pool);
     check(rte_transpose_f32(f32(wd), ptr(wdT16), d, F, 1, 0, dev.st), "rte_transpose_f32");
-    check(rte_gather_rows(ptr(wug16), i32(idx_ug), ptr(wug_pool), idx_ug.numel(), d * 2, dev.st), "rte_gather_rows");
     check(rte_gather_rows(ptr(wdT16), i32(idx_d), ptr(wd_pool), idx_d.numel(), d * 2, dev.st), "rte_gather_rows");
   }
   void gather(const Dev& dev, const Tensor& src, const Tensor& idx, const Tensor& dst) {
