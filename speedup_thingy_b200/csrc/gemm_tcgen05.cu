@@ -693,8 +693,7 @@ float tile_us(const rte_gemm_args* a, int bn, int ksplit, int sms) {
   if (ksplit > kb || grid > 2 * limit || (ksplit > 1 && grid > limit)) return 1e9f;
   static const float base64[4] = {3.0f, 4.3f, 3.9f, 4.2f}, base128[4] = {4.1f, 6.2f, 5.4f, 5.4f};
   const float base = (bn == 64 ? base64 : base128)[ksplit == 1 ? 0 : ksplit == 2 ? 1 : ksplit == 4 ? 2 : 3];
-  const float slope = bn == 64 ? 0.21f : 0.2f + 0.035f * float(grid < 148 ? grid : 148) / 148.f;
-  const float per = float(rte::ceil_div(kb, ksplit)) * slope, f32 = a->epilogue == RTE_EPI_F32 ? (bn == 64 ? 0.2f : 0.5f) : 0.f;
+  const float per = float(rte::ceil_div(kb, ksplit)) * 0.21f, f32 = a->epilogue == RTE_EPI_F32 ? (bn == 64 ? 0.2f : 0.5f) : 0.f;
   return base + f32 + (grid <= limit ? per : 1.f + 2.2f * per);
 }
 
@@ -837,7 +836,8 @@ extern "C" int rte_gemm_wgrad_splits(const rte_gemm_args* a, int32_t max_splits)
     if (rte::ceil_div(kb, rte::ceil_div(kb, s)) != s) continue;               // every split gets k-blocks
     float us;
     pick_tile(a, s, sms, &us);
-    us += 1.2f + float(s + 1) * float(a->M) * float(a->N) * 4e-6f / 8.f;        // ... and one launch adds the partials (in L2)
+    us += 1.8f + float(s + 1) * float(a->M) * float(a->N) * 4e-6f / 5.f;        // ... and one launch adds the partials (cautious: in a
+                                                                                 // training step its traffic competes with the other stream's)
     if (us < best) { best = us; splits = s; }
   }
   return splits;
