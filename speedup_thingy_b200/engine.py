@@ -13,6 +13,7 @@ PyTorch is used for device memory, streams and graph capture only.
 from __future__ import annotations
 
 import contextlib
+import gc
 import os
 
 import math
@@ -226,6 +227,19 @@ def teardown_data_parallel(engine: "TrainEngine | None", watchdog_s: float = 30.
     timer.start()
     dist.destroy_process_group()
     timer.cancel()
+
+
+@contextlib.contextmanager
+def _no_collection():
+    """Keeps Python's collector out of a stream capture: an engine that it finds there would destroy its graphs, which the
+    runtime does not permit while a stream is capturing (and which ends the capture)."""
+    was = gc.isenabled()
+    gc.disable()
+    try:
+        yield
+    finally:
+        if was:
+            gc.enable()
 
 
 # --------------------------------------------------------------------------- results
@@ -567,10 +581,6 @@ class TrainEngine:
         self.dxa, self.dxb, self.dxc, self.partial = t_.dxa, t_.dxb, t_.dxc, t_.partial
         self.partial_final = torch.empty_like(self.partial)     # the final norm's column partials (its reduction is deferred too)
         self.gn_partial = e(self.plan.total_chunks)
-        max_ws = 0
-        for (mm, nn) in ((3 * d, d), (d, d), (2 * cfg.d_ff, d), (d, cfg.d_ff), (V, d)):
-            max_ws = max(max_ws, ops.pick_splits(mm, nn, M) * mm * nn)
-        ops.split_workspace(max_ws)
         if not self.dense:
             r, k, m, hid = cfg.recipe_count, len(cfg.depth_choices), cfg.macro_rank, cfg.router_hidden_dim
             self.h_phi = e(M, d)
@@ -584,10 +594,10 @@ class TrainEngine:
             self.macro_teacher_delta_rms = torch.zeros(r, k)               # carried through checkpoints only (macro.py:122)
             self.depth_values = torch.tensor(list(cfg.depth_choices), dtype=torch.int32, device=dev)
             i32 = torch.int32
+            zeros = lambda *shape: torch.zeros(*shape, dtype=i32, device=dev)  # noqa: E731  (ids: valid from the start)
             self.route = dict(pooled=e(B, d), r_hidden_pre=e(B, hid), d_hidden_pre=e(B, hid), recipe_logits=e(B, r),
                               recipe_probs=e(B, r), depth_probs=e(B, k), expected_depth=e(B), router_entropy=e(B),
-                              recipe_id=self._results[8 + B:8 + 2 * B].view(i32), recipe_id_by_pass=e(B, cfg.t_max, dtype=i32),
-                              depth_id=e(B, dtype=i32), depth=e(B, dtype=i32))
+                              recipe_id=self._results[8 + B:8 + 2 * B].view(i32), recipe_id_by_pass=zeros(B, cfg.t_max), depth_id=zeros(B), depth=zeros(B))
             self.router_scratch = e(A.ROUTER_MAX_R + B * (2 * hid + r + k + A.ROUTER_DPOOLED_PARTS * d) + 4)
             self._mean_prob = torch.zeros(A.ROUTER_MAX_R, dtype=f32, device=dev)
             if self._grad_mem is not None:              # exchanged by the peer kernel: lives in the shared allocation
@@ -614,6 +624,9 @@ class TrainEngine:
         self._side_stream = torch.cuda.Stream(device=dev, priority=-1) if (self.audit_k and dev.type == "cuda") else None
         if self._side_stream is not None and hasattr(ops, "gemm_max_ctas"):
             ops.gemm_max_ctas = max(ops.sm_count - int(os.environ.get("RTE_SIDE_SMS", "8")), 1)
+        # (after the limit on the products' CTAs is known: it decides the split counts)
+        ops.split_workspace(max(ops.pick_splits(mm, nn, M) * mm * nn
+                                for mm, nn in ((3 * d, d), (d, d), (2 * cfg.d_ff, d), (d, cfg.d_ff), (V, d))))
         self._param_stream = torch.cuda.Stream(device=dev) if ((self.audit_k or self.exact) and dev.type == "cuda") else None
         self._merge_stream = torch.cuda.Stream(device=dev) if (self.audit_k and dev.type == "cuda") else None
         self.exact_core = None
@@ -1462,7 +1475,7 @@ class TrainEngine:
             graph = torch.cuda.CUDAGraph()
             # (capturing the hot pass on a raised-priority stream, so that its kernels are served before the
             # weight-gradient streams, was measured: +3 % step time; all streams but the replay's keep the default)
-            with torch.cuda.graph(graph):
+            with _no_collection(), torch.cuda.graph(graph):
                 body()
             self._graphs[key] = graph
             if optimizer:
@@ -1537,7 +1550,7 @@ class TrainEngine:
         if self._graphs.get("forward") is None:
             torch.cuda.synchronize(self.device)
             graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(graph):
+            with _no_collection(), torch.cuda.graph(graph):
                 self._forward_backward(forward_only=True)
             self._graphs["forward"] = graph
         self._graphs["forward"].replay()

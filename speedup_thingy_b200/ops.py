@@ -44,6 +44,7 @@ class CudaOps:
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.launches = 0          # kernels-entry calls issued (for bench accounting)
         self._split_ws: torch.Tensor | None = None
+        self._retired_ws: list[torch.Tensor] = []
         self._splits: dict[tuple[int, int, int, int], int] = {}      # pick_splits by size
         self.small_gemm_rows = 256  # split products with at most this many rows go to the few-row kernel (0: every product to the persistent kernel)
         # ... and so can weight gradients over that few rows (RTE_SMALL_WGRAD=1).  Off by default: inside the training
@@ -98,6 +99,8 @@ class CudaOps:
 
     def split_workspace(self, numel: int) -> torch.Tensor:
         if self._split_ws is None or self._split_ws.numel() < numel:
+            if self._split_ws is not None:
+                self._retired_ws.append(self._split_ws)      # launches already captured into a graph still write there
             self._split_ws = torch.empty(numel, dtype=torch.float32, device=self.device)
         return self._split_ws
 
