@@ -652,7 +652,7 @@ int make_store_tmap(CUtensorMap* map, const void* base, long long rows, long lon
   cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * es, static_cast<cuuint64_t>(plane_stride) * es};
   cuuint32_t box[3] = {f32 ? 32u : 64u, 32, 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base),
+  CUresult r = encode_tiled(fn, map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, cuuint32_t(3), const_cast<void*>(base),
                   dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                   CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? RTE_OK : RTE_ERR_TENSOR_MAP;

@@ -209,6 +209,17 @@ EncodeTiledFn get_encode_fn() {
   return fn;
 }
 
+// Encodes a map.  A thread that has made no call that binds the device's context yet (an autograd worker whose first work
+// is a product on inputs that need no conversion) gets it bound and tries again.
+template <typename... A>
+CUresult encode_tiled(EncodeTiledFn fn, A... args) {
+  const CUresult r = fn(args...);
+  if (r != CUDA_ERROR_INVALID_CONTEXT && r != CUDA_ERROR_NOT_INITIALIZED) return r;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return r;
+  return fn(args...);
+}
+
 // 2-D bf16 tensor map over a row-major [rows, cols] matrix with row stride ld: box = box_cols x box_rows,
 // 128-byte swizzle, out-of-range elements read as zero.
 int make_tmap(CUtensorMap* map, const void* base, long long rows, long long cols, long long ld, int box_cols, int box_rows) {
@@ -218,7 +229,7 @@ int make_tmap(CUtensorMap* map, const void* base, long long rows, long long cols
   cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2ull};
   cuuint32_t box[2] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows)};
   cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
+  CUresult r = encode_tiled(fn, map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, cuuint32_t(2), const_cast<void*>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? RTE_OK : RTE_ERR_TENSOR_MAP;
