@@ -310,6 +310,23 @@ def test_embedding_fwd_bwd(ops):
     _close(dt2, 2 * torch.zeros(V, d).index_add_(0, tok, dx), 1e-5, "embedding grad accumulates")
 
 
+@pytest.mark.parametrize("V,d,n", [(4096, 64, 700), (2000, 65, 1000), (1999, 128, 1000)])
+def test_embedding_bwd_of_a_table_larger_than_the_batch(ops, V, d, n):
+    """Only the batch's rows of the accumulator are cleared and applied (the line is at twice the tokens); repeated tokens
+    are visited once per occurrence and must count once."""
+    g = torch.Generator().manual_seed(V)
+    tok, dx = torch.randint(0, V, (n,), generator=g), torch.randn(n, d, generator=g)
+    tok[:200] = tok[0]
+    base = torch.randn(V, d, generator=g)
+    acc = torch.full((V * d,), -77, dtype=torch.int64, device=DEV)
+    out = base.to(DEV)
+    ops.embed_bwd(tok.to(DEV), dx.to(DEV), out, acc)
+    _close(out, base.clone().index_add_(0, tok, dx), 1e-5, "embedding grad")
+    again = base.to(DEV)
+    ops.embed_bwd(tok.to(DEV), dx.to(DEV), again, acc)
+    assert torch.equal(out, again)
+
+
 # ------------------------------------------------------------------ attention (+RoPE)
 @pytest.mark.parametrize("B,S,H,hd", [(2, 16, 4, 8), (3, 64, 4, 32), (2, 64, 8, 64), (1, 200, 2, 64), (2, 33, 2, 128), (2, 256, 2, 64)])
 def test_attention_fwd_bwd(ops, B, S, H, hd):
@@ -663,6 +680,48 @@ def test_macro_phi_fwd_bwd(ops, B, S, d, m, R, tensor):
     _close(gr["bias"], leaves["macro.bias"].grad, 2e-4, "phi dbias")
     _close(gr["u"], leaves["macro.u"].grad, 2e-4, "phi du")
     _close(gr["v"], leaves["macro.v"].grad, 2e-4, "phi dv")
+
+
+@pytest.mark.parametrize("B,S,d,m,R", [(300, 5, 32, 4, 2), (2, 70, 160, 40, 3), (3, 129, 1056, 32, 2), (2, 9, 2052, 8, 2)])
+def test_macro_phi_edges_of_tokens_columns_ranks_and_samples(ops, B, S, d, m, R):
+    """More samples than a compaction round, tokens past a staging block, columns past a CTA's, ranks past 32, a width
+    that the preparation holds in sixteen pieces and one that it leaves to the one-CTA form."""
+    test_macro_phi_fwd_bwd(ops, B, S, d, m, R, True)
+
+
+@pytest.mark.parametrize("B,S,d,hid", [(17, 33, 132, 100), (9, 5, 64, 260), (40, 130, 520, 36)])
+def test_router_edges_of_samples_columns_and_hidden_units(ops, B, S, d, hid):
+    """Sample, column, token and hidden counts that no tile divides: forward products, input and weight gradients."""
+    R, K, T = 5, 3, 4
+    g = torch.Generator().manual_seed(B)
+    h0 = torch.randn(B, S, d, generator=g)
+    w = {n: torch.randn(*s, generator=g) * 0.2 for n, s in dict(r_w0=(hid, d), r_b0=(hid,), r_w2=(R, hid), r_b2=(R,), d_w0=(hid, d), d_b0=(hid,),
+                                                                d_w2=(K, hid), d_b2=(K,)).items()}
+    leaf = {n: t.clone().requires_grad_(True) for n, t in w.items()}
+    hr = h0.clone().requires_grad_(True)
+    pooled = hr.mean(1)
+    head = lambda a: torch.nn.functional.silu(pooled @ leaf[f"{a}_w0"].t() + leaf[f"{a}_b0"]) @ leaf[f"{a}_w2"].t() + leaf[f"{a}_b2"]  # noqa: E731
+    rp, dp = head("r").softmax(-1), head("d").softmax(-1)
+    depths = torch.tensor([1.0, 2.0, 4.0])
+    (0.3 * (R * rp.mean(0).pow(2).sum() - 1) + 0.7 * (dp @ depths).mean()).backward()
+    e = lambda *s, dt=torch.float32: torch.zeros(*s, dtype=dt, device=DEV)  # noqa: E731
+    i32 = torch.int32
+    out = dict(pooled=e(B, d), r_hidden_pre=e(B, hid), d_hidden_pre=e(B, hid), recipe_logits=e(B, R), recipe_probs=e(B, R), depth_probs=e(B, K),
+               expected_depth=e(B), router_entropy=e(B), recipe_id=e(B, dt=i32), recipe_id_by_pass=e(B, T, dt=i32), depth_id=e(B, dt=i32), depth=e(B, dt=i32))
+    wd = {n: t.to(DEV) for n, t in w.items()} | {"pass_recipe_bias": e(T, R)}
+    dv = torch.tensor([1, 2, 4], dtype=i32, device=DEV)
+    hd = h0.to(DEV)
+    ops.router_fwd(hd, wd, dv, out, B=B, S=S, d=d, hid=hid, R=R, K=K, T=T, fixed_recipe=None, fixed_depth_id=None)
+    _close(out["recipe_probs"], rp, 1e-4, "recipe probabilities")
+    _close(out["depth_probs"], dp, 1e-4, "depth probabilities")
+    assert torch.equal(out["recipe_id_by_pass"].cpu().long(), rp.argmax(-1)[:, None].expand(B, T))
+    aux, dh0 = e(2), e(B * S, d)
+    grads = {n: e(*t.shape) for n, t in w.items()}
+    scratch = e(A.ROUTER_MAX_R + B * (2 * hid + R + K + A.ROUTER_DPOOLED_PARTS * d) + 4)
+    ops.router_aux_bwd(wd, out, dv, 0.3, 0.7, aux, grads, dh0, scratch, B=B, S=S, d=d, hid=hid, R=R, K=K)
+    _close(dh0.view(B, S, d), hr.grad, 2e-4, "dh0")
+    for n in w:
+        _close(grads[n], leaf[n].grad, 2e-4, n)
 
 
 @pytest.mark.parametrize("B,S,d,m,R,tensor", [(3, 16, 64, 8, 4, True), (2, 12, 40, 6, 3, False), (4, 64, 128, 32, 5, True),

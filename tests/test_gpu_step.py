@@ -249,3 +249,16 @@ def test_c3_shapes_one_step_finite_and_close():
         err = (g.cpu() - ref_grads[n]).abs().max().item()
         scale = ref_grads[n].abs().max().item()
         assert err <= 2e-2 * max(scale, 1e-3) + 2e-4, (n, err, scale)
+
+
+def test_split_workspace_is_sized_before_the_step_is_captured():
+    """A width for which the products split further once SMs are set aside for the replay: the workspace must not be
+    replaced inside the capture."""
+    model = dict(vocab_size=1592, d_model=960, n_heads=15, d_ff=2368, n_prelude=1, n_coda=1, t_max=2, depth_choices=(1, 2), attn_banks=1, ffn_banks=1,
+                 head_groups=15, ffn_groups=16, active_head_groups=3, active_ffn_groups=4, recipe_count=5, macro_rank=32)
+    train = dict(mode="recursive_macro", lr=1e-3, weight_decay=0.1, batch_size=203, seq_len=72, seed=0, fixed_depth=2, audit_fixed_count_per_batch=1)
+    cfg, params, eng = _engine(model, train)
+    before = eng.ops._split_ws.data_ptr()
+    batch = next(_stream(cfg, 1))
+    assert all(torch.isfinite(torch.tensor(eng.train_step(batch).loss)) for _ in range(2))
+    assert eng.ops._split_ws.data_ptr() == before and not eng.ops._retired_ws
