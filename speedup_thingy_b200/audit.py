@@ -15,6 +15,7 @@ and -- through the cached h0 -- the prelude, exactly as under ``audit_mode: grad
 from __future__ import annotations
 
 import math
+import weakref
 
 import torch
 
@@ -94,12 +95,18 @@ CORE_SHADOWED = ["core.attn.wqkv", "core.attn.wo", "core.mlp.wug", "core.mlp.wd"
 class AuditReplay:
     """Buffers and launch sequences of the replay; owned by ``TrainEngine`` (``eng``)."""
 
+    @property
+    def eng(self):
+        """The engine that owns the replay; not kept alive by it, so that an engine's memory and graphs go with its last
+        reference instead of at some later collection."""
+        return self._eng()
+
     def __init__(self, eng, k: int, direct_grads: bool = False):
         """`direct_grads`: write the gradients of final norm / coda / embedding straight into the engine's buffers
         (the `recursive_exact` mode, where no hot pass shares them) instead of a private mirror."""
         from .engine import _Block, _Temps
 
-        self.eng, self.k, self.direct = eng, k, direct_grads
+        self._eng, self.k, self.direct = weakref.ref(eng), k, direct_grads
         self._stage = None
         self._prepared = None
         self._prelude_copied = None

@@ -9,6 +9,7 @@ import torch
 import torch.nn.functional as F
 
 from oracle import rte_oracle as O
+from speedup_thingy_b200 import _abi as A
 
 pytestmark = pytest.mark.gpu
 
