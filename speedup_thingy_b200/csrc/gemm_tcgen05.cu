@@ -130,32 +130,15 @@ __device__ __forceinline__ void load_bf16x32(const __nv_bfloat16* src, float (&v
     for (int j = 0; j < 32; ++j) v[j] = (j < ncols_valid) ? __bfloat162float(src[j]) : 0.f;
   }
 }
-// 32 bf16 of one row as 16 packed pairs (zeros beyond ncols_valid); src must be 16-byte aligned.
-__device__ __forceinline__ void load_bf16x32_packed(const __nv_bfloat16* src, uint32_t (&w)[16], int ncols_valid) {
-  if (ncols_valid >= 32) {
-    const uint4* s4 = reinterpret_cast<const uint4*>(src);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      uint4 t = s4[q];
-      w[4 * q] = t.x; w[4 * q + 1] = t.y; w[4 * q + 2] = t.z; w[4 * q + 3] = t.w;
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const float lo = (2 * j < ncols_valid) ? __bfloat162float(src[2 * j]) : 0.f;
-      const float hi = (2 * j + 1 < ncols_valid) ? __bfloat162float(src[2 * j + 1]) : 0.f;
-      w[j] = rte::pack_bf16x2(lo, hi);
-    }
-  }
-}
 
-template <int BN, int CTAS>
+template <int BN, int CTAS, bool SWB>
 struct SmemLayout {
   static constexpr int A_BYTES = BM * BK * 2;            // this CTA's 128 rows of A: 16 KB
   static constexpr int B_ROWS = BN / CTAS;               // rows of the B tile this CTA stages
   static constexpr int B_BYTES = B_ROWS * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int SLOTS = (BN == 256 && CTAS == 1) ? 1 : 2;     // staging slots per epilogue warp
+  // staging slots per epilogue warp; with SWB two pairs: (up | gate) arrive there and (d up | d gate) leave from there
+  static constexpr int SLOTS = SWB ? 4 : (BN == 256 && CTAS == 1) ? 1 : 2;
   static constexpr int STAGING_BYTES = EPI_WARPS * SLOTS * SLOT_BYTES;
   static constexpr int BAR_BYTES = 512;
   static constexpr int STAGES_FIT = (MAX_DYN_SMEM - 1024 - BAR_BYTES - STAGING_BYTES) / STAGE_BYTES;
@@ -166,12 +149,15 @@ struct SmemLayout {
 };
 
 // ------------------------------------------------------------------ kernel
-template <int BN, int CTAS>
+// SWB: the epilogue is SwiGLU's backward with its operands brought in by the TMA (see there); a kernel of its own because
+// its staging slots take shared memory from the operand stages.
+template <int BN, int CTAS, bool SWB>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_c2,
+                    const __grid_constant__ CUtensorMap tmap_r, const __grid_constant__ CUtensorMap tmap_r2,
                     const KParams p) {
-  using L = SmemLayout<BN, CTAS>;
+  using L = SmemLayout<BN, CTAS, SWB>;
   constexpr int STAGES = L::STAGES;
   constexpr uint32_t TMEM_COLS = 2 * BN;
   constexpr int HALF = BN / 2;               // columns of a tile per epilogue warp of a quadrant
@@ -188,6 +174,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   volatile uint32_t* tmem_slot_ptr =
       reinterpret_cast<volatile uint32_t*>(smem_raw + (tmem_slot - smem_u32(smem_raw)));
   volatile uint32_t* err_flag = tmem_slot_ptr + 2;     // set by a role whose wait ran out
+  auto operand_bar = [&](int epi_warp, uint32_t set) { return bar_base + 256u + uint32_t(epi_warp) * 16u + set * 8u; };   // SWB
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t cta_rank = (CTAS == 2) ? cluster_ctarank() : 0u;
@@ -197,6 +184,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(tfull_bar(b), 1); mbar_init(tempty_bar(b), EPI_WARPS * CTAS); }
+    if (SWB) for (int e = 0; e < EPI_WARPS; ++e) { mbar_init(operand_bar(e, 0), 1); mbar_init(operand_bar(e, 1), 1); }
     *err_flag = 0;
     fence_barrier_init();
     prefetch_tmap(&tmap_a);
@@ -355,6 +343,27 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     auto epi_wait = [&](uint32_t bar, uint32_t parity) -> bool {
       return mbar_wait<CTAS>(bar, parity);
     };
+    // ---- SWB: acc = dz; (d up | d gate) from the saved (up | gate), 64 columns at a time.  The pass is bound by the bytes
+    // of (up | gate) in and (d up | d gate) out; read row by row by the lanes that own the rows, the operands cost more
+    // than the product (8192 x 2048 x 512: 51 us, of which 18 are the product's).  So the TMA brings a piece's up and gate
+    // into a pair of slots while the piece before is worked on, the results take their place there and leave from there:
+    // 37 us (3.6 TB/s of the pass's own bytes); 16384 x 2048 x 512 89 -> 65, 8192 x 4096 x 1024 95 -> 85.
+    // tmap_c / tmap_r view columns [0, F), tmap_c2 / tmap_r2 columns [F, 2F): each clips at its own edge, and a piece
+    // outside the matrix reads zeros and is not written.
+    uint32_t piece = 0;
+    auto fetch_piece = [&](uint32_t q, int w, int c0) {
+      if (w < total_work && lane == 0) {
+        bulk_wait_read<0>();                   // the results that left from this pair two pieces ago
+        const uint32_t pair = wslots + (q & 1u) * uint32_t(2 * SLOT_BYTES), bar = operand_bar(warp - 2, q & 1u);
+        const int y = ((w % p.num_m_blocks) * CTAS + int(cta_rank)) * BM + quad * 32, x = (w / p.num_m_blocks) * BN + c0;
+        mbar_arrive_expect_tx(bar, 2 * SLOT_BYTES);
+        tma_load_3d(pair, &tmap_r, bar, x, y, 0);
+        tma_load_3d(pair + SLOT_BYTES, &tmap_r2, bar, x, y, 0);
+      }
+      __syncwarp();
+    };
+    if (SWB) fetch_piece(0, unit, grp * HALF);
+
     for (int w = unit; w < total_work && ok; w += n_units) {
       const int split = w / tiles, t = w % tiles;
       const int mblk = t % p.num_m_blocks, nblk = t / p.num_m_blocks;
@@ -369,7 +378,56 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
       const uint32_t t_row = tmem_base + (uint32_t(quad * 32) << 16) + acc * BN;
       uint32_t raw[32];
 
-      if (p.tma_store && p.epilogue == RTE_EPI_F32) {
+      if (SWB) {
+        if (!epi_wait(tfull_bar(acc), acc_phase)) {
+          if (p.status && lane == 0) atomicExch(p.status, RTE_DEV_WAIT_TIMEOUT_EPILOGUE);
+          *err_flag = 1;
+          ok = false; break;
+        }
+        tc_fence_after();
+        for (int c0 = grp * HALF; c0 < (grp + 1) * HALF; c0 += 64, ++piece) {
+          const bool last = c0 + 64 >= (grp + 1) * HALF;
+          fetch_piece(piece + 1, last ? w + n_units : w, last ? grp * HALF : c0 + 64);
+          if (!mbar_wait<1>(operand_bar(warp - 2, piece & 1u), (piece >> 1) & 1u)) {
+            if (p.status && lane == 0) atomicExch(p.status, RTE_DEV_WAIT_TIMEOUT_EPILOGUE);
+            *err_flag = 1;
+            ok = false;
+          }
+          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+          const int col = n0 + c0;
+          if (!warp_rows || col >= p.N) continue;
+          const uint32_t slot = wslots + (piece & 1u) * uint32_t(2 * SLOT_BYTES), slot2 = slot + uint32_t(SLOT_BYTES);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            uint32_t u[16], g[16];
+            tmem_ld32(t_row + c0 + 32 * h, raw);
+#pragma unroll
+            for (uint32_t c = 0; c < 4; ++c) {
+              const uint32_t at = uint32_t(lane) * 128u + (((4u * h + c) ^ (uint32_t(lane) & 7u)) << 4);
+              ld_shared_v4(slot + at, u[4 * c], u[4 * c + 1], u[4 * c + 2], u[4 * c + 3]);
+              ld_shared_v4(slot2 + at, g[4 * c], g[4 * c + 1], g[4 * c + 2], g[4 * c + 3]);
+            }
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              const float2 u_ = rte::unpack_bf16x2(u[j]), g_ = rte::unpack_bf16x2(g[j]);
+              const float dz0 = __uint_as_float(raw[2 * j]), dz1 = __uint_as_float(raw[2 * j + 1]);
+              const float s0 = fast_sigmoid(g_.x), s1 = fast_sigmoid(g_.y);
+              u[j] = rte::pack_bf16x2(dz0 * g_.x * s0, dz1 * g_.y * s1);
+              g[j] = rte::pack_bf16x2(dz0 * u_.x * s0 * (1.f + g_.x * (1.f - s0)), dz1 * u_.y * s1 * (1.f + g_.y * (1.f - s1)));
+            }
+#pragma unroll
+            for (uint32_t c = 0; c < 4; ++c) {
+              put16(slot, 4 * h + c, u[4 * c], u[4 * c + 1], u[4 * c + 2], u[4 * c + 3]);
+              put16(slot2, 4 * h + c, g[4 * c], g[4 * c + 1], g[4 * c + 2], g[4 * c + 3]);
+            }
+          }
+          fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) { tma_store_3d(&tmap_c, slot, col, y0, 0); tma_store_3d(&tmap_c2, slot2, col, y0, 0); bulk_commit(); }
+        }
+        if (!ok) break;
+      } else if (p.tma_store && p.epilogue == RTE_EPI_F32) {
         // ---- fp32 (+ residual): 32-column pieces; the residual of the next piece is fetched while this one is staged
         const float* Rf = reinterpret_cast<const float*>(p.R);
         float rres[32];
@@ -445,48 +503,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                       rte::pack_bf16x2(__uint_as_float(raw2[8 * c + 6]), __uint_as_float(raw2[8 * c + 7])));
               submit(&tmap_c, slot, col, y0, 0);
             }
-          }
-        } else if (p.tma_store && p.epilogue == RTE_EPI_SWIGLU_BWD) {
-          // ---- acc = dz; (d up | d gate) from the saved (up | gate): two 64-column pieces per 64 columns of dz.
-          // tmap_c views columns [0, F) of the output, tmap_c2 columns [F, 2F): each clips at its own edge.
-          const int F = p.pair_off;
-          for (int c0 = grp * HALF; c0 < (grp + 1) * HALF; c0 += 64) {
-            const int col = n0 + c0;
-            if (col >= p.N) break;
-            uint32_t dgp[32];                  // d gate of the 64 columns, packed, until d up has left
-            const uint32_t slot = acquire();
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const int cc = col + 32 * h;
-              uint32_t upk[16], gpk[16];
-              tmem_ld32(t_row + c0 + 32 * h, raw);
-              if (row_ok && cc < p.N) {
-                const __nv_bfloat16* ug = reinterpret_cast<const __nv_bfloat16*>(p.R) + size_t(row) * p.ldr;
-                load_bf16x32_packed(ug + cc, upk, p.N - cc);
-                load_bf16x32_packed(ug + F + cc, gpk, p.N - cc);
-              } else {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) { upk[j] = 0u; gpk[j] = 0u; }
-              }
-              tmem_ld_wait();
-              uint32_t dup[16];
-#pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                const float2 u_ = rte::unpack_bf16x2(upk[j]), g_ = rte::unpack_bf16x2(gpk[j]);
-                const float dz0 = __uint_as_float(raw[2 * j]), dz1 = __uint_as_float(raw[2 * j + 1]);
-                const float s0 = fast_sigmoid(g_.x), s1 = fast_sigmoid(g_.y);
-                dup[j] = rte::pack_bf16x2(dz0 * g_.x * s0, dz1 * g_.y * s1);
-                dgp[16 * h + j] = rte::pack_bf16x2(dz0 * u_.x * s0 * (1.f + g_.x * (1.f - s0)),
-                                                   dz1 * u_.y * s1 * (1.f + g_.y * (1.f - s1)));
-              }
-#pragma unroll
-              for (uint32_t c = 0; c < 4; ++c) put16(slot, 4 * h + c, dup[4 * c], dup[4 * c + 1], dup[4 * c + 2], dup[4 * c + 3]);
-            }
-            if (warp_rows) submit(&tmap_c, slot, col, y0, 0);
-            const uint32_t slot2 = acquire();
-#pragma unroll
-            for (uint32_t c = 0; c < 8; ++c) put16(slot2, c, dgp[4 * c], dgp[4 * c + 1], dgp[4 * c + 2], dgp[4 * c + 3]);
-            if (warp_rows) submit(&tmap_c2, slot2, col, y0, 0);
           }
         } else if (p.tma_store && p.epilogue == RTE_EPI_SWIGLU_FWD) {
           // ---- the tile holds BN/2 (up, gate) column pairs: columns [0, BN/2) = up_j, [BN/2, BN) = gate_j for hidden
@@ -680,7 +696,8 @@ float persistent_us(const rte_gemm_args* a, TileConfig t, int splits, int sms) {
   const int conc = (a->max_ctas > 0 ? a->max_ctas : sms) / t.ctas, waves = rte::ceil_div(units, conc > 0 ? conc : 1);
   const float kb = float(rte::ceil_div(rte::ceil_div(a->K, BK), splits));
   const float slope = waves > 1 ? slope_busy[i] : slope_idle[i] + (slope_busy[i] - slope_idle[i]) * float(units) / float(conc);
-  const float store = store_bf16[i] * (res ? 3.8f : f32 ? 2.f : 1.f);
+  static const float store_swb[4] = {9.f, 9.f, 5.3f, 5.3f};                // SwiGLU's backward: (up | gate) in, (d up | d gate) out
+  const float store = a->epilogue == RTE_EPI_SWIGLU_BWD ? store_swb[i] : store_bf16[i] * (res ? 3.8f : f32 ? 2.f : 1.f);
   const float loop = kb * slope;
   return (res ? base_res[i] : f32 ? base_f32[i] : base_bf16[i]) + loop + float(waves - 1) * (loop > store ? loop : store);
 }
@@ -707,7 +724,8 @@ float small_us(const rte_gemm_args* a) {
 
 TileConfig pick_tile(const rte_gemm_args* a, int splits, int sms, float* us = nullptr) {
   const bool grouped = a->tile_group != nullptr || a->split_kblocks != nullptr;   // per-128-row-block bookkeeping
-  TileConfig best = {256, 1};
+  const bool swb = a->epilogue == RTE_EPI_SWIGLU_BWD;
+  TileConfig best = {swb ? 128 : 256, 1};
   float best_us = 1e30f;
   for (int bn = 128; bn <= 256; bn += 128)
     for (int ctas = 1; ctas <= 2; ++ctas) {
@@ -715,6 +733,7 @@ TileConfig pick_tile(const rte_gemm_args* a, int splits, int sms, float* us = nu
       if (ctas == 1 && a->cta_pair == 2 && !grouped && a->M > BM) continue;
       if ((a->tile_n == 128 || a->tile_n == 256) && bn != a->tile_n) continue;
       if (a->epilogue == RTE_EPI_SWIGLU_FWD && bn != 256) continue;            // the paired epilogue takes 64 (up, gate) pairs per warp
+      if (swb && bn == 256 && ctas == 1) continue;                             // two stages would be left of its shared memory
       const float t = persistent_us(a, {bn, ctas}, splits, sms);
       if (t < best_us) { best_us = t; best = {bn, ctas}; }
     }
@@ -739,14 +758,14 @@ Choice choose(const rte_gemm_args* a, int splits, int sms) {
 }
 
 // Work units (CTAs or CTA pairs) that can run at the same time under `max_ctas`.
-template <int BN, int CTAS>
+template <int BN, int CTAS, bool SWB = false>
 int concurrent_units(int max_ctas, int sm_count) {
-  using L = SmemLayout<BN, CTAS>;
+  using L = SmemLayout<BN, CTAS, SWB>;
   int ctas = max_ctas > 0 ? max_ctas : sm_count;
   if (CTAS == 1) return ctas;
   static int max_clusters = -1;
   if (max_clusters < 0) {
-    if (cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, CTAS, SWB>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL) != cudaSuccess)
       return ctas / 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(sm_count / 2 * 2));
@@ -757,26 +776,26 @@ int concurrent_units(int max_ctas, int sm_count) {
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_tcgen05_kernel<BN, CTAS>, &cfg) == cudaSuccess && n > 0) max_clusters = n;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_tcgen05_kernel<BN, CTAS, SWB>, &cfg) == cudaSuccess && n > 0) max_clusters = n;
     else { (void)cudaGetLastError(); max_clusters = sm_count / 2; }
   }
   int units = ctas / 2;
   return units < max_clusters ? units : max_clusters;
 }
 
-template <int BN, int CTAS>
+template <int BN, int CTAS, bool SWB = false>
 int launch(const rte_gemm_args* a, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc,
-           const CUtensorMap& tc2, KParams& kp, int sm_count, cudaStream_t st) {
-  using L = SmemLayout<BN, CTAS>;
+           const CUtensorMap& tc2, const CUtensorMap& tr, const CUtensorMap& tr2, KParams& kp, int sm_count, cudaStream_t st) {
+  using L = SmemLayout<BN, CTAS, SWB>;
   static_assert(L::STAGES >= 3, "too few pipeline stages fit");
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, CTAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, CTAS, SWB>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL) != cudaSuccess)
       return RTE_ERR_LAUNCH;
     attr_set = true;
   }
   const int total = kp.num_m_blocks * kp.num_n_blocks * kp.splits;
-  int units = concurrent_units<BN, CTAS>(a->max_ctas, sm_count);
+  int units = concurrent_units<BN, CTAS, SWB>(a->max_ctas, sm_count);
   if (units > total) units = total;
   if (units < 1) units = 1;
   cudaLaunchConfig_t cfg = {};
@@ -790,7 +809,7 @@ int launch(const rte_gemm_args* a, const CUtensorMap& ta, const CUtensorMap& tb,
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = CTAS; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr; cfg.numAttrs = (CTAS == 2) ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, CTAS>, ta, tb, tc, tc2, kp) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, CTAS, SWB>, ta, tb, tc, tc2, tr, tr2, kp) != cudaSuccess) {
     (void)cudaGetLastError();
     return RTE_ERR_LAUNCH;
   }
@@ -916,7 +935,7 @@ extern "C" int rte_gemm_bf16(const rte_gemm_args* a, rte_stream_t stream) {
 
   // Outputs through TMA bulk stores whenever their addresses and strides allow it (16-byte rules of the TMA);
   // otherwise the epilogue writes with plain vector stores.
-  CUtensorMap tc = ta, tc2 = ta;
+  CUtensorMap tc = ta, tc2 = ta, tr = ta, tr2 = ta;
   const bool out_f32 = a->epilogue == RTE_EPI_F32;
   const long long es = out_f32 ? 4 : 2;
   auto aligned = [&](const void* ptr, long long ld) { return ptr && (reinterpret_cast<uintptr_t>(ptr) & 15) == 0 && (ld * es) % 16 == 0; };
@@ -924,7 +943,7 @@ extern "C" int rte_gemm_bf16(const rte_gemm_args* a, rte_stream_t stream) {
   if (splits > 1) tma_ok = tma_ok && (a->split_stride * es) % 16 == 0;
   if (out_f32 && a->R != nullptr) tma_ok = tma_ok && (reinterpret_cast<uintptr_t>(a->R) & 15) == 0 && (a->ldr % 4) == 0;
   if (swiglu_f) tma_ok = tma_ok && aligned(a->C2, a->ldc2);
-  if (swiglu_b) tma_ok = tma_ok && (a->N % 8 == 0) && (reinterpret_cast<uintptr_t>(a->R) & 15) == 0 && (a->ldr % 8) == 0;
+  if (swiglu_b) tma_ok = tma_ok && a->tile_group == nullptr && (a->N % 8 == 0) && (reinterpret_cast<uintptr_t>(a->R) & 15) == 0 && (a->ldr % 8) == 0;
   if (tma_ok) {
     const long long plane = splits > 1 ? a->split_stride : (long long)a->M * a->ldc;
     if (swiglu_f) {
@@ -934,6 +953,9 @@ extern "C" int rte_gemm_bf16(const rte_gemm_args* a, rte_stream_t stream) {
       rc = make_store_tmap(&tc, a->C, a->M, a->N, a->ldc, 1, (long long)a->M * a->ldc, false);
       if (rc == RTE_OK)
         rc = make_store_tmap(&tc2, reinterpret_cast<const __nv_bfloat16*>(a->C) + a->N, a->M, a->N, a->ldc, 1, (long long)a->M * a->ldc, false);
+      const __nv_bfloat16* r = reinterpret_cast<const __nv_bfloat16*>(a->R);
+      if (rc == RTE_OK) rc = make_store_tmap(&tr, r, a->M, a->N, a->ldr, 1, (long long)a->M * a->ldr, false);
+      if (rc == RTE_OK) rc = make_store_tmap(&tr2, r + a->N, a->M, a->N, a->ldr, 1, (long long)a->M * a->ldr, false);
     } else {
       rc = make_store_tmap(&tc, a->C, a->M, a->N, a->ldc, splits, plane, out_f32);
     }
@@ -943,7 +965,13 @@ extern "C" int rte_gemm_bf16(const rte_gemm_args* a, rte_stream_t stream) {
   if (DIAG && (kp.diag & 16)) kp.tma_store = 0;
 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (swiglu_b && tma_ok && !(DIAG && (kp.diag & 16)) && !(bn == 256 && ctas == 1)) {
+    if (ctas == 1) return launch<128, 1, true>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st);
+    return bn == 256 ? launch<256, 2, true>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st)
+                     : launch<128, 2, true>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st);
+  }
+  if (swiglu_b) kp.tma_store = 0;
   if (ctas == 2)
-    return bn == 256 ? launch<256, 2>(a, ta, tb, tc, tc2, kp, sms, st) : launch<128, 2>(a, ta, tb, tc, tc2, kp, sms, st);
-  return bn == 256 ? launch<256, 1>(a, ta, tb, tc, tc2, kp, sms, st) : launch<128, 1>(a, ta, tb, tc, tc2, kp, sms, st);
+    return bn == 256 ? launch<256, 2>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st) : launch<128, 2>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st);
+  return bn == 256 ? launch<256, 1>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st) : launch<128, 1>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st);
 }

@@ -966,10 +966,11 @@ class TrainEngine:
     def _router_grad_names() -> list[str]:
         return [f"router.{m}.{i}.{k}" for m in ("recipe_mlp", "depth_mlp") for i in (0, 2) for k in ("weight", "bias")]
 
-    def _fuse_swiglu(self, rows: int) -> bool:
+    def _fuse_swiglu(self, rows: int, backward: bool = False) -> bool:
         """SwiGLU inside the tcgen05 GEMM's epilogue for large activations (swiglu_fuse_max_rows = 0: never).  Below the line
         the separate pass finds its input in L2 and the product can take the kernels for few tiles."""
-        return self.swiglu_fuse_max_rows > 0 and rows * self.cfg.d_ff >= getattr(self.ops, "swiglu_fuse_min", 0)
+        return self.swiglu_fuse_max_rows > 0 and rows * self.cfg.d_ff >= getattr(
+            self.ops, "swiglu_fuse_min_bwd" if backward else "swiglu_fuse_min", 0)
 
     def _block_fwd(self, blk: _Block, x_in: torch.Tensor) -> torch.Tensor:
         o, cfg, p, sh, M = self.ops, self.cfg, self.params, self.shadow, blk.M
@@ -1000,7 +1001,7 @@ class TrainEngine:
         d, f, pre = cfg.d_model, cfg.d_ff, blk.prefix.split("@")[0]
         ready = self._grad_ready if mark_ready else (lambda *names: None)
         # --- MLP: x_out = u + wd(up * silu(gate)),  (up | gate) = wug(norm2(u))
-        if self._fuse_swiglu(M):
+        if self._fuse_swiglu(M, backward=True):
             o.gemm(dout16, sh[f"{pre}.mlp.wd.weight"], t.dug, M=M, N=f, K=d, b_mn=True, epilogue=A.EPI_SWIGLU_BWD,
                    residual=blk.ug, pair=f)
         else:

@@ -59,9 +59,11 @@ class CudaOps:
         self._split_counters = torch.zeros(1024, dtype=torch.int32, device=self.device)      # per-tile arrival counters
         self.few_rows_max_splits = int(os.environ.get("RTE_FEWROW_SPLITS", "4"))
         # hidden activations (rows x d_ff) from which a product carries the SwiGLU pass in its epilogue.  us, separate -> fused:
-        # 8192 x 512 -> 2048 forward 54.6 -> 45.6, backward 53.7 -> 51.0; 8192 x 1024 -> 4096 138 -> 112, 114 -> 94; 6144 x 512
-        # -> 2048 42.3 -> 38.8, 40.2 -> 39.8; 8192 x 256 -> 1024 23.2 -> 25.7, 20.7 -> 21.8; 512 x 128 -> 512 5.3 -> 8.8
+        # forward 8192 x 512 -> 2048 53.8 -> 46.0, 6144 x 512 -> 2048 42.0 -> 39.0; 8192 x 256 -> 1024 23.1 -> 25.9, 512 x 128 ->
+        # 512 5.4 -> 8.8; backward (its operands come by TMA, so it pays earlier) 8192 x 512 -> 2048 53.7 -> 37.3, 8192 x 256 ->
+        # 1024 20.8 -> 17.3, 1000 x 256 -> 1024 7.8 -> 6.7; 512 x 128 -> 512 4.9 -> 6.0
         self.swiglu_fuse_min = 12_000_000
+        self.swiglu_fuse_min_bwd = 1_000_000
         self.gemm_max_ctas = 0     # 0 = one persistent CTA per SM; smaller values leave SMs to kernels of other streams
         # tile hints passed to every GEMM (0 = the library's choice of kernel and tile): RTE_GEMM_PAIR=0 keeps every tile on
         # one CTA of the persistent kernel, RTE_GEMM_TILE_N forces it with 128 or 256 columns per tile

@@ -208,6 +208,24 @@ def test_swiglu_epilogues(ops, M, d, f):
     _close(dug[:, f:], dz * ups * sg * (1 + gts * (1 - sg)), 1.5e-2, "d gate")
 
 
+@pytest.mark.parametrize("M,d,f", [(1, 64, 64), (129, 72, 200), (300, 128, 520), (5000, 136, 1000), (40000, 64, 264)])
+def test_swiglu_backward_operand_pieces(ops, M, d, f):
+    """Pieces that the tile's or the matrix's edge cuts, fewer and more tiles than CTAs, each tile the epilogue has."""
+    g = torch.Generator().manual_seed(M)
+    dout, wd, ug = _bf(torch.randn(M, d, generator=g)), _bf(torch.randn(d, f, generator=g) * 0.05), _bf(torch.randn(M, 2 * f, generator=g))
+    dz, up, gate = dout.float() @ wd.float(), ug[:, :f].float(), ug[:, f:].float()
+    sg = torch.sigmoid(gate)
+    want = torch.cat([dz * gate * sg, dz * up * sg * (1 + gate * (1 - sg))], 1)
+    for tile_n, pair in [(0, 0), (128, 1), (128, 2), (256, 2)]:
+        dug = torch.full((M + 2, 2 * f), 7.0, dtype=torch.bfloat16, device=DEV)
+        ops.gemm(dout.to(DEV), wd.to(DEV), dug, M=M, N=f, K=d, b_mn=True, epilogue=3, residual=ug.to(DEV), pair=f,
+                 tile_n=tile_n, cta_pair=pair)
+        torch.cuda.synchronize()
+        ops.check_status()
+        _close(dug[:M], want, 1.5e-2, "(d up | d gate)")
+        assert (dug[M:] == 7).all()
+
+
 # ------------------------------------------------------------------ norm / CE / embedding
 @pytest.mark.parametrize("rows,d", [(64, 128), (1000, 512), (333, 1024), (17, 64)])
 def test_rmsnorm_fwd_bwd(ops, rows, d):
