@@ -478,3 +478,18 @@ def test_deferred_grouped_exact_mode_follows_the_reference(fused, monkeypatch):
     two_banks = ExperimentConfig(ModelConfig(**{**case["model"], "ffn_banks": 2}), TrainingConfig(**case["train"]), OutputConfig())
     with pytest.raises(NotImplementedError, match="ffn_banks"):
         TrainEngine(two_banks, params, device="cpu", ops=EmulOps(), use_cuda_graph=False)
+
+
+def test_swiglu_backward_keeps_fp32_hidden_gradients_up_to_the_row_limit():
+    """`swiglu_fuse_max_rows` is a line in rows: beyond the few-row kernel's range and up to it, backward's hidden gradient is
+    not rounded to bf16 between two passes, whatever the width; larger activations fuse by size; 0 switches fusion off."""
+    cfg, _, _ = _pair("dense")
+    params = init_parameters(cfg.model, seed=0, num_clusters=cfg.output.num_clusters)
+    for limit in (0, 1024, 4096):
+        eng = TrainEngine(cfg, params, device="cpu", ops=EmulOps(), use_cuda_graph=False, swiglu_fuse_max_rows=limit)
+        eng.ops.small_gemm_rows, eng.ops.swiglu_fuse_min, eng.ops.swiglu_fuse_min_bwd = 256, 12_000_000, 1_000_000
+        f = cfg.model.d_ff
+        for rows in (1, 256, 257, 512, 1024, 1025, 4096, 4097, -(-1_000_000 // f), -(-12_000_000 // f)):
+            by_size = limit > 0 and rows * f >= 1_000_000
+            assert eng._fuse_swiglu(rows, backward=True) == (by_size or 256 < rows <= limit), (limit, rows)
+            assert eng._fuse_swiglu(rows) == (limit > 0 and rows * f >= 12_000_000), (limit, rows)
