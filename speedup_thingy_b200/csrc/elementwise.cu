@@ -470,14 +470,18 @@ __device__ __forceinline__ int ce_target(const int64_t* targets, int row, int V,
   if (status && threadIdx.x == 0) atomicExch(status, RTE_DEV_INDEX_OUT_OF_RANGE);
   return 0;
 }
-// (maximum, sum of exponentials) of the row from every warp's
+// Exponentials are taken relative to a maximum that may be -inf (columns masked out, or nothing but NaN, which a maximum
+// passes over): relative to zero then, so that exp(-inf) is 0 and a NaN stays one and reaches the sum.
+__device__ __forceinline__ float ce_reference(float m) { return m == -INFINITY ? 0.f : m; }
+
+// (maximum, sum of exponentials) of the row from every warp's; a warp without a finite column brings 0, or NaN
 template <int WARPS>
 __device__ __forceinline__ float ce_lse(const float (&red_m)[WARPS], const float (&red_s)[WARPS]) {
   float mx = red_m[0], se = 0.f;
 #pragma unroll
   for (int w = 1; w < WARPS; ++w) mx = fmaxf(mx, red_m[w]);
 #pragma unroll
-  for (int w = 0; w < WARPS; ++w) se += red_m[w] == -INFINITY ? 0.f : red_s[w] * __expf(red_m[w] - mx);      // (a warp without columns)
+  for (int w = 0; w < WARPS; ++w) se += red_m[w] == -INFINITY ? red_s[w] : red_s[w] * __expf(red_m[w] - mx);
   return mx + __logf(se);
 }
 
@@ -517,6 +521,7 @@ ce_row_kernel(const T* __restrict__ logits, int ldl, const int64_t* __restrict__
       for (int j = 0; j < W; ++j) m = fmaxf(m, e[i][j]);
     }
   m = rte::warp_max(m);
+  const float ref = ce_reference(m);
   float s = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i)
@@ -527,7 +532,7 @@ ce_row_kernel(const T* __restrict__ logits, int ldl, const int64_t* __restrict__
           if (j == tj) target_logit = e[i][j];
       }
 #pragma unroll
-      for (int j = 0; j < W; ++j) s += e[i][j] = __expf(e[i][j] - m);
+      for (int j = 0; j < W; ++j) s += e[i][j] = __expf(e[i][j] - ref);
     }
   s = warp_sum(s);
   if (lane == 0) { red_m[warp] = m; red_s[warp] = s; }
@@ -535,7 +540,8 @@ ce_row_kernel(const T* __restrict__ logits, int ldl, const int64_t* __restrict__
   const float lse = ce_lse(red_m, red_s);
   if (threadIdx.x == 0) loss_tok[row] = lse - target_logit;
   if (dlogits == nullptr) return;
-  const float wgt = row_weight[row / S], scale = wgt * __expf(m - lse);
+  // (a warp without a finite column: zeros, whatever lse is, unless the whole row has none)
+  const float wgt = row_weight[row / S], scale = m == -INFINITY ? wgt + (lse - lse) : wgt * __expf(m - lse);
   T* dr = dlogits + (size_t)row * ldl;
   const bool whole = EVEN || ce_offset(dr) == off;
 #pragma unroll
@@ -585,14 +591,13 @@ ce_stream_kernel(const T* __restrict__ logits, int ldl, const int64_t* __restric
 #pragma unroll
         for (int j = 1; j < W; ++j) gm = fmaxf(gm, v[j]);
         if (gm > m) { s *= __expf(m - gm); m = gm; }
-        if (m > -INFINITY) {
+        const float ref = ce_reference(m);
 #pragma unroll
-          for (int j = 0; j < W; ++j) s += __expf(v[j] - m);
-        }
+        for (int j = 0; j < W; ++j) s += __expf(v[j] - ref);
       }
   }
   const float wm = rte::warp_max(m);
-  s = warp_sum(m == -INFINITY ? 0.f : s * __expf(m - wm));
+  s = warp_sum(m == -INFINITY ? s : s * __expf(m - wm));
   if (lane == 0) { red_m[warp] = wm; red_s[warp] = s; }
   __syncthreads();
   const float lse = ce_lse(red_m, red_s);

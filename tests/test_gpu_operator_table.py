@@ -326,6 +326,33 @@ def test_cross_entropy_row_widths(rows, V, dtype):
     assert torch.allclose(x.grad.cpu().float(), ref.grad, atol=1e-5, rtol=1e-2 if dtype == torch.bfloat16 else 1e-4)
 
 
+@pytest.mark.parametrize("V,dtype", [(512, torch.bfloat16), (511, torch.bfloat16), (8192, torch.bfloat16), (9001, torch.bfloat16), (16384, torch.bfloat16),
+                                     (512, torch.float32), (4099, torch.float32), (8192, torch.float32)])
+@pytest.mark.parametrize("level,fill", [(0.0, "-inf"), (-300.0, "-inf"), (0.0, "lowest")])
+def test_cross_entropy_of_masked_and_nan_columns(V, dtype, level, fill):
+    """Rows whose unmasked logits sit in one thread's, one warp's or half of the columns, at zero and far below it: the masked
+    columns' gradient is exactly zero, loss and gradient are the plain row's.  A block of NaN logits makes the loss NaN."""
+    gen = torch.Generator().manual_seed(V)
+    keeps = [(0, 4), (0, V // 2), (V // 2, V), (V - 3, V)]
+    x = (level + torch.randn(len(keeps), V, generator=gen)).to(dtype)
+    targets = torch.tensor([b - 1 for _, b in keeps])
+    fill = -torch.inf if fill == "-inf" else torch.finfo(dtype).min
+    for r, (a, b) in enumerate(keeps):
+        x[r, :a] = x[r, b:] = fill
+    ref = x.float().requires_grad_(True)
+    loss = torch.nn.functional.cross_entropy(ref, targets, reduction="none")
+    loss.sum().backward()
+    got = x.cuda().requires_grad_(True)
+    out = K.k_cross_entropy_unreduced(got, targets.cuda())
+    out.sum().backward()
+    assert torch.allclose(out.detach().cpu(), loss.detach(), atol=1e-4, rtol=1e-5)
+    g = got.grad.cpu().float()
+    assert (g[x == fill] == 0).all() and torch.allclose(g, ref.grad, atol=1e-5, rtol=1e-2 if dtype == torch.bfloat16 else 1e-4)
+    bad = x.clone()
+    bad[x == fill] = torch.nan
+    assert K.k_cross_entropy_unreduced(bad.cuda(), targets.cuda()).isnan().all()
+
+
 @pytest.mark.parametrize("d", [4, 132, 512, 2048])
 @pytest.mark.parametrize("xt,wt,rt", [(torch.bfloat16, torch.bfloat16, None), (torch.bfloat16, torch.float32, torch.float32), (torch.float32, torch.bfloat16, torch.bfloat16),
                                       (torch.float16, torch.float32, None)])
