@@ -150,15 +150,18 @@ std::vector<int64_t> with_last(c10::IntArrayRef sizes, int64_t n) {
   return s;
 }
 
+// Kernels that take 16 bytes at a time: a contiguous tensor on a 16-byte boundary (a view into the middle of a buffer is
+// copied; torch's own allocations start on 512).
+Tensor on16(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 ? t.clone() : t; }
+
 // --------------------------------------------------------------------------- RMSNorm
 struct RmsNorm : Function<RmsNorm> {
+  static Tensor plain(const Tensor& t) {       // contiguous bf16 or fp32 on a 16-byte boundary
+    const Tensor u = t.contiguous();
+    return on16(direct(u.scalar_type()) ? u : u.to(F32));
+  }
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const OptTensor& residual, double eps) {
     Dev dev(x);
-    auto plain = [](const Tensor& t) {         // contiguous bf16 or fp32 on a 16-byte boundary
-      Tensor u = t.contiguous();
-      if (!direct(u.scalar_type())) u = u.to(F32);
-      return reinterpret_cast<uintptr_t>(u.data_ptr()) % 16 ? u.clone() : u;
-    };
     const Tensor xc = plain(x), wc = plain(weight), rc = residual ? plain(residual->expand(x.sizes())) : Tensor();
     const auto d = x.size(-1), rows = x.numel() / d;
     const auto out_t = at::result_type(x, weight), sum_t = residual ? at::result_type(x, *residual) : x.scalar_type();
@@ -186,9 +189,8 @@ struct RmsNorm : Function<RmsNorm> {
     const auto types = ctx->saved_data["types"].toIntVector();
     const bool has_res = types[2] >= 0;
     const auto d = y.size(-1), rows = y.numel() / d;
-    Tensor dy = grads[0].defined() ? grads[0].contiguous() : torch::zeros_like(y);
-    if (!direct(dy.scalar_type())) dy = dy.to(F32);
-    Tensor dres = has_res && grads.size() > 1 && grads[1].defined() ? grads[1].to(F32).contiguous() : Tensor();
+    const Tensor dy = grads[0].defined() ? plain(grads[0]) : torch::zeros_like(y);
+    const Tensor dres = has_res && grads.size() > 1 && grads[1].defined() ? plain(grads[1].to(F32)) : Tensor();
     const auto x_t = at::ScalarType(types[0]);
     const bool x16 = x_t == BF;
     const bool need_f32 = !x16 || (has_res && at::ScalarType(types[2]) != BF);
@@ -287,7 +289,7 @@ struct Attention : Function<Attention> {
     const auto dims = ctx->saved_data["dims"].toIntVector();
     const auto B = dims[0], H = dims[1], S = dims[2], hd = dims[3];
     Tensor dy = g[0].permute({0, 2, 1, 3});
-    dy = to_bf16(dev, {dy})[0].view({B * S, H * hd});
+    dy = on16(to_bf16(dev, {dy})[0]).view({B * S, H * hd});
     const Tensor dqkv = at::empty_like(qkv);
     check(rte_attn_bwd(ptr(qkv), 3 * H * hd, H * hd, ptr(y), ptr(dy), H * hd, f32(lse), ptr(dqkv), f32(saved[3]), B, S, H, hd, dev.st), "rte_attn_bwd");
     const Tensor all = dqkv.view({B, S, 3, H, hd}).permute({2, 0, 3, 1, 4}).to(at::ScalarType(dims[4]));

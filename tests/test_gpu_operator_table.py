@@ -405,6 +405,26 @@ def test_rope_and_attention_take_strided_views(layout, dtype):
     assert out.dtype == dtype and torch.allclose(out.cpu().float(), ref, atol=3e-2, rtol=3e-2)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gradients_off_the_16_byte_grid(dtype):
+    """A gradient that is a contiguous view one element into its buffer: the results of an aligned one."""
+    gen = torch.Generator().manual_seed(1)
+
+    def both(run, shape):
+        base = torch.randn(shape, generator=gen).to(dtype).cuda()
+        odd = torch.cat([base.new_zeros(1), base.view(-1)])[1:].view(shape)
+        assert odd.data_ptr() % 16 and odd.is_contiguous()
+        for a, b in zip(run(base), run(odd)):
+            assert torch.equal(a, b)
+
+    x, w, r = (torch.randn(*s, generator=gen).to(dtype).cuda().requires_grad_() for s in ((9, 64), (64,), (9, 64)))
+    out, total = K.k_fused_rmsnorm(x, w, r)
+    both(lambda g: torch.autograd.grad((out, total), (x, w, r), (g, g), retain_graph=True), (9, 64))
+    q, k, v = (torch.randn(2, 33, 3, 32, generator=gen).to(dtype).cuda().transpose(1, 2).requires_grad_() for _ in range(3))
+    y = K.k_flash_causal_dense(q, k, v).transpose(1, 2)
+    both(lambda g: torch.autograd.grad(y, (q, k, v), g, retain_graph=True), (2, 33, 3, 32))
+
+
 @pytest.mark.parametrize("N,d,m", [(5901, 64, 2048), (5800, 64, 2048)])
 def test_packed_swiglu_on_both_sides_of_the_fusion_rule(N, d, m):
     gen = torch.Generator().manual_seed(N)
