@@ -516,6 +516,18 @@ void cast_into(const Dev& dev, const Tensor& src, const Tensor& dst) {
   else dst.copy_(src);
 }
 
+// What a caller hands a module beside x is read and written through raw pointers sized by the module: checked here, before
+// any launch.
+void is_dense_f32(const Tensor& t, const Tensor& like, int64_t numel, const char* what) {
+  TORCH_CHECK_VALUE(t.device() == like.device() && t.scalar_type() == F32 && t.is_contiguous() && t.numel() == numel, what,
+                    " must be a contiguous fp32 tensor of ", numel, " elements on ", like.device(), ", got ", t.sizes(), " ", t.scalar_type(), " on ", t.device());
+}
+Tensor token_rows(const Tensor& x, int64_t d) {
+  TORCH_CHECK_VALUE(x.dim() > 0 && x.size(-1) == d, "the last dimension must be d_model = ", d, ", got ", x.sizes());
+  const Tensor flat = x.reshape({-1, d}).contiguous();
+  return direct(flat.scalar_type()) ? flat : flat.to(F32);
+}
+
 struct PoolModule {
   Tensor status, selector16, centers, idx_ug, idx_d, ug_ptr, ug_rows, d_ptr, d_rows, wdT16, wug_pool, wd_pool, q, assign, pos, perm, tile_group, counts,
       offsets, kblocks, x16, xp, ugp, zp, yp, dyp, dzp, dugp, dxp, dwug_pool, dwd_pool, dwdT;
@@ -553,11 +565,17 @@ struct PoolModule {
 
   Tensor forward(const Tensor& x, const Tensor& wug, const Tensor& wd, const OptTensor& assignments) {
     Dev dev(x, status);
-    Tensor flat = x.reshape({-1, d}).contiguous();
-    if (!direct(flat.scalar_type())) flat = flat.to(F32);
-    const auto N = tokens = flat.size(0);
+    const Tensor flat = token_rows(x, d);
+    const auto N = flat.size(0);
+    TORCH_CHECK_VALUE(N <= x16.size(0), N, " tokens exceed max_tokens=", x16.size(0));
+    is_dense_f32(wug, x, 2 * F * d, "wug");
+    is_dense_f32(wd, x, F * d, "wd");
+    if (assignments)
+      TORCH_CHECK_VALUE(assignments->device() == x.device() && assignments->numel() == N, "assignments must name the cluster of each of the ", N, " tokens on ",
+                        x.device(), ", got ", assignments->sizes(), " on ", assignments->device());
+    tokens = N;
     Tensor a = assign.narrow(0, 0, N);
-    if (assignments) a = assignments->to(torch::kInt32).contiguous();
+    if (assignments) a = assignments->to(torch::kInt32).contiguous().view({-1});
     else route(dev, flat);
     pack(dev, a);
     prepare_pools(dev, wug, wd);
@@ -572,8 +590,10 @@ struct PoolModule {
 
   Tensor backward(const Tensor& dout, const Tensor& dwug, const Tensor& dwd, bool accumulate) {
     Dev dev(dout, status);
-    Tensor flat = dout.reshape({-1, d}).contiguous();
-    if (!direct(flat.scalar_type())) flat = flat.to(F32);
+    const Tensor flat = token_rows(dout, d);
+    TORCH_CHECK_VALUE(flat.size(0) == tokens, "the gradient of ", tokens, " tokens has ", flat.size(0), " rows");
+    is_dense_f32(dwug, dout, 2 * F * d, "dwug");
+    is_dense_f32(dwd, dout, F * d, "dwd");
     gather(dev, flat, perm, dyp);
     Gemm(dev, ptr(dyp), d, false, ptr(wd_pool), d, false, ptr(dzp), Mc, cap, Mc, d, RTE_EPI_BF16).groups(tile_group, C, Mc).run();
     check(rte_swiglu_bwd(ptr(ugp), ptr(dzp), ptr(dugp), cap, Mc, dev.st), "rte_swiglu_bwd");
@@ -606,9 +626,13 @@ struct SvdModule {
 
   Tensor forward(const Tensor& x, const Tensor& w_up, const Tensor& w_gate, const Tensor& w_down) {
     Dev dev(x, status);
-    Tensor flat = x.reshape({-1, d}).contiguous();
-    if (!direct(flat.scalar_type())) flat = flat.to(F32);
-    const auto N = tokens = flat.size(0);
+    const Tensor flat = token_rows(x, d);
+    const auto N = flat.size(0);
+    TORCH_CHECK_VALUE(N <= x16.size(0), N, " tokens exceed max_tokens=", x16.size(0));
+    is_dense_f32(w_up, x, F * d, "w_up");
+    is_dense_f32(w_gate, x, F * d, "w_gate");
+    is_dense_f32(w_down, x, F * d, "w_down");
+    tokens = N;
     const auto* qb = static_cast<char*>(ptr(q16));
     auto* hb = f32(hats);
     {
@@ -634,9 +658,11 @@ struct SvdModule {
   // dw_up and dw_gate may be the two halves of one [2F, d] tensor: the product then writes them itself
   Tensor backward(const Tensor& dout, const Tensor& dw_up, const Tensor& dw_gate, const Tensor& dw_down) {
     Dev dev(dout, status);
-    const Tensor flat = dout.reshape({-1, d}).contiguous();
+    const Tensor flat = token_rows(dout, d);
     const auto N = tokens;
-    cast_into(dev, direct(flat.scalar_type()) ? flat : flat.to(F32), dout16.narrow(0, 0, N));
+    TORCH_CHECK_VALUE(flat.size(0) == N, "the gradient of ", N, " tokens has ", flat.size(0), " rows");
+    is_dense_f32(dw_down, dout, F * d, "dw_down");
+    cast_into(dev, flat, dout16.narrow(0, 0, N));
     Gemm(dev, ptr(dout16), d, false, ptr(wd16), d, false, ptr(dz), F, N, F, d, RTE_EPI_BF16).run();
     check(rte_svd_ffn_swiglu_bwd(ptr(ug), ptr(dz), static_cast<uint8_t*>(ptr(selected)), ptr(dug), N, F, dev.st), "rte_svd_ffn_swiglu_bwd");
     const Tensor dx = empty({N, d}, F32, dout);

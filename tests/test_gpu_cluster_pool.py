@@ -148,3 +148,36 @@ def test_c3_shaped_pools_against_the_oracle():
     _close(xg.grad, xr.grad)
     _close(m.wug.grad, wug.grad)
     _close(m.wd.grad, wd.grad)
+
+
+def test_what_the_buffers_cannot_hold_is_refused_before_a_launch():
+    """Assignments of another device or length, weights and gradient outputs that are no dense fp32 tensors of their shape,
+    tokens of another width: a ValueError, and the module still works."""
+    t = cluster_pool_inputs()
+    m = _module(t, 256)
+    x = t["x"].reshape(-1, 64)[:200].to(DEV)
+    ids = torch.from_numpy(GOLD["assignments"])[:200].to(DEV, torch.int32)
+    want = m.forward(x, ids)
+    for bad in (ids.cpu(), ids[:-1], torch.cat([ids, ids])):
+        with pytest.raises(ValueError, match="assignments"):
+            m.forward(x, bad)
+    assert torch.equal(m.forward(x, ids.long()), want)              # any integer type
+    for name in ("wug", "wd"):
+        good = getattr(m, name)
+        for bad in (good.bfloat16(), good.cpu(), good.t(), good[:-1]):
+            setattr(m, name, bad)
+            with pytest.raises(ValueError, match=name):
+                m.forward(x, ids)
+        setattr(m, name, good)
+    with pytest.raises(ValueError, match="last dimension"):
+        m.forward(x.view(100, 128), ids[:100])
+    assert torch.equal(m.forward(x, ids), want)
+    dw = [torch.empty_like(m.wug), torch.empty_like(m.wd)]
+    with pytest.raises(ValueError, match="rows"):
+        m.backward(x[:100], *dw)
+    with pytest.raises(ValueError, match="dwug"):
+        m.backward(x, dw[0].bfloat16(), dw[1])
+    with pytest.raises(ValueError, match="dwd"):
+        m.backward(x, dw[0], dw[1].t())
+    m.backward(x, *dw)
+    m.ops.check_status()

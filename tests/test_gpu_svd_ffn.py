@@ -148,3 +148,27 @@ def test_c4_shaped_module_against_the_oracle():
     # and the fp32 oracle's own selection overlaps almost everywhere
     _, sel32 = O.svd_sparse_ffn(x, t["w_up"], t["w_gate"], t["w_down"], t["up_a"], t["up_b"], t["gate_a"], t["gate_b"], **c)
     assert (sel & sel32).sum() >= 0.93 * sel32.sum()
+
+
+def test_what_the_buffers_cannot_hold_is_refused_before_a_launch():
+    c, t = SVD_FFN, svd_ffn_inputs()
+    m = _module(t, c, 64)
+    x = t["x"].to(DEV)
+    want = m.forward(x)
+    for name in ("w_up", "w_gate", "w_down"):
+        good = getattr(m, name)
+        for bad in (good.bfloat16(), good.cpu(), good.t(), good[:-1]):
+            setattr(m, name, bad)
+            with pytest.raises(ValueError, match=name):
+                m.forward(x)
+        setattr(m, name, good)
+    with pytest.raises(ValueError, match="last dimension"):
+        m.forward(x.reshape(-1, m.d)[:32].reshape(16, 2 * m.d))
+    assert torch.equal(m.forward(x), want)
+    dw = [torch.empty_like(m.w_up) for _ in range(3)]
+    with pytest.raises(ValueError, match="rows"):
+        m.backward(want.reshape(-1, m.d)[:-1], *dw)
+    with pytest.raises(ValueError, match="dw_down"):
+        m.backward(want, dw[0], dw[1], dw[2].bfloat16())
+    m.backward(want, *dw)
+    m.ops.check_status()
