@@ -252,14 +252,19 @@ struct Rope : Function<Rope> {
     const auto S = q.size(-2), hd = q.size(-1);
     const Tensor c = cos.to(F32).contiguous().view({S, hd}), s = sin.to(F32).contiguous().view({S, hd});
     ctx->save_for_backward({c, s});
+    ctx->saved_data["q"] = q.sizes().vec();
+    ctx->saved_data["k"] = k.sizes().vec();
+    ctx->saved_data["types"] = std::vector<int64_t>{int64_t(q.scalar_type()), int64_t(k.scalar_type())};
     return rotate(q, k, c, s, false);
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto saved = ctx->get_saved_variables();
-    Tensor dq = g[0], dk = g[1];
-    if (!dq.defined()) dq = torch::zeros_like(dk);
-    if (!dk.defined()) dk = torch::zeros_like(dq);
-    auto out = rotate(dq, dk, saved[0], saved[1], true);
+    // (an output that no loss used: zeros of its own shape and type; q and k may differ in both)
+    const auto types = ctx->saved_data["types"].toIntVector();
+    auto grad = [&](int i, const char* shape) {
+      return g[i].defined() ? g[i] : torch::zeros(ctx->saved_data[shape].toIntVector(), saved[0].options().dtype(at::ScalarType(types[i])));
+    };
+    auto out = rotate(grad(0, "q"), grad(1, "k"), saved[0], saved[1], true);
     return {out[0], out[1], Tensor(), Tensor()};
   }
 };

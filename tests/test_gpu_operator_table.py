@@ -425,6 +425,27 @@ def test_gradients_off_the_16_byte_grid(dtype):
     both(lambda g: torch.autograd.grad(y, (q, k, v), g, retain_graph=True), (2, 33, 3, 32))
 
 
+@pytest.mark.parametrize("hq,hk,kt", [(3, 3, torch.float32), (8, 2, torch.float32), (4, 4, torch.bfloat16)])
+@pytest.mark.parametrize("used", ["q", "k", "both"])
+def test_rope_gradient_through_either_output(hq, hk, kt, used):
+    """q and k with equal and unequal head counts and types; the input of an output that no loss used gets zeros."""
+    gen = torch.Generator().manual_seed(hq)
+    q, k = torch.randn(2, hq, 7, 16, generator=gen), torch.randn(2, hk, 7, 16, generator=gen).to(kt)
+    ang = torch.randn(7, 16, generator=gen)
+    probes = [torch.randn(t.shape, generator=gen) for t in (q, k)]
+    rot = lambda t: torch.stack([-t[..., 1::2], t[..., 0::2]], -1).flatten(-2)  # noqa: E731
+    ref = [t.float().requires_grad_() for t in (q, k)]
+    sum((((t * ang.cos() + rot(t) * ang.sin()) * p).sum() for t, p in zip(ref, probes))).backward()
+    dev = [t.cuda().requires_grad_() for t in (q, k)]
+    outs = K.k_rope_apply(*dev, ang.cos().cuda(), ang.sin().cuda())
+    terms = [(o.float() * p.cuda()).sum() for o, p in zip(outs, probes)]
+    grads = torch.autograd.grad(sum(t for t, n in zip(terms, "qk") if used in (n, "both")), dev)
+    for g, t, n in zip(grads, ref, "qk"):
+        want = t.grad if used in (n, "both") else torch.zeros_like(t)
+        tol = 2e-2 if g.dtype == torch.bfloat16 else 1e-5
+        assert g.shape == t.shape and torch.allclose(g.cpu().float(), want, atol=tol, rtol=tol)
+
+
 @pytest.mark.parametrize("N,d,m", [(5901, 64, 2048), (5800, 64, 2048)])
 def test_packed_swiglu_on_both_sides_of_the_fusion_rule(N, d, m):
     gen = torch.Generator().manual_seed(N)
