@@ -162,6 +162,7 @@ struct RmsNorm : Function<RmsNorm> {
   }
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight, const OptTensor& residual, double eps) {
     Dev dev(x);
+    TORCH_CHECK_VALUE(x.dim() > 0 && x.size(-1) > 0, "k_fused_rmsnorm: rows without columns, got ", x.sizes());
     const Tensor xc = plain(x), wc = plain(weight), rc = residual ? plain(residual->expand(x.sizes())) : Tensor();
     const auto d = x.size(-1), rows = x.numel() / d;
     const auto out_t = at::result_type(x, weight), sum_t = residual ? at::result_type(x, *residual) : x.scalar_type();
@@ -198,11 +199,12 @@ struct RmsNorm : Function<RmsNorm> {
     const int parts = 8 * rte_device_sm_count();
     const Tensor partial = empty({parts, d}, F32, y), dw = empty_as(w, F32);
     int32_t n_part = 0;
+    auto as = [&](int64_t t) { return at::ScalarType(t) == BF ? (dx16.defined() ? dx16 : dx32.to(BF)) : dx32.to(at::ScalarType(t)); };
+    if (rows == 0) return {as(types[0]), dw.zero_().to(at::ScalarType(types[1])), has_res ? as(types[2]) : Tensor(), Tensor()};
     check(rte_rmsnorm_bwd(f32(y), f32(w), nullptr, f32(rstd), dy.scalar_type() == BF ? ptr(dy) : nullptr, dy.scalar_type() == F32 ? f32(dy) : nullptr, f32(dres),
                           f32(dx32), ptr(dx16), f32(partial), nullptr, nullptr, rows, d, parts, &n_part, dev.st),
           "rte_rmsnorm_bwd");
     check(rte_colsum_partials(f32(partial), n_part, d, f32(dw), 0, dev.st), "rte_colsum_partials");
-    auto as = [&](int64_t t) { return at::ScalarType(t) == BF ? (dx16.defined() ? dx16 : dx32.to(BF)) : dx32.to(at::ScalarType(t)); };
     return {as(types[0]), dw.to(at::ScalarType(types[1])), has_res ? as(types[2]) : Tensor(), Tensor()};
   }
 };
@@ -225,6 +227,7 @@ struct Bhs {                                  // a [..., S, hd] tensor as a [B, 
 };
 variable_list rotate(const Tensor& q, const Tensor& k, const Tensor& cos, const Tensor& sin, bool adjoint) {
   Dev dev(q);
+  TORCH_CHECK_VALUE(q.size(-2) > 0 && q.size(-1) > 0, "k_rope_apply: no positions or no head columns, got ", q.sizes());
   auto plain = [](const Tensor& t) { return direct(t.scalar_type()) ? t : t.to(F32); };
   Tensor in[2] = {plain(q), plain(k)}, out[2];
   if (in[0].sizes() == in[1].sizes() && in[0].scalar_type() == in[1].scalar_type()) {

@@ -446,6 +446,21 @@ def test_rope_gradient_through_either_output(hq, hk, kt, used):
         assert g.shape == t.shape and torch.allclose(g.cpu().float(), want, atol=tol, rtol=tol)
 
 
+def test_empty_rows_and_columns():
+    """No columns, positions or head columns: an error in Python (the host divides by them).  No rows: empty results and
+    zero parameter gradients."""
+    e = lambda *s: torch.zeros(*s, device=DEV)  # noqa: E731
+    with pytest.raises(ValueError, match="k_fused_rmsnorm"):
+        K.k_fused_rmsnorm(e(3, 0), e(0))
+    for shape in ((2, 3, 0, 8), (2, 3, 5, 0), (0, 8), (1, 2, 3, 0, 8), (1, 2, 3, 5, 0)):
+        with pytest.raises(ValueError, match="k_rope_apply"):
+            K.k_rope_apply(e(*shape), e(*shape), e(*shape[-2:]), e(*shape[-2:]))
+    x, w = e(0, 64).requires_grad_(), torch.ones(64, device=DEV, requires_grad=True)
+    out, _ = K.k_fused_rmsnorm(x, w)
+    out.sum().backward()
+    assert out.shape == x.grad.shape == (0, 64) and (w.grad == 0).all()
+
+
 @pytest.mark.parametrize("N,d,m", [(5901, 64, 2048), (5800, 64, 2048)])
 def test_packed_swiglu_on_both_sides_of_the_fusion_rule(N, d, m):
     gen = torch.Generator().manual_seed(N)
