@@ -65,8 +65,9 @@ cluster_route_kernel(const float* __restrict__ q, int ldq, const float* __restri
       const float score = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
       const int c = c0 + who;                                // (lanes 2j and 2j + 1 hold the same cluster)
       if (scores_out && !(lane & 1) && c < C) scores_out[(size_t)tok * C + c] = score;
-      float m = c < C ? score : -INFINITY;
-      int mc = c < C ? c : 0x7fffffff;
+      const bool counts = c < C && score == score;            // (a NaN is larger than nothing)
+      float m = counts ? score : -INFINITY;
+      int mc = counts ? c : 0x7fffffff;
 #pragma unroll
       for (int o = 16; o >= 2; o >>= 1) {
         const float om = __shfl_xor_sync(0xffffffffu, m, o);

@@ -48,6 +48,24 @@ def test_routing_matches_reference_where_scores_are_separated():
     assert torch.equal(got, O.argmax_lowest(scores.cpu()))
 
 
+@pytest.mark.parametrize("C", [4, 16, 40])
+def test_routing_passes_over_nan_scores(C):
+    """A centre with a NaN takes no token, whichever lanes hold its score; a token of NaNs goes to cluster 0."""
+    from speedup_thingy_b200.ops import CudaOps
+    ops = CudaOps(DEV)
+    g = torch.Generator().manual_seed(C)
+    q = torch.randn(64, 32, generator=g)
+    q[5] = torch.nan
+    for bad in sorted({0, 1, C // 2, C - 1}):
+        cen = torch.randn(C, 32, generator=g)
+        cen[bad, 3] = torch.nan
+        assign = torch.empty(64, dtype=torch.int32, device=DEV)
+        ops.cluster_route(q.to(DEV), cen.to(DEV), assign, None)
+        ref = q.double() @ cen.double().t()
+        ref[ref.isnan()] = -torch.inf
+        assert torch.equal(assign.cpu().long(), ref.argmax(-1))
+
+
 @pytest.mark.parametrize("n,C,pattern", [(200, 4, "golden"), (1000, 16, "random"), (777, 8, "one_cluster"),
                                           (4096, 16, "skewed"), (130, 64, "random")])
 def test_pack_is_the_stable_counting_sort(n, C, pattern):
