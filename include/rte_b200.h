@@ -60,7 +60,7 @@ int rte_device_sm_count(void);
  * lda / ldb are the row strides of the STORED matrices.
  */
 enum {
-  RTE_EPI_BF16 = 0,        /* C bf16 = acc                                                   */
+  RTE_EPI_BF16 = 0,        /* C bf16 = acc (R is not read)                                    */
   RTE_EPI_F32 = 1,         /* C f32 = acc (+ R f32 when R != NULL; R may alias C).            */
                            /* With splits > 1 partial s goes to C + s*split_stride (no R).    */
   RTE_EPI_SWIGLU_FWD = 2,  /* B rows [0,F) = up, [F,2F) = gate, F = b_pair_offset (N = 2F): */

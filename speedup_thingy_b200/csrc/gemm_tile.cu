@@ -241,11 +241,11 @@ template <int BN>
 int launch_tile(const rte_gemm_args* a, int ksplit, cudaStream_t st) {
   TileParams p;
   p.M = a->M; p.N = a->N; p.a_mn = a->a_mn_major ? 1 : 0; p.b_mn = a->b_mn_major ? 1 : 0;
-  p.C = a->C; p.ldc = a->ldc; p.R = reinterpret_cast<const float*>(a->R); p.ldr = a->ldr;
   p.out_f32 = a->epilogue == RTE_EPI_F32 ? 1 : 0;
+  p.C = a->C; p.ldc = a->ldc; p.R = p.out_f32 ? reinterpret_cast<const float*>(a->R) : nullptr; p.ldr = a->ldr;      // (bf16 outputs take no R)
   const long long es = p.out_f32 ? 4 : 2;
   p.vec = (reinterpret_cast<uintptr_t>(a->C) & 15) == 0 && (a->ldc * es) % 16 == 0 &&
-          (a->R == nullptr || ((reinterpret_cast<uintptr_t>(a->R) & 15) == 0 && a->ldr % 4 == 0));
+          (p.R == nullptr || ((reinterpret_cast<uintptr_t>(p.R) & 15) == 0 && p.ldr % 4 == 0));
   p.m_blocks = rte::ceil_div(a->M, BM);
   p.kblocks = rte::ceil_div(a->K, BK);
   p.ksplit = ksplit;
@@ -294,7 +294,6 @@ int launch_tile(const rte_gemm_args* a, int ksplit, cudaStream_t st) {
 extern "C" int rte_gemm_bf16_tile(const rte_gemm_args* a, int32_t tile_n, int32_t ksplit, rte_stream_t stream) {
   RTE_CHECK_ARG(a != nullptr && a->A && a->B && a->C && a->M > 0 && a->N > 0 && a->K > 0);
   RTE_CHECK_ARG(a->epilogue == RTE_EPI_BF16 || a->epilogue == RTE_EPI_F32);
-  RTE_CHECK_ARG(a->epilogue == RTE_EPI_F32 || a->R == nullptr);
   RTE_CHECK_ARG(a->splits <= 1 && a->tile_group == nullptr && a->split_kblocks == nullptr);
   RTE_CHECK_ARG((tile_n == 64 || tile_n == 128) && ksplit >= 1 && ksplit <= 8 && ksplit <= rte::ceil_div(a->K, BK));
   if ((reinterpret_cast<uintptr_t>(a->A) & 15) || (reinterpret_cast<uintptr_t>(a->B) & 15) || (a->lda % 8) || (a->ldb % 8))

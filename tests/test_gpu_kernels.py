@@ -143,6 +143,18 @@ def test_gemm_f32_residual_and_alias(ops):
     _close(out, ref, 2e-3, "gemm f32 + residual (aliased)")
 
 
+@pytest.mark.parametrize("M,N,K", [(64, 512, 512), (512, 384, 128), (1050, 512, 4096), (4096, 4096, 512)])
+def test_gemm_bf16_output_does_not_read_a_residual(ops, M, N, K):
+    """Whichever kernel the size picks: R of a bf16 product is neither read nor refused."""
+    g = torch.Generator().manual_seed(M)
+    a, b = (torch.randn(*s, generator=g).bfloat16().to(DEV) for s in ((M, K), (N, K)))
+    want, got = (torch.empty(M, N, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    ops.gemm(a, b, want, M=M, N=N, K=K)
+    ops.gemm(a, b, got, M=M, N=N, K=K, residual=torch.full((M, N), torch.nan, device=DEV))
+    assert torch.equal(want, got)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("Mo,No,Kred", [(1536, 512, 8192), (512, 512, 8192), (4096, 512, 4096), (96, 64, 1024), (200, 72, 520)])
 def test_gemm_wgrad_split_k(ops, Mo, No, Kred):
     g = torch.Generator().manual_seed(Mo + No)
