@@ -719,7 +719,7 @@ float small_us(const rte_gemm_args* a) {
   const int rows = rte::ceil_div(a->M, 64), wide = rte::ceil_div(a->N, 64) * rows, ctas = wide < 74 ? rte::ceil_div(a->N, 32) * rows : wide;
   if (ctas > 148) return 1e9f;
   const float kb = float(rte::ceil_div(a->K, BK));
-  return 2.0f + (a->R != nullptr ? 0.2f : 0.f) + kb * (wide < 74 ? 0.28f : 0.53f);
+  return 2.0f + (a->R != nullptr && a->epilogue == RTE_EPI_F32 ? 0.2f : 0.f) + kb * (wide < 74 ? 0.28f : 0.53f);
 }
 
 TileConfig pick_tile(const rte_gemm_args* a, int splits, int sms, float* us = nullptr) {
