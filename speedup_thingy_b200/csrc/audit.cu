@@ -176,23 +176,24 @@ __global__ void swiglu_masked_bwd_kernel(const __nv_bfloat16* __restrict__ ug, c
   }
 }
 
-// V = 4: sample_elems is a multiple of four and every pointer starts on 16 bytes; else V = 1.
+// V = 4: sample_elems is a multiple of four and every pointer starts on 16 bytes; else V = 1.  I: what counts the groups, 32
+// bits below 2^31 of them (an index that a grid stride may carry past the last one must not wrap), else 64.
 template <int V> struct Group;
 template <> struct Group<1> { float v[1]; };
 template <> struct __align__(16) Group<4> { float v[4]; };
 template <int V>
-__device__ __forceinline__ Group<V> get(const float* p, unsigned i) { return reinterpret_cast<const Group<V>*>(p)[i]; }
+__device__ __forceinline__ Group<V> get(const float* p, size_t i) { return reinterpret_cast<const Group<V>*>(p)[i]; }
 template <int V>
-__device__ __forceinline__ void put(float* p, unsigned i, const Group<V>& g) { reinterpret_cast<Group<V>*>(p)[i] = g; }
+__device__ __forceinline__ void put(float* p, size_t i, const Group<V>& g) { reinterpret_cast<Group<V>*>(p)[i] = g; }
 
-template <int V>
+template <int V, typename I>
 __global__ void __launch_bounds__(NTHR)
 scaled_residual_fwd_kernel(const float* __restrict__ base, const float* __restrict__ branch,
                            const float* __restrict__ scale, const int32_t* __restrict__ active,
-                           const float* __restrict__ pass, float* __restrict__ out, unsigned groups, unsigned per_sample) {
+                           const float* __restrict__ pass, float* __restrict__ out, I groups, I per_sample) {
   rte::after_previous_grid();
   const float s = *scale;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < groups; i += gridDim.x * blockDim.x) {
+  for (I i = blockIdx.x * blockDim.x + threadIdx.x; i < groups; i += gridDim.x * blockDim.x) {
     const bool on = active == nullptr || active[i / per_sample] != 0;
     Group<V> o;
     if (on) {
@@ -206,20 +207,20 @@ scaled_residual_fwd_kernel(const float* __restrict__ base, const float* __restri
   }
 }
 
-template <int V>
+template <int V, typename I>
 __global__ void __launch_bounds__(NTHR)
 scaled_residual_bwd_kernel(const float* __restrict__ dout, const float* __restrict__ branch, const float* __restrict__ scale,
                            const int32_t* __restrict__ active, float* __restrict__ dbase, __nv_bfloat16* __restrict__ db16,
                            float* __restrict__ db32, float* __restrict__ dpass, float* __restrict__ dscale_part,
-                           const int32_t* __restrict__ frozen_active, const float* __restrict__ frozen_src, unsigned groups,
-                           unsigned per_sample) {
+                           const int32_t* __restrict__ frozen_active, const float* __restrict__ frozen_src, I groups,
+                           I per_sample) {
   rte::after_previous_grid();
   __shared__ float red[32];
   const float s = *scale;
   float acc = 0.f;
 #pragma unroll 2
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < groups; i += gridDim.x * blockDim.x) {
-    const unsigned sample = i / per_sample;
+  for (I i = blockIdx.x * blockDim.x + threadIdx.x; i < groups; i += gridDim.x * blockDim.x) {
+    const I sample = i / per_sample;
     const bool on = active == nullptr || active[sample] != 0;
     const Group<V> g = get<V>(dout, i), br = get<V>(branch, i);
 #pragma unroll
@@ -662,7 +663,7 @@ extern "C" int rte_gather_rows(const void* src, const int32_t* idx, void* dst, i
   const long long row16 = row_bytes / 16;
   const auto* from = reinterpret_cast<const uint4*>(src);
   auto* to = reinterpret_cast<uint4*>(dst);
-  if (row16 < NTHR && (long long)n * row16 < (1ll << 32))
+  if (row16 < NTHR && (long long)n * row16 < (1ll << 31))             // (the index of a grid stride must not wrap)
     rte::launch(gather_short_rows_kernel, grid_for((long long)n * row16, NTHR, 148 * 16), NTHR, 0, ST(stream), from, idx, to, (unsigned)(n * row16), (unsigned)row16);
   else
     for (int at = 0; at < n; at += 65535)                 // (gridDim.y)
@@ -725,11 +726,13 @@ extern "C" int rte_scaled_residual_fwd(const float* base, const float* branch, c
                                        const float* passthrough, float* out, int32_t n, int64_t sample_elems,
                                        rte_stream_t stream) {
   RTE_CHECK_ARG(base && branch && scale && out && n > 0 && sample_elems > 0 && (active == nullptr || passthrough != nullptr));
-  RTE_CHECK_ARG((long long)n * sample_elems < (1ll << 32));
   const bool wide = sample_elems % 4 == 0 && aligned16(base) && aligned16(branch) && aligned16(out) && aligned16(passthrough);
-  const int v = wide ? 4 : 1;
-  rte::launch(wide ? scaled_residual_fwd_kernel<4> : scaled_residual_fwd_kernel<1>, grid_for((long long)n * sample_elems / v, NTHR), NTHR, 0, ST(stream),
-              base, branch, scale, active, passthrough, out, (unsigned)(n * sample_elems / v), (unsigned)(sample_elems / v));
+  const long long per = sample_elems / (wide ? 4 : 1), groups = n * per;
+#define RTE_SR_FWD(V, I) rte::launch(scaled_residual_fwd_kernel<V, I>, grid_for(groups, NTHR), NTHR, 0, ST(stream), base, branch, scale, active, passthrough, \
+                                     out, (I)groups, (I)per)
+  if (groups < (1ll << 31)) { if (wide) RTE_SR_FWD(4, unsigned); else RTE_SR_FWD(1, unsigned); }
+  else { if (wide) RTE_SR_FWD(4, unsigned long long); else RTE_SR_FWD(1, unsigned long long); }
+#undef RTE_SR_FWD
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
@@ -741,19 +744,21 @@ extern "C" int rte_scaled_residual_bwd(const float* dout, const float* branch, c
                                        int64_t sample_elems, rte_stream_t stream) {
   RTE_CHECK_ARG(dout && branch && scale && n > 0 && sample_elems > 0);
   RTE_CHECK_ARG((frozen_active == nullptr) == (frozen_src == nullptr) && (frozen_src == nullptr || dbase != nullptr));
-  RTE_CHECK_ARG((long long)n * sample_elems < (1ll << 32));
   const bool wide = sample_elems % 4 == 0 && aligned16(dout) && aligned16(branch) && aligned16(dbase) && aligned16(dbranch_bf16) &&
                     aligned16(dbranch_f32_accum) && aligned16(dpassthrough) && aligned16(frozen_src);
-  const int v = wide ? 4 : 1;
-  int grid = grid_for((long long)n * sample_elems / v, NTHR, 592);
+  const long long per = sample_elems / (wide ? 4 : 1), groups = n * per;
+  int grid = grid_for(groups, NTHR, 592);
   if (dscale_partial) {
     RTE_CHECK_ARG(max_partials >= 1);
     if (grid > max_partials) grid = max_partials;
   }
   if (n_partials) *n_partials = grid;
-  rte::launch(wide ? scaled_residual_bwd_kernel<4> : scaled_residual_bwd_kernel<1>, grid, NTHR, 0, ST(stream), dout, branch, scale, active, dbase,
-              reinterpret_cast<__nv_bfloat16*>(dbranch_bf16), dbranch_f32_accum, dpassthrough, dscale_partial, frozen_active,
-              frozen_src, (unsigned)(n * sample_elems / v), (unsigned)(sample_elems / v));
+#define RTE_SR_BWD(V, I) rte::launch(scaled_residual_bwd_kernel<V, I>, grid, NTHR, 0, ST(stream), dout, branch, scale, active, dbase, \
+                                     reinterpret_cast<__nv_bfloat16*>(dbranch_bf16), dbranch_f32_accum, dpassthrough, dscale_partial, frozen_active, frozen_src, \
+                                     (I)groups, (I)per)
+  if (groups < (1ll << 31)) { if (wide) RTE_SR_BWD(4, unsigned); else RTE_SR_BWD(1, unsigned); }
+  else { if (wide) RTE_SR_BWD(4, unsigned long long); else RTE_SR_BWD(1, unsigned long long); }
+#undef RTE_SR_BWD
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }

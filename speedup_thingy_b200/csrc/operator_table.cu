@@ -77,21 +77,22 @@ rmsnorm_op_kernel(const void* __restrict__ x, int x16, const void* __restrict__ 
 struct View4 { const void* p; long long sb, sh, ss; };          // [B, H, S, hd], unit stride along hd
 struct View4Out { void* p; long long sb, sh, ss; };
 
-// out = rotation (or its transpose) of adjacent pairs with caller's cos / sin [S, hd]; blockIdx.y: q | k
-template <typename T>
+// out = rotation (or its transpose) of adjacent pairs with caller's cos / sin [S, hd]; blockIdx.y: q | k.  I counts the
+// pairs: 32 bits below 2^31 of them (a grid stride past the last one must not wrap), else 64.
+template <typename T, typename I>
 __global__ void __launch_bounds__(256)
 rope_views_kernel(View4 q, View4 k, View4Out oq, View4Out ok, const float* __restrict__ cs, const float* __restrict__ sn, int H, int S, int hd,
-                  unsigned pairs, int adjoint) {
+                  I pairs, int adjoint) {
   rte::after_previous_grid();
   const View4& v = blockIdx.y == 0 ? q : k;
   const View4Out& o = blockIdx.y == 0 ? oq : ok;
   const unsigned hp = hd / 2;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < pairs; i += gridDim.x * blockDim.x) {
+  for (I i = blockIdx.x * blockDim.x + threadIdx.x; i < pairs; i += gridDim.x * blockDim.x) {
     // (pair, head, position, sample): neighbouring threads stay inside one token's row of a [B, S, H, hd] layout
-    unsigned r = i / hp;
-    const unsigned pr = i - r * hp, h = r % (unsigned)H;
+    I r = i / hp;
+    const unsigned pr = (unsigned)(i - r * hp), h = (unsigned)(r % (unsigned)H);
     r /= (unsigned)H;
-    const unsigned s = r % (unsigned)S, b = r / (unsigned)S;
+    const unsigned s = (unsigned)(r % (unsigned)S), b = (unsigned)(r / (unsigned)S);
     const T* x = reinterpret_cast<const T*>(v.p) + b * v.sb + h * v.sh + s * v.ss + 2 * pr;
     T* y = reinterpret_cast<T*>(o.p) + b * o.sb + h * o.sh + s * o.ss + 2 * pr;
     const float a = (float)x[0], c = (float)x[1];
@@ -187,11 +188,13 @@ extern "C" int rte_rope_views(const void* q, const int64_t* q_strides, const voi
                               int32_t hd, int32_t is_bf16, int32_t adjoint, rte_stream_t stream) {
   RTE_CHECK_ARG(q && k && q_out && k_out && cos_tab && sin_tab && B > 0 && H > 0 && S > 0 && hd > 0 && hd % 2 == 0);
   const long long pairs = (long long)B * H * S * (hd / 2);
-  RTE_CHECK_ARG(pairs < (1ll << 32));
   const View4 vq = {q, q_strides[0], q_strides[1], q_strides[2]}, vk = {k, k_strides[0], k_strides[1], k_strides[2]};
   const View4Out oq = {q_out, qo_strides[0], qo_strides[1], qo_strides[2]}, ok = {k_out, ko_strides[0], ko_strides[1], ko_strides[2]};
-  rte::launch(is_bf16 ? rope_views_kernel<__nv_bfloat16> : rope_views_kernel<float>, dim3(blocks_for(pairs, 148 * 8), 2), 256, 0, ST(stream), vq, vk, oq, ok,
-              cos_tab, sin_tab, H, S, hd, (unsigned)pairs, adjoint);
+#define RTE_ROPE(T, I) rte::launch(rope_views_kernel<T, I>, dim3(blocks_for(pairs, 148 * 8), 2), 256, 0, ST(stream), vq, vk, oq, ok, cos_tab, sin_tab, H, S, hd, \
+                                   (I)pairs, adjoint)
+  if (pairs < (1ll << 31)) { if (is_bf16) RTE_ROPE(__nv_bfloat16, unsigned); else RTE_ROPE(float, unsigned); }
+  else { if (is_bf16) RTE_ROPE(__nv_bfloat16, unsigned long long); else RTE_ROPE(float, unsigned long long); }
+#undef RTE_ROPE
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }

@@ -1180,3 +1180,42 @@ def test_row_passes_of_the_replay(ops, n, S, cols):
 
     for a, b in zip(run(ops, DEV), run(emu, "cpu")):
         assert (a - b).abs().max() <= 1e-2 * max(b.abs().max().item(), 1e-3)
+
+
+def test_row_passes_beyond_32_bit_counts(ops):
+    """More elements than 32 bits count: the scaled residual one element at a time, the rotary embedding of an expanded view,
+    the gather of short rows past 2^31 groups (34 GB at a time)."""
+    if torch.cuda.mem_get_info()[0] < 45 << 30:
+        pytest.skip("needs 45 GB of free device memory")
+    from speedup_thingy_b200 import kernels as K
+
+    def ends(t, n=1 << 20):
+        return t[:n], t[t.numel() // 2:t.numel() // 2 + n], t[-n:]
+
+    try:
+        n = (1 << 32) + 5
+        base, out, scale = torch.ones(n, device=DEV), torch.zeros(n, device=DEV), torch.tensor([0.5], device=DEV)
+        base[-3:] = 4.0
+        ops.scaled_residual_fwd(base, base, scale, None, None, out, 1, n)
+        assert all(bool((o == 1.5 * b).all()) for o, b in zip(ends(out), ends(base)))
+        part = torch.zeros(592, device=DEV)
+        ops.scaled_residual_bwd(base, base, scale, None, out, None, None, None, part, 1, n)
+        assert all(bool((o == b).all()) for o, b in zip(ends(out), ends(base)))
+        assert abs(float(part.double().sum()) - (n + 3 * 15)) <= 1e-6 * n
+        del base, out
+        one = torch.randn(1, 64, 256, 128, device=DEV).bfloat16()
+        ang = torch.randn(256, 128, device=DEV)
+        want = K.k_rope_apply(one, one, ang.cos(), ang.sin())[0][0]
+        many = one.expand(4097, 64, 256, 128)                         # 4097 * 2^20 pairs
+        for got in K.k_rope_apply(many, many, ang.cos(), ang.sin()):
+            assert all(torch.equal(got[i], want) for i in (0, 2048, 4095, 4096))
+        del many, got
+        rows, row = (1 << 24) + 1, 2048                               # 2^31 + 128 groups of 16 bytes
+        src = torch.arange(3 * row // 4, dtype=torch.int32, device=DEV).view(3, -1)
+        idx = (torch.arange(rows, device=DEV) % 3).to(torch.int32)
+        dst = torch.zeros(rows, row // 4, dtype=torch.int32, device=DEV)
+        ops.gather_rows(src, idx, dst, rows, row)
+        for r in (0, 65534, 65535, 65536, rows // 2, rows - 1):
+            assert torch.equal(dst[r], src[r % 3])
+    finally:
+        torch.cuda.empty_cache()
