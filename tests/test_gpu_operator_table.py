@@ -339,7 +339,7 @@ def test_cross_entropy_of_masked_and_nan_columns(V, dtype, level, fill):
     fill = -torch.inf if fill == "-inf" else torch.finfo(dtype).min
     for r, (a, b) in enumerate(keeps):
         x[r, :a] = x[r, b:] = fill
-    ref = x.float().requires_grad_(True)
+    ref = x.float().clone().requires_grad_(True)
     loss = torch.nn.functional.cross_entropy(ref, targets, reduction="none")
     loss.sum().backward()
     got = x.cuda().requires_grad_(True)
