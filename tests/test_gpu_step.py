@@ -262,3 +262,62 @@ def test_split_workspace_is_sized_before_the_step_is_captured():
     batch = next(_stream(cfg, 1))
     assert all(torch.isfinite(torch.tensor(eng.train_step(batch).loss)) for _ in range(2))
     assert eng.ops._split_ws.data_ptr() == before and not eng.ops._retired_ws
+
+
+@pytest.mark.parametrize("name", ["dense", "macro_fixed_depth", "macro_audit_two_banks", "macro_bernoulli_cap", "macro_shortlist", "exact_one_bank", "exact_two_banks"])
+def test_captured_evaluation_equals_eager_and_leaves_training_alone(name):
+    """`evaluate` replays a captured forward over rotating input images: the eager losses, bit for bit, over more batches than
+    there are images, from one host buffer overwritten in place and from device tensors, before the first step and between
+    steps; the steps around it are those of an engine that never evaluates."""
+    model, train, *rest = CASES[name]
+    cfg, params, eng = _engine(model, train, *rest)
+    _, _, eager = _engine(model, train, *rest, use_cuda_graph=False)
+    _, _, plain = _engine(model, train, *rest)
+    batches = [b for _, b in zip(range(12), _stream(cfg, 12))]
+    held, steps = batches[:7], batches[7:]
+    buf = [t.clone().pin_memory() for t in held[0]]
+
+    def in_place():
+        for b in held:
+            for dst, src in zip(buf, b):
+                dst.copy_(src)
+            yield tuple(buf)
+
+    def check():
+        want = eager.evaluate(held)
+        last = eager.loss_per_sample.clone()
+        for src in (held, in_place(), [tuple(t.cuda() for t in b) for b in held]):
+            assert eng.evaluate(src) == want and torch.equal(eng.loss_per_sample, last)
+        assert want["samples"] == 7 * cfg.training.batch_size
+        assert eng.evaluate(held[:1])["eval_loss_per_sample"] == eager.evaluate(held[:1])["eval_loss_per_sample"]
+
+    check()
+    for n, b in enumerate(steps):
+        losses = [e.train_step(b).loss for e in (eng, eager, plain)]
+        assert losses[0] == losses[1] == losses[2]
+        if n in (0, 2):
+            check()
+    for k in params:
+        assert torch.equal(eng.params[k], plain.params[k]) and torch.equal(eng.params[k], eager.params[k]), k
+
+
+def test_an_engine_goes_with_its_last_reference_and_frees_its_memory():
+    """No collection is needed: graphs and buffers are released by `del`, in every kind of engine that captures."""
+    import gc
+    import weakref
+    for name in ("dense", "macro_audit_two_banks", "exact_one_bank"):
+        model, train, *rest = CASES[name]
+        cfg, _, eng = _engine(model, train, *rest)
+        batch = next(_stream(cfg, 2))
+        torch.cuda.synchronize()
+        gc.collect()
+        gc.disable()
+        try:
+            before, ref = torch.cuda.memory_allocated(), weakref.ref(eng)
+            eng.train_step(batch)
+            eng.evaluate([batch])
+            held = torch.cuda.memory_allocated()
+            del eng
+            assert ref() is None and torch.cuda.memory_allocated() < min(before, held)
+        finally:
+            gc.enable()
