@@ -44,7 +44,14 @@ struct Dev {                                 // makes the tensor's device curren
   }
 };
 
-void check(int rc, const char* what) { TORCH_CHECK(rc == 0, what, " failed: ", rte_status_string(rc), " (code ", rc, ")"); }
+// A refused launch raises what the ctypes binding raises for it, also out of a backward on an autograd thread.
+void check(int rc, const char* what) {
+  if (rc == 0) return;
+  pybind11::gil_scoped_acquire gil;
+  const auto type = pybind11::module_::import("speedup_thingy_b200._abi").attr("RteError");
+  PyErr_SetString(type.ptr(), c10::str(what, " failed: ", rte_status_string(rc), " (code ", rc, ")").c_str());
+  throw pybind11::error_already_set();
+}
 
 Tensor empty(std::initializer_list<int64_t> shape, at::ScalarType dt, const Tensor& like) {
   return at::empty(c10::IntArrayRef(shape.begin(), shape.size()), like.options().dtype(dt));

@@ -461,6 +461,19 @@ def test_empty_rows_and_columns():
     assert out.shape == x.grad.shape == (0, 64) and (w.grad == 0).all()
 
 
+def test_a_refused_launch_raises_rte_error_forward_and_backward():
+    from speedup_thingy_b200._abi import RteError
+    wide = torch.zeros(3, 4096, device=DEV)
+    with pytest.raises(RteError, match="rte_rmsnorm_op_fwd failed"):
+        K.k_fused_rmsnorm(wide, wide[0])
+    x, w = (torch.zeros(16, 16, dtype=torch.bfloat16, device=DEV, requires_grad=True) for _ in range(2))
+    odd = torch.zeros(16 * 16 + 1, dtype=torch.bfloat16, device=DEV)[1:].view(16, 16)        # a product's operand off 16 bytes
+    with pytest.raises(RteError, match="rte_gemm_bf16 failed"):
+        K.k_logits_full(x, w).backward(odd)
+    with pytest.raises(RteError, match="rte_gemm_bf16 failed"):
+        K.k_logits_full(odd, w)
+
+
 @pytest.mark.parametrize("N,d,m", [(5901, 64, 2048), (5800, 64, 2048)])
 def test_packed_swiglu_on_both_sides_of_the_fusion_rule(N, d, m):
     gen = torch.Generator().manual_seed(N)
