@@ -239,12 +239,13 @@ def _capture(graph, device: torch.device):
     The allocator's cache is given back only when the device is short of memory, not before every capture: the memory of
     engines that are gone (5 GB in 290 segments) took 0.9 s to unmap in the first step of the next one, which then had
     to map as much again; that step takes 11 ms now.  A capture itself allocates next to nothing (the engine's buffers are there
-    before it), a sixteenth of the device is room enough.  What is free only the driver knows, other processes hold memory too
-    (0.1 ms, one call in fifty 10 ms and more); an allocation inside the capture cannot give the cache back any more."""
+    before it), a sixteenth of the device is room enough.  The driver is asked for what is free (0.1 ms, at times 5 to 50)
+    only once this process holds half of the device."""
     torch.cuda.synchronize(device)
-    free, total = torch.cuda.mem_get_info(device)
-    if free < total // 16:
-        torch.cuda.empty_cache()
+    if torch.cuda.memory_reserved(device) > torch.cuda.get_device_properties(device).total_memory // 2:
+        free, total = torch.cuda.mem_get_info(device)
+        if free < total // 16:
+            torch.cuda.empty_cache()
     stream = _capture_streams.get(device)
     if stream is None:
         stream = _capture_streams[device] = torch.cuda.Stream(device)
