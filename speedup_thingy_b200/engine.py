@@ -238,9 +238,10 @@ def _capture(graph, device: torch.device):
     permit while a stream is capturing (and which ends the capture).
     The allocator's cache is given back only when the device is short of memory, not before every capture: the memory of
     engines that are gone (5 GB in 290 segments) took 0.9 s to unmap in the first step of the next one, which then had
-    to map as much again; that step takes 11 ms now.  A capture itself allocates next to nothing (the engine's buffers are there
-    before it), a sixteenth of the device is room enough.  The driver is asked for what is free (0.1 ms, at times 5 to 50)
-    only once this process holds half of the device."""
+    to map as much again; that step takes 11 ms now.  What is captured allocates nothing (the engine's buffers are there before
+    it), only the graph itself needs room, of which a sixteenth of the device is plenty.  The driver is asked for what is free
+    only once this process holds half of the device: that is 0.1 ms as a rule, but 20 ms and more at times, several times the
+    rest of a first step."""
     torch.cuda.synchronize(device)
     if torch.cuda.memory_reserved(device) > torch.cuda.get_device_properties(device).total_memory // 2:
         free, total = torch.cuda.mem_get_info(device)

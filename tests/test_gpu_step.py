@@ -321,3 +321,43 @@ def test_an_engine_goes_with_its_last_reference_and_frees_its_memory():
             assert ref() is None and torch.cuda.memory_allocated() < min(before, held)
         finally:
             gc.enable()
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_a_capture_allocates_nothing(monkeypatch, name):
+    """Inside a capture the allocator cannot give its cache back to a device that others have filled: nothing may need it."""
+    import contextlib
+
+    from speedup_thingy_b200 import engine as E
+    capture, allocated = E._capture, []
+
+    @contextlib.contextmanager
+    def counted(graph, device):
+        with capture(graph, device):
+            before = torch.cuda.memory_stats()["allocation.all.allocated"]
+            yield
+            allocated.append(torch.cuda.memory_stats()["allocation.all.allocated"] - before)
+
+    monkeypatch.setattr(E, "_capture", counted)
+    model, train, *rest = CASES[name]
+    cfg, _, eng = _engine(model, train, *rest)
+    batch = next(_stream(cfg, 2))
+    eng.train_step(batch)
+    eng.evaluate([batch])
+    assert allocated == [0, 0]
+
+
+@pytest.mark.parametrize("thirds,share,emptied", [(1, 20, 0), (2, 20, 1), (2, 15, 0)])
+def test_a_capture_gives_the_cache_back_when_memory_is_short(monkeypatch, thirds, share, emptied):
+    """The process holds so many thirds of the device's memory, one part in `share` of it is free."""
+    from speedup_thingy_b200 import engine as E
+    calls, total = [], torch.cuda.get_device_properties(0).total_memory
+    monkeypatch.setattr(torch.cuda, "memory_reserved", lambda device=None: thirds * total // 3)
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device=None: (total // share, total))
+    monkeypatch.setattr(torch.cuda, "empty_cache", lambda: calls.append(1))
+    x, graph = torch.zeros(4, device="cuda:0"), torch.cuda.CUDAGraph()
+    with E._capture(graph, x.device):
+        x.add_(1.0)
+    assert len(calls) == emptied
+    graph.replay()
+    assert torch.equal(x.cpu(), torch.ones(4))
