@@ -155,6 +155,32 @@ def test_gemm_bf16_output_does_not_read_a_residual(ops, M, N, K):
     ops.check_status()
 
 
+@pytest.mark.parametrize("M,N,K", [(64, 512, 512), (512, 384, 128), (1050, 512, 4096), (8192, 512, 512)])
+def test_gemm_max_ctas_bounds_every_kernel_of_a_product(ops, M, N, K, monkeypatch):
+    """The grid of the captured launch, with and without a limit; the result is the same product either way."""
+    import ctypes
+    g = torch.Generator().manual_seed(N)
+    a, b = (torch.randn(*s, generator=g).bfloat16().to(DEV) for s in ((M, K), (N, K)))
+    ref, cuda = a.float() @ b.float().t(), ctypes.CDLL("libcuda.so.1")
+
+    def ctas(limit):
+        monkeypatch.setattr(ops, "gemm_max_ctas", limit)
+        out, graph = torch.zeros(M, N, device=DEV), torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            ops.gemm(a, b, out, M=M, N=N, K=K, epilogue=1)
+        nodes, count, params = (ctypes.c_void_p * 1)(), ctypes.c_size_t(1), (ctypes.c_uint32 * 64)()
+        assert cuda.cuGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), nodes, ctypes.byref(count)) == 0 and count.value == 1
+        assert cuda.cuGraphKernelNodeGetParams_v2(ctypes.c_void_p(nodes[0]), params) == 0          # function pointer, then gridDim
+        graph.instantiate()
+        graph.replay()
+        _close(out, ref, 1e-4)
+        return params[2] * params[3] * params[4]
+
+    free = ctas(0)
+    for limit in (140, 6):
+        assert ctas(limit) <= max(limit, 2) and (free > limit or ctas(limit) == free)
+
+
 @pytest.mark.parametrize("Mo,No,Kred", [(1536, 512, 8192), (512, 512, 8192), (4096, 512, 4096), (96, 64, 1024), (200, 72, 520)])
 def test_gemm_wgrad_split_k(ops, Mo, No, Kred):
     g = torch.Generator().manual_seed(Mo + No)
