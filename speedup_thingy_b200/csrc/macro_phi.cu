@@ -49,7 +49,7 @@ phi_prep_kernel(const float* __restrict__ h0, const float* __restrict__ v, const
                 const int32_t* __restrict__ sid, float* __restrict__ rstd, float* __restrict__ pooled,
                 float* __restrict__ pa, PhiDims D, float eps) {
   rte::after_previous_grid();
-  extern __shared__ float sm[];            // warp sums [NTHR / 32][d] -> (row 0) this CTA's column sums; then pooled [d], products [m]
+  extern __shared__ __align__(16) float sm[];            // warp sums [NTHR / 32][d] -> (row 0) this CTA's column sums; then pooled [d], products [m]
   constexpr int WARPS = NTHR / 32;
   float* ps = sm + (size_t)WARPS * D.d;
   float* pj = ps + D.d;
@@ -126,7 +126,7 @@ phi_prep_any_kernel(const float* __restrict__ h0, const float* __restrict__ v, c
                 const int32_t* __restrict__ sid, float* __restrict__ rstd, float* __restrict__ pooled,
                 float* __restrict__ pa, PhiDims D, float eps) {
   rte::after_previous_grid();
-  extern __shared__ float sm[];            // rstd_s[S] then pooled_s[d]
+  extern __shared__ __align__(16) float sm[];            // rstd_s[S] then pooled_s[d]
   float* rs = sm;
   float* ps = sm + D.S;
   const int b = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

@@ -66,7 +66,7 @@ router_hidden_kernel(const float* __restrict__ pooled, const float* __restrict__
                      float* __restrict__ prea, const float* __restrict__ w0b, const float* __restrict__ b0b,
                      float* __restrict__ preb, int B, int d, int hid) {
   rte::after_previous_grid();
-  extern __shared__ float xs[];                 // [RH_SAMPLES][d]
+  extern __shared__ __align__(16) float xs[];                 // [RH_SAMPLES][d]
   const float* w0 = blockIdx.z == 0 ? w0a : w0b;
   const float* b0 = blockIdx.z == 0 ? b0a : b0b;
   float* pre = blockIdx.z == 0 ? prea : preb;
@@ -352,7 +352,7 @@ struct Dw0Jobs { Dw0Job job[2]; };
 __global__ void __launch_bounds__(NTHR)
 router_dw0_kernel(const Dw0Jobs jobs, const float* __restrict__ pooled, int B, int d, int hid) {
   rte::after_previous_grid();
-  __shared__ float sj[W0_SAMPLES][W0_TILE], sc[W0_SAMPLES][W0_TILE];
+  __shared__ __align__(16) float sj[W0_SAMPLES][W0_TILE], sc[W0_SAMPLES][W0_TILE];
   const Dw0Job& job = jobs.job[blockIdx.z];
   const int j0 = blockIdx.y * W0_TILE, c0 = blockIdx.x * W0_TILE, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   float acc[4][4], accb = 0.f;
