@@ -113,15 +113,12 @@ int rte_gemm_bf16(const rte_gemm_args* args, rte_stream_t stream);
 /* How many splits (1 .. max_splits) a product with fp32 output and a long reduction should be cut into when its partials
  * are added by rte_reduce_splits; 1: one rte_gemm_bf16 launch is faster.                                             */
 int rte_gemm_wgrad_splits(const rte_gemm_args* args, int32_t max_splits);
-/* The tile shape the persistent kernel would use for `args` (M, N, epilogue, grouping, tile hints and max_ctas are read) and
- * how many tiles run at the same time: what a caller needs to choose a split count.  Any output may be NULL.  */
-int rte_gemm_tile_plan(const rte_gemm_args* args, int32_t* tile_m, int32_t* tile_n, int32_t* concurrent_tiles);
 /* The same product for FEW TILES: one 128 x tile_n tile per CTA (tile_n 64 or 128), the reduction split over the `ksplit`
  * (1..8, at most one per 64-wide k-block) CTAs of a cluster, which add their partial tiles in rank order.  RTE_EPI_BF16 or
  * RTE_EPI_F32 (+R); no grouping, no splits; either major for either operand.                                       */
 int rte_gemm_bf16_tile(const rte_gemm_args* args, int32_t tile_n, int32_t ksplit, rte_stream_t stream);
 /* The same product for FEW ROWS (the audited samples' replay, models.py:605-679: M = one or two samples): one
- * 128-thread CTA per 64x64 output tile, cp.async + mma.sync, no tensor maps or TMEM set-up, so a dependent chain of
+ * 256-thread CTA per 64x64 or 64x32 output tile, cp.async + mma.sync, no tensor maps or TMEM set-up, so a dependent chain of
  * such launches is not dominated by set-up time.  Subset of rte_gemm_args: A K-major, B either major, RTE_EPI_BF16
  * or RTE_EPI_F32 (+R), equal split-K (fp32, no R), no grouping; K % 8 == 0 (and N % 8 == 0 when B is MN-major).   */
 int rte_gemm_bf16_small(const rte_gemm_args* args, rte_stream_t stream);

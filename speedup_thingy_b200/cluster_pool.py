@@ -8,8 +8,9 @@ over clusters, gather the pool weights, pad every cluster to the largest one, th
   route   GEMM x @ [up_a | gate_a] (tcgen05) + ``rte_cluster_route`` (arg-max, lowest index on ties)
   pack    ``rte_cluster_pack``: stable counting sort into one row order whose clusters start on 128-row
           boundaries (capacity = tokens rounded up to 128, plus 128 rows per cluster)
-  pools   ``rte_gather_rows`` of the bf16 weight rows named by ``candidate_ids`` (the dense weights stay the
-          trainable source of truth, so this is redone every forward exactly as the reference does)
+  pools   bf16 copies of the weight rows named by ``candidate_ids``: ``rte_gather_rows_convert`` from wug, ``rte_transpose_f32``
+          and ``rte_gather_rows`` from wd (the dense weights stay the trainable source of truth, so this is redone every
+          forward exactly as the reference does)
   FFN     two grouped ``rte_gemm_bf16`` launches (tile -> cluster table) with the SwiGLU pass between them
   grads   grouped data-gradient GEMMs, ragged split-K weight-gradient GEMMs (one split per cluster), and a
           CSR gather-reduce of pool rows into dense rows (``scatter_cluster_pool_grads`` without atomics)
@@ -83,7 +84,7 @@ class StaticClusterPoolSwiGLU:
         N = self.max_tokens
         self.cap = -(-N // 128) * 128 + 128 * C
         e = lambda *s, dtype=bf: torch.empty(*s, dtype=dtype, device=dev)  # noqa: E731
-        self.wug16, self.wdT16 = e(2 * F, d), e(F, d)
+        self.wdT16 = e(F, d)
         self.wug_pool, self.wd_pool = e(C * 2 * Mc, d), e(C * Mc, d)
         self.q = e(N, 2 * r, dtype=f32)
         self.assign, self.pos = e(N, dtype=i32), e(N, dtype=i32)
@@ -96,13 +97,13 @@ class StaticClusterPoolSwiGLU:
         self.dxp = e(self.cap, d, dtype=f32)
         self.dwug_pool, self.dwd_pool = e(C * 2 * Mc, d, dtype=f32), e(C * Mc, d, dtype=f32)
         self.dwdT = e(F, d, dtype=f32)
-        names = ("selector16 centers idx_ug idx_d wug16 wdT16 wug_pool wd_pool q assign pos perm tile_group counts offsets kblocks x16 "
+        names = ("selector16 centers idx_ug idx_d wdT16 wug_pool wd_pool q assign pos perm tile_group counts offsets kblocks x16 "
                  "xp ugp zp yp dyp dzp dugp dxp dwug_pool dwd_pool dwdT").split()
         self._native = A.load_host().PoolModule(
             {**{k: getattr(self, k) for k in names}, "status": self.ops.status, "ug_ptr": self.csr_ug[0], "ug_rows": self.csr_ug[1],
              "d_ptr": self.csr_d[0], "d_rows": self.csr_d[1]}, dict(rank=r, C=C, Mc=Mc, cap=self.cap, d=d, F=F))
 
-    # ------------------------------------------------------------------ routing / packing
+    # ------------------------------------------------------------------ routing
     def route(self, x: torch.Tensor, scores: torch.Tensor | None = None) -> torch.Tensor:
         """assignments int32 [tokens] (route_to_static_centers, cluster_pool_ffn.py:127-139)."""
         o, N = self.ops, x.shape[0]
@@ -110,19 +111,6 @@ class StaticClusterPoolSwiGLU:
         o.gemm(self.x16[:N], self.selector16, self.q[:N], M=N, N=2 * self.rank, K=self.d, epilogue=A.EPI_F32)
         o.cluster_route(self.q[:N], self.centers, self.assign[:N], scores)
         return self.assign[:N]
-
-    def pack(self, assignments: torch.Tensor) -> None:
-        """Fills perm / pos / tile_group / kblocks for `assignments` (build_static_pack_gather_indices)."""
-        self.ops.cluster_pack(assignments, self.C, self.perm, self.pos[: assignments.numel()], self.counts, self.offsets,
-                              self.tile_group, self.kblocks)
-
-    def prepare_pools(self) -> None:
-        """bf16 pool weights from the current dense weights (prepare_cluster_pool_weights, cluster_pool_ffn.py:90-124)."""
-        o = self.ops
-        o.cast_bf16(self.wug, self.wug16)
-        o.transpose(self.wd, self.wdT16)
-        o.gather_rows(self.wug16, self.idx_ug, self.wug_pool, self.idx_ug.numel(), self.d * 2)
-        o.gather_rows(self.wdT16, self.idx_d, self.wd_pool, self.idx_d.numel(), self.d * 2)
 
     # ------------------------------------------------------------------ forward / backward
     def forward(self, x: torch.Tensor, assignments: torch.Tensor | None = None) -> torch.Tensor:
@@ -146,12 +134,11 @@ class StaticClusterPoolSwiGLU:
         flat = x.reshape(-1, d).contiguous()
         N = flat.shape[0]
         x16 = flat.to(torch.bfloat16)
-        o.cast_bf16(self.wug, self.wug16)
-        wd16 = self.wd.to(torch.bfloat16)
+        wug16, wd16 = self.wug.to(torch.bfloat16), self.wd.to(torch.bfloat16)
         ug = torch.empty(N, 2 * F, dtype=torch.bfloat16, device=x.device)
         z = torch.empty(N, F, dtype=torch.bfloat16, device=x.device)
         out = torch.empty(N, d, dtype=torch.float32, device=x.device)
-        o.gemm(x16, self.wug16, ug, M=N, N=2 * F, K=d)
+        o.gemm(x16, wug16, ug, M=N, N=2 * F, K=d)
         o.swiglu_fwd(ug, z, N, F)
         o.gemm(z, wd16, out, M=N, N=d, K=F, epilogue=A.EPI_F32)
         return out.view(*x.shape[:-1], d)

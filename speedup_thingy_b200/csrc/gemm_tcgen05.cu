@@ -833,22 +833,6 @@ extern "C" int rte_device_sm_count(void) {
   return n;
 }
 
-extern "C" int rte_gemm_tile_plan(const rte_gemm_args* a, int32_t* tile_m, int32_t* tile_n, int32_t* concurrent) {
-  RTE_CHECK_ARG(a != nullptr && a->M > 0 && a->N > 0);
-  const TileConfig c = pick_tile(a, a->splits < 1 ? 1 : a->splits, rte_device_sm_count());
-  if (tile_m) *tile_m = BM * c.ctas;
-  if (tile_n) *tile_n = c.bn;
-  if (concurrent) {
-    const int sms = rte_device_sm_count();
-    if (sms <= 0) return RTE_ERR_NO_DEVICE;
-    int u;
-    if (c.ctas == 2) u = c.bn == 256 ? concurrent_units<256, 2>(a->max_ctas, sms) : concurrent_units<128, 2>(a->max_ctas, sms);
-    else u = a->max_ctas > 0 ? a->max_ctas : sms;
-    *concurrent = u;
-  }
-  return RTE_OK;
-}
-
 extern "C" int rte_gemm_wgrad_splits(const rte_gemm_args* a, int32_t max_splits) {
   if (a == nullptr || a->M <= 0 || a->N <= 0 || a->K <= 0) return 1;
   const int sms = rte_device_sm_count(), kb = rte::ceil_div(a->K, BK);

@@ -200,8 +200,8 @@ aux_kernel(const float* __restrict__ recipe_probs, const float* __restrict__ exp
 }
 
 // per-sample backward through softmax and both MLP heads; dh0 += dpooled / S
-__device__ void mlp_backward_sample(const float* __restrict__ w0, const float* __restrict__ w2, const float* dlog,
-                                    const float* __restrict__ pre, float* dpre_out, float* dhs, int d, int hid, int nout) {
+__device__ void mlp_backward_sample(const float* __restrict__ w2, const float* dlog, const float* __restrict__ pre, float* dpre_out, float* dhs,
+                                    int hid, int nout) {
   for (int j = threadIdx.x; j < hid; j += NTHR) {
     float acc = 0.f;
     for (int r = 0; r < nout; ++r) acc += w2[(size_t)r * hid + j] * dlog[r];
@@ -211,7 +211,6 @@ __device__ void mlp_backward_sample(const float* __restrict__ w0, const float* _
     dpre_out[j] = v;
   }
   __syncthreads();
-  (void)w0; (void)d;
 }
 
 __global__ void __launch_bounds__(NTHR)
@@ -244,8 +243,8 @@ router_bwd_sample_kernel(rte_router_weights w, rte_router_out o, const int32_t* 
     }
   }
   __syncthreads();
-  mlp_backward_sample(w.r_w0, w.r_w2, dlr, o.r_hidden_pre + (size_t)b * hid, dpre_r + (size_t)b * hid, dhr, d, hid, R);
-  mlp_backward_sample(w.d_w0, w.d_w2, dld, o.d_hidden_pre + (size_t)b * hid, dpre_d + (size_t)b * hid, dhd, d, hid, K);
+  mlp_backward_sample(w.r_w2, dlr, o.r_hidden_pre + (size_t)b * hid, dpre_r + (size_t)b * hid, dhr, hid, R);
+  mlp_backward_sample(w.d_w2, dld, o.d_hidden_pre + (size_t)b * hid, dpre_d + (size_t)b * hid, dhd, hid, K);
 }
 
 // dst[r,:] += sum_p vec[p][r / seg,:]   (nparts partial vectors, part_stride floats apart, added in fixed order).  CTA = 256
