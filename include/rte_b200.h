@@ -113,6 +113,8 @@ int rte_gemm_bf16(const rte_gemm_args* args, rte_stream_t stream);
 /* How many splits (1 .. max_splits) a product with fp32 output and a long reduction should be cut into when its partials
  * are added by rte_reduce_splits; 1: one rte_gemm_bf16 launch is faster.                                             */
 int rte_gemm_wgrad_splits(const rte_gemm_args* args, int32_t max_splits);
+/* Hidden activations (rows x F) from which a SwiGLU epilogue (forward | backward) is faster than a plain product and a pass. */
+int64_t rte_swiglu_fuse_min(int32_t backward);
 /* The same product for FEW TILES: one 128 x tile_n tile per CTA (tile_n 64 or 128), the reduction split over the `ksplit`
  * (1..8, at most one per 64-wide k-block) CTAs of a cluster, which add their partial tiles in rank order.  RTE_EPI_BF16 or
  * RTE_EPI_F32 (+R); no grouping, no splits; either major for either operand.                                       */

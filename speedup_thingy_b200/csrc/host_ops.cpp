@@ -476,11 +476,6 @@ struct CrossEntropy : Function<CrossEntropy> {
 Tensor cross_entropy(const Tensor& logits, const Tensor& targets) { return CrossEntropy::apply(logits, targets)[0]; }
 
 // --------------------------------------------------------------------------- packed SwiGLU FFN
-// The SwiGLU pass rides in the product's epilogue where that is faster: forward from about 12 M hidden activations on
-// (us: 8192 x 2048 53.8 -> 46.0, 6144 x 2048 42.0 -> 39.0; 4096 x 2048 even, 8192 x 1024 23.1 -> 25.9), backward from
-// 1 M (8192 x 2048 53.7 -> 37.3, 1000 x 1024 7.8 -> 6.7; 512 x 512 4.9 -> 6.0).
-constexpr int64_t SWIGLU_FUSE_MIN = 12000000, SWIGLU_FUSE_MIN_BWD = 1000000;
-
 struct PackedFfn : Function<PackedFfn> {
   static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& wug, const Tensor& wdown) {
     Dev dev(x);
@@ -489,7 +484,7 @@ struct PackedFfn : Function<PackedFfn> {
     const Tensor &x16 = conv[0], &wug16 = conv[1], &wd16 = conv[2];
     const Tensor ug = empty({N, 2 * m}, BF, x), z = empty({N, m}, BF, x), y = empty({N, wdown.size(1)}, direct(x.scalar_type()) ? x.scalar_type() : F32, x);
     if (N > 0) {
-      if (m % 64 == 0 && N * m >= SWIGLU_FUSE_MIN) {
+      if (m % 64 == 0 && N * m >= rte_swiglu_fuse_min(0)) {
         Gemm(dev, ptr(x16), d, false, ptr(wug16), d, false, ptr(z), m, N, 2 * m, d, RTE_EPI_SWIGLU_FWD).pair(ptr(ug), 2 * m, m).run();
       } else {
         mm_oi(dev, x16, wug16, ug);
@@ -511,7 +506,7 @@ struct PackedFfn : Function<PackedFfn> {
     const auto x_t = at::ScalarType(types[0]);
     const Tensor dx = empty({N, d}, direct(x_t) ? x_t : F32, x16);
     if (N > 0) {
-      if (m % 64 == 0 && N * m >= SWIGLU_FUSE_MIN_BWD) {
+      if (m % 64 == 0 && N * m >= rte_swiglu_fuse_min(1)) {
         Gemm(dev, ptr(dy), dout, false, ptr(wd16), dout, false, ptr(dug), 2 * m, N, m, dout, RTE_EPI_SWIGLU_BWD).residual(ptr(ug), 2 * m).pair(nullptr, 0, m).run();
       } else {
         const Tensor dz = empty({N, m}, BF, x16);

@@ -971,7 +971,7 @@ class TrainEngine:
 
     def _fuse_swiglu(self, rows: int, backward: bool = False) -> bool:
         """SwiGLU inside the tcgen05 product's epilogue?  For large activations, where it is the faster form (the two lines and
-        their times are in ops.py); below them the separate pass finds its input in L2 and the product can take the kernels
+        their times stand beside `rte_swiglu_fuse_min`); below them the separate pass finds its input in L2 and the product can take the kernels
         for few tiles.  Backward also beyond the few-row kernel's range up to `swiglu_fuse_max_rows` rows, whatever the width:
         the gradient of the hidden activations then stays in the fp32 accumulators instead of being rounded to bf16 between the
         two passes (512 x 128 -> 512: 6.0 us against 4.9; relative error of a two-block model's gradient 4.31e-3 against 4.35e-3,

@@ -58,12 +58,8 @@ class CudaOps:
         self.small_fused_reduce = os.environ.get("RTE_SMALL_FUSED_REDUCE", "0") == "1"
         self._split_counters = torch.zeros(1024, dtype=torch.int32, device=self.device)      # per-tile arrival counters
         self.few_rows_max_splits = int(os.environ.get("RTE_FEWROW_SPLITS", "4"))
-        # hidden activations (rows x d_ff) from which a product carries the SwiGLU pass in its epilogue.  us, separate -> fused:
-        # forward 8192 x 512 -> 2048 53.8 -> 46.0, 6144 x 512 -> 2048 42.0 -> 39.0; 8192 x 256 -> 1024 23.1 -> 25.9, 512 x 128 ->
-        # 512 5.4 -> 8.8; backward (its operands come by TMA, so it pays earlier) 8192 x 512 -> 2048 53.7 -> 37.3, 8192 x 256 ->
-        # 1024 20.8 -> 17.3, 1000 x 256 -> 1024 7.8 -> 6.7; 512 x 128 -> 512 4.9 -> 6.0
-        self.swiglu_fuse_min = 12_000_000
-        self.swiglu_fuse_min_bwd = 1_000_000
+        # hidden activations (rows x d_ff) from which a product carries the SwiGLU pass in its epilogue
+        self.swiglu_fuse_min, self.swiglu_fuse_min_bwd = (int(self.lib.rte_swiglu_fuse_min(b)) for b in (0, 1))
         self.gemm_max_ctas = 0     # 0 = one persistent CTA per SM; smaller values leave SMs to kernels of other streams
         # tile hints passed to every GEMM (0 = the library's choice of kernel and tile): RTE_GEMM_PAIR=0 keeps every tile on
         # one CTA of the persistent kernel, RTE_GEMM_TILE_N forces it with 128 or 256 columns per tile
