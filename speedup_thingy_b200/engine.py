@@ -641,7 +641,7 @@ class TrainEngine:
             self.shortlist_dups = e(M, dtype=i32)
         self.audit = None
         # The replay is a long chain of small launches beside a hot pass that fills every SM: its stream gets the
-        # higher priority and the persistent GEMM leaves a few SMs free, so a replay kernel never waits for a whole
+        # higher priority and the products leave a few SMs free, so a replay kernel never waits for a whole
         # hot-pass kernel to drain (measured: -2.5 % step time).
         self._side_stream = torch.cuda.Stream(device=dev, priority=-1) if (self.audit_k and dev.type == "cuda") else None
         if self._side_stream is not None and hasattr(ops, "gemm_max_ctas"):
@@ -974,8 +974,8 @@ class TrainEngine:
         their times stand beside `rte_swiglu_fuse_min`); below them the separate pass finds its input in L2 and the product can take the kernels
         for few tiles.  Backward also beyond the few-row kernel's range up to `swiglu_fuse_max_rows` rows, whatever the width:
         the gradient of the hidden activations then stays in the fp32 accumulators instead of being rounded to bf16 between the
-        two passes (512 x 128 -> 512: 6.0 us against 4.9; relative error of a two-block model's gradient 4.31e-3 against 4.35e-3,
-        300 x 512 -> 2048 6.83e-3 against 6.90e-3).  swiglu_fuse_max_rows = 0: never fused."""
+        two passes (512 x 128 -> 512: 6.0 us against 4.9; with the rounding the gradient of wug is 0.8 % further from the fp32
+        oracle's, eight seeds, +- 0.1).  swiglu_fuse_max_rows = 0: never fused."""
         if self.swiglu_fuse_max_rows <= 0:
             return False
         if backward and getattr(self.ops, "small_gemm_rows", 0) < rows <= self.swiglu_fuse_max_rows:
@@ -1442,7 +1442,8 @@ class TrainEngine:
 
     def _load_batch(self, batch, negatives_seed: int | None = None) -> None:
         """Queues the copy of a step's inputs: the batch, the audited subset with its loss weights, the random negatives.
-        Host tensors are copied into the pinned image first, so the batch may be reused as soon as this returns."""
+        When both tensors of a batch are on the host they are copied into the pinned image first and may be reused as soon as
+        this returns; otherwise each is copied where it lies, in stream order."""
         tokens, targets = self._check_batch(batch)
         inp = self.inputs
         i = inp.image()
@@ -1657,8 +1658,9 @@ class TrainEngine:
         """Queues one training call on a [B,S] int64 (tokens, targets) batch and returns without waiting for the
         device: the batch copy, the step's kernels (one graph replay) and the copy of its results into pinned host
         memory are all stream-ordered.  With `grad_accum_steps` = A the call is a micro-batch: the optimiser runs on
-        every A-th call.  At most `MAX_IN_FLIGHT` steps may be queued before `collect` is called; a host batch must
-        stay untouched until its step has been collected."""
+        every A-th call.  At most `MAX_IN_FLIGHT` steps may be queued before `collect` is called.  A host batch may be
+        reused as soon as this returns (it is in a pinned image then); device tensors, whose copy is only queued, may be
+        overwritten by work on the current stream."""
         if len(self._pending) >= self._max_in_flight:
             raise RuntimeError(f"{len(self._pending)} steps already in flight: call collect() first")
         self._load_batch(batch)
