@@ -80,8 +80,9 @@ typedef struct rte_gemm_args {
   int32_t b_pair_offset;    /* F for the SwiGLU epilogues, else 0 */
   int32_t splits;           /* >= 1; > 1 only with RTE_EPI_F32 (split along K) */
   int64_t split_stride;     /* elements between partial results */
-  int32_t max_ctas;         /* rte_gemm_bf16 launches at most this many CTAs (0: as many as pay), so that other streams' */
-                            /* kernels find SMs free                                                                    */
+  int32_t max_ctas;         /* rte_gemm_bf16: > 0 at most this many CTAs, so that other streams' kernels find SMs free;    */
+                            /* < 0 at most -max_ctas that stay for the whole launch (the persistent kernel), CTAs of one   */
+                            /* tile each are not bounded: they make room as they end; 0 as many as pay                     */
   int32_t* status;
   /* Grouped mode (cluster-pool FFN, cluster_pool_ffn.py:206-241): the rows of A/C are packed by group in blocks of
    * 128 rows; tile_group int32 [M/128] (device) names each block's group (< 0: unused block, skipped).  B is the

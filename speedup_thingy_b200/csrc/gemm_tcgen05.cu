@@ -685,6 +685,8 @@ int make_store_tmap(CUtensorMap* map, const void* base, long long rows, long lon
 struct TileConfig { int bn, ctas; };
 struct Choice { int kernel; TileConfig tile; int ksplit; float us; };      // kernel: 0 persistent, 1 cluster tile, 2 mma.sync
 
+int persistent_ctas(const rte_gemm_args* a, int sms) { return a->max_ctas > 0 ? a->max_ctas : a->max_ctas < 0 ? -a->max_ctas : sms; }
+
 float persistent_us(const rte_gemm_args* a, TileConfig t, int splits, int sms) {
   const int i = (t.bn == 256 ? 0 : 2) + (t.ctas == 2 ? 0 : 1);              // 256 pair | 256 | 128 pair | 128
   static const float base_bf16[4] = {5.2f, 4.0f, 4.5f, 3.2f}, base_f32[4] = {6.3f, 5.4f, 5.3f, 3.9f}, base_res[4] = {10.1f, 8.9f, 7.5f, 5.7f};
@@ -693,7 +695,7 @@ float persistent_us(const rte_gemm_args* a, TileConfig t, int splits, int sms) {
   const bool f32 = a->epilogue == RTE_EPI_F32, res = f32 && a->R != nullptr;
   const int cols = a->epilogue == RTE_EPI_SWIGLU_FWD ? 2 * a->b_pair_offset : a->N;
   const int units = rte::ceil_div(a->M, BM * t.ctas) * rte::ceil_div(cols, t.bn) * splits;
-  const int conc = (a->max_ctas > 0 ? a->max_ctas : sms) / t.ctas, waves = rte::ceil_div(units, conc > 0 ? conc : 1);
+  const int conc = persistent_ctas(a, sms) / t.ctas, waves = rte::ceil_div(units, conc > 0 ? conc : 1);
   const float kb = float(rte::ceil_div(rte::ceil_div(a->K, BK), splits));
   const float slope = waves > 1 ? slope_busy[i] : slope_idle[i] + (slope_busy[i] - slope_idle[i]) * float(units) / float(conc);
   static const float store_swb[4] = {9.f, 9.f, 5.3f, 5.3f};                // SwiGLU's backward: (up | gate) in, (d up | d gate) out
@@ -702,13 +704,12 @@ float persistent_us(const rte_gemm_args* a, TileConfig t, int splits, int sms) {
   return (res ? base_res[i] : f32 ? base_f32[i] : base_bf16[i]) + loop + float(waves - 1) * (loop > store ? loop : store);
 }
 
-// The kernels for few tiles launch a CTA per tile: under `max_ctas` they are out for products that have more (in the audited
-// steps no product is: the same outputs, 5.76 ms against 5.73 for four of them with one audited sample, within the runs' spread).
+// The kernels for few tiles launch a CTA per tile: under a positive `max_ctas` they are out for products that have more.
 bool too_many(const rte_gemm_args* a, int ctas) { return a->max_ctas > 0 && ctas > a->max_ctas; }
 
 float tile_us(const rte_gemm_args* a, int bn, int ksplit, int sms) {
   const int grid = rte::ceil_div(a->M, BM) * rte::ceil_div(a->N, bn) * ksplit, kb = rte::ceil_div(a->K, BK);
-  const float full = float(a->max_ctas > 0 ? a->max_ctas : sms) / float(sms);
+  const float full = float(persistent_ctas(a, sms)) / float(sms);
   // clusters of 2 / 4 / 8 that are resident together (a cluster sits inside one GPC)
   const int limit = int(full * (ksplit == 1 ? 148.f : ksplit == 2 ? 146.f : ksplit == 4 ? 132.f : 112.f));
   if (ksplit > kb || grid > 2 * limit || (ksplit > 1 && grid > limit) || too_many(a, grid)) return 1e9f;
@@ -761,11 +762,10 @@ Choice choose(const rte_gemm_args* a, int splits, int sms) {
   return c;
 }
 
-// Work units (CTAs or CTA pairs) that can run at the same time under `max_ctas`.
+// Work units (CTAs or CTA pairs) that can run at the same time on `ctas` CTAs.
 template <int BN, int CTAS, bool SWB = false>
-int concurrent_units(int max_ctas, int sm_count) {
+int concurrent_units(int ctas, int sm_count) {
   using L = SmemLayout<BN, CTAS, SWB>;
-  int ctas = max_ctas > 0 ? max_ctas : sm_count;
   if (CTAS == 1) return ctas;
   static int max_clusters = -1;
   if (max_clusters < 0) {
@@ -799,7 +799,7 @@ int launch(const rte_gemm_args* a, const CUtensorMap& ta, const CUtensorMap& tb,
     attr_set = true;
   }
   const int total = kp.num_m_blocks * kp.num_n_blocks * kp.splits;
-  int units = concurrent_units<BN, CTAS, SWB>(a->max_ctas, sm_count);
+  int units = concurrent_units<BN, CTAS, SWB>(persistent_ctas(a, sm_count), sm_count);
   if (units > total) units = total;
   if (units < 1) units = 1;
   cudaLaunchConfig_t cfg = {};

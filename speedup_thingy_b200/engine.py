@@ -641,11 +641,12 @@ class TrainEngine:
             self.shortlist_dups = e(M, dtype=i32)
         self.audit = None
         # The replay is a long chain of small launches beside a hot pass that fills every SM: its stream gets the
-        # higher priority and the products leave a few SMs free, so a replay kernel never waits for a whole
-        # hot-pass kernel to drain (measured: -2.5 % step time).
+        # higher priority and the persistent products leave a few SMs free, so a replay kernel never waits for a whole
+        # hot-pass kernel to drain (measured: -2.5 % step time).  Products with a CTA per tile are not bounded: bounding
+        # them too sends the two residual products of a block to the persistent kernel, +0.5 % step time.
         self._side_stream = torch.cuda.Stream(device=dev, priority=-1) if (self.audit_k and dev.type == "cuda") else None
         if self._side_stream is not None and hasattr(ops, "gemm_max_ctas"):
-            ops.gemm_max_ctas = max(ops.sm_count - int(os.environ.get("RTE_SIDE_SMS", "8")), 1)
+            ops.gemm_max_ctas = -max(ops.sm_count - int(os.environ.get("RTE_SIDE_SMS", "8")), 1)
         # (after the limit on the products' CTAs is known: it decides the split counts)
         ops.split_workspace(max(ops.pick_splits(mm, nn, M) * mm * nn
                                 for mm, nn in ((3 * d, d), (d, d), (2 * cfg.d_ff, d), (d, cfg.d_ff), (V, d))))

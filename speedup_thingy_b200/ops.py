@@ -60,7 +60,8 @@ class CudaOps:
         self.few_rows_max_splits = int(os.environ.get("RTE_FEWROW_SPLITS", "4"))
         # hidden activations (rows x d_ff) from which a product carries the SwiGLU pass in its epilogue
         self.swiglu_fuse_min, self.swiglu_fuse_min_bwd = (int(self.lib.rte_swiglu_fuse_min(b)) for b in (0, 1))
-        self.gemm_max_ctas = 0     # 0 = one persistent CTA per SM; smaller values leave SMs to kernels of other streams
+        # products leave SMs to kernels of other streams: > 0 at most this many CTAs, < 0 at most -this many persistent ones
+        self.gemm_max_ctas = 0
         # tile hints passed to every GEMM (0 = the library's choice of kernel and tile): RTE_GEMM_PAIR=0 keeps every tile on
         # one CTA of the persistent kernel, RTE_GEMM_TILE_N forces it with 128 or 256 columns per tile
         self.gemm_cta_pair = 1 if os.environ.get("RTE_GEMM_PAIR", "1") == "0" else 0

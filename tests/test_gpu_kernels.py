@@ -179,6 +179,8 @@ def test_gemm_max_ctas_bounds_every_kernel_of_a_product(ops, M, N, K, monkeypatc
     free = ctas(0)
     for limit in (140, 6):
         assert ctas(limit) <= max(limit, 2) and (free > limit or ctas(limit) == free)
+    # a limit on the persistent kernel alone: what a CTA per tile would do stays, else the bound holds
+    assert ctas(-140) <= 140 or ctas(-140) == free
 
 
 @pytest.mark.parametrize("Mo,No,Kred", [(1536, 512, 8192), (512, 512, 8192), (4096, 512, 4096), (96, 64, 1024), (200, 72, 520)])
