@@ -11,7 +11,8 @@
 //             of the leader CTA reads both halves, and each CTA's TMEM receives the
 //             accumulators of its 128 rows.  Per FLOP this moves a third less operand
 //             data from L2 into shared memory than two independent 128 x BN tiles,
-//             which is what bounds the short-K products of the training step.
+//             which pays for long reductions; short products are bound by set-up, drain
+//             and their stores and run in either shape within a few per cent.
 //
 // Roles per CTA (320 threads): warp 0 = TMA producer, warp 1 = TMEM owner + MMA
 // issuer (the leader CTA's only, with CTAS = 2), warps 2..9 = epilogue: warp w may

@@ -3,7 +3,10 @@
 //
 // A launch through ctypes costs the host 15-20 us with its tensors and argument struct, several times what most of these
 // kernels run: the attention half of a block on 256 tokens took 330 us for 46 us of device time.  Here an operator's
-// allocations, launches and saved tensors are C++: about 4 us per launch.  Products write the type the caller gets (fp32
+// allocations, launches and saved tensors are C++: 6 us or so per call (Python entry, autograd node, output tensors) and 3
+// to 4 per launch -- RMSNorm 10 us, rotary embedding 11, attention 13 with its two launches, the three projections and the
+// output projection with its gather 17 each; the attention half takes 84 us of host time for ten launches, 23 us of device
+// time.  Products write the type the caller gets (fp32
 // straight from the accumulators), type conversions of an operator's inputs share one launch, views are read with their
 // strides.
 #include <ATen/cuda/CUDAContext.h>

@@ -7,7 +7,7 @@ six operators the reference model actually calls -- ``k_fused_rmsnorm`` (layers.
 ``k_out_proj_grouped`` (layers.py:727), ``k_logits_shortlist`` (output.py:125) -- and the benchmarked
 ``k_logits_full`` / ``k_qkv_dense`` / ``k_cross_entropy_unreduced`` through the sm_100a kernels of the C ABI.
 Every operator is an autograd function whose forward and backward are C-ABI launches, native where it is called per layer
-(csrc/host_ops.cpp: the host spends 4 us per launch there against 15-20 us from Python); tensors go in and come out as the
+(csrc/host_ops.cpp, where a launch costs the host 3-4 us and a call 6 more, against 15-20 us per launch from Python); tensors go in and come out as the
 reference's do (fresh outputs, inputs untouched, non-contiguous inputs accepted).
 
 There is no fallback: CPU tensors raise ``RuntimeError`` mentioning ``strict_cuda`` whatever the flag says
