@@ -14,11 +14,11 @@
 // bit-exact with a stable sort by (value descending, index ascending), the tie rule of this build.
 //
 // What bounds it: the latency of each warp's own search.  13 KB of shared memory per token leave 16 warps on an SM, four
-// per scheduler, and each alternates a sweep over its keys with a reduction that it has to wait for: issue slots are 47 %
-// used (stalled per issue: 2.2 warps on fixed latencies, 1.9 on global loads, 1.0 on shared memory), HBM at 26 %.  The
-// instructions alone (~10 per neuron for each of the four scores, about five counting passes of two per key for each
-// selection) would take 75 us at 16384 x 2048.  16384 tokens, F = 2048, k = 256: 1092 us with four 8-bit radix passes per selection (shared-memory atomics whose
-// bins are the few exponents a row holds, so they serialise) -> 379 us with this search.
+// per scheduler, and each alternates a sweep over its keys with a reduction that it has to wait for: 47 % of the issue
+// slots are used (per instruction issued 2.2 warps wait on fixed latencies, 1.9 on global loads, 1.0 on shared memory), HBM
+// at 26 %.  The instructions executed would take 176 us of the 374.  16384 tokens, F = 2048, k = 256: 1092 us with four
+// 8-bit radix passes per selection (shared-memory atomics whose bins are the few exponents a row holds, so they
+// serialise) -> 379 us with this search.
 
 #include "rte_common.cuh"
 
