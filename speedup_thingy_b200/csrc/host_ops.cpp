@@ -265,17 +265,20 @@ struct Rope : Function<Rope> {
     const auto S = q.size(-2), hd = q.size(-1);
     const Tensor c = cos.to(F32).contiguous().view({S, hd}), s = sin.to(F32).contiguous().view({S, hd});
     ctx->save_for_backward({c, s});
-    ctx->saved_data["q"] = q.sizes().vec();
-    ctx->saved_data["k"] = k.sizes().vec();
-    ctx->saved_data["types"] = std::vector<int64_t>{int64_t(q.scalar_type()), int64_t(k.scalar_type())};
+    if (q.sizes() != k.sizes() || q.scalar_type() != k.scalar_type()) {      // (what backward cannot tell from the other gradient)
+      ctx->saved_data["q"] = q.sizes().vec();
+      ctx->saved_data["k"] = k.sizes().vec();
+      ctx->saved_data["types"] = std::vector<int64_t>{int64_t(q.scalar_type()), int64_t(k.scalar_type())};
+    }
     return rotate(q, k, c, s, false);
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto saved = ctx->get_saved_variables();
     // (an output that no loss used: zeros of its own shape and type; q and k may differ in both)
-    const auto types = ctx->saved_data["types"].toIntVector();
     auto grad = [&](int i, const char* shape) {
-      return g[i].defined() ? g[i] : torch::zeros(ctx->saved_data[shape].toIntVector(), saved[0].options().dtype(at::ScalarType(types[i])));
+      if (g[i].defined()) return g[i];
+      if (!ctx->saved_data.count(shape)) return torch::zeros_like(g[1 - i]);
+      return torch::zeros(ctx->saved_data[shape].toIntVector(), saved[0].options().dtype(at::ScalarType(ctx->saved_data["types"].toIntVector()[i])));
     };
     auto out = rotate(grad(0, "q"), grad(1, "k"), saved[0], saved[1], true);
     return {out[0], out[1], Tensor(), Tensor()};
