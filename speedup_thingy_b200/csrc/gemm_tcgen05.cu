@@ -700,6 +700,7 @@ float persistent_us(const rte_gemm_args* a, TileConfig t, int splits, int sms) {
   const float kb = float(rte::ceil_div(rte::ceil_div(a->K, BK), splits));
   const float slope = waves > 1 ? slope_busy[i] : slope_idle[i] + (slope_busy[i] - slope_idle[i]) * float(units) / float(conc);
   static const float store_swb[4] = {9.f, 9.f, 5.3f, 5.3f};                // SwiGLU's backward: (up | gate) in, (d up | d gate) out
+  // (SwiGLU's forward writes three pieces per 64 hidden units instead of two and has no term of its own yet)
   const float store = a->epilogue == RTE_EPI_SWIGLU_BWD ? store_swb[i] : store_bf16[i] * (res ? 3.8f : f32 ? 2.f : 1.f);
   const float loop = kb * slope;
   return (res ? base_res[i] : f32 ? base_f32[i] : base_bf16[i]) + loop + float(waves - 1) * (loop > store ? loop : store);

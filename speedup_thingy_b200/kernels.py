@@ -183,6 +183,7 @@ def k_logits_shortlist(hidden, vocab_weight, shortlist):
 
 # --------------------------------------------------------------------------- cross entropy (reference.py:146-147)
 def k_cross_entropy_unreduced(logits, targets):
+    """Per-token loss.  Backward reads the logits again: autograd refuses it if they have been modified in place by then."""
     _require_cuda_tensor(logits, targets)
     if logits.shape[:-1] != targets.shape:
         raise ValueError("k_cross_entropy_unreduced: logits [..., V] with targets [...]")
