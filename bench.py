@@ -1,4 +1,4 @@
-"""Benchmark of the `recursive_macro` training step (BASELINE metric: train tokens/sec).
+"""Benchmark of the `recursive_macro` training step (metric: train tokens/sec).
 
     python bench.py --gpus 1 --steps 20 --warmup 5 [--config c3]
     python -m torch.distributed.run --nnodes=1 --nproc-per-node N ... bench.py --gpus N --steps K --warmup W
@@ -326,7 +326,7 @@ def main() -> None:
     ap.add_argument("--warmup", type=int, default=5)
     ap.add_argument("--impl", default="b200", choices=["b200", "reference"])
     ap.add_argument("--config", default="c3", choices=["c1", "c2", "c3", "c4", "c5"],
-                    help="BASELINE workload (default: c3 = configs[2], the configuration the metric is quoted on)")
+                    help="workload (default: c3, the configuration the metric is quoted on)")
     ap.add_argument("--repeats", type=int, default=5, help="timed regions of --steps steps each (median and spread reported)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-torch-baseline", action="store_true")

@@ -123,7 +123,7 @@ class TrainCfg:
     lambda_delta_rms: float = 2.0
     lambda_endpoint_normed: float = 1.0
     lambda_endpoint_raw: float = 0.05
-    lambda_cons: float = 0.0                        # (the reference's default is 1e-3; the BASELINE workloads use 0)
+    lambda_cons: float = 0.0                        # (the reference's default is 1e-3; the benchmark's workloads use 0)
     distill_temperature: float = 2.0
     coverage_min: float = 0.01
     coverage_beta: float = 0.98

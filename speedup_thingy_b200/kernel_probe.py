@@ -2,7 +2,7 @@
 (`python bench.py --probe-kernels`): one JSON line per kernel with its duration, the bytes one launch has to move,
 the achieved GB/s and the fraction of the measured HBM copy bandwidth.
 
-Shapes are those of BASELINE configs[2] (8192 tokens, d 512, F 2048, V 2048, 8 heads, batch 128 x 64).  Every
+Shapes are those of the c3 workload (8192 tokens, d 512, F 2048, V 2048, 8 heads, batch 128 x 64).  Every
 kernel runs from a CUDA graph of `iters` launches that rotate over enough operand sets to exceed the 126 MB L2, so the
 figures are DRAM figures; the same command under `ncu -k regex:<kernel> -c 1` gives the per-kernel DRAM counters.
 """

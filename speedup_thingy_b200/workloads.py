@@ -20,24 +20,24 @@ from .config import ExperimentConfig, ModelConfig, OutputConfig, TrainingConfig
 
 WORKLOADS: dict[str, dict] = {
     "c1": dict(
-        title="BASELINE configs[0]: recursive_macro depth 4, d128 H4 F512 (8x64 slabs, 2 active) V2048, batch 8x64, no audit",
+        title="recursive_macro depth 4, d128 H4 F512 (8x64 slabs, 2 active) V2048, batch 8x64, no audit",
         model=dict(vocab_size=2048, d_model=128, n_heads=4, d_ff=512, n_prelude=1, n_coda=1, t_max=4, depth_choices=(1, 2, 4),
                    attn_banks=1, ffn_banks=1, head_groups=4, ffn_groups=8, active_head_groups=2, active_ffn_groups=2,
                    recipe_count=5, macro_rank=32, n_dense_layers=4),
         train=dict(mode="recursive_macro", lr=1e-3, weight_decay=0.1, batch_size=8, seq_len=64, seed=0, fixed_depth=4)),
     "c2": dict(
-        title="BASELINE configs[1]: dense_exact 4 layers, d512 H8 F2048 V2048, batch 128x64",
+        title="dense_exact 4 layers, d512 H8 F2048 V2048, batch 128x64",
         model=dict(topology="dense", vocab_size=2048, d_model=512, n_heads=8, d_ff=2048, n_dense_layers=4),
         train=dict(mode="dense_exact", lr=1e-3, weight_decay=0.1, batch_size=128, seq_len=64, seed=0)),
     "c3": dict(
-        title="BASELINE configs[2]: recursive_macro depth 4, d512 H8 F2048 (16x128 slabs, 4 active) V2048, batch 128x64, audit 1/128",
+        title="recursive_macro depth 4, d512 H8 F2048 (16x128 slabs, 4 active) V2048, batch 128x64, audit 1/128",
         model=dict(vocab_size=2048, d_model=512, n_heads=8, d_ff=2048, n_prelude=1, n_coda=1, t_max=4, depth_choices=(1, 2, 4),
                    attn_banks=1, ffn_banks=1, head_groups=8, ffn_groups=16, active_head_groups=2, active_ffn_groups=4,
                    recipe_count=5, macro_rank=32),
         train=dict(mode="recursive_macro", lr=1e-3, weight_decay=0.1, batch_size=128, seq_len=64, seed=0, fixed_depth=4,
                    audit_fixed_count_per_batch=1)),
     "c4": dict(
-        title="BASELINE configs[3]: recursive_macro_shortlist depth 8, d512 H8 F2048 V2048, batch 128x128, audit 2/128, "
+        title="recursive_macro_shortlist depth 8, d512 H8 F2048 V2048, batch 128x128, audit 2/128, "
               "shortlist head (64 clusters, top 2, 128 tokens)",
         model=dict(vocab_size=2048, d_model=512, n_heads=8, d_ff=2048, n_prelude=1, n_coda=1, t_max=8, depth_choices=(1, 2, 4, 8),
                    attn_banks=1, ffn_banks=1, head_groups=8, ffn_groups=16, active_head_groups=2, active_ffn_groups=4,
@@ -47,7 +47,7 @@ WORKLOADS: dict[str, dict] = {
         output=dict(mode="shortlist", num_clusters=64, shortlist_top_clusters=2, shortlist_max_tokens=128, hard_negatives=32,
                     random_negatives=32)),
     "c5": dict(
-        title="BASELINE configs[4] per rank: recursive_macro depth 16, d1024 H16 F4096 (32x128 slabs, 8 active) V32768, "
+        title="recursive_macro depth 16 (per rank), d1024 H16 F4096 (32x128 slabs, 8 active) V32768, "
               "batch 32x256, no audit",
         model=dict(vocab_size=32768, d_model=1024, n_heads=16, d_ff=4096, n_prelude=1, n_coda=1, t_max=16,
                    depth_choices=(1, 2, 4, 8, 16), attn_banks=1, ffn_banks=1, head_groups=16, ffn_groups=32,

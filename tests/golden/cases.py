@@ -3,7 +3,7 @@ Kept free of any import of the reference so that the fixtures can be consumed wh
 from oracle import rte_oracle as O
 
 GOLDEN_CASES = {
-    # BASELINE config 1 (the reference's CPU-runnable case), audit probability 0.
+    # the c1 workload (the reference's CPU-runnable case), audit probability 0.
     "c1_macro": dict(
         model=dict(vocab_size=2048, d_model=128, n_heads=4, d_ff=512, n_dense_layers=4, n_prelude=1, n_coda=1,
                    t_max=4, depth_choices=(1, 2, 4), attn_banks=1, ffn_banks=1, head_groups=4, ffn_groups=8,

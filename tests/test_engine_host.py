@@ -235,7 +235,7 @@ def test_pipelined_train_steps_equal_synchronous_steps(name):
 
 
 def test_hot_budget_matches_reference_estimators_and_enforces_limits():
-    """training.py:707-740 / metrics.py:69-94, pinned to values the reference computed for BASELINE config 1."""
+    """training.py:707-740 / metrics.py:69-94, pinned to values the reference computed for the c1 workload."""
     from pathlib import Path
 
     from speedup_thingy_b200.engine import dense_aligned_param_count, hot_budget

@@ -1,6 +1,6 @@
 """Per-kernel parity on a B200: every C-ABI entry point against the CPU oracle (or, for the plain
 GEMM, an fp32 matmul of the same bf16 inputs).  Tolerances: bf16 kernels max-abs 2e-2 relative to the
-output scale (BASELINE north_star), fp32 kernels 1e-4, indices bit-exact."""
+output scale, fp32 kernels 1e-4, indices bit-exact."""
 import math
 
 import numpy as np

@@ -234,7 +234,7 @@ def test_pipelined_train_steps_equal_synchronous_steps():
 
 
 def test_c3_shapes_one_step_finite_and_close():
-    """BASELINE configs[2] shapes without the audited sample: one step against the fp32 oracle."""
+    """The c3 workload's shapes without the audited sample: one step against the fp32 oracle."""
     model = dict(vocab_size=2048, d_model=512, n_heads=8, d_ff=2048, n_prelude=1, n_coda=1, t_max=4, depth_choices=(1, 2, 4),
                  attn_banks=1, ffn_banks=1, head_groups=8, ffn_groups=16, active_head_groups=2, active_ffn_groups=4,
                  recipe_count=5, macro_rank=32)
