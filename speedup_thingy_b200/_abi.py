@@ -102,6 +102,7 @@ PROTOTYPES = {
     "rte_gemm_bf16_small": (C.c_int, [P(GemmArgs), c_vp]),
     "rte_gemm_bf16_tile": (C.c_int, [P(GemmArgs), C.c_int32, C.c_int32, c_vp]),
     "rte_cast_many_f32_bf16": (C.c_int, [c_vp, c_vp, c_vp, c_i32, c_vp]),
+    "rte_gemm_bf16_resident": (C.c_int, [P(GemmArgs), C.c_int32, c_vp]),
     "rte_rmsnorm_op_fwd": (C.c_int, [c_vp, c_i32, c_vp, c_i32, c_vp, c_i32, c_vp, c_vp, c_i32, c_vp, c_i32, c_vp, c_vp, c_i32, c_i32, C.c_float, c_vp]),
     "rte_rope_views": (C.c_int, [c_vp] * 10 + [c_i32] * 6 + [c_vp]),
     "rte_pack_qkv": (C.c_int, [c_vp] * 7 + [c_i32] * 5 + [c_vp]),

@@ -684,7 +684,7 @@ int make_store_tmap(CUtensorMap* map, const void* base, long long rows, long lon
 // Against one fixed rule (256-column pairs above 128 rows), e.g. 512 x 384 x 128: 6.6 -> 2.6 us, 512 x 384 x 1152 with
 // residual 17.3 -> 6.3 us, 1050 x 512 x 4096: 26.4 -> 12 us, 5000 x 384 x 384 with residual 13.9 -> 5.9 us.
 struct TileConfig { int bn, ctas; };
-struct Choice { int kernel; TileConfig tile; int ksplit; float us; };      // kernel: 0 persistent, 1 cluster tile, 2 mma.sync
+struct Choice { int kernel; TileConfig tile; int ksplit; float us; };      // kernel: 0 persistent, 1 cluster tile, 2 mma.sync, 3 resident A
 
 int persistent_ctas(const rte_gemm_args* a, int sms) { return a->max_ctas > 0 ? a->max_ctas : a->max_ctas < 0 ? -a->max_ctas : sms; }
 
@@ -748,8 +748,24 @@ TileConfig pick_tile(const rte_gemm_args* a, int splits, int sms, float* us = nu
   return best;
 }
 
+// Short reductions with many tiles go to the kernel that keeps A in shared memory (gemm_resident.cu): three or more 256 x 256 tiles per
+// CTA pair for plain results (two: 4096 x 1536 x 512 11.7 -> 12.3 us, three: 8192 x 1536 x 512 16.8 -> 15.5), any number with SwiGLU.  Not
+// reductions of at most 256 (16384 x 1024 x 256 14.5 -> 14.8) nor more than 32 tiles along N (8192 x 16384 x 512 116 -> 119, 8192 x 32768
+// x 512 237 -> 265), where every pair would stream all of a B that no longer stays in L2 beside the results.
+bool resident(const rte_gemm_args* a, int splits, int sms) {
+  const bool swiglu = a->epilogue == RTE_EPI_SWIGLU_FWD;
+  if ((a->epilogue != RTE_EPI_BF16 && !swiglu) || a->K > 512 || a->a_mn_major || splits > 1 || a->tile_group != nullptr || a->split_kblocks != nullptr ||
+      a->tile_n != 0 || a->cta_pair != 0 || a->M <= BM || ((reinterpret_cast<uintptr_t>(a->C) | reinterpret_cast<uintptr_t>(swiglu ? a->C2 : nullptr)) & 31) ||
+      a->ldc % 16 || (swiglu && a->ldc2 % 16))
+    return false;
+  const int pairs = persistent_ctas(a, sms) / 2, n_blocks = rte::ceil_div(a->N, 256);
+  if (pairs < 1) return false;
+  return swiglu || (a->K > 256 && n_blocks <= 32 && (long long)rte::ceil_div(a->M, 256) * n_blocks > 2LL * pairs);
+}
+
 Choice choose(const rte_gemm_args* a, int splits, int sms) {
   Choice c = {0, {0, 0}, 1, 0.f};
+  if (resident(a, splits, sms)) return {3, {0, 0}, 1, 0.f};
   c.tile = pick_tile(a, splits, sms, &c.us);
   if (a->tile_n != 0 || a->cta_pair != 0 || splits > 1 || a->tile_group != nullptr || a->split_kblocks != nullptr ||
       (a->epilogue != RTE_EPI_BF16 && a->epilogue != RTE_EPI_F32))
@@ -835,10 +851,10 @@ extern "C" int rte_device_sm_count(void) {
   return n;
 }
 
-// us, separate -> fused: forward 8192 x 512 -> 2048 53.8 -> 46.0, 6144 x 512 -> 2048 42.0 -> 39.0, 4096 x 512 -> 2048 even; 8192 x
-// 256 -> 1024 23.1 -> 25.9, 512 x 128 -> 512 5.4 -> 8.8; backward (its operands come by TMA, so it pays earlier) 8192 x 512 ->
+// us, separate -> fused: forward 8192 x 512 -> 2048 50.2 -> 39.6, 5000 x 384 -> 1536 24.7 -> 21.4, 2048 x 1024 -> 2048 23.4 -> 22.8, 1024 x
+// 512 -> 2048 11.4 -> 10.1; 2048 x 1024 -> 1024 14.5 -> 15.5, 512 x 512 -> 2048 8.4 -> 9.1, 512 x 128 -> 512 5.2 -> 7.3; backward (its operands come by TMA, so it pays earlier) 8192 x 512 ->
 // 2048 53.7 -> 37.3, 8192 x 256 -> 1024 20.8 -> 17.3, 1000 x 256 -> 1024 7.8 -> 6.7; 512 x 128 -> 512 4.9 -> 6.0
-extern "C" int64_t rte_swiglu_fuse_min(int32_t backward) { return backward ? 1000000 : 12000000; }
+extern "C" int64_t rte_swiglu_fuse_min(int32_t backward) { return backward ? 1000000 : 4000000; }
 
 extern "C" int rte_gemm_wgrad_splits(const rte_gemm_args* a, int32_t max_splits) {
   if (a == nullptr || a->M <= 0 || a->N <= 0 || a->K <= 0) return 1;
@@ -877,6 +893,7 @@ extern "C" int rte_gemm_bf16(const rte_gemm_args* a, rte_stream_t stream) {
   const Choice c = choose(a, splits, sms);
   if (c.kernel == 1) return rte_gemm_bf16_tile(a, c.tile.bn, c.ksplit, stream);
   if (c.kernel == 2) return rte_gemm_bf16_small(a, stream);
+  if (c.kernel == 3) return rte_gemm_bf16_resident(a, persistent_ctas(a, sms), stream);
   const int bn = c.tile.bn, ctas = c.tile.ctas;
 
   KParams kp;

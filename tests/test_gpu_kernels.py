@@ -87,6 +87,43 @@ def test_gemm_cluster_tiles(ops, M, N, K, a_mn, b_mn):
                 _close(out, ref + r if mode == "f32_residual" else ref, 1e-2 if mode == "bf16" else 2e-3, f"{M}x{N}x{K} tile {bn} ksplit {ks} {mode}")
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 16, 8), (300, 272, 136), (257, 512, 512), (1050, 1152, 384), (2600, 1040, 448), (700, 4112, 64)])
+@pytest.mark.parametrize("b_mn", [False, True])
+@pytest.mark.parametrize("ctas", [2, 6, 148])
+def test_gemm_resident_rows(ops, M, N, K, b_mn, ctas):
+    """rte_gemm_bf16_resident: one k-block to eight, ragged rows / columns / k-blocks, runs of tiles that change their rows in the
+    middle (few CTAs) and single tiles; SwiGLU's forward where the columns pair up."""
+    import ctypes as C
+
+    from speedup_thingy_b200 import _abi as A
+    g = torch.Generator().manual_seed(M + N + K)
+    a, b = _bf(torch.randn(M, K, generator=g)), _bf(torch.randn(N, K, generator=g) * K ** -0.5)
+    ref = a.float() @ b.float().t()
+    a_dev, b_dev = a.to(DEV), (b.t().contiguous() if b_mn else b).to(DEV)
+    args = A.GemmArgs()
+    args.M, args.N, args.K, args.splits, args.status = M, N, K, 1, ops.status.data_ptr()
+    args.A, args.lda, args.B, args.ldb, args.b_mn_major = a_dev.data_ptr(), K, b_dev.data_ptr(), b_dev.stride(0), int(b_mn)
+    out = torch.full((M + 1, N), 7.0, device=DEV, dtype=torch.bfloat16)
+    args.C, args.ldc, args.epilogue = out.data_ptr(), N, A.EPI_BF16
+    A.check(ops.lib.rte_gemm_bf16_resident(C.byref(args), ctas, ops.stream), "rte_gemm_bf16_resident")
+    torch.cuda.synchronize()
+    ops.check_status()
+    _close(out[:M], ref, 1e-2, f"{M}x{N}x{K}")
+    assert bool((out[M] == 7.0).all())
+    if b_mn or N % 64:
+        return
+    F_ = N // 2
+    ug, z = torch.full((M + 1, N), 7.0, device=DEV, dtype=torch.bfloat16), torch.full((M + 1, F_), 7.0, device=DEV, dtype=torch.bfloat16)
+    args.C, args.ldc, args.C2, args.ldc2, args.b_pair_offset, args.epilogue = z.data_ptr(), F_, ug.data_ptr(), N, F_, A.EPI_SWIGLU_FWD
+    A.check(ops.lib.rte_gemm_bf16_resident(C.byref(args), ctas, ops.stream), "rte_gemm_bf16_resident")
+    torch.cuda.synchronize()
+    ops.check_status()
+    up, gate = out[:M, :F_].float(), out[:M, F_:].float()
+    assert torch.equal(ug[:M], out[:M])
+    _close(z[:M], up * torch.nn.functional.silu(gate), 1e-2, "z")                  # (z is formed from the rounded up and gate)
+    assert bool((ug[M] == 7.0).all()) and bool((z[M] == 7.0).all())
+
+
 @pytest.mark.parametrize("M,N,K", [(64, 1536, 512), (64, 512, 4096), (70, 104, 136), (256, 2048, 512), (1, 8, 8), (130, 96, 72)])
 @pytest.mark.parametrize("b_mn", [False, True])
 @pytest.mark.parametrize("mode", ["bf16", "f32_residual", "f32_split"])
