@@ -157,6 +157,14 @@ int rte_embed_fwd(const int64_t* tokens, const float* table, float* out, int32_t
  * any contents) as 64-bit fixed point (2^-40 resolution, order-free integer atomics) and are added to dtable once. */
 int rte_embed_bwd(const int64_t* tokens, const float* dx, float* dtable, int64_t* accum, int32_t n_tokens, int32_t d,
                   int32_t vocab, int32_t* status, rte_stream_t stream);
+/* The same in two halves, for callers that know the tokens before dx: _group orders the token positions by id in `accum`,
+ * _grouped (ordered after it, same `accum`, sizes and dtable) adds the rows: the bits of rte_embed_bwd.
+ * RTE_ERR_UNSUPPORTED where that does not pay or fit (fewer than 2^18 elements, d % 4, vocab > 49152, a scratch smaller than the
+ * lists need).                                                                                                        */
+int rte_embed_bwd_group(const int64_t* tokens, const float* dtable, int64_t* accum, int32_t n_tokens, int32_t d, int32_t vocab,
+                        int32_t* status, rte_stream_t stream);
+int rte_embed_bwd_grouped(const float* dx, float* dtable, int64_t* accum, int32_t n_tokens, int32_t d, int32_t vocab,
+                          rte_stream_t stream);
 
 /* ------------------------------------------------- RMSNorm (kernels/reference.py:9-17)
  * y = x * rsqrt(mean(x^2) + eps) * w [* (1 + film_gamma) + film_beta]  (FiLM: layers.py:841-847)

@@ -89,6 +89,154 @@ embed_bwd_rows_kernel(const int64_t* __restrict__ tokens, unsigned long long* __
   }
 }
 
+// The same sums with the tokens grouped by id beforehand (the ids are known when a step begins, so a caller groups them beside
+// its forward pass): a warp adds up to 16 rows of one id and 128 columns in registers, all its loads in flight at once, and writes
+// the table once; the pieces of an id with more meet in 64-bit accumulators, and the last one to arrive converts.  Every sum is the integer it was,
+// so the bits are the same.  Bound by the read of dx: one atomic per element and a pass over all accumulators are gone (us,
+// accumulate and apply -> grouped: 8192 x 512 of 2048 ids 24.5 -> 10.9, 16384 x 512 45 -> 24, 8192 x 1024 of 32768 ids 80 -> 30; 512 x 128
+// 5.3 -> 6.3, hence the line at 2^18 elements; the grouping itself takes 4..19 us beside other work).
+constexpr int EG_THREADS = 1024, EG_PIECE = 16, EG_COLS = 128;
+constexpr int EG_MAX_VOCAB = 48 * 1024;                      // one counter per id in shared memory
+struct EmbedGroups {
+  int* head;                 // [0]: pieces
+  int4* piece;               // id, first entry of `order`, entries | pieces of the id << 8, row of `sums` (< 0: the id's only piece)
+  int* order;                // token positions grouped by id
+  int* ticket;               // per row of `sums` and column block: pieces that have arrived
+  unsigned long long* sums;
+};
+inline size_t embed_groups_layout(void* scratch, int n, int d, EmbedGroups* g, size_t* clear_from = nullptr) {
+  auto up = [](size_t x) { return (x + 15) & ~(size_t)15; };
+  const size_t multi = (size_t)n / EG_PIECE, blocks = rte::ceil_div(d, EG_COLS);
+  const size_t piece = 16, order = piece + 16 * (size_t)n, ticket = up(order + 4 * (size_t)n), sums = up(ticket + 4 * multi * blocks);
+  char* at = reinterpret_cast<char*>(scratch);
+  if (g) *g = {reinterpret_cast<int*>(at), reinterpret_cast<int4*>(at + piece), reinterpret_cast<int*>(at + order), reinterpret_cast<int*>(at + ticket),
+               reinterpret_cast<unsigned long long*>(at + sums)};
+  if (clear_from) *clear_from = ticket;
+  return sums + 8 * multi * d;
+}
+inline bool embed_groups_fit(const void* scratch, const void* dtable, int n, int d, int vocab) {
+  return d % 4 == 0 && (long long)n * d >= (1 << 18) && vocab <= EG_MAX_VOCAB && n < (1 << 23) && ((reinterpret_cast<uintptr_t>(scratch) | reinterpret_cast<uintptr_t>(dtable)) & 15) == 0 &&
+         embed_groups_layout(nullptr, n, d, nullptr) <= (size_t)vocab * d * 8;
+}
+
+// One CTA: counts per id in shared memory, their running sums (ids dealt to the threads round robin), pieces, order.
+__global__ void __launch_bounds__(EG_THREADS)
+embed_group_kernel(const int64_t* __restrict__ tokens, int n, int vocab, EmbedGroups G, int* status) {
+  rte::after_previous_grid();
+  extern __shared__ int eg_count[];
+  __shared__ int wsum[3][32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int v = tid; v < vocab; v += EG_THREADS) eg_count[v] = 0;
+  __syncthreads();
+#pragma unroll 4
+  for (int t = tid; t < n; t += EG_THREADS) {
+    const long long tok = tokens[t];
+    if (tok >= 0 && tok < vocab) atomicAdd(&eg_count[tok], 1);
+    else if (status) atomicExch(status, RTE_DEV_INDEX_OUT_OF_RANGE);
+  }
+  __syncthreads();
+  int a[3] = {0, 0, 0};                                      // tokens, pieces, ids of several pieces
+  for (int v = tid; v < vocab; v += EG_THREADS) {
+    const int k = eg_count[v];
+    a[0] += k; a[1] += (k + EG_PIECE - 1) / EG_PIECE; a[2] += k > EG_PIECE;
+  }
+  int upto[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    int x = a[q];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += y; }
+    upto[q] = x;
+    if (lane == 31) wsum[q][warp] = x;
+  }
+  __syncthreads();
+  if (warp < 3) {
+    int x = wsum[warp][lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int y = __shfl_up_sync(0xffffffffu, x, o); if (lane >= o) x += y; }
+    wsum[warp][lane] = x;
+  }
+  __syncthreads();
+  int at[3];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) at[q] = upto[q] - a[q] + (warp > 0 ? wsum[q][warp - 1] : 0);
+  if (tid == 0) G.head[0] = wsum[1][31];
+  for (int v = tid; v < vocab; v += EG_THREADS) {
+    const int k = eg_count[v], pieces = (k + EG_PIECE - 1) / EG_PIECE;
+    for (int q = 0; q < pieces; ++q)
+      G.piece[at[1] + q] = make_int4(v, at[0] + q * EG_PIECE, min(EG_PIECE, k - q * EG_PIECE) | pieces << 8, pieces > 1 ? at[2] : -1);
+    eg_count[v] = at[0];
+    at[0] += k; at[1] += pieces; at[2] += pieces > 1;
+  }
+  __syncthreads();
+#pragma unroll 4
+  for (int t = tid; t < n; t += EG_THREADS) {
+    const long long tok = tokens[t];
+    if (tok >= 0 && tok < vocab) G.order[atomicAdd(&eg_count[tok], 1)] = t;
+  }
+}
+
+__global__ void __launch_bounds__(256)
+embed_sum_kernel(const float* __restrict__ dx, float* dtable, EmbedGroups G, int d) {
+  rte::after_previous_grid();
+  const int lane = threadIdx.x & 31, blocks = (d + EG_COLS - 1) / EG_COLS, d4 = d >> 2;
+  const long long jobs = (long long)G.head[0] * blocks;
+  for (long long j = blockIdx.x * 8LL + (threadIdx.x >> 5); j < jobs; j += gridDim.x * 8LL) {
+    const int4 piece = G.piece[j / blocks];
+    const int cb = int(j % blocks), c = cb * (EG_COLS / 4) + lane, count = piece.z & 255, pieces = piece.z >> 8;      // c: in float4
+    const int mine = lane < count ? G.order[piece.y + lane] : 0;
+    const bool in = c < d4;
+    float4 x[EG_PIECE];
+#pragma unroll
+    for (int i = 0; i < EG_PIECE; ++i) {
+      const int row = __shfl_sync(0xffffffffu, mine, i);
+      x[i] = in && i < count ? reinterpret_cast<const float4*>(dx)[(size_t)row * d4 + c] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    long long acc[4] = {0, 0, 0, 0};
+    unsigned bad = 0;
+#pragma unroll
+    for (int i = 0; i < EG_PIECE; ++i) {
+      if (i >= count) break;
+      const float v[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (isfinite(v[e])) acc[e] += __float2ll_rn(v[e] * EMBED_FX_SCALE);
+        else bad |= 1u << e;
+      }
+    }
+    float* out = dtable + (size_t)piece.x * d + 4 * c;
+    const unsigned long long* sums = nullptr;
+    if (piece.w >= 0) {                                       // one of several pieces
+      unsigned long long* into = G.sums + (size_t)piece.w * d + 4 * c;
+      if (in) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (bad >> e & 1) out[e] = __int_as_float(0x7fffffff);      // NaN stays NaN through the final add
+          atomicAdd(into + e, (unsigned long long)acc[e]);
+        }
+      }
+      __threadfence();
+      __syncwarp();
+      int arrived = 0;
+      if (lane == 0) arrived = atomicAdd(&G.ticket[piece.w * blocks + cb], 1);
+      if (__shfl_sync(0xffffffffu, arrived, 0) != pieces - 1) continue;
+      __threadfence();
+      sums = into;
+      bad = 0;
+    }
+    if (!in) continue;
+    float4 o = __ldcg(reinterpret_cast<float4*>(out));
+    float* ov = &o.x;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const long long v = sums ? (long long)__ldcg(sums + e) : acc[e];
+      if (bad >> e & 1) ov[e] = __int_as_float(0x7fffffff);
+      else if (v != 0) ov[e] += __ll2float_rn(v) * (1.f / EMBED_FX_SCALE);
+    }
+    *reinterpret_cast<float4*>(out) = o;
+  }
+}
+
 // ------------------------------------------------------------------ RMSNorm
 // One warp per row, row held in registers (d <= 32 * 4 * RN_MAX_V4).
 constexpr int RN_MAX_V4 = 16;   // d up to 2048
@@ -1048,6 +1196,34 @@ extern "C" int rte_embed_bwd(const int64_t* tokens, const float* dx, float* dtab
   rte::launch(embed_bwd_accum_kernel, grid, 128, 0, ST(stream), tokens, dx, fx, dtable, n_tokens, d, vocab, status);
   if (rows) rte::launch(embed_bwd_rows_kernel, grid, 256, 0, ST(stream), tokens, fx, dtable, n_tokens, d, vocab, 1);
   else rte::launch(embed_bwd_apply_kernel, grid_for(n, 256), 256, 0, ST(stream), reinterpret_cast<const unsigned long long*>(accum), dtable, n);
+  RTE_LAUNCH_CHECK();
+  return RTE_OK;
+}
+
+extern "C" int rte_embed_bwd_group(const int64_t* tokens, const float* dtable, int64_t* accum, int32_t n_tokens, int32_t d, int32_t vocab,
+                                   int32_t* status, rte_stream_t stream) {
+  RTE_CHECK_ARG(tokens && dtable && accum && n_tokens > 0 && d > 0 && vocab > 0);
+  if (!embed_groups_fit(accum, dtable, n_tokens, d, vocab)) return RTE_ERR_UNSUPPORTED;
+  EmbedGroups g;
+  size_t clear = 0;
+  const size_t bytes = embed_groups_layout(accum, n_tokens, d, &g, &clear);
+  if (bytes > clear && cudaMemsetAsync(reinterpret_cast<char*>(accum) + clear, 0, bytes - clear, ST(stream)) != cudaSuccess) return RTE_ERR_LAUNCH;
+  const size_t smem = (size_t)vocab * sizeof(int);
+  if (cudaFuncSetAttribute(embed_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, EG_MAX_VOCAB * (int)sizeof(int)) != cudaSuccess)
+    return RTE_ERR_LAUNCH;
+  rte::launch(embed_group_kernel, 1, EG_THREADS, smem, ST(stream), tokens, n_tokens, vocab, g, status);
+  RTE_LAUNCH_CHECK();
+  return RTE_OK;
+}
+extern "C" int rte_embed_bwd_grouped(const float* dx, float* dtable, int64_t* accum, int32_t n_tokens, int32_t d, int32_t vocab,
+                                     rte_stream_t stream) {
+  RTE_CHECK_ARG(dx && dtable && accum && n_tokens > 0 && d > 0 && vocab > 0);
+  if (!embed_groups_fit(accum, dtable, n_tokens, d, vocab)) return RTE_ERR_UNSUPPORTED;
+  if (reinterpret_cast<uintptr_t>(dx) & 15) return RTE_ERR_ALIGNMENT;
+  EmbedGroups g;
+  embed_groups_layout(accum, n_tokens, d, &g);
+  const long long most = rte::ceil_div64((long long)n_tokens * rte::ceil_div(d, EG_COLS), 8);
+  rte::launch(embed_sum_kernel, (int)(most < 148 * 16 ? most : 148 * 16), 256, 0, ST(stream), dx, dtable, g, d);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }

@@ -1039,6 +1039,27 @@ class TrainEngine:
                       g[f"{pre}.norm1.weight"], t.partial2, accumulate_dw=accumulate)
         ready(f"{pre}.norm1.weight")
 
+    # ------------------------------------------------------------------ the embedding's gradient
+    def _group_tokens(self) -> None:
+        """The order in which the embedding's gradient adds its rows needs the tokens only: it is prepared ahead, on the
+        weight-gradient stream in use (`_embed_bwd` then takes one launch; not on a stream of its own from the step's start:
+        a fork there delays the first launches)."""
+        o = self.ops
+        self._tokens_grouped = None
+        stream = getattr(o, "param_stream", None)
+        if stream is None:
+            return
+        with o._deferred():
+            if o.embed_bwd_group(self.tokens, self.grads["embed.weight"], self.embed_accum):
+                self._tokens_grouped = torch.cuda.Event()
+                self._tokens_grouped.record(stream)
+
+    def _embed_bwd(self, dx: torch.Tensor) -> None:
+        if self._tokens_grouped is None:
+            return self.ops.embed_bwd(self.tokens.view(-1), dx, self.grads["embed.weight"], self.embed_accum)
+        torch.cuda.current_stream(self.device).wait_event(self._tokens_grouped)
+        self.ops.embed_bwd_grouped(self.M, dx, self.grads["embed.weight"], self.embed_accum)
+
     # ------------------------------------------------------------------ forward + backward
     def _forward_backward_exact(self, forward_only: bool = False) -> None:
         """`recursive_exact`: embed -> prelude -> router -> t_max banked passes for every sample -> coda -> logits ->
@@ -1085,13 +1106,14 @@ class TrainEngine:
         ps = self._param_stream if hasattr(o, "param_stream") else None
         if ps is not None:
             o.param_stream = ps
+        self._group_tokens()
         for j, blk in enumerate(reversed(self.prelude)):
             self._block_bwd(blk, dcur, g16[j], dalt, g16[j + 1], self.dxc, tmp=self.block_tmps[j], mark_ready=False)
             dcur, dalt = dalt, dcur
         if ps is not None:
             o.param_stream = None
             torch.cuda.current_stream(self.device).wait_stream(ps)       # (the embedding gradient starts from the logits product's share)
-        o.embed_bwd(tokens, dcur, g["embed.weight"], self.embed_accum)
+        self._embed_bwd(dcur)
         self._grad_ready(*self.trainable)
         self._finish_backward()
 
@@ -1268,6 +1290,7 @@ class TrainEngine:
 
         g16 = self.grad16
         defer(True)
+        self._group_tokens()
         o.rmsnorm_bwd(x_last, p["final_norm.weight"], self.rstd_f, self.dn16, None, self.dxa, g16[0],
                       g["final_norm.weight"], self.partial_final)
         audited = self.audit is not None and self.audit.grad       # the replay contributes gradients of its own
@@ -1378,7 +1401,7 @@ class TrainEngine:
                                 mark_ready=not late)
                 dcur, dalt = dalt, dcur
             defer(False)
-        o.embed_bwd(tokens, dcur, g["embed.weight"], self.embed_accum)
+        self._embed_bwd(dcur)
         if audited and self.audit.own_prelude:
             # last join: the replay's prelude and embedding gradients meet the hot pass's
             self._main_wait_side(side_done)

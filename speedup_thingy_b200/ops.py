@@ -212,6 +212,19 @@ class CudaOps:
         self._call("rte_embed_bwd", _ptr(tokens), _ptr(dx), _ptr(dtable), _ptr(accum), tokens.numel(), dtable.shape[1],
                    dtable.shape[0], _ptr(self.status), self.stream)
 
+    def embed_bwd_group(self, tokens, dtable, accum) -> bool:
+        """Orders the tokens by id in `accum` ahead of `embed_bwd_grouped`; False where only `embed_bwd` serves."""
+        rc = self.lib.rte_embed_bwd_group(_ptr(tokens), _ptr(dtable), _ptr(accum), tokens.numel(), dtable.shape[1], dtable.shape[0],
+                                          _ptr(self.status), self.stream)
+        if rc == A.ERR_UNSUPPORTED:
+            return False
+        self.launches += 1
+        A.check(rc, "rte_embed_bwd_group")
+        return True
+
+    def embed_bwd_grouped(self, n_tokens: int, dx, dtable, accum) -> None:
+        self._call("rte_embed_bwd_grouped", _ptr(dx), _ptr(dtable), _ptr(accum), n_tokens, dtable.shape[1], dtable.shape[0], self.stream)
+
     def rmsnorm_fwd(self, x, w, y_bf16, rstd, *, y_f32=None, film_gamma=None, film_beta=None, eps: float = 1e-5,
                     rows: int | None = None) -> None:
         _require_cuda(x, w)

@@ -406,6 +406,27 @@ def test_embedding_fwd_bwd(ops):
     _close(dt2, 2 * torch.zeros(V, d).index_add_(0, tok, dx), 1e-5, "embedding grad accumulates")
 
 
+@pytest.mark.parametrize("V,d,n,same", [(2048, 132, 2500, 700), (300, 512, 600, 17), (5000, 1024, 3000, 16), (700, 128, 3000, 2000), (9, 4, 70000, 0)])
+def test_embedding_bwd_of_grouped_tokens(ops, V, d, n, same):
+    """Tokens grouped by id ahead: the bits of the ungrouped sum -- ids of one piece, of several, of exactly a piece, absent ids, a
+    column block past the width, accumulation onto what is there, a gradient that is not finite."""
+    g = torch.Generator().manual_seed(n)
+    tok, dx, base = torch.randint(0, V, (n,), generator=g), torch.randn(n, d, generator=g), torch.randn(V, d, generator=g)
+    tok[:same] = V - 1
+    dx[n // 2, d // 2], dx[0, d - 1] = float("inf"), float("nan")
+    tok, dx = tok.to(DEV), dx.to(DEV)
+    acc = torch.full((max(V * d, 4 * n),), 12345, dtype=torch.int64, device=DEV)
+    one, two = base.to(DEV), base.to(DEV)
+    ops.embed_bwd(tok, dx, one, acc)
+    grouped = ops.embed_bwd_group(tok, two, acc)
+    assert grouped == ops.embed_bwd_group(tok, two, acc)                           # (again: the scratch may hold anything)
+    assert grouped or n * d < 2 ** 18 or V * d < 4 * n
+    if grouped:
+        ops.embed_bwd_grouped(n, dx, two, acc)
+        torch.cuda.synchronize()
+        assert torch.equal(one.isnan(), two.isnan()) and torch.equal(one.nan_to_num(), two.nan_to_num())
+
+
 @pytest.mark.parametrize("V,d,n", [(4096, 64, 700), (2000, 65, 1000), (1999, 128, 1000)])
 def test_embedding_bwd_of_a_table_larger_than_the_batch(ops, V, d, n):
     """Only the batch's rows of the accumulator are cleared and applied (the line is at twice the tokens); repeated tokens
