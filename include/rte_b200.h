@@ -375,6 +375,13 @@ int rte_macro_phi_bwd_data(const float* h0, const float* dout, const rte_phi_par
                            const int32_t* stride_id, float s_cfg, const float* rstd, const float* act, float* dh0,
                            float* scratch, int32_t B, int32_t S, int32_t d, int32_t m, int32_t K_strides,
                            rte_stream_t stream);
+/* _data with what usually follows it: router_scratch != NULL adds the router's share of d h0 (rte_router_aux_add_dh0 of that
+ * scratch, hidden width hid, R recipes), dh0_bf16 != NULL receives the bf16 copy of the sum (rte_cast_f32_bf16): in _data's last
+ * launch where the tensor-core form runs, otherwise as those launches behind it.                                          */
+int rte_macro_phi_bwd_data_finish(const float* h0, const float* dout, const rte_phi_params* p, const int32_t* recipe_id,
+                                  const int32_t* stride_id, float s_cfg, const float* rstd, const float* act, float* dh0,
+                                  float* scratch, const float* router_scratch, int32_t hid, int32_t R, void* dh0_bf16,
+                                  int32_t B, int32_t S, int32_t d, int32_t m, int32_t K_strides, rte_stream_t stream);
 int rte_macro_phi_bwd_params(const float* h0, const int32_t* recipe_id, const int32_t* stride_id, const float* rstd,
                              const float* pooled, const float* act, const rte_phi_grads* g, float* scratch,
                              int32_t B, int32_t S, int32_t d, int32_t m, int32_t R, int32_t K_strides,

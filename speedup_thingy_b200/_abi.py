@@ -102,8 +102,8 @@ PROTOTYPES = {
     "rte_gemm_bf16": (C.c_int, [P(GemmArgs), c_vp]),
     "rte_gemm_bf16_small": (C.c_int, [P(GemmArgs), c_vp]),
     "rte_gemm_bf16_tile": (C.c_int, [P(GemmArgs), C.c_int32, C.c_int32, c_vp]),
-    "rte_cast_many_f32_bf16": (C.c_int, [c_vp, c_vp, c_vp, c_i32, c_vp]),
     "rte_gemm_bf16_resident": (C.c_int, [P(GemmArgs), C.c_int32, c_vp]),
+    "rte_cast_many_f32_bf16": (C.c_int, [c_vp, c_vp, c_vp, c_i32, c_vp]),
     "rte_rmsnorm_op_fwd": (C.c_int, [c_vp, c_i32, c_vp, c_i32, c_vp, c_i32, c_vp, c_vp, c_i32, c_vp, c_i32, c_vp, c_vp, c_i32, c_i32, C.c_float, c_vp]),
     "rte_rope_views": (C.c_int, [c_vp] * 10 + [c_i32] * 6 + [c_vp]),
     "rte_pack_qkv": (C.c_int, [c_vp] * 7 + [c_i32] * 5 + [c_vp]),
@@ -151,6 +151,8 @@ PROTOTYPES = {
                                        P(PhiGrads), c_vp] + [c_i32] * 6 + [c_vp]),
     "rte_sqdiff_grad": (C.c_int, [c_vp, c_vp, c_i64, c_f32, c_vp, c_vp, c_vp, c_i32, c_vp]),
     "rte_macro_phi_bwd_data": (C.c_int, [c_vp, c_vp, P(PhiParams), c_vp, c_vp, c_f32, c_vp, c_vp, c_vp, c_vp] + [c_i32] * 5 + [c_vp]),
+    "rte_macro_phi_bwd_data_finish": (C.c_int, [c_vp, c_vp, P(PhiParams), c_vp, c_vp, c_f32, c_vp, c_vp, c_vp, c_vp, c_vp, c_i32, c_i32, c_vp]
+                                      + [c_i32] * 5 + [c_vp]),
     "rte_macro_phi_bwd_params": (C.c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, P(PhiGrads), c_vp] + [c_i32] * 6 + [c_vp]),
     "rte_cluster_route": (C.c_int, [c_vp, c_i32, c_vp, c_vp, c_vp, c_i32, c_i32, c_i32, c_vp]),
     "rte_cluster_pack": (C.c_int, [c_vp, c_i32, c_i32, c_i32, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp]),

@@ -345,7 +345,7 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
 }
 
 __device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
@@ -897,7 +897,8 @@ template <int KC>
 __global__ void __launch_bounds__(NTHR, KC == 1 ? 2 : 1)
 phi_dz_mma_kernel(const float* __restrict__ h0, const float* __restrict__ rstd, const float* __restrict__ da,
                   const float* __restrict__ dpool, const float* __restrict__ v, const int32_t* __restrict__ rid,
-                  const int32_t* __restrict__ sid, float* dh0, float* dhx, PhiDims D) {
+                  const int32_t* __restrict__ sid, float* dh0, float* dhx, const float* __restrict__ row_add, int parts, long long part_stride,
+                  __nv_bfloat16* __restrict__ dh16, PhiDims D) {
   rte::after_previous_grid();
   __shared__ float sdot[TT][4];
   const int tiles = rte::ceil_div(D.S, TT);
@@ -1006,6 +1007,14 @@ phi_dz_mma_kernel(const float* __restrict__ h0, const float* __restrict__ rstd, 
     product(v1, cb, c1);
     product(v3, cb, c3);
     const float4 dpa = *reinterpret_cast<const float4*>(dpb + col), dpc = *reinterpret_cast<const float4*>(dpb + col + 4);
+    float4 ra = zero4, rb = zero4;                   // what every token of the sample gets on top
+    if (row_add)
+      for (int k = 0; k < parts; ++k) {
+        const float* r = row_add + k * part_stride + (size_t)b * D.d + col;
+        const float4 xa = *reinterpret_cast<const float4*>(r), xb = *reinterpret_cast<const float4*>(r + 4);
+        ra.x += xa.x; ra.y += xa.y; ra.z += xa.z; ra.w += xa.w;
+        rb.x += xb.x; rb.y += xb.y; rb.z += xb.z; rb.w += xb.w;
+      }
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       const bool ok = half ? ok1 : ok0;
@@ -1020,7 +1029,14 @@ phi_dz_mma_kernel(const float* __restrict__ h0, const float* __restrict__ rstd, 
       float4 oa = q[0], ob = q[1];
       finish(oa, l1, own3 ? zero4 : l3, dpa, ha, rs, dot);
       finish(ob, h1, own3 ? zero4 : h3, dpc, hb, rs, dot);
+      if (row_add) {
+        oa.x += ra.x; oa.y += ra.y; oa.z += ra.z; oa.w += ra.w;
+        ob.x += rb.x; ob.y += rb.y; ob.z += rb.z; ob.w += rb.w;
+      }
       q[0] = oa; q[1] = ob;
+      if (dh16)
+        *reinterpret_cast<uint4*>(dh16 + row * D.d + col) = make_uint4(rte::pack_bf16x2(oa.x, oa.y), rte::pack_bf16x2(oa.z, oa.w),
+                                                                       rte::pack_bf16x2(ob.x, ob.y), rte::pack_bf16x2(ob.z, ob.w));
       if (own3) {
         float4* qx = reinterpret_cast<float4*>(dhx + row * D.d + col);
         float4 xa = qx[0], xb = qx[1];
@@ -1221,7 +1237,7 @@ namespace {
 int phi_bwd_data_impl(const float* h0, const float* dout, const rte_phi_params* p, const int32_t* recipe_id,
                       const int32_t* stride_id, float s_cfg, const float* rstd, const float* act, float* dh0, float* dhx,
                       float* scratch, int32_t B, int32_t S, int32_t d, int32_t m, int32_t K_strides,
-                      rte_stream_t stream) {
+                      rte_stream_t stream, const float* row_add = nullptr, void* dh16 = nullptr) {
   RTE_CHECK_ARG(h0 && dhx && dout && p && recipe_id && stride_id && rstd && act && dh0 && scratch && B > 0 && S > 0 && d > 0 && m > 0 &&
                 K_strides > 0);
   if (m > MMAX || B > 1024) return RTE_ERR_UNSUPPORTED;
@@ -1254,11 +1270,25 @@ int phi_bwd_data_impl(const float* h0, const float* dout, const rte_phi_params* 
   RTE_LAUNCH_CHECK();
   rte::launch(phi_dpool_kernel, B * rte::ceil_div(d, NTHR), NTHR, 0, ST(stream), x.da, p->v, recipe_id, stride_id, x.dpool, D);
   RTE_LAUNCH_CHECK();
-  if (mma && m <= 32) rte::launch(phi_dz_mma_kernel<1>, B * tiles, NTHR, 0, ST(stream), h0, rstd, x.da, x.dpool, p->v, recipe_id, stride_id, dh0, dhx, D);
-  else if (mma) rte::launch(phi_dz_mma_kernel<2>, B * tiles, NTHR, 0, ST(stream), h0, rstd, x.da, x.dpool, p->v, recipe_id, stride_id, dh0, dhx, D);
+  if (mma) {                       // (with the sum's last terms and its copy, where they are wanted: one pass over dh0 instead of three)
+    const bool wide = ((reinterpret_cast<uintptr_t>(row_add) | reinterpret_cast<uintptr_t>(dh16)) & 15) == 0;
+    const float* ra = wide ? row_add : nullptr;
+    __nv_bfloat16* o16 = wide ? reinterpret_cast<__nv_bfloat16*>(dh16) : nullptr;
+    if (m <= 32)
+      rte::launch(phi_dz_mma_kernel<1>, B * tiles, NTHR, 0, ST(stream), h0, rstd, x.da, x.dpool, p->v, recipe_id, stride_id, dh0, dhx, ra,
+                  RTE_ROUTER_DPOOLED_PARTS, (long long)B * d, o16, D);
+    else
+      rte::launch(phi_dz_mma_kernel<2>, B * tiles, NTHR, 0, ST(stream), h0, rstd, x.da, x.dpool, p->v, recipe_id, stride_id, dh0, dhx, ra,
+                  RTE_ROUTER_DPOOLED_PARTS, (long long)B * d, o16, D);
+    if (wide) { row_add = nullptr; dh16 = nullptr; }
+  }
   else rte::launch(phi_dz_kernel, B * tiles, NTHR, 0, ST(stream), h0, rstd, x.da, x.dpool, p->v, recipe_id, stride_id, dh0, dhx, D);
   RTE_LAUNCH_CHECK();
-  return RTE_OK;
+  if (row_add) {
+    const int rc = rte::add_router_dpooled(dh0, row_add, B, S, d, ST(stream));
+    if (rc != RTE_OK) return rc;
+  }
+  return dh16 ? rte_cast_f32_bf16(dh0, dh16, (int64_t)B * S * d, stream) : RTE_OK;
 }
 }  // namespace
 
@@ -1268,6 +1298,17 @@ extern "C" int rte_macro_phi_bwd_data(const float* h0, const float* dout, const 
                                       float* scratch, int32_t B, int32_t S, int32_t d, int32_t m, int32_t K_strides,
                                       rte_stream_t stream) {
   return phi_bwd_data_impl(h0, dout, p, recipe_id, stride_id, s_cfg, rstd, act, dh0, dh0, scratch, B, S, d, m, K_strides, stream);
+}
+
+extern "C" int rte_macro_phi_bwd_data_finish(const float* h0, const float* dout, const rte_phi_params* p, const int32_t* recipe_id,
+                                             const int32_t* stride_id, float s_cfg, const float* rstd, const float* act, float* dh0,
+                                             float* scratch, const float* router_scratch, int32_t hid, int32_t R, void* dh0_bf16,
+                                             int32_t B, int32_t S, int32_t d, int32_t m, int32_t K_strides, rte_stream_t stream) {
+  RTE_CHECK_ARG(router_scratch == nullptr || (hid > 0 && R > 0));
+  if (router_scratch && d % 4 != 0) return RTE_ERR_UNSUPPORTED;
+  if (reinterpret_cast<uintptr_t>(router_scratch) & 15) return RTE_ERR_ALIGNMENT;
+  return phi_bwd_data_impl(h0, dout, p, recipe_id, stride_id, s_cfg, rstd, act, dh0, dh0, scratch, B, S, d, m, K_strides, stream,
+                           router_scratch ? rte::router_dpooled(router_scratch, B, hid, R, K_strides) : nullptr, dh0_bf16);
 }
 
 // Parameter-gradient half: reads dupd and da left in `scratch` by rte_macro_phi_bwd_data (may run on another

@@ -482,7 +482,7 @@ extern "C" int rte_router_aux_bwd_data(const rte_router_weights* w, const rte_ro
   float* dpre_d = dpre_r + (size_t)B * hid;         // [B, hid]
   float* dlog_r = dpre_d + (size_t)B * hid;         // [B, R]
   float* dlog_d = dlog_r + (size_t)B * R;           // [B, K]
-  float* dpooled = scratch + (((size_t)RTE_ROUTER_MAX_R + (size_t)B * (2 * hid + R + K) + 3) & ~(size_t)3);   // [B, d], 16-byte aligned
+  float* dpooled = const_cast<float*>(rte::router_dpooled(scratch, B, hid, R, K));   // [B, d], 16-byte aligned
   if (reinterpret_cast<uintptr_t>(scratch) & 15) return RTE_ERR_ALIGNMENT;
   rte::launch(aux_kernel, 1, NTHR, 0, ST(stream), fwd->recipe_probs, fwd->expected_depth, lambda_load, lambda_depth, aux, mean_prob,
                                          mean_prob_in, B, R);
@@ -506,16 +506,19 @@ extern "C" int rte_router_aux_bwd_data(const rte_router_weights* w, const rte_ro
   return RTE_OK;
 }
 
+int rte::add_router_dpooled(float* dh0, const float* dpooled, int B, int S, int d, cudaStream_t st) {
+  rte::launch(bcast_add_kernel, dim3(rte::ceil_div(d / 4, NTHR), rte::ceil_div(S, BC_ROWS), B), NTHR, 0, st, dh0, dpooled, B * S, S, d, RTE_ROUTER_DPOOLED_PARTS, (long long)B * d);
+  RTE_LAUNCH_CHECK();
+  return RTE_OK;
+}
+
 // dh0[b,s,:] += dpooled[b,:] / S from the `scratch` a call of rte_router_aux_bwd_data(dh0 = NULL) left behind.
 extern "C" int rte_router_aux_add_dh0(float* dh0, const float* scratch, int32_t B, int32_t S, int32_t d, int32_t hid, int32_t R,
                                       int32_t K, rte_stream_t stream) {
   RTE_CHECK_ARG(dh0 && scratch && B > 0 && S > 0 && d > 0 && hid > 0 && R > 0 && K > 0);
   if (d % 4 != 0) return RTE_ERR_UNSUPPORTED;
   if (reinterpret_cast<uintptr_t>(scratch) & 15) return RTE_ERR_ALIGNMENT;
-  const float* dpooled = scratch + (((size_t)RTE_ROUTER_MAX_R + (size_t)B * (2 * hid + R + K) + 3) & ~(size_t)3);
-  rte::launch(bcast_add_kernel, dim3(rte::ceil_div(d / 4, NTHR), rte::ceil_div(S, BC_ROWS), B), NTHR, 0, ST(stream), dh0, dpooled, B * S, S, d, RTE_ROUTER_DPOOLED_PARTS, (long long)B * d);
-  RTE_LAUNCH_CHECK();
-  return RTE_OK;
+  return rte::add_router_dpooled(dh0, rte::router_dpooled(scratch, B, hid, R, K), B, S, d, ST(stream));
 }
 
 // Parameter-gradient half of the auxiliary-loss backward: reads dpre / dlog left in `scratch` by the data half.

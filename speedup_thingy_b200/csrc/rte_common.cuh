@@ -58,6 +58,13 @@ inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cud
   (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);      // (an error stays pending for RTE_LAUNCH_CHECK)
 }
 
+// Where a call of rte_router_aux_bwd_data(dh0 = NULL) leaves the parts of d pooled in its scratch, and their add into every
+// token's gradient (router.cu).
+inline const float* router_dpooled(const float* scratch, int B, int hid, int R, int K) {
+  return scratch + (((size_t)RTE_ROUTER_MAX_R + (size_t)B * (2 * hid + R + K) + 3) & ~(size_t)3);
+}
+int add_router_dpooled(float* dh0, const float* dpooled, int B, int S, int d, cudaStream_t st);
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

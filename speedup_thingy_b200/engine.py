@@ -1321,12 +1321,21 @@ class TrainEngine:
             misc = self._misc_param_stream if (split and self._misc_param_stream is not None) else hot
             if split:
                 o.param_stream = misc
+            # where only the router adds to dh0, its share and the bf16 copy of the sum leave with the operator's own launch
+            finish = (split and not getattr(self, "_cons_pending", False) and (not audited or self.audit.own_prelude)
+                      and (tr.disable_router_aux or self._router_early is not None))
+            extra = {}
+            if finish:
+                extra["dh0_16"] = g16[n_tail]
+                if not tr.disable_router_aux:
+                    torch.cuda.current_stream(self.device).wait_event(self._router_early)
+                    extra.update(router_scratch=self.router_scratch, hid=cfg.router_hidden_dim)
             o.macro_phi_bwd_split(self.prelude[-1].out if self.prelude else self.x0, dcur, self._phi_param_dict(),
                                   self.route["recipe_id"], self.route["depth_id"], cfg.macro_update_scale, self.phi_rstd,
                                   self.phi_pooled, self.phi_act, dalt,
                                   dict(gain=g["macro.d_gain"], v=g["macro.v"], u=g["macro.u"], bias=g["macro.bias"]),
                                   self.phi_scratch, B=B, S=S, d=d, m=cfg.macro_rank, R=cfg.recipe_count,
-                                  K=len(cfg.depth_choices))
+                                  K=len(cfg.depth_choices), **extra)
             if split:
                 o.param_stream = None
             if getattr(self, "_cons_pending", False):
@@ -1381,7 +1390,9 @@ class TrainEngine:
                 # under data parallelism each rank contributes 1/world of the auxiliary losses' gradient on its own
                 # samples, with the load-balance term's batch mean taken over ALL shards (`_global_mean_prob`)
                 dims = dict(B=B, S=S, d=d, hid=cfg.router_hidden_dim, R=cfg.recipe_count, K=len(cfg.depth_choices))
-                if self._router_early is not None:
+                if finish:
+                    pass
+                elif self._router_early is not None:
                     torch.cuda.current_stream(self.device).wait_event(self._router_early)
                     o.router_aux_add_dh0(dcur, self.router_scratch, **dims)
                 else:
@@ -1393,7 +1404,8 @@ class TrainEngine:
                     if split:
                         o.param_stream = None
                 self._grad_ready(*self._router_grad_names())
-            o.cast_bf16(dcur, g16[n_tail])
+            if not finish:
+                o.cast_bf16(dcur, g16[n_tail])
             defer(True)
             late = audited and self.audit.own_prelude       # their other share arrives at the last join
             for j, blk in enumerate(reversed(self.prelude)):
