@@ -7,18 +7,20 @@
 // and z_masked = selected ? z : 0, so the down projection is a dense GEMM whose zero rows cost nothing extra.
 //
 // One warp per token, persistent over tokens.  A selection needs only the threshold that separates the k largest from
-// the rest, so it is a root search on count(key >= t) = k over order-preserving integer keys in shared memory: a
-// secant step on log(count) that starts from the previous token's threshold, safeguarded by bisection.  It ends as
-// soon as a probe counts exactly k, or once at most 32 keys are left between the brackets (they are then ranked
-// against each other, one per lane); keys equal to the threshold are taken in ascending index order.  Results are
-// bit-exact with a stable sort by (value descending, index ascending), the tie rule of this build.
+// the rest, so it is a root search on count(key >= t) = k: a secant step on log(count) that starts from the previous token's
+// threshold, safeguarded by bisection.  The keys are the upper halves of the scores, packed as bf16 pairs in shared memory and
+// clamped into the normal range, so that one HSET2 and one HADD2 compare and count two of them.  The search ends as soon as a
+// probe counts exactly k, or once at most 32 keys are left between the brackets; those are ranked against each other, one per
+// lane, by their full scores, which are computed again, equal ones in ascending index order.  Should more than 32 share their upper
+// half (a row of equal scores), the search goes on over the full scores.  Results are bit-exact with a stable sort by (value
+// descending, index ascending), the tie rule of this build.
 //
-// What bounds it: the latency of each warp's own search.  13 KB of shared memory per token leave 16 warps on an SM, four
-// per scheduler, and each alternates a sweep over its keys with a reduction that it has to wait for: 47 % of the issue
-// slots are used (per instruction issued 2.2 warps wait on fixed latencies, 1.9 on global loads, 1.0 on shared memory), HBM
-// at 26 %.  The instructions executed would take 176 us of the 374.  16384 tokens, F = 2048, k = 256: 1092 us with four
-// 8-bit radix passes per selection (shared-memory atomics whose bins are the few exponents a row holds, so they
-// serialise) -> 379 us with this search.
+// What bounds it: the issue slots, 57 % of them used by 9.3 K instructions per token (24 warps on an SM, 9 KB of shared memory each;
+// per instruction issued 3.1 warps wait on global loads, 1.9 on fixed latencies, 0.7 on shared memory).  us, with 32-bit keys and an
+// IEEE divide in the SiLU -> now: 16384 tokens, F = 2048, k = 256 375 -> 249, 5000 x 2000, k = 200 168 -> 107, 3000 x 512, k = 60
+// 41 -> 26 (of the first: 375 -> 345 by the keys, -> 271 by the divide, -> 249 by probes that aim past k and a better first guess:
+// 20 -> 12 probes per token).  With all keys in registers and the three lists searched together it took 583: the unrolled code
+// does not stay in the instruction cache.
 
 #include "rte_common.cuh"
 
@@ -28,131 +30,154 @@ constexpr int SEL_MAX_WARPS = 4;               // warps per CTA
 constexpr int SEL_SMEM = 224 * 1024;           // shared memory an SM has for these CTAs
 constexpr int SEL_LIST = 32;                   // keys left between the brackets when the search turns to ranking
 
-// Scores are non-negative (magnitudes times norms), so their bits order like integers; one less keeps a NaN below the
-// open upper bracket.  Neurons that are no candidates get NO_KEY, below every score.
-constexpr int NO_KEY = -0x7fffffff - 1;
-__device__ __forceinline__ int score_key(float v) { return __float_as_int(v) - 1; }
-__device__ __forceinline__ float key_score(int k) { return __int_as_float(k + 1); }
+// Scores are not negative (magnitudes times norms), so their bits order like integers, a NaN above infinity.  A key is the upper
+// half, clamped and moved by KEY_MIN so that every candidate's is a normal bf16 number; 0: no candidate.
+constexpr uint32_t KEY_MIN = 0x0080u, KEY_END = 0x7f80u;              // KEY_MIN <= key < KEY_END
+__device__ __forceinline__ uint32_t pair_keys(float a, float b) {
+  return __vminu2(__byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632), 0x7eff7effu) + 0x00800080u;
+}
+__device__ __forceinline__ float key_value(uint32_t t) { return __uint_as_float((t - KEY_MIN) << 16); }
+__device__ __forceinline__ __nv_bfloat162 as_pair(uint32_t v) { return *reinterpret_cast<__nv_bfloat162*>(&v); }
+
+// g / (1 + exp(-g)) in five instructions (an IEEE divide takes twenty, and there are three of these per neuron): within 3 ulp, like the
+// exp alone, where the scores and the bf16 z that come of it keep 8 bits; exp(-g) = infinity gives -0, as the divide does.
+__device__ __forceinline__ float silu(float g) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * -1.4426950408889634f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+  return g * r;
+}
 
 // per warp: the keys of one selection, the exact z as bf16, candidate | selected bits per four neurons, the ranking list
-__host__ __device__ constexpr size_t sel_list_offset(int F) { return ((size_t)F * 6 + (size_t)F / 4 + 15) / 16 * 16; }
+__host__ __device__ constexpr int sel_pad(int F) { return (F + 7) / 8 * 8; }
+__host__ __device__ constexpr size_t sel_list_offset(int F) { return ((size_t)sel_pad(F) * 4 + (size_t)sel_pad(F) / 4 + 15) / 16 * 16; }
 __host__ __device__ constexpr size_t sel_warp_bytes(int F) { return sel_list_offset(F) + (SEL_LIST + 4 + 8) * 4; }      // + four Guess
 static_assert(sel_warp_bytes(100) % 16 == 0 && sel_warp_bytes(2048) % 16 == 0 && (SEL_LIST + 12) % 4 == 0, "every warp's keys start on 16 bytes");
 
-struct Cut { int t, need; };     // keys >= t are taken; need >= 0: of the keys == t only the first `need` by index
-
 struct Guess { int t; float slope; };          // where the last search of this list ended, and d value / d log(count) there
 
-__device__ __forceinline__ int warp_count_ge(const int4* k4, int n4, int t, int lane) {
+// A token's inputs, for the scores of single neurons: list 0 |up_hat|, 1 |silu(gate_hat)|, 2 |up_hat * silu(gate_hat)|, 3 |z|, times wn.
+struct Token { const float* hat; const __nv_bfloat16* ug; const float* wn; int F; };
+__device__ __forceinline__ int full_score(const Token& x, int which, int i) {
+  float v;
+  if (which == 0) v = x.hat[i];
+  else if (which == 1) v = silu(x.hat[x.F + i]);
+  else if (which == 2) v = x.hat[i] * silu(x.hat[x.F + i]);
+  else v = __bfloat162float(x.ug[i]) * silu(__bfloat162float(x.ug[x.F + i]));
+  return __float_as_int(fabsf(v) * x.wn[i]);
+}
+
+__device__ __forceinline__ int warp_count_ge(const uint4* k8, int n8, uint32_t t, int lane) {
+  const __nv_bfloat162 t2 = as_pair(t | t << 16);
   int c = 0;
+  for (int i0 = 0; i0 < n8; i0 += 32 * 32) {                          // (a half counts to at most 128 per round: exact in bf16)
+    __nv_bfloat162 a = as_pair(0u), b = a;
 #pragma unroll 4
-  for (int i = lane; i < n4; i += 32) {
-    const int4 v = k4[i];
-    c += (v.x >= t) + (v.y >= t) + (v.z >= t) + (v.w >= t);
+    for (int i = i0 + lane; i < min(n8, i0 + 32 * 32); i += 32) {
+      const uint4 v = k8[i];
+      a = __hadd2(a, __hge2(as_pair(v.x), t2)); b = __hadd2(b, __hge2(as_pair(v.y), t2));
+      a = __hadd2(a, __hge2(as_pair(v.z), t2)); b = __hadd2(b, __hge2(as_pair(v.w), t2));
+    }
+    const float2 fa = __bfloat1622float2(a), fb = __bfloat1622float2(b);
+    c += int((fa.x + fa.y) + (fb.x + fb.y));
   }
   return __reduce_add_sync(0xffffffffu, c);
 }
-
-// Threshold of the k largest of the 4 * n4 keys, 0 < k < 4 * n4.  `list`: SEL_LIST + 4 ints of this warp's shared memory.
-__device__ Cut warp_cut(const int4* k4, int n4, int k, Guess& guess, int* list, int lane) {
-  int lo = NO_KEY, hi = 0x7fffffff, c_lo = 4 * n4, c_hi = 0;      // count(>= lo) > k > count(>= hi)
-  int t = guess.t;
-  float slope = guess.slope, x_prev = 0.f, l_prev = 0.f;
-  Cut cut = {0, -1};
-  for (int it = 0;; ++it) {
-    const int c = warp_count_ge(k4, n4, t, lane);
-    if (c == k) { cut.t = t; break; }
-    if (c > k) { lo = t; c_lo = c; } else { hi = t; c_hi = c; }
-    if (c_lo - c_hi <= SEL_LIST) {
-      if (lane == 0) list[SEL_LIST] = 0;
-      __syncwarp();
-      const unsigned first = (unsigned)lo, span = (unsigned)hi - first;
-#pragma unroll 4
-      for (int i = lane; i < n4; i += 32) {
-        const int4 v = k4[i];
-        if ((unsigned)v.x - first < span) list[atomicAdd(&list[SEL_LIST], 1)] = v.x;
-        if ((unsigned)v.y - first < span) list[atomicAdd(&list[SEL_LIST], 1)] = v.y;
-        if ((unsigned)v.z - first < span) list[atomicAdd(&list[SEL_LIST], 1)] = v.z;
-        if ((unsigned)v.w - first < span) list[atomicAdd(&list[SEL_LIST], 1)] = v.w;
-      }
-      __syncwarp();
-      const int m = c_lo - c_hi, r = k - c_hi;             // the r-th largest of these m keys, 1 <= r <= m
-      const int mine = lane < m ? list[lane] : NO_KEY;
-      int gt = 0, ge = 0;
-      for (int j = 0; j < m; ++j) { const int w = list[j]; gt += w > mine; ge += w >= mine; }
-      const unsigned who = __ballot_sync(0xffffffffu, lane < m && gt < r && r <= ge);
-      const int src = __ffs(who) - 1;
-      cut.t = __shfl_sync(0xffffffffu, mine, src);
-      const int taken = r - __shfl_sync(0xffffffffu, gt, src), equal = __shfl_sync(0xffffffffu, ge - gt, src);
-      cut.need = taken == equal ? -1 : taken;
-      __syncwarp();
-      break;
-    }
-    if ((unsigned)hi - (unsigned)lo <= 1u) { cut.t = lo; cut.need = k - c_hi; break; }      // more than SEL_LIST equal keys
-    // next probe: secant on log(count) from the last two probes; the middle of the bracket when that leaves it
-    const float x = key_score(t), l = __logf(c > 0 ? (float)c : 0.5f);
-    if (it > 0 && l != l_prev) { const float s = (x - x_prev) / (l_prev - l); if (s > 0.f) slope = s; }
-    x_prev = x; l_prev = l;
-    int next = score_key(x + slope * (l - __logf((float)k)));
-    if (it >= 12 || next <= lo || next >= hi) next = (int)((unsigned)lo + (((unsigned)hi - (unsigned)lo) >> 1));
-    t = next;
-  }
-  guess.t = cut.t;
-  guess.slope = slope;
-  return cut;
+// bit j: key j of the eight >= t
+__device__ __forceinline__ uint32_t ge_bits(const uint4& v, __nv_bfloat162 t2) {
+  const uint32_t x = (__hge2_mask(as_pair(v.x), t2) & 0x00020001u) | (__hge2_mask(as_pair(v.y), t2) & 0x00080004u) |
+                     (__hge2_mask(as_pair(v.z), t2) & 0x00200010u) | (__hge2_mask(as_pair(v.w), t2) & 0x00800040u);
+  return (x | x >> 16) & 0xffu;
 }
 
-// ORs the selected keys' bits (bit j = element 4 i + j of the group i = it * 32 + lane) into flags[i] at `shift`.
-__device__ void warp_flag(const int4* k4, int n4, Cut cut, uint8_t* flags, int shift, int lane) {
-  if (cut.need < 0) {
-#pragma unroll 4
-    for (int i = lane; i < n4; i += 32) {
-      const int4 v = k4[i];
-      const int m = (v.x >= cut.t) | (v.y >= cut.t) << 1 | (v.z >= cut.t) << 2 | (v.w >= cut.t) << 3;
-      flags[i] |= (uint8_t)(m << shift);
-    }
-  } else {
-    int taken = 0;                                   // equal keys with lower indices so far
-    for (int i0 = 0; i0 < n4; i0 += 32) {
-      const int i = i0 + lane;
-      int gt = 0, eq = 0;
-      if (i < n4) {
-        const int4 v = k4[i];
-        gt = (v.x > cut.t) | (v.y > cut.t) << 1 | (v.z > cut.t) << 2 | (v.w > cut.t) << 3;
-        eq = (v.x == cut.t) | (v.y == cut.t) << 1 | (v.z == cut.t) << 2 | (v.w == cut.t) << 3;
-      }
-      const int mine = __popc(eq);
-      int upto = mine;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, upto, o); if (lane >= o) upto += u; }
-      int room = cut.need - (taken + upto - mine);   // how many of this lane's equal keys are still taken
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (eq >> j & 1) { if (room > 0) gt |= 1 << j; --room; }
-      if (i < n4) flags[i] |= (uint8_t)(gt << shift);
-      taken += __shfl_sync(0xffffffffu, upto, 31);
-    }
-  }
-}
-
+// ORs the k largest of a list into `flags` (a byte per four neurons) at `shift`, 0 < k < total keys that are not 0.
 // (not inlined four times: the kernel's code then stays in the instruction cache)
-__device__ __noinline__ void warp_take(const int4* k4, int n4, int k, Guess* start, int* list, uint8_t* flags, int shift, int lane) {
+__device__ __noinline__ void warp_take(const uint4* k8, int n8, int k, int total, Guess* start, int* list, uint16_t* flags, int shift, const Token x,
+                                       int which, int lane) {
   Guess guess = *start;                              // this warp's shared memory
   __syncwarp();
-  if (k > 0) {
-    Cut cut = {NO_KEY, -1};                            // k >= F: everything
-    if (k < 4 * n4) {
-      if (guess.slope == 0.f) {                      // this warp's first token: the k / F quantile of 32 of its keys
-        const int mine = k4[lane % n4].x, want = min(31, k * 8 / n4);
-        int gt = 0;
-        for (int j = 0; j < 32; ++j) { const int w = __shfl_sync(0xffffffffu, mine, j); gt += w > mine || (w == mine && j < lane); }
-        guess.t = __shfl_sync(0xffffffffu, mine, __ffs(__ballot_sync(0xffffffffu, gt == want)) - 1);
-        guess.slope = 0.3f * fabsf(key_score(guess.t)) + 1e-30f;
-      }
-      cut = warp_cut(k4, n4, k, guess, list, lane);
-      if (lane == 0) *start = guess;
+  if (guess.slope == 0.f) {                          // this warp's first token: the k / total quantile of 32 keys, those that are candidates
+    const uint32_t mine = k8[lane % n8].x & 0xffffu;
+    const int some = __popc(__ballot_sync(0xffffffffu, mine != 0u)), want = min(max(some - 1, 0), (int)((long long)k * some / total));
+    int gt = 0;
+    for (int j = 0; j < 32; ++j) { const uint32_t w = __shfl_sync(0xffffffffu, mine, j); gt += w > mine || (w == mine && j < lane); }
+    guess.t = max((int)__shfl_sync(0xffffffffu, mine, __ffs(__ballot_sync(0xffffffffu, gt == want)) - 1), (int)KEY_MIN + 1);
+    guess.slope = 0.3f * key_value((uint32_t)guess.t) + 1e-30f;
+  }
+  uint32_t lo = KEY_MIN, hi = KEY_END, t = min(max((uint32_t)guess.t, KEY_MIN + 1), KEY_END - 1);
+  int c_lo = total, c_hi = 0;                        // count(>= lo) > k > count(>= hi), or lo == hi: exactly k at or above
+  float slope = guess.slope, x_prev = 0.f, l_prev = 0.f;
+  const float l_below = __logf(fmaxf((float)k - 8.f, 0.5f)), l_above = __logf((float)k + 8.f);
+  for (int it = 0; c_lo - c_hi > SEL_LIST && hi - lo > 1; ++it) {
+    const int c = warp_count_ge(k8, n8, t, lane);
+    if (c == k) { lo = hi = t; c_lo = c_hi = c; break; }
+    if (c > k) { lo = t; c_lo = c; } else { hi = t; c_hi = c; }
+    // next probe: secant on log(count) from the last two probes, aimed a few keys past k, so that the bracket closes around it;
+    // bisection when that does not converge
+    const float v = key_value(t), l = __logf(c > 0 ? (float)c : 0.5f);
+    if (it > 0 && l != l_prev) { const float s = (v - x_prev) / (l_prev - l); if (s > 0.f) slope = s; }
+    x_prev = v; l_prev = l;
+    const float aim = v + slope * (l - (c > k ? l_below : l_above));
+    const uint32_t next = aim > 0.f ? (__float_as_uint(aim) >> 16) + KEY_MIN : 0u;
+    t = it >= 8 ? (lo + hi) >> 1 : min(max(next, lo + 1), hi - 1);
+  }
+  if (lane == 0) { start->t = (int)lo; start->slope = slope; list[SEL_LIST] = 0; }
+  __syncwarp();
+  // what lies above is taken; what lies between is listed
+  const __nv_bfloat162 hi2 = as_pair(hi | hi << 16), lo2 = as_pair(lo | lo << 16);
+  const int n = c_lo - c_hi, need = k - c_hi;
+  const bool few = n <= SEL_LIST;
+#pragma unroll 4
+  for (int i = lane; i < n8; i += 32) {
+    const uint4 v = k8[i];
+    const uint32_t above = ge_bits(v, hi2);
+    if (lo != hi && few) {
+      for (uint32_t in = ge_bits(v, lo2) & ~above; in; in &= in - 1) list[atomicAdd(&list[SEL_LIST], 1)] = 8 * i + __ffs(in) - 1;
     }
-    warp_flag(k4, n4, cut, flags, shift, lane);
+    flags[i] |= (uint16_t)(((above & 15u) | (above & 240u) << 4) << shift);
+  }
+  if (lo == hi) { __syncwarp(); return; }
+  __syncwarp();
+  if (few) {
+    const int who = lane < n ? list[lane] : 0x7fffffff, score = lane < n ? full_score(x, which, who) : -1;
+    int above = 0;
+    for (int j = 0; j < n; ++j) {
+      const int s = __shfl_sync(0xffffffffu, score, j), i = __shfl_sync(0xffffffffu, who, j);
+      above += s > score || (s == score && i < who);
+    }
+    if (lane < n && above < need) atomicOr(reinterpret_cast<unsigned*>(flags) + (who >> 4), 1u << (8 * (who >> 2 & 3) + (who & 3) + shift));
+    return;
+  }
+  // more keys than the list holds share their upper half: the threshold among their full scores, then equal ones by index
+  auto between = [&](int i) { const uint4 v = k8[i]; return ge_bits(v, lo2) & ~ge_bits(v, hi2); };
+  int a = 0, b = 0x7fffffff;                         // count(score >= a) >= need; a becomes the largest such score
+  while (a < b) {
+    const int mid = a + (b - a) / 2 + 1;
+    int c = 0;
+    for (int i = lane; i < n8; i += 32)
+      for (uint32_t in = between(i); in; in &= in - 1) c += full_score(x, which, 8 * i + __ffs(in) - 1) >= mid;
+    if (__reduce_add_sync(0xffffffffu, c) >= need) a = mid; else b = mid - 1;
+  }
+  int c = 0;
+  for (int i = lane; i < n8; i += 32)
+    for (uint32_t in = between(i); in; in &= in - 1) c += full_score(x, which, 8 * i + __ffs(in) - 1) > a;
+  int room = need - __reduce_add_sync(0xffffffffu, c);      // how many of the equal ones, in ascending index order
+  for (int i0 = 0; i0 < n8; i0 += 32) {
+    const int i = i0 + lane;
+    uint32_t gt = 0u, eq = 0u;
+    for (uint32_t in = i < n8 ? between(i) : 0u; in; in &= in - 1) {
+      const int s = full_score(x, which, 8 * i + __ffs(in) - 1);
+      const uint32_t bit = in & (0u - in);
+      if (s > a) gt |= bit; else if (s == a) eq |= bit;
+    }
+    const int have = __popc(eq);
+    int upto = have;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xffffffffu, upto, o); if (lane >= o) upto += u; }
+    int left = room - (upto - have);
+    for (; eq && left > 0; eq &= eq - 1, --left) gt |= eq & (0u - eq);
+    if (i < n8) flags[i] |= (uint16_t)(((gt & 15u) | (gt & 240u) << 4) << shift);
+    room -= __shfl_sync(0xffffffffu, upto, 31);
   }
   __syncwarp();
 }
@@ -179,24 +204,28 @@ __device__ __forceinline__ void prefetch_l2(const void* p, int bytes, int lane) 
 
 // hats f32 [rows, 2F] = (up_hat | gate_hat); ug bf16 [rows, 2F] = exact (up | gate); wn f32 [F], not negative
 // z_masked bf16 [rows, F]; selected uint8 [rows, F] (1 = selected); cand_count int32 [rows] (optional)
-__global__ void __launch_bounds__(SEL_MAX_WARPS * 32, 4)
+__global__ void __launch_bounds__(SEL_MAX_WARPS * 32, 6)
 svd_select_kernel(const float* __restrict__ hats, const __nv_bfloat16* __restrict__ ug, const float* __restrict__ wn,
                   __nv_bfloat16* __restrict__ z_masked, uint8_t* __restrict__ selected, int32_t* __restrict__ cand_count,
                   int rows, int F, int up_m, int gate_m, int product_m, int top_k) {
   rte::after_previous_grid();
   extern __shared__ __align__(16) uint8_t sm_raw[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, n4 = F / 4;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, n4 = F / 4, n8 = sel_pad(F) / 8;
   uint8_t* base = sm_raw + warp * sel_warp_bytes(F);
-  int4* k4 = reinterpret_cast<int4*>(base);
-  uint2* z4 = reinterpret_cast<uint2*>(k4 + n4);
-  uint8_t* flags = reinterpret_cast<uint8_t*>(z4 + n4);
+  uint2* key = reinterpret_cast<uint2*>(base);                       // four keys each
+  uint2* z4 = key + 2 * n8;
+  uint8_t* flags = reinterpret_cast<uint8_t*>(z4 + 2 * n8);
   int* list = reinterpret_cast<int*>(base + sel_list_offset(F));
+  const uint4* k8 = reinterpret_cast<const uint4*>(key);
+  uint16_t* flags16 = reinterpret_cast<uint16_t*>(flags);
   const float4* wn4 = reinterpret_cast<const float4*>(wn);
   Guess* guess = reinterpret_cast<Guess*>(list + SEL_LIST + 4);
   if (lane < 4) guess[lane] = Guess{0, 0.f};
+  if (lane == 0 && n4 < 2 * n8) key[n4] = make_uint2(0u, 0u);        // (the padding of an odd number of groups: no candidates)
   __syncwarp();
   for (int row = blockIdx.x * warps + warp; row < rows; row += gridDim.x * warps) {
-    const float4* uh = reinterpret_cast<const float4*>(hats + (size_t)row * 2 * F);
+    const Token tok = {hats + (size_t)row * 2 * F, ug + (size_t)row * 2 * F, wn, F};
+    const float4* uh = reinterpret_cast<const float4*>(tok.hat);
     const float4* gh = uh + n4;
     const int next = row + gridDim.x * warps;          // the next token's inputs start on their way to L2
     if (next < rows) {
@@ -204,39 +233,50 @@ svd_select_kernel(const float* __restrict__ hats, const __nv_bfloat16* __restric
       prefetch_l2(ug + (size_t)next * 2 * F, 4 * F, lane);
     }
     // --- three candidate lists
+    auto take = [&](int k, int which) {
+      __syncwarp();
+      if (k >= F) { for (int i = lane; i < n8; i += 32) flags16[i] |= 0x0f0fu; }
+      else if (k > 0) warp_take(k8, n8, k, F, guess + which, list, flags16, 0, tok, which, lane);
+      __syncwarp();
+    };
+    for (int i = lane; i < n8; i += 32) flags16[i] = 0;
     for_groups<4>(uh, uh, wn4, n4, lane, [&](int i, float4 u, float4, float4 w) {
-      k4[i] = make_int4(score_key(fabsf(u.x) * w.x), score_key(fabsf(u.y) * w.y), score_key(fabsf(u.z) * w.z), score_key(fabsf(u.w) * w.w));
-      flags[i] = 0;
+      key[i] = make_uint2(pair_keys(fabsf(u.x) * w.x, fabsf(u.y) * w.y), pair_keys(fabsf(u.z) * w.z, fabsf(u.w) * w.w));
     });
-    warp_take(k4, n4, up_m, guess + 0, list, flags, 0, lane);
+    take(up_m, 0);
     if (gate_m > 0) {
       for_groups<4>(gh, gh, wn4, n4, lane, [&](int i, float4 g, float4, float4 w) {
-        k4[i] = make_int4(score_key(fabsf(rte::silu_f(g.x)) * w.x), score_key(fabsf(rte::silu_f(g.y)) * w.y),
-                          score_key(fabsf(rte::silu_f(g.z)) * w.z), score_key(fabsf(rte::silu_f(g.w)) * w.w));
+        key[i] = make_uint2(pair_keys(fabsf(silu(g.x)) * w.x, fabsf(silu(g.y)) * w.y),
+                            pair_keys(fabsf(silu(g.z)) * w.z, fabsf(silu(g.w)) * w.w));
       });
-      warp_take(k4, n4, gate_m, guess + 1, list, flags, 0, lane);
+      take(gate_m, 1);
     }
     if (product_m > 0) {
       for_groups<2>(uh, gh, wn4, n4, lane, [&](int i, float4 u, float4 g, float4 w) {
-        k4[i] = make_int4(score_key(fabsf(u.x * rte::silu_f(g.x)) * w.x), score_key(fabsf(u.y * rte::silu_f(g.y)) * w.y),
-                          score_key(fabsf(u.z * rte::silu_f(g.z)) * w.z), score_key(fabsf(u.w * rte::silu_f(g.w)) * w.w));
+        key[i] = make_uint2(pair_keys(fabsf(u.x * silu(g.x)) * w.x, fabsf(u.y * silu(g.y)) * w.y),
+                            pair_keys(fabsf(u.z * silu(g.z)) * w.z, fabsf(u.w * silu(g.w)) * w.w));
       });
-      warp_take(k4, n4, product_m, guess + 2, list, flags, 0, lane);
+      take(product_m, 2);
     }
     // --- exact re-rank over the candidates
-    const uint2* up = reinterpret_cast<const uint2*>(ug + (size_t)row * 2 * F);
+    const uint2* up = reinterpret_cast<const uint2*>(tok.ug);
     int n_cand = 0;
     for_groups<2>(up, up + n4, wn4, n4, lane, [&](int i, uint2 u, uint2 g, float4 w) {
       const float2 u0 = rte::unpack_bf16x2(u.x), u1 = rte::unpack_bf16x2(u.y), g0 = rte::unpack_bf16x2(g.x), g1 = rte::unpack_bf16x2(g.y);
-      const int m = flags[i];
-      const float z0 = u0.x * rte::silu_f(g0.x), z1 = u0.y * rte::silu_f(g0.y), z2 = u1.x * rte::silu_f(g1.x), z3 = u1.y * rte::silu_f(g1.y);
+      const uint32_t m = flags[i];
+      const float z0 = u0.x * silu(g0.x), z1 = u0.y * silu(g0.y), z2 = u1.x * silu(g1.x), z3 = u1.y * silu(g1.y);
       n_cand += __popc(m);
-      k4[i] = make_int4(m & 1 ? score_key(fabsf(z0) * w.x) : NO_KEY, m & 2 ? score_key(fabsf(z1) * w.y) : NO_KEY,
-                        m & 4 ? score_key(fabsf(z2) * w.z) : NO_KEY, m & 8 ? score_key(fabsf(z3) * w.w) : NO_KEY);
+      key[i] = make_uint2(pair_keys(fabsf(z0) * w.x, fabsf(z1) * w.y) & ((m & 1u) * 0xffffu | (m & 2u) * 0x7fff8000u),
+                          pair_keys(fabsf(z2) * w.z, fabsf(z3) * w.w) & ((m >> 2 & 1u) * 0xffffu | (m >> 2 & 2u) * 0x7fff8000u));
       z4[i] = make_uint2(rte::pack_bf16x2(z0, z1), rte::pack_bf16x2(z2, z3));
     });
-    warp_take(k4, n4, top_k, guess + 3, list, flags, 4, lane);
     n_cand = __reduce_add_sync(0xffffffffu, n_cand);
+    __syncwarp();
+    if (lane == 0 && guess[3].slope == 0.f) guess[3] = guess[2];       // (a warp's first token: the products' scores estimate these)
+    __syncwarp();
+    if (top_k < n_cand) warp_take(k8, n8, top_k, n_cand, guess + 3, list, flags16, 4, tok, 3, lane);
+    else for (int i = lane; i < n8; i += 32) flags16[i] |= (uint16_t)(flags16[i] << 4);
+    __syncwarp();
     if (cand_count && lane == 0) cand_count[row] = n_cand;
     uint2* zo = reinterpret_cast<uint2*>(z_masked + (size_t)row * F);
     uint32_t* so = reinterpret_cast<uint32_t*>(selected + (size_t)row * F);

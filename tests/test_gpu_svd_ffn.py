@@ -65,6 +65,25 @@ def test_threshold_search_selects_the_k_largest_in_every_row(rows, F_, k):
     assert torch.equal(z.cpu() != 0, want & (ug[:, :F_] != 0))
 
 
+@pytest.mark.parametrize("rows,F_,k", [(40, 2048, 256), (9, 132, 40), (600, 1024, 3)])
+def test_scores_that_share_their_upper_bits(rows, F_, k):
+    """More scores than the ranking list holds between two neighbouring keys, different below, some equal; an infinite score and
+    one that is not a number rank first, in that order from the top: NaN, infinity."""
+    ops = CudaOps(DEV)
+    g = torch.Generator().manual_seed(rows + F_)
+    uh = 1.0 + torch.randint(0, 500, (rows, F_), generator=g) * 2.0 ** -20
+    uh[1::2, : F_ // 2] *= 4.0
+    uh[0, 7], uh[0, 3] = float("nan"), float("inf")
+    hats = torch.cat([uh, torch.zeros(rows, F_)], dim=1)
+    ug = torch.cat([torch.ones(rows, F_), torch.zeros(rows, F_)], dim=1).bfloat16()
+    z, sel = torch.empty(rows, F_, dtype=torch.bfloat16, device=DEV), torch.empty(rows, F_, dtype=torch.uint8, device=DEV)
+    ops.svd_ffn_select(hats.to(DEV), ug.to(DEV), torch.ones(F_, device=DEV), z, sel, None, up_m=k, gate_m=0, product_m=0, top_k=k)
+    torch.cuda.synchronize()
+    order = uh.clone()
+    order[0, 7], order[0, 3] = 1e30, 1e29
+    assert torch.equal(sel.cpu().bool(), O.topk_membership(order, k))
+
+
 @pytest.mark.parametrize("rows,F_", [(37, 2048), (5, 100)])            # eight neurons per thread | one
 def test_swiglu_backward_of_the_selected_neurons(rows, F_):
     ops = CudaOps(DEV)
