@@ -707,6 +707,30 @@ def test_shortlist_build_bit_exact(ops, B, S, V, C, TC, HN, RN, K):
     assert torch.equal(out[:, 0].cpu().long(), targets.view(-1))
 
 
+@pytest.mark.parametrize("V,C,TC,HN,RN,K", [(20, 3, 1, 45, 40, 20), (33, 33, 2, 0, 33, 1), (64, 2, 2, 7, 64, 40), (1500, 64, 1, 40, 0, 1300),
+                                            (2047, 5, 1, 3, 70, 700)])
+def test_shortlist_runs_at_their_edges(ops, V, C, TC, HN, RN, K):
+    """Every target (each start and wrap of its run), runs longer than the vocabulary, repeated random negatives; and the same list
+    without the duplicate count, where the walk ends at the K-th id."""
+    g = torch.Generator().manual_seed(V)
+    oc = O.OutputCfg(mode="shortlist", num_clusters=C, shortlist_top_clusters=TC, shortlist_max_tokens=K,
+                     hard_negatives=HN, random_negatives=RN)
+    targets = torch.arange(V).view(1, V)
+    top = torch.stack([torch.randperm(C, generator=g)[:TC] for _ in range(V)]).view(1, V, TC)
+    rnd = torch.randint(0, max(1, V // 2), (1, V, RN), generator=g)
+    cands = O.shortlist_candidates(targets, top, rnd, V, oc)
+    want = O.dedupe_preserve_first(cands, K)[0].to(torch.int32)
+    dups = torch.tensor([cands.shape[-1] - len(set(r.tolist())) for r in cands[0]], dtype=torch.int32)
+    out, short = (torch.full((V, K), -1, dtype=torch.int32, device=DEV) for _ in range(2))
+    dc = torch.zeros(V, dtype=torch.int32, device=DEV)
+    rnd_dev = rnd[0].to(torch.int32).to(DEV) if RN else torch.zeros(1, dtype=torch.int32, device=DEV)
+    for ids, count in ((out, dc), (short, None)):
+        ops.shortlist_build(targets.to(DEV), top[0].to(torch.int32).to(DEV), rnd_dev, ids, count, V=V, C=C, TC=TC, HN=HN, RN=RN, K=K)
+    ops.check_status()
+    assert torch.equal(out.cpu(), want) and torch.equal(short.cpu(), want)
+    assert torch.equal(dc.cpu(), dups)
+
+
 @pytest.mark.parametrize("rows,S,d,V,K", [(21, 7, 64, 96, 16), (256, 64, 512, 2048, 128)])
 def test_shortlist_ce_matches_reference_math(ops, rows, S, d, V, K):
     g = torch.Generator().manual_seed(rows)
