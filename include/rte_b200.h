@@ -217,6 +217,18 @@ int rte_colsum_partials(const float* partial, int32_t n_rows, int32_t d, float* 
 int rte_colsum_partials3(const float* const* partials, float* const* outs, const int32_t* accumulate, int32_t count,
                          int32_t n_rows, int32_t d, rte_stream_t stream);
 
+/* Every sum of partials of the recurrent core's backward pass in ONE launch.  partials: [T][2][3][pr][d], pass by pass, norm 2
+ * then norm 1, the weight's, gamma's and beta's partial rows (n_rows <= pr of them written; 16-byte aligned); dw[i] gets
+ * the sum over the passes, dgamma[i] / dbeta[i] ([T][d]) each pass's own.  part_mlp / part_attn / part_alpha: [T][P]. */
+typedef struct {
+  const float* partials;
+  float* dw[2]; float* dgamma[2]; float* dbeta[2];
+  const float* part_mlp; const float* part_attn; const float* part_alpha;
+  float* d_mlp_scale; float* d_attn_scale; float* d_alpha;
+} rte_core_sums;
+int rte_core_gradient_sums(const rte_core_sums* sums, int32_t T, int32_t pr, int32_t n_rows, int32_t d, int32_t P,
+                           rte_stream_t stream);
+
 /* --------------------- causal attention with RoPE (layers.py:36-50,64-75; reference.py:20-28,40-41)
  * qkv bf16 [B*S, 3*d] with columns (q | k | v), head-major inside each; adjacent-pair rotary
  * embedding (base 10000, positions 0..S-1) applied to q and k inside the kernel; softmax scale

@@ -59,6 +59,11 @@ class RouterGrads(C.Structure):
     _fields_ = [(n, c_vp) for n in ("r_w0", "r_b0", "r_w2", "r_b2", "d_w0", "d_b0", "d_w2", "d_b2")]
 
 
+class CoreSums(C.Structure):
+    _fields_ = [("partials", c_vp), ("dw", c_vp * 2), ("dgamma", c_vp * 2), ("dbeta", c_vp * 2), ("part_mlp", c_vp), ("part_attn", c_vp),
+                ("part_alpha", c_vp), ("d_mlp_scale", c_vp), ("d_attn_scale", c_vp), ("d_alpha", c_vp)]
+
+
 class PhiParams(C.Structure):
     _fields_ = [(n, c_vp) for n in ("gain", "v", "u", "bias", "scale", "wt")] + [("n_keys", C.c_int32)]
 
@@ -122,6 +127,7 @@ PROTOTYPES = {
     "rte_residual_rmsnorm_fwd_splits": (C.c_int, [c_vp, c_vp, c_i32, c_i64, c_vp, c_vp, c_vp, c_vp, c_i32, c_vp, c_vp, c_vp, c_vp,
                                                   c_vp, c_vp, c_vp, c_vp, c_vp, c_i32, c_i32, C.c_float, c_vp]),
     "rte_colsum_partials3": (C.c_int, [c_vp, c_vp, c_vp, c_i32, c_i32, c_i32, c_vp]),
+    "rte_core_gradient_sums": (C.c_int, [C.POINTER(CoreSums), c_i32, c_i32, c_i32, c_i32, c_i32, c_vp]),
     "rte_colsum_partials": (C.c_int, [c_vp, c_i32, c_i32, c_vp, c_i32, c_vp]),
     "rte_rope_table": (C.c_int, [c_vp, c_i32, c_i32, c_vp]),
     "rte_rope_apply": (C.c_int, [c_vp, c_vp, c_vp, c_vp, c_i64, c_i32, c_i32, c_i32, c_i32, c_vp]),

@@ -201,10 +201,12 @@ class AuditReplay:
         self.d16_mlp, self.d16_attn = per_pass("d16_mlp", d), per_pass("d16_attn", d)
         self.dug16, self.dqkv16 = per_pass("dug16", 2 * f), per_pass("dqkv16", 3 * d)
         PR = 128
-        self.partials = [[(e(PR, d), e(PR, d), e(PR, d)) for _ in range(2)] for _ in range(T)]
+        self.partials_flat = e(T, 2, 3, PR, d)
+        self.partials = [[tuple(self.partials_flat[t, k]) for k in range(2)] for t in range(T)]
         self.coda_tmps = [_Temps(Ma, cfg, dev) for _ in range(cfg.n_coda)]
         # bf16 gradient between the coda blocks: one buffer each, the deferred weight gradients still read them
         self.coda_dx16 = [self.tmp.dx16] + [e(Ma, d, dtype=bf) for _ in range(cfg.n_coda)]
+        self._scalars_summed = False
         self.P = 296               # partial sums per pass of the scalar parameters' gradients (one per CTA of their launch)
         self.part_alpha, self.part_attn, self.part_mlp = e(T * self.P), e(T * self.P), e(T * self.P)
         # The replay runs on its own stream beside the hot pass, so the gradients it contributes to parameters the
@@ -641,6 +643,11 @@ class AuditReplay:
         if not defer and eng._param_stream is not None:
             torch.cuda.current_stream(eng.device).wait_stream(eng._param_stream)
         self._defer_param_grads(defer)
+        # Beside a hot pass the sums of partials of all passes are one launch after the loop: each launch of the weight-gradient
+        # stream waits for a place there (steps of 8192 x 512 with 4 passes 1415 -> 1404 us, of 16384 x 512 with 8 passes
+        # 2719 -> 2674).  Alone they fit into the chain's gaps pass by pass (0.84 ms step: + 6 us if summed at the end).
+        one_sum = defer and not self.direct and hasattr(o, "core_gradient_sums")
+        deferred_sums, n_part = ({"sums": False}, 0) if one_sum else ({}, 0)
         dnext, dthis = dh_last, (self.dcur if dh_last is not self.dcur else self.dalt)
         for t in reversed(range(T)):
             rid, first = self.rid[t], t == T - 1
@@ -663,10 +670,10 @@ class AuditReplay:
                 if not fused:
                     o.gemm_wgrad(self.n2[t], dug16, g["core.mlp.wug"][bk], M=d, N=2 * f, K=Ma, accumulate=acc, ws=self.ws)
             # (one bank: the norm backward sums the product's split-K partials itself, in split order)
-            o.rmsnorm_bwd(self.u[t], p["core.norm2.weight"], self.rstd2[t], self.ws_chain if sp2[0] > 1 else self.dn_f32,
-                          du, du, None, g["core.norm2.weight"], pw2, film_gamma=p["core.pass_gamma2"][t],
+            n_part = o.rmsnorm_bwd(self.u[t], p["core.norm2.weight"], self.rstd2[t],
+                          self.ws_chain if sp2[0] > 1 else self.dn_f32, du, du, None, g["core.norm2.weight"], pw2, film_gamma=p["core.pass_gamma2"][t],
                           dgamma_out=g["core.pass_gamma2"][t], dbeta_out=g["core.pass_beta2"][t],
-                          partial_g=pg2, partial_b=pb2, accumulate_dw=acc, dy_splits=sp2)
+                          partial_g=pg2, partial_b=pb2, accumulate_dw=acc, dy_splits=sp2, **deferred_sums)
             # u = ht + s_attn * attn
             o.scaled_residual_bwd(du, self.attn_acc[t], p["core.pass_attn_scale"][t:t + 1], None, dht, d16a, None, None,
                                   self.part_attn[t * P:(t + 1) * P], n, S * d)
@@ -683,7 +690,7 @@ class AuditReplay:
             o.rmsnorm_bwd(self.ht[t], p["core.norm1.weight"], self.rstd1[t], self.ws_chain if sp1[0] > 1 else self.dn_f32,
                           dht, dht, None, g["core.norm1.weight"], pw1, film_gamma=p["core.pass_gamma1"][t],
                           dgamma_out=g["core.pass_gamma1"][t], dbeta_out=g["core.pass_beta1"][t],
-                          partial_g=pg1, partial_b=pb1, accumulate_dw=acc, dy_splits=sp1)
+                          partial_g=pg1, partial_b=pb1, accumulate_dw=acc, dy_splits=sp1, **deferred_sums)
             # ht = h_in + alpha * h0
             # (samples that were frozen in this pass hand their gradient `dnext` straight through: same launch)
             o.scaled_residual_bwd(dht, self.h0a, alpha, None, dthis, None, self.dh0_acc, None,
@@ -691,6 +698,12 @@ class AuditReplay:
                                   frozen_src=dnext)
             dnext, dthis = dthis, (self.dalt if dthis is self.dcur else self.dcur)
         self.dh_first = dnext
+        self._scalars_summed = one_sum
+        if one_sum:
+            o.core_gradient_sums(self.partials_flat, n_part, *((g[f"core.{k}2{w}"], g[f"core.{k}1{w}"])
+                                                               for k, w in (("norm", ".weight"), ("pass_gamma", ""), ("pass_beta", ""))),
+                                 self.part_mlp, self.part_attn, self.part_alpha, g["core.pass_mlp_scale"],
+                                 g["core.pass_attn_scale"], g["core.alpha_inj"])
         if fused:
             st, K = self._stacked, T * Ma
             o.gemm_wgrad(st["zm"], st["d16_mlp"], g["core.mlp.wd"][0], M=f, N=d, K=K, ws=self.ws)
@@ -804,7 +817,9 @@ class AuditReplay:
 
     def _scalar_grads(self) -> None:
         """Scalar parameters of the core: per-CTA partial sums -> gradients, in fixed order (slots of part_* beyond the
-        CTAs actually launched stay at their initial zero)."""
+        CTAs actually launched stay at their initial zero).  Nothing to do where `backward_core` has summed them."""
+        if self._scalars_summed:
+            return
         eng = self.eng
         o, g, T, P = eng.ops, eng.grads, self.T, self.P
         o.segment_sum(self.part_mlp, g["core.pass_mlp_scale"], T, P)

@@ -246,9 +246,11 @@ class CudaOps:
 
     def rmsnorm_bwd(self, x, w, rstd, dy, dres, dx_f32, dx_bf16, dw_out, partial, *, film_gamma=None,
                     dgamma_out=None, dbeta_out=None, partial_g=None, partial_b=None, accumulate_dw: bool = False,
-                    accumulate_film: bool = False, rows: int | None = None, dy_splits: tuple[int, int] = (1, 0)) -> None:
+                    accumulate_film: bool = False, rows: int | None = None, dy_splits: tuple[int, int] = (1, 0),
+                    sums: bool = True) -> int:
         """dx = rmsnorm_backward(dy) + dres; dw_out (+)= column sums (two-stage, deterministic).
-        `dy_splits` = (count, stride): `dy` (fp32) holds split-K partials of the gradient, summed in the launch."""
+        `dy_splits` = (count, stride): `dy` (fp32) holds split-K partials of the gradient, summed in the launch.
+        `sums=False` leaves the second stage to the caller (`core_gradient_sums`).  Returns the partial rows written."""
         d = x.shape[-1]
         rows = rows if rows is not None else x.numel() // d
         n_part = C.c_int32(0)
@@ -259,8 +261,8 @@ class CudaOps:
                    dy_splits[0], dy_splits[1],
                    _ptr(dres), _ptr(dx_f32), _ptr(dx_bf16), _ptr(partial if dw_out is not None else None),
                    _ptr(partial_g), _ptr(partial_b), rows, d, max_partials, C.byref(n_part), self.stream)
-        if dw_out is None and dgamma_out is None:
-            return
+        if not sums or (dw_out is None and dgamma_out is None):
+            return n_part.value
         jobs = []
         if dw_out is not None:
             jobs.append((partial, dw_out, accumulate_dw))
@@ -275,6 +277,19 @@ class CudaOps:
                 outs = (C.c_void_p * k)(*[j[1].data_ptr() for j in jobs])
                 acc = (C.c_int32 * k)(*[int(j[2]) for j in jobs])
                 self._call("rte_colsum_partials3", parts, outs, acc, k, n_part.value, d, self.stream)
+        return n_part.value
+
+    def core_gradient_sums(self, partials, n_rows: int, dw, dgamma, dbeta, part_mlp, part_attn, part_alpha, d_mlp_scale,
+                           d_attn_scale, d_alpha) -> None:
+        """All sums of partials of the core's backward pass in one launch: `partials` [T, 2, 3, rows, d] (norm 2, norm 1;
+        weight, gamma, beta), `dw` / `dgamma` / `dbeta` their outputs as (norm 2, norm 1) pairs, `part_*` [T * P]."""
+        _require_cuda(partials)
+        T, _, _, pr, d = partials.shape
+        pair = lambda ts: (C.c_void_p * 2)(*[t.data_ptr() for t in ts])      # noqa: E731
+        job = A.CoreSums(_ptr(partials), pair(dw), pair(dgamma), pair(dbeta), _ptr(part_mlp), _ptr(part_attn), _ptr(part_alpha),
+                         _ptr(d_mlp_scale), _ptr(d_attn_scale), _ptr(d_alpha))
+        with self._deferred():
+            self._call("rte_core_gradient_sums", C.byref(job), T, pr, n_rows, d, part_mlp.numel() // T, self.stream)
 
     def ce_fwd_bwd(self, logits, targets, row_weight, S: int, loss_tok, dlogits) -> None:
         rows, V = logits.shape

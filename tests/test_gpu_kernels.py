@@ -1,6 +1,7 @@
 """Per-kernel parity on a B200: every C-ABI entry point against the CPU oracle (or, for the plain
 GEMM, an fp32 matmul of the same bf16 inputs).  Tolerances: bf16 kernels max-abs 2e-2 relative to the
 output scale, fp32 kernels 1e-4, indices bit-exact."""
+import ctypes as C
 import math
 
 import numpy as np
@@ -680,6 +681,33 @@ def test_swiglu_standalone_pass_matches_fused_epilogue_math(ops):
     assert (z.cpu().float() - z_ref.detach()).abs().max() <= 1e-2 * z_ref.abs().max()
     ref = torch.cat([up.grad, gate.grad], dim=1)
     assert (dug.cpu().float() - ref).abs().max() <= 1e-2 * ref.abs().max()
+
+
+@pytest.mark.parametrize("T,d,n_rows,P", [(1, 4, 1, 3), (3, 36, 33, 296), (2, 512, 31, 130), (8, 512, 128, 296), (5, 1028, 64, 1)])
+def test_core_gradient_sums(ops, T, d, n_rows, P):
+    """One launch against the launch for each norm and pass and for each scalar parameter: the same sums in the same order, so the
+    same bits; rows beyond the written ones are not read."""
+    g = torch.Generator().manual_seed(d)
+    pr = 128
+    part = torch.randn(T, 2, 3, pr, d, generator=g)
+    part[:, :, :, n_rows:] = float("nan")
+    part, scal = part.to(DEV), [torch.randn(T * P, generator=g).to(DEV) for _ in range(3)]
+    new = lambda *s: torch.full(s, 7.0, device=DEV)      # noqa: E731
+
+    def outputs():
+        return [new(2, d), new(2, T, d), new(2, T, d), new(T), new(T), new(1)]
+
+    want, got = outputs(), outputs()
+    for t in reversed(range(T)):
+        for k in range(2):
+            outs = [want[0][k], want[1][k, t], want[2][k, t]]
+            ops._call("rte_colsum_partials3", (C.c_void_p * 3)(*[x.data_ptr() for x in part[t, k]]),
+                      (C.c_void_p * 3)(*[x.data_ptr() for x in outs]), (C.c_int32 * 3)(int(t < T - 1), 0, 0), 3, n_rows, d, ops.stream)
+    for src, dst, n, length in ((scal[0], want[3], T, P), (scal[1], want[4], T, P), (scal[2], want[5], 1, T * P)):
+        ops.segment_sum(src, dst, n, length)
+    ops.core_gradient_sums(part, n_rows, *[list(x) for x in got[:3]], *scal, *got[3:])
+    for a, b in zip(want, got):
+        assert torch.isfinite(b).all() and torch.equal(a, b)
 
 
 # ------------------------------------------------------------------ vocabulary shortlist
