@@ -355,6 +355,14 @@ int rte_macro_phi_fwd(const float* h0, const rte_phi_params* p, const int32_t* r
                       const int32_t* stride_id, float s_cfg, float* out, float* rstd, float* pooled,
                       float* act, int32_t B, int32_t S, int32_t d, int32_t m, int32_t K_strides,
                       float eps, rte_stream_t stream);
+/* The same forward in two calls: rte_macro_phi_rows makes rstd and the pooled rows, which do not depend on the route (it may run
+ * beside the router; RTE_ERR_UNSUPPORTED for d % 4 != 0, d > 2048 or h0 off 16 bytes), and ..._from_rows the rest. */
+int rte_macro_phi_rows(const float* h0, float* rstd, float* pooled, int32_t B, int32_t S, int32_t d, int32_t m, float eps,
+                       rte_stream_t stream);
+int rte_macro_phi_fwd_from_rows(const float* h0, const rte_phi_params* p, const int32_t* recipe_id,
+                                const int32_t* stride_id, float s_cfg, float* out, float* rstd, float* pooled,
+                                float* act, int32_t B, int32_t S, int32_t d, int32_t m, int32_t K_strides,
+                                float eps, rte_stream_t stream);
 /* dh0 f32 [B*S,d] (overwritten), parameter grads f32 (zeroed then accumulated, full [R,K,...] tensors).
  * scratch f32 >= B*S*d + B*S*m + 3*B*d + B*m*d + B*3*d*m.                                           */
 typedef struct rte_phi_grads { float *gain, *v, *u, *bias; } rte_phi_grads;

@@ -29,6 +29,10 @@ __device__ __forceinline__ size_t key_of(const int32_t* rid, const int32_t* sid,
 // A cluster of PREP_CTAS CTAs per sample: warps take tokens, a token stays in registers between its norm and the column
 // sums (one pass over h0), the CTAs add their column sums and products through distributed shared memory in rank order.
 // One CTA per sample left most SMs without work and read h0 twice: 32 x 256 x 1024 136 -> 29 us in the step (34 MB).
+// PART 1 is what does not depend on the route (the pass over h0), which the caller may run beside the router; PART 2 is the product
+// with the slice of v that the route picks, from the pooled rows in memory: the same sums in the same order as PART 0, both.
+// Between the router and the operator's first product, transposed parameters included, 32 x 256 x 1024: 39 -> 6 us; 128 x 64 x 512
+// in an audited step 26 -> 6.
 constexpr int PREP_CTAS = 8;
 
 __device__ __forceinline__ float dsmem_read(const float* p, int rank) {
@@ -43,7 +47,7 @@ __device__ __forceinline__ void cluster_sync() {
 }
 
 // NV float4 per lane hold a token (d <= 128 * NV, d % 4 == 0)
-template <int NV>
+template <int NV, int PART>
 __global__ void __cluster_dims__(PREP_CTAS, 1, 1) __launch_bounds__(NTHR)
 phi_prep_kernel(const float* __restrict__ h0, const float* __restrict__ v, const int32_t* __restrict__ rid,
                 const int32_t* __restrict__ sid, float* __restrict__ rstd, float* __restrict__ pooled,
@@ -51,48 +55,57 @@ phi_prep_kernel(const float* __restrict__ h0, const float* __restrict__ v, const
   rte::after_previous_grid();
   extern __shared__ __align__(16) float sm[];            // warp sums [NTHR / 32][d] -> (row 0) this CTA's column sums; then pooled [d], products [m]
   constexpr int WARPS = NTHR / 32;
-  float* ps = sm + (size_t)WARPS * D.d;
+  float* ps = PART == 2 ? sm : sm + (size_t)WARPS * D.d;
   float* pj = ps + D.d;
   const int b = blockIdx.x / PREP_CTAS, rank = blockIdx.x % PREP_CTAS, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d4 = D.d >> 2;
-  const float4* hb = reinterpret_cast<const float4*>(h0 + (size_t)b * D.S * D.d);
-  float4 acc[NV];
+  // this CTA's slice of the columns
+  const int per = rte::ceil_div(D.d, PREP_CTAS), c0 = rank * per, n = min(D.d, c0 + per) - c0;
+  if constexpr (PART != 2) {
+    const float4* hb = reinterpret_cast<const float4*>(h0 + (size_t)b * D.S * D.d);
+    float4 acc[NV];
 #pragma unroll
-  for (int i = 0; i < NV; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int s = rank * WARPS + warp; s < D.S; s += PREP_CTAS * WARPS) {
-    float4 x[NV];
-    float ss = 0.f;
+    for (int i = 0; i < NV; ++i) acc[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int s = rank * WARPS + warp; s < D.S; s += PREP_CTAS * WARPS) {
+      float4 x[NV];
+      float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int c = lane + 32 * i;
-      x[i] = c < d4 ? hb[(size_t)s * d4 + c] : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < NV; ++i) {
+        const int c = lane + 32 * i;
+        x[i] = c < d4 ? hb[(size_t)s * d4 + c] : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int i = 0; i < NV; ++i) ss += x[i].x * x[i].x + x[i].y * x[i].y + x[i].z * x[i].z + x[i].w * x[i].w;
+      const float r = rsqrtf(rte::warp_sum(ss) / (float)D.d + eps);
+      if (lane == 0) rstd[(size_t)b * D.S + s] = r;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) { acc[i].x += x[i].x * r; acc[i].y += x[i].y * r; acc[i].z += x[i].z * r; acc[i].w += x[i].w * r; }
     }
 #pragma unroll
-    for (int i = 0; i < NV; ++i) ss += x[i].x * x[i].x + x[i].y * x[i].y + x[i].z * x[i].z + x[i].w * x[i].w;
-    const float r = rsqrtf(rte::warp_sum(ss) / (float)D.d + eps);
-    if (lane == 0) rstd[(size_t)b * D.S + s] = r;
+    for (int i = 0; i < NV; ++i)
+      if (lane + 32 * i < d4) reinterpret_cast<float4*>(sm + (size_t)warp * D.d)[lane + 32 * i] = acc[i];
+    __syncthreads();
+    for (int c = threadIdx.x; c < D.d; c += NTHR) {
+      float t = sm[c];
 #pragma unroll
-    for (int i = 0; i < NV; ++i) { acc[i].x += x[i].x * r; acc[i].y += x[i].y * r; acc[i].z += x[i].z * r; acc[i].w += x[i].w * r; }
-  }
+      for (int w = 1; w < WARPS; ++w) t += sm[(size_t)w * D.d + c];
+      sm[c] = t;
+    }
+    cluster_sync();
+    // its sum over the cluster
+    for (int c = threadIdx.x; c < n; c += NTHR) {
+      float t = 0.f;
 #pragma unroll
-  for (int i = 0; i < NV; ++i)
-    if (lane + 32 * i < d4) reinterpret_cast<float4*>(sm + (size_t)warp * D.d)[lane + 32 * i] = acc[i];
-  __syncthreads();
-  for (int c = threadIdx.x; c < D.d; c += NTHR) {
-    float t = sm[c];
-#pragma unroll
-    for (int w = 1; w < WARPS; ++w) t += sm[(size_t)w * D.d + c];
-    sm[c] = t;
-  }
-  cluster_sync();
-  // this CTA's slice of the columns: sum over the cluster, then its part of the product
-  const int per = rte::ceil_div(D.d, PREP_CTAS), c0 = rank * per, n = min(D.d, c0 + per) - c0;
-  for (int c = threadIdx.x; c < n; c += NTHR) {
-    float t = 0.f;
-#pragma unroll
-    for (int k = 0; k < PREP_CTAS; ++k) t += dsmem_read(sm + c0 + c, k);
-    t /= (float)D.S;
-    ps[c] = t;
-    pooled[(size_t)b * D.d + c0 + c] = t;
+      for (int k = 0; k < PREP_CTAS; ++k) t += dsmem_read(sm + c0 + c, k);
+      t /= (float)D.S;
+      ps[c] = t;
+      pooled[(size_t)b * D.d + c0 + c] = t;
+    }
+    if constexpr (PART == 1) {
+      cluster_sync();                      // (no CTA leaves while another reads its shared memory)
+      return;
+    }
+  } else {
+    for (int c = threadIdx.x; c < n; c += NTHR) ps[c] = pooled[(size_t)b * D.d + c0 + c];
   }
   __syncthreads();
   // threads = column groups x ranks: neighbouring threads read neighbouring elements of v
@@ -118,6 +131,7 @@ phi_prep_kernel(const float* __restrict__ h0, const float* __restrict__ v, const
   }
   cluster_sync();                          // (no CTA leaves while another reads its shared memory)
 }
+inline size_t prep_product_smem(int d) { return ((size_t)d + 4 + MMAX + NTHR) * sizeof(float); }
 inline size_t prep_smem(int d) { return ((size_t)(NTHR / 32 + 1) * d + 4 + MMAX + NTHR) * sizeof(float); }
 
 // The same for widths the registers do not hold (d > 2048 or d % 4 != 0) or rows off 16 bytes: one CTA per sample.
@@ -1138,12 +1152,34 @@ extern "C" int rte_macro_phi_prepare(const float* v, const float* u, float* wt, 
 }
 
 namespace {
+// the cluster kernel's shapes; others take one CTA per sample
+bool phi_rows_path(const float* h0, int d) { return d % 4 == 0 && d <= 2048 && (reinterpret_cast<uintptr_t>(h0) & 15) == 0; }
+
+template <int PART>
+int launch_prep(const float* h0, const float* v, const int32_t* recipe_id, const int32_t* stride_id, float* rstd, float* pooled,
+                float* pa, PhiDims D, float eps, rte_stream_t stream) {
+#define RTE_PREP(NV)                                                                                                         \
+  do {                                                                                                                       \
+    if (prep_smem(128 * NV) > 48 * 1024 &&                                                                                   \
+        cudaFuncSetAttribute(phi_prep_kernel<NV, PART>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_smem(128 * NV)) != cudaSuccess) \
+      return RTE_ERR_LAUNCH;                                                                                                 \
+    rte::launch(phi_prep_kernel<NV, PART>, D.B * PREP_CTAS, NTHR, prep_smem(D.d), ST(stream), h0, v, recipe_id, stride_id, rstd, pooled, pa, D, eps); \
+  } while (0)
+  if (D.d <= 128) RTE_PREP(1);
+  else if (D.d <= 256) RTE_PREP(2);
+  else if (D.d <= 512) RTE_PREP(4);
+  else if (D.d <= 1024) RTE_PREP(8);
+  else RTE_PREP(16);
+#undef RTE_PREP
+  return RTE_OK;
+}
+
 // `h0`: the state Phi is applied to (norm, pooled mean, gain and residual terms); `hx`: the injected state of the third
 // slice of z (the same pointer on the hot path).
 int phi_fwd_impl(const float* h0, const float* hx, const rte_phi_params* p, const int32_t* recipe_id,
                  const int32_t* stride_id, float s_cfg, float* out, float* rstd, float* pooled,
                  float* act, int32_t B, int32_t S, int32_t d, int32_t m, int32_t K_strides,
-                 float eps, rte_stream_t stream) {
+                 float eps, rte_stream_t stream, bool rows_done = false) {
   RTE_CHECK_ARG(h0 && hx && p && p->gain && p->v && p->u && p->bias && p->scale && recipe_id && stride_id && out && rstd &&
                 pooled && act && B > 0 && S > 0 && d > 0 && m > 0 && K_strides > 0);
   if (m > MMAX) return RTE_ERR_UNSUPPORTED;
@@ -1152,20 +1188,12 @@ int phi_fwd_impl(const float* h0, const float* hx, const rte_phi_params* p, cons
   // `act` doubles as the home of pa (B*m floats) is NOT safe; pa lives at the tail of `pooled`'s
   // companion: callers give pooled >= B*d + B*m floats.
   float* pa = pooled + (size_t)B * d;
-  if (d % 4 == 0 && d <= 2048 && (reinterpret_cast<uintptr_t>(h0) & 15) == 0) {
-#define RTE_PREP(NV)                                                                                                         \
-  do {                                                                                                                       \
-    if (prep_smem(128 * NV) > 48 * 1024 &&                                                                                   \
-        cudaFuncSetAttribute(phi_prep_kernel<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)prep_smem(128 * NV)) != cudaSuccess) \
-      return RTE_ERR_LAUNCH;                                                                                                 \
-    rte::launch(phi_prep_kernel<NV>, B * PREP_CTAS, NTHR, prep_smem(d), ST(stream), h0, p->v, recipe_id, stride_id, rstd, pooled, pa, D, eps); \
-  } while (0)
-    if (d <= 128) RTE_PREP(1);
-    else if (d <= 256) RTE_PREP(2);
-    else if (d <= 512) RTE_PREP(4);
-    else if (d <= 1024) RTE_PREP(8);
-    else RTE_PREP(16);
-#undef RTE_PREP
+  if (rows_done) {
+    if (!phi_rows_path(h0, d)) return RTE_ERR_UNSUPPORTED;
+    rte::launch(phi_prep_kernel<1, 2>, B * PREP_CTAS, NTHR, prep_product_smem(d), ST(stream), h0, p->v, recipe_id, stride_id, rstd, pooled, pa, D, eps);
+  } else if (phi_rows_path(h0, d)) {
+    const int rc = launch_prep<0>(h0, p->v, recipe_id, stride_id, rstd, pooled, pa, D, eps, stream);
+    if (rc != RTE_OK) return rc;
   } else {
     rte::launch(phi_prep_any_kernel, B, NTHR, (size_t)(S + d) * sizeof(float), ST(stream), h0, p->v, recipe_id, stride_id, rstd, pooled, pa, D, eps);
   }
@@ -1205,6 +1233,23 @@ extern "C" int rte_macro_phi_fwd(const float* h0, const rte_phi_params* p, const
                                  float* act, int32_t B, int32_t S, int32_t d, int32_t m, int32_t K_strides,
                                  float eps, rte_stream_t stream) {
   return phi_fwd_impl(h0, h0, p, recipe_id, stride_id, s_cfg, out, rstd, pooled, act, B, S, d, m, K_strides, eps, stream);
+}
+
+extern "C" int rte_macro_phi_rows(const float* h0, float* rstd, float* pooled, int32_t B, int32_t S, int32_t d, int32_t m, float eps,
+                                  rte_stream_t stream) {
+  RTE_CHECK_ARG(h0 && rstd && pooled && B > 0 && S > 0 && d > 0 && m > 0);
+  if (m > MMAX || !phi_rows_path(h0, d)) return RTE_ERR_UNSUPPORTED;
+  const int rc = launch_prep<1>(h0, nullptr, nullptr, nullptr, rstd, pooled, nullptr, PhiDims{B, S, d, m, 1}, eps, stream);
+  if (rc != RTE_OK) return rc;
+  RTE_LAUNCH_CHECK();
+  return RTE_OK;
+}
+
+extern "C" int rte_macro_phi_fwd_from_rows(const float* h0, const rte_phi_params* p, const int32_t* recipe_id,
+                                           const int32_t* stride_id, float s_cfg, float* out, float* rstd, float* pooled,
+                                           float* act, int32_t B, int32_t S, int32_t d, int32_t m, int32_t K_strides,
+                                           float eps, rte_stream_t stream) {
+  return phi_fwd_impl(h0, h0, p, recipe_id, stride_id, s_cfg, out, rstd, pooled, act, B, S, d, m, K_strides, eps, stream, true);
 }
 
 extern "C" int rte_macro_phi_fwd_hx(const float* h, const float* h0, const rte_phi_params* p, const int32_t* recipe_id,

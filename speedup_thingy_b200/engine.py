@@ -1153,6 +1153,18 @@ class TrainEngine:
             x = self._block_fwd(blk, x)
         if not self.dense:
             h0 = x
+            # What the macro operator needs besides the route -- its transposed parameters, the norms and pooled rows of h0 -- is
+            # made beside the router on the stream of its parameter gradients, idle until then (8 x 64 tokens of width 128: step 273.7 ->
+            # 266.9 us; audited shortlist step of 16384 x 512 2670 -> 2651; forward pass alone of the evaluation 282.6 -> 278.8).
+            phi_rows = phi_ready = None
+            if self.phi_wt is not None and self._misc_param_stream is not None:
+                ms = self._misc_param_stream
+                ms.wait_stream(torch.cuda.current_stream(self.device))
+                with torch.cuda.stream(ms):
+                    o.macro_phi_prepare(self._phi_param_dict())
+                    phi_rows = o.macro_phi_rows(h0, self.phi_rstd, self.phi_pooled, B=B, S=S, d=d, m=cfg.macro_rank)
+                    phi_ready = torch.cuda.Event()
+                    phi_ready.record(ms)
             fixed_depth_id = None if tr.fixed_depth is None else list(cfg.depth_choices).index(tr.fixed_depth)
             if self.audit is not None and not self.audit.bernoulli:
                 if self.audit.own_prelude:
@@ -1208,14 +1220,16 @@ class TrainEngine:
                 self._side_wait_main()
                 with self._on_side():
                     self.audit.forward_replay(h0, head_done=True)
-            if self.phi_wt is not None:
+            if phi_ready is not None:
+                torch.cuda.current_stream(self.device).wait_event(phi_ready)
+            elif self.phi_wt is not None:
                 o.macro_phi_prepare(self._phi_param_dict())
             self._cons_done, self._cons_pending = None, False
             if self.cons_pairs and not forward_only:
                 self._cons_done, self._cons_pending = self._consistency_branch(h0), True
             o.macro_phi_fwd(h0, self._phi_param_dict(), self.route["recipe_id"], self.route["depth_id"],
                             cfg.macro_update_scale, self.h_phi, self.phi_rstd, self.phi_pooled, self.phi_act,
-                            B=B, S=S, d=d, m=cfg.macro_rank, K=len(cfg.depth_choices))
+                            B=B, S=S, d=d, m=cfg.macro_rank, K=len(cfg.depth_choices), **({"rows_done": True} if phi_rows else {}))
             x = self.h_phi
             if self.audit is not None:
                 self.audit.forward_distill(self.h_phi)           # (picks its stream itself)

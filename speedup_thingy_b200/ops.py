@@ -444,10 +444,20 @@ class CudaOps:
             raise ValueError("macro_phi_prepare: wt too small")
         self._call("rte_macro_phi_prepare", _ptr(p["v"]), _ptr(p["u"]), _ptr(p["wt"]), R * K, d, m, self.stream)
 
-    def macro_phi_fwd(self, h0, p: dict, recipe_id, stride_id, s_cfg, out, rstd, pooled, act, *, B, S, d, m, K):
+    def macro_phi_rows(self, h0, rstd, pooled, *, B, S, d, m) -> bool:
+        """The part of `macro_phi_fwd` that needs no route; False where only the whole of it serves."""
+        rc = self.lib.rte_macro_phi_rows(_ptr(h0), _ptr(rstd), _ptr(pooled), B, S, d, m, 1e-5, self.stream)
+        if rc == A.ERR_UNSUPPORTED:
+            return False
+        self.launches += 1
+        A.check(rc, "rte_macro_phi_rows")
+        return True
+
+    def macro_phi_fwd(self, h0, p: dict, recipe_id, stride_id, s_cfg, out, rstd, pooled, act, *, B, S, d, m, K, rows_done: bool = False):
+        """`rows_done`: `macro_phi_rows` has filled `rstd` and `pooled`."""
         sp = self._phi_params(p)
-        self._call("rte_macro_phi_fwd", _ptr(h0), C.byref(sp), _ptr(recipe_id), _ptr(stride_id), s_cfg, _ptr(out),
-                   _ptr(rstd), _ptr(pooled), _ptr(act), B, S, d, m, K, 1e-5, self.stream)
+        self._call("rte_macro_phi_fwd_from_rows" if rows_done else "rte_macro_phi_fwd", _ptr(h0), C.byref(sp), _ptr(recipe_id),
+                   _ptr(stride_id), s_cfg, _ptr(out), _ptr(rstd), _ptr(pooled), _ptr(act), B, S, d, m, K, 1e-5, self.stream)
 
     def macro_phi_bwd(self, h0, dout, p: dict, recipe_id, stride_id, s_cfg, rstd, pooled, act, dh0, grads: dict,
                       scratch, *, B, S, d, m, R, K):

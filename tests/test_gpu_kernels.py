@@ -710,6 +710,31 @@ def test_core_gradient_sums(ops, T, d, n_rows, P):
         assert torch.isfinite(b).all() and torch.equal(a, b)
 
 
+@pytest.mark.parametrize("B,S,d,m", [(1, 1, 4, 4), (3, 5, 36, 3), (2, 64, 128, 32), (2, 130, 512, 33), (4, 7, 1024, 32), (1, 40, 2048, 64)])
+def test_macro_phi_from_rows(ops, B, S, d, m):
+    """The forward in two calls, the route known only to the second: the same bits as in one."""
+    g = torch.Generator().manual_seed(d + m)
+    R, K = 2, 2
+    rn = lambda *s: torch.randn(*s, generator=g).to(DEV)      # noqa: E731
+    p = dict(gain=rn(R, K, d), v=rn(R, K, 3 * d, m) * d ** -0.5, u=rn(R, K, m, d) * m ** -0.5, bias=rn(R, K, d), scale=rn(R, K),
+             wt=torch.zeros(R * K * 4 * d * m, device=DEV))
+    h0 = rn(B * S, d)
+    rid, sid = (torch.randint(0, n, (B,), generator=g, dtype=torch.int32).to(DEV) for n in (R, K))
+    ops.macro_phi_prepare(p)
+
+    def run(split):
+        out, rstd, pooled, act = (torch.full(s, 7.0, device=DEV) for s in ((B * S, d), (B * S,), (B * (d + m),), (B * S, m)))
+        if split:
+            assert ops.macro_phi_rows(h0, rstd, pooled, B=B, S=S, d=d, m=m)
+        ops.macro_phi_fwd(h0, p, rid, sid, 0.5, out, rstd, pooled, act, B=B, S=S, d=d, m=m, K=K, rows_done=split)
+        return out, rstd, pooled, act
+
+    for a, b in zip(run(False), run(True)):
+        assert torch.equal(a, b)
+    assert not ops.macro_phi_rows(h0, h0, h0, B=B, S=S, d=d - 1, m=m)      # widths of the kernel with a CTA per sample
+    assert not ops.macro_phi_rows(h0.view(-1)[1:], h0, h0, B=B, S=S, d=d, m=m)
+
+
 # ------------------------------------------------------------------ vocabulary shortlist
 @pytest.mark.parametrize("B,S,V,C,TC,HN,RN,K", [(3, 7, 96, 8, 2, 4, 4, 16), (4, 33, 2048, 64, 2, 32, 32, 128),
                                                 (2, 5, 50, 7, 3, 60, 0, 50), (2, 9, 4096, 64, 1, 0, 8, 256)])
