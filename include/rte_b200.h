@@ -111,6 +111,9 @@ typedef struct rte_gemm_args {
 } rte_gemm_args;
 
 int rte_gemm_bf16(const rte_gemm_args* args, rte_stream_t stream);
+/* RTE_EPI_SWIGLU_BWD over the selected neurons only: C = 0 where the byte of selected [M][N] is 0.  RTE_ERR_UNSUPPORTED unless N % 16 == 0,
+ * `selected` lies on 16 bytes and C, R and their strides suit the TMA. */
+int rte_gemm_bf16_swiglu_bwd_selected(const rte_gemm_args* args, const uint8_t* selected, rte_stream_t stream);
 /* How many splits (1 .. max_splits) a product with fp32 output and a long reduction should be cut into when its partials
  * are added by rte_reduce_splits; 1: one rte_gemm_bf16 launch is faster.                                             */
 int rte_gemm_wgrad_splits(const rte_gemm_args* args, int32_t max_splits);

@@ -105,6 +105,7 @@ PROTOTYPES = {
     "rte_status_string": (C.c_char_p, [C.c_int]),
     "rte_device_sm_count": (C.c_int, []),
     "rte_gemm_bf16": (C.c_int, [P(GemmArgs), c_vp]),
+    "rte_gemm_bf16_swiglu_bwd_selected": (C.c_int, [P(GemmArgs), c_vp, c_vp]),
     "rte_gemm_bf16_small": (C.c_int, [P(GemmArgs), c_vp]),
     "rte_gemm_bf16_tile": (C.c_int, [P(GemmArgs), C.c_int32, C.c_int32, c_vp]),
     "rte_gemm_bf16_resident": (C.c_int, [P(GemmArgs), C.c_int32, c_vp]),

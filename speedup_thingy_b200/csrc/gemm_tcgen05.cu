@@ -65,6 +65,7 @@ struct KParams {
   int b_group_stride;       // grouped mode: rows of the stacked B between consecutive groups
   const int* split_kb;      // ragged split-K: k-block range [split_kb[s], split_kb[s+1]) of split s, else null
   int* status;
+  const uint8_t* selected;  // MASK: [M, N] bytes, 0 where the gradient is zero; else null
 };
 
 // ------------------------------------------------------------------ epilogue helpers
@@ -152,7 +153,8 @@ struct SmemLayout {
 // ------------------------------------------------------------------ kernel
 // SWB: the epilogue is SwiGLU's backward with its operands brought in by the TMA (see there); a kernel of its own because
 // its staging slots take shared memory from the operand stages.
-template <int BN, int CTAS, bool SWB>
+// MASK: gradients of the selected neurons only (zeros elsewhere).
+template <int BN, int CTAS, bool SWB, bool MASK>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                     const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_c2,
@@ -388,6 +390,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         tc_fence_after();
         for (int c0 = grp * HALF; c0 < (grp + 1) * HALF; c0 += 64, ++piece) {
           const bool last = c0 + 64 >= (grp + 1) * HALF;
+          uint32_t sel[MASK ? 16 : 1];         // this row's 64 bytes, under way while the operands arrive
+          if constexpr (MASK) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              uint4 b = make_uint4(0u, 0u, 0u, 0u);
+              if (row_ok && n0 + c0 + 16 * k < p.N) b = __ldg(reinterpret_cast<const uint4*>(p.selected + size_t(row) * p.N + n0 + c0 + 16 * k));
+              sel[4 * k] = b.x; sel[4 * k + 1] = b.y; sel[4 * k + 2] = b.z; sel[4 * k + 3] = b.w;
+            }
+          }
           fetch_piece(piece + 1, last ? w + n_units : w, last ? grp * HALF : c0 + 64);
           if (!mbar_wait<1>(operand_bar(warp - 2, piece & 1u), (piece >> 1) & 1u)) {
             if (p.status && lane == 0) atomicExch(p.status, RTE_DEV_WAIT_TIMEOUT_EPILOGUE);
@@ -414,8 +425,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
               const float2 u_ = rte::unpack_bf16x2(u[j]), g_ = rte::unpack_bf16x2(g[j]);
               const float dz0 = __uint_as_float(raw[2 * j]), dz1 = __uint_as_float(raw[2 * j + 1]);
               const float s0 = fast_sigmoid(g_.x), s1 = fast_sigmoid(g_.y);
-              u[j] = rte::pack_bf16x2(dz0 * g_.x * s0, dz1 * g_.y * s1);
-              g[j] = rte::pack_bf16x2(dz0 * u_.x * s0 * (1.f + g_.x * (1.f - s0)), dz1 * u_.y * s1 * (1.f + g_.y * (1.f - s1)));
+              float du0 = dz0 * g_.x * s0, du1 = dz1 * g_.y * s1;
+              float dg0 = dz0 * u_.x * s0 * (1.f + g_.x * (1.f - s0)), dg1 = dz1 * u_.y * s1 * (1.f + g_.y * (1.f - s1));
+              if constexpr (MASK) {
+                const uint32_t two = sel[8 * h + (j >> 1)] >> (16 * (j & 1));
+                if ((two & 0xffu) == 0u) du0 = dg0 = 0.f;
+                if ((two & 0xff00u) == 0u) du1 = dg1 = 0.f;
+              }
+              u[j] = rte::pack_bf16x2(du0, du1);
+              g[j] = rte::pack_bf16x2(dg0, dg1);
             }
 #pragma unroll
             for (uint32_t c = 0; c < 4; ++c) {
@@ -781,13 +799,13 @@ Choice choose(const rte_gemm_args* a, int splits, int sms) {
 }
 
 // Work units (CTAs or CTA pairs) that can run at the same time on `ctas` CTAs.
-template <int BN, int CTAS, bool SWB = false>
+template <int BN, int CTAS, bool SWB = false, bool MASK = false>
 int concurrent_units(int ctas, int sm_count) {
   using L = SmemLayout<BN, CTAS, SWB>;
   if (CTAS == 1) return ctas;
   static int max_clusters = -1;
   if (max_clusters < 0) {
-    if (cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, CTAS, SWB>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, CTAS, SWB, MASK>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL) != cudaSuccess)
       return ctas / 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(sm_count / 2 * 2));
@@ -798,26 +816,26 @@ int concurrent_units(int ctas, int sm_count) {
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_tcgen05_kernel<BN, CTAS, SWB>, &cfg) == cudaSuccess && n > 0) max_clusters = n;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm_tcgen05_kernel<BN, CTAS, SWB, MASK>, &cfg) == cudaSuccess && n > 0) max_clusters = n;
     else { (void)cudaGetLastError(); max_clusters = sm_count / 2; }
   }
   int units = ctas / 2;
   return units < max_clusters ? units : max_clusters;
 }
 
-template <int BN, int CTAS, bool SWB = false>
+template <int BN, int CTAS, bool SWB = false, bool MASK = false>
 int launch(const rte_gemm_args* a, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc,
            const CUtensorMap& tc2, const CUtensorMap& tr, const CUtensorMap& tr2, KParams& kp, int sm_count, cudaStream_t st) {
   using L = SmemLayout<BN, CTAS, SWB>;
   static_assert(L::STAGES >= 3, "too few pipeline stages fit");
   static bool attr_set = false;
   if (!attr_set) {
-    if (cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, CTAS, SWB>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_tcgen05_kernel<BN, CTAS, SWB, MASK>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL) != cudaSuccess)
       return RTE_ERR_LAUNCH;
     attr_set = true;
   }
   const int total = kp.num_m_blocks * kp.num_n_blocks * kp.splits;
-  int units = concurrent_units<BN, CTAS, SWB>(persistent_ctas(a, sm_count), sm_count);
+  int units = concurrent_units<BN, CTAS, SWB, MASK>(persistent_ctas(a, sm_count), sm_count);
   if (units > total) units = total;
   if (units < 1) units = 1;
   cudaLaunchConfig_t cfg = {};
@@ -831,7 +849,7 @@ int launch(const rte_gemm_args* a, const CUtensorMap& ta, const CUtensorMap& tb,
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = CTAS; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr; cfg.numAttrs = (CTAS == 2) ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, CTAS, SWB>, ta, tb, tc, tc2, tr, tr2, kp) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, gemm_tcgen05_kernel<BN, CTAS, SWB, MASK>, ta, tb, tc, tc2, tr, tr2, kp) != cudaSuccess) {
     (void)cudaGetLastError();
     return RTE_ERR_LAUNCH;
   }
@@ -873,7 +891,9 @@ extern "C" int rte_gemm_wgrad_splits(const rte_gemm_args* a, int32_t max_splits)
   return splits;
 }
 
-extern "C" int rte_gemm_bf16(const rte_gemm_args* a, rte_stream_t stream) {
+namespace {
+// `selected` (SwiGLU's backward only): RTE_ERR_UNSUPPORTED where the epilogue that takes it does not serve
+int run_gemm(const rte_gemm_args* a, const uint8_t* selected, rte_stream_t stream) {
   RTE_CHECK_ARG(a != nullptr && a->A && a->B && a->C);
   RTE_CHECK_ARG(a->M > 0 && a->N > 0 && a->K > 0);
   RTE_CHECK_ARG(a->epilogue >= RTE_EPI_BF16 && a->epilogue <= RTE_EPI_SWIGLU_BWD);
@@ -912,6 +932,7 @@ extern "C" int rte_gemm_bf16(const rte_gemm_args* a, rte_stream_t stream) {
   kp.kblocks_total = rte::ceil_div(a->K, BK);
   kp.kblocks_per_split = rte::ceil_div(kp.kblocks_total, splits);
   kp.status = a->status;
+  kp.selected = selected;
   kp.tile_group = a->tile_group;
   kp.b_group_stride = a->b_group_stride;
   kp.split_kb = a->split_kblocks;
@@ -977,7 +998,14 @@ extern "C" int rte_gemm_bf16(const rte_gemm_args* a, rte_stream_t stream) {
   if (DIAG && (kp.diag & 16)) kp.tma_store = 0;
 
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (swiglu_b && tma_ok && !(DIAG && (kp.diag & 16)) && !(bn == 256 && ctas == 1)) {
+  const bool swb = swiglu_b && tma_ok && !(DIAG && (kp.diag & 16)) && !(bn == 256 && ctas == 1);
+  if (selected != nullptr) {
+    if (!swb || a->N % 16 != 0 || (reinterpret_cast<uintptr_t>(selected) & 15)) return RTE_ERR_UNSUPPORTED;
+    if (ctas == 1) return launch<128, 1, true, true>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st);
+    return bn == 256 ? launch<256, 2, true, true>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st)
+                     : launch<128, 2, true, true>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st);
+  }
+  if (swb) {
     if (ctas == 1) return launch<128, 1, true>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st);
     return bn == 256 ? launch<256, 2, true>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st)
                      : launch<128, 2, true>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st);
@@ -986,4 +1014,12 @@ extern "C" int rte_gemm_bf16(const rte_gemm_args* a, rte_stream_t stream) {
   if (ctas == 2)
     return bn == 256 ? launch<256, 2>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st) : launch<128, 2>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st);
   return bn == 256 ? launch<256, 1>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st) : launch<128, 1>(a, ta, tb, tc, tc2, tr, tr2, kp, sms, st);
+}
+}  // namespace
+
+extern "C" int rte_gemm_bf16(const rte_gemm_args* a, rte_stream_t stream) { return run_gemm(a, nullptr, stream); }
+
+extern "C" int rte_gemm_bf16_swiglu_bwd_selected(const rte_gemm_args* a, const uint8_t* selected, rte_stream_t stream) {
+  RTE_CHECK_ARG(a != nullptr && selected != nullptr && a->epilogue == RTE_EPI_SWIGLU_BWD);
+  return run_gemm(a, selected, stream);
 }

@@ -735,6 +735,36 @@ def test_macro_phi_from_rows(ops, B, S, d, m):
     assert not ops.macro_phi_rows(h0.view(-1)[1:], h0, h0, B=B, S=S, d=d, m=m)
 
 
+@pytest.mark.parametrize("M,F_,K", [(1, 16, 8), (130, 80, 64), (300, 272, 72), (2100, 1040, 136), (5000, 2048, 128)])
+def test_gemm_swiglu_bwd_of_selected_neurons(ops, M, F_, K):
+    """Against the product without a mask (tested against the oracle above): its bits where selected, zeros elsewhere, whatever the saved
+    values there; and what the epilogue does not take is refused before a launch."""
+    g = torch.Generator().manual_seed(M)
+    dy, w = (torch.randn(n, K, generator=g).bfloat16().to(DEV) for n in (M, F_))
+    sel = (torch.rand(M, F_, generator=g) < 0.3).to(torch.uint8).to(DEV)
+    sel[0] = 0
+    sel[-1, -1] = 255
+    ug = torch.randn(M, 2 * F_, generator=g).bfloat16().to(DEV)
+    want, got = (torch.full((M, 2 * F_), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+
+    def args(out, saved, n=F_):
+        a = A.GemmArgs()
+        a.A, a.B, a.C, a.R, a.status = dy.data_ptr(), w.data_ptr(), out.data_ptr(), saved.data_ptr(), ops.status.data_ptr()
+        a.M, a.N, a.K, a.lda, a.ldb, a.ldc, a.ldr = M, n, K, K, K, 2 * n, 2 * n
+        a.epilogue, a.splits, a.b_pair_offset = A.EPI_SWIGLU_BWD, 1, n
+        return a
+
+    A.check(ops.lib.rte_gemm_bf16(C.byref(args(want, ug)), ops.stream), "rte_gemm_bf16")
+    want = want * sel.bool().repeat(1, 2)
+    saved = torch.where(sel.bool().repeat(1, 2), ug, torch.full_like(ug, float("nan")))
+    fn = ops.lib.rte_gemm_bf16_swiglu_bwd_selected
+    A.check(fn(C.byref(args(got, saved)), sel.data_ptr(), ops.stream), "selected")
+    ops.check_status()
+    assert torch.equal(got, want + 0.0)
+    assert fn(C.byref(args(got, saved, F_ - 8)), sel.data_ptr(), ops.stream) == A.ERR_UNSUPPORTED
+    assert fn(C.byref(args(got, saved)), sel.data_ptr() + 1, ops.stream) == A.ERR_UNSUPPORTED
+
+
 # ------------------------------------------------------------------ vocabulary shortlist
 @pytest.mark.parametrize("B,S,V,C,TC,HN,RN,K", [(3, 7, 96, 8, 2, 4, 4, 16), (4, 33, 2048, 64, 2, 32, 32, 128),
                                                 (2, 5, 50, 7, 3, 60, 0, 50), (2, 9, 4096, 64, 1, 0, 8, 256)])
