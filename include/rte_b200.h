@@ -277,6 +277,12 @@ int rte_ce_fwd_bwd(const void* logits, int32_t ldl, const int64_t* targets, cons
 /* The same over f32 logits and gradients.                                                                              */
 int rte_ce_fwd_bwd_f32(const float* logits, int32_t ldl, const int64_t* targets, const float* row_weight, int32_t S,
                        float* loss_tok, float* dlogits, int32_t rows, int32_t V, int32_t* status, rte_stream_t stream);
+/* Loss and gradient in two calls for rows of more than 16 KB (RTE_ERR_UNSUPPORTED for others): the first keeps the rows' logsumexp
+ * (lse f32 [rows]), the second then reads the logits once.  logits / dlogits f32 or bf16 (`f32`). */
+int rte_ce_loss_lse(const void* logits, int32_t f32, int32_t ldl, const int64_t* targets, float* loss_tok, float* lse, int32_t rows,
+                    int32_t V, int32_t* status, rte_stream_t stream);
+int rte_ce_gradient(const void* logits, int32_t f32, int32_t ldl, const int64_t* targets, const float* row_weight, int32_t S,
+                    const float* lse, void* dlogits, int32_t rows, int32_t V, int32_t* status, rte_stream_t stream);
 /* out[b] = sum_s in[b*S + s]  (per-sample loss sums, models.py:75) */
 int rte_segment_sum(const float* in, float* out, int32_t n_seg, int32_t seg_len, rte_stream_t stream);
 

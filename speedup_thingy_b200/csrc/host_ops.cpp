@@ -464,18 +464,28 @@ struct CrossEntropy : Function<CrossEntropy> {
     if (!direct(lg.scalar_type())) lg = lg.to(F32);
     lg = lg.view({-1, V});
     const Tensor tg = targets.to(torch::kInt64).contiguous().view({-1}), loss = empty({lg.size(0)}, F32, logits);
-    run(dev, lg, tg, Tensor(), loss, Tensor());
-    ctx->save_for_backward({lg, tg});
+    Tensor lse;                                                           // long rows: kept, so that the gradient is one pass
+    if (lg.size(0) > 0 && V * lg.element_size() > 16 * 1024 - 32) {
+      lse = empty({lg.size(0)}, F32, logits);
+      const int rc = rte_ce_loss_lse(ptr(lg), lg.scalar_type() == F32, V, tg.data_ptr<int64_t>(), f32(loss), f32(lse), lg.size(0), V, dev.status, dev.st);
+      if (rc == RTE_ERR_UNSUPPORTED) lse = Tensor();
+      else check(rc, "rte_ce_loss_lse");
+    }
+    if (!lse.defined()) run(dev, lg, tg, Tensor(), loss, Tensor());
+    ctx->save_for_backward({lg, tg, lse});
     ctx->saved_data["shape"] = logits.sizes().vec();
     ctx->saved_data["type"] = int64_t(logits.scalar_type());
     return {loss.view(targets.sizes())};
   }
   static variable_list backward(AutogradContext* ctx, variable_list g) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &lg = saved[0], &tg = saved[1];
+    const Tensor &lg = saved[0], &tg = saved[1], &lse = saved[2];
     Dev dev(lg);
-    const Tensor grad = at::empty_like(lg), scratch = empty({lg.size(0)}, F32, lg);
-    run(dev, lg, tg, g[0].to(F32).contiguous(), scratch, grad);           // (softmax - onehot) * dloss[row]
+    const Tensor grad = at::empty_like(lg), dloss = g[0].to(F32).contiguous();         // (softmax - onehot) * dloss[row]
+    if (lse.defined())
+      check(rte_ce_gradient(ptr(lg), lg.scalar_type() == F32, lg.size(1), tg.data_ptr<int64_t>(), f32(dloss), 1, f32(lse), ptr(grad), lg.size(0),
+                            lg.size(1), dev.status, dev.st), "rte_ce_gradient");
+    else run(dev, lg, tg, dloss, empty({lg.size(0)}, F32, lg), grad);
     return {grad.to(at::ScalarType(ctx->saved_data["type"].toInt())).view(ctx->saved_data["shape"].toIntVector()), Tensor()};
   }
 };

@@ -765,6 +765,40 @@ def test_gemm_swiglu_bwd_of_selected_neurons(ops, M, F_, K):
     assert fn(C.byref(args(got, saved)), sel.data_ptr() + 1, ops.stream) == A.ERR_UNSUPPORTED
 
 
+@pytest.mark.parametrize("dtype,rows,V,off", [("f32", 3, 4096, 0), ("f32", 5, 4100, 0), ("f32", 3, 4093, 1), ("f32", 7, 9001, 3), ("bf16", 3, 8192, 0),
+                                              ("bf16", 5, 8200, 0), ("bf16", 3, 8187, 5), ("bf16", 600, 12345, 0)])
+def test_ce_gradient_from_kept_sums(ops, dtype, rows, V, off):
+    """Two calls against one over long rows (and the longest that are refused): the same bits, with masked columns, a row of nothing but
+    masked ones and a NaN; `off` moves the logits off the 16-byte boundary."""
+    g = torch.Generator().manual_seed(V)
+    dt, f32 = (torch.float32, 1) if dtype == "f32" else (torch.bfloat16, 0)
+    buf = torch.empty(rows * V + off, dtype=dt, device=DEV)
+    x = buf[off:].view(rows, V)
+    x.copy_(torch.randn(rows, V, generator=g) * 3)
+    x[0, : V // 2] = float("-inf")
+    x[1] = torch.finfo(dt).min
+    x[2, 7] = float("nan")
+    tg = torch.randint(V // 2, V, (rows,), generator=g).to(DEV)
+    w = torch.randn(rows, generator=g).to(DEV)
+    loss, want_loss, lse = (torch.full((rows,), 7.0, device=DEV) for _ in range(3))
+    want, got = torch.empty_like(x), torch.empty_like(x)
+    one = ops.lib.rte_ce_fwd_bwd_f32 if f32 else ops.lib.rte_ce_fwd_bwd
+    st = ops.status.data_ptr()
+    A.check(one(x.data_ptr(), V, tg.data_ptr(), w.data_ptr(), 1, want_loss.data_ptr(), want.data_ptr(), rows, V, st, ops.stream), "one")
+    rc = ops.lib.rte_ce_loss_lse(x.data_ptr(), f32, V, tg.data_ptr(), loss.data_ptr(), lse.data_ptr(), rows, V, st, ops.stream)
+    W = 4 if f32 else 8
+    even = V % W == 0 and x.data_ptr() % 16 == 0
+    if (V if even else V + 2 * (W - 1)) // W <= 1024:
+        assert rc == A.ERR_UNSUPPORTED
+        return
+    A.check(rc, "rte_ce_loss_lse")
+    A.check(ops.lib.rte_ce_gradient(x.data_ptr(), f32, V, tg.data_ptr(), w.data_ptr(), 1, lse.data_ptr(), got.data_ptr(), rows, V, st,
+                                    ops.stream), "rte_ce_gradient")
+    ops.check_status()
+    assert torch.equal(loss.nan_to_num(123.0), want_loss.nan_to_num(123.0))
+    assert torch.equal(got.nan_to_num(123.0), want.nan_to_num(123.0))
+
+
 # ------------------------------------------------------------------ vocabulary shortlist
 @pytest.mark.parametrize("B,S,V,C,TC,HN,RN,K", [(3, 7, 96, 8, 2, 4, 4, 16), (4, 33, 2048, 64, 2, 32, 32, 128),
                                                 (2, 5, 50, 7, 3, 60, 0, 50), (2, 9, 4096, 64, 1, 0, 8, 256)])
