@@ -799,6 +799,37 @@ def test_ce_gradient_from_kept_sums(ops, dtype, rows, V, off):
     assert torch.equal(got.nan_to_num(123.0), want.nan_to_num(123.0))
 
 
+@pytest.mark.parametrize("B,S,d,m,tensor", [(2, 5, 64, 4, True), (3, 64, 128, 32, True), (2, 33, 36, 3, False), (1, 40, 512, 48, True)])
+def test_macro_phi_bwd_with_the_routers_share(ops, B, S, d, m, tensor):
+    """d h0 with the router's share and its bf16 copy from the operator's last launch (or, on the scalar kernels, the launches it stands
+    for) against the three launches: the same bits."""
+    g = torch.Generator().manual_seed(d + m)
+    R, K, hid = 2, 3, 16
+    rn = lambda *s: torch.randn(*s, generator=g).to(DEV)      # noqa: E731
+    p = dict(gain=rn(R, K, d), v=rn(R, K, 3 * d, m) * d ** -0.5, u=rn(R, K, m, d) * m ** -0.5, bias=rn(R, K, d), scale=rn(R, K))
+    if tensor:
+        p["wt"] = torch.zeros(R * K * 4 * d * m, device=DEV)
+        ops.macro_phi_prepare(p)
+    h0, dout = rn(B * S, d), rn(B * S, d)
+    rid, sid = (torch.randint(0, n, (B,), generator=g, dtype=torch.int32).to(DEV) for n in (R, K))
+    out, rstd, pooled, act = (torch.empty(s, device=DEV) for s in ((B * S, d), (B * S,), (B * (d + m),), (B * S, m)))
+    ops.macro_phi_fwd(h0, p, rid, sid, 0.5, out, rstd, pooled, act, B=B, S=S, d=d, m=m, K=K)
+    share = rn(A.ROUTER_MAX_R + B * (2 * hid + R + K + A.ROUTER_DPOOLED_PARTS * d) + 4)
+    got = []
+    for together in (False, True):
+        dh0, dh16 = torch.full((B * S, d), 7.0, device=DEV), torch.full((B * S, d), 7.0, dtype=torch.bfloat16, device=DEV)
+        grads = {n: torch.empty_like(p[n]) for n in ("gain", "v", "u", "bias")}
+        scratch = torch.empty(ops.phi_bwd_scratch_floats(B, S, d, m), device=DEV)
+        extra = dict(router_scratch=share, hid=hid, dh0_16=dh16) if together else {}
+        ops.macro_phi_bwd_split(h0, dout, p, rid, sid, 0.5, rstd, pooled, act, dh0, grads, scratch, B=B, S=S, d=d, m=m, R=R, K=K, **extra)
+        if not together:
+            ops.router_aux_add_dh0(dh0, share, B=B, S=S, d=d, hid=hid, R=R, K=K)
+            ops.cast_bf16(dh0, dh16)
+        got.append((dh0, dh16, *grads.values()))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+
+
 # ------------------------------------------------------------------ vocabulary shortlist
 @pytest.mark.parametrize("B,S,V,C,TC,HN,RN,K", [(3, 7, 96, 8, 2, 4, 4, 16), (4, 33, 2048, 64, 2, 32, 32, 128),
                                                 (2, 5, 50, 7, 3, 60, 0, 50), (2, 9, 4096, 64, 1, 0, 8, 256)])
