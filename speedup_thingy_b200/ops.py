@@ -665,6 +665,10 @@ class CudaOps:
     def add_(self, dst, src) -> None:
         self._call("rte_add_f32", _ptr(dst), _ptr(src), dst.numel(), self.stream)
 
+    def add2_(self, dst0, src0, dst1, src1) -> None:
+        """Two of `add_` over ranges that do not overlap, in one launch."""
+        self._call("rte_add2_f32", _ptr(dst0), _ptr(src0), dst0.numel(), _ptr(dst1), _ptr(src1), dst1.numel(), self.stream)
+
     def axpy_rows(self, dst, vec, alpha: float, rows: int, seg: int, d: int) -> None:
         self._call("rte_axpy_rows_f32", _ptr(dst), _ptr(vec), alpha, rows, seg, d, self.stream)
 

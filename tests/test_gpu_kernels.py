@@ -830,6 +830,22 @@ def test_macro_phi_bwd_with_the_routers_share(ops, B, S, d, m, tensor):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("n0,n1,off", [(1, 3, 0), (4, 1030, 0), (4099, 7, 1), (1 << 20, 3_000_001, 0), (70000, 1 << 20, 3)])
+def test_add_of_one_and_two_ranges(ops, n0, n1, off):
+    """Whole 16-byte groups, their remainders and ranges off the 16-byte boundary; what lies around a range stays."""
+    g = torch.Generator().manual_seed(n0)
+    def pair(n):
+        d, s = (torch.randn(n + 8, generator=g).to(DEV) for _ in range(2))
+        want = d.clone()
+        want[off:off + n] += s[off:off + n]
+        return d, s, want
+    (d0, s0, w0), (d1, s1, w1), (d2, s2, w2) = pair(n0), pair(n1), pair(n1)
+    ops.add2_(d0[off:off + n0], s0[off:off + n0], d1[off:off + n1], s1[off:off + n1])
+    ops.add_(d2[off:off + n1], s2[off:off + n1])
+    for d, w in ((d0, w0), (d1, w1), (d2, w2)):
+        assert torch.equal(d, w)
+
+
 # ------------------------------------------------------------------ vocabulary shortlist
 @pytest.mark.parametrize("B,S,V,C,TC,HN,RN,K", [(3, 7, 96, 8, 2, 4, 4, 16), (4, 33, 2048, 64, 2, 32, 32, 128),
                                                 (2, 5, 50, 7, 3, 60, 0, 50), (2, 9, 4096, 64, 1, 0, 8, 256)])
