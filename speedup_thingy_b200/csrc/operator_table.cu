@@ -8,19 +8,34 @@
 
 namespace {
 
-struct CastJobs { const float* src[4]; __nv_bfloat16* dst[4]; long long n4[4]; long long n[4]; };
+// Bound by HBM (6 bytes an element).  Every CTA takes 4096 consecutive elements of one tensor, four 16-byte loads a thread before the
+// first store: with the largest tensor's grid for each of them and one load a trip, small tensors left CTAs without work
+// and a thread waited for each load: 4 M elements + two small tensors 17.5 -> 6.0 us, 8 M + three of 1 M 29.5 -> 12.4, 34 M alone
+// 41.7 -> 33.2 (6.1 TB/s).
+constexpr int CAST_CTA = 4096;
+struct CastJobs { const float* src[4]; __nv_bfloat16* dst[4]; long long n4[4]; long long n[4]; int first[4]; int count; };
 
-__global__ void __launch_bounds__(256) cast_many_kernel(const CastJobs jobs) {
+__global__ void __launch_bounds__(256) cast_many_kernel(const __grid_constant__ CastJobs jobs) {
   rte::after_previous_grid();
-  const float* src = jobs.src[blockIdx.y];
-  __nv_bfloat16* dst = jobs.dst[blockIdx.y];
-  const long long n4 = jobs.n4[blockIdx.y], n = jobs.n[blockIdx.y];
-  const long long at = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
-  for (long long i = at; i < n4; i += step) {
-    const float4 v = reinterpret_cast<const float4*>(src)[i];
-    reinterpret_cast<uint2*>(dst)[i] = make_uint2(rte::pack_bf16x2(v.x, v.y), rte::pack_bf16x2(v.z, v.w));
+  int j = 0;
+  while (j + 1 < jobs.count && (int)blockIdx.x >= jobs.first[j + 1]) ++j;
+  const float* __restrict__ src = jobs.src[j];
+  __nv_bfloat16* __restrict__ dst = jobs.dst[j];
+  const long long n4 = jobs.n4[j], n = jobs.n[j], base = (long long)((int)blockIdx.x - jobs.first[j]) * CAST_CTA;
+  if (n4 > 0) {
+    const long long at = base / 4 + threadIdx.x;
+    float4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (at + 256 * u < n4) v[u] = reinterpret_cast<const float4*>(src)[at + 256 * u];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (at + 256 * u < n4) reinterpret_cast<uint2*>(dst)[at + 256 * u] = make_uint2(rte::pack_bf16x2(v[u].x, v[u].y), rte::pack_bf16x2(v[u].z, v[u].w));
+    const long long rest = 4 * n4 + threadIdx.x;                       // (at most three elements: the last CTA's)
+    if (base + CAST_CTA >= n && rest < n) dst[rest] = __float2bfloat16_rn(src[rest]);
+  } else {
+    for (long long i = base + threadIdx.x; i < n && i < base + CAST_CTA; i += 256) dst[i] = __float2bfloat16_rn(src[i]);
   }
-  for (long long i = 4 * n4 + at; i < n; i += step) dst[i] = __float2bfloat16_rn(src[i]);
 }
 
 __device__ __forceinline__ float4 load4(const void* p, int is_bf16, size_t i4) {
@@ -151,16 +166,19 @@ inline bool on16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) =
 extern "C" int rte_cast_many_f32_bf16(const float* const* src, void* const* dst, const int64_t* n, int32_t count, rte_stream_t stream) {
   RTE_CHECK_ARG(src && dst && n && count >= 1 && count <= 4);
   CastJobs jobs = {};
-  long long most = 0;
+  long long ctas = 0;
   for (int j = 0; j < count; ++j) {
     RTE_CHECK_ARG(src[j] && dst[j] && n[j] > 0);
     jobs.src[j] = src[j];
     jobs.dst[j] = reinterpret_cast<__nv_bfloat16*>(dst[j]);
     jobs.n[j] = n[j];
     jobs.n4[j] = on16(src[j]) && (reinterpret_cast<uintptr_t>(dst[j]) & 7) == 0 ? n[j] / 4 : 0;
-    if (n[j] > most) most = n[j];
+    jobs.first[j] = (int)ctas;
+    ctas += (n[j] + CAST_CTA - 1) / CAST_CTA;
+    RTE_CHECK_ARG(ctas < (1ll << 31));
   }
-  rte::launch(cast_many_kernel, dim3(blocks_for(most / 4, 148 * 8), count), 256, 0, ST(stream), jobs);
+  jobs.count = count;
+  rte::launch(cast_many_kernel, (unsigned)ctas, 256, 0, ST(stream), jobs);
   RTE_LAUNCH_CHECK();
   return RTE_OK;
 }

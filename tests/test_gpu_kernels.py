@@ -846,6 +846,21 @@ def test_add_of_one_and_two_ranges(ops, n0, n1, off):
         assert torch.equal(d, w)
 
 
+@pytest.mark.parametrize("sizes,off", [([1], 0), ([4096, 4097, 3], 0), ([4095, 8192, 5, 20000], 1), ([1_000_003, 2], 2), ([7, 4096 * 3 + 1], 4)])
+def test_casts_of_several_tensors(ops, sizes, off):
+    """Whole and partial CTAs of each tensor, remainders of four, sources and results off their boundaries; nothing else is written."""
+    g = torch.Generator().manual_seed(sum(sizes))
+    src = [torch.randn(n + off, generator=g).to(DEV) for n in sizes]
+    dst = [torch.full((n + off + 8,), 7.0, dtype=torch.bfloat16, device=DEV) for n in sizes]
+    k = len(sizes)
+    a = (C.c_void_p * k)(*[t[off:].data_ptr() for t in src])
+    b = (C.c_void_p * k)(*[t[off:].data_ptr() for t in dst])
+    A.check(ops.lib.rte_cast_many_f32_bf16(a, b, (C.c_int64 * k)(*sizes), k, ops.stream), "rte_cast_many_f32_bf16")
+    for s, d, n in zip(src, dst, sizes):
+        assert torch.equal(d[off:off + n], s[off:].bfloat16())
+        assert bool((d[:off] == 7).all()) and bool((d[off + n:] == 7).all())
+
+
 # ------------------------------------------------------------------ vocabulary shortlist
 @pytest.mark.parametrize("B,S,V,C,TC,HN,RN,K", [(3, 7, 96, 8, 2, 4, 4, 16), (4, 33, 2048, 64, 2, 32, 32, 128),
                                                 (2, 5, 50, 7, 3, 60, 0, 50), (2, 9, 4096, 64, 1, 0, 8, 256)])
