@@ -552,12 +552,15 @@ int rte_transpose_f32(const float* src, void* dst, int32_t rows, int32_t cols, i
  * cand_count int32 [rows] optional.  max(up_m, gate_m, product_m) >= top_k is required; wd_norm is not negative; hats
  * and wd_norm start on 16 bytes, ug and z_masked on 8, selected on 4 (RTE_ERR_ALIGNMENT otherwise).
  * rte_svd_ffn_swiglu_bwd: dug bf16 [rows, 2F] = SwiGLU backward of dz bf16 [rows, F] on selected neurons, else 0.
+ * rte_svd_ffn_hidden_bwd: the product that makes dz and that pass in one launch, rounded like the two (args as for
+ * rte_gemm_bf16_swiglu_bwd_selected, which keeps dz in fp32; the same RTE_ERR_UNSUPPORTED).
  * rte_row_norm_f32: out[r] = ||w[r, :]||_2.                                                                    */
 int rte_svd_ffn_select(const float* hats, const void* ug, const float* wd_norm, void* z_masked, uint8_t* selected,
                        int32_t* cand_count, int32_t rows, int32_t F, int32_t up_m, int32_t gate_m, int32_t product_m,
                        int32_t top_k, rte_stream_t stream);
 int rte_svd_ffn_swiglu_bwd(const void* ug, const void* dz, const uint8_t* selected, void* dug, int64_t rows, int32_t F,
                            rte_stream_t stream);
+int rte_svd_ffn_hidden_bwd(const rte_gemm_args* args, const uint8_t* selected, rte_stream_t stream);
 int rte_row_norm_f32(const float* w, float* out, int32_t rows, int32_t d, rte_stream_t stream);
 
 /* ------------------------------------------------ offline cluster-pool codebook build (cli.py:3297-3389, 4703-4782)

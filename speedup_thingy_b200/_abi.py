@@ -172,6 +172,7 @@ PROTOTYPES = {
     "rte_csr_row_reduce_f32": (C.c_int, [c_vp, c_vp, c_vp, c_vp, c_i64, c_i32, c_i32, c_vp]),
     "rte_transpose_f32": (C.c_int, [c_vp, c_vp, c_i32, c_i32, c_i32, c_i32, c_vp]),
     "rte_svd_ffn_select": (C.c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_i32, c_i32, c_i32, c_i32, c_i32, c_i32, c_vp]),
+    "rte_svd_ffn_hidden_bwd": (C.c_int, [P(GemmArgs), c_vp, c_vp]),
     "rte_svd_ffn_swiglu_bwd": (C.c_int, [c_vp, c_vp, c_vp, c_vp, c_i64, c_i32, c_vp]),
     "rte_row_norm_f32": (C.c_int, [c_vp, c_vp, c_i32, c_i32, c_vp]),
     "rte_residual_rmsnorm_fwd": (C.c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_i32, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp, c_vp,

@@ -66,6 +66,7 @@ struct KParams {
   const int* split_kb;      // ragged split-K: k-block range [split_kb[s], split_kb[s+1]) of split s, else null
   int* status;
   const uint8_t* selected;  // MASK: [M, N] bytes, 0 where the gradient is zero; else null
+  int as_two;               // MASK: the bits of a product with a bf16 result and the pass behind it (svd_ffn.cu)
 };
 
 // ------------------------------------------------------------------ epilogue helpers
@@ -420,11 +421,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
               ld_shared_v4(slot2 + at, g[4 * c], g[4 * c + 1], g[4 * c + 2], g[4 * c + 3]);
             }
             tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
+            auto form = [&](int j, float dz0, float dz1, float s0, float s1) {
               const float2 u_ = rte::unpack_bf16x2(u[j]), g_ = rte::unpack_bf16x2(g[j]);
-              const float dz0 = __uint_as_float(raw[2 * j]), dz1 = __uint_as_float(raw[2 * j + 1]);
-              const float s0 = fast_sigmoid(g_.x), s1 = fast_sigmoid(g_.y);
               float du0 = dz0 * g_.x * s0, du1 = dz1 * g_.y * s1;
               float dg0 = dz0 * u_.x * s0 * (1.f + g_.x * (1.f - s0)), dg1 = dz1 * u_.y * s1 * (1.f + g_.y * (1.f - s1));
               if constexpr (MASK) {
@@ -434,6 +432,20 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
               }
               u[j] = rte::pack_bf16x2(du0, du1);
               g[j] = rte::pack_bf16x2(dg0, dg1);
+            };
+            if (MASK && p.as_two) {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const float2 dz = rte::unpack_bf16x2(rte::pack_bf16x2(__uint_as_float(raw[2 * j]), __uint_as_float(raw[2 * j + 1])));
+                const float2 g_ = rte::unpack_bf16x2(g[j]);
+                form(j, dz.x, dz.y, rte::sigmoid_rn(g_.x), rte::sigmoid_rn(g_.y));
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) {
+                const float2 g_ = rte::unpack_bf16x2(g[j]);
+                form(j, __uint_as_float(raw[2 * j]), __uint_as_float(raw[2 * j + 1]), fast_sigmoid(g_.x), fast_sigmoid(g_.y));
+              }
             }
 #pragma unroll
             for (uint32_t c = 0; c < 4; ++c) {
@@ -893,7 +905,7 @@ extern "C" int rte_gemm_wgrad_splits(const rte_gemm_args* a, int32_t max_splits)
 
 namespace {
 // `selected` (SwiGLU's backward only): RTE_ERR_UNSUPPORTED where the epilogue that takes it does not serve
-int run_gemm(const rte_gemm_args* a, const uint8_t* selected, rte_stream_t stream) {
+int run_gemm(const rte_gemm_args* a, const uint8_t* selected, bool as_two, rte_stream_t stream) {
   RTE_CHECK_ARG(a != nullptr && a->A && a->B && a->C);
   RTE_CHECK_ARG(a->M > 0 && a->N > 0 && a->K > 0);
   RTE_CHECK_ARG(a->epilogue >= RTE_EPI_BF16 && a->epilogue <= RTE_EPI_SWIGLU_BWD);
@@ -933,6 +945,7 @@ int run_gemm(const rte_gemm_args* a, const uint8_t* selected, rte_stream_t strea
   kp.kblocks_per_split = rte::ceil_div(kp.kblocks_total, splits);
   kp.status = a->status;
   kp.selected = selected;
+  kp.as_two = as_two ? 1 : 0;
   kp.tile_group = a->tile_group;
   kp.b_group_stride = a->b_group_stride;
   kp.split_kb = a->split_kblocks;
@@ -1017,9 +1030,14 @@ int run_gemm(const rte_gemm_args* a, const uint8_t* selected, rte_stream_t strea
 }
 }  // namespace
 
-extern "C" int rte_gemm_bf16(const rte_gemm_args* a, rte_stream_t stream) { return run_gemm(a, nullptr, stream); }
+extern "C" int rte_gemm_bf16(const rte_gemm_args* a, rte_stream_t stream) { return run_gemm(a, nullptr, false, stream); }
 
 extern "C" int rte_gemm_bf16_swiglu_bwd_selected(const rte_gemm_args* a, const uint8_t* selected, rte_stream_t stream) {
   RTE_CHECK_ARG(a != nullptr && selected != nullptr && a->epilogue == RTE_EPI_SWIGLU_BWD);
-  return run_gemm(a, selected, stream);
+  return run_gemm(a, selected, false, stream);
+}
+
+extern "C" int rte_svd_ffn_hidden_bwd(const rte_gemm_args* a, const uint8_t* selected, rte_stream_t stream) {
+  RTE_CHECK_ARG(a != nullptr && selected != nullptr && a->epilogue == RTE_EPI_SWIGLU_BWD);
+  return run_gemm(a, selected, true, stream);
 }

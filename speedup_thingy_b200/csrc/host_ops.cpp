@@ -689,14 +689,16 @@ struct SvdModule {
     TORCH_CHECK_VALUE(flat.size(0) == N, "the gradient of ", N, " tokens has ", flat.size(0), " rows");
     is_dense_f32(dw_down, dout, F * d, "dw_down");
     cast_into(dev, flat, dout16.narrow(0, 0, N));
-    // d z stays in the product's accumulators where its epilogue takes the mask: two passes over [N, F] less.  16384 x 512 x 2048, forward and backward:
-    // 714 -> 687 us, 8192 x 1024 x 4096 959 -> 928, 2048 x 512 x 2048 179 -> 177; 512 x 2048 neurons and fewer are even.
+    // Where the product's epilogue takes the mask, d z does not go through memory: two passes over [N, F] less, and the bits of the two launches
+    // (d z rounded to bf16, the same divide), so that a gradient does not depend on which of them its size takes.
+    // us, two launches -> one: 16384 x 2048 x 512 101.5 -> 84.6, 8192 x 4096 x 1024 121.4 -> 95.0, 8192 x 2048 x 512 55.8 -> 50.9, 2048 x 2048 x 512 18.5 -> 17.9,
+    // 5000 x 1536 x 384 26.5 -> 28.1 (d z stays in L2 there), 512 x 2048 x 512 9.7 -> 9.1.
     int rc = RTE_ERR_UNSUPPORTED;
     if (N * F >= rte_swiglu_fuse_min(1)) {
       Gemm fused(dev, ptr(dout16), d, false, ptr(wd16), d, false, ptr(dug), 2 * F, N, F, d, RTE_EPI_SWIGLU_BWD);
       fused.residual(ptr(ug), 2 * F).pair(nullptr, 0, F);
-      rc = rte_gemm_bf16_swiglu_bwd_selected(&fused.a, static_cast<uint8_t*>(ptr(selected)), dev.st);
-      if (rc != RTE_ERR_UNSUPPORTED) check(rc, "rte_gemm_bf16_swiglu_bwd_selected");
+      rc = rte_svd_ffn_hidden_bwd(&fused.a, static_cast<uint8_t*>(ptr(selected)), dev.st);
+      if (rc != RTE_ERR_UNSUPPORTED) check(rc, "rte_svd_ffn_hidden_bwd");
     }
     if (rc == RTE_ERR_UNSUPPORTED) {
       Gemm(dev, ptr(dout16), d, false, ptr(wd16), d, false, ptr(dz), F, N, F, d, RTE_EPI_BF16).run();

@@ -101,6 +101,20 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 __device__ __forceinline__ float silu_f(float g) { return g / (1.f + __expf(-g)); }
 __device__ __forceinline__ float sigmoid_f(float g) { return 1.f / (1.f + __expf(-g)); }
 
+// The bits of sigmoid_f without the branches of its divide, for epilogues: an approximate reciprocal, then a Newton step with fused
+// multiply-adds, after which it is correctly rounded (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990).  A quarter of the denominator keeps the approximation out of the range that it flushes; the maximum takes
+// the place of infinity * 0.  Compared with sigmoid_f for all 2^32 arguments.
+__device__ __forceinline__ float quarter_rcp(float y) {          // about 1 / y
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(0.25f * y));
+  return 0.25f * r;
+}
+__device__ __forceinline__ float sigmoid_rn(float g) {
+  const float y = 1.f + __expf(-g), r = quarter_rcp(y);
+  return __fmaf_rn(fmaxf(__fmaf_rn(-y, r, 1.f), -1.f), r, r);
+}
+
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);

@@ -765,6 +765,33 @@ def test_gemm_swiglu_bwd_of_selected_neurons(ops, M, F_, K):
     assert fn(C.byref(args(got, saved)), sel.data_ptr() + 1, ops.stream) == A.ERR_UNSUPPORTED
 
 
+@pytest.mark.parametrize("M,F_,K", [(1, 16, 8), (130, 80, 64), (520, 272, 72), (2100, 1040, 136), (2048, 2048, 512)])
+def test_svd_hidden_backward_has_the_bits_of_the_two_launches(ops, M, F_, K):
+    """The product that forms SwiGLU's backward of the selected neurons against the product and the pass behind it.  Integer operands, so
+    that d z is exact before it is rounded, whatever the order of its sum; among the gates all bf16 numbers (as far as they fit)."""
+    g = torch.Generator().manual_seed(M + K)
+    dy, w = (torch.randint(-8, 9, (n, K), generator=g).bfloat16().to(DEV) for n in (M, F_))
+    sel = (torch.rand(M, F_, generator=g) < 0.5).to(torch.uint8).to(DEV)
+    ug = torch.randn(M, 2 * F_, generator=g).bfloat16()
+    n = min(M * F_, 65536)
+    gates = (torch.arange(n, dtype=torch.int32) * (65536 // n)).to(torch.int16).view(torch.bfloat16)
+    ug[:, F_:].copy_(gates.repeat(-(-M * F_ // n))[: M * F_].view(M, F_))
+    ug = ug.to(DEV)
+    dz = torch.empty(M, F_, dtype=torch.bfloat16, device=DEV)
+    want, got = (torch.full((M, 2 * F_), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    ops.gemm(dy, w, dz, M=M, N=F_, K=K)
+    ops.svd_ffn_swiglu_bwd(ug, dz, sel, want)
+    a = A.GemmArgs()
+    a.A, a.B, a.C, a.R, a.status = dy.data_ptr(), w.data_ptr(), got.data_ptr(), ug.data_ptr(), ops.status.data_ptr()
+    a.M, a.N, a.K, a.lda, a.ldb, a.ldc, a.ldr = M, F_, K, K, K, 2 * F_, 2 * F_
+    a.epilogue, a.splits, a.b_pair_offset = A.EPI_SWIGLU_BWD, 1, F_
+    A.check(ops.lib.rte_svd_ffn_hidden_bwd(C.byref(a), sel.data_ptr(), ops.stream), "rte_svd_ffn_hidden_bwd")
+    ops.check_status()
+    assert torch.equal(want.isnan(), got.isnan())
+    keep = ~want.isnan()
+    assert torch.equal(want.view(torch.int16)[keep], got.view(torch.int16)[keep])
+
+
 @pytest.mark.parametrize("dtype,rows,V,off", [("f32", 3, 4096, 0), ("f32", 5, 4100, 0), ("f32", 3, 4093, 1), ("f32", 7, 9001, 3), ("bf16", 3, 8192, 0),
                                               ("bf16", 5, 8200, 0), ("bf16", 3, 8187, 5), ("bf16", 600, 12345, 0)])
 def test_ce_gradient_from_kept_sums(ops, dtype, rows, V, off):

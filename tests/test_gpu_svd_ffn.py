@@ -169,6 +169,26 @@ def test_c4_shaped_module_against_the_oracle():
     assert (sel & sel32).sum() >= 0.93 * sel32.sum()
 
 
+@pytest.mark.parametrize("N,F_", [(300, 512), (700, 2048), (513, 2064)])          # below and above a million activations
+def test_module_backward_rounds_like_the_two_launches_at_every_size(N, F_):
+    """Whichever route the size takes, the hidden gradients are those of the product with a bf16 result and the masked SwiGLU pass.  Integer
+    gradients and down weights: d z is exact before it is rounded."""
+    d, r, k = 128, 16, 40
+    g = torch.Generator().manual_seed(N)
+    rn = lambda *s: torch.randn(*s, generator=g) * 0.1  # noqa: E731
+    w_down = torch.randint(-8, 9, (F_, d), generator=g).float()
+    t = dict(w_up=rn(F_, d), w_gate=rn(F_, d), w_down=w_down, up_a=rn(d, r), up_b=rn(r, F_), gate_a=rn(d, r), gate_b=rn(r, F_))
+    m = _module(t, dict(top_k=k, up_m=k, gate_m=k, product_m=k), N)
+    m.forward(torch.randn(N, d, generator=g).to(DEV))
+    dout = torch.randint(-8, 9, (N, d), generator=g).float().to(DEV)
+    m.backward(dout, *(torch.empty(F_, d, device=DEV) for _ in range(3)))
+    dz, want = torch.empty(N, F_, dtype=torch.bfloat16, device=DEV), torch.empty(N, 2 * F_, dtype=torch.bfloat16, device=DEV)
+    m.ops.gemm(dout.bfloat16(), m.wd16, dz, M=N, N=F_, K=d)
+    m.ops.svd_ffn_swiglu_bwd(m.ug[:N], dz, m.selected[:N], want)
+    m.ops.check_status()
+    assert torch.equal(m.dug[:N], want)
+
+
 def test_what_the_buffers_cannot_hold_is_refused_before_a_launch():
     c, t = SVD_FFN, svd_ffn_inputs()
     m = _module(t, c, 64)
