@@ -101,10 +101,11 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 __device__ __forceinline__ float silu_f(float g) { return g / (1.f + __expf(-g)); }
 __device__ __forceinline__ float sigmoid_f(float g) { return 1.f / (1.f + __expf(-g)); }
 
-// The bits of sigmoid_f without the branches of its divide, for epilogues: an approximate reciprocal, then a Newton step with fused
-// multiply-adds, after which it is correctly rounded (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", 1990).  A quarter of the denominator keeps the approximation out of the range that it flushes; the maximum takes
-// the place of infinity * 0.  Compared with sigmoid_f for all 2^32 arguments.
+// The bits of sigmoid_f and silu_f without the branches of their divide: an approximate reciprocal, then a step with fused multiply-adds
+// that corrects the quotient by its remainder (P. Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990).  A quarter of the denominator keeps the approximation out of the range that it flushes; maximum and minimum
+// take the place of infinity * 0.  Compared with sigmoid_f for all 2^32 arguments; silu_of_bf16 with silu_f for all bf16 ones
+// (of the others, two of 2^32 differ in the last bit).
 __device__ __forceinline__ float quarter_rcp(float y) {          // about 1 / y
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(0.25f * y));
@@ -113,6 +114,10 @@ __device__ __forceinline__ float quarter_rcp(float y) {          // about 1 / y
 __device__ __forceinline__ float sigmoid_rn(float g) {
   const float y = 1.f + __expf(-g), r = quarter_rcp(y);
   return __fmaf_rn(fmaxf(__fmaf_rn(-y, r, 1.f), -1.f), r, r);
+}
+__device__ __forceinline__ float silu_of_bf16(float g) {
+  const float y = 1.f + __expf(-g), r = quarter_rcp(y), q = g * r;
+  return __fmaf_rn(-fminf(__fmaf_rn(y, q, -g), 3.40282347e38f), r, q);
 }
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {

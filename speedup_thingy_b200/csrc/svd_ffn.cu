@@ -15,12 +15,11 @@
 // half (a row of equal scores), the search goes on over the full scores.  Results are bit-exact with a stable sort by (value
 // descending, index ascending), the tie rule of this build.
 //
-// What bounds it: the issue slots, 57 % of them used by 9.3 K instructions per token (24 warps on an SM, 9 KB of shared memory each;
-// per instruction issued 3.1 warps wait on global loads, 1.9 on fixed latencies, 0.7 on shared memory).  us, with 32-bit keys and an
-// IEEE divide in the SiLU -> now: 16384 tokens, F = 2048, k = 256 375 -> 249, 5000 x 2000, k = 200 168 -> 107, 3000 x 512, k = 60
-// 41 -> 26 (of the first: 375 -> 345 by the keys, -> 271 by the divide, -> 249 by probes that aim past k and a better first guess:
-// 20 -> 12 probes per token).  With all keys in registers and the three lists searched together it took 583: the unrolled code
-// does not stay in the instruction cache.
+// What bounds it: the instructions of a token, waited for by the loads of its scores (24 warps on an SM, 9 KB of shared memory each).
+// us, with 32-bit keys and a divide for every list -> now: 16384 tokens, F = 2048, k = 256 377 -> 271, 5000 x 2000, k = 200
+// 172 -> 165, 3000 x 512, k = 60 44 -> 27.  The SiLU of the fp32 lists is the correctly rounded quotient, made once for two lists (302 us
+// with a divide for each, 245 with an approximate reciprocal, which loses the order of gates below -87).  With all keys in
+// registers and the three lists searched together it took 583: the unrolled code does not stay in the instruction cache.
 
 #include "rte_common.cuh"
 
@@ -39,15 +38,6 @@ __device__ __forceinline__ uint32_t pair_keys(float a, float b) {
 __device__ __forceinline__ float key_value(uint32_t t) { return __uint_as_float((t - KEY_MIN) << 16); }
 __device__ __forceinline__ __nv_bfloat162 as_pair(uint32_t v) { return *reinterpret_cast<__nv_bfloat162*>(&v); }
 
-// g / (1 + exp(-g)) in five instructions (an IEEE divide takes twenty, and there are three of these per neuron): within 3 ulp, like the
-// exp alone, where the scores and the bf16 z that come of it keep 8 bits; exp(-g) = infinity gives -0, as the divide does.
-__device__ __forceinline__ float silu(float g) {
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * -1.4426950408889634f));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
-  return g * r;
-}
-
 // per warp: the keys of one selection, the exact z as bf16, candidate | selected bits per four neurons, the ranking list
 __host__ __device__ constexpr int sel_pad(int F) { return (F + 7) / 8 * 8; }
 __host__ __device__ constexpr size_t sel_list_offset(int F) { return ((size_t)sel_pad(F) * 4 + (size_t)sel_pad(F) / 4 + 15) / 16 * 16; }
@@ -61,9 +51,9 @@ struct Token { const float* hat; const __nv_bfloat16* ug; const float* wn; int F
 __device__ __forceinline__ int full_score(const Token& x, int which, int i) {
   float v;
   if (which == 0) v = x.hat[i];
-  else if (which == 1) v = silu(x.hat[x.F + i]);
-  else if (which == 2) v = x.hat[i] * silu(x.hat[x.F + i]);
-  else v = __bfloat162float(x.ug[i]) * silu(__bfloat162float(x.ug[x.F + i]));
+  else if (which == 1) v = rte::silu_f(x.hat[x.F + i]);
+  else if (which == 2) v = x.hat[i] * rte::silu_f(x.hat[x.F + i]);
+  else v = __bfloat162float(x.ug[i]) * rte::silu_of_bf16(__bfloat162float(x.ug[x.F + i]));
   return __float_as_int(fabsf(v) * x.wn[i]);
 }
 
@@ -221,7 +211,7 @@ svd_select_kernel(const float* __restrict__ hats, const __nv_bfloat16* __restric
   const float4* wn4 = reinterpret_cast<const float4*>(wn);
   Guess* guess = reinterpret_cast<Guess*>(list + SEL_LIST + 4);
   if (lane < 4) guess[lane] = Guess{0, 0.f};
-  if (lane == 0 && n4 < 2 * n8) key[n4] = make_uint2(0u, 0u);        // (the padding of an odd number of groups: no candidates)
+  if (lane == 0 && n4 < 2 * n8) key[n4] = z4[n4] = make_uint2(0u, 0u);      // (the padding of an odd number of groups: no candidates)
   __syncwarp();
   for (int row = blockIdx.x * warps + warp; row < rows; row += gridDim.x * warps) {
     const Token tok = {hats + (size_t)row * 2 * F, ug + (size_t)row * 2 * F, wn, F};
@@ -233,30 +223,25 @@ svd_select_kernel(const float* __restrict__ hats, const __nv_bfloat16* __restric
       prefetch_l2(ug + (size_t)next * 2 * F, 4 * F, lane);
     }
     // --- three candidate lists
-    auto take = [&](int k, int which) {
+    auto take = [&](const uint4* keys, int k, int which) {
       __syncwarp();
       if (k >= F) { for (int i = lane; i < n8; i += 32) flags16[i] |= 0x0f0fu; }
-      else if (k > 0) warp_take(k8, n8, k, F, guess + which, list, flags16, 0, tok, which, lane);
+      else if (k > 0) warp_take(keys, n8, k, F, guess + which, list, flags16, 0, tok, which, lane);
       __syncwarp();
     };
     for (int i = lane; i < n8; i += 32) flags16[i] = 0;
     for_groups<4>(uh, uh, wn4, n4, lane, [&](int i, float4 u, float4, float4 w) {
       key[i] = make_uint2(pair_keys(fabsf(u.x) * w.x, fabsf(u.y) * w.y), pair_keys(fabsf(u.z) * w.z, fabsf(u.w) * w.w));
     });
-    take(up_m, 0);
-    if (gate_m > 0) {
-      for_groups<4>(gh, gh, wn4, n4, lane, [&](int i, float4 g, float4, float4 w) {
-        key[i] = make_uint2(pair_keys(fabsf(silu(g.x)) * w.x, fabsf(silu(g.y)) * w.y),
-                            pair_keys(fabsf(silu(g.z)) * w.z, fabsf(silu(g.w)) * w.w));
-      });
-      take(gate_m, 1);
-    }
-    if (product_m > 0) {
+    take(k8, up_m, 0);
+    if (gate_m > 0 || product_m > 0) {                // one divide per gate: the products' keys lie where z will
       for_groups<2>(uh, gh, wn4, n4, lane, [&](int i, float4 u, float4 g, float4 w) {
-        key[i] = make_uint2(pair_keys(fabsf(u.x * silu(g.x)) * w.x, fabsf(u.y * silu(g.y)) * w.y),
-                            pair_keys(fabsf(u.z * silu(g.z)) * w.z, fabsf(u.w * silu(g.w)) * w.w));
+        g = make_float4(rte::silu_f(g.x), rte::silu_f(g.y), rte::silu_f(g.z), rte::silu_f(g.w));
+        key[i] = make_uint2(pair_keys(fabsf(g.x) * w.x, fabsf(g.y) * w.y), pair_keys(fabsf(g.z) * w.z, fabsf(g.w) * w.w));
+        z4[i] = make_uint2(pair_keys(fabsf(u.x * g.x) * w.x, fabsf(u.y * g.y) * w.y), pair_keys(fabsf(u.z * g.z) * w.z, fabsf(u.w * g.w) * w.w));
       });
-      take(product_m, 2);
+      take(k8, gate_m, 1);
+      take(reinterpret_cast<const uint4*>(z4), product_m, 2);
     }
     // --- exact re-rank over the candidates
     const uint2* up = reinterpret_cast<const uint2*>(tok.ug);
@@ -264,7 +249,7 @@ svd_select_kernel(const float* __restrict__ hats, const __nv_bfloat16* __restric
     for_groups<2>(up, up + n4, wn4, n4, lane, [&](int i, uint2 u, uint2 g, float4 w) {
       const float2 u0 = rte::unpack_bf16x2(u.x), u1 = rte::unpack_bf16x2(u.y), g0 = rte::unpack_bf16x2(g.x), g1 = rte::unpack_bf16x2(g.y);
       const uint32_t m = flags[i];
-      const float z0 = u0.x * silu(g0.x), z1 = u0.y * silu(g0.y), z2 = u1.x * silu(g1.x), z3 = u1.y * silu(g1.y);
+      const float z0 = u0.x * rte::silu_of_bf16(g0.x), z1 = u0.y * rte::silu_of_bf16(g0.y), z2 = u1.x * rte::silu_of_bf16(g1.x), z3 = u1.y * rte::silu_of_bf16(g1.y);
       n_cand += __popc(m);
       key[i] = make_uint2(pair_keys(fabsf(z0) * w.x, fabsf(z1) * w.y) & ((m & 1u) * 0xffffu | (m & 2u) * 0x7fff8000u),
                           pair_keys(fabsf(z2) * w.z, fabsf(z3) * w.w) & ((m >> 2 & 1u) * 0xffffu | (m >> 2 & 2u) * 0x7fff8000u));

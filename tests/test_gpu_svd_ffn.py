@@ -84,6 +84,37 @@ def test_scores_that_share_their_upper_bits(rows, F_, k):
     assert torch.equal(sel.cpu().bool(), O.topk_membership(order, k))
 
 
+def test_z_of_every_gate_has_the_bits_of_the_swiglu_pass():
+    """Everything selected: z over all 65536 bf16 gates against rte_swiglu_fwd, whose divide rounds correctly.  Gates from -88.7 to
+    -87.3 among them, whose denominators are above 2^126."""
+    ops = CudaOps(DEV)
+    F_ = 2048
+    gate = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16).view(32, F_)
+    ups = torch.randn(3, F_, generator=torch.Generator().manual_seed(0)).bfloat16()
+    ug = torch.cat([torch.cat([torch.full_like(u, 1.0) * u for u in ups.unsqueeze(1).expand(3, 32, F_)]), gate.repeat(3, 1)], dim=1).to(DEV)
+    z, want = (torch.empty(96, F_, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    ops.svd_ffn_select(torch.ones(96, 2 * F_, device=DEV), ug, torch.ones(F_, device=DEV), z, None, None, up_m=F_, gate_m=0, product_m=0, top_k=F_)
+    ops.swiglu_fwd(ug, want, 96, F_)
+    assert torch.equal(z.isnan(), want.isnan())
+    keep = ~want.isnan()
+    assert torch.equal(z.view(torch.int16)[keep], want.view(torch.int16)[keep])
+
+
+@pytest.mark.parametrize("gate_m,product_m", [(20, 0), (0, 20)])
+def test_scores_of_gates_far_below_zero_keep_their_order(gate_m, product_m):
+    """Gates whose exp(-gate) is finite and above 2^126: |silu| shrinks by at least 1 % from one to the next, so the largest are known."""
+    ops = CudaOps(DEV)
+    rows, F_ = 40, 128
+    place = torch.stack([torch.randperm(F_, generator=torch.Generator().manual_seed(i)) for i in range(rows)])
+    gate = (-87.4 - 0.01 * torch.arange(F_)).expand(rows, F_).gather(1, place)
+    hats = torch.cat([torch.full((rows, F_), 2.0), gate], dim=1).to(DEV)
+    ug = torch.ones(rows, 2 * F_, dtype=torch.bfloat16, device=DEV)
+    z, sel = torch.empty(rows, F_, dtype=torch.bfloat16, device=DEV), torch.empty(rows, F_, dtype=torch.uint8, device=DEV)
+    ops.svd_ffn_select(hats, ug, torch.ones(F_, device=DEV), z, sel, None, up_m=0, gate_m=gate_m, product_m=product_m, top_k=20)
+    ops.check_status()
+    assert torch.equal(sel.cpu().bool(), place < 20)
+
+
 @pytest.mark.parametrize("rows,F_", [(37, 2048), (5, 100)])            # eight neurons per thread | one
 def test_swiglu_backward_of_the_selected_neurons(rows, F_):
     ops = CudaOps(DEV)
