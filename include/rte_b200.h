@@ -119,6 +119,8 @@ int rte_gemm_bf16_swiglu_bwd_selected(const rte_gemm_args* args, const uint8_t* 
 int rte_gemm_wgrad_splits(const rte_gemm_args* args, int32_t max_splits);
 /* Hidden activations (rows x F) from which a SwiGLU epilogue (forward | backward) is faster than a plain product and a pass. */
 int64_t rte_swiglu_fuse_min(int32_t backward);
+/* The same for SwiGLU's forward behind a reduction of length K.                                                       */
+int64_t rte_swiglu_fuse_min_fwd(int32_t K);
 /* The same product for FEW TILES: one 128 x tile_n tile per CTA (tile_n 64 or 128), the reduction split over the `ksplit`
  * (1..8, at most one per 64-wide k-block) CTAs of a cluster, which add their partial tiles in rank order.  RTE_EPI_BF16 or
  * RTE_EPI_F32 (+R); no grouping, no splits; either major for either operand.                                       */

@@ -116,6 +116,7 @@ PROTOTYPES = {
     "rte_ce_fwd_bwd_f32": (C.c_int, [c_vp, c_i32, c_vp, c_vp, c_i32, c_vp, c_vp, c_i32, c_i32, c_vp, c_vp]),
     "rte_host_randint": (C.c_int, [C.c_uint64, c_i64, C.c_int32, c_vp]),
     "rte_swiglu_fuse_min": (c_i64, [c_i32]),
+    "rte_swiglu_fuse_min_fwd": (c_i64, [c_i32]),
     "rte_gemm_wgrad_splits": (C.c_int, [P(GemmArgs), C.c_int32]),
     "rte_reduce_splits": (C.c_int, [c_vp, c_i32, c_i64, c_i64, c_vp, c_i32, c_vp]),
     "rte_embed_fwd": (C.c_int, [c_vp, c_vp, c_vp, c_i32, c_i32, c_i32, c_vp, c_vp]),

@@ -53,7 +53,8 @@ struct ResidentParams {
   int* status;
 };
 
-template <int EPI>
+// EXACT: z has the bits of the separate pass (rte_swiglu_fwd), else those of the persistent kernel's epilogue.
+template <int EPI, bool EXACT>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_c,
                      const ResidentParams p) {
@@ -220,7 +221,8 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           const float2 u = rte::unpack_bf16x2(v0[j]), g = rte::unpack_bf16x2(v1[j]);
-          v0[j] = rte::pack_bf16x2(u.x * (g.x * fast_sigmoid(g.x)), u.y * (g.y * fast_sigmoid(g.y)));
+          v0[j] = EXACT ? rte::pack_bf16x2(u.x * rte::silu_of_bf16(g.x), u.y * rte::silu_of_bf16(g.y))
+                        : rte::pack_bf16x2(u.x * (g.x * fast_sigmoid(g.x)), u.y * (g.y * fast_sigmoid(g.y)));
         }
         by_row(p.C + size_t(row) * p.ldc + col, v0);
       } else {
@@ -251,11 +253,11 @@ int resident_stages(int epi, int kblocks) {
   return fit < MAX_STAGES ? fit : MAX_STAGES;
 }
 
-template <int EPI>
+template <int EPI, bool EXACT>
 int max_pairs(int sms) {
   static int pairs = 0;
   if (pairs > 0) return pairs;
-  if (cudaFuncSetAttribute(gemm_resident_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, resident_smem(EPI, MAX_KB, resident_stages(EPI, MAX_KB))) != cudaSuccess)
+  if (cudaFuncSetAttribute(gemm_resident_kernel<EPI, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize, resident_smem(EPI, MAX_KB, resident_stages(EPI, MAX_KB))) != cudaSuccess)
     return 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(sms / 2 * 2));
@@ -266,7 +268,7 @@ int max_pairs(int sms) {
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr; cfg.numAttrs = 1;
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, gemm_resident_kernel<EPI>, &cfg) == cudaSuccess && n > 0) pairs = n;
+  if (cudaOccupancyMaxActiveClusters(&n, gemm_resident_kernel<EPI, EXACT>, &cfg) == cudaSuccess && n > 0) pairs = n;
   else { (void)cudaGetLastError(); pairs = sms / 2; }
   return pairs;
 }
@@ -283,7 +285,7 @@ int store_tmap(CUtensorMap* map, const void* base, long long rows, long long col
   return r == CUDA_SUCCESS ? RTE_OK : RTE_ERR_TENSOR_MAP;
 }
 
-template <int EPI>
+template <int EPI, bool EXACT>
 int launch_resident(const rte_gemm_args* a, int ctas, cudaStream_t st) {
   ResidentParams p;
   p.M = a->M; p.N = a->N; p.b_mn = a->b_mn_major ? 1 : 0; p.pair_off = a->b_pair_offset;
@@ -302,7 +304,7 @@ int launch_resident(const rte_gemm_args* a, int ctas, cudaStream_t st) {
   CUtensorMap tc = ta;
   if (EPI == RTE_EPI_BF16) rc = store_tmap(&tc, a->C, a->M, a->N, a->ldc);
   if (rc != RTE_OK) return rc;
-  const int sms = rte_device_sm_count(), fit = max_pairs<EPI>(sms);
+  const int sms = rte_device_sm_count(), fit = max_pairs<EPI, EXACT>(sms);
   int pairs = ctas / 2 < fit ? ctas / 2 : fit;
   const long long tiles = (long long)p.m_blocks * p.n_blocks;
   if (tiles < pairs) pairs = int(tiles);
@@ -318,7 +320,7 @@ int launch_resident(const rte_gemm_args* a, int ctas, cudaStream_t st) {
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim.x = 2; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr; cfg.numAttrs = 2;
-  if (cudaLaunchKernelEx(&cfg, gemm_resident_kernel<EPI>, ta, tb, tc, p) != cudaSuccess) {
+  if (cudaLaunchKernelEx(&cfg, gemm_resident_kernel<EPI, EXACT>, ta, tb, tc, p) != cudaSuccess) {
     (void)cudaGetLastError();
     return RTE_ERR_LAUNCH;
   }
@@ -337,8 +339,10 @@ extern "C" int rte_gemm_bf16_resident(const rte_gemm_args* a, int32_t ctas, rte_
       a->ldb % 8 || a->ldc % 16)
     return RTE_ERR_ALIGNMENT;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (a->epilogue == RTE_EPI_BF16) return launch_resident<RTE_EPI_BF16>(a, ctas, st);
+  if (a->epilogue == RTE_EPI_BF16) return launch_resident<RTE_EPI_BF16, false>(a, ctas, st);
   RTE_CHECK_ARG(a->C2 != nullptr && a->b_pair_offset > 0 && a->b_pair_offset % 32 == 0 && a->N == 2 * a->b_pair_offset && !a->b_mn_major);
   if ((reinterpret_cast<uintptr_t>(a->C2) & 31) || a->ldc2 % 16) return RTE_ERR_ALIGNMENT;
-  return launch_resident<RTE_EPI_SWIGLU_FWD>(a, ctas, st);
+  // z by the bits of the route that a caller would otherwise take: the separate pass below the persistent kernel's line, that kernel above
+  if ((long long)a->M * a->b_pair_offset < rte_swiglu_fuse_min(0)) return launch_resident<RTE_EPI_SWIGLU_FWD, true>(a, ctas, st);
+  return launch_resident<RTE_EPI_SWIGLU_FWD, false>(a, ctas, st);
 }

@@ -881,10 +881,17 @@ extern "C" int rte_device_sm_count(void) {
   return n;
 }
 
-// us, separate -> fused: forward 8192 x 512 -> 2048 50.2 -> 39.6, 5000 x 384 -> 1536 24.7 -> 21.4, 2048 x 1024 -> 2048 23.4 -> 22.8, 1024 x
-// 512 -> 2048 11.4 -> 10.1; 2048 x 1024 -> 1024 14.5 -> 15.5, 512 x 512 -> 2048 8.4 -> 9.1, 512 x 128 -> 512 5.2 -> 7.3; backward (its operands come by TMA, so it pays earlier) 8192 x 512 ->
-// 2048 53.7 -> 37.3, 8192 x 256 -> 1024 20.8 -> 17.3, 1000 x 256 -> 1024 7.8 -> 6.7; 512 x 128 -> 512 4.9 -> 6.0
-extern "C" int64_t rte_swiglu_fuse_min(int32_t backward) { return backward ? 1000000 : 4000000; }
+// us, separate -> fused.  Forward in the persistent kernel: 4096 x 576 -> 1152 19.4 -> 20.7, 8192 x 640 -> 512 20.3 -> 21.7, 4096 x 640 -> 1536 26.3 ->
+// 26.5, 3000 x 768 -> 1536 21.3 -> 21.6, 8192 x 512 -> 1024 30.3 -> 31.3, 8192 x 512 -> 2048 53.8 -> 46.0 (with K = 1024 it would pay from 4 M: 4096 x 1024
+// -> 2048 40.1 -> 34.3, but its z is not the separate pass's to the last bit, and with the exact quotient 4096 x 768 -> 1536 takes
+// 30.7 against 28.4).  Backward (its operands come by TMA, so it pays
+// earlier) 8192 x 512 -> 2048 53.7 -> 37.3, 8192 x 256 -> 1024 20.8 -> 17.3, 1000 x 256 -> 1024 7.8 -> 6.7; 512 x 128 -> 512 4.9 -> 6.0
+extern "C" int64_t rte_swiglu_fuse_min(int32_t backward) { return backward ? 1000000 : 12000000; }
+
+// The kernel that keeps A in shared memory (gemm_resident.cu) pays earlier, with the separate pass's bits: 8192 x 512 -> 512 18.4 -> 16.6, 4096 x 384
+// -> 1536 21.2 -> 19.3, 5000 x 384 -> 1536 24.8 -> 24.1, 8192 x 320 -> 1024 25.1 -> 25.0, 8192 x 264 -> 512 18.4 -> 15.5; not 8192 x 256
+// -> 1024 23.6 -> 24.8, 8192 x 128 -> 512 12.9 -> 14.0.
+extern "C" int64_t rte_swiglu_fuse_min_fwd(int32_t K) { return K > 256 && K <= 512 ? 4000000 : rte_swiglu_fuse_min(0); }
 
 extern "C" int rte_gemm_wgrad_splits(const rte_gemm_args* a, int32_t max_splits) {
   if (a == nullptr || a->M <= 0 || a->N <= 0 || a->K <= 0) return 1;

@@ -500,7 +500,7 @@ struct PackedFfn : Function<PackedFfn> {
     const Tensor &x16 = conv[0], &wug16 = conv[1], &wd16 = conv[2];
     const Tensor ug = empty({N, 2 * m}, BF, x), z = empty({N, m}, BF, x), y = empty({N, wdown.size(1)}, direct(x.scalar_type()) ? x.scalar_type() : F32, x);
     if (N > 0) {
-      if (m % 64 == 0 && N * m >= rte_swiglu_fuse_min(0)) {
+      if (m % 64 == 0 && N * m >= rte_swiglu_fuse_min_fwd(d)) {
         Gemm(dev, ptr(x16), d, false, ptr(wug16), d, false, ptr(z), m, N, 2 * m, d, RTE_EPI_SWIGLU_FWD).pair(ptr(ug), 2 * m, m).run();
       } else {
         mm_oi(dev, x16, wug16, ug);

@@ -994,7 +994,7 @@ class TrainEngine:
 
     def _fuse_swiglu(self, rows: int, backward: bool = False) -> bool:
         """SwiGLU inside the tcgen05 product's epilogue?  For large activations, where it is the faster form (the two lines and
-        their times stand beside `rte_swiglu_fuse_min`); below them the separate pass finds its input in L2 and the product can take the kernels
+        their times stand beside `rte_swiglu_fuse_min` and `rte_swiglu_fuse_min_fwd`); below them the separate pass finds its input in L2 and the product can take the kernels
         for few tiles.  Backward also beyond the few-row kernel's range up to `swiglu_fuse_max_rows` rows, whatever the width:
         the gradient of the hidden activations then stays in the fp32 accumulators instead of being rounded to bf16 between the
         two passes (512 x 128 -> 512: 6.0 us against 4.9; with the rounding the gradient of wug is 0.8 % further from the fp32
@@ -1003,6 +1003,8 @@ class TrainEngine:
             return False
         if backward and getattr(self.ops, "small_gemm_rows", 0) < rows <= self.swiglu_fuse_max_rows:
             return True
+        if not backward and hasattr(self.ops, "swiglu_fuse_min_fwd"):
+            return rows * self.cfg.d_ff >= self.ops.swiglu_fuse_min_fwd(self.cfg.d_model)
         return rows * self.cfg.d_ff >= getattr(self.ops, "swiglu_fuse_min_bwd" if backward else "swiglu_fuse_min", 0)
 
     def _block_fwd(self, blk: _Block, x_in: torch.Tensor) -> torch.Tensor:

@@ -84,6 +84,10 @@ class CudaOps:
             self.status.zero_()
             raise A.RteError(f"device status {code}: {self.lib.rte_status_string(code).decode()}")
 
+    def swiglu_fuse_min_fwd(self, K: int) -> int:
+        """`swiglu_fuse_min` behind a product with a reduction of length K."""
+        return int(self.lib.rte_swiglu_fuse_min_fwd(K))
+
     def _deferred(self):
         import contextlib
         ps = self.param_stream

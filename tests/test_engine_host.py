@@ -1,10 +1,13 @@
 """Host-side logic of the engine (hand-written backward sequencing, buffer reuse, optimiser plan)
 checked against the CPU oracle with the test-only operator emulation (tests/emul_ops.py)."""
+from types import SimpleNamespace
+
 import numpy as np
 import pytest
 import torch
 
 from oracle import rte_oracle as O
+from speedup_thingy_b200 import _abi as A
 from speedup_thingy_b200.config import ExperimentConfig, ModelConfig, OutputConfig, TrainingConfig
 from speedup_thingy_b200.engine import TrainEngine, init_parameters, parameter_shapes
 from tests.emul_ops import EmulOps
@@ -493,3 +496,15 @@ def test_swiglu_backward_keeps_fp32_hidden_gradients_up_to_the_row_limit():
             by_size = limit > 0 and rows * f >= 1_000_000
             assert eng._fuse_swiglu(rows, backward=True) == (by_size or 256 < rows <= limit), (limit, rows)
             assert eng._fuse_swiglu(rows) == (limit > 0 and rows * f >= 12_000_000), (limit, rows)
+
+
+def test_swiglu_forward_fuses_earlier_behind_the_reductions_of_the_resident_kernel():
+    cfg, _, _ = _pair("dense")
+    params = init_parameters(cfg.model, seed=0, num_clusters=cfg.output.num_clusters)
+    eng = TrainEngine(cfg, params, device="cpu", ops=EmulOps(), use_cuda_graph=False)
+    eng.ops.swiglu_fuse_min_fwd = A.load().rte_swiglu_fuse_min_fwd
+    f = cfg.model.d_ff
+    for d in (64, 256, 264, 512, 520, 768, 1024):
+        eng.cfg = SimpleNamespace(d_ff=f, d_model=d)
+        line = 4_000_000 if 256 < d <= 512 else 12_000_000
+        assert [eng._fuse_swiglu(rows) for rows in ((line - 1) // f, -(-line // f))] == [False, True], d

@@ -407,6 +407,31 @@ def test_embedding_fwd_bwd(ops):
     _close(dt2, 2 * torch.zeros(V, d).index_add_(0, tok, dx), 1e-5, "embedding grad accumulates")
 
 
+@pytest.mark.parametrize("M,F_,K", [(300, 512, 384), (1090, 64, 320), (129, 192, 512), (5003, 1536, 328), (24600, 512, 384)])
+def test_swiglu_forward_has_the_bits_of_the_route_it_replaces(ops, M, F_, K):
+    """rte_gemm_bf16 with SwiGLU where A stays resident: below the line of `rte_swiglu_fuse_min` the bits of the product and the separate
+    pass, above it those of the persistent kernel.  Row i of A picks column i % K of B, so the gates are chosen: every finite bf16
+    number up to 2^100 in turn, those from -88.7 to -87.3 (whose denominators are above 2^126) most often."""
+    g = torch.Generator().manual_seed(M)
+    far = torch.tensor([-87.5, -88.0, -88.5, -86.5, -89.0, -64.5, -1.0, 90.0]).bfloat16()
+    every = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    every = every[every.abs().float() < 2.0 ** 100]
+    gate = every[torch.randint(0, len(every), (F_, K), generator=g)]
+    gate[::3] = far[torch.randint(0, len(far), (F_, K), generator=g)][::3]
+    b = torch.cat([torch.randn(F_, K, generator=g).bfloat16(), gate]).to(DEV)
+    a = torch.nn.functional.one_hot(torch.arange(M) % K, K).bfloat16().to(DEV)
+    ug, z, want_ug, want = (torch.full((M, n), 7.0, dtype=torch.bfloat16, device=DEV) for n in (2 * F_, F_, 2 * F_, F_))
+    ops.gemm(a, b, z, M=M, N=2 * F_, K=K, epilogue=A.EPI_SWIGLU_FWD, out2=ug, pair=F_)
+    if M * F_ < ops.swiglu_fuse_min:
+        ops.gemm(a, b, want_ug, M=M, N=2 * F_, K=K)
+        ops.swiglu_fwd(want_ug, want, M, F_)
+    else:
+        ops.gemm(a, b, want, M=M, N=2 * F_, K=K, epilogue=A.EPI_SWIGLU_FWD, out2=want_ug, pair=F_, tile_n=256)
+    ops.check_status()
+    assert torch.equal(ug.view(torch.int16), want_ug.view(torch.int16))
+    assert torch.equal(z.view(torch.int16), want.view(torch.int16))
+
+
 @pytest.mark.parametrize("V,d,n,same", [(2048, 132, 2500, 700), (300, 512, 600, 17), (5000, 1024, 3000, 16), (700, 128, 3000, 2000), (9, 4, 70000, 0)])
 def test_embedding_bwd_of_grouped_tokens(ops, V, d, n, same):
     """Tokens grouped by id ahead: the bits of the ungrouped sum -- ids of one piece, of several, of exactly a piece, absent ids, a
