@@ -213,23 +213,25 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
       if (SWIGLU) {
         const int row = y + lane, col = n * (BN / 2) + 32 * part;
-        if (row >= p.M || col >= p.pair_off) continue;
-        __nv_bfloat16* ug = p.C2 + size_t(row) * p.ldc2 + col;
-        by_row(ug, v0);
-        by_row(ug + p.pair_off, v1);
-        // z = up * silu(gate) from the ROUNDED up and gate: what backward re-reads must agree with what was multiplied here
+        if (row < p.M && col < p.pair_off) {
+          __nv_bfloat16* ug = p.C2 + size_t(row) * p.ldc2 + col;
+          by_row(ug, v0);
+          by_row(ug + p.pair_off, v1);
+          // z = up * silu(gate) from the ROUNDED up and gate: what backward re-reads must agree with what was multiplied here
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const float2 u = rte::unpack_bf16x2(v0[j]), g = rte::unpack_bf16x2(v1[j]);
-          v0[j] = EXACT ? rte::pack_bf16x2(u.x * rte::silu_of_bf16(g.x), u.y * rte::silu_of_bf16(g.y))
-                        : rte::pack_bf16x2(u.x * (g.x * fast_sigmoid(g.x)), u.y * (g.y * fast_sigmoid(g.y)));
+          for (int j = 0; j < 16; ++j) {
+            const float2 u = rte::unpack_bf16x2(v0[j]), g = rte::unpack_bf16x2(v1[j]);
+            v0[j] = EXACT ? rte::pack_bf16x2(u.x * rte::silu_of_bf16(g.x), u.y * rte::silu_of_bf16(g.y))
+                          : rte::pack_bf16x2(u.x * (g.x * fast_sigmoid(g.x)), u.y * (g.y * fast_sigmoid(g.y)));
+          }
+          by_row(p.C + size_t(row) * p.ldc + col, v0);
         }
-        by_row(p.C + size_t(row) * p.ldc + col, v0);
       } else {
         const int col = n * BN + 64 * part;
         if (y < p.M && col < p.N) by_tma(v0, col, y);
         if (y < p.M && col + 32 < p.N) by_tma(v1, col + 32, y);
       }
+      __syncwarp();                            // (lanes whose row lies outside stored nothing: the next tile's loads from TMEM want the whole warp)
     }
     if (lane == 0) bulk_wait_read<0>();
     __syncwarp();

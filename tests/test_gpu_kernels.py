@@ -407,6 +407,28 @@ def test_embedding_fwd_bwd(ops):
     _close(dt2, 2 * torch.zeros(V, d).index_add_(0, tok, dx), 1e-5, "embedding grad accumulates")
 
 
+@pytest.mark.parametrize("M,F_,K,ctas", [(37, 32, 64, 2), (431, 160, 72, 2), (1001, 320, 136, 6), (2050, 192, 64, 4), (777, 2080, 8, 148)])
+def test_gemm_resident_swiglu_edges(ops, M, F_, K, ctas):
+    """SwiGLU's forward through rte_gemm_bf16_resident: one k-block and a ragged last one, (up, gate) pairs that end 32 or 64 columns into a
+    tile, several tiles per pair whose last rows fill no warp; nothing is written past the rows or between them."""
+    g = torch.Generator().manual_seed(M + K)
+    a, b = torch.randn(M, K, generator=g).bfloat16().to(DEV), (torch.randn(2 * F_, K, generator=g) * K ** -0.5).bfloat16().to(DEV)
+    ug, z = (torch.full((M + 1, n + 16), 7.0, device=DEV, dtype=torch.bfloat16) for n in (2 * F_, F_))
+    args = A.GemmArgs()
+    args.M, args.N, args.K, args.splits, args.status = M, 2 * F_, K, 1, ops.status.data_ptr()
+    args.A, args.lda, args.B, args.ldb, args.epilogue = a.data_ptr(), K, b.data_ptr(), K, A.EPI_SWIGLU_FWD
+    args.C, args.ldc, args.C2, args.ldc2, args.b_pair_offset = z.data_ptr(), F_ + 16, ug.data_ptr(), 2 * F_ + 16, F_
+    A.check(ops.lib.rte_gemm_bf16_resident(C.byref(args), ctas, ops.stream), "rte_gemm_bf16_resident")
+    ops.check_status()
+    _close(ug[:M, : 2 * F_], a.float() @ b.float().t(), 1e-2, "up, gate")
+    want = torch.empty(M, F_, device=DEV, dtype=torch.bfloat16)
+    ops.swiglu_fwd(ug[:M, : 2 * F_].contiguous(), want, M, F_)
+    assert torch.equal(z[:M, :F_], want)
+    assert bool((ug[M] == 7.0).all() and (ug[:, 2 * F_:] == 7.0).all() and (z[M] == 7.0).all() and (z[:, F_:] == 7.0).all())
+    args.ldc = F_ + 8
+    assert ops.lib.rte_gemm_bf16_resident(C.byref(args), ctas, ops.stream) == A.ERR_ALIGNMENT
+
+
 @pytest.mark.parametrize("M,F_,K", [(300, 512, 384), (1090, 64, 320), (129, 192, 512), (5003, 1536, 328), (24600, 512, 384)])
 def test_swiglu_forward_has_the_bits_of_the_route_it_replaces(ops, M, F_, K):
     """rte_gemm_bf16 with SwiGLU where A stays resident: below the line of `rte_swiglu_fuse_min` the bits of the product and the separate
