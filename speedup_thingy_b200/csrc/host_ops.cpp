@@ -482,10 +482,13 @@ struct CrossEntropy : Function<CrossEntropy> {
     const Tensor &lg = saved[0], &tg = saved[1], &lse = saved[2];
     Dev dev(lg);
     const Tensor grad = at::empty_like(lg), dloss = g[0].to(F32).contiguous();         // (softmax - onehot) * dloss[row]
-    if (lse.defined())
-      check(rte_ce_gradient(ptr(lg), lg.scalar_type() == F32, lg.size(1), tg.data_ptr<int64_t>(), f32(dloss), 1, f32(lse), ptr(grad), lg.size(0),
-                            lg.size(1), dev.status, dev.st), "rte_ce_gradient");
-    else run(dev, lg, tg, dloss, empty({lg.size(0)}, F32, lg), grad);
+    int rc = RTE_ERR_UNSUPPORTED;
+    if (lse.defined()) {
+      rc = rte_ce_gradient(ptr(lg), lg.scalar_type() == F32, lg.size(1), tg.data_ptr<int64_t>(), f32(dloss), 1, f32(lse), ptr(grad), lg.size(0), lg.size(1),
+                           dev.status, dev.st);
+      if (rc != RTE_ERR_UNSUPPORTED) check(rc, "rte_ce_gradient");           // (saved-tensor hooks may bring the logits back on another boundary)
+    }
+    if (rc == RTE_ERR_UNSUPPORTED) run(dev, lg, tg, dloss, empty({lg.size(0)}, F32, lg), grad);
     return {grad.to(at::ScalarType(ctx->saved_data["type"].toInt())).view(ctx->saved_data["shape"].toIntVector()), Tensor()};
   }
 };

@@ -326,6 +326,24 @@ def test_cross_entropy_row_widths(rows, V, dtype):
     assert torch.allclose(x.grad.cpu().float(), ref.grad, atol=1e-5, rtol=1e-2 if dtype == torch.bfloat16 else 1e-4)
 
 
+@pytest.mark.parametrize("dtype,V", [(torch.float32, 4096), (torch.bfloat16, 8192), (torch.float32, 9000)])
+def test_cross_entropy_whose_saved_logits_come_back_on_another_boundary(dtype, V):
+    """Logits off the 16-byte boundary whose saved copy (`save_on_cpu`) returns on it: rows of just that length are too long for one
+    kernel in forward and not in backward.  The same gradients as without the hooks."""
+    g = torch.Generator().manual_seed(V)
+    rows = 37
+    buf = torch.empty(rows * V + 1, dtype=dtype, device=DEV)
+    x = buf[1:].view(rows, V)
+    x.copy_(torch.randn(rows, V, generator=g) * 3)
+    x.requires_grad_()
+    targets, w = torch.randint(0, V, (rows,), generator=g).to(DEV), torch.randn(rows, generator=g).to(DEV)
+    want, = torch.autograd.grad(K.k_cross_entropy_unreduced(x, targets), x, w)
+    with torch.autograd.graph.save_on_cpu():
+        loss = K.k_cross_entropy_unreduced(x, targets)
+    got, = torch.autograd.grad(loss, x, w)
+    _close(got, want.cpu(), 1e-6 if dtype == torch.float32 else 2 ** -8)       # (one rounding of the result; the sums' order may differ)
+
+
 @pytest.mark.parametrize("V,dtype", [(512, torch.bfloat16), (511, torch.bfloat16), (8192, torch.bfloat16), (9001, torch.bfloat16), (16384, torch.bfloat16),
                                      (512, torch.float32), (4099, torch.float32), (8192, torch.float32)])
 @pytest.mark.parametrize("level,fill", [(0.0, "-inf"), (-300.0, "-inf"), (0.0, "lowest")])
