@@ -209,15 +209,20 @@ class CudaOps:
         self._call("rte_embed_fwd", _ptr(tokens), _ptr(table), _ptr(out), tokens.numel(), table.shape[1],
                    table.shape[0], _ptr(self.status), self.stream)
 
+    @staticmethod
+    def _embed_accum(name: str, dtable, accum) -> None:
+        if accum.dtype != torch.int64 or accum.numel() < dtable.numel():
+            raise ValueError(f"{name}: accum must be int64 with at least dtable.numel() elements")
+
     def embed_bwd(self, tokens, dx, dtable, accum) -> None:
         """`accum`: int64 scratch of dtable.numel() elements (fixed-point meeting place of the scatter-add)."""
-        if accum.dtype != torch.int64 or accum.numel() < dtable.numel():
-            raise ValueError("embed_bwd: accum must be int64 with at least dtable.numel() elements")
+        self._embed_accum("embed_bwd", dtable, accum)
         self._call("rte_embed_bwd", _ptr(tokens), _ptr(dx), _ptr(dtable), _ptr(accum), tokens.numel(), dtable.shape[1],
                    dtable.shape[0], _ptr(self.status), self.stream)
 
     def embed_bwd_group(self, tokens, dtable, accum) -> bool:
         """Orders the tokens by id in `accum` ahead of `embed_bwd_grouped`; False where only `embed_bwd` serves."""
+        self._embed_accum("embed_bwd_group", dtable, accum)
         rc = self.lib.rte_embed_bwd_group(_ptr(tokens), _ptr(dtable), _ptr(accum), tokens.numel(), dtable.shape[1], dtable.shape[0],
                                           _ptr(self.status), self.stream)
         if rc == A.ERR_UNSUPPORTED:
@@ -227,6 +232,10 @@ class CudaOps:
         return True
 
     def embed_bwd_grouped(self, n_tokens: int, dx, dtable, accum) -> None:
+        """`embed_bwd` of the tokens that the last `embed_bwd_group` with this `accum` and `dtable` ordered, `n_tokens` of them."""
+        self._embed_accum("embed_bwd_grouped", dtable, accum)
+        if dx.numel() != n_tokens * dtable.shape[1]:
+            raise ValueError(f"embed_bwd_grouped: dx must hold {n_tokens} rows of {dtable.shape[1]}, got {tuple(dx.shape)}")
         self._call("rte_embed_bwd_grouped", _ptr(dx), _ptr(dtable), _ptr(accum), n_tokens, dtable.shape[1], dtable.shape[0], self.stream)
 
     def rmsnorm_fwd(self, x, w, y_bf16, rstd, *, y_f32=None, film_gamma=None, film_beta=None, eps: float = 1e-5,

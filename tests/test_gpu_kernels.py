@@ -475,6 +475,23 @@ def test_embedding_bwd_of_grouped_tokens(ops, V, d, n, same):
         assert torch.equal(one.isnan(), two.isnan()) and torch.equal(one.nan_to_num(), two.nan_to_num())
 
 
+def test_embedding_bwd_scratch_of_another_size_is_refused(ops):
+    V, d, n = 2048, 128, 4096
+    tok, dx, table = torch.zeros(n, dtype=torch.int64, device=DEV), torch.zeros(n, d, device=DEV), torch.zeros(V, d, device=DEV)
+    good = torch.empty(V * d, dtype=torch.int64, device=DEV)
+    for bad in (good[:-1], good.view(torch.int32), torch.empty(V * d, device=DEV)):
+        for call in (lambda a: ops.embed_bwd(tok, dx, table, a), lambda a: ops.embed_bwd_group(tok, table, a),
+                     lambda a: ops.embed_bwd_grouped(n, dx, table, a)):
+            with pytest.raises(ValueError, match="accum"):
+                call(bad)
+    assert ops.embed_bwd_group(tok, table, good)
+    for rows, grad in ((n + 1, dx), (n, dx[:-1]), (n, dx[:, :-4])):
+        with pytest.raises(ValueError, match="rows"):
+            ops.embed_bwd_grouped(rows, grad, table, good)
+    ops.embed_bwd_grouped(n, dx, table, good)
+    ops.check_status()
+
+
 @pytest.mark.parametrize("V,d,n", [(4096, 64, 700), (2000, 65, 1000), (1999, 128, 1000)])
 def test_embedding_bwd_of_a_table_larger_than_the_batch(ops, V, d, n):
     """Only the batch's rows of the accumulator are cleared and applied (the line is at twice the tokens); repeated tokens
