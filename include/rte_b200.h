@@ -125,8 +125,11 @@ int64_t rte_swiglu_fuse_min_fwd(int32_t K);
  * (1..8, at most one per 64-wide k-block) CTAs of a cluster, which add their partial tiles in rank order.  RTE_EPI_BF16 or
  * RTE_EPI_F32 (+R); no grouping, no splits; either major for either operand.                                       */
 int rte_gemm_bf16_tile(const rte_gemm_args* args, int32_t tile_n, int32_t ksplit, rte_stream_t stream);
-/* For K <= 512 and many tiles: A [M,K] stays in shared memory while B streams past (BF16 and SWIGLU_FWD epilogues, A K-major, B
- * either way, all addresses and row strides on 16 bytes).  ctas: how many CTAs at most (pairs of them work together).        */
+/* For K <= 512 and many tiles: A [M,K] stays in shared memory while B streams past.  RTE_EPI_BF16 (B either way) and
+ * RTE_EPI_SWIGLU_FWD (B K-major, b_pair_offset a multiple of 32, N twice that); A K-major, no R, splits or groups.  ctas >= 2: how
+ * many CTAs at most (pairs of them work together).  RTE_ERR_ALIGNMENT unless A and B lie on 16 bytes with lda % 8 == ldb % 8 == 0 and
+ * C (and C2) on 32 bytes with ldc % 16 == 0 (ldc2 % 16 == 0).  z has the bits of rte_swiglu_fwd below
+ * rte_swiglu_fuse_min(0) hidden activations, those of rte_gemm_bf16's other epilogue from there on.                 */
 int rte_gemm_bf16_resident(const rte_gemm_args* args, int32_t ctas, rte_stream_t stream);
 /* The same product for FEW ROWS (the audited samples' replay, models.py:605-679: M = one or two samples): one
  * 256-thread CTA per 64x64 or 64x32 output tile, cp.async + mma.sync, no tensor maps or TMEM set-up, so a dependent chain of

@@ -332,7 +332,8 @@ int launch_resident(const rte_gemm_args* a, int ctas, cudaStream_t st) {
 
 }  // namespace
 
-// What the kernel takes: rows that start on 32 bytes (the stores' sectors), (up, gate) pairs in whole pieces.
+// What the kernel takes: rows of results that start on 32 bytes (SwiGLU's stores are whole sectors; plain results leave by the TMA and could do
+// with 16, not measured), (up, gate) pairs in whole pieces.
 extern "C" int rte_gemm_bf16_resident(const rte_gemm_args* a, int32_t ctas, rte_stream_t stream) {
   RTE_CHECK_ARG(a != nullptr && a->A && a->B && a->C && a->M > 0 && a->N > 0 && a->K > 0 && a->K <= MAX_KB * BK && ctas >= 2);
   RTE_CHECK_ARG(a->epilogue == RTE_EPI_BF16 || a->epilogue == RTE_EPI_SWIGLU_FWD);
