@@ -37,14 +37,6 @@ __device__ __forceinline__ void st_global_v8(void* p, uint32_t a, uint32_t b, ui
                ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d), "r"(e), "r"(f), "r"(g), "r"(h) : "memory");
 }
 
-// 1 / (1 + exp(-g)) in four instructions: what it goes into is rounded to bf16, so flushed denormals and the last bits of the two
-// approximations do not show; exp(-g) = infinity gives 0, as it should.
-__device__ __forceinline__ float fast_sigmoid(float g) {
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * -1.4426950408889634f));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
-  return r;
-}
 struct ResidentParams {
   int M, N, b_mn, pair_off;
   __nv_bfloat16 *C, *C2;        // (SwiGLU)
@@ -222,7 +214,7 @@ gemm_resident_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           for (int j = 0; j < 16; ++j) {
             const float2 u = rte::unpack_bf16x2(v0[j]), g = rte::unpack_bf16x2(v1[j]);
             v0[j] = EXACT ? rte::pack_bf16x2(u.x * rte::silu_of_bf16(g.x), u.y * rte::silu_of_bf16(g.y))
-                          : rte::pack_bf16x2(u.x * (g.x * fast_sigmoid(g.x)), u.y * (g.y * fast_sigmoid(g.y)));
+                          : rte::pack_bf16x2(u.x * rte::fast_silu(g.x), u.y * rte::fast_silu(g.y));
           }
           by_row(p.C + size_t(row) * p.ldc + col, v0);
         }

@@ -70,12 +70,6 @@ struct KParams {
 };
 
 // ------------------------------------------------------------------ epilogue helpers
-// SiLU / sigmoid for the fused epilogues: ex2.approx + the fast divide (2 ulp), with no slow path for huge or
-// denormal denominators (an IEEE divide takes hundreds of cycles there and would stall the whole epilogue warp).
-// The results are rounded to bf16 right away, so the difference from the exact functions is far below one bf16 ulp.
-__device__ __forceinline__ float fast_sigmoid(float g) { return __fdividef(1.f, 1.f + __expf(-g)); }
-__device__ __forceinline__ float fast_silu(float g) { return __fdividef(g, 1.f + __expf(-g)); }
-
 __device__ __forceinline__ void store_bf16x32(__nv_bfloat16* dst, const float (&v)[32], int ncols_valid) {
   if (ncols_valid >= 32 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
     uint4* d4 = reinterpret_cast<uint4*>(dst);
@@ -444,7 +438,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 #pragma unroll
               for (int j = 0; j < 16; ++j) {
                 const float2 g_ = rte::unpack_bf16x2(g[j]);
-                form(j, __uint_as_float(raw[2 * j]), __uint_as_float(raw[2 * j + 1]), fast_sigmoid(g_.x), fast_sigmoid(g_.y));
+                form(j, __uint_as_float(raw[2 * j]), __uint_as_float(raw[2 * j + 1]), rte::fast_sigmoid(g_.x), rte::fast_sigmoid(g_.y));
               }
             }
 #pragma unroll
@@ -573,7 +567,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
                 const float2 u_ = rte::unpack_bf16x2(upk[4 * c + i]), g_ = rte::unpack_bf16x2(gpk[4 * c + i]);
-                zz[i] = rte::pack_bf16x2(u_.x * fast_silu(g_.x), u_.y * fast_silu(g_.y));
+                zz[i] = rte::pack_bf16x2(u_.x * rte::fast_silu(g_.x), u_.y * rte::fast_silu(g_.y));
               }
               put16(slot, c, zz[0], zz[1], zz[2], zz[3]);
             }
@@ -626,7 +620,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                   // round to bf16 first: the saved (up | gate) and z must agree with what backward re-reads
                   up[j] = __bfloat162float(__float2bfloat16_rn(__uint_as_float(raw[j])));
                   gt[j] = __bfloat162float(__float2bfloat16_rn(__uint_as_float(rawg[j])));
-                  v[j] = up[j] * fast_silu(gt[j]);
+                  v[j] = up[j] * rte::fast_silu(gt[j]);
                 }
                 const int nv = p.pair_off - col;
                 store_bf16x32(ug + col, up, nv);
@@ -648,7 +642,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
                   const float dz = __uint_as_float(raw[j]);
-                  const float sg = fast_sigmoid(gt[j]);
+                  const float sg = rte::fast_sigmoid(gt[j]);
                   v[j] = dz * gt[j] * sg;                                    // d up
                   dg[j] = dz * up[j] * sg * (1.f + gt[j] * (1.f - sg));      // d gate
                 }

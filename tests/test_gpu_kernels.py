@@ -407,6 +407,24 @@ def test_embedding_fwd_bwd(ops):
     _close(dt2, 2 * torch.zeros(V, d).index_add_(0, tok, dx), 1e-5, "embedding grad accumulates")
 
 
+def test_fused_silu_is_within_its_bound_for_every_gate(ops):
+    """z of the persistent kernel's epilogue for up = 1 and all bf16 gates above -64: (4 + 2 |g|) 2^-24 of the quotient and one rounding to
+    bf16 (8 significant bits: 2^-8 of the result, 2^-134 among the subnormal ones)."""
+    every = torch.arange(65536, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    every = every[(every.float() > -64) & (every.abs().float() < 2.0 ** 100)]
+    K, F_ = 128, 512
+    gate = torch.ones(F_ * K).bfloat16()
+    gate[: len(every)] = every
+    b = torch.cat([torch.ones(F_, K).bfloat16(), gate.view(F_, K)]).to(DEV)
+    a = torch.eye(K).bfloat16().to(DEV)
+    ug, z = torch.empty(K, 2 * F_, dtype=torch.bfloat16, device=DEV), torch.empty(K, F_, dtype=torch.bfloat16, device=DEV)
+    ops.gemm(a, b, z, M=K, N=2 * F_, K=K, epilogue=A.EPI_SWIGLU_FWD, out2=ug, pair=F_, tile_n=256)
+    ops.check_status()
+    g = ug[:, F_:].double()
+    want = g / (1 + torch.exp(-g))
+    assert bool(((z.double() - want).abs() <= (2.0 ** -8 + (4 + 2 * g.abs()) * 2.0 ** -24) * want.abs() + 2.0 ** -134).all())
+
+
 @pytest.mark.parametrize("M,F_,K,ctas", [(37, 32, 64, 2), (431, 160, 72, 2), (1001, 320, 136, 6), (2050, 192, 64, 4), (777, 2080, 8, 148)])
 def test_gemm_resident_swiglu_edges(ops, M, F_, K, ctas):
     """SwiGLU's forward through rte_gemm_bf16_resident: one k-block and a ragged last one, (up, gate) pairs that end 32 or 64 columns into a
