@@ -115,6 +115,44 @@ def test_scores_of_gates_far_below_zero_keep_their_order(gate_m, product_m):
     assert torch.equal(sel.cpu().bool(), place < 20)
 
 
+@pytest.mark.parametrize("rows,F_,up_m,gate_m,product_m,top_k", [
+    (60, 2048, 300, 280, 310, 256),                  # three lists, more candidates than are selected
+    (300, 132, 40, 30, 20, 25),                      # F % 8 == 4
+    (50, 260, 90, 0, 60, 64), (50, 260, 0, 70, 0, 33), (50, 1028, 120, 40, 0, 100),       # a list or two missing
+    (3700, 64, 20, 20, 20, 7),                       # several tokens per warp
+    (40, 128, 128, 0, 5, 60), (33, 4, 3, 2, 2, 2),   # everything a candidate; one group of four
+])
+@pytest.mark.parametrize("spread", [False, True])
+def test_selection_is_bit_exact_over_all_lists(rows, F_, up_m, gate_m, product_m, top_k, spread):
+    """Selected neurons and candidate counts against the oracle in 64 bits, where no score hangs on a last bit: four gates whose SiLU differ by
+    more than 0.2 % from one another's multiples, norms that are powers of two, ups of two mantissa bits -- so scores are equal or far
+    apart, and many more than 32 share a key and a score across every cut.  `spread`: bf16 ups of all mantissas in rows of one gate."""
+    ops = CudaOps(DEV)
+    g = torch.Generator().manual_seed(F_ + top_k)
+    gates = torch.tensor([1.0, 20.0, -3.0, 0.0])
+    pick = lambda *s: torch.randint(0, s[0], s[1:], generator=g)  # noqa: E731
+
+    def side():
+        sign = 1 - 2 * pick(2, rows, F_).float()
+        if spread:
+            return torch.randn(rows, F_, generator=g).bfloat16().float(), gates[pick(3, rows, 1)].expand(rows, F_)
+        return sign * (1 + pick(4, rows, F_) * 0.25) * 2.0 ** pick(3, rows, F_), gates[pick(4, rows, F_)]
+
+    (uh, gh), (up, gate) = side(), side()
+    wn = 2.0 ** pick(3, F_).float()
+    hats, ug = torch.cat([uh, gh], dim=1).to(DEV), torch.cat([up, gate], dim=1).bfloat16().to(DEV)
+    z, sel = torch.empty(rows, F_, dtype=torch.bfloat16, device=DEV), torch.empty(rows, F_, dtype=torch.uint8, device=DEV)
+    cnt = torch.empty(rows, dtype=torch.int32, device=DEV)
+    ops.svd_ffn_select(hats, ug, wn.to(DEV), z, sel, cnt, up_m=up_m, gate_m=gate_m, product_m=product_m, top_k=top_k)
+    ops.check_status()
+    cand = O.svd_ffn_candidates(uh.double(), gh.double(), wn.double(), up_m, gate_m, product_m)
+    zd = up.double() * torch.nn.functional.silu(gate.double())
+    want = O.svd_ffn_select(zd, cand, wn.double(), top_k)
+    assert torch.equal(cnt.cpu().long(), cand.sum(-1))
+    assert torch.equal(sel.cpu().bool(), want)
+    assert torch.equal(z.cpu() != 0, want & (zd != 0))
+
+
 @pytest.mark.parametrize("rows,F_", [(37, 2048), (5, 100)])            # eight neurons per thread | one
 def test_swiglu_backward_of_the_selected_neurons(rows, F_):
     ops = CudaOps(DEV)
