@@ -233,6 +233,42 @@ def test_pipelined_train_steps_equal_synchronous_steps():
         assert torch.equal(a.params[n], b.params[n]), n
 
 
+@pytest.mark.parametrize("name", ["macro_audit_two_banks", "macro_shortlist", "exact_one_bank"])
+@pytest.mark.parametrize("pinned", [True, False])
+def test_steps_in_flight_keep_their_inputs_and_results_apart(name, pinned):
+    """Two steps in flight behind a busy device (so that every copy of a step's inputs, random negatives among them, and of the results of the
+    step before waits), one pair of host tensors for all batches, overwritten as soon as `submit` returns, evaluations between
+    the phases: the losses, metrics and weights of one synchronous step after the other on batches of their own."""
+    model, train, *rest = CASES[name]
+    cfg, params, a = _engine(model, train, *rest)
+    _, _, b = _engine(model, train, *rest)
+    batches = [x for _, x in zip(range(21), _stream(cfg, 21))]
+    buf = [t.clone().pin_memory() if pinned else t.clone() for t in batches[0]]
+
+    def submit(batch):
+        for dst, src in zip(buf, batch):
+            dst.copy_(src)
+        torch.cuda._sleep(4_000_000)                       # about two milliseconds
+        b.submit(tuple(buf))
+        for t in buf:
+            t.fill_(1)
+
+    for phase in range(3):
+        steps, held = batches[7 * phase:7 * phase + 5], batches[7 * phase + 5:7 * phase + 7]
+        want, got = [a.train_step(x) for x in steps], []
+        for x in steps:
+            if len(b._pending) == b.MAX_IN_FLIGHT:
+                got.append(b.collect())
+            submit(x)
+        while b._pending:
+            got.append(b.collect())
+        assert [r.loss for r in got] == [r.loss for r in want]
+        assert [r.metrics for r in got] == [r.metrics for r in want]
+        assert b.evaluate(held + held) == a.evaluate(held + held)
+    for n in a.params:
+        assert torch.equal(a.params[n], b.params[n]), n
+
+
 def test_c3_shapes_one_step_finite_and_close():
     """The c3 workload's shapes without the audited sample: one step against the fp32 oracle."""
     model = dict(vocab_size=2048, d_model=512, n_heads=8, d_ff=2048, n_prelude=1, n_coda=1, t_max=4, depth_choices=(1, 2, 4),
