@@ -514,11 +514,12 @@ def main() -> None:
                                 "peak_sustained": peaks["bf16_tflops_sustained"],
                                 # DRAM bytes per launch (read + write), mean over the hot-pass shapes of the ncu capture
                                 # summarised in profiles/gemm_tcgen05_c3_shapes_ncu_full.md (cold operand reads; outputs that
-                                # fit the L2 do not reach DRAM inside the launch); only meaningful for workload c3
+                                # fit the L2 do not reach DRAM inside the launch; the products that gemm_resident_kernel takes
+                                # move the same bytes); only meaningful for workload c3
                                 "traffic": 41.0e6 if args.config == "c3" else None,
                                 "traffic_unit": "bytes per launch (ncu dram__bytes_read+write, c3 shapes)",
                                 "of": which + " (burst)",
-                                "kernel": "gemm_tcgen05_kernel", "launches_per_step": roof["launches"],
+                                "kernel": "gemm_tcgen05_kernel, gemm_resident_kernel, gemm_tile_kernel (by shape)", "launches_per_step": roof["launches"],
                                 "gemm_ms_per_step": roof["gemm_ms_per_step"],
                                 "timing": "event-record nodes around each launch inside a captured step",
                                 "scope": "hot-pass launches (main stream + its weight-gradient stream); the audit replay's "

@@ -96,7 +96,7 @@ embed_bwd_rows_kernel(const int64_t* __restrict__ tokens, unsigned long long* __
 // accumulate and apply -> grouped: 8192 x 512 of 2048 ids 24.5 -> 10.9, 16384 x 512 45 -> 24, 8192 x 1024 of 32768 ids 80 -> 30; 512 x 128
 // 5.3 -> 6.3, hence the line at 2^18 elements; the grouping itself takes 4..19 us beside other work).
 constexpr int EG_THREADS = 1024, EG_PIECE = 16, EG_COLS = 128;
-constexpr int EG_MAX_VOCAB = 48 * 1024;                      // one counter per id in shared memory
+constexpr int EG_MAX_VOCAB = 48 * 1024;                      // one counter per id in shared memory, 192 KB (56 K would fit; the configurations here stop at 32768)
 struct EmbedGroups {
   int* head;                 // [0]: pieces
   int4* piece;               // id, first entry of `order`, entries | pieces of the id << 8, row of `sums` (< 0: the id's only piece)

@@ -15,7 +15,8 @@
 // half (a row of equal scores), the search goes on over the full scores.  Results are bit-exact with a stable sort by (value
 // descending, index ascending), the tie rule of this build.
 //
-// What bounds it: the instructions of a token, waited for by the loads of its scores (24 warps on an SM, 9 KB of shared memory each).
+// What bounds it: 9.5 K instructions per token at 54 % of the issue slots, and the loads they wait for (24 warps on an SM, 9 KB of shared
+// memory each; per instruction issued 3.2 warps wait on global loads, 2.0 on fixed latencies, 1.0 on shared memory; DRAM at 35 %).
 // us, with 32-bit keys and a divide for every list -> now: 16384 tokens, F = 2048, k = 256 377 -> 271, 5000 x 2000, k = 200
 // 172 -> 165, 3000 x 512, k = 60 44 -> 27.  The SiLU of the fp32 lists is the correctly rounded quotient, made once for two lists (302 us
 // with a divide for each, 245 with an approximate reciprocal, which loses the order of gates below -87).  With all keys in
