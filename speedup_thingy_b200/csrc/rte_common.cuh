@@ -101,11 +101,11 @@ __device__ __forceinline__ float block_max(float v, float* red) {
 __device__ __forceinline__ float silu_f(float g) { return g / (1.f + __expf(-g)); }
 __device__ __forceinline__ float sigmoid_f(float g) { return 1.f / (1.f + __expf(-g)); }
 
-// SiLU and sigmoid of the fused epilogues of large products: four instructions, no slow path for huge denominators (a correctly rounded
-// divide's stalls the whole epilogue warp; with the intrinsics, whose bits these are, 16384 x 512 -> 2048 takes 80.0 us instead of
-// 76).  Relative error up to (4 + 2 |g|) 2^-24 for g > -64, most of it the exp's (all 2^32 arguments compared with 64 bits; with a
-// correctly rounded quotient (3.5 + 2 |g|) 2^-24); 0 below -87.3, where the denominator passes 2^126.  What they go into is
-// rounded to bf16.
+// SiLU and sigmoid of the fused epilogues of large products: 1 / (1 + 2^(-g log2 e)) with the approximate ex2 and rcp of the PTX ISA, four
+// instructions and no slow path for huge denominators (a correctly rounded divide's stalls the whole epilogue warp; __expf with
+// __fdividef, which give the same for all 2^32 arguments, take 80.0 us instead of 76 for 16384 x 512 -> 2048).  Relative error up to
+// (4 + 2 |g|) 2^-24 for g > -64, most of it the exponential's (all arguments compared with 64 bits; with a correctly rounded
+// quotient (3.5 + 2 |g|) 2^-24); 0 below -87.3, where the denominator passes 2^126.  What they go into is rounded to bf16.
 __device__ __forceinline__ float fast_sigmoid(float g) {
   float e, r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(g * -1.4426950408889634f));
